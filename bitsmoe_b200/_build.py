@@ -1,8 +1,9 @@
-"""In-tree build of the CUDA library: nvcc for sm_100a -> bitsmoe_b200/_lib/libbitsmoe_b200.so.
+"""In-tree build: nvcc for sm_100a -> bitsmoe_b200/_lib/libbitsmoe_b200.so (the C ABI), and with the C++ compiler the
+host path over it, bitsmoe_b200/_lib/_bm_host.so (a CPython module against torch's headers).
 
     python -m bitsmoe_b200._build [--force] [--verbose]
 
-The shared object is loaded with ctypes (bitsmoe_b200.capi); there is no JIT cache and no
+The library is loaded with ctypes (bitsmoe_b200.capi), the host module by the same file; there is no JIT cache and no
 fallback: if the library is missing the package raises when the op is first used.
 """
 from __future__ import annotations
@@ -17,6 +18,8 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(LIB_DIR, "libbitsmoe_b200.so")
+HOST_SRC = os.path.join(CSRC, "host", "bindings.cpp")
+HOST_LIB = os.path.join(LIB_DIR, "_bm_host.so")
 INCLUDE = os.path.join(os.path.dirname(PKG), "include")
 
 NVCC_FLAGS = [
@@ -31,7 +34,7 @@ def sources():
 
 def _stamp() -> str:
     h = hashlib.sha256()
-    for f in sorted(os.listdir(CSRC)) + ["../../include/bitsmoe_b200.h"]:
+    for f in sorted(os.listdir(CSRC)) + ["host/bindings.cpp", "../../include/bitsmoe_b200.h"]:
         p = os.path.normpath(os.path.join(CSRC, f))
         if os.path.isfile(p):
             h.update(f.encode())
@@ -42,7 +45,25 @@ def _stamp() -> str:
 
 def needs_build() -> bool:
     stamp = os.path.join(LIB_DIR, "stamp.txt")
-    return not (os.path.exists(LIB) and os.path.exists(stamp) and open(stamp).read().strip() == _stamp())
+    return not (os.path.exists(LIB) and os.path.exists(HOST_LIB) and os.path.exists(stamp) and open(stamp).read().strip() == _stamp())
+
+
+def build_host() -> None:
+    """The CPython module; it finds the library beside itself ($ORIGIN)."""
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
+           sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + [f"-I{i}" for i in inc]
+    cmd += [HOST_SRC, "-o", HOST_LIB, f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
+            f"-L{LIB_DIR}", "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+        raise RuntimeError("building the host module failed")
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -71,6 +92,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError("link failed")
     for o in objs:
         os.remove(o)
+    build_host()
     with open(os.path.join(LIB_DIR, "stamp.txt"), "w") as f:
         f.write(_stamp())
     return LIB

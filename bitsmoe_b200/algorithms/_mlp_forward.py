@@ -13,6 +13,7 @@ from typing import Dict, Sequence, Tuple
 
 import torch
 
+from bitsmoe_b200 import capi
 from bitsmoe_b200.layer import PackedLayer
 
 _FIELDS = ("payload", "rank_idx", "tile_meta", "slab_meta", "scale", "s")
@@ -39,6 +40,7 @@ def _layer_key(lists: Sequence[Sequence[torch.Tensor]], rank_out: int, intermedi
 
 
 def clear_cache() -> None:
+    capi.host().op_clear()
     for layer in _cache.values():
         layer.close()
     _cache.clear()
@@ -49,6 +51,14 @@ def moe_packed_forward(h_gate, h_up, token_indices, expert_offsets, route_weight
                        up_payload, up_rank_idx, up_tile_meta, up_slab_meta, up_scale, up_s,
                        down_payload, down_rank_idx, down_tile_meta, down_slab_meta, down_scale, down_s,
                        rank_out, intermediate_size, act_type, path: int = 0):
+    # well-formed arguments and weight lists met before: checked and looked up natively (the key is 3 E addresses)
+    out = capi.host().op_forward(h_gate, h_up, token_indices, expert_offsets, route_weights,
+                                 gate_payload, gate_rank_idx, gate_tile_meta, gate_slab_meta, gate_scale, gate_s,
+                                 up_payload, up_rank_idx, up_tile_meta, up_slab_meta, up_scale, up_s,
+                                 down_payload, down_rank_idx, down_tile_meta, down_slab_meta, down_scale, down_s,
+                                 rank_out, intermediate_size, act_type, path)
+    if out is not None:
+        return out
     _check(h_gate.dim() == 2, "h_gate must be 2D [tokens, rank]")
     _check(h_up.dim() == 2, "h_up must be 2D [tokens, rank]")
     _check(h_gate.shape[0] == h_up.shape[0], "h_gate/h_up token dim mismatch")
@@ -88,4 +98,6 @@ def moe_packed_forward(h_gate, h_up, token_indices, expert_offsets, route_weight
         layer = PackedLayer(tabs[0], tabs[1], tabs[2], int(intermediate_size), int(rank_out),
                             rank_in=int(h_gate.shape[1]), act_type=int(act_type), device=h_gate.device)
         _cache[key] = layer
+        capi.host().op_register(*lists, int(rank_out), int(intermediate_size), int(h_gate.shape[1]), h_gate.device.index, layer,
+                                layer._native)
     return layer.experts_forward(h_gate, h_up, token_indices, expert_offsets, route_weights, path=path)

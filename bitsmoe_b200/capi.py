@@ -13,6 +13,7 @@ import torch
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "_lib", "libbitsmoe_b200.so")
+HOST_PATH = os.path.join(_PKG, "_lib", "_bm_host.so")
 
 BM_OK = 0
 BM_F16, BM_BF16, BM_F32 = 0, 1, 2
@@ -40,6 +41,13 @@ class Matrix(C.Structure):
         ("slab_meta", C.c_void_p), ("n_slabs", C.c_int32),
         ("scale", C.c_void_p), ("n_scales", C.c_int64),
         ("s", C.c_void_p),
+    ]
+
+
+class BlockDense(C.Structure):
+    _fields_ = [
+        ("gate_w", C.c_void_p), ("sh_gate", C.c_void_p), ("sh_up", C.c_void_p), ("sh_down", C.c_void_p),
+        ("sh_token_gate", C.c_void_p), ("sh_intermediate", C.c_int32), ("w_dtype", C.c_int32),
     ]
 
 
@@ -75,6 +83,9 @@ _SIGS = {
     "bm_dense_mlp_workspace_bytes": (C.c_size_t, [C.c_int32, C.c_int32]),
     "bm_dense_mlp_forward": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32,
                                        C.c_int32, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_size_t, C.c_void_p]),
+    "bm_block_workspace_bytes": (C.c_size_t, [C.c_void_p, C.POINTER(BlockDense), C.c_int32, C.c_int32, C.c_int32]),
+    "bm_block_forward": (C.c_int, [C.c_void_p, C.POINTER(BlockDense), C.c_void_p, C.c_int, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
+                                   C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_size_t, C.c_void_p]),
     "bm_ep_flag_bytes": (C.c_size_t, []),
     "bm_ep_barrier": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
     "bm_ep_push": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),
@@ -124,6 +135,24 @@ def lib() -> C.CDLL:
             fn.restype, fn.argtypes = res, args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host path (csrc/host/bindings.cpp) over the library."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"bitsmoe_b200 host module not found at {HOST_PATH}; build it with `python -m bitsmoe_b200._build`")
+        import importlib.util
+        spec = importlib.util.spec_from_file_location("_bm_host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    return _host
 
 
 def check(status: int) -> None:

@@ -4,28 +4,11 @@
 //                   (bitsmoe/models/deepseekv2/bitsmoe_block.py:123-124, bitsmoe/models/qwen3next/bitsmoe_block.py:144-147)
 // The products run on the same kernels as the shared-basis projections: the cluster split-K kernel for decode-sized
 // batches, the tcgen05 GEMM above that, a CUDA-core GEMM for shapes neither takes.
-#include "common.cuh"
+#include "skinny.cuh"
 
 namespace bm {
 
-struct SkinnyArgs {
-  const __half* W[2];
-  void* C[2];
-  const void* X;
-  const void* residual;
-  int rows_per_w, n_w;
-  int N, K;
-  int x_dtype, c_dtype;
-  int round_x_f16;
-  int splits;
-  int mrows;
-  float4* zero;
-  int zero_n;
-};
-int launch_skinny_nt(SkinnyArgs a, cudaStream_t st);
 int launch_gemm_nt(const GemmArgs& g, int problems, cudaStream_t st);
-
-constexpr int DENSE_SKINNY_MAX_TOKENS = 256;
 
 // C_i [T, N] = X [T, K] . W_i [N, K]^T for `problems` (1 or 2) weight matrices sharing X; residual (problem 0 only) may
 // be null.  Chooses the kernel by shape.
@@ -33,25 +16,15 @@ int dense_xwT(const void* X, int x_dtype, const __half* W0, const __half* W1, vo
               const void* residual, int T, int N, int K, int problems, int* status, cudaStream_t st) {
   if (T == 0) return BM_OK;
   const bool aligned = (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
-  if (T <= DENSE_SKINNY_MAX_TOKENS && aligned && N % 32 == 0) {
-    // the fewest k-splits whose slice fits shared memory; 32 output rows per CTA when the cluster splits k
-    for (int splits = 1; splits <= 8; splits *= 2) {
-      if (K % (16 * splits)) continue;
-      const int mrows = splits == 1 ? 16 : 32;
-      const size_t smem = static_cast<size_t>(mrows + 64) * (K / splits + 8) * 2 + (splits > 1 ? static_cast<size_t>(mrows) * 64 * 4 : 0);
-      const int ctas = (N * problems / mrows) * splits;
-      if (smem > 160 * 1024 || (splits < 8 && ctas < 96 && K / splits > 256)) continue;   // spread small products over the SMs
-      SkinnyArgs a{};
-      a.W[0] = W0; a.W[1] = problems > 1 ? W1 : W0;
-      a.C[0] = C0; a.C[1] = problems > 1 ? C1 : C0;
-      a.X = X; a.residual = residual;
-      a.rows_per_w = N; a.n_w = problems;
-      a.N = T; a.K = K;
-      a.x_dtype = x_dtype; a.c_dtype = c_dtype; a.round_x_f16 = 1;
-      a.splits = splits; a.mrows = mrows;
-      const int rc = launch_skinny_nt(a, st);
-      if (rc != BM_ERR_UNSUPPORTED) return rc;
-    }
+  if (T <= SKINNY_MAX_TOKENS && aligned && K % 8 == 0) {
+    SkinnyArgs a{};
+    a.n_seg = problems;
+    a.seg[0] = SkSeg{W0, nullptr, C0, N, c_dtype, 0, 0};
+    a.seg[1] = SkSeg{W1, nullptr, C1, N, c_dtype, 0, 0};
+    a.X = X; a.N = T; a.K = K; a.x_dtype = x_dtype; a.residual = residual;
+    a.splits = skinny_splits(N * problems, K);
+    const int rc = launch_skinny_nt(a, st);
+    if (rc != BM_ERR_UNSUPPORTED) return rc;
   }
   if (aligned && K % 64 == 0 && N % 8 == 0) {
     GemmTcArgs t{};
@@ -67,6 +40,32 @@ int dense_xwT(const void* X, int x_dtype, const __half* W0, const __half* W1, vo
   g.a_dtype = x_dtype; g.c_dtype = c_dtype; g.round_a_f16 = x_dtype == BM_F32 ? 1 : 0;
   g.M = T; g.N = N; g.K = K;
   return launch_gemm_nt(g, problems, st);
+}
+
+// The whole MLP of a decode batch in two launches: gate and up rows paired in the same CTA (z = silu(g) * u leaves in
+// fp32) with the per-token gate's logit beside them, then the down product, which scales z by the gate as it rounds it.
+static int dense_mlp_small(const void* x, int x_dtype, const __half* wg, const __half* wu, const __half* wd, const __half* token_gate_w,
+                           int T, int H, int I, const void* residual, void* y, int y_dtype, float* z, float* gate, cudaStream_t st) {
+  if (token_gate_w && x_dtype == BM_F32) return BM_ERR_UNSUPPORTED;     // the gate's logit is taken from the unrounded fp32 row
+  if (T > SKINNY_MAX_TOKENS || H % 8 != 0 || I % 8 != 0 || !skinny_fits(H, 0, 8) || !skinny_fits(I, 0, skinny_splits(H, I)))
+    return BM_ERR_UNSUPPORTED;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wg) | reinterpret_cast<uintptr_t>(wu) | reinterpret_cast<uintptr_t>(wd) |
+       reinterpret_cast<uintptr_t>(token_gate_w)) & 15u)
+    return BM_ERR_UNSUPPORTED;
+  SkinnyArgs a{};
+  a.seg[0] = SkSeg{wg, wu, z, I, BM_F32, 0, 0};
+  a.seg[1] = SkSeg{token_gate_w, nullptr, gate, 1, BM_F32, 0, 0};
+  a.n_seg = token_gate_w ? 2 : 1;
+  a.X = x; a.N = T; a.K = H; a.x_dtype = x_dtype;
+  a.splits = 8;
+  int rc = launch_skinny_nt(a, st);
+  if (rc) return rc;
+  SkinnyArgs d{};
+  d.seg[0] = SkSeg{wd, nullptr, y, H, y_dtype, 0, 0};
+  d.n_seg = 1;
+  d.X = z; d.N = T; d.K = I; d.x_dtype = BM_F32; d.x_gate = token_gate_w ? gate : nullptr; d.residual = residual;
+  d.splits = skinny_splits(H, I);
+  return launch_skinny_nt(d, st);
 }
 
 // gate[t] = sigmoid(x[t] . w): one warp per token.
@@ -133,8 +132,12 @@ extern "C" int bm_dense_mlp_forward(const void* x, int x_dtype, const uint16_t* 
   __half* u = reinterpret_cast<__half*>(ws + mat);
   __half* z = reinterpret_cast<__half*>(ws + 2 * mat);
   float* gate = reinterpret_cast<float*>(ws + 3 * mat);
-  int rc = dense_xwT(x, x_dtype, reinterpret_cast<const __half*>(w_gate), reinterpret_cast<const __half*>(w_up), g, u, BM_F16, nullptr,
-                     T, intermediate, hidden, 2, nullptr, st);
+  int rc = dense_mlp_small(x, x_dtype, reinterpret_cast<const __half*>(w_gate), reinterpret_cast<const __half*>(w_up),
+                           reinterpret_cast<const __half*>(w_down), reinterpret_cast<const __half*>(token_gate_w), T, hidden, intermediate,
+                           residual, y, y_dtype, reinterpret_cast<float*>(ws), gate, st);
+  if (rc != BM_ERR_UNSUPPORTED) return rc;
+  rc = dense_xwT(x, x_dtype, reinterpret_cast<const __half*>(w_gate), reinterpret_cast<const __half*>(w_up), g, u, BM_F16, nullptr,
+                 T, intermediate, hidden, 2, nullptr, st);
   if (rc) return rc;
   if (token_gate_w) {
     row_gate_kernel<<<(T + 7) / 8, 256, 0, st>>>(x, x_dtype, reinterpret_cast<const __half*>(token_gate_w), T, hidden, gate);

@@ -247,6 +247,9 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
     tc::mbar_init_fence();
     abort_raw = 0;
   }
+  // everything above runs while the kernel before this one (launched with programmatic serialisation) drains
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   // ---- passes per expert (ceil(assignments / 8)) and their exclusive prefix: 4 consecutive experts per thread
   int total_passes;
   {
@@ -729,8 +732,17 @@ int launch_experts_decode(const bm_layer* L, const __half* h_gate, const __half*
   P.ring = L->dec_ring;
   P.act_bufs = L->dec_act_bufs;
   P.wait_limit_ns = tc::WAIT_LIMIT_NS;
-  if (L->max_slots <= 128 * 2) experts_decode_kernel<2><<<L->dec_grid, DEC_THREADS, L->dec_smem, st>>>(P);
-  else experts_decode_kernel<DEC_MAX_MB><<<L->dec_grid, DEC_THREADS, L->dec_smem, st>>>(P);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(L->dec_grid);
+  cfg.blockDim = dim3(DEC_THREADS);
+  cfg.dynamicSmemBytes = L->dec_smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  BM_CUDA(cudaLaunchKernelEx(&cfg, L->max_slots <= 128 * 2 ? experts_decode_kernel<2> : experts_decode_kernel<DEC_MAX_MB>, P));
   BM_LAUNCH_CHECK("experts_decode_kernel");
   return BM_OK;
 }

@@ -5,7 +5,7 @@
 #include <new>
 #include <string>
 
-#include "common.cuh"
+#include "skinny.cuh"
 
 namespace bm {
 
@@ -24,22 +24,6 @@ void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 
 // from the other translation units
 int launch_gemm_nt(const GemmArgs& g, int problems, cudaStream_t st);
-struct SkinnyArgs {
-  const __half* W[2];
-  void* C[2];
-  const void* X;
-  const void* residual;
-  int rows_per_w, n_w;
-  int N, K;
-  int x_dtype, c_dtype;
-  int round_x_f16;
-  int splits;
-  int mrows;
-  float4* zero;
-  int zero_n;
-};
-int launch_skinny_nt(SkinnyArgs a, cudaStream_t st);
-constexpr int SKINNY_MAX_TOKENS = 256;
 void plan_fast(const bm_layer* L, size_t base_bytes, FastPlan* P);
 int build_fast(bm_layer* L, const FastPlan& P, cudaStream_t st);
 size_t fast_build_scratch_bytes(const FastPlan& P);
@@ -401,34 +385,22 @@ extern "C" int bm_layer_decode_codes(const bm_layer_t* L, int32_t e, int32_t whi
   return BM_OK;
 }
 
-// `zero` / `zero_bytes`: a buffer (16-byte multiple) the projection kernel clears as a side job; `*zeroed` tells
-// the caller whether the path taken did it.
-static int basis_project_impl(const bm_layer_t* L, const void* x, int x_dtype, int32_t T, uint16_t* h_gate, uint16_t* h_up,
-                              void* zero, size_t zero_bytes, bool* zeroed, void* stream) {
-  if (zeroed) *zeroed = false;
+extern "C" int bm_basis_project(const bm_layer_t* L, const void* x, int x_dtype, int32_t T, uint16_t* h_gate,
+                                uint16_t* h_up, void* stream) {
+  bm::NvtxRange nvtx_range("bm_basis_project");
   BM_REQUIRE(L != nullptr, BM_ERR_INVALID_ARG, "basis_project: null layer");
   BM_REQUIRE(L->vh_gate && L->vh_up, BM_ERR_INVALID_ARG, "missing shared_vh basis for packed routed experts");
   BM_REQUIRE(T >= 0 && x_dtype >= BM_F16 && x_dtype <= BM_F32, BM_ERR_INVALID_ARG, "basis_project: bad arguments");
   if (T == 0) return BM_OK;
   BM_REQUIRE(x && h_gate && h_up, BM_ERR_INVALID_ARG, "basis_project: null pointer");
-  if (T <= SKINNY_MAX_TOKENS && L->hidden % 128 == 0 && L->rank_in % 32 == 0 &&
-      (reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+  if (T <= SKINNY_MAX_TOKENS && L->hidden % 128 == 0) {
     SkinnyArgs a{};
-    a.W[0] = L->vh_gate; a.W[1] = L->vh_up;
-    a.C[0] = h_gate; a.C[1] = h_up;
-    a.X = x; a.residual = nullptr;
-    a.rows_per_w = L->rank_in; a.n_w = 2;
-    a.N = T; a.K = L->hidden;
-    a.x_dtype = x_dtype; a.c_dtype = BM_F16; a.round_x_f16 = 1;
-    a.splits = 8; a.mrows = 32;
-    if (zero != nullptr && zero_bytes % 16 == 0 && (reinterpret_cast<uintptr_t>(zero) & 15u) == 0 && zero_bytes / 16 < (1u << 30)) {
-      a.zero = static_cast<float4*>(zero);
-      a.zero_n = static_cast<int>(zero_bytes / 16);
-      if (zeroed) *zeroed = true;
-    }
+    a.seg[0] = SkSeg{L->vh_gate, nullptr, h_gate, L->rank_in, BM_F16, 0, 0};
+    a.seg[1] = SkSeg{L->vh_up, nullptr, h_up, L->rank_in, BM_F16, 0, 0};
+    a.n_seg = 2;
+    a.X = x; a.N = T; a.K = L->hidden; a.x_dtype = x_dtype; a.splits = 8;
     const int rc = launch_skinny_nt(a, static_cast<cudaStream_t>(stream));
-    if (rc != BM_ERR_UNSUPPORTED) return rc;
-    if (zeroed) *zeroed = false;       // shape does not tile (e.g. a very wide hidden size): the general GEMMs below take it
+    if (rc != BM_ERR_UNSUPPORTED) return rc;       // shape does not tile (e.g. a very wide hidden size): the general GEMMs take it
   }
   if (L->hidden % 64 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
     GemmTcArgs t{};
@@ -450,12 +422,6 @@ static int basis_project_impl(const bm_layer_t* L, const void* x, int x_dtype, i
   g.N = L->rank_in;
   g.K = L->hidden;
   return launch_gemm_nt(g, 2, static_cast<cudaStream_t>(stream));
-}
-
-extern "C" int bm_basis_project(const bm_layer_t* L, const void* x, int x_dtype, int32_t T, uint16_t* h_gate,
-                                uint16_t* h_up, void* stream) {
-  bm::NvtxRange nvtx_range("bm_basis_project");
-  return basis_project_impl(L, x, x_dtype, T, h_gate, h_up, nullptr, 0, nullptr, stream);
 }
 
 // fixed-point accumulators -> fp32 rank_accum (deterministic mode)
@@ -531,6 +497,19 @@ extern "C" int bm_experts_forward(const bm_layer_t* L, const uint16_t* h_gate, c
                               false, workspace, workspace_bytes, stream);
 }
 
+// y = fp16(rank_accum) . U_down^T (+ (z * sigmoid(gate)) . W_down^T of a shared expert) (+ residual), one launch.
+static int combine_small(const bm_layer_t* L, const float* rank_accum, int T, const __half* w_down, int w_bf16, const float* z, const float* gate,
+                         int inter, const void* residual, void* y, int y_dtype, cudaStream_t st) {
+  SkinnyArgs a{};
+  a.seg[0] = SkSeg{L->u_down, nullptr, y, L->hidden, y_dtype, 0, 0};
+  a.n_seg = 1;
+  a.X = rank_accum; a.N = T; a.K = L->rank_out; a.x_dtype = BM_F32;
+  a.W2 = w_down; a.w2_bf16 = w_bf16; a.X2 = z; a.x2_gate = gate; a.K2 = inter;
+  a.residual = residual;
+  a.splits = 1;
+  return launch_skinny_nt(a, st);
+}
+
 extern "C" int bm_combine_down_basis(const bm_layer_t* L, const float* rank_accum, int32_t T, const void* residual,
                                      void* y, int y_dtype, void* stream) {
   bm::NvtxRange nvtx_range("bm_combine_down_basis");
@@ -539,16 +518,8 @@ extern "C" int bm_combine_down_basis(const bm_layer_t* L, const float* rank_accu
   BM_REQUIRE(T >= 0 && y_dtype >= BM_F16 && y_dtype <= BM_F32, BM_ERR_INVALID_ARG, "combine: bad arguments");
   if (T == 0) return BM_OK;
   BM_REQUIRE(rank_accum && y, BM_ERR_INVALID_ARG, "combine: null pointer");
-  if (T <= SKINNY_MAX_TOKENS && L->rank_out % 16 == 0 && L->hidden % 16 == 0 && L->rank_out <= 1024) {
-    SkinnyArgs a{};
-    a.W[0] = L->u_down; a.W[1] = L->u_down;
-    a.C[0] = y; a.C[1] = y;
-    a.X = rank_accum; a.residual = residual;
-    a.rows_per_w = L->hidden; a.n_w = 1;
-    a.N = T; a.K = L->rank_out;
-    a.x_dtype = BM_F32; a.c_dtype = y_dtype; a.round_x_f16 = 1;
-    a.splits = 1; a.mrows = 16;
-    const int rc = launch_skinny_nt(a, static_cast<cudaStream_t>(stream));
+  if (T <= SKINNY_MAX_TOKENS && skinny_fits(L->rank_out, 0, 1)) {
+    const int rc = combine_small(L, rank_accum, T, nullptr, 0, nullptr, nullptr, 0, residual, y, y_dtype, static_cast<cudaStream_t>(stream));
     if (rc != BM_ERR_UNSUPPORTED) return rc;
   }
   if (L->rank_out % 64 == 0) {
@@ -576,6 +547,56 @@ extern "C" size_t bm_layer_workspace_bytes(const bm_layer_t* L, int32_t T, int32
   return carve_layer_ws(L, nullptr, T, k).total;
 }
 
+// A decode batch (up to 256 tokens) in three or four launches, each starting while the one before drains:
+//   1. everything that multiplies x -- the basis projection and, for a whole block, router logits, the shared expert's
+//      gated pair and its token gate -- with the expert stage's accumulator cleared on the way; given logits are routed
+//      by one more cluster of the same grid
+//   2. routing of computed logits (whole block only)
+//   3. packed experts
+//   4. down basis, shared expert's down product and residual
+// BM_ERR_UNSUPPORTED, with nothing launched, when a shape does not tile; the general path takes it.
+static int forward_small(const bm_layer_t* L, const bm_block_dense_t* d, const void* x, int x_dtype, void* logits, int logits_dtype, int T,
+                         int k, int renorm, int weight_round, const void* residual, void* y, int path, const LayerWs& w, float* z, float* gate,
+                         cudaStream_t st) {
+  const bool shared = d && d->sh_intermediate > 0;
+  if (!x || !y || !logits || x_dtype < BM_F16 || x_dtype > BM_F32 || logits_dtype < BM_F16 || logits_dtype > BM_F32) return BM_ERR_UNSUPPORTED;
+  if (T > SKINNY_MAX_TOKENS || L->hidden % 128 != 0 || (reinterpret_cast<uintptr_t>(x) & 15u) || !L->vh_gate || !L->vh_up || !L->u_down ||
+      !skinny_fits(L->hidden, 0, 8) || !skinny_fits(L->rank_out, shared ? d->sh_intermediate : 0, 1) || !route_small_fits(T, L->num_experts, k))
+    return BM_ERR_UNSUPPORTED;
+  auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
+  if (!aligned(L->vh_gate) || !aligned(L->vh_up) || !aligned(L->u_down)) return BM_ERR_UNSUPPORTED;
+  if (d && !(aligned(d->gate_w) && aligned(d->sh_gate) && aligned(d->sh_up) && aligned(d->sh_down) && aligned(d->sh_token_gate)))
+    return BM_ERR_UNSUPPORTED;
+  const size_t acc_bytes = sizeof(float) * static_cast<size_t>(T) * L->rank_out;     // rank_out is a multiple of 16 here
+  auto h = [](const uint16_t* p) { return reinterpret_cast<const __half*>(p); };
+  RouteSmallArgs r{};
+  r.logits = logits; r.logits_dtype = logits_dtype;
+  r.T = T; r.E = L->num_experts; r.k = k; r.renorm = renorm; r.weight_round = weight_round;
+  r.token_indices = w.token_indices; r.expert_offsets = w.expert_offsets; r.route_flat = w.route_flat;
+  SkinnyArgs a{};
+  const int bf16 = d && d->w_dtype == BM_BF16;
+  int n = 0;
+  if (d) a.seg[n++] = SkSeg{h(d->gate_w), nullptr, logits, L->num_experts, logits_dtype, bf16, 0};
+  a.seg[n++] = SkSeg{L->vh_gate, nullptr, w.h_gate, L->rank_in, BM_F16, 0, 0};
+  a.seg[n++] = SkSeg{L->vh_up, nullptr, w.h_up, L->rank_in, BM_F16, 0, 0};
+  if (shared) {
+    a.seg[n++] = SkSeg{h(d->sh_gate), h(d->sh_up), z, d->sh_intermediate, BM_F32, bf16, 0};
+    if (d->sh_token_gate) a.seg[n++] = SkSeg{h(d->sh_token_gate), nullptr, gate, 1, BM_F32, bf16, 0};
+  }
+  a.n_seg = n;
+  a.X = x; a.N = T; a.K = L->hidden; a.x_dtype = x_dtype; a.splits = 8;
+  a.zero = reinterpret_cast<float4*>(w.rank_accum); a.zero_n = static_cast<int>(acc_bytes / 16);
+  if (!d) a.route = r;
+  int rc = launch_skinny_nt(a, st);
+  if (rc) return rc;
+  if (d && (rc = launch_route_small(r, st))) return rc;
+  rc = experts_forward_impl(L, reinterpret_cast<const uint16_t*>(w.h_gate), reinterpret_cast<const uint16_t*>(w.h_up), w.token_indices,
+                            w.expert_offsets, w.route_flat, T, T * k, w.rank_accum, path, true, w.experts_ws, w.experts_ws_bytes, st);
+  if (rc) return rc;
+  return combine_small(L, w.rank_accum, T, shared ? h(d->sh_down) : nullptr, bf16, z, shared && d->sh_token_gate ? gate : nullptr,
+                       shared ? d->sh_intermediate : 0, residual, y, x_dtype, st);
+}
+
 extern "C" int bm_layer_forward(const bm_layer_t* L, const void* x, int x_dtype, const void* logits, int logits_dtype,
                                 int32_t T, int32_t num_routed, int32_t k, int32_t renorm, int32_t weight_round,
                                 const int32_t* global_to_local, const void* residual, void* y, int32_t path,
@@ -590,6 +611,11 @@ extern "C" int bm_layer_forward(const bm_layer_t* L, const void* x, int x_dtype,
   BM_REQUIRE(workspace && workspace_bytes >= w.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0,
              BM_ERR_WORKSPACE, "layer_forward: workspace must be 256-byte aligned and hold %zu bytes (%zu given)", w.total,
              workspace_bytes);
+  if (global_to_local == nullptr) {
+    const int rc = forward_small(L, nullptr, x, x_dtype, const_cast<void*>(logits), logits_dtype, T, k, renorm, weight_round, residual, y, path,
+                                 w, nullptr, nullptr, static_cast<cudaStream_t>(stream));
+    if (rc != BM_ERR_UNSUPPORTED) return rc;
+  }
   // routing depends only on the logits and the basis projection only on x: run them side by side
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const bool fork = L->side_stream != nullptr && L->ev_fork != nullptr && L->ev_join != nullptr;
@@ -602,13 +628,10 @@ extern "C" int bm_layer_forward(const bm_layer_t* L, const void* x, int x_dtype,
   int rc = bm_route(logits, logits_dtype, T, num_routed, k, renorm, weight_round, global_to_local, L->num_experts, TILE_ROWS,
                     w.topk_idx, w.topk_w, w.token_indices, w.expert_offsets, w.route_flat, /*tile_table=*/nullptr, /*counts=*/nullptr,
                     w.route_ws, w.route_ws_bytes, route_stream);
-  // the accumulator of the expert stage is cleared off the critical path: by the projection kernel when the
-  // skinny one runs, else by a memset beside the routing
-  bool zeroed = false;
+  // the accumulator of the expert stage is cleared off the critical path, beside the routing
   const size_t acc_bytes = sizeof(float) * static_cast<size_t>(T) * L->rank_out;
-  const int rc_basis = basis_project_impl(L, x, x_dtype, T, reinterpret_cast<uint16_t*>(w.h_gate),
-                                          reinterpret_cast<uint16_t*>(w.h_up), w.rank_accum, acc_bytes, &zeroed, stream);
-  if (!zeroed && cudaMemsetAsync(w.rank_accum, 0, acc_bytes, static_cast<cudaStream_t>(route_stream)) == cudaSuccess) zeroed = true;
+  const int rc_basis = bm_basis_project(L, x, x_dtype, T, reinterpret_cast<uint16_t*>(w.h_gate), reinterpret_cast<uint16_t*>(w.h_up), stream);
+  const bool zeroed = cudaMemsetAsync(w.rank_accum, 0, acc_bytes, static_cast<cudaStream_t>(route_stream)) == cudaSuccess;
   if (fork) {
     // always join, also on error, so that the side stream never stays attached to a capture
     cudaEventRecord(L->ev_join, L->side_stream);
@@ -623,4 +646,101 @@ extern "C" int bm_layer_forward(const bm_layer_t* L, const void* x, int x_dtype,
                             w.experts_ws_bytes, stream);
   if (rc) return rc;
   return bm_combine_down_basis(L, w.rank_accum, T, residual, y, x_dtype == BM_F32 ? BM_F32 : x_dtype, stream);
+}
+
+// bf16 weights -> fp16, several matrices per launch (piece i: n[i] groups of eight values)
+struct CastArgs { const uint4* src[5]; uint4* dst[5]; int n[5]; };
+__global__ void __launch_bounds__(256) cast_weights_kernel(const __grid_constant__ CastArgs a) {
+  const int p = blockIdx.y;
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < a.n[p]; i += gridDim.x * 256) {
+    uint4 v = __ldg(a.src[p] + i);
+    uint32_t* o = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const __half2 h = __floats2half2_rn(__uint_as_float(o[j] << 16), __uint_as_float(o[j] & 0xffff0000u));
+      o[j] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    a.dst[p][i] = v;
+  }
+}
+
+// Extra workspace of a block on the general path: the shared expert's contribution (y is written by the last launch
+// only), its intermediates, and fp16 copies of bf16 weights.
+struct BlockWs { void* res; void* dense_ws; size_t dense_ws_bytes; uint16_t* w[5]; size_t total; };
+static BlockWs carve_block_ws(const bm_layer_t* L, const bm_block_dense_t* d, int num_routed, void* base, int T) {
+  Carver c(base, 0);
+  BlockWs w{};
+  const size_t H = static_cast<size_t>(L->hidden), I = d->sh_intermediate > 0 ? d->sh_intermediate : 0;
+  if (I) {
+    w.res = c.take<uint16_t>(static_cast<size_t>(T) * H);
+    w.dense_ws_bytes = bm_dense_mlp_workspace_bytes(T, static_cast<int32_t>(I));
+    w.dense_ws = c.take<unsigned char>(w.dense_ws_bytes);
+  }
+  if (d->w_dtype == BM_BF16) {
+    const size_t n[5] = {static_cast<size_t>(num_routed) * H, I * H, I * H, I * H, H};
+    for (int i = 0; i < 5; ++i) w.w[i] = c.take<uint16_t>(n[i]);
+  }
+  w.total = c.off;
+  return w;
+}
+
+extern "C" size_t bm_block_workspace_bytes(const bm_layer_t* L, const bm_block_dense_t* d, int32_t num_routed, int32_t T, int32_t k) {
+  if (!L || !d || T < 0 || k <= 0) return 0;
+  return carve_layer_ws(L, nullptr, T, k).total + carve_block_ws(L, d, num_routed, nullptr, T).total;
+}
+
+extern "C" int bm_block_forward(const bm_layer_t* L, const bm_block_dense_t* dense, const void* x, int x_dtype, int32_t T, int32_t num_routed,
+                                int32_t k, int32_t renorm, int32_t weight_round, const int32_t* global_to_local, void* logits, void* y,
+                                void* workspace, size_t workspace_bytes, void* stream) {
+  bm::NvtxRange nvtx_range("bm_block_forward");
+  BM_REQUIRE(L != nullptr && dense != nullptr && dense->gate_w != nullptr, BM_ERR_INVALID_ARG, "block_forward: null layer or router");
+  BM_REQUIRE(T >= 0 && k > 0 && num_routed > 0 && (x_dtype == BM_F16 || x_dtype == BM_BF16) &&
+                 (dense->w_dtype == BM_F16 || dense->w_dtype == BM_BF16),
+             BM_ERR_INVALID_ARG, "block_forward: bad arguments");
+  bm_block_dense_t d = *dense;
+  const bool shared = d.sh_intermediate > 0;
+  BM_REQUIRE(!shared || (d.sh_gate && d.sh_up && d.sh_down && d.sh_intermediate % 2 == 0), BM_ERR_INVALID_ARG,
+             "block_forward: incomplete shared expert");
+  BM_REQUIRE(global_to_local != nullptr || num_routed == L->num_experts, BM_ERR_INVALID_ARG,
+             "block_forward: %d routed experts but %d packed and no id map", num_routed, L->num_experts);
+  if (T == 0) return BM_OK;
+  BM_REQUIRE(x && logits && y, BM_ERR_INVALID_ARG, "block_forward: null pointer");
+  const LayerWs w = carve_layer_ws(L, workspace, T, k);
+  const BlockWs b = carve_block_ws(L, &d, num_routed, static_cast<unsigned char*>(workspace) + w.total, T);
+  BM_REQUIRE(workspace && workspace_bytes >= w.total + b.total && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0, BM_ERR_WORKSPACE,
+             "block_forward: workspace must be 256-byte aligned and hold %zu bytes (%zu given)", w.total + b.total, workspace_bytes);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (global_to_local == nullptr) {
+    // z fp32 [T, intermediate] fits the g and u areas of the shared expert's workspace, the token gate behind it in z's
+    float* z = static_cast<float*>(b.dense_ws);
+    float* gate = shared ? z + align_up(static_cast<size_t>(T) * d.sh_intermediate, 64) : nullptr;
+    const int rc = forward_small(L, &d, x, x_dtype, logits, x_dtype, T, k, renorm, weight_round, nullptr, y, BM_PATH_AUTO, w, z, gate, st);
+    if (rc != BM_ERR_UNSUPPORTED) return rc;
+  }
+  if (d.w_dtype == BM_BF16) {
+    const size_t H = static_cast<size_t>(L->hidden), I = shared ? d.sh_intermediate : 0;
+    BM_REQUIRE(H % 8 == 0, BM_ERR_UNSUPPORTED, "block_forward: hidden=%d must be a multiple of 8 with bf16 weights", L->hidden);
+    const uint16_t** src[5] = {&d.gate_w, &d.sh_gate, &d.sh_up, &d.sh_down, &d.sh_token_gate};
+    const size_t n[5] = {static_cast<size_t>(num_routed) * H, I * H, I * H, I * H, H};
+    CastArgs c{};
+    for (int i = 0; i < 5; ++i) {
+      if (!*src[i] || (i > 0 && !shared)) continue;
+      BM_REQUIRE((reinterpret_cast<uintptr_t>(*src[i]) & 15u) == 0, BM_ERR_UNSUPPORTED, "block_forward: bf16 weights must be 16-byte aligned");
+      c.src[i] = reinterpret_cast<const uint4*>(*src[i]);
+      c.dst[i] = reinterpret_cast<uint4*>(b.w[i]);
+      c.n[i] = static_cast<int>(n[i] / 8);
+      *src[i] = b.w[i];
+    }
+    cast_weights_kernel<<<dim3(148, 5), 256, 0, st>>>(c);
+    BM_LAUNCH_CHECK("cast_weights_kernel");
+  }
+  int rc = bm_gate_logits(x, x_dtype, d.gate_w, T, num_routed, L->hidden, logits, x_dtype, stream);
+  if (rc) return rc;
+  if (shared) {
+    rc = bm_dense_mlp_forward(x, x_dtype, d.sh_gate, d.sh_up, d.sh_down, d.sh_token_gate, T, L->hidden, d.sh_intermediate, nullptr, b.res,
+                              x_dtype, b.dense_ws, b.dense_ws_bytes, stream);
+    if (rc) return rc;
+  }
+  return bm_layer_forward(L, x, x_dtype, logits, x_dtype, T, num_routed, k, renorm, weight_round, global_to_local, b.res, y, BM_PATH_AUTO,
+                          workspace, w.total, stream);
 }

@@ -1,36 +1,28 @@
-// Shared-basis products for small token counts:  C[n][m] = sum_k W[m][k] * X[n][k]
-//   h_gate / h_up = x . Vh^T        (W = Vh_gate | Vh_up, K = hidden, split over a cluster)
-//   y = fp16(rank_accum) . U_down^T  (W = U_down, K = rank_out) (+ residual)
-// These are weight-streaming GEMVs: every CTA reads a [rows x k-slice] block of W exactly once,
-// keeps it in shared memory and multiplies it with the (few) token rows on the tensor cores
-// (mma.sync m16n8k16, W rows as the A operand, tokens as N).  When the contraction is long
-// (hidden = 2048) it is split over the CTAs of a thread-block cluster, whose partial sums are
-// reduced through distributed shared memory, so no atomics and no second pass are needed.
-#include <cooperative_groups.h>
-
-#include "common.cuh"
+// Products of a decode batch with streamed weights:  C[n][m] = sum_k W[m][k] * X[n][k], up to 256 tokens.
+//   logits / h_gate / h_up / shared-expert gate and up = x . W^T   (stacks of output rows sharing x, K = hidden)
+//   y = fp16(rank_accum) . U_down^T (+ shared down product) (+ residual)
+// These are weight-streaming GEMVs: a CTA reads a [rows x k-slice] block of W once, keeps it in shared memory and
+// multiplies it with 64 token rows on the tensor cores (mma.sync m16n8k16, W rows as the A operand, tokens as N).
+// A long contraction is split over the CTAs of a thread-block cluster whose partial sums meet through distributed shared
+// memory: no atomics, no second pass.  More tokens than 64 are more CTAs (grid y), not a loop: the weights come from L2
+// then, and the chunks run side by side.
+//
+// What bounds a launch is latency: weights -> shared memory -> MMA -> cluster exchange.  Three things shorten the chain:
+// everything that multiplies the same x is one launch (SkSeg stacks; the gated pair of a shared expert leaves as
+// silu(g) * u), the routing of given logits is one more cluster of the same grid, and the kernel is launched with
+// programmatic stream serialisation: its weights, which no kernel of this library writes, are on their way to shared
+// memory while the previous kernel still runs.
+#include "route_small.cuh"
 
 namespace cg = cooperative_groups;
 
 namespace bm {
 
 constexpr int SK_THREADS = 256;
-constexpr int SK_NTOK = 64;   // tokens per chunk
+constexpr int SK_NTOK = 64;          // tokens per CTA
+constexpr int SK_RECV = 72;          // floats per received row: four neighbouring rows start eight banks apart
 
-struct SkinnyArgs {
-  const __half* W[2];    // up to two weight matrices stacked along m (rows_per_w rows each)
-  void* C[2];            // C[i] is [N, rows_per_w]
-  const void* X;         // [N, K]
-  const void* residual;  // [N, rows_per_w] or null (W[0] only)
-  int rows_per_w, n_w;   // total m = rows_per_w * n_w
-  int N, K;
-  int x_dtype, c_dtype;
-  int round_x_f16;       // X is fp32 and is rounded through fp16 (always true for fp32 here)
-  int splits;            // cluster size along k
-  int mrows;             // W rows per CTA: 16 or 32
-  float4* zero;          // optional buffer the grid clears on its way (the next kernel's accumulator), 16-byte units
-  int zero_n;
-};
+__host__ __device__ constexpr int sk_mrows(int splits) { return splits == 1 ? 16 : 32; }
 
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -44,218 +36,320 @@ __device__ __forceinline__ void ldsm_x4(const __half* p, uint32_t& r0, uint32_t&
                : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))));
 }
 
-// smem: Ws [mrows][ks + 8] half | Xs [64][ks + 8] half | recv [splits][mrows / splits][64] float (only when splits > 1)
-__global__ void __launch_bounds__(SK_THREADS) skinny_nt_kernel(SkinnyArgs a) {
-  extern __shared__ __align__(16) unsigned char sk_smem[];
-  const int ks = a.K / a.splits;
-  const int stride = ks + 8;
-  __half* Ws = reinterpret_cast<__half*>(sk_smem);
-  __half* Xs = Ws + static_cast<size_t>(a.mrows) * stride;
-  float* recv = reinterpret_cast<float*>(Xs + static_cast<size_t>(SK_NTOK) * stride);
-  const int split = blockIdx.x % a.splits;
-  const int m0 = (blockIdx.x / a.splits) * a.mrows;     // first global output row of this CTA
-  const int wsel = m0 / a.rows_per_w;                    // which stacked matrix
-  const int mloc0 = m0 - wsel * a.rows_per_w;
-  const __half* W = a.W[wsel] + static_cast<size_t>(mloc0) * a.K + static_cast<size_t>(split) * ks;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
 
-  // peers' shared memory may be written only once every CTA of the cluster runs: arrive now, wait before the first push
-  bool peers_up = a.splits == 1;
-  cg::cluster_group::arrival_token started;
-  if (a.splits > 1) started = cg::this_cluster().barrier_arrive();
-  // W slice -> smem with cp.async (16-byte vectors), so it streams in while the token rows are converted
-  const int vec_per_row = ks / 8;
-  for (int v = threadIdx.x; v < a.mrows * vec_per_row; v += SK_THREADS) {
-    const int r = v / vec_per_row, c = (v - r * vec_per_row) * 8;
-    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(Ws + static_cast<size_t>(r) * stride + c));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(W + static_cast<size_t>(r) * a.K + c) : "memory");
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  if (a.zero != nullptr) {
-    for (int i = blockIdx.x * SK_THREADS + threadIdx.x; i < a.zero_n; i += gridDim.x * SK_THREADS) a.zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  const int mblocks = a.mrows / 16;
-  for (int n0 = 0; n0 < a.N; n0 += SK_NTOK) {
-    const int nn = min(SK_NTOK, a.N - n0);
-    const int nblocks = (nn + 7) / 8;
-    __syncthreads();   // previous chunk's readers of Xs / part are done
-    // X slice -> fp16 smem; the loads of eight vectors are issued before the first conversion
-    const int nvec = nblocks * 8 * vec_per_row;
-    for (int v0 = threadIdx.x; v0 < nvec; v0 += 8 * SK_THREADS) {
-      uint4 raw[8][2];
+// Columns [k0, k0 + width) of the rows n0 .. n0 + nn of a row-major [*, ld] matrix -> fp16 at dst (row stride `stride`),
+// rows up to `rows` zero; the loads of eight 8-element vectors are issued before the first conversion.
+template <int XD>
+__device__ __forceinline__ void stage_rows(const void* X, int64_t ld, int k0, int width, int n0, int nn, int rows, const float* gate,
+                                           __half* dst, int stride) {
+  const int vpr = width >> 3, nvec = rows * vpr;
+  constexpr int U = XD == BM_F32 ? 4 : 8;
+  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * SK_THREADS) {
+    uint4 raw[U][XD == BM_F32 ? 2 : 1];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int v = v0 + u * SK_THREADS;
-        const int r = v / vec_per_row, c = (v - r * vec_per_row) * 8;
-        raw[u][0] = raw[u][1] = make_uint4(0u, 0u, 0u, 0u);
-        if (v < nvec && r < nn) {
-          const size_t idx = static_cast<size_t>(n0 + r) * a.K + static_cast<size_t>(split) * ks + c;
-          if (a.x_dtype == BM_F32) {
-            raw[u][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(a.X) + idx);
-            raw[u][1] = *reinterpret_cast<const uint4*>(reinterpret_cast<const float*>(a.X) + idx + 4);
-          } else {
-            raw[u][0] = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.X) + idx);
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int v = v0 + u * SK_THREADS;
-        if (v >= nvec) break;
-        const int r = v / vec_per_row, c = (v - r * vec_per_row) * 8;
-        uint4 out = raw[u][0];
-        if (a.x_dtype == BM_BF16) {
-          const uint32_t w[4] = {raw[u][0].x, raw[u][0].y, raw[u][0].z, raw[u][0].w};
-          uint32_t o[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const __half2 h2 = __floats2half2_rn(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
-            o[i] = *reinterpret_cast<const uint32_t*>(&h2);
-          }
-          out = make_uint4(o[0], o[1], o[2], o[3]);
-        } else if (a.x_dtype == BM_F32) {
-          const uint32_t w[8] = {raw[u][0].x, raw[u][0].y, raw[u][0].z, raw[u][0].w, raw[u][1].x, raw[u][1].y, raw[u][1].z, raw[u][1].w};
-          uint32_t o[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const __half2 h2 = __floats2half2_rn(__uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
-            o[i] = *reinterpret_cast<const uint32_t*>(&h2);
-          }
-          out = make_uint4(o[0], o[1], o[2], o[3]);
-        }
-        *reinterpret_cast<uint4*>(Xs + static_cast<size_t>(r) * stride + c) = out;
-      }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
-    // (mblock, nblock) items round-robin over the warps, two at a time: items `it` and `it + 8` share the W rows when
-    // mblocks divides the warp count, so one A fragment feeds two MMAs; a lone item splits its contraction over two
-    // accumulators instead.  Fragments come from ldmatrix (rows are 16-byte aligned and 16 bytes apart modulo 128).
-    const int n_items = mblocks * nblocks;
-    const int a_row = (lane & 7) + 8 * ((lane >> 3) & 1), a_kofs = 8 * (lane >> 4);   // ldmatrix.x4 address roles, A operand
-    const int b_row = lane & 7, b_sel = lane >> 3;                                     // B operand: matrix b_sel of four
-    for (int it = warp; it < n_items; it += 2 * (SK_THREADS / 32)) {
-      const int it2 = it + SK_THREADS / 32;
-      const int mb = it % mblocks, nb = it / mblocks;
-      const bool pair = it2 < n_items && (it2 % mblocks) == mb;
-      const int nb2 = pair ? it2 / mblocks : nb;
-      float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      const __half* wa = Ws + static_cast<size_t>(mb * 16 + a_row) * stride + a_kofs;
-      if (pair) {
-        // B matrices: (nb, k 0-7) (nb, k 8-15) (nb2, k 0-7) (nb2, k 8-15)
-        const __half* xb = Xs + static_cast<size_t>((b_sel < 2 ? nb : nb2) * 8 + b_row) * stride + 8 * (b_sel & 1);
-#pragma unroll 4
-        for (int k = 0; k < ks; k += 16) {
-          uint32_t a0, a1, a2, a3, b0, b1, c0, c1;
-          ldsm_x4(wa + k, a0, a1, a2, a3);
-          ldsm_x4(xb + k, b0, b1, c0, c1);
-          mma16816(acc[0], a0, a1, a2, a3, b0, b1);
-          mma16816(acc[1], a0, a1, a2, a3, c0, c1);
-        }
-      } else {
-        // B matrices: (nb, k 0-7) (nb, k 8-15) (nb, k 16-23) (nb, k 24-31); even / odd 16-steps in separate accumulators
-        const __half* xb = Xs + static_cast<size_t>(nb * 8 + b_row) * stride + 8 * b_sel;
-        int k = 0;
-#pragma unroll 2
-        for (; k + 32 <= ks; k += 32) {
-          uint32_t a0, a1, a2, a3, e0, e1, e2, e3, b0, b1, c0, c1;
-          ldsm_x4(wa + k, a0, a1, a2, a3);
-          ldsm_x4(wa + k + 16, e0, e1, e2, e3);
-          ldsm_x4(xb + k, b0, b1, c0, c1);
-          mma16816(acc[0], a0, a1, a2, a3, b0, b1);
-          mma16816(acc[1], e0, e1, e2, e3, c0, c1);
-        }
-        if (k < ks) {   // one 16-step left: the upper two B matrices repeat the lower ones instead of reading past the row
-          uint32_t a0, a1, a2, a3, b0, b1, c0, c1;
-          ldsm_x4(wa + k, a0, a1, a2, a3);
-          ldsm_x4(Xs + static_cast<size_t>(nb * 8 + b_row) * stride + 8 * (b_sel & 1) + k, b0, b1, c0, c1);
-          mma16816(acc[0], a0, a1, a2, a3, b0, b1);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { acc[0][j] += acc[1][j]; acc[1][j] = 0.f; }
-      }
-      // D: rows m = mb*16 + g (+8), cols n = nb*8 + 2t (+1)
-#pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        if (q == 1 && !pair) break;
-        const int nbq = q ? nb2 : nb;
-        if (a.splits == 1) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int m = mloc0 + mb * 16 + g + (j >= 2 ? 8 : 0), n = nbq * 8 + 2 * t + (j & 1);
-            if (n < nn) {
-              const size_t idx = static_cast<size_t>(n0 + n) * a.rows_per_w + m;
-              float v = acc[q][j];
-              if (a.residual && wsel == 0) v += load_act(a.residual, a.c_dtype, idx);
-              store_act(a.C[wsel], a.c_dtype, idx, v);
-            }
-          }
+    for (int u = 0; u < U; ++u) {
+      const int v = v0 + u * SK_THREADS;
+      const int r = v / vpr, c = (v - r * vpr) * 8;
+      raw[u][0] = make_uint4(0u, 0u, 0u, 0u);
+      if (XD == BM_F32) raw[u][XD == BM_F32 ? 1 : 0] = make_uint4(0u, 0u, 0u, 0u);
+      if (v < nvec && r < nn) {
+        const int64_t idx = static_cast<int64_t>(n0 + r) * ld + k0 + c;
+        if (XD == BM_F32) {
+          const uint4* src = reinterpret_cast<const uint4*>(static_cast<const float*>(X) + idx);
+          raw[u][0] = src[0];
+          raw[u][XD == BM_F32 ? 1 : 0] = src[1];
         } else {
-          // push the partial sums into the shared memory of the CTA that owns these output rows
-          if (!peers_up) { cg::this_cluster().barrier_wait(std::move(started)); peers_up = true; }
-          const int rows_per_owner = a.mrows / a.splits;
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int m = mb * 16 + g + 8 * h;
-            float* dst = cg::this_cluster().map_shared_rank(recv, m / rows_per_owner) +
-                         (static_cast<size_t>(split) * rows_per_owner + m % rows_per_owner) * SK_NTOK + nbq * 8 + 2 * t;
-            *reinterpret_cast<float2*>(dst) = make_float2(acc[q][2 * h], acc[q][2 * h + 1]);
-          }
+          raw[u][0] = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(X) + idx);
         }
       }
     }
-    if (a.splits > 1) {
-      cg::cluster_group cluster = cg::this_cluster();
-      if (!peers_up) { cluster.barrier_wait(std::move(started)); peers_up = true; }
-      cluster.sync();   // every CTA's partial sums have landed in their owners
-      // this CTA owns rows [split * rows_per_owner, +rows_per_owner) of the mrows x nn tile: sum the `splits` copies
-      const int rows_per_owner = a.mrows / a.splits;
-      const int total = rows_per_owner * nblocks * 8;
-      for (int o = threadIdx.x; o < total; o += SK_THREADS) {
-        const int r = o / (nblocks * 8), n = o - r * (nblocks * 8);
-        float pv[8];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) pv[c] = c < a.splits ? recv[(static_cast<size_t>(c) * rows_per_owner + r) * SK_NTOK + n] : 0.f;
-        float v = ((pv[0] + pv[1]) + (pv[2] + pv[3])) + ((pv[4] + pv[5]) + (pv[6] + pv[7]));
-        if (n < nn) {
-          const size_t idx = static_cast<size_t>(n0 + n) * a.rows_per_w + mloc0 + split * rows_per_owner + r;
-          if (a.residual && wsel == 0) v += load_act(a.residual, a.c_dtype, idx);
-          store_act(a.C[wsel], a.c_dtype, idx, v);
-        }
+    for (int u = 0; u < U; ++u) {
+      const int v = v0 + u * SK_THREADS;
+      if (v >= nvec) break;
+      const int r = v / vpr, c = (v - r * vpr) * 8;
+      uint4 out = raw[u][0];
+      if (XD == BM_BF16) {
+        uint32_t* o = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = pack_half2(__uint_as_float(o[i] << 16), __uint_as_float(o[i] & 0xffff0000u));
+      } else if (XD == BM_F32) {
+        const float* f0 = reinterpret_cast<const float*>(&raw[u][0]);
+        const float* f1 = reinterpret_cast<const float*>(&raw[u][XD == BM_F32 ? 1 : 0]);
+        const float s = gate && r < nn ? 1.f / (1.f + __expf(-gate[n0 + r])) : 1.f;
+        out = make_uint4(pack_half2(f0[0] * s, f0[1] * s), pack_half2(f0[2] * s, f0[3] * s), pack_half2(f1[0] * s, f1[1] * s),
+                         pack_half2(f1[2] * s, f1[3] * s));
       }
-      if (n0 + SK_NTOK < a.N) cluster.sync();   // the next chunk overwrites the receive buffers
+      *reinterpret_cast<uint4*>(dst + static_cast<size_t>(r) * stride + c) = out;
     }
   }
 }
 
-// Returns BM_ERR_UNSUPPORTED when the shape does not fit; the caller then uses the general GEMM.
+// smem: Ws [mrows][kw + 8] half | Xs [64][kw + 8] half | recv [splits][mrows / splits][72] float (only when splits > 1),
+// kw = K / splits + K2
+__host__ __device__ inline size_t sk_smem_bytes(int K, int K2, int splits) {
+  const int mrows = sk_mrows(splits);
+  size_t s = static_cast<size_t>(mrows + SK_NTOK) * (K / splits + K2 + 8) * 2;
+  if (splits > 1) s += static_cast<size_t>(mrows) * SK_RECV * 4;
+  return s;
+}
+constexpr size_t SK_SMEM_LIMIT = 160 * 1024;
+
+__global__ void __launch_bounds__(SK_THREADS) skinny_nt_kernel(const __grid_constant__ SkinnyArgs a) {
+  extern __shared__ __align__(16) unsigned char sk_smem[];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int split = blockIdx.x % a.splits, row_tile = blockIdx.x / a.splits;
+  if (row_tile >= a.row_tiles) {      // the routing cluster
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (blockIdx.y == 0) route_small(a.route, reinterpret_cast<RouteSmallSmem*>(sk_smem));
+    return;
+  }
+  const int ks = a.K / a.splits, kw = ks + a.K2;
+  const int stride = kw + 8;
+  const int mrows = sk_mrows(a.splits);
+  __half* Ws = reinterpret_cast<__half*>(sk_smem);
+  __half* Xs = Ws + static_cast<size_t>(mrows) * stride;
+  float* recv = reinterpret_cast<float*>(Xs + static_cast<size_t>(SK_NTOK) * stride);
+  int si = 0;
+  while (si + 1 < a.n_seg && row_tile >= a.seg[si + 1].tile0) ++si;
+  const SkSeg& sg = a.seg[si];
+  const bool glu = sg.W_up != nullptr;
+  const int m0 = (row_tile - sg.tile0) * (glu ? mrows / 2 : mrows);      // first output row of the stack in this CTA
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+
+  // peers' shared memory may be written only once every CTA of the cluster runs: arrive now, wait before the first push
+  cg::cluster_group::arrival_token started;
+  if (a.splits > 1) started = cg::this_cluster().barrier_arrive();
+  // W block -> smem.  A gated pair alternates gate and up rows, so that one CTA of the cluster owns both sums of an output.
+  {
+    const int vpr = kw >> 3;
+    for (int v = threadIdx.x; v < mrows * vpr; v += SK_THREADS) {
+      const int r = v / vpr, c = (v - r * vpr) * 8;
+      const int m = m0 + (glu ? r >> 1 : r);
+      __half* dst = Ws + static_cast<size_t>(r) * stride + c;
+      const bool live = m < sg.rows;
+      const __half* src = c < ks ? (glu && (r & 1) ? sg.W_up : sg.W) + static_cast<size_t>(live ? m : 0) * a.K + split * ks + c
+                                 : a.W2 + static_cast<size_t>(live ? m : 0) * a.K2 + (c - ks);
+      if (c < ks ? sg.w_bf16 : a.w2_bf16) {
+        uint4 raw = live ? __ldg(reinterpret_cast<const uint4*>(src)) : make_uint4(0u, 0u, 0u, 0u);
+        uint32_t* o = reinterpret_cast<uint32_t*>(&raw);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o[i] = pack_half2(__uint_as_float(o[i] << 16), __uint_as_float(o[i] & 0xffff0000u));
+        *reinterpret_cast<uint4*>(dst) = raw;
+      } else {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src),
+                     "r"(live ? 16 : 0)
+                     : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (a.zero != nullptr) {
+    const int nthr = gridDim.x * gridDim.y * SK_THREADS;
+    for (int i = (blockIdx.y * gridDim.x + blockIdx.x) * SK_THREADS + threadIdx.x; i < a.zero_n; i += nthr) a.zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  const int n0 = blockIdx.y * SK_NTOK;
+  const int nn = min(SK_NTOK, a.N - n0);
+  const int nblocks = (nn + 7) >> 3;
+  if (a.x_dtype == BM_F32) stage_rows<BM_F32>(a.X, a.K, split * ks, ks, n0, nn, nblocks * 8, a.x_gate, Xs, stride);
+  else if (a.x_dtype == BM_BF16) stage_rows<BM_BF16>(a.X, a.K, split * ks, ks, n0, nn, nblocks * 8, nullptr, Xs, stride);
+  else stage_rows<BM_F16>(a.X, a.K, split * ks, ks, n0, nn, nblocks * 8, nullptr, Xs, stride);
+  if (a.K2) stage_rows<BM_F32>(a.X2, a.K2, 0, a.K2, n0, nn, nblocks * 8, a.x2_gate, Xs + ks, stride);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  if (a.splits > 1) cg::this_cluster().barrier_wait(std::move(started));
+  // (mblock, nblock) items round-robin over the warps, two at a time: items `it` and `it + 8` share the W rows when
+  // mblocks divides the warp count, so one A fragment feeds two MMAs; a lone item splits its contraction over two
+  // accumulators instead.  Fragments come from ldmatrix (rows are 16-byte aligned and 16 bytes apart modulo 128).
+  const int mblocks = mrows / 16;
+  const int n_items = mblocks * nblocks;
+  const int a_row = (lane & 7) + 8 * ((lane >> 3) & 1), a_kofs = 8 * (lane >> 4);   // ldmatrix.x4 address roles, A operand
+  const int b_row = lane & 7, b_sel = lane >> 3;                                     // B operand: matrix b_sel of four
+  for (int it = warp; it < n_items; it += 2 * (SK_THREADS / 32)) {
+    const int it2 = it + SK_THREADS / 32;
+    const int mb = it % mblocks, nb = it / mblocks;
+    const bool pair = it2 < n_items && (it2 % mblocks) == mb;
+    const int nb2 = pair ? it2 / mblocks : nb;
+    float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+    const __half* wa = Ws + static_cast<size_t>(mb * 16 + a_row) * stride + a_kofs;
+    if (pair) {
+      // B matrices: (nb, k 0-7) (nb, k 8-15) (nb2, k 0-7) (nb2, k 8-15)
+      const __half* xb = Xs + static_cast<size_t>((b_sel < 2 ? nb : nb2) * 8 + b_row) * stride + 8 * (b_sel & 1);
+#pragma unroll 4
+      for (int k = 0; k < kw; k += 16) {
+        uint32_t a0, a1, a2, a3, b0, b1, c0, c1;
+        ldsm_x4(wa + k, a0, a1, a2, a3);
+        ldsm_x4(xb + k, b0, b1, c0, c1);
+        mma16816(acc[0], a0, a1, a2, a3, b0, b1);
+        mma16816(acc[1], a0, a1, a2, a3, c0, c1);
+      }
+    } else {
+      // B matrices: (nb, k 0-7) (nb, k 8-15) (nb, k 16-23) (nb, k 24-31); even / odd 16-steps in separate accumulators
+      const __half* xb = Xs + static_cast<size_t>(nb * 8 + b_row) * stride + 8 * b_sel;
+      int k = 0;
+#pragma unroll 4
+      for (; k + 32 <= kw; k += 32) {
+        uint32_t a0, a1, a2, a3, e0, e1, e2, e3, b0, b1, c0, c1;
+        ldsm_x4(wa + k, a0, a1, a2, a3);
+        ldsm_x4(wa + k + 16, e0, e1, e2, e3);
+        ldsm_x4(xb + k, b0, b1, c0, c1);
+        mma16816(acc[0], a0, a1, a2, a3, b0, b1);
+        mma16816(acc[1], e0, e1, e2, e3, c0, c1);
+      }
+      if (k < kw) {   // one 16-step left: the upper two B matrices repeat the lower ones instead of reading past the row
+        uint32_t a0, a1, a2, a3, b0, b1, c0, c1;
+        ldsm_x4(wa + k, a0, a1, a2, a3);
+        ldsm_x4(Xs + static_cast<size_t>(nb * 8 + b_row) * stride + 8 * (b_sel & 1) + k, b0, b1, c0, c1);
+        mma16816(acc[0], a0, a1, a2, a3, b0, b1);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) { acc[0][j] += acc[1][j]; acc[1][j] = 0.f; }
+    }
+    // D: rows m = mb*16 + g (+8), cols n = nb*8 + 2t (+1)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      if (q == 1 && !pair) break;
+      const int nbq = q ? nb2 : nb;
+      if (a.splits == 1) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int m = m0 + mb * 16 + g + (j >= 2 ? 8 : 0), n = nbq * 8 + 2 * t + (j & 1);
+          if (n < nn && m < sg.rows) {
+            const int64_t idx = static_cast<int64_t>(n0 + n) * sg.rows + m;
+            float v = acc[q][j];
+            if (a.residual && si == 0) v += load_act(a.residual, sg.c_dtype, idx);
+            store_act(sg.C, sg.c_dtype, idx, v);
+          }
+        }
+      } else {
+        // push the partial sums into the shared memory of the CTA that owns these output rows
+        const int rows_per_owner = mrows / a.splits;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m = mb * 16 + g + 8 * h;
+          float* dst = cg::this_cluster().map_shared_rank(recv, m / rows_per_owner) +
+                       (static_cast<size_t>(split) * rows_per_owner + m % rows_per_owner) * SK_RECV + nbq * 8 + 2 * t;
+          *reinterpret_cast<float2*>(dst) = make_float2(acc[q][2 * h], acc[q][2 * h + 1]);
+        }
+      }
+    }
+  }
+  if (a.splits > 1) {
+    cg::this_cluster().sync();   // every CTA's partial sums have landed in their owners
+    // this CTA owns rows [split * rows_per_owner, +rows_per_owner) of the mrows x nn tile: sum the `splits` copies
+    const int rows_per_owner = mrows / a.splits, outs = glu ? rows_per_owner / 2 : rows_per_owner;
+    auto total = [&](int r, int n) {
+      float pv[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) pv[c] = c < a.splits ? recv[(static_cast<size_t>(c) * rows_per_owner + r) * SK_RECV + n] : 0.f;
+      return ((pv[0] + pv[1]) + (pv[2] + pv[3])) + ((pv[4] + pv[5]) + (pv[6] + pv[7]));
+    };
+    // consecutive threads take consecutive rows of a token: an owner's rows are one short piece of the output row
+    for (int o = threadIdx.x; o < outs * nn; o += SK_THREADS) {
+      const int n = o / outs, r = o - n * outs;
+      const int m = m0 + split * outs + r;
+      if (m >= sg.rows) continue;
+      float v;
+      if (glu) {
+        const float gv = total(2 * r, n), uv = total(2 * r + 1, n);
+        v = __fdividef(gv, 1.f + __expf(-gv)) * uv;
+      } else {
+        v = total(r, n);
+      }
+      const int64_t idx = static_cast<int64_t>(n0 + n) * sg.rows + m;
+      if (a.residual && si == 0) v += load_act(a.residual, sg.c_dtype, idx);
+      store_act(sg.C, sg.c_dtype, idx, v);
+    }
+  }
+}
+
+bool skinny_fits(int K, int K2, int splits) {
+  return K % (16 * splits) == 0 && K2 % 16 == 0 && (K2 == 0 || splits == 1) && sk_smem_bytes(K, K2, splits) <= SK_SMEM_LIMIT;
+}
+
+// The fewest splits whose k-slice fits shared memory and whose grid reaches most SMs.
+int skinny_splits(int rows, int K) {
+  for (int s = 1; s < 8; s *= 2)
+    if (skinny_fits(K, 0, s) && ((rows + sk_mrows(s) - 1) / sk_mrows(s) * s >= 96 || K / s <= 256)) return s;
+  return 8;
+}
+
 int launch_skinny_nt(SkinnyArgs a, cudaStream_t st) {
-  BM_REQUIRE(a.K % (16 * a.splits) == 0 && a.rows_per_w % a.mrows == 0 && a.splits <= 8 && a.mrows % a.splits == 0, BM_ERR_UNSUPPORTED, "skinny_nt: shape does not tile");
-  const int ks = a.K / a.splits;
-  size_t smem = static_cast<size_t>(a.mrows + SK_NTOK) * (ks + 8) * 2;
-  if (a.splits > 1) smem += static_cast<size_t>(a.mrows) * SK_NTOK * 4;
-  BM_REQUIRE(smem <= 160 * 1024, BM_ERR_UNSUPPORTED, "skinny_nt: k-slice of %d does not fit shared memory", ks);
+  BM_REQUIRE(a.N >= 1 && a.N <= SKINNY_MAX_TOKENS && a.n_seg >= 1 && a.n_seg <= SK_MAX_SEG && a.splits >= 1 && a.splits <= 8 &&
+                 (a.splits & (a.splits - 1)) == 0 && skinny_fits(a.K, a.K2, a.splits) && (reinterpret_cast<uintptr_t>(a.X) & 15u) == 0,
+             BM_ERR_UNSUPPORTED, "skinny_nt: shape does not tile");
+  const int mrows = sk_mrows(a.splits);
+  a.row_tiles = 0;
+  for (int i = 0; i < a.n_seg; ++i) {
+    const bool glu = a.seg[i].W_up != nullptr;
+    BM_REQUIRE(((reinterpret_cast<uintptr_t>(a.seg[i].W) | reinterpret_cast<uintptr_t>(a.seg[i].W_up)) & 15u) == 0 && (!glu || a.splits > 1) &&
+                   (!glu || mrows / a.splits % 2 == 0),
+               BM_ERR_UNSUPPORTED, "skinny_nt: weights are not aligned");
+    a.seg[i].tile0 = a.row_tiles;
+    const int per = glu ? mrows / 2 : mrows;
+    a.row_tiles += (a.seg[i].rows + per - 1) / per;
+  }
+  size_t smem = sk_smem_bytes(a.K, a.K2, a.splits);
+  const bool route = a.route.T > 0;
+  BM_REQUIRE(!route || a.splits == RS_CLUSTER, BM_ERR_UNSUPPORTED, "skinny_nt: routing needs clusters of %d", RS_CLUSTER);
+  if (route && smem < sizeof(RouteSmallSmem)) smem = sizeof(RouteSmallSmem);
   static PerDeviceOnce attr_once;
   int dev = -1;
   BM_CUDA(cudaGetDevice(&dev));
   if (!attr_once.is_done(dev)) {
-    BM_CUDA(cudaFuncSetAttribute(skinny_nt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+    BM_CUDA(cudaFuncSetAttribute(skinny_nt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SK_SMEM_LIMIT)));
     attr_once.mark(dev);
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((a.rows_per_w * a.n_w / a.mrows) * a.splits);
+  cfg.gridDim = dim3((a.row_tiles + (route ? 1 : 0)) * a.splits, (a.N + SK_NTOK - 1) / SK_NTOK);
   cfg.blockDim = dim3(SK_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = a.splits;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = a.splits;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = a.splits > 1 ? 2 : 1;
   count_launch();
   BM_CUDA(cudaLaunchKernelEx(&cfg, skinny_nt_kernel, a));
+  return BM_OK;
+}
+
+// ---- routing on its own, behind the launch that computes the logits
+__global__ void __launch_bounds__(RS_THREADS) route_small_kernel(const __grid_constant__ RouteSmallArgs a) {
+  __shared__ RouteSmallSmem sm;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  route_small(a, &sm);
+}
+
+bool route_small_fits(int T, int E, int k) { return T >= 1 && T <= RS_MAX_TOKENS && E >= 1 && E <= RS_MAX_E && k >= 1 && k <= 32 && k <= E; }
+
+int launch_route_small(const RouteSmallArgs& a, cudaStream_t st) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(RS_CLUSTER);
+  cfg.blockDim = dim3(RS_THREADS);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = RS_CLUSTER;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  count_launch();
+  BM_CUDA(cudaLaunchKernelEx(&cfg, route_small_kernel, a));
   return BM_OK;
 }
 

@@ -97,7 +97,8 @@ class PackedLayer:
             capi.check(lib.bm_layer_create(C.byref(d), self._arena.data_ptr(), self._arena.numel(),
                                            capi.stream_ptr(device), C.byref(h)))
         self._handle = h
-        self._ws: Dict[Tuple[int, int], torch.Tensor] = {}
+        self._host = capi.host()
+        self._native = self._host.layer_new(h.value, device.index)
 
     # -- construction helpers -------------------------------------------------------------------------
     @classmethod
@@ -111,6 +112,7 @@ class PackedLayer:
 
     def close(self) -> None:
         if getattr(self, "_handle", None) is not None:
+            self._host.layer_close(self._native)
             capi.lib().bm_layer_destroy(self._handle)
             self._handle = None
 
@@ -132,7 +134,7 @@ class PackedLayer:
         """Packed-expert kernels add into rank_accum through 64-bit fixed-point atomics: bit-identical results from run
         to run (the reference's fp32 atomics, bitsmoe/algorithms/cpp/mlp_forward.cu:2062, depend on arrival order)."""
         capi.check(capi.lib().bm_layer_set_option(self._handle, 1, int(bool(on))))
-        self._ws.clear()
+        self._host.layer_drop_workspaces(self._native)
 
     def set_decode_ctas_per_sm(self, n: int = 0) -> None:
         capi.check(capi.lib().bm_layer_set_option(self._handle, 0, int(n)))
@@ -168,17 +170,7 @@ class PackedLayer:
 
     def experts_forward(self, h_gate, h_up, token_indices, expert_offsets, route_weights,
                         path: int = capi.PATH_AUTO) -> torch.Tensor:
-        T = h_gate.shape[0]
-        A = token_indices.numel()
-        out = torch.empty((T, self.rank_out), dtype=torch.float32, device=self.device)
-        lib = capi.lib()
-        with torch.cuda.device(self.device):
-            need = int(lib.bm_experts_workspace_bytes(self._handle, T, A, path))
-            ws = torch.empty(max(need, 1), dtype=torch.uint8, device=self.device) if need else None
-            capi.check(lib.bm_experts_forward(self._handle, h_gate.data_ptr(), h_up.data_ptr(), token_indices.data_ptr(),
-                                              expert_offsets.data_ptr(), route_weights.data_ptr(), T, A, out.data_ptr(),
-                                              path, capi.ptr(ws), need, capi.stream_ptr(self.device)))
-        return out
+        return self._host.experts_forward(self._native, h_gate, h_up, token_indices, expert_offsets, route_weights, self.rank_out, path)
 
     def combine_down_basis(self, rank_accum: torch.Tensor, out_dtype: torch.dtype,
                            residual: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -193,35 +185,24 @@ class PackedLayer:
         return y
 
     def workspace(self, T: int, k: int) -> torch.Tensor:
-        key = (T, k)
-        ws = self._ws.get(key)
-        if ws is None:
-            need = int(capi.lib().bm_layer_workspace_bytes(self._handle, T, k))
-            ws = torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
-            if len(self._ws) > 8:
-                self._ws.clear()
-            self._ws[key] = ws
-        return ws
+        return self._host.layer_workspace(self._native, T, k)
 
     def forward(self, x: torch.Tensor, logits: torch.Tensor, top_k: int, norm_topk_prob: bool = True,
                 weight_dtype=torch.float16, residual: Optional[torch.Tensor] = None,
                 global_to_local: Optional[torch.Tensor] = None, path: int = capi.PATH_AUTO,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
         """x [T, H] (fp16 / bf16), logits [T, E_routed] -> y [T, H] in x's dtype.  One stream, no host sync."""
-        x = x.contiguous()
-        logits = logits.contiguous()
-        T = x.shape[0]
-        y = out if out is not None else torch.empty_like(x)
-        if residual is not None:
-            residual = residual.to(x.dtype).contiguous()
-        ws = self.workspace(T, top_k)
-        with torch.cuda.device(self.device):
-            capi.check(capi.lib().bm_layer_forward(
-                self._handle, x.data_ptr(), capi.dtype_code(x.dtype), logits.data_ptr(), capi.dtype_code(logits.dtype),
-                T, logits.shape[1], top_k, int(bool(norm_topk_prob)), capi.round_code(weight_dtype),
-                capi.ptr(global_to_local), capi.ptr(residual), y.data_ptr(), path, ws.data_ptr(), ws.numel(),
-                capi.stream_ptr(self.device)))
-        return y
+        return self._host.layer_forward(self._native, x, logits, top_k, norm_topk_prob, capi.round_code(weight_dtype), residual,
+                                        global_to_local, path, out)
+
+    def block_forward(self, x: torch.Tensor, gate_weight: torch.Tensor, top_k: int, norm_topk_prob: bool = True,
+                      weight_dtype=torch.float16, shared: Optional[Tuple] = None, global_to_local: Optional[torch.Tensor] = None):
+        """The whole block for x [T, H]: router Linear, packed experts and, with ``shared`` = (gate, up, down, token gate or
+        None) weights, the shared expert -> (y [T, H], router logits [T, E]).  None when the weights are not of one 16-bit
+        type on x's device; the caller then goes through the stages."""
+        sg, su, sd, st = shared if shared is not None else (None, None, None, None)
+        return self._host.block_forward(self._native, x, gate_weight, sg, su, sd, st, top_k, norm_topk_prob,
+                                        capi.round_code(weight_dtype), global_to_local)
 
 
 def route_topk(logits: torch.Tensor, top_k: int, norm_topk_prob: bool = True, weight_dtype=torch.float16):
@@ -290,19 +271,4 @@ def dense_mlp(x: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, w_down:
     sigmoid(x . token_gate_weight) when that is given, plus ``residual``.  Weights fp16; result in x's dtype."""
     if not x.is_cuda:
         raise RuntimeError("dense_mlp requires CUDA tensors; there is no CPU path")
-    x = x.contiguous()
-    dev = x.device
-    wg, wu, wd = (_as(w.detach(), torch.float16, dev) for w in (w_gate, w_up, w_down))
-    tg = None if token_gate_weight is None else _as(token_gate_weight.detach().reshape(-1), torch.float16, dev)
-    T, H, I = x.shape[0], x.shape[1], wg.shape[0]
-    y = torch.empty_like(x)
-    if residual is not None:
-        residual = residual.to(x.dtype).contiguous()
-    lib = capi.lib()
-    need = int(lib.bm_dense_mlp_workspace_bytes(T, I))
-    ws = torch.empty(max(need, 256), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
-        capi.check(lib.bm_dense_mlp_forward(x.data_ptr(), capi.dtype_code(x.dtype), wg.data_ptr(), wu.data_ptr(), wd.data_ptr(),
-                                            capi.ptr(tg), T, H, I, capi.ptr(residual), y.data_ptr(), capi.dtype_code(y.dtype),
-                                            ws.data_ptr(), ws.numel(), capi.stream_ptr(dev)))
-    return y
+    return capi.host().dense_mlp(x, w_gate, w_up, w_down, None if token_gate_weight is None else token_gate_weight.reshape(-1), residual)

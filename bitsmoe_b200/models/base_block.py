@@ -252,6 +252,30 @@ class BitsMoE_BaseSparseMoeBlock(nn.Module):
         return dense_mlp(x, parts[0].weight, parts[1].weight, parts[2].weight,
                          None if token_gate is None else token_gate.weight)
 
+    def _bare_weight(self, module) -> Optional[torch.Tensor]:
+        """The weight of a bias-free nn.Linear, else None (dict look-ups: this runs per layer and step)."""
+        if not isinstance(module, nn.Linear) or module._parameters.get("bias") is not None:
+            return None
+        return module._parameters.get("weight")
+
+    def _shared_weights(self):
+        """(gate, up, down, token gate or None) weights of a shared expert the library can run, None when the block has
+        no shared expert, False when it has one that only its own module can run."""
+        return None
+
+    def _one_call_forward(self, hidden_states: torch.Tensor):
+        """Router, packed experts and shared expert in one library call -> (y in the input's shape, router logits), or
+        None when a part of the block is not of the kind the library runs (the caller then goes through the stages)."""
+        layer = self._packed_layer
+        if layer is None or self._super_expert_items or not hidden_states.is_cuda or torch.is_grad_enabled():
+            return None
+        gate = self._bare_weight(self._modules.get("gate"))
+        shared = self._shared_weights()
+        if gate is None or shared is False:
+            return None
+        return layer.block_forward(hidden_states, gate, self.top_k, self.norm_topk_prob, hidden_states.dtype, shared,
+                                   None if self._identity_map else self._packed_global_to_local)
+
     # ---- fused path -----------------------------------------------------------------------------------
     def _require_fused(self, x: torch.Tensor):
         if self.shared_vh_gate_proj.numel() == 0 or self.shared_vh_up_proj.numel() == 0:

@@ -40,8 +40,11 @@ class BitsMoE_Qwen3MoeSparseMoeBlock(BitsMoE_BaseSparseMoeBlock):
 
     def forward(self, hidden_states: torch.Tensor):
         batch, seq, hidden = hidden_states.shape
+        self._ensure_runtime_cache(hidden_states.device)
+        done = self._one_call_forward(hidden_states)
+        if done is not None:
+            return done if getattr(self, "return_router_logits", True) else done[0]
         x = hidden_states.reshape(-1, hidden)
-        self._ensure_runtime_cache(x.device)
         router_logits = self._library_gate_logits(x)
         if router_logits is None:
             router_logits = self.gate(x)

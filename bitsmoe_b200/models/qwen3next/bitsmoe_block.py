@@ -34,6 +34,17 @@ class BitsMoE_Qwen3NextSparseMoeBlock(BitsMoE_Qwen3MoeSparseMoeBlock):
                                         unexpected_keys, error_msgs)
         self._invalidate_runtime_cache()
 
+    def _shared_weights(self):
+        mods = self._modules
+        if "shared_expert" not in mods or "shared_expert_gate" not in mods:
+            return None
+        parts = mods["shared_expert"]._modules
+        w = tuple(self._bare_weight(parts.get(n)) for n in ("gate_proj", "up_proj", "down_proj"))
+        token_gate = self._bare_weight(mods["shared_expert_gate"])
+        if any(p is None for p in w) or token_gate is None or token_gate.shape[0] != 1 or w[0].shape[0] % 2:
+            return False
+        return (*w, token_gate)
+
     def _shared_contribution(self, x: torch.Tensor) -> Optional[torch.Tensor]:
         if hasattr(self, "shared_expert") and hasattr(self, "shared_expert_gate"):
             y = self._library_dense_mlp(x, self.shared_expert, self.shared_expert_gate)

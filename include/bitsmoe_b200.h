@@ -233,6 +233,27 @@ BM_API int bm_dense_mlp_forward(const void* x, int x_dtype, const uint16_t* w_ga
                                 const uint16_t* token_gate_w, int32_t T, int32_t hidden, int32_t intermediate,
                                 const void* residual, void* y, int y_dtype, void* workspace, size_t workspace_bytes, void* stream);
 
+/* ---- whole block -------------------------------------------------------
+ * The dense parts of a block beside its packed experts, in the model's own type (w_dtype: BM_F16, or BM_BF16, which is
+ * rounded to fp16 on the way to the tensor cores); pointers that are NULL are left out.  `gate_w` [num_routed, hidden] is
+ * the router, sh_* the shared expert (sh_token_gate: its per-token sigmoid gate, [hidden]). */
+typedef struct bm_block_dense {
+  const uint16_t* gate_w;
+  const uint16_t* sh_gate;
+  const uint16_t* sh_up;
+  const uint16_t* sh_down;
+  const uint16_t* sh_token_gate;
+  int32_t sh_intermediate;
+  int32_t w_dtype;
+} bm_block_dense_t;
+/* bm_gate_logits -> bm_layer_forward with bm_dense_mlp_forward's result added: the whole forward of
+ * bitsmoe/models/qwen3moe/bitsmoe_block.py:39-98 (and of the qwen3next block) in one call.  `logits` [T, num_routed] of
+ * x_dtype receives the router logits.  dense->gate_w must be given; x is fp16 or bf16. */
+BM_API size_t bm_block_workspace_bytes(const bm_layer_t* layer, const bm_block_dense_t* dense, int32_t num_routed, int32_t T, int32_t k);
+BM_API int bm_block_forward(const bm_layer_t* layer, const bm_block_dense_t* dense, const void* x, int x_dtype, int32_t T,
+                            int32_t num_routed, int32_t k, int32_t renorm, int32_t weight_round, const int32_t* global_to_local,
+                            void* logits, void* y, void* workspace, size_t workspace_bytes, void* stream);
+
 /* ---- expert parallelism ------------------------------------------------
  * The reference has no distributed code (bitsmoe/models/deepseekv2/bitsmoe_block.py:57-62 copies ep_size / ep_rank and
  * never reads them).  These two kernels are the exchange that sharding the experts over the GPUs of one box needs; they
