@@ -9,6 +9,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <algorithm>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -353,9 +355,100 @@ PyObject* op_clear(PyObject*, PyObject*) {
   Py_RETURN_NONE;
 }
 
+// ---- packing one matrix
+at::Tensor ints(const std::vector<int32_t>& v, int64_t cols) {
+  const int64_t n = static_cast<int64_t>(v.size());
+  const at::Tensor t = cols ? at::empty({n / cols, cols}, at::kInt) : at::empty({n}, at::kInt);
+  if (n) memcpy(t.data_ptr(), v.data(), v.size() * 4);
+  return t;
+}
+
+// (rank_major fp32 [rank, dim] CUDA, s fp32 [rank] on the same device, [(bits, [(start, end), ...]), ...], to_host) ->
+// (payload, rank_idx, tile_meta, slab_meta, scale, s, segments): payload, scale and s on the factor's device, or with
+// to_host fetched in one copy into host tensors of their own
+PyObject* pack_matrix(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  return guarded([&]() -> PyObject* {
+    need_args(n, 4);
+    const at::Tensor w = tensor(a[0]), s = tensor(a[1]);
+    const bool to_host = PyObject_IsTrue(a[3]) == 1;
+    constexpr int SLAB = 64, TILE = 128, MICROS = 4;
+    const int64_t dim = w.size(1), tiles = (dim + TILE - 1) / TILE;
+    std::vector<int32_t> rows, slabs, slab_meta, tile_meta, segments;
+    int64_t words = 0, scales = 0;
+    PyObject* buckets = a[2];
+    for (Py_ssize_t b = 0; b < PyList_Size(buckets); ++b) {
+      PyObject* bucket = PyList_GetItem(buckets, b);
+      const int32_t bits = static_cast<int32_t>(integer(PyTuple_GetItem(bucket, 0)));
+      const int32_t wpr = bits == 16 ? 16 : bits, first = static_cast<int32_t>(rows.size());
+      PyObject* ranges = PyTuple_GetItem(bucket, 1);
+      for (Py_ssize_t i = 0; i < PyList_Size(ranges); ++i) {
+        PyObject* r = PyList_GetItem(ranges, i);
+        const int32_t e = static_cast<int32_t>(integer(PyTuple_GetItem(r, 1)));
+        for (int32_t x = static_cast<int32_t>(integer(PyTuple_GetItem(r, 0))); x < e; ++x) rows.push_back(x);
+      }
+      const int32_t end = static_cast<int32_t>(rows.size());
+      segments.insert(segments.end(), {bits, first, end});
+      for (int32_t r0 = first; r0 < end; r0 += SLAB) {
+        const int32_t k = std::min(SLAB, end - r0);
+        slabs.insert(slabs.end(), {bits, k});
+        slab_meta.insert(slab_meta.end(), {bits, k, r0, static_cast<int32_t>(tile_meta.size() / 3)});
+        const int64_t wpt = static_cast<int64_t>(k) * MICROS * wpr;
+        for (int64_t t = 0; t < tiles; ++t, words += wpt, scales += k)
+          tile_meta.insert(tile_meta.end(), {static_cast<int32_t>(words), static_cast<int32_t>(scales),
+                                             static_cast<int32_t>(std::min<int64_t>(TILE, dim - t * TILE))});
+      }
+    }
+    const int64_t stored = static_cast<int64_t>(rows.size());
+    const c10::cuda::CUDAGuard guard(w.device());
+    const auto dev = at::TensorOptions().device(w.device());
+    at::Tensor payload, scale, s_out;
+    if (to_host) {
+      // one device buffer and one pinned one: a single copy, then plain memory copies
+      auto up = [](int64_t v) { return (v + 255) & ~static_cast<int64_t>(255); };
+      const int64_t o_scale = up(words * 4), o_s = o_scale + up(scales * 2), total = o_s + stored * 2;
+      payload = at::empty({words}, at::kUInt32);
+      scale = at::empty({scales}, at::kHalf);
+      s_out = at::empty({stored}, at::kHalf);
+      if (total > 0) {
+        const at::Tensor d = at::empty({total}, dev.dtype(at::kByte));
+        const at::Tensor h = at::empty({total}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
+        char* base = static_cast<char*>(d.data_ptr());
+        check(bm_quantize_pack_matrix(static_cast<const float*>(w.data_ptr()), w.stride(0), static_cast<const float*>(s.data_ptr()),
+                                      static_cast<int32_t>(dim), rows.data(), slabs.data(), static_cast<int32_t>(slabs.size() / 2),
+                                      reinterpret_cast<uint32_t*>(base), reinterpret_cast<uint16_t*>(base + o_scale),
+                                      reinterpret_cast<uint16_t*>(base + o_s), stream_of(w.device())));
+        const auto stream = c10::cuda::getCurrentCUDAStream(w.device().index());
+        const cudaError_t e = cudaMemcpyAsync(h.data_ptr(), base, total, cudaMemcpyDeviceToHost, stream.stream());
+        if (e != cudaSuccess) fail(PyExc_RuntimeError, cudaGetErrorString(e));
+        cudaError_t done;
+        Py_BEGIN_ALLOW_THREADS
+        done = cudaStreamSynchronize(stream.stream());
+        Py_END_ALLOW_THREADS
+        if (done != cudaSuccess) fail(PyExc_RuntimeError, cudaGetErrorString(done));
+        const char* hb = static_cast<const char*>(h.data_ptr());
+        memcpy(payload.data_ptr(), hb, words * 4);
+        memcpy(scale.data_ptr(), hb + o_scale, scales * 2);
+        memcpy(s_out.data_ptr(), hb + o_s, stored * 2);
+      }
+    } else {
+      payload = at::empty({words}, dev.dtype(at::kUInt32));
+      scale = at::empty({scales}, dev.dtype(at::kHalf));
+      s_out = at::empty({stored}, dev.dtype(at::kHalf));
+      check(bm_quantize_pack_matrix(static_cast<const float*>(w.data_ptr()), w.stride(0), static_cast<const float*>(s.data_ptr()),
+                                    static_cast<int32_t>(dim), rows.data(), slabs.data(), static_cast<int32_t>(slabs.size() / 2),
+                                    static_cast<uint32_t*>(payload.data_ptr()), static_cast<uint16_t*>(scale.data_ptr()),
+                                    static_cast<uint16_t*>(s_out.data_ptr()), stream_of(w.device())));
+    }
+    const at::Tensor out[7] = {payload, ints(rows, 0), ints(tile_meta, 3), ints(slab_meta, 4), scale, s_out, ints(segments, 3)};
+    PyObject* r = PyTuple_New(7);
+    for (int i = 0; i < 7; ++i) PyTuple_SET_ITEM(r, i, THPVariable_Wrap(out[i]));
+    return r;
+  });
+}
+
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {FAST(layer_new), FAST(layer_close), FAST(layer_drop_workspaces), FAST(layer_workspace), FAST(layer_forward),
-                         FAST(block_forward), FAST(dense_mlp), FAST(experts_forward), FAST(op_forward), FAST(op_register),
+                         FAST(block_forward), FAST(dense_mlp), FAST(experts_forward), FAST(op_forward), FAST(op_register), FAST(pack_matrix),
                          {"op_clear", op_clear, METH_NOARGS, nullptr}, {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_bm_host", "Native host path of bitsmoe_b200.", -1, methods, nullptr, nullptr, nullptr, nullptr};
 

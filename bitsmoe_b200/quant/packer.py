@@ -26,6 +26,8 @@ MICROS_PER_TILE = N_TILE // N_MICRO
 _SUPPORTED_BITS = {1, 2, 3, 4, 6, 8, 16}
 _BIT_OFFSETS = {1: 1, 2: 2, 3: 4, 4: 8, 6: 32, 8: 128}
 
+_EXACT_IN_FP32 = (torch.float32, torch.float16, torch.bfloat16)
+
 RUNTIME_KEYS = ("payload_buffer", "rank_idx_buffer", "tile_meta_buffer", "slab_meta_buffer", "scale_buffer")
 
 
@@ -120,9 +122,9 @@ def quantize_rows(rows: Tensor, bits: int) -> Tuple[Tensor, Tensor]:
     return q.view(n, tiles * N_TILE), sc
 
 
-def bucket_segments(segments: Sequence[Tuple[int, Tuple[int, int]]], rank: int) -> List[Tuple[int, Tensor]]:
-    """Rows per bit width, widest bucket first, ranges by ascending start; 0-bit rows are dropped."""
-    taken = torch.zeros(rank, dtype=torch.bool)
+def bucket_ranges(segments: Sequence[Tuple[int, Tuple[int, int]]], rank: int) -> List[Tuple[int, List[Tuple[int, int]]]]:
+    """Row ranges per bit width, widest bucket first, ranges by ascending start; 0-bit rows are dropped."""
+    taken: List[Tuple[int, int]] = []
     by_bits: Dict[int, List[Tuple[int, int]]] = {}
     for bits, (s, e) in segments:
         bits, s, e = int(bits), int(s), int(e)
@@ -132,17 +134,17 @@ def bucket_segments(segments: Sequence[Tuple[int, Tuple[int, int]]], rank: int) 
             raise ValueError(f"Invalid segment range (s={s}, e={e}) for rank={rank}")
         if s == e:
             continue
-        if bool(taken[s:e].any()):
+        if any(s < b and a < e for a, b in taken):
             raise ValueError(f"Overlapping segments in range [{s}, {e})")
-        taken[s:e] = True
+        taken.append((s, e))
         by_bits.setdefault(bits, []).append((s, e))
-    out = []
-    for bits in sorted(by_bits, reverse=True):
-        if bits == 0:
-            continue
-        idx = torch.cat([torch.arange(s, e, dtype=torch.int32) for s, e in sorted(by_bits[bits])])
-        out.append((bits, idx))
-    return out
+    return [(bits, sorted(by_bits[bits])) for bits in sorted(by_bits, reverse=True) if bits != 0]
+
+
+def bucket_segments(segments: Sequence[Tuple[int, Tuple[int, int]]], rank: int) -> List[Tuple[int, Tensor]]:
+    """Rows per bit width, in the order of ``bucket_ranges``."""
+    return [(bits, torch.cat([torch.arange(s, e, dtype=torch.int32) for s, e in ranges]))
+            for bits, ranges in bucket_ranges(segments, rank)]
 
 
 def quantize_pack_slab(rows: Tensor, bits: int, want_codes: bool = False):
@@ -168,10 +170,10 @@ def quantize_pack_slab(rows: Tensor, bits: int, want_codes: bool = False):
 
 def pack_rank_major(rank_major: Tensor, s_vec: Tensor, segments, groupsize: int = N_TILE,
                     precomputed: Optional[Dict[int, Tuple[Tensor, Tensor]]] = None,
-                    fused: Optional[bool] = None) -> Dict[str, Tensor]:
+                    fused: Optional[bool] = None, to_host: bool = False) -> Dict[str, Tensor]:
     """Quantise + pack a rank-major factor [rank, dim].  ``precomputed[bits] = (plane words
     [rank, tiles, 4, bits], scales [rank, tiles])`` lets a caller that quantised and bit-sliced many
-    experts in one batch skip both steps.  Buffers stay on the factor's device."""
+    experts in one batch skip both steps.  Buffers stay on the factor's device unless ``to_host``."""
     if groupsize != N_TILE:
         raise ValueError(f"Current runtime layout requires groupsize == N_TILE ({N_TILE}), got {groupsize}")
     rank, dim = rank_major.shape
@@ -184,6 +186,18 @@ def pack_rank_major(rank_major: Tensor, s_vec: Tensor, segments, groupsize: int 
     dev = rank_major.device
     if fused is None:
         fused = dev.type == "cuda" and precomputed is None
+    if fused and s_vec.device == dev and rank_major.dtype in _EXACT_IN_FP32 and s_vec.dtype in _EXACT_IN_FP32:
+        # the whole matrix in one launch: quantise, bit-plane pack, reorder
+        from .. import capi
+        rows = rank_major.detach().to(torch.float32)
+        if rows.stride(1) != 1 or rows.stride(0) < dim:
+            rows = rows.contiguous()
+        out = capi.host().pack_matrix(rows, s_vec.detach().to(torch.float32).contiguous(), bucket_ranges(segments, rank), to_host)
+        buf = dict(zip(("payload_buffer", "rank_idx_buffer", "tile_meta_buffer", "slab_meta_buffer", "scale_buffer", "s_buffer", "segments"), out))
+        buf["original_indices"] = buf["rank_idx_buffer"].clone()
+        buf["original_rank"] = torch.tensor(rank, dtype=torch.int32)
+        buf["groupsize"] = torch.tensor(groupsize, dtype=torch.int16)
+        return buf
     tiles = (dim + N_TILE - 1) // N_TILE
     payload, scales, ridx, s_parts = [], [], [], []
     slab_rows, tile_rows, seg_rows = [], [], []
@@ -347,7 +361,7 @@ def pack_single_weight(moe_dict, segments, state_dict: Dict[str, Tensor], layer_
     device = torch.device("cuda") if torch.cuda.is_available() else torch.device("cpu")
     t0 = time.perf_counter()
     rank_major, s_vec, field = _rank_major_and_s(moe_dict, layer_idx, expert_idx, mtype, device)
-    buf = pack_rank_major(rank_major, s_vec, segments, groupsize)
+    buf = pack_rank_major(rank_major, s_vec, segments, groupsize, to_host=True)
     prefix = f"quantized.layer{layer_idx}.expert{expert_idx}.{mtype}"
     for key in RUNTIME_KEYS:
         state_dict[f"{prefix}.{field}.{key}"] = buf[key].cpu()

@@ -67,6 +67,12 @@ BM_API int bm_unpack_bitplanes_i8(const uint32_t* words, int8_t* q, int64_t rows
  * the signed codes.  bits in {1, 2, 3, 4, 6, 8}. */
 BM_API int bm_quantize_pack_slab(const float* rows, int64_t row_stride, int32_t k, int32_t dim, int32_t bits, uint32_t* payload,
                                  uint16_t* scale, int8_t* codes, void* stream);
+/* All slabs of one matrix: rank_major fp32 [*, dim] (row_stride elements between rows), s fp32 per rank; `slabs` (host)
+ * holds n_slabs pairs (bits, rows <= 64) in stored order, `rows` (host) the logical row of every stored row.  payload,
+ * scale and s_out are the matrix's payload_buffer, scale_buffer and s_buffer; bits 16 stores the rows as raw fp16. */
+BM_API int bm_quantize_pack_matrix(const float* rank_major, int64_t row_stride, const float* s, int32_t dim, const int32_t* rows,
+                                   const int32_t* slabs, int32_t n_slabs, uint32_t* payload, uint16_t* scale, uint16_t* s_out,
+                                   void* stream);
 
 /* ---- layer state -------------------------------------------------------
  * One packed expert matrix exactly as the reference stores it: the six

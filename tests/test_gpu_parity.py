@@ -568,3 +568,22 @@ def test_deterministic_mode_is_bit_reproducible(q30_small, path, T):
     assert torch.equal(y1, y2)
     helpers.assert_close(runs[0], plain, rtol=1e-5, atol=1e-7, what="deterministic vs fp32-atomic accumulation")
     helpers.assert_close(runs[0], o["rank_accum"], rtol=1e-2, atol=3e-4, what="deterministic mode vs fp32 oracle")
+
+
+@pytest.mark.parametrize("rank,dim,segs", [
+    (256, 768, [(4, (0, 12)), (3, (12, 51)), (2, (51, 256))]),
+    (70, 160, [(8, (0, 3)), (2, (10, 70)), (16, (3, 8)), (0, (8, 10))]),           # wide rows, dropped rows, ragged tile
+    (1100, 128, [(2, (0, 500)), (1, (500, 1000)), (2, (1000, 1100))]),             # more rows than one launch takes
+    (3, 32, [(6, (0, 1)), (3, (2, 3))])])
+def test_matrix_packer_matches_host_packer(rank, dim, segs):
+    from bitsmoe_b200.quant import packer as ppacker
+    g = torch.Generator().manual_seed(rank)
+    R, S = torch.randn(dim, rank, generator=g) * 0.02, torch.rand(rank, generator=g) + 0.2
+    host = ppacker.pack_rank_major(R.T.contiguous(), S, segs)
+    for to_host in (False, True):
+        dev = ppacker.pack_rank_major(R.T.contiguous().to(DEV), S.to(DEV), segs, to_host=to_host)
+        assert dev["payload_buffer"].is_cuda != to_host
+        for key in host:
+            a, b = host[key], dev[key].cpu()
+            assert a.dtype == b.dtype and a.shape == b.shape, key
+            assert torch.equal(a.view(torch.int32) if a.dtype == torch.uint32 else a, b.view(torch.int32) if b.dtype == torch.uint32 else b), key
