@@ -1,9 +1,28 @@
 // Planning and building of the arena layout (see fast_layout.cuh), and decoding it back to
 // integer codes for the bit-exactness tests.
+#include <algorithm>
+
 #include "fast_layout.cuh"
 
 namespace bm {
 
+
+// Rows of a group by ascending rank, the ranks that come as whole aligned octets first: the kernels move such an octet of
+// a token's row as one 16-byte piece and take the remaining ranks one by one.
+static void order_by_octets(std::vector<int16_t>& rows, const std::vector<int32_t>& rank_idx) {
+  std::sort(rows.begin(), rows.end(), [&](int16_t a, int16_t b) { return rank_idx[a] != rank_idx[b] ? rank_idx[a] < rank_idx[b] : a < b; });
+  std::vector<int16_t> whole, rest;
+  for (size_t i = 0; i < rows.size();) {
+    const int r = rank_idx[rows[i]];
+    bool oct = r >= 0 && r % 8 == 0 && i + 8 <= rows.size();
+    for (int j = 1; oct && j < 8; ++j) oct = rank_idx[rows[i + j]] == r + j;
+    const size_t n = oct ? 8 : 1;
+    (oct ? whole : rest).insert((oct ? whole : rest).end(), rows.begin() + i, rows.begin() + i + n);
+    i += n;
+  }
+  whole.insert(whole.end(), rest.begin(), rest.end());
+  rows.swap(whole);
+}
 
 // Decides whether the layer fits the fast layout and lays it out after `base_bytes` of arena.
 void plan_fast(const bm_layer* L, size_t base_bytes, FastPlan* P) {
@@ -44,18 +63,21 @@ void plan_fast(const bm_layer* L, size_t base_bytes, FastPlan* P) {
           const long cost = 16L * p0 + 8L * p1 + 128L * ((p0 + p1) / 16);
           if (best_cost < 0 || cost < best_cost) { best_cost = cost; best_m = m; }
         }
-        for (int i = 0; i < best_m; ++i) {
-          rows[0].push_back(rows[1].back());
-          rows[1].pop_back();
-        }
+        // the rows next to the nibble group go over: with wide rows at the low ranks both groups stay runs of ranks
+        rows[0].insert(rows[0].end(), rows[1].begin(), rows[1].begin() + best_m);
+        rows[1].erase(rows[1].begin(), rows[1].begin() + best_m);
       }
       int total_blk = 0;
       for (int g = 0; g < 2; ++g) {
         const int padded = (static_cast<int>(rows[g].size()) + gran - 1) / gran * gran;
         fm.nblk[g] = padded / 16;
         total_blk += fm.nblk[g];
-        for (int i = 0; i < padded; ++i)
-          P->slot_row.push_back(i < static_cast<int>(rows[g].size()) ? rows[g][i] : static_cast<int16_t>(-1));
+        const size_t first = P->slot_row.size();
+        P->slot_row.resize(first + padded, static_cast<int16_t>(-1));
+        order_by_octets(rows[g], mh.rank_idx);
+        // gate / up: rows in the order of the token-side operand, so that an aligned octet of ranks is one 16-byte piece
+        for (int i = 0; i < static_cast<int>(rows[g].size()); ++i)
+          P->slot_row[first + (w < 2 ? (i & ~31) + pos32_inv(i & 31) : i)] = rows[g][i];
       }
       if (total_blk == 0) return;
       fm.nslots = total_blk * 16;
@@ -131,8 +153,9 @@ __global__ void __launch_bounds__(128) repack_tables_kernel(const ExpertDev* __r
         break;
       }
     }
-    // gate / up scales are stored in the order of the token-side operand (see pos32)
-    scale_out[w < 2 ? slot_pos(slot) : slot] = sc;
+    // gate / up scales are stored in the order of the token-side operand (see pos32), down scales with the two rows of
+    // an MMA fragment (g, g + 8) side by side
+    scale_out[w < 2 ? slot_pos(slot) : down_scale_pos(slot)] = sc;
     if (tile == 0) {
       int rk = row >= 0 ? md.rank_idx[row] : -1;
       if (rk < 0 || rk > 32000) rk = -1;

@@ -81,6 +81,7 @@ struct SlabHost {
 struct MatHost {
   std::vector<SlabHost> slabs;
   std::vector<int32_t> tile_meta;  // [n_tile_rows * 3]
+  std::vector<int32_t> rank_idx;   // [n_rows]
   int64_t bytes = 0;               // as stored by the reference
   int32_t n_rows = 0;
 };

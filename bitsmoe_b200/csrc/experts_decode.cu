@@ -593,7 +593,8 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
                 mma_pairs<true>(dwords + fd.nblk[0] * 256 + (mb - fd.nblk[0]) * 128 + lane, 32, 4, zrow, dacc);
                 off = static_cast<float>(FAST_DENSE_OFFSET);
               }
-              const float sc_lo = __half2float(scale_d[mb * 16 + g]), sc_hi = __half2float(scale_d[mb * 16 + g + 8]);
+              const float2 sc = __half22float2(*reinterpret_cast<const __half2*>(scale_d + mb * 16 + 2 * g));     // rows g and g + 8
+              const float sc_lo = sc.x, sc_hi = sc.y;
               dtot[i2][0] += sc_lo * (dacc[0] * DEC_UNSCALE_LO - off * zsum[0]);
               dtot[i2][1] += sc_lo * (dacc[1] * DEC_UNSCALE_LO - off * zsum[1]);
               dtot[i2][2] += sc_hi * (dacc[2] * DEC_UNSCALE_HI - off * zsum[0]);

@@ -1,56 +1,62 @@
 // Packed routed-expert forward for large token counts (prefill): fused mixed-bit grouped GEMM on the
 // 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory).
 //
-// Work item = (expert, block of up to NT of its assignments; NT -- 64 where it fits -- is chosen per layer so that the
-// activation operand of an item, two z tiles and enough copy / conversion stages fit in shared memory and seven
-// accumulators of NT columns fit in tensor memory).  One persistent CTA per SM walks the
-// items.  For an item the three products of every 128-column tile run with the WEIGHTS as the 128-row operand:
-//   gate/up:  D_g[c, n] = sum_slot  W_g[c, slot] * act_g[n, slot]      (M = 128 columns c, N = the item's tokens)
-//   down:     D_d[slot, n] += sum_c W_d[slot, c] * z[n, c]             (M = 128 row slots x 2 or 3, same N)
-// N of the MMAs is the item's token count rounded up to 16, so a short item costs a short MMA; every code is converted
-// once per item, so the conversion work per token falls with NT.  D_d accumulates over all tiles in TMEM.
-// Warp roles (608 threads):
-//   warps 0-7   epilogue (two per TMEM lane quarter, alternate 32-token column chunks): tcgen05.ld D_g/D_u ->
-//               z = silu(g)*u -> fp16 z tile in shared memory; at the end of the item D_d * s * route weight is
-//               transposed through the idle operand ring and added to rank_accum row by row (16-byte vector
-//               reductions).  Warp 0 also looks up the next item while the current one runs.
-//   warp  8     producer: cp.async.bulk of the packed words + scales of (tile, matrix) sections into a ring of slots
-//   warps 9,10  MMA issue, one thread each.  tcgen05.mma blocks its thread until the tensor pipe accepts it, so the
+// Work item = (expert, block of up to NT of its assignments; NT = 128 where it fits).  One persistent CTA per SM walks
+// the items.  The item's tokens are the 128 rows (M) of every product and the weights its columns (N); the tile's columns
+// are taken 64 at a time ("chunk"):
+//   gate/up:  D_g[n, c] = sum_slot act_g[n, slot] * W_g[c, slot]     (N = 64 columns c, K = row slots)
+//   down:     D_d[n, slot] += sum_c z[n, c] * W_d[slot, c]           (N = 128 row slots x 1..3, K = 64 columns c)
+// Tokens as rows make the epilogue cheap: a thread owns a token, so eight z values leave as one 16-byte store in the
+// order the down product reads them (the transposed orientation stored every z on its own, two bytes at a time), and 128
+// tokens share one conversion of the weights.  64 columns at a time leave room in tensor memory for two gate/up
+// accumulator pairs (2 x 128 columns) beside the down accumulator (256), so the products of a chunk run while the
+// previous one is turned into z.
+//
+// Warp roles (640 threads; warp 19 completes the last warpgroup):
+//   warps 0-7   epilogue (two per TMEM lane quarter, 32 columns each): tcgen05.ld D_g/D_u -> z = silu(g)*u -> fp16 z
+//               operand in shared memory; at the end of the item D_d * s * route weight is transposed through the idle
+//               activation area and added to rank_accum row by row (16-byte vector reductions).
+//   warp  16    looks up the next item while the current one runs and asks L2 for its weights
+//   warps 17,18 MMA issue, one thread each.  tcgen05.mma blocks its thread until the tensor pipe accepts it, so the
 //               waits and commits around a stage cost tensor time when one thread issues everything; two pipelines
-//               (9: gate products and the down product's even row tiles, 10: up products and the odd row tiles)
-//               hide one another's bookkeeping and never write the same accumulator.
-//   warps 11-18 converters, one team of four warps per pipeline: arena words (nibble / dense 2-bit codes) -> fp16
-//               (q * scale) operand stages of 128 rows x 64 contraction positions in the canonical K-major
-//               core-matrix layout, a ring of stages per pipeline; together with the epilogue warps they also build
-//               the activation operand act[n, slot] = fp16(h[token, rank(slot)] * s(slot)) once per item
-// Order of the (tile, matrix) sections of an item, the same for the producer, the converters and the MMA issuer:
-//   G0 U0 | G1 U1 D0 | G2 U2 D1 | ... | D(last)
-// The down product of a tile is issued one tile late, and the gate/up accumulators and the z tile are double-buffered,
-// so the tensor pipe works on the next tile's gate/up products while the epilogue warps turn the current tile's
-// accumulators into z.
-// Every mbarrier wait is bounded in time and aborts the whole CTA through a shared flag.
+//               (17: gate products and the down product's even slot tiles, 18: up products and the odd ones) hide one
+//               another's bookkeeping and never write the same accumulator.
+//   warps 8-15  converters, one team of four warps per pipeline: arena words (nibble / dense 2-bit codes), read straight
+//               from L2 one stage ahead into registers, -> fp16 (q * scale) operand stages of 64 rows x 32 positions in the
+//               canonical K-major core-matrix layout, a ring of stages per pipeline, a stage per warp.
+// Epilogue and converter warps together build the activation operand act[n, slot] = fp16(h[token, rank(slot)] * s(slot))
+// once per item.
+//
+// The down product of a chunk is issued one chunk late (G0 U0 | G1 U1 D0 | G2 U2 D1 | ...).  Every mbarrier wait is
+// bounded in time and aborts the whole CTA through a shared flag.
 #include "fast_layout.cuh"
 #include "tc05.cuh"
 
 namespace bm {
 
-constexpr int XT_NT_MAX = 96;             // most tokens (assignments) per item = largest MMA N
-constexpr int XT_THREADS = 608;
-constexpr int XT_EPI_WARPS = 8, XT_PRODUCER_WARP = 8, XT_MMA_WARP0 = 9, XT_DQ_WARP0 = 11, XT_DQ_WARPS = 8;
-constexpr int XT_RING_MAX = 8;            // A-operand stages (at most)
-constexpr int XT_STAGE_BLOCKS = 4;        // contraction blocks of 16 per stage (one per dequantiser warp pair)
-constexpr int XT_A_CHUNK = 128 * 16 + 32;  // bytes between 8-position chunks of a weight stage (padded: conflict-free 16-byte stores)
-constexpr int XT_STAGE_BYTES = 2 * XT_STAGE_BLOCKS * XT_A_CHUNK;
+constexpr int XT_NT_MAX = 128;            // most tokens (assignments) per item: the rows of one MMA
+constexpr int XT_THREADS = 640;
+constexpr int XT_EPI_WARPS = 8, XT_DQ_WARP0 = 8, XT_DQ_WARPS = 8, XT_LOOKUP_WARP = 16, XT_MMA_WARP0 = 17;
+// Registers per thread at launch and per role afterwards.  The converters keep two stages' words and four independent
+// blocks in flight; at the launch's 96 they spilled, and a spilled load result stalls its warp for the load's latency.
+constexpr int XT_REGS = 96, XT_REGS_EPI = 96, XT_REGS_DQ = 120, XT_REGS_MISC = 48;
+static_assert(32 * (XT_EPI_WARPS * XT_REGS_EPI + XT_DQ_WARPS * XT_REGS_DQ + 4 * XT_REGS_MISC) <= XT_THREADS * XT_REGS,
+              "the roles' registers come out of the launch's");
+constexpr int XT_CHUNK = 64;              // tile columns per step
+constexpr int XT_RING_MAX = 8;            // operand stages per pipeline (at most)
+// A weight stage: 64 operand rows (columns of the chunk, or slots) x 32 contraction positions; bytes between its
+// 8-position chunks (padded: conflict-free 16-byte stores)
+constexpr int XT_W_STRIDE = 64 * 16 + 32;
+constexpr int XT_STAGE_BYTES = 4 * XT_W_STRIDE;
 // bytes between 8-position chunks of the token-side operands (padded: conflict-free stores)
 __host__ __device__ constexpr int xt_chunk_stride(int nt) { return nt * 16 + 16; }
 constexpr int XT_MAX_E = 1024;
-constexpr int XT_SEC_MAX = 6;             // section slots (at most): (tile, matrix) sections this many ahead
+constexpr int XT_SLOTS_MAX = 384, XT_RANK_MAX = 1024;
 
 struct XtBars {
-  uint64_t sec_full[XT_SEC_MAX], sec_empty[XT_SEC_MAX];
-  uint64_t w_full[XT_RING_MAX], w_empty[XT_RING_MAX];
+  uint64_t w_full[2 * XT_RING_MAX], w_empty[2 * XT_RING_MAX];
   uint64_t act_ready, down_done;
-  // per buffer (running tile number & 1): gate/up accumulators complete / read out, z tile written / consumed
+  // gate/up accumulators complete / read out, z operand written / consumed, per buffer
   uint64_t gu_done[2], tmem_gu_free[2], z_ready[2], z_free[2];
 };
 
@@ -60,16 +66,27 @@ struct XtCycle {
   __device__ __forceinline__ void next(uint32_t n) {
     if (++i == n) { i = 0; ph ^= 1u; }
   }
+  __device__ __forceinline__ void advance(uint32_t k, uint32_t n) {
+    const uint32_t to = i + k, wraps = to / n;
+    i = to - wraps * n;
+    ph ^= wraps & 1u;
+  }
 };
 
 struct XtItem {
   FastExpert fe;
   int tok[XT_NT_MAX];
   float rw[XT_NT_MAX];
-  int n, expert;
+  __align__(16) float s_d[XT_SLOTS_MAX];         // the down product's slots: factor,
+  __align__(16) int16_t rank_d[XT_SLOTS_MAX];    // rank or -1,
+  int16_t oct_d[XT_SLOTS_MAX / 8];               // first rank of eight slots that hold an aligned octet of ranks, or -1
+  uint32_t broken[2][XT_RANK_MAX / 256];         // gate, up: octets of ranks that are not one piece of the operand row
+  int n, chunk0, nchunk;
+  int padded;                                    // gate or up has slots without a row
+  int all_ranks;                                 // every rank of rank_accum has a down slot
 };
 
-__device__ __noinline__ bool xt_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+__device__ __forceinline__ bool xt_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   const uint32_t addr = tc::smem_u32(bar);
   uint64_t t0 = 0;
   for (uint32_t i = 0;; ++i) {
@@ -136,84 +153,180 @@ __device__ __forceinline__ void dequant_pair_store(uint32_t word0, uint32_t word
 
 struct XtSmem {
   unsigned char* act;     // [2][nchunks][nt rows] canonical K-major, 16-byte chunks
-  unsigned char* z;       // [2 buffers][16 chunks][nt rows]
+  unsigned char* z;       // [2 buffers][8 chunks][nt rows]
   unsigned char* ring;    // [2 pipelines][ring_h][XT_STAGE_BYTES]
-  unsigned char* sec0;    // sec_n section buffers of sec_stride bytes: [scale (sec_scale_bytes) | words]
-  uint32_t sec_stride;
   int* prefix;            // [E + 1] items before each expert
-  int32_t* dst_r;         // [2][h_rank] byte offset of a rank's contraction position inside an operand row (gate, up), or -1
-  __half* s_r;            // [2][h_rank] its factor s
+  // per item (two of them) and matrix (gate, up), by rank: its factor s, its contraction position (or -1), and per octet of
+  // ranks the 16-byte piece of the operand row that holds it (or -1)
+  __half* s_r;            // [h_rank]
+  int16_t* pos_r;         // [h_rank]
+  int16_t* oct_r;         // [h_rank / 8]
 };
 
-__host__ __device__ inline size_t xt_sec_bytes(int max_slots, int max_words) {
-  return align_up_c(static_cast<size_t>(max_slots) * 2, 128) + align_up_c(static_cast<size_t>(max_words) * 4, 128);
-}
-__host__ __device__ inline size_t xt_smem_bytes(int max_slots, int max_words, int num_experts, int h_rank, int nt, int ring_n, int sec_n) {
-  size_t o = 0;
-  o += static_cast<size_t>(2) * (max_slots / 8) * xt_chunk_stride(nt);   // act
-  o += static_cast<size_t>(2) * (N_TILE / 8) * xt_chunk_stride(nt);      // z, two buffers
-  o = align_up_c(o, 128) + static_cast<size_t>(ring_n) * XT_STAGE_BYTES;       // ring
-  o += sec_n * xt_sec_bytes(max_slots, max_words);
+__host__ __device__ inline size_t xt_act_bytes(int max_slots, int nt) { return static_cast<size_t>(2) * (max_slots / 8) * xt_chunk_stride(nt); }
+__host__ __device__ inline size_t xt_z_bytes(int nt) { return static_cast<size_t>(XT_CHUNK / 8) * xt_chunk_stride(nt); }
+__host__ __device__ inline size_t xt_smem_bytes(int max_slots, int num_experts, int h_rank, int nt, int ring_h) {
+  size_t o = align_up_c(xt_act_bytes(max_slots, nt) + 2 * xt_z_bytes(nt), 128);
+  o += static_cast<size_t>(2 * ring_h) * XT_STAGE_BYTES;
   o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);
-  o += align_up_c(static_cast<size_t>(2) * h_rank * 6, 128);         // per-rank tables of the activation staging
-  return o + 1024;                                          // slack for the 1024-byte base alignment
+  o += align_up_c(static_cast<size_t>(4) * (h_rank * 4 + h_rank / 4), 128);         // per-rank tables of the activation staging
+  // the MMAs read 128 operand rows whatever nt is: rows past nt of the last chunk lie in what follows the z buffers
+  return o + 1024;                                                   // slack for the 1024-byte base alignment
 }
 
-// Locates item `it` (last expert e with prefix[e] <= it) and copies what the roles need; one warp.
-__device__ __forceinline__ void xt_load_item(XtItem& item, int it, const int* prefix, int num_experts, int nt, int T,
-                                             const FastExpert* __restrict__ fast, const int32_t* __restrict__ token_indices,
-                                             const int32_t* __restrict__ expert_offsets, const float* __restrict__ route_w,
-                                             int lane) {
-  int lo = 0, hi = num_experts - 1;
+// Units of work.  Items that fill whole rounds of the grid are units of their own; the items of the last, partial round
+// are cut along the tile columns so that the round's CTAs share them evenly (their down sums meet in rank_accum anyway).
+struct XtUnits {
+  int full, split, per, n_units;
+  __device__ __forceinline__ XtUnits(int n_items, int grid, int n_chunks) {
+    const int rem = n_items % grid;
+    full = n_items - rem;
+    split = rem ? grid / rem : 1;
+    split = split > n_chunks ? n_chunks : split;
+    per = (n_chunks + split - 1) / split;
+    split = (n_chunks + per - 1) / per;
+    n_units = full + rem * split;
+  }
+};
+
+struct XtArgs {
+  const FastExpert* fast;
+  const unsigned char* arena;
+  const __half* h_gate;
+  const __half* h_up;
+  const int32_t* token_indices;
+  const int32_t* expert_offsets;
+  const float* route_w;
+  float* rank_accum;
+  long long* acc64;
+  int* status;
+  int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, ring_h, gu_bufs;
+};
+
+// Locates unit `u` and copies what the roles need, its tables turned into the order the roles read them; one warp, an item
+// ahead of the roles.
+__device__ __forceinline__ void xt_load_item(XtItem& item, const XtSmem& sm, int buf, int u, const XtUnits& units, int n_chunks,
+                                             const XtArgs& A, int lane) {
+  const int* prefix = sm.prefix;
+  __half* s_r = sm.s_r + buf * 2 * A.h_rank;
+  int16_t* pos_r = sm.pos_r + buf * 2 * A.h_rank;
+  int16_t* oct_r = sm.oct_r + buf * 2 * (A.h_rank / 8);
+  int it = u, chunk0 = 0, nchunk = n_chunks;
+  if (u >= units.full) {
+    const int r = u - units.full, part = r % units.split;
+    it = units.full + r / units.split;
+    chunk0 = part * units.per;
+    nchunk = min(units.per, n_chunks - chunk0);
+  }
+  int lo = 0, hi = A.num_experts - 1;           // last expert e with prefix[e] <= it
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (prefix[mid] <= it) lo = mid; else hi = mid - 1;
   }
   const int e = lo;
-  const int a0 = expert_offsets[e] + (it - prefix[e]) * nt;
-  const int n = min(nt, expert_offsets[e + 1] - a0);
   for (int i = lane; i < static_cast<int>(sizeof(FastExpert) / 4); i += 32)
-    reinterpret_cast<uint32_t*>(&item.fe)[i] = reinterpret_cast<const uint32_t*>(&fast[e])[i];
-  for (int i = lane; i < nt; i += 32) {
-    const int tk = i < n ? token_indices[a0 + i] : 0;
-    const bool good = i < n && tk >= 0 && tk < T;
+    reinterpret_cast<uint32_t*>(&item.fe)[i] = reinterpret_cast<const uint32_t*>(&A.fast[e])[i];
+  // an expert's assignments are spread evenly over its items
+  const int begin = A.expert_offsets[e], cnt = A.expert_offsets[e + 1] - begin, parts = prefix[e + 1] - prefix[e], j = it - prefix[e];
+  const int a0 = begin + static_cast<int>(static_cast<int64_t>(cnt) * j / parts);
+  const int n = begin + static_cast<int>(static_cast<int64_t>(cnt) * (j + 1) / parts) - a0;
+#pragma unroll
+  for (int q = 0; q < XT_NT_MAX / 32; ++q) {
+    const int i = lane + 32 * q;
+    const int tk = i < n ? A.token_indices[a0 + i] : 0;
+    const bool good = i < n && tk >= 0 && tk < A.T;
     item.tok[i] = good ? tk : 0;
-    item.rw[i] = good ? route_w[a0 + i] : 0.f;
+    item.rw[i] = good ? A.route_w[a0 + i] : 0.f;
   }
-  if (lane == 0) { item.n = n; item.expert = e; }
+  for (int i = lane; i < 2 * A.h_rank; i += 32) {
+    pos_r[i] = -1;
+    s_r[i] = __float2half(0.f);
+  }
+  for (int i = lane; i < 2 * (A.h_rank / 8); i += 32) oct_r[i] = -1;
+  __syncwarp();
+  bool padded = false;
+  int live_d = 0;
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    const FastMat& fm = item.fe.m[m];
+    const int16_t* rank_t = reinterpret_cast<const int16_t*>(A.arena + fm.tab_off);
+    const __half* s_t = reinterpret_cast<const __half*>(A.arena + fm.tab_off + fm.nslots * 2);
+#pragma unroll 8
+    for (int i = lane; i < fm.nslots; i += 32) {
+      const int rk = rank_t[i];
+      const __half sv = s_t[i];
+      if (m == 2) {
+        const bool live = rk >= 0 && rk < A.rank_out;
+        item.rank_d[i] = static_cast<int16_t>(live ? rk : -1);
+        item.s_d[i] = __half2float(sv);
+        live_d += live;
+      } else if (rk >= 0 && rk < A.h_rank) {
+        pos_r[m * A.h_rank + rk] = static_cast<int16_t>(slot_pos(i));
+        s_r[m * A.h_rank + rk] = sv;
+      } else {
+        padded = true;
+      }
+    }
+  }
+  __syncwarp();
+  for (int m = 0; m < 2; ++m)
+    for (int o0 = 0; o0 < A.h_rank / 8; o0 += 32) {
+      const int o = o0 + lane;
+      bool whole = o < A.h_rank / 8;
+      if (whole) {
+        const int16_t* p = pos_r + m * A.h_rank + 8 * o;
+        whole = p[0] >= 0 && (p[0] & 7) == 0;
+        for (int j = 1; j < 8; ++j) whole &= p[j] == p[0] + j;
+        if (whole) oct_r[m * (A.h_rank / 8) + o] = static_cast<int16_t>(p[0] >> 3);
+      }
+      const uint32_t broken = __ballot_sync(0xffffffffu, !whole && o < A.h_rank / 8);
+      if (lane == 0) item.broken[m][o0 >> 5] = broken;
+    }
+  for (int c = lane; c < item.fe.m[2].nslots >> 3; c += 32) {
+    const int16_t* r = item.rank_d + 8 * c;
+    bool whole = r[0] >= 0 && (r[0] & 7) == 0;
+    for (int j = 1; j < 8; ++j) whole &= r[j] == r[0] + j;
+    item.oct_d[c] = static_cast<int16_t>(whole ? r[0] : -1);
+  }
+  padded = __any_sync(0xffffffffu, padded);
+  live_d = __reduce_add_sync(0xffffffffu, live_d);
+  if (lane == 0) { item.padded = padded; item.all_ranks = live_d == A.rank_out; }
+  if (lane == 0) { item.n = n; item.chunk0 = chunk0; item.nchunk = nchunk; }
 }
 
-__global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(
-    const FastExpert* __restrict__ fast, const unsigned char* __restrict__ arena, const __half* __restrict__ h_gate,
-    const __half* __restrict__ h_up, int h_rank, const int32_t* __restrict__ token_indices,
-    const int32_t* __restrict__ expert_offsets, const float* __restrict__ route_w, int rank_out, int T, int num_experts,
-    int n_tiles, int max_slots, int max_words, int nt, int ring_h, int sec_n, int acc_stride,
-    float* __restrict__ rank_accum, long long* __restrict__ acc64, int* __restrict__ status) {
+// One converter stage's words and scales, on their way from L2.
+struct XtPre {
+  uint2 w[4];
+  uint4 s;
+};
+
+
+__global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_constant__ XtArgs A) {
   extern __shared__ unsigned char xt_raw[];
   __shared__ __align__(8) XtBars bars;
   __shared__ XtItem items[2];             // this item and the next one (looked up while this one runs)
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag_s;
   volatile int* abort_flag = &abort_flag_s;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::warp_index(), lane = threadIdx.x & 31;
+  const int nt = A.nt, ring_h = A.ring_h, h_rank = A.h_rank, num_experts = A.num_experts;
   const int cs = xt_chunk_stride(nt);     // bytes between 8-position chunks of act / z
+  const int n_chunks = A.n_tiles * (N_TILE / XT_CHUNK);
+  const uint32_t act_m_bytes = static_cast<uint32_t>(A.max_slots / 8) * cs, z_bytes = static_cast<uint32_t>(xt_z_bytes(nt));
   XtSmem sm;
   {
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(xt_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-    size_t o = 0;
-    sm.act = base; o += static_cast<size_t>(2) * (max_slots / 8) * cs;
-    sm.z = base + o; o += static_cast<size_t>(2) * (N_TILE / 8) * cs;
-    o = align_up_c(o, 128);
+    sm.act = base;
+    sm.z = base + xt_act_bytes(A.max_slots, nt);
+    size_t o = align_up_c(xt_act_bytes(A.max_slots, nt) + 2 * xt_z_bytes(nt), 128);
     sm.ring = base + o; o += static_cast<size_t>(2 * ring_h) * XT_STAGE_BYTES;
-    sm.sec0 = base + o; sm.sec_stride = static_cast<uint32_t>(xt_sec_bytes(max_slots, max_words)); o += static_cast<size_t>(sec_n) * sm.sec_stride;
     sm.prefix = reinterpret_cast<int*>(base + o); o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);
-    sm.dst_r = reinterpret_cast<int32_t*>(base + o);
-    sm.s_r = reinterpret_cast<__half*>(base + o + static_cast<size_t>(2) * h_rank * 4);
+    sm.s_r = reinterpret_cast<__half*>(base + o);
+    sm.pos_r = reinterpret_cast<int16_t*>(sm.s_r + 4 * h_rank);
+    sm.oct_r = sm.pos_r + 4 * h_rank;
   }
-  const size_t sec_scale_bytes = align_up_c(static_cast<size_t>(max_slots) * 2, 128);
   if (threadIdx.x == 0) {
-    for (int i = 0; i < XT_SEC_MAX; ++i) { tc::mbar_init(&bars.sec_full[i], 1); tc::mbar_init(&bars.sec_empty[i], XT_DQ_WARPS); }
-    for (int i = 0; i < XT_RING_MAX; ++i) { tc::mbar_init(&bars.w_full[i], XT_DQ_WARPS / 2); tc::mbar_init(&bars.w_empty[i], 1); }
+    for (int i = 0; i < 2 * XT_RING_MAX; ++i) { tc::mbar_init(&bars.w_full[i], 1); tc::mbar_init(&bars.w_empty[i], 1); }
     tc::mbar_init(&bars.act_ready, 1);
     tc::mbar_init(&bars.down_done, 2);
     for (int i = 0; i < 2; ++i) {
@@ -229,7 +342,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(
   // items before each expert (an item = up to nt consecutive assignments of one expert): every thread loads
   // its experts' counts in parallel, one warp then scans them
   for (int e = threadIdx.x; e < num_experts; e += XT_THREADS)
-    sm.prefix[e + 1] = (expert_offsets[e + 1] - expert_offsets[e] + nt - 1) / nt;
+    sm.prefix[e + 1] = (A.expert_offsets[e + 1] - A.expert_offsets[e] + nt - 1) / nt;
   __syncthreads();
   if (warp == 1) {
     int carry = 0;
@@ -250,437 +363,444 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
-  const int n_items = sm.prefix[num_experts];
-  // accumulators acc_stride columns apart: (gate, up) of buffer 0, of buffer 1, then the down product's row tiles
-  const uint32_t d_down = tmem_base + 4 * acc_stride;
-  const uint32_t z_bytes = static_cast<uint32_t>(N_TILE / 8) * cs;
-  if (warp == 0 && static_cast<int>(blockIdx.x) < n_items)
-    xt_load_item(items[0], blockIdx.x, sm.prefix, num_experts, nt, T, fast, token_indices, expert_offsets, route_w, lane);
+  const XtUnits units(sm.prefix[num_experts], static_cast<int>(gridDim.x), n_chunks);
+  // tensor memory: gu_bufs x (gate 64 columns, up 64 columns), then the down product's slot tiles of 128 columns
+  const uint32_t d_down = tmem_base + A.gu_bufs * 2 * XT_CHUNK;
+  if (warp == XT_LOOKUP_WARP && static_cast<int>(blockIdx.x) < units.n_units)
+    xt_load_item(items[0], sm, 0, blockIdx.x, units, n_chunks, A, lane);
 
-  // Positions in the cyclic buffers; every role steps through the same sequence of sections and stages, so each keeps
-  // its own copy across items.
-  XtCycle sec_c{0, 0};      // section slots (producer, converters)
+  // Positions in the cyclic buffers; every role steps through the same sequence of stages and chunks, so each keeps its
+  // own copy across items.
   XtCycle ring_c{0, 0};     // this pipeline's operand stages (converter team / its MMA issuer)
-  uint32_t gu_round = 0;    // tiles so far: tile number g uses accumulator / z buffer g & 1 for the (g >> 1)-th time
+  uint32_t gu_round = 0;    // chunks so far: chunk number g uses z buffer g & 1 for the (g >> 1)-th time
   uint32_t item_round = 0;
 
-  for (int it = blockIdx.x; it < n_items; it += gridDim.x, ++item_round) {
-    __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
-    const XtItem& item = items[item_round & 1];
+  // Activation operand of an item, once per item, by the epilogue and converter warps.
+  auto stage_item = [&](const XtItem& item) {
     const FastExpert& fe = item.fe;
     const int n_tok = item.n;
-    const int n_mma = max(16, (n_tok + 15) & ~15);        // N of this item's MMAs; rows n_tok .. n_mma - 1 are zero
-    const uint32_t idesc = tc::idesc_f16(128, n_mma);
-    const int nblk_d = fe.m[2].nslots >> 4;
-    const int n_mt = (nblk_d + 7) >> 3;   // 128-row tiles of the down product (<= 3)
-
-    // ---- activation operand, once per item, by the epilogue and converter warps
-    if (warp < XT_EPI_WARPS || warp >= XT_DQ_WARP0) {
-      constexpr int XT_STAGERS = (XT_EPI_WARPS + XT_DQ_WARPS) * 32;
-      const int tid_s = warp < XT_EPI_WARPS ? threadIdx.x : threadIdx.x - (XT_DQ_WARP0 - XT_EPI_WARPS) * 32;
-      const uint32_t act_m_bytes = static_cast<uint32_t>(max_slots / 8) * cs;
-      // act[m][chunk][n] = 8 consecutive contraction positions of token n: fp16(h[token, rank(slot)] * s(slot)).
-      // A warp takes a token; its lanes read consecutive ranks of the row (reading in slot order instead would touch
-      // every 32-byte sector of a row eight times) and store every value where its row slot sits in the operand.
-      // Consecutive ranks sit at mostly consecutive positions, so the lanes' 2-byte stores fall into distinct banks.
-      // Two tables per matrix, indexed by rank: where the value goes (or -1) and its factor.
-      const int warp_s = tid_s >> 5;
-      for (int i = tid_s; i < 2 * h_rank; i += XT_STAGERS) {
-        sm.dst_r[i] = -1;
-        sm.s_r[i] = __float2half(0.f);
-      }
-      // rows 0 .. n_mma - 1 of every chunk start as zero (padding slots, rows past the item's tokens)
-      {
-        const int nch0 = fe.m[0].nslots >> 3, nch_all = nch0 + (fe.m[1].nslots >> 3);
-        for (int c8 = warp_s; c8 < nch_all; c8 += XT_STAGERS / 32) {
-          unsigned char* chunk = sm.act + (c8 >= nch0 ? act_m_bytes + (c8 - nch0) * cs : c8 * cs);
-          for (int n = lane; n < n_mma; n += 32) *reinterpret_cast<uint4*>(chunk + n * 16) = make_uint4(0, 0, 0, 0);
-        }
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(XT_STAGERS) : "memory");
+    constexpr int XT_STAGERS = (XT_EPI_WARPS + XT_DQ_WARPS) * 32;
+    const int tid_s = threadIdx.x, warp_s = warp;
+    // act[m][chunk][n] = 8 consecutive contraction positions of token n: fp16(h[token, rank(slot)] * s(slot)).
+    // A warp takes tokens; a lane owns an octet of ranks, which the arena layout keeps together: one 16-byte load, four
+    // multiplications, one 16-byte store (pieces of one row are 16 bytes apart modulo 128: no bank conflicts).  Octets
+    // that straddle two groups of rows follow rank by rank.  Operand rows past the item's tokens keep whatever they
+    // hold: they only reach accumulator rows that nobody reads.
+    const int n_oct = h_rank >> 3;
+    const int16_t* pos_r = sm.pos_r + (item_round & 1) * 2 * h_rank;
+    const __half* s_r = sm.s_r + (item_round & 1) * 2 * h_rank;
+    const int16_t* oct_r = sm.oct_r + (item_round & 1) * 2 * n_oct;
+    for (int o0 = 0; o0 < n_oct; o0 += 32) {
+      const int o = o0 + lane;
+      int dst[2];
+      uint4 sc[2];
+#pragma unroll
       for (int m = 0; m < 2; ++m) {
-        const FastMat& fm = fe.m[m];
-        const int16_t* rank_t = reinterpret_cast<const int16_t*>(arena + fm.tab_off);
-        const __half* s_t = reinterpret_cast<const __half*>(arena + fm.tab_off + fm.nslots * 2);
-        for (int i = tid_s; i < fm.nslots; i += XT_STAGERS) {
-          const int rk = rank_t[i];
-          if (rk >= 0 && rk < h_rank) {
-            const int pos = slot_pos(i);
-            sm.dst_r[m * h_rank + rk] = (pos >> 3) * cs + (pos & 7) * 2;
-            sm.s_r[m * h_rank + rk] = s_t[i];
-          }
+        const int c = o < n_oct ? oct_r[m * n_oct + o] : -1;
+        dst[m] = c < 0 ? -1 : static_cast<int>(m * act_m_bytes) + c * cs;
+        sc[m] = c < 0 ? make_uint4(0u, 0u, 0u, 0u) : *reinterpret_cast<const uint4*>(s_r + m * h_rank + 8 * o);
+      }
+      for (int n0 = warp_s; n0 < n_tok; n0 += 4 * (XT_STAGERS / 32)) {
+        uint4 hv[4][2];                     // four tokens per round: eight loads in flight per lane
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int n = min(n0 + j * (XT_STAGERS / 32), n_tok - 1);
+          const int64_t row = static_cast<int64_t>(item.tok[n]) * h_rank + 8 * o;
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+            if (dst[m] >= 0) hv[j][m] = __ldg(reinterpret_cast<const uint4*>((m ? A.h_up : A.h_gate) + row));
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int n = n0 + j * (XT_STAGERS / 32);
+          if (n >= n_tok) break;
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+            if (dst[m] >= 0) {
+              uint4 r;
+              const __half2 *hp = reinterpret_cast<const __half2*>(&hv[j][m]), *sp = reinterpret_cast<const __half2*>(&sc[m]);
+              __half2* rp = reinterpret_cast<__half2*>(&r);
+#pragma unroll
+              for (int q = 0; q < 4; ++q) rp[q] = __hmul2(hp[q], sp[q]);       // one rounding of the exact product
+              *reinterpret_cast<uint4*>(sm.act + dst[m] + n * 16) = r;
+            }
         }
       }
-      asm volatile("bar.sync 1, %0;" ::"n"(XT_STAGERS) : "memory");
-      for (int m = 0; m < 2; ++m) {
-        const __half* h = m == 0 ? h_gate : h_up;
-        for (int r0 = 0; r0 < h_rank; r0 += 256) {        // lane l takes the ranks r0 + l + 32 k
-          int dst[8];
-          __half sc[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) {
-            const int r = r0 + lane + 32 * k;
-            dst[k] = r < h_rank ? sm.dst_r[m * h_rank + r] : -1;
-            sc[k] = r < h_rank ? sm.s_r[m * h_rank + r] : __float2half(0.f);
-          }
-          for (int n = warp_s; n < n_tok; n += 2 * (XT_STAGERS / 32)) {
-            // two tokens per round: sixteen loads in flight per lane
-            const int n2 = n + XT_STAGERS / 32;
-            const __half* row0 = h + static_cast<int64_t>(item.tok[n]) * h_rank + r0 + lane;
-            const __half* row1 = h + static_cast<int64_t>(item.tok[n2 < n_tok ? n2 : n]) * h_rank + r0 + lane;
-            __half hv0[8], hv1[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              hv0[k] = dst[k] >= 0 ? row0[32 * k] : __float2half(0.f);
-              hv1[k] = dst[k] >= 0 ? row1[32 * k] : __float2half(0.f);
-            }
-            unsigned char* out0 = sm.act + m * act_m_bytes + (n >> 3) * 128 + (n & 7) * 16;
-            unsigned char* out1 = sm.act + m * act_m_bytes + (n2 >> 3) * 128 + (n2 & 7) * 16;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-              if (dst[k] >= 0) {
-                *reinterpret_cast<__half*>(out0 + dst[k]) = __hmul(hv0[k], sc[k]);      // one rounding of the exact product
-                if (n2 < n_tok) *reinterpret_cast<__half*>(out1 + dst[k]) = __hmul(hv1[k], sc[k]);
-              }
-            }
-          }
-        }
-      }
-      tc::fence_async_smem();
-      asm volatile("bar.sync 1, %0;" ::"n"(XT_STAGERS) : "memory");
-      if (tid_s == 0) tc::mbar_arrive(&bars.act_ready);
-      // the next item's description, while this one runs
-      if (warp == 0 && it + static_cast<int>(gridDim.x) < n_items)
-        xt_load_item(items[(item_round + 1) & 1], it + gridDim.x, sm.prefix, num_experts, nt, T, fast, token_indices,
-                     expert_offsets, route_w, lane);
     }
-    if (warp == XT_PRODUCER_WARP) {
-      // ------------------------------------------------------------------ producer
-      if (lane == 0) {
-        for (int t = 0; t <= n_tiles && !*abort_flag; ++t) {
-          // sections in issue order: gate and up of tile t, then down of tile t - 1
-          for (int m = 0; m < 3; ++m) {
-            const int tile = m < 2 ? t : t - 1;
-            if (tile < 0 || tile >= n_tiles) continue;
-            const unsigned char* unit = arena + fe.unit_base + static_cast<int64_t>(tile) * fe.unit_bytes;
-            const uint32_t ss = sec_c.i;
-            if (!xt_wait(&bars.sec_empty[ss], sec_c.ph ^ 1, abort_flag)) break;
-            const uint32_t sb = static_cast<uint32_t>(fe.m[m].nslots) * 2u, wb = static_cast<uint32_t>(fe.m[m].words) * 4u;
-            tc::mbar_expect_tx(&bars.sec_full[ss], sb + wb);
-            tc::bulk_g2s(sm.sec0 + ss * sm.sec_stride, unit + fe.sec_off[m], sb, &bars.sec_full[ss]);
-            tc::bulk_g2s(sm.sec0 + ss * sm.sec_stride + sec_scale_bytes, unit + fe.sec_off[3 + m], wb, &bars.sec_full[ss]);
-            sec_c.next(sec_n);
+    for (int m = 0; m < 2; ++m)
+      for (int w = 0; w < (n_oct + 31) >> 5; ++w)
+        for (uint32_t left = item.broken[m][w]; left; left &= left - 1) {
+          const int o = 32 * w + __ffs(left) - 1;
+          for (int i = tid_s; i < 8 * n_tok; i += XT_STAGERS) {
+            const int n = i >> 3, rk = 8 * o + (i & 7), pos = pos_r[m * h_rank + rk];
+            if (pos >= 0)
+              *reinterpret_cast<__half*>(sm.act + m * act_m_bytes + (pos >> 3) * cs + (pos & 7) * 2 + n * 16) =
+                  __hmul((m ? A.h_up : A.h_gate)[static_cast<int64_t>(item.tok[n]) * h_rank + rk], s_r[m * h_rank + rk]);
           }
+        }
+    if (item.padded) {        // padding slots: their weights are zero, their activations have to be finite
+      for (int m = 0; m < 2; ++m) {
+        const int16_t* rank_t = reinterpret_cast<const int16_t*>(A.arena + fe.m[m].tab_off);
+        for (int i = warp_s; i < fe.m[m].nslots; i += XT_STAGERS / 32) {
+          const int rk = rank_t[i], pos = slot_pos(i);
+          if (rk >= 0 && rk < h_rank) continue;
+          for (int n = lane; n < n_tok; n += 32)
+            *reinterpret_cast<__half*>(sm.act + m * act_m_bytes + (pos >> 3) * cs + (pos & 7) * 2 + n * 16) = __float2half(0.f);
         }
       }
-    } else if (warp == XT_MMA_WARP0 || warp == XT_MMA_WARP0 + 1) {
-      // ------------------------------------------------------------------ MMA issue, one thread per pipeline
-      // pipeline 0: gate products and the down product's even row tiles; pipeline 1: up products and the odd row tiles
-      const int pl = warp - XT_MMA_WARP0;
-      // The whole warp waits (a lone waiting lane wakes up several times slower); lane 0 issues.
-      {
-        bool ok = xt_wait(&bars.act_ready, item_round & 1, abort_flag);
-        const uint32_t act_m_bytes = static_cast<uint32_t>(max_slots / 8) * cs;
-        // descriptors: constant upper part, start-address field advanced per block
-        const uint64_t a_desc0 = tc::smem_desc_kmajor(tc::smem_u32(sm.ring) + pl * ring_h * XT_STAGE_BYTES, XT_A_CHUNK, 128);
-        const uint64_t b_desc0 = tc::smem_desc_kmajor(tc::smem_u32(sm.act) + pl * act_m_bytes, cs, 128);
-        const uint64_t z_desc0 = tc::smem_desc_kmajor(tc::smem_u32(sm.z), cs, 128);
-        uint64_t* w_full = &bars.w_full[pl * ring_h];
-        uint64_t* w_empty = &bars.w_empty[pl * ring_h];
-        const int nkb = fe.m[pl].nslots >> 4;
-        for (int t = 0; t <= n_tiles && ok; ++t) {
-          if (t < n_tiles) {
-            const uint32_t g = gu_round + t, b = g & 1u, k = g >> 1;
-            if (g >= 2) ok = xt_wait(&bars.tmem_gu_free[b], (k - 1) & 1, abort_flag);   // buffer b read out two tiles ago
-            tc::fence_after_sync();
-            const uint32_t d_acc = tmem_base + (2 * b + pl) * acc_stride;
-            for (int kb0 = 0; kb0 < nkb && ok; kb0 += XT_STAGE_BLOCKS) {
-              if (!(ok = xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag))) break;
-              if (lane == 0) {
-                const int cnt = min(XT_STAGE_BLOCKS, nkb - kb0);
-                const uint64_t ad = a_desc0 + ((ring_c.i * XT_STAGE_BYTES) >> 4);
-                const uint64_t bd = b_desc0 + ((2 * kb0 * cs) >> 4);
-                for (int j = 0; j < cnt; ++j)
-                  tc::mma_f16(d_acc, ad + ((2 * j * XT_A_CHUNK) >> 4), bd + ((2 * j * cs) >> 4), idesc, (kb0 + j) > 0 ? 1u : 0u);
-                tc::mma_commit(&w_empty[ring_c.i]);
-              }
-              __syncwarp();
-              ring_c.next(ring_h);
-            }
-            if (!ok) break;
-            if (lane == 0) tc::mma_commit(&bars.gu_done[b]);
-            __syncwarp();
-          }
-          if (t > 0) {
-            const int tile = t - 1;
-            const uint32_t g = gu_round + tile, zb = g & 1u, k = g >> 1;
-            ok = xt_wait(&bars.z_ready[zb], k & 1, abort_flag);
-            tc::fence_after_sync();
-            const uint64_t zd = z_desc0 + ((zb * z_bytes) >> 4);
-            for (int mt = pl; mt < n_mt && ok; mt += 2) {
-              for (int kb0 = 0; kb0 < 8; kb0 += XT_STAGE_BLOCKS) {
-                if (!(ok = xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag))) break;
-                if (lane == 0) {
-                  const uint64_t ad = a_desc0 + ((ring_c.i * XT_STAGE_BYTES) >> 4);
-                  const uint64_t bd = zd + ((2 * kb0 * cs) >> 4);
-                  for (int j = 0; j < XT_STAGE_BLOCKS; ++j)
-                    tc::mma_f16(d_down + mt * acc_stride, ad + ((2 * j * XT_A_CHUNK) >> 4), bd + ((2 * j * cs) >> 4), idesc,
-                                (tile > 0 || kb0 + j > 0) ? 1u : 0u);
-                  tc::mma_commit(&w_empty[ring_c.i]);
-                }
-                __syncwarp();
-                ring_c.next(ring_h);
-              }
-            }
-            if (ok && lane == 0) {
-              tc::mma_commit(&bars.z_free[zb]);
-              if (t == n_tiles) tc::mma_commit(&bars.down_done);
-            }
-            __syncwarp();
-          }
-        }
-      }
-    } else if (warp >= XT_DQ_WARP0) {
-      // ------------------------------------------------------------------ converters
-      // Team 0 (four warps) feeds pipeline 0, team 1 pipeline 1; inside a team warp `wt` converts the operand-row
-      // blocks x = wt and wt + 4 of every stage (128 operand rows x 4 blocks of 16 contraction positions).
-      const int dw = warp - XT_DQ_WARP0;
-      const int team = dw >> 2, wt = dw & 3, g = lane >> 2, t = lane & 3;
-      unsigned char* ring = sm.ring + team * ring_h * XT_STAGE_BYTES;
-      uint64_t* w_full = &bars.w_full[team * ring_h];
-      uint64_t* w_empty = &bars.w_empty[team * ring_h];
-      bool ok = true;
-      for (int tl = 0; tl <= n_tiles && ok; ++tl) {
-        for (int m = 0; m < 2 && ok && tl < n_tiles; ++m) {
-          const uint32_t ss = sec_c.i;
-          // every converter warp waits for and releases every section, also the other team's: a slot's release
-          // counts all eight warps whatever the section holds
-          ok = xt_wait(&bars.sec_full[ss], sec_c.ph, abort_flag);
-          sec_c.next(sec_n);
-          if (!ok) break;
-          if (m == team) {
-            const FastMat& fm = fe.m[m];
-            const unsigned char* sec = sm.sec0 + ss * sm.sec_stride;
-            const uint32_t* words = reinterpret_cast<const uint32_t*>(sec + sec_scale_bytes);
-            const uint4* scale4 = reinterpret_cast<const uint4*>(sec);    // 8 halves per (pair, t)
-            const int npairs = fm.nslots >> 5, nib_pairs = fm.nblk[0] >> 1;
-            const uint32_t* dense_words = words + fm.nblk[0] * 256;
-            for (int p0 = 0; p0 < npairs; p0 += 2) {
-              if (!(ok = xt_wait(&w_empty[ring_c.i], ring_c.ph ^ 1, abort_flag))) break;
-              unsigned char* stage = ring + ring_c.i * XT_STAGE_BYTES;
-#pragma unroll
-              for (int pp = 0; pp < 2; ++pp) {
-                const int pr = p0 + pp;
-                if (pr >= npairs) break;
-                const uint4 sv = scale4[pr * 4 + t];
-                const __half2 sc[4] = {*reinterpret_cast<const __half2*>(&sv.x), *reinterpret_cast<const __half2*>(&sv.y),
-                                       *reinterpret_cast<const __half2*>(&sv.z), *reinterpret_cast<const __half2*>(&sv.w)};
-                unsigned char* dst = stage + (pp * 4 + t) * XT_A_CHUNK + g * 16;
-                if (pr < nib_pairs) {
-                  const uint2 w0 = reinterpret_cast<const uint2*>(words)[(pr * 8 + wt) * 32 + lane];
-                  const uint2 w1 = reinterpret_cast<const uint2*>(words)[(pr * 8 + wt + 4) * 32 + lane];
-                  dequant_pair_store<false>(w0.x, w0.y, sc, sc, dst + wt * 256);
-                  dequant_pair_store<false>(w1.x, w1.y, sc, sc, dst + (wt + 4) * 256);
-                } else {
-                  const int dp = pr - nib_pairs;
-                  const uint32_t w0 = dense_words[(dp * 8 + wt) * 32 + lane];
-                  const uint32_t w1 = dense_words[(dp * 8 + wt + 4) * 32 + lane];
-                  dequant_pair_store<true>(w0, w0 >> 8, sc, sc, dst + wt * 256);
-                  dequant_pair_store<true>(w1, w1 >> 8, sc, sc, dst + (wt + 4) * 256);
-                }
-              }
-              tc::fence_async_smem();
-              __syncwarp();
-              if (lane == 0) tc::mbar_arrive(&w_full[ring_c.i]);
-              ring_c.next(ring_h);
-            }
-          }
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(&bars.sec_empty[ss]);
-        }
-        if (!ok) break;
-        if (tl == 0) continue;                      // the down product runs one tile behind
-        const uint32_t sd = sec_c.i;
-        ok = xt_wait(&bars.sec_full[sd], sec_c.ph, abort_flag);
-        sec_c.next(sec_n);
-        if (!ok) break;
-        const FastMat& fd = fe.m[2];
-        const unsigned char* sec = sm.sec0 + sd * sm.sec_stride;
-        const uint32_t* dwords = reinterpret_cast<const uint32_t*>(sec + sec_scale_bytes);
-        const uint32_t* ddense = dwords + fd.nblk[0] * 256;
-        const __half* scale_d = reinterpret_cast<const __half*>(sec);
-        for (int mt = team; mt < n_mt && ok; mt += 2) {
-          // this thread's two operand-row blocks: slot blocks 8*mt + wt and 8*mt + wt + 4
-          __half2 sg[2], sh[2];
-          int mbu[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            mbu[u] = 8 * mt + wt + 4 * u;
-            sg[u] = sh[u] = __float2half2_rn(0.f);
-            if (mbu[u] < nblk_d) {
-              sg[u] = __half2half2(scale_d[16 * mbu[u] + g]);
-              sh[u] = __half2half2(scale_d[16 * mbu[u] + g + 8]);
-            }
-          }
-          for (int p0 = 0; p0 < 4; p0 += 2) {
-            if (!(ok = xt_wait(&w_empty[ring_c.i], ring_c.ph ^ 1, abort_flag))) break;
-            unsigned char* stage = ring + ring_c.i * XT_STAGE_BYTES;
-#pragma unroll
-            for (int pp = 0; pp < 2; ++pp) {
-              const int pr = p0 + pp;
-#pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                unsigned char* dst = stage + (pp * 4 + t) * XT_A_CHUNK + g * 16 + (wt + 4 * u) * 256;
-                const __half2 sa[4] = {sg[u], sg[u], sg[u], sg[u]};
-                const __half2 sb[4] = {sh[u], sh[u], sh[u], sh[u]};
-                const int mb = mbu[u];
-                if (mb >= nblk_d) {
-                  *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
-                  *reinterpret_cast<uint4*>(dst + 128) = make_uint4(0, 0, 0, 0);
-                } else if (mb < fd.nblk[0]) {
-                  const uint2 w = reinterpret_cast<const uint2*>(dwords)[(mb * 4 + pr) * 32 + lane];
-                  dequant_pair_store<false>(w.x, w.y, sa, sb, dst);
-                } else {
-                  const uint32_t w = ddense[((mb - fd.nblk[0]) * 4 + pr) * 32 + lane];
-                  dequant_pair_store<true>(w, w >> 8, sa, sb, dst);
-                }
-              }
-            }
-            tc::fence_async_smem();
-            __syncwarp();
-            if (lane == 0) tc::mbar_arrive(&w_full[ring_c.i]);
-            ring_c.next(ring_h);
-          }
-        }
-        __syncwarp();
-        if (ok && lane == 0) tc::mbar_arrive(&bars.sec_empty[sd]);
-      }
-    } else {
+    }
+    tc::fence_async_smem();
+    asm volatile("bar.sync 1, %0;" ::"n"(XT_STAGERS) : "memory");
+    if (tid_s == 0) tc::mbar_arrive(&bars.act_ready);
+  };
+
+  if (warp < XT_EPI_WARPS) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XT_REGS_EPI));
+    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++item_round) {
+      __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
+      const XtItem& item = items[item_round & 1];
+      const FastExpert& fe = item.fe;
+      const int n_tok = item.n, nchunk = item.nchunk;
+      stage_item(item);
       // ------------------------------------------------------------------ epilogue warps 0-7
-      // warp = (TMEM lane quarter q, parity of the 32-token column chunks it takes)
-      const int q = warp & 3, n_first = (warp >> 2) * 32;
+      // warp = (TMEM lane quarter q: tokens 32 q .. 32 q + 31, half of the chunk's 64 columns); a thread owns a token
+      const int q = warp & 3, half = warp >> 2;
       const uint32_t lane_sel = static_cast<uint32_t>(32 * q) << 16;
+      const int n = 32 * q + lane;
+      const bool busy = 32 * q < n_tok;                               // any token in this quarter
+      unsigned char* zrow = sm.z + (4 * half) * cs + n * 16;
       bool ok = true;
-      const int c = 32 * q + lane;                                   // row of D_g / D_u = column of the tile
-      const int c_pos = slot_pos(c);
-      unsigned char* zrow = sm.z + (c_pos >> 3) * cs + (c_pos & 7) * 2;
-      for (int tile = 0; tile < n_tiles && ok; ++tile) {
-        const uint32_t gt = gu_round + tile, b = gt & 1u, k = gt >> 1;
+      for (int t = 0; t < nchunk && ok; ++t) {
+        const uint32_t gt = gu_round + t, zb = gt & 1u;
+        const uint32_t b = A.gu_bufs == 2 ? zb : 0u, k = A.gu_bufs == 2 ? gt >> 1 : gt;
         ok = xt_wait(&bars.gu_done[b], k & 1, abort_flag);
-        if (ok && gt >= 2) ok = xt_wait(&bars.z_free[b], (k - 1) & 1, abort_flag);     // z buffer b consumed two tiles ago
+        if (ok && gt >= 2) ok = xt_wait(&bars.z_free[zb], ((gt >> 1) - 1) & 1, abort_flag);     // z buffer consumed two chunks ago
         if (!ok) break;
         tc::fence_after_sync();
-        const uint32_t d_gate = tmem_base + 2 * b * acc_stride, d_up = d_gate + acc_stride;
-        unsigned char* zr = zrow + b * z_bytes;
-        for (int n0 = n_first; n0 < n_mma; n0 += 64) {
-          // 16 columns at a time: two 32-column loads would hold 64 registers per thread
+        if (busy) {
+          const uint32_t d_gate = tmem_base + 2 * b * XT_CHUNK + lane_sel + 32 * half, d_up = d_gate + XT_CHUNK;
+          uint32_t zp[2][8];
 #pragma unroll
-          for (int hh = 0; hh < 2; ++hh) {
-            const int nb = n0 + 16 * hh;
-            if (nb >= n_mma) break;
+          for (int hh = 0; hh < 2; ++hh) {          // 16 columns at a time: 32 of both would hold 64 registers
             float gv[16], uv[16];
-            tc::tmem_ld16(d_gate + lane_sel + nb, gv);
-            tc::tmem_ld16(d_up + lane_sel + nb, uv);
+            tc::tmem_ld16(d_gate + 16 * hh, gv);
+            tc::tmem_ld16(d_up + 16 * hh, uv);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const int n = nb + i;
-              const float zf = __fdividef(gv[i] * uv[i], 1.f + __expf(-gv[i]));
-              *reinterpret_cast<__half*>(zr + (n >> 3) * 128 + (n & 7) * 16) = __float2half_rn(n < n_tok ? zf : 0.f);
+            for (int i = 0; i < 8; ++i) {
+              const float z0 = __fdividef(gv[2 * i] * uv[2 * i], 1.f + __expf(-gv[2 * i]));
+              const float z1 = __fdividef(gv[2 * i + 1] * uv[2 * i + 1], 1.f + __expf(-gv[2 * i + 1]));
+              const __half2 h2 = __floats2half2_rn(z0, z1);
+              zp[hh][i] = *reinterpret_cast<const uint32_t*>(&h2);
             }
+          }
+          // chunk c of the contraction order (pos32): columns 2c, 2c+1, 2c+8, 2c+9 of both blocks of 16
+          if (n < nt) {
+            unsigned char* zr = zrow + zb * z_bytes;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(zr + c * cs) = make_uint4(zp[0][c], zp[0][c + 4], zp[1][c], zp[1][c + 4]);
           }
         }
         tc::fence_before_sync();
         tc::fence_async_smem();
         __syncwarp();
-        if (lane == 0) { tc::mbar_arrive(&bars.tmem_gu_free[b]); tc::mbar_arrive(&bars.z_ready[b]); }
+        if (lane == 0) { tc::mbar_arrive(&bars.tmem_gu_free[b]); tc::mbar_arrive(&bars.z_ready[zb]); }
       }
       if (ok) ok = xt_wait(&bars.down_done, item_round & 1, abort_flag);
-      if (ok) {
+      if (busy) {                      // both warps of the quarter go on or neither: they meet at barriers below
+        uint32_t both;
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.and.aligned.pred q, %2, 64, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                     : "=r"(both)
+                     : "r"(static_cast<uint32_t>(ok)), "r"(2 + q)
+                     : "memory");
+        ok = both != 0;
+      }
+      if (ok && busy) {
         tc::fence_after_sync();
-        const FastMat& fd = fe.m[2];
-        const int16_t* rank_d = reinterpret_cast<const int16_t*>(arena + fd.tab_off);
-        const __half* s_d = reinterpret_cast<const __half*>(arena + fd.tab_off + fd.nslots * 2);
-        // A thread owns a row slot, and the slots of a warp map to scattered ranks: adding straight from the registers
-        // costs one 32-byte sector per lane and instruction.  With room for it (the operand ring is idle by now) the
-        // four warps that share a 32-token chunk transpose it through shared memory and add whole rows, 16 bytes per
-        // lane; ranks without a slot add zero.
-        const int grp = warp >> 2;
-        const bool transpose = acc64 == nullptr && (rank_out & 3) == 0 &&
-                               static_cast<size_t>(2) * 32 * rank_out * 4 <= static_cast<size_t>(2 * ring_h) * XT_STAGE_BYTES;
-        float* tbuf = reinterpret_cast<float*>(sm.ring) + grp * 32 * rank_out;
-        for (int n0 = n_first; n0 < n_mma; n0 += 64) {
-          if (transpose) {
-            for (int i = (warp & 3) * 32 + lane; i < 8 * rank_out; i += 128) reinterpret_cast<float4*>(tbuf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
+        const int rank_out = A.rank_out;
+        const float rw = n < n_tok ? item.rw[n] : 0.f;
+        // A thread owns a token: adding straight from the registers costs a 32-byte sector per lane and instruction.  The
+        // quarter's two warps turn their 32 tokens x rank_out sums through the idle activation area, 16 bytes at a time
+        // where eight slots hold an aligned octet of ranks (piece index XORed with the token: conflict-free both ways),
+        // and add whole rows, 16 bytes per lane; ranks without a slot add zero.
+        const bool turn = A.acc64 == nullptr && (rank_out & 31) == 0 &&
+                          static_cast<size_t>(4) * 32 * rank_out * 4 <= xt_act_bytes(A.max_slots, nt) + 2 * xt_z_bytes(nt);
+        float* tbuf = reinterpret_cast<float*>(sm.act) + q * 32 * rank_out;
+        float* trow = tbuf + lane * rank_out;
+        const int x7 = lane & 7;
+        if (turn && !item.all_ranks) {
+          for (int i = half * 32 + lane; i < 8 * rank_out; i += 64) reinterpret_cast<float4*>(tbuf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+          asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
+        }
+        const int nslots_d = fe.m[2].nslots;
+        for (int s0 = 16 * half; s0 < nslots_d; s0 += 32) {
+          float v[16];
+          tc::tmem_ld16(d_down + lane_sel + s0, v);
+#pragma unroll
+          for (int i = 0; i < 16; i += 4) {
+            const float4 sv = *reinterpret_cast<const float4*>(item.s_d + s0 + i);
+            v[i] *= sv.x * rw; v[i + 1] *= sv.y * rw; v[i + 2] *= sv.z * rw; v[i + 3] *= sv.w * rw;
           }
-          for (int mt = 0; mt < n_mt; ++mt) {
-            const int slot = 128 * mt + 32 * q + lane;
-            int rk = -1;
-            float sv = 0.f;
-            if (slot < fd.nslots) { rk = rank_d[slot]; sv = __half2float(s_d[slot]); }
-            const bool live = rk >= 0 && rk < rank_out;
 #pragma unroll
-            for (int hh = 0; hh < 2; ++hh) {
-              const int nb = n0 + 16 * hh;
-              if (nb >= n_mma) break;
-              float v[16];
-              tc::tmem_ld16(d_down + mt * acc_stride + lane_sel + nb, v);
-              if (live) {
+          for (int h8 = 0; h8 < 2; ++h8) {
+            const int r0 = item.oct_d[(s0 >> 3) + h8];
+            const float* w = v + 8 * h8;
+            if (turn && r0 >= 0) {
+              *reinterpret_cast<float4*>(trow + 4 * ((r0 >> 2) ^ x7)) = make_float4(w[0], w[1], w[2], w[3]);
+              *reinterpret_cast<float4*>(trow + 4 * (((r0 >> 2) + 1) ^ x7)) = make_float4(w[4], w[5], w[6], w[7]);
+            } else {
 #pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                  const int n = nb + i;
-                  if (n < n_tok) {
-                    const float val = v[i] * sv * item.rw[n];
-                    if (transpose) tbuf[(16 * hh + i) * rank_out + rk] = val;
-                    else acc_add(rank_accum, acc64, static_cast<int64_t>(item.tok[n]) * rank_out + rk, val);
-                  }
-                }
+              for (int i = 0; i < 8; ++i) {
+                const int r = item.rank_d[s0 + 8 * h8 + i];
+                if (r < 0) continue;
+                if (turn) trow[4 * ((r >> 2) ^ x7) + (r & 3)] = w[i];
+                else if (n < n_tok) acc_add(A.rank_accum, A.acc64, static_cast<int64_t>(item.tok[n]) * rank_out + r, w[i]);
               }
             }
           }
-          if (transpose) {
-            asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
-            for (int i = q; i < 32 && n0 + i < n_tok; i += 4) {
-              float* dst = rank_accum + static_cast<int64_t>(item.tok[n0 + i]) * rank_out;
-              for (int c0 = lane * 4; c0 < rank_out; c0 += 128) {
-                const float4 x = *reinterpret_cast<const float4*>(tbuf + i * rank_out + c0);
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + c0), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
-              }
+        }
+        if (turn) {
+          asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
+          for (int i = half; i < 32 && 32 * q + i < n_tok; i += 2) {
+            float* dst = A.rank_accum + static_cast<int64_t>(item.tok[32 * q + i]) * rank_out;
+            const float* row = tbuf + i * rank_out;
+            for (int c = lane; c < rank_out >> 2; c += 32) {
+              const float4 x = *reinterpret_cast<const float4*>(row + 4 * (c ^ (i & 7)));
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * c), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
             }
-            if (n0 + 64 < n_mma) asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
           }
         }
         tc::fence_before_sync();
       }
+      gu_round += nchunk;
     }
-    gu_round += n_tiles;
+    // every role ends on its own (they do not share a register count to come together with)
+    tc::fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
+    if (threadIdx.x == 0 && abort_flag_s) atomicExch(A.status, BM_ERR_TIMEOUT);
+    return;
   }
-  tc::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
-  if (threadIdx.x == 0 && abort_flag_s) atomicExch(status, BM_ERR_TIMEOUT);
+  if (warp < XT_DQ_WARP0 + XT_DQ_WARPS) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(XT_REGS_DQ));
+    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++item_round) {
+      __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
+      const XtItem& item = items[item_round & 1];
+      const FastExpert& fe = item.fe;
+      const int chunk0 = item.chunk0, nchunk = item.nchunk;
+      const int nblk_d = fe.m[2].nslots >> 4;
+      const int n_mt = (nblk_d + 7) >> 3;   // 128-slot tiles of the down product (<= 3)
+      stage_item(item);
+      // ------------------------------------------------------------------ converters
+      // Team 0 (four warps) feeds pipeline 0, team 1 pipeline 1; a team's warps take its stages in turn.  Step t of an item:
+      // a stage per 32 slots of chunk t's gate (up) product, then four stages (64 slots x 32 columns) per 128-slot tile
+      // of chunk t - 1's down product.  A stage is four 16 x 32 blocks; lane (g, t4) turns its words of each into two
+      // 16-byte pieces.  What bounds a warp is latency, not issue: a whole stage per warp gives it four independent
+      // blocks, one barrier wait, one proxy fence and one arrival per 2048 codes, and the next stage's words are on their
+      // way from L2 in a second register set meanwhile.
+      const int dw = warp - XT_DQ_WARP0;
+      const int team = dw >> 2, g = lane >> 2, t4 = lane & 3;
+      unsigned char* ring = sm.ring + team * ring_h * XT_STAGE_BYTES + t4 * XT_W_STRIDE + g * 16;
+      uint64_t* w_full = &bars.w_full[team * ring_h];
+      uint64_t* w_empty = &bars.w_empty[team * ring_h];
+      // everything about the expert in registers: the barriers' memory clobbers would have it read again every stage
+      const int npairs = fe.m[team].nslots >> 5, nib_pairs = fe.m[team].nblk[0] >> 1, nib_d = fe.m[2].nblk[0];
+      const int n_d = team < n_mt ? 4 * ((n_mt - team + 1) >> 1) : 0;
+      const int unit_bytes = fe.unit_bytes;
+      const unsigned char* unit0 = A.arena + fe.unit_base;
+      const unsigned char* scale_gu = unit0 + fe.sec_off[team] + t4 * 16;
+      const unsigned char* words_gu = unit0 + fe.sec_off[3 + team];
+      const unsigned char* scale_d = unit0 + fe.sec_off[2] + g * 4;
+      const unsigned char* words_d = unit0 + fe.sec_off[5];
+      auto fetch = [&](int t, int i, XtPre& p) {
+        if (t < nchunk && i < npairs) {
+          const int ch = chunk0 + t;
+          const int64_t tile = static_cast<int64_t>(ch >> 1) * unit_bytes;
+          p.s = __ldg(reinterpret_cast<const uint4*>(scale_gu + tile + i * 64));
+          if (i < nib_pairs) {              // columns 0-63 or 64-127 of the tile: blocks 0-3 or 4-7
+            const uint2* w = reinterpret_cast<const uint2*>(words_gu + tile + i * 2048 + (ch & 1) * 1024) + lane;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) p.w[x] = __ldg(w + x * 32);
+          } else {
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(words_gu + tile + nib_pairs * 2048 + (i - nib_pairs) * 1024 + (ch & 1) * 512) + lane;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) p.w[x].x = __ldg(w + x * 32);
+          }
+        } else {
+          const int j = t < nchunk ? i - npairs : i, ch = chunk0 + t - 1;
+          const int64_t tile = static_cast<int64_t>(ch >> 1) * unit_bytes;
+          const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * ((j >> 1) & 1), pr = 2 * (ch & 1) + (j & 1);
+          uint32_t* ps = reinterpret_cast<uint32_t*>(&p.s);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            const int mb = mb0 + v;
+            if (mb >= nblk_d) break;
+            ps[v] = __ldg(reinterpret_cast<const uint32_t*>(scale_d + tile + mb * 32));
+            if (mb < nib_d) p.w[v] = __ldg(reinterpret_cast<const uint2*>(words_d + tile + (mb * 4 + pr) * 256) + lane);
+            else p.w[v].x = __ldg(reinterpret_cast<const uint32_t*>(words_d + tile + nib_d * 1024 + ((mb - nib_d) * 4 + pr) * 128) + lane);
+          }
+        }
+      };
+      XtCycle my_c = ring_c;
+      my_c.advance(dw & 3, ring_h);
+      auto convert = [&](int t, int i, const XtPre& p) -> bool {
+        if (!xt_wait(&w_empty[my_c.i], my_c.ph ^ 1, abort_flag)) return false;
+        unsigned char* dst = ring + my_c.i * XT_STAGE_BYTES;
+        if (t < nchunk && i < npairs) {
+          const __half2* sp = reinterpret_cast<const __half2*>(&p.s);
+          const __half2 sc[4] = {sp[0], sp[1], sp[2], sp[3]};
+          if (i < nib_pairs) {
+#pragma unroll
+            for (int x = 0; x < 4; ++x) dequant_pair_store<false>(p.w[x].x, p.w[x].y, sc, sc, dst + x * 256);
+          } else {
+#pragma unroll
+            for (int x = 0; x < 4; ++x) dequant_pair_store<true>(p.w[x].x, p.w[x].x >> 8, sc, sc, dst + x * 256);
+          }
+        } else {
+          const int j = t < nchunk ? i - npairs : i;
+          const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * ((j >> 1) & 1);
+          const __half2* sp = reinterpret_cast<const __half2*>(&p.s);
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            if (mb0 + v >= nblk_d) break;             // slots past the matrix: accumulator columns that nobody reads
+            const __half2 lo = __low2half2(sp[v]), hi = __high2half2(sp[v]);
+            const __half2 sa[4] = {lo, lo, lo, lo}, sb[4] = {hi, hi, hi, hi};
+            if (mb0 + v < nib_d) dequant_pair_store<false>(p.w[v].x, p.w[v].y, sa, sb, dst + v * 256);
+            else dequant_pair_store<true>(p.w[v].x, p.w[v].x >> 8, sa, sb, dst + v * 256);
+          }
+        }
+        tc::fence_async_smem();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&w_full[my_c.i]);
+        my_c.i += 4;                         // ring_h >= 4: at most one wrap
+        if (my_c.i >= static_cast<uint32_t>(ring_h)) { my_c.i -= ring_h; my_c.ph ^= 1u; }
+        return true;
+      };
+      // this warp's stage after (t, i); false past its last one
+      auto step = [&](int& t, int& i) -> bool {
+        i += 4;
+        for (int n = (t < nchunk ? npairs : 0) + (t > 0 ? n_d : 0); t <= nchunk && i >= n; n = (t < nchunk ? npairs : 0) + n_d) {
+          i -= n;
+          ++t;
+        }
+        return t <= nchunk;
+      };
+      XtPre p0, p1;
+      int t0 = 0, i0 = (dw & 3) - 4, t1, i1;
+      bool more = step(t0, i0);
+      if (more) fetch(t0, i0, p0);
+      t1 = t0; i1 = i0;
+      while (more) {
+        const bool more1 = step(t1, i1);
+        if (more1) fetch(t1, i1, p1);
+        if (!convert(t0, i0, p0) || !more1) break;
+        t0 = t1; i0 = i1;
+        more = step(t0, i0);
+        if (more) fetch(t0, i0, p0);
+        if (!convert(t1, i1, p1)) break;
+        t1 = t0; i1 = i0;
+      }
+      ring_c.advance(nchunk * (npairs + n_d), ring_h);
+    }
+    __syncthreads();
+    return;
+  }
+  {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XT_REGS_MISC));
+    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++item_round) {
+      __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
+      const XtItem& item = items[item_round & 1];
+      const FastExpert& fe = item.fe;
+      const int nchunk = item.nchunk;
+      const int nblk_d = fe.m[2].nslots >> 4;
+      const int n_mt = (nblk_d + 7) >> 3;   // 128-slot tiles of the down product (<= 3)
+      if (warp == XT_LOOKUP_WARP) {
+        // ------------------------------------------------------------------ the next item, while this one runs
+        if (u + static_cast<int>(gridDim.x) < units.n_units) {
+          XtItem& nx = items[(item_round + 1) & 1];
+          xt_load_item(nx, sm, (item_round + 1) & 1, u + gridDim.x, units, n_chunks, A, lane);
+          __syncwarp();
+          // its weights on their way to L2, one tile per lane (sizes and offsets are multiples of 16 bytes)
+          const int t0 = nx.chunk0 >> 1, t1 = (nx.chunk0 + nx.nchunk + 1) >> 1;
+          for (int t = t0 + lane; t < t1; t += 32)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A.arena + nx.fe.unit_base + static_cast<int64_t>(t) * nx.fe.unit_bytes),
+                         "r"(nx.fe.unit_bytes)
+                         : "memory");
+        }
+      } else if (warp < XT_MMA_WARP0 + 2) {
+        // ------------------------------------------------------------------ MMA issue, one thread per pipeline
+        // The whole warp waits (a lone waiting lane wakes up several times slower); one issues.
+        const int pl = warp - XT_MMA_WARP0;
+        const uint32_t idesc = tc::idesc_f16(128, 64);
+        bool ok = xt_wait(&bars.act_ready, item_round & 1, abort_flag);
+        tc::fence_after_sync();
+        // descriptors: constant upper part, start-address field advanced per block
+        const uint64_t a_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.act) + pl * act_m_bytes, cs, 128);
+        const uint64_t z_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.z), cs, 128);
+        const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring_h * XT_STAGE_BYTES;
+        const uint64_t b_desc = tc::smem_desc_kmajor(ring0, XT_W_STRIDE, 128);
+        uint64_t* w_full = &bars.w_full[pl * ring_h];
+        uint64_t* w_empty = &bars.w_empty[pl * ring_h];
+        const int npairs = fe.m[pl].nslots >> 5;
+        // two MMAs of 64 columns on the next stage: A operand at ad, accumulator d, first MMA overwriting or adding
+        auto stage_mmas = [&](uint32_t d, uint64_t ad, uint32_t accumulate) -> bool {
+          if (!xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag)) return false;
+          if (tc::elect_one()) {
+            const uint64_t bd = b_desc + ((ring_c.i * XT_STAGE_BYTES) >> 4);
+            tc::mma_f16(d, ad, bd, idesc, accumulate);
+            tc::mma_f16(d, ad + ((2 * cs) >> 4), bd + ((2 * XT_W_STRIDE) >> 4), idesc, 1u);
+            tc::mma_commit(&w_empty[ring_c.i]);
+          }
+          __syncwarp();
+          ring_c.next(ring_h);
+          return true;
+        };
+        for (int t = 0; t <= nchunk && ok; ++t) {
+          if (t < nchunk) {
+            const uint32_t g = gu_round + t, b = A.gu_bufs == 2 ? g & 1u : 0u, k = A.gu_bufs == 2 ? g >> 1 : g;
+            if (k >= 1) ok = xt_wait(&bars.tmem_gu_free[b], (k - 1) & 1, abort_flag);   // this accumulator's last contents are read out
+            tc::fence_after_sync();
+            const uint32_t d_acc = tmem_base + (2 * b + pl) * XT_CHUNK;
+            for (int pr = 0; pr < npairs && ok; ++pr) ok = stage_mmas(d_acc, a_desc + ((4 * pr * cs) >> 4), pr > 0 ? 1u : 0u);
+            if (!ok) break;
+            if (tc::elect_one()) tc::mma_commit(&bars.gu_done[b]);
+            __syncwarp();
+          }
+          if (t > 0) {
+            const uint32_t g = gu_round + t - 1, zb = g & 1u;
+            ok = xt_wait(&bars.z_ready[zb], (g >> 1) & 1, abort_flag);
+            tc::fence_after_sync();
+            const uint64_t zd = z_desc + ((zb * z_bytes) >> 4);
+            for (int mt = pl; mt < n_mt && ok; mt += 2)
+              for (int q = 0; q < 4 && ok; ++q)               // 64 slots and 32 columns of z per stage
+                ok = stage_mmas(d_down + mt * 128 + (q >> 1) * 64, zd + ((4 * (q & 1) * cs) >> 4), (t > 1 || (q & 1)) ? 1u : 0u);
+            if (ok && tc::elect_one()) {
+              tc::mma_commit(&bars.z_free[zb]);
+              if (t == nchunk) tc::mma_commit(&bars.down_done);
+            }
+            __syncwarp();
+          }
+        }
+      }
+      gu_round += nchunk;
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+  }
 }
 
-// Item size and pipeline depths for a layer: the first candidate that fits.  Larger items convert every code for more
-// tokens at once, but the item's activation operand (1 KB per token at 256 row slots) and the two z tiles compete with
-// the copy and conversion stages for shared memory, and tensor memory has to hold two (gate, up) accumulator pairs
-// plus the down product's two or three row tiles of nt columns each.
-struct XtPlan { int nt, ring_h, sec_n, acc_stride; size_t smem; };
-constexpr size_t XT_SMEM_LIMIT = 227 * 1024 - 4096;     // dynamic part: the kernel's static shared memory (two item descriptions, barriers) stays below 4 KB
+// Item size and ring depth for a layer: the first candidate whose activation operand (2 KB per token at 256 row slots per
+// matrix), z buffers and stages fit shared memory.  Tensor memory holds 128 columns per gate/up buffer and 128 per 128
+// slots of the down product.
+struct XtPlan { int nt, ring_h, gu_bufs; size_t smem; };
+constexpr size_t XT_SMEM_LIMIT = 227 * 1024 - 8192;     // dynamic part: the static part (two item descriptions, barriers) stays below 8 KB
 static bool xt_plan(const bm_layer* L, XtPlan* out) {
   if (L->num_experts > XT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > 3 * 128) return false;
   const int n_mt = (L->max_slots + 127) / 128;
-  // {tokens per item, operand stages per pipeline, section slots}
-  static const int cand[][3] = {{64, 2, 4}, {64, 2, 3}, {64, 2, 2}, {48, 2, 3}, {48, 2, 2}, {32, 2, 3}, {32, 2, 2}, {16, 2, 2}};
+  static const int cand[][2] = {{128, 6}, {128, 4}, {112, 6}, {112, 4}, {96, 6}, {96, 4}, {80, 6}, {80, 4}, {64, 6}, {64, 4}, {48, 4}, {32, 4}, {16, 4}};
   for (const auto& c : cand) {
-    const int nt = c[0], ring_h = c[1], sec_n = c[2];
-    const bool shape_ok = nt % 16 == 0 && nt >= 16 && nt <= XT_NT_MAX && ring_h >= 1 && 2 * ring_h <= XT_RING_MAX && sec_n >= 2 &&
-                          sec_n <= XT_SEC_MAX;
-    // the epilogue reads accumulators in 32-column pieces, so the last one may be read up to the next multiple of 32
-    const bool tmem_ok = (3 + n_mt) * nt + (nt + 31) / 32 * 32 <= 512;
-    const size_t smem = xt_smem_bytes(L->max_slots, L->max_words, L->num_experts, L->rank_in, nt, 2 * ring_h, sec_n);
-    if (shape_ok && tmem_ok && smem <= XT_SMEM_LIMIT) {
-      *out = XtPlan{nt, ring_h, sec_n, nt, smem};
+    const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, L->rank_in, c[0], c[1]);
+    if (smem <= XT_SMEM_LIMIT) {
+      *out = XtPlan{c[0], c[1], n_mt > 2 ? 1 : 2, smem};
       return true;
     }
   }
@@ -704,7 +824,6 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
              BM_ERR_UNSUPPORTED, "experts_tc: rank-space rows must be 16-byte aligned (rank %d)", L->rank_in);
   XtPlan plan;
   BM_REQUIRE(xt_plan(L, &plan), BM_ERR_UNSUPPORTED, "experts_tc: the layer's largest expert does not fit in shared memory");
-  const size_t smem = plan.smem;
   static PerDeviceOnce attr_once;
   static int sm_counts[MAX_DEVICES];
   int dev = -1;
@@ -713,13 +832,20 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
   if (!attr_once.is_done(dev)) {
     BM_CUDA(cudaFuncSetAttribute(experts_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(XT_SMEM_LIMIT)));
     BM_CUDA(cudaDeviceGetAttribute(&sm_counts[dev], cudaDevAttrMultiProcessorCount, dev));
+    cudaFuncAttributes fa;
+    BM_CUDA(cudaFuncGetAttributes(&fa, experts_tc_kernel));
+    BM_REQUIRE(fa.numRegs >= XT_REGS, BM_ERR_UNSUPPORTED, "experts_tc: built with %d registers per thread, %d expected", fa.numRegs, XT_REGS);
     attr_once.mark(dev);
   }
-  const int sm_count = sm_counts[dev];
-  experts_tc_kernel<<<sm_count, XT_THREADS, smem, st>>>(
-      L->fast_dev, static_cast<const unsigned char*>(L->arena), h_gate, h_up, L->rank_in, token_indices, expert_offsets,
-      route_w, L->rank_out, T, L->num_experts, L->n_tiles, L->max_slots, L->max_words, plan.nt, plan.ring_h, plan.sec_n,
-      plan.acc_stride, rank_accum, acc64, L->status_dev);
+  XtArgs a{};
+  a.fast = L->fast_dev;
+  a.arena = static_cast<const unsigned char*>(L->arena);
+  a.h_gate = h_gate; a.h_up = h_up; a.h_rank = L->rank_in;
+  a.token_indices = token_indices; a.expert_offsets = expert_offsets; a.route_w = route_w;
+  a.rank_accum = rank_accum; a.acc64 = acc64; a.status = L->status_dev;
+  a.rank_out = L->rank_out; a.T = T; a.num_experts = L->num_experts; a.n_tiles = L->n_tiles; a.max_slots = L->max_slots;
+  a.nt = plan.nt; a.ring_h = plan.ring_h; a.gu_bufs = plan.gu_bufs;
+  experts_tc_kernel<<<sm_counts[dev], XT_THREADS, plan.smem, st>>>(a);
   BM_LAUNCH_CHECK("experts_tc_kernel");
   return BM_OK;
 }

@@ -55,6 +55,9 @@ __host__ __device__ inline int pos32_inv(int p) {
 }
 __host__ __device__ inline int slot_pos(int slot) { return (slot & ~31) + pos32(slot & 31); }
 
+// where the scale of down slot `slot` is stored: rows g and g + 8 of a 16-slot block next to each other
+__host__ __device__ inline int down_scale_pos(int slot) { return (slot & ~15) + 2 * (slot & 7) + ((slot >> 3) & 1); }
+
 // bit position of code (row half `hi8`, k) inside the word owned by thread t = (k & 7) >> 1
 __host__ __device__ inline int nib_shift(int hi8, int k) { return 16 * (k & 1) + 4 * ((k >> 3) * 2 + hi8); }
 __host__ __device__ inline int dense_shift(int blk, int hi8, int k) { return 16 * (k & 1) + 8 * blk + 4 * hi8 + 2 * (k >> 3); }

@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(GemmTcArgs a) {
   __shared__ __align__(8) uint64_t bar_free[TC_STAGES];   // MMAs that read stage s are complete
   __shared__ __align__(8) uint64_t bar_done;              // all MMAs of the tile are complete
   __shared__ uint32_t tmem_slot;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::warp_index(), lane = threadIdx.x & 31;
   const int m0 = blockIdx.x * TC_BM, n0 = blockIdx.y * TC_BN, z = blockIdx.z;
   const __half* W = a.W[z];
   if (threadIdx.x == 0) {
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(GemmTcArgs a) {
     cp_async_wait<TC_AHEAD - 1>();     // this thread's copies of slice s have landed
     tc::fence_async_smem();
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (warp == 0 && tc::elect_one()) {
       tc::fence_after_sync();
       const uint32_t a_base = tc::smem_u32(tc_smem + buf * TC_STAGE_BYTES), b_base = a_base + TC_A_BYTES;
 #pragma unroll

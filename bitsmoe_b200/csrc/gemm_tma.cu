@@ -66,7 +66,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
   __shared__ __align__(8) uint64_t loaded[GT_MAX_STAGES], ready[GT_MAX_STAGES], empty[GT_MAX_STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gt_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::warp_index(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int i = 0; i < GT_MAX_STAGES; ++i) {
       tc::mbar_init(&loaded[i], 1);
@@ -88,31 +88,27 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
   bool ok = true;
 
   if (warp == 0) {
-    // ------------------------------------------------------------------ producer
-    if (lane == 0) {
-      uint32_t st = 0, ph = 0;
-      for (int tile = blockIdx.x; tile < p.ntiles && ok; tile += gridDim.x) {
-        const int per_m = p.tiles_n * p.problems, m_t = tile / per_m, rem = tile - m_t * per_m;
-        const int z = rem / p.tiles_n, n_t = rem - z * p.tiles_n;
-        const CUtensorMap* mw = z ? &map_w1 : &map_w0;
-        for (int s = 0; s < nslices; ++s) {
-          if (!(ok = tc::mbar_wait(&empty[st], ph ^ 1))) break;
+    // ------------------------------------------------------------------ producer (the whole warp waits, one lane issues)
+    uint32_t st = 0, ph = 0;
+    for (int tile = blockIdx.x; tile < p.ntiles && ok; tile += gridDim.x) {
+      const int per_m = p.tiles_n * p.problems, m_t = tile / per_m, rem = tile - m_t * per_m;
+      const int z = rem / p.tiles_n, n_t = rem - z * p.tiles_n;
+      const CUtensorMap* mw = z ? &map_w1 : &map_w0;
+      for (int s = 0; s < nslices; ++s) {
+        if (!(ok = tc::mbar_wait(&empty[st], ph ^ 1))) break;
+        if (tc::elect_one()) {
           unsigned char* sa = smem + st * STAGE;
           tc::mbar_expect_tx(&loaded[st], A_BYTES + B_BYTES);
-          if (XD == BM_F32) {
-            // an fp32 row of 64 values is two 128-byte boxes
-            tma_load_2d(sa, &map_x, s * GT_BK, m_t * GT_BM, &loaded[st]);
-            tma_load_2d(sa + A_BYTES / 2, &map_x, s * GT_BK + 32, m_t * GT_BM, &loaded[st]);
-          } else {
-            tma_load_2d(sa, &map_x, s * GT_BK, m_t * GT_BM, &loaded[st]);
-          }
+          tma_load_2d(sa, &map_x, s * GT_BK, m_t * GT_BM, &loaded[st]);
+          if (XD == BM_F32) tma_load_2d(sa + A_BYTES / 2, &map_x, s * GT_BK + 32, m_t * GT_BM, &loaded[st]);   // an fp32 row of 64 values is two 128-byte boxes
           tma_load_2d(sa + A_BYTES, mw, s * GT_BK, n_t * BN, &loaded[st]);
-          if (++st == NST) { st = 0; ph ^= 1; }
         }
+        __syncwarp();
+        if (++st == NST) { st = 0; ph ^= 1; }
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issue (the whole warp waits, lane 0 issues)
+    // ------------------------------------------------------------------ MMA issue (the whole warp waits, one issues)
     uint32_t st = 0, ph = 0, ti = 0;
     const uint32_t idesc = tc::idesc_f16(GT_BM, BN);
     for (int tile = blockIdx.x; tile < p.ntiles && ok; tile += gridDim.x, ++ti) {
@@ -121,7 +117,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
       tc::fence_after_sync();
       for (int s = 0; s < nslices; ++s) {
         if (!(ok = tc::mbar_wait(XD == BM_F16 ? &loaded[st] : &ready[st], ph))) break;
-        if (lane == 0) {
+        if (tc::elect_one()) {
           const uint32_t sa = tc::smem_u32(smem + st * STAGE);
           const uint64_t ad = gt_desc_sw128(sa), bd = gt_desc_sw128(sa + A_BYTES);
 #pragma unroll
@@ -132,7 +128,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
         __syncwarp();
         if (++st == NST) { st = 0; ph ^= 1; }
       }
-      if (ok && lane == 0) tc::mma_commit(&acc_full[ab]);
+      if (ok && tc::elect_one()) tc::mma_commit(&acc_full[ab]);
       __syncwarp();
     }
   } else if (warp >= GT_WARP_TR0 || warp == 2 || warp == 3) {

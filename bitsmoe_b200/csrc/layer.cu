@@ -60,6 +60,8 @@ static int ingest_matrix(const bm_matrix_t& m, int which, int expert, int interm
     BM_REQUIRE(m.tile_meta, BM_ERR_INVALID_ARG, "%s[%d]: null tile_meta", which_name(which), expert);
     BM_CUDA(cudaMemcpy(out->tile_meta.data(), m.tile_meta, out->tile_meta.size() * 4, cudaMemcpyDeviceToHost));
   }
+  out->rank_idx.assign(static_cast<size_t>(m.n_rows), -1);
+  if (m.n_slabs && m.n_rows) BM_CUDA(cudaMemcpy(out->rank_idx.data(), m.rank_idx, out->rank_idx.size() * 4, cudaMemcpyDeviceToHost));
   for (int i = 0; i < m.n_slabs; ++i) {
     SlabHost s;
     s.bits = slab[i * 4 + 0];
@@ -239,7 +241,7 @@ using namespace bm;
 extern "C" int bm_abi_version(void) { return 2; }
 extern "C" const char* bm_last_error(void) { return g_err; }
 extern "C" uint64_t bm_launch_count(void) { return g_launches.load(std::memory_order_relaxed); }
-extern "C" int bm_arena_layout_version(void) { return 3; }   // 3: one contiguous [scales | words] section per matrix and tile
+extern "C" int bm_arena_layout_version(void) { return 4; }   // 4: octets of ranks kept together, down scales by fragment rows
 extern "C" const char* bm_status_string(int s) {
   switch (s) {
     case BM_OK: return "ok";

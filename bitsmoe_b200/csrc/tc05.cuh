@@ -58,6 +58,19 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 // generic-proxy shared-memory writes -> visible to the async proxy (tensor core / bulk copy engines)
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
+// ---- one issuing thread -----------------------------------------------------------------------
+// tcgen05.mma and tcgen05.commit take their operands from uniform registers.  Behind `if (lane == 0)` the compiler has to
+// assume that several threads may be active and serialises the warp around every instruction: 159 cycles per MMA whatever
+// its shape.  Behind elect.sync it knows that one thread is, and the MMA runs at the tensor pipe's rate (M = 128, K = 16:
+// 48 cycles at N = 64, 64 at 128, 128 at 256, shared-memory operands in any K-major layout).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+// the warp's index as a value the compiler can keep in a uniform register
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0); }
+
 // ---- tensor memory ----------------------------------------------------------------------------
 // One full warp allocates `ncols` (power of two >= 32) columns; the base address lands in *slot (shared).
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
