@@ -35,15 +35,16 @@
 namespace bm {
 
 constexpr int XT_NT_MAX = 128;            // most tokens (assignments) per item: the rows of one MMA
-constexpr int XT_THREADS = 640;
-constexpr int XT_EPI_WARPS = 8, XT_DQ_WARP0 = 8, XT_DQ_WARPS = 8, XT_LOOKUP_WARP = 16, XT_MMA_WARP0 = 17;
+constexpr int XT_THREADS = 768;
+constexpr int XT_EPI_WARPS = 8, XT_DQ_WARP0 = 8, XT_DQ_WARPS = 12, XT_LOOKUP_WARP = 20, XT_MMA_WARP0 = 21;
+constexpr int XT_TEAM = XT_DQ_WARPS / 2;  // converter warps per pipeline
 // Registers per thread at launch and per role afterwards.  The converters keep two stages' words and four independent
 // blocks in flight; at the launch's 96 they spilled, and a spilled load result stalls its warp for the load's latency.
-constexpr int XT_REGS = 96, XT_REGS_EPI = 96, XT_REGS_DQ = 120, XT_REGS_MISC = 48;
+constexpr int XT_REGS = 80, XT_REGS_EPI = 80, XT_REGS_DQ = 88, XT_REGS_MISC = 56;
 static_assert(32 * (XT_EPI_WARPS * XT_REGS_EPI + XT_DQ_WARPS * XT_REGS_DQ + 4 * XT_REGS_MISC) <= XT_THREADS * XT_REGS,
               "the roles' registers come out of the launch's");
 constexpr int XT_CHUNK = 64;              // tile columns per step
-constexpr int XT_RING_MAX = 8;            // operand stages per pipeline (at most)
+constexpr int XT_RING_MAX = 10;           // operand stages per pipeline (at most)
 // A weight stage: 64 operand rows (columns of the chunk, or slots) x 32 contraction positions; bytes between its
 // 8-position chunks (padded: conflict-free 16-byte stores)
 constexpr int XT_W_STRIDE = 64 * 16 + 32;
@@ -56,8 +57,8 @@ constexpr int XT_SLOTS_MAX = 384, XT_RANK_MAX = 1024;
 struct XtBars {
   uint64_t w_full[2 * XT_RING_MAX], w_empty[2 * XT_RING_MAX];
   uint64_t act_ready, down_done;
-  // gate/up accumulators complete / read out, z operand written / consumed, per buffer
-  uint64_t gu_done[2], tmem_gu_free[2], z_ready[2], z_free[2];
+  // per gate/up accumulator pair: products complete, z written over the gate half, z consumed by the down product
+  uint64_t gu_done[2], z_ready[2], z_free[2];
 };
 
 // Position in a cyclic buffer of n slots with the phase bit of its mbarriers.
@@ -151,9 +152,17 @@ __device__ __forceinline__ void dequant_pair_store(uint32_t word0, uint32_t word
   *reinterpret_cast<uint4*>(dst + 128) = make_uint4(r0[1], r0[3], r1[1], r1[3]);
 }
 
+// silu(g) * u with the hardware's exponential and reciprocal; flushing a subnormal exponential to zero does not reach the
+// sum 1 + e, and leaves out the rescaling around both instructions
+__device__ __forceinline__ float silu_mul(float g, float u) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * g));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return g * u * r;
+}
+
 struct XtSmem {
   unsigned char* act;     // [2][nchunks][nt rows] canonical K-major, 16-byte chunks
-  unsigned char* z;       // [2 buffers][8 chunks][nt rows]
   unsigned char* ring;    // [2 pipelines][ring_h][XT_STAGE_BYTES]
   int* prefix;            // [E + 1] items before each expert
   // per item (two of them) and matrix (gate, up), by rank: its factor s, its contraction position (or -1), and per octet of
@@ -164,13 +173,12 @@ struct XtSmem {
 };
 
 __host__ __device__ inline size_t xt_act_bytes(int max_slots, int nt) { return static_cast<size_t>(2) * (max_slots / 8) * xt_chunk_stride(nt); }
-__host__ __device__ inline size_t xt_z_bytes(int nt) { return static_cast<size_t>(XT_CHUNK / 8) * xt_chunk_stride(nt); }
 __host__ __device__ inline size_t xt_smem_bytes(int max_slots, int num_experts, int h_rank, int nt, int ring_h) {
-  size_t o = align_up_c(xt_act_bytes(max_slots, nt) + 2 * xt_z_bytes(nt), 128);
+  size_t o = align_up_c(xt_act_bytes(max_slots, nt), 128);
   o += static_cast<size_t>(2 * ring_h) * XT_STAGE_BYTES;
   o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);
   o += align_up_c(static_cast<size_t>(4) * (h_rank * 4 + h_rank / 4), 128);         // per-rank tables of the activation staging
-  // the MMAs read 128 operand rows whatever nt is: rows past nt of the last chunk lie in what follows the z buffers
+  // the MMAs read 128 operand rows whatever nt is: rows past nt of the last chunk lie in what follows the operand
   return o + 1024;                                                   // slack for the 1024-byte base alignment
 }
 
@@ -312,13 +320,12 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   const int nt = A.nt, ring_h = A.ring_h, h_rank = A.h_rank, num_experts = A.num_experts;
   const int cs = xt_chunk_stride(nt);     // bytes between 8-position chunks of act / z
   const int n_chunks = A.n_tiles * (N_TILE / XT_CHUNK);
-  const uint32_t act_m_bytes = static_cast<uint32_t>(A.max_slots / 8) * cs, z_bytes = static_cast<uint32_t>(xt_z_bytes(nt));
+  const uint32_t act_m_bytes = static_cast<uint32_t>(A.max_slots / 8) * cs;
   XtSmem sm;
   {
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(xt_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     sm.act = base;
-    sm.z = base + xt_act_bytes(A.max_slots, nt);
-    size_t o = align_up_c(xt_act_bytes(A.max_slots, nt) + 2 * xt_z_bytes(nt), 128);
+    size_t o = align_up_c(xt_act_bytes(A.max_slots, nt), 128);
     sm.ring = base + o; o += static_cast<size_t>(2 * ring_h) * XT_STAGE_BYTES;
     sm.prefix = reinterpret_cast<int*>(base + o); o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);
     sm.s_r = reinterpret_cast<__half*>(base + o);
@@ -331,7 +338,6 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     tc::mbar_init(&bars.down_done, 2);
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&bars.gu_done[i], 2);
-      tc::mbar_init(&bars.tmem_gu_free[i], XT_EPI_WARPS);
       tc::mbar_init(&bars.z_ready[i], XT_EPI_WARPS);
       tc::mbar_init(&bars.z_free[i], 2);
     }
@@ -366,6 +372,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   const XtUnits units(sm.prefix[num_experts], static_cast<int>(gridDim.x), n_chunks);
   // tensor memory: gu_bufs x (gate 64 columns, up 64 columns), then the down product's slot tiles of 128 columns
   const uint32_t d_down = tmem_base + A.gu_bufs * 2 * XT_CHUNK;
+  // the down product of a chunk is issued `lag` chunks late: one where tensor memory holds two gate/up accumulator pairs
+  const int lag = A.gu_bufs - 1;
   if (warp == XT_LOOKUP_WARP && static_cast<int>(blockIdx.x) < units.n_units)
     xt_load_item(items[0], sm, 0, blockIdx.x, units, n_chunks, A, lane);
 
@@ -468,18 +476,17 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       const uint32_t lane_sel = static_cast<uint32_t>(32 * q) << 16;
       const int n = 32 * q + lane;
       const bool busy = 32 * q < n_tok;                               // any token in this quarter
-      unsigned char* zrow = sm.z + (4 * half) * cs + n * 16;
       bool ok = true;
       for (int t = 0; t < nchunk && ok; ++t) {
-        const uint32_t gt = gu_round + t, zb = gt & 1u;
-        const uint32_t b = A.gu_bufs == 2 ? zb : 0u, k = A.gu_bufs == 2 ? gt >> 1 : gt;
-        ok = xt_wait(&bars.gu_done[b], k & 1, abort_flag);
-        if (ok && gt >= 2) ok = xt_wait(&bars.z_free[zb], ((gt >> 1) - 1) & 1, abort_flag);     // z buffer consumed two chunks ago
+        const uint32_t gt = gu_round + t, b = lag ? gt & 1u : 0u;
+        ok = xt_wait(&bars.gu_done[b], (lag ? gt >> 1 : gt) & 1, abort_flag);
         if (!ok) break;
         tc::fence_after_sync();
         if (busy) {
           const uint32_t d_gate = tmem_base + 2 * b * XT_CHUNK + lane_sel + 32 * half, d_up = d_gate + XT_CHUNK;
-          uint32_t zp[2][8];
+          // z in the contraction order of the down weights (pos32): 16-byte piece c holds columns 2c, 2c+1, 2c+8, 2c+9 of
+          // both blocks of 16
+          uint32_t zp[16];
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {          // 16 columns at a time: 32 of both would hold 64 registers
             float gv[16], uv[16];
@@ -487,23 +494,15 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             tc::tmem_ld16(d_up + 16 * hh, uv);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-              const float z0 = __fdividef(gv[2 * i] * uv[2 * i], 1.f + __expf(-gv[2 * i]));
-              const float z1 = __fdividef(gv[2 * i + 1] * uv[2 * i + 1], 1.f + __expf(-gv[2 * i + 1]));
-              const __half2 h2 = __floats2half2_rn(z0, z1);
-              zp[hh][i] = *reinterpret_cast<const uint32_t*>(&h2);
+              const __half2 h2 = __floats2half2_rn(silu_mul(gv[2 * i], uv[2 * i]), silu_mul(gv[2 * i + 1], uv[2 * i + 1]));
+              zp[4 * (i & 3) + 2 * hh + (i >> 2)] = *reinterpret_cast<const uint32_t*>(&h2);
             }
           }
-          // chunk c of the contraction order (pos32): columns 2c, 2c+1, 2c+8, 2c+9 of both blocks of 16
-          if (n < nt) {
-            unsigned char* zr = zrow + zb * z_bytes;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(zr + c * cs) = make_uint4(zp[0][c], zp[0][c + 4], zp[1][c], zp[1][c + 4]);
-          }
+          tc::tmem_st16(d_gate, zp);                // over the gate values this warp has just read
         }
         tc::fence_before_sync();
-        tc::fence_async_smem();
         __syncwarp();
-        if (lane == 0) { tc::mbar_arrive(&bars.tmem_gu_free[b]); tc::mbar_arrive(&bars.z_ready[zb]); }
+        if (lane == 0) tc::mbar_arrive(&bars.z_ready[b]);
       }
       if (ok) ok = xt_wait(&bars.down_done, item_round & 1, abort_flag);
       if (busy) {                      // both warps of the quarter go on or neither: they meet at barriers below
@@ -523,7 +522,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         // where eight slots hold an aligned octet of ranks (piece index XORed with the token: conflict-free both ways),
         // and add whole rows, 16 bytes per lane; ranks without a slot add zero.
         const bool turn = A.acc64 == nullptr && (rank_out & 31) == 0 &&
-                          static_cast<size_t>(4) * 32 * rank_out * 4 <= xt_act_bytes(A.max_slots, nt) + 2 * xt_z_bytes(nt);
+                          static_cast<size_t>((nt + 31) / 32) * 32 * rank_out * 4 <= xt_act_bytes(A.max_slots, nt);
         float* tbuf = reinterpret_cast<float*>(sm.act) + q * 32 * rank_out;
         float* trow = tbuf + lane * rank_out;
         const int x7 = lane & 7;
@@ -595,10 +594,9 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       // a stage per 32 slots of chunk t's gate (up) product, then four stages (64 slots x 32 columns) per 128-slot tile
       // of chunk t - 1's down product.  A stage is four 16 x 32 blocks; lane (g, t4) turns its words of each into two
       // 16-byte pieces.  What bounds a warp is latency, not issue: a whole stage per warp gives it four independent
-      // blocks, one barrier wait, one proxy fence and one arrival per 2048 codes, and the next stage's words are on their
-      // way from L2 in a second register set meanwhile.
+      // blocks, one barrier wait, one proxy fence and one arrival per 2048 codes; six warps per team cover one another's loads.
       const int dw = warp - XT_DQ_WARP0;
-      const int team = dw >> 2, g = lane >> 2, t4 = lane & 3;
+      const int team = dw / XT_TEAM, wt = dw - team * XT_TEAM, g = lane >> 2, t4 = lane & 3;
       unsigned char* ring = sm.ring + team * ring_h * XT_STAGE_BYTES + t4 * XT_W_STRIDE + g * 16;
       uint64_t* w_full = &bars.w_full[team * ring_h];
       uint64_t* w_empty = &bars.w_empty[team * ring_h];
@@ -626,7 +624,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             for (int x = 0; x < 4; ++x) p.w[x].x = __ldg(w + x * 32);
           }
         } else {
-          const int j = t < nchunk ? i - npairs : i, ch = chunk0 + t - 1;
+          const int j = t < nchunk ? i - npairs : i, ch = chunk0 + t - lag;
           const int64_t tile = static_cast<int64_t>(ch >> 1) * unit_bytes;
           const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * ((j >> 1) & 1), pr = 2 * (ch & 1) + (j & 1);
           uint32_t* ps = reinterpret_cast<uint32_t*>(&p.s);
@@ -641,7 +639,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         }
       };
       XtCycle my_c = ring_c;
-      my_c.advance(dw & 3, ring_h);
+      my_c.advance(wt, ring_h);
       auto convert = [&](int t, int i, const XtPre& p) -> bool {
         if (!xt_wait(&w_empty[my_c.i], my_c.ph ^ 1, abort_flag)) return false;
         unsigned char* dst = ring + my_c.i * XT_STAGE_BYTES;
@@ -668,36 +666,33 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             else dequant_pair_store<true>(p.w[v].x, p.w[v].x >> 8, sa, sb, dst + v * 256);
           }
         }
+        return true;
+      };
+      auto publish = [&]() {
         tc::fence_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&w_full[my_c.i]);
-        my_c.i += 4;                         // ring_h >= 4: at most one wrap
+        my_c.i += XT_TEAM;                   // ring_h >= XT_TEAM: at most one wrap
         if (my_c.i >= static_cast<uint32_t>(ring_h)) { my_c.i -= ring_h; my_c.ph ^= 1u; }
-        return true;
       };
       // this warp's stage after (t, i); false past its last one
       auto step = [&](int& t, int& i) -> bool {
-        i += 4;
-        for (int n = (t < nchunk ? npairs : 0) + (t > 0 ? n_d : 0); t <= nchunk && i >= n; n = (t < nchunk ? npairs : 0) + n_d) {
+        i += XT_TEAM;
+        for (int n = (t < nchunk ? npairs : 0) + (t >= lag ? n_d : 0); t < nchunk + lag && i >= n; n = (t < nchunk ? npairs : 0) + n_d) {
           i -= n;
           ++t;
         }
-        return t <= nchunk;
+        return t < nchunk + lag;
       };
-      XtPre p0, p1;
-      int t0 = 0, i0 = (dw & 3) - 4, t1, i1;
-      bool more = step(t0, i0);
-      if (more) fetch(t0, i0, p0);
-      t1 = t0; i1 = i0;
+      XtPre p;
+      int t = 0, i = wt - XT_TEAM;
+      bool more = step(t, i);
+      if (more) fetch(t, i, p);
       while (more) {
-        const bool more1 = step(t1, i1);
-        if (more1) fetch(t1, i1, p1);
-        if (!convert(t0, i0, p0) || !more1) break;
-        t0 = t1; i0 = i1;
-        more = step(t0, i0);
-        if (more) fetch(t0, i0, p0);
-        if (!convert(t1, i1, p1)) break;
-        t1 = t0; i1 = i0;
+        if (!convert(t, i, p)) break;
+        more = step(t, i);
+        if (more) fetch(t, i, p);           // on its way while the converted stage is published and the next one is waited for
+        publish();
       }
       ring_c.advance(nchunk * (npairs + n_d), ring_h);
     }
@@ -735,47 +730,52 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         tc::fence_after_sync();
         // descriptors: constant upper part, start-address field advanced per block
         const uint64_t a_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.act) + pl * act_m_bytes, cs, 128);
-        const uint64_t z_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.z), cs, 128);
-        const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring_h * XT_STAGE_BYTES;
+          const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring_h * XT_STAGE_BYTES;
         const uint64_t b_desc = tc::smem_desc_kmajor(ring0, XT_W_STRIDE, 128);
         uint64_t* w_full = &bars.w_full[pl * ring_h];
         uint64_t* w_empty = &bars.w_empty[pl * ring_h];
         const int npairs = fe.m[pl].nslots >> 5;
-        // two MMAs of 64 columns on the next stage: A operand at ad, accumulator d, first MMA overwriting or adding
-        auto stage_mmas = [&](uint32_t d, uint64_t ad, uint32_t accumulate) -> bool {
+        // the two MMAs of the next stage: `issue(b_desc, second)` with the stage's operand
+        auto on_stage = [&](auto&& issue) -> bool {
           if (!xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag)) return false;
           if (tc::elect_one()) {
             const uint64_t bd = b_desc + ((ring_c.i * XT_STAGE_BYTES) >> 4);
-            tc::mma_f16(d, ad, bd, idesc, accumulate);
-            tc::mma_f16(d, ad + ((2 * cs) >> 4), bd + ((2 * XT_W_STRIDE) >> 4), idesc, 1u);
+            issue(bd, 0u);
+            issue(bd + ((2 * XT_W_STRIDE) >> 4), 1u);
             tc::mma_commit(&w_empty[ring_c.i]);
           }
           __syncwarp();
           ring_c.next(ring_h);
           return true;
         };
-        for (int t = 0; t <= nchunk && ok; ++t) {
+        for (int t = 0; t < nchunk + lag && ok; ++t) {
           if (t < nchunk) {
-            const uint32_t g = gu_round + t, b = A.gu_bufs == 2 ? g & 1u : 0u, k = A.gu_bufs == 2 ? g >> 1 : g;
-            if (k >= 1) ok = xt_wait(&bars.tmem_gu_free[b], (k - 1) & 1, abort_flag);   // this accumulator's last contents are read out
+            const uint32_t g = gu_round + t, b = lag ? g & 1u : 0u, k = lag ? g >> 1 : g;
+            if (k >= 1) ok = xt_wait(&bars.z_free[b], (k - 1) & 1, abort_flag);   // the z that took this accumulator's place is consumed
             tc::fence_after_sync();
             const uint32_t d_acc = tmem_base + (2 * b + pl) * XT_CHUNK;
-            for (int pr = 0; pr < npairs && ok; ++pr) ok = stage_mmas(d_acc, a_desc + ((4 * pr * cs) >> 4), pr > 0 ? 1u : 0u);
+            for (int pr = 0; pr < npairs && ok; ++pr) {
+              const uint64_t ad = a_desc + ((4 * pr * cs) >> 4);
+              ok = on_stage([&](uint64_t bd, uint32_t j) { tc::mma_f16(d_acc, ad + ((j * 2 * cs) >> 4), bd, idesc, (pr > 0 ? 1u : 0u) | j); });
+            }
             if (!ok) break;
             if (tc::elect_one()) tc::mma_commit(&bars.gu_done[b]);
             __syncwarp();
           }
-          if (t > 0) {
-            const uint32_t g = gu_round + t - 1, zb = g & 1u;
-            ok = xt_wait(&bars.z_ready[zb], (g >> 1) & 1, abort_flag);
+          if (t >= lag) {
+            const uint32_t g = gu_round + t - lag, b = lag ? g & 1u : 0u;
+            ok = xt_wait(&bars.z_ready[b], (lag ? g >> 1 : g) & 1, abort_flag);
             tc::fence_after_sync();
-            const uint64_t zd = z_desc + ((zb * z_bytes) >> 4);
+            // 64 slots and 32 columns of z (16 tensor-memory columns, at the start of the half they came from) per stage
             for (int mt = pl; mt < n_mt && ok; mt += 2)
-              for (int q = 0; q < 4 && ok; ++q)               // 64 slots and 32 columns of z per stage
-                ok = stage_mmas(d_down + mt * 128 + (q >> 1) * 64, zd + ((4 * (q & 1) * cs) >> 4), (t > 1 || (q & 1)) ? 1u : 0u);
+              for (int q = 0; q < 4 && ok; ++q) {
+                const uint32_t d_acc = d_down + mt * 128 + (q >> 1) * 64, za = tmem_base + 2 * b * XT_CHUNK + (q & 1) * 32;
+                const uint32_t add = t > lag || (q & 1) ? 1u : 0u;
+                ok = on_stage([&](uint64_t bd, uint32_t j) { tc::mma_f16_ta(d_acc, za + 8 * j, bd, idesc, add | j); });
+              }
             if (ok && tc::elect_one()) {
-              tc::mma_commit(&bars.z_free[zb]);
-              if (t == nchunk) tc::mma_commit(&bars.down_done);
+              tc::mma_commit(&bars.z_free[b]);
+              if (t == nchunk + lag - 1) tc::mma_commit(&bars.down_done);
             }
             __syncwarp();
           }
@@ -789,19 +789,21 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
 }
 
 // Item size and ring depth for a layer: the first candidate whose activation operand (2 KB per token at 256 row slots per
-// matrix), z buffers and stages fit shared memory.  Tensor memory holds 128 columns per gate/up buffer and 128 per 128
+// matrix) and stages fit shared memory.  Tensor memory holds 128 columns per gate/up buffer and 128 per 128
 // slots of the down product.
 struct XtPlan { int nt, ring_h, gu_bufs; size_t smem; };
 constexpr size_t XT_SMEM_LIMIT = 227 * 1024 - 8192;     // dynamic part: the static part (two item descriptions, barriers) stays below 8 KB
 static bool xt_plan(const bm_layer* L, XtPlan* out) {
   if (L->num_experts > XT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > 3 * 128) return false;
   const int n_mt = (L->max_slots + 127) / 128;
-  static const int cand[][2] = {{128, 6}, {128, 4}, {112, 6}, {112, 4}, {96, 6}, {96, 4}, {80, 6}, {80, 4}, {64, 6}, {64, 4}, {48, 4}, {32, 4}, {16, 4}};
-  for (const auto& c : cand) {
-    const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, L->rank_in, c[0], c[1]);
-    if (smem <= XT_SMEM_LIMIT) {
-      *out = XtPlan{c[0], c[1], n_mt > 2 ? 1 : 2, smem};
-      return true;
+  static const int cand[] = {128, 112, 96, 80, 64, 48, 32, 16};
+  for (const int nt : cand) {
+    for (int ring = XT_RING_MAX; ring >= XT_TEAM; --ring) {
+      const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, L->rank_in, nt, ring);
+      if (smem <= XT_SMEM_LIMIT) {
+        *out = XtPlan{nt, ring, n_mt > 2 ? 1 : 2, smem};
+        return true;
+      }
     }
   }
   return false;
