@@ -90,6 +90,10 @@ void plan_fast(const bm_layer* L, size_t base_bytes, FastPlan* P) {
     }
   }
   off = align_up(off, 256);
+  if (L->rank_in % 8 == 0 && L->rank_in <= TOKTAB_MAX_RANK) {
+    P->toktab_off = off;
+    off = align_up(off + static_cast<size_t>(TokTab(L->rank_in, P->max_slots).bytes) * E, 256);
+  }
   P->units_off = off;
   for (int e = 0; e < E; ++e) {
     FastExpert& fe = P->experts[e];
@@ -164,6 +168,67 @@ __global__ void __launch_bounds__(128) repack_tables_kernel(const ExpertDev* __r
       t_row[slot] = static_cast<int16_t>(row);
     }
   }
+}
+
+// Token-side tables, one block per expert; reads the slot tables of repack_tables_kernel.
+__global__ void __launch_bounds__(128) build_toktab_kernel(const FastExpert* __restrict__ fast, int rank_in, int rank_out, int max_slots,
+                                                          const unsigned char* __restrict__ arena, unsigned char* __restrict__ out) {
+  const FastExpert& fe = fast[blockIdx.x];
+  const TokTab lay(rank_in, max_slots);
+  unsigned char* t = out + static_cast<size_t>(blockIdx.x) * lay.bytes;
+  TokTabHead* head = reinterpret_cast<TokTabHead*>(t);
+  __half* s_r = reinterpret_cast<__half*>(t + lay.s_r);
+  int16_t *pos_r = reinterpret_cast<int16_t*>(t + lay.pos_r), *oct_r = reinterpret_cast<int16_t*>(t + lay.oct_r);
+  float* s_d = reinterpret_cast<float*>(t + lay.s_d);
+  int16_t *rank_d = reinterpret_cast<int16_t*>(t + lay.rank_d), *oct_d = reinterpret_cast<int16_t*>(t + lay.oct_d);
+  __shared__ int padded, live_d;
+  __shared__ uint32_t broken[2][4];
+  if (threadIdx.x == 0) { padded = 0; live_d = 0; }
+  if (threadIdx.x < 8) broken[threadIdx.x >> 2][threadIdx.x & 3] = 0u;
+  for (int i = threadIdx.x; i < 2 * rank_in; i += blockDim.x) { pos_r[i] = -1; s_r[i] = __float2half(0.f); }
+  for (int i = threadIdx.x; i < max_slots; i += blockDim.x) { rank_d[i] = -1; s_d[i] = 0.f; }
+  __syncthreads();
+  for (int m = 0; m < 3; ++m) {
+    const FastMat& fm = fe.m[m];
+    const int16_t* rank_t = reinterpret_cast<const int16_t*>(arena + fm.tab_off);
+    const __half* s_t = reinterpret_cast<const __half*>(arena + fm.tab_off + fm.nslots * 2);
+    for (int i = threadIdx.x; i < fm.nslots; i += blockDim.x) {
+      const int rk = rank_t[i];
+      if (m == 2) {
+        const bool live = rk >= 0 && rk < rank_out;
+        rank_d[i] = static_cast<int16_t>(live ? rk : -1);
+        s_d[i] = __half2float(s_t[i]);
+        if (live) atomicAdd(&live_d, 1);
+      } else if (rk >= 0 && rk < rank_in) {
+        pos_r[m * rank_in + rk] = static_cast<int16_t>(slot_pos(i));
+        s_r[m * rank_in + rk] = s_t[i];
+      } else {
+        padded = 1;
+      }
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * (rank_in / 8); i += blockDim.x) {
+    const int m = i / (rank_in / 8), o = i - m * (rank_in / 8);
+    const int16_t* p = pos_r + m * rank_in + 8 * o;
+    bool whole = p[0] >= 0 && (p[0] & 7) == 0;
+    for (int j = 1; j < 8; ++j) whole &= p[j] == p[0] + j;
+    oct_r[i] = static_cast<int16_t>(whole ? p[0] >> 3 : -1);
+    if (!whole) atomicOr(&broken[m][o >> 5], 1u << (o & 31));
+  }
+  for (int c = threadIdx.x; c < max_slots / 8; c += blockDim.x) {
+    const int16_t* r = rank_d + 8 * c;
+    bool whole = r[0] >= 0 && (r[0] & 7) == 0;
+    for (int j = 1; j < 8; ++j) whole &= r[j] == r[0] + j;
+    oct_d[c] = static_cast<int16_t>(whole ? r[0] : -1);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    head->fe = fe;
+    head->padded = padded;
+    head->all_ranks = live_d == rank_out;
+  }
+  if (threadIdx.x < 8) head->broken[threadIdx.x >> 2][threadIdx.x & 3] = broken[threadIdx.x >> 2][threadIdx.x & 3];
 }
 
 // Where the codes of word `i` of a matrix section come from.  `first_blk` = the word's first 16-slot (gate/up:
@@ -278,6 +343,11 @@ int build_fast(bm_layer* L, const FastPlan& P, cudaStream_t st) {
   BM_LAUNCH_CHECK("repack_tables_kernel");
   repack_words_kernel<<<grid, 256, 0, st>>>(L->experts_dev, d_fast, d_rows, d_offs, arena);
   BM_LAUNCH_CHECK("repack_words_kernel");
+  if (P.toktab_off) {
+    L->toktab_dev = arena + P.toktab_off;
+    build_toktab_kernel<<<L->num_experts, 128, 0, st>>>(d_fast, L->rank_in, L->rank_out, P.max_slots, arena, arena + P.toktab_off);
+    BM_LAUNCH_CHECK("build_toktab_kernel");
+  }
   BM_CUDA(cudaStreamSynchronize(st));
   return BM_OK;
 }

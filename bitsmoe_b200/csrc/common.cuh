@@ -104,6 +104,31 @@ struct FastExpert {
   int32_t pad_;
 };
 
+// Token-side table of one expert, built at load time: what a kernel needs to put token rows into an expert's operand order
+// and its sums back into rank order, as one contiguous copy.  All experts of a layer share the offsets.
+struct TokTabHead {
+  FastExpert fe;
+  int32_t padded;           // gate or up has slots without a row
+  int32_t all_ranks;        // every rank of rank_accum has a down slot
+  uint32_t broken[2][4];    // gate, up: octets of ranks that are not one 16-byte piece of the operand row (bit per octet)
+};
+constexpr int TOKTAB_MAX_RANK = 1024;
+struct TokTab {
+  int s_r, pos_r, oct_r;    // [gate, up][rank] factor s (fp16), contraction position or -1 (int16); per octet: its piece or -1 (int16)
+  int s_d, rank_d, oct_d;   // per down slot: factor (fp32), rank or -1 (int16); per eight slots: first rank of an aligned octet or -1
+  int bytes;
+  __host__ __device__ TokTab(int rank_in, int max_slots) {
+    auto up = [](int v) { return (v + 15) & ~15; };
+    s_r = up(static_cast<int>(sizeof(TokTabHead)));
+    pos_r = s_r + 4 * rank_in;
+    oct_r = pos_r + 4 * rank_in;
+    s_d = up(oct_r + rank_in / 2);
+    rank_d = s_d + 4 * max_slots;
+    oct_d = rank_d + 2 * max_slots;
+    bytes = up(oct_d + max_slots / 4);
+  }
+};
+
 struct FastPlan {
   bool ok = false;
   std::vector<FastExpert> experts;
@@ -112,6 +137,7 @@ struct FastPlan {
   size_t table_off = 0;               // FastExpert table
   size_t tabs_off = 0;                // per-matrix rank/s/row tables
   size_t units_off = 0;
+  size_t toktab_off = 0;              // token-side tables (rank_in <= TOKTAB_MAX_RANK), 0 = none
   size_t total = 0;
   int max_unit_bytes = 0, max_slots = 0, max_words = 0;
 };
@@ -205,6 +231,7 @@ struct bm_layer {
   bool fast_ok = false;            // every slab is 1/2/3/4-bit and shapes fit the decode / tensor paths
   const bm::FastExpert* fast_dev = nullptr;   // in the arena
   std::vector<bm::FastExpert> fast_host;
+  const unsigned char* toktab_dev = nullptr;  // in the arena
   int max_unit_bytes = 0, max_slots = 0, max_words = 0;
   // launch geometry of the decode kernel on this layer's device (plan_experts_decode)
   bool dec_ok = false;

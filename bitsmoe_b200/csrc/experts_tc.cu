@@ -44,19 +44,20 @@ constexpr int XT_REGS = 80, XT_REGS_EPI = 80, XT_REGS_DQ = 88, XT_REGS_MISC = 56
 static_assert(32 * (XT_EPI_WARPS * XT_REGS_EPI + XT_DQ_WARPS * XT_REGS_DQ + 4 * XT_REGS_MISC) <= XT_THREADS * XT_REGS,
               "the roles' registers come out of the launch's");
 constexpr int XT_CHUNK = 64;              // tile columns per step
-constexpr int XT_RING_MAX = 10;           // operand stages per pipeline (at most)
+constexpr int XT_RING_MAX = 5;            // operand slots per pipeline (at most), two stages each
 // A weight stage: 64 operand rows (columns of the chunk, or slots) x 32 contraction positions; bytes between its
 // 8-position chunks (padded: conflict-free 16-byte stores)
 constexpr int XT_W_STRIDE = 64 * 16 + 32;
 constexpr int XT_STAGE_BYTES = 4 * XT_W_STRIDE;
+constexpr int XT_SLOT_BYTES = 2 * XT_STAGE_BYTES;     // the MMA issuers take two stages per barrier
 // bytes between 8-position chunks of the token-side operands (padded: conflict-free stores)
 __host__ __device__ constexpr int xt_chunk_stride(int nt) { return nt * 16 + 16; }
 constexpr int XT_MAX_E = 1024;
-constexpr int XT_SLOTS_MAX = 384, XT_RANK_MAX = 1024;
 
 struct XtBars {
   uint64_t w_full[2 * XT_RING_MAX], w_empty[2 * XT_RING_MAX];
   uint64_t act_ready, down_done;
+  uint64_t tab[2];                        // an item's token-side table has landed
   // per gate/up accumulator pair: products complete, z written over the gate half, z consumed by the down product
   uint64_t gu_done[2], z_ready[2], z_free[2];
 };
@@ -75,16 +76,10 @@ struct XtCycle {
 };
 
 struct XtItem {
-  FastExpert fe;
   int tok[XT_NT_MAX];
   float rw[XT_NT_MAX];
-  __align__(16) float s_d[XT_SLOTS_MAX];         // the down product's slots: factor,
-  __align__(16) int16_t rank_d[XT_SLOTS_MAX];    // rank or -1,
-  int16_t oct_d[XT_SLOTS_MAX / 8];               // first rank of eight slots that hold an aligned octet of ranks, or -1
-  uint32_t broken[2][XT_RANK_MAX / 256];         // gate, up: octets of ranks that are not one piece of the operand row
   int n, chunk0, nchunk;
-  int padded;                                    // gate or up has slots without a row
-  int all_ranks;                                 // every rank of rank_accum has a down slot
+  int ok;                                 // the table has landed
 };
 
 __device__ __forceinline__ bool xt_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
@@ -165,19 +160,16 @@ struct XtSmem {
   unsigned char* act;     // [2][nchunks][nt rows] canonical K-major, 16-byte chunks
   unsigned char* ring;    // [2 pipelines][ring_h][XT_STAGE_BYTES]
   int* prefix;            // [E + 1] items before each expert
-  // per item (two of them) and matrix (gate, up), by rank: its factor s, its contraction position (or -1), and per octet of
-  // ranks the 16-byte piece of the operand row that holds it (or -1)
-  __half* s_r;            // [h_rank]
-  int16_t* pos_r;         // [h_rank]
-  int16_t* oct_r;         // [h_rank / 8]
+  int* offset;            // [E + 1] assignments before each expert
+  unsigned char* tab;     // [2 items] token-side table of the item's expert (TokTab)
 };
 
 __host__ __device__ inline size_t xt_act_bytes(int max_slots, int nt) { return static_cast<size_t>(2) * (max_slots / 8) * xt_chunk_stride(nt); }
-__host__ __device__ inline size_t xt_smem_bytes(int max_slots, int num_experts, int h_rank, int nt, int ring_h) {
+__host__ __device__ inline size_t xt_smem_bytes(int max_slots, int num_experts, int tab_bytes, int nt, int ring_h) {
   size_t o = align_up_c(xt_act_bytes(max_slots, nt), 128);
-  o += static_cast<size_t>(2 * ring_h) * XT_STAGE_BYTES;
-  o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);
-  o += align_up_c(static_cast<size_t>(4) * (h_rank * 4 + h_rank / 4), 128);         // per-rank tables of the activation staging
+  o += static_cast<size_t>(2 * ring_h) * XT_SLOT_BYTES;
+  o += align_up_c(static_cast<size_t>(2 * num_experts + 2) * 4, 128);     // items and assignments before each expert
+  o += static_cast<size_t>(2) * tab_bytes;
   // the MMAs read 128 operand rows whatever nt is: rows past nt of the last chunk lie in what follows the operand
   return o + 1024;                                                   // slack for the 1024-byte base alignment
 }
@@ -198,8 +190,8 @@ struct XtUnits {
 };
 
 struct XtArgs {
-  const FastExpert* fast;
   const unsigned char* arena;
+  const unsigned char* toktab;
   const __half* h_gate;
   const __half* h_up;
   const int32_t* token_indices;
@@ -208,17 +200,12 @@ struct XtArgs {
   float* rank_accum;
   long long* acc64;
   int* status;
-  int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, ring_h, gu_bufs;
+  int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, ring_h, gu_bufs, tab_bytes;
 };
 
-// Locates unit `u` and copies what the roles need, its tables turned into the order the roles read them; one warp, an item
-// ahead of the roles.
-__device__ __forceinline__ void xt_load_item(XtItem& item, const XtSmem& sm, int buf, int u, const XtUnits& units, int n_chunks,
-                                             const XtArgs& A, int lane) {
-  const int* prefix = sm.prefix;
-  __half* s_r = sm.s_r + buf * 2 * A.h_rank;
-  int16_t* pos_r = sm.pos_r + buf * 2 * A.h_rank;
-  int16_t* oct_r = sm.oct_r + buf * 2 * (A.h_rank / 8);
+// Locates unit `u` and copies what the roles need; one warp, an item ahead of the roles.
+__device__ __forceinline__ void xt_load_item(XtItem& item, unsigned char* tab, uint64_t* bar, int u, const XtUnits& units, int n_chunks,
+                                             const XtSmem& sm, const XtArgs& A, int lane) {
   int it = u, chunk0 = 0, nchunk = n_chunks;
   if (u >= units.full) {
     const int r = u - units.full, part = r % units.split;
@@ -229,76 +216,31 @@ __device__ __forceinline__ void xt_load_item(XtItem& item, const XtSmem& sm, int
   int lo = 0, hi = A.num_experts - 1;           // last expert e with prefix[e] <= it
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (prefix[mid] <= it) lo = mid; else hi = mid - 1;
+    if (sm.prefix[mid] <= it) lo = mid; else hi = mid - 1;
   }
   const int e = lo;
-  for (int i = lane; i < static_cast<int>(sizeof(FastExpert) / 4); i += 32)
-    reinterpret_cast<uint32_t*>(&item.fe)[i] = reinterpret_cast<const uint32_t*>(&A.fast[e])[i];
+  if (lane == 0) {
+    tc::mbar_expect_tx(bar, A.tab_bytes);
+    tc::bulk_g2s(tab, A.toktab + static_cast<size_t>(e) * A.tab_bytes, A.tab_bytes, bar);
+  }
   // an expert's assignments are spread evenly over its items
-  const int begin = A.expert_offsets[e], cnt = A.expert_offsets[e + 1] - begin, parts = prefix[e + 1] - prefix[e], j = it - prefix[e];
+  const int begin = sm.offset[e], cnt = sm.offset[e + 1] - begin, parts = sm.prefix[e + 1] - sm.prefix[e], j = it - sm.prefix[e];
   const int a0 = begin + static_cast<int>(static_cast<int64_t>(cnt) * j / parts);
   const int n = begin + static_cast<int>(static_cast<int64_t>(cnt) * (j + 1) / parts) - a0;
+  int tk[XT_NT_MAX / 32];
+  float rw[XT_NT_MAX / 32];
 #pragma unroll
   for (int q = 0; q < XT_NT_MAX / 32; ++q) {
     const int i = lane + 32 * q;
-    const int tk = i < n ? A.token_indices[a0 + i] : 0;
-    const bool good = i < n && tk >= 0 && tk < A.T;
-    item.tok[i] = good ? tk : 0;
-    item.rw[i] = good ? A.route_w[a0 + i] : 0.f;
+    tk[q] = i < n ? A.token_indices[a0 + i] : -1;
+    rw[q] = i < n ? A.route_w[a0 + i] : 0.f;
   }
-  for (int i = lane; i < 2 * A.h_rank; i += 32) {
-    pos_r[i] = -1;
-    s_r[i] = __float2half(0.f);
-  }
-  for (int i = lane; i < 2 * (A.h_rank / 8); i += 32) oct_r[i] = -1;
-  __syncwarp();
-  bool padded = false;
-  int live_d = 0;
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    const FastMat& fm = item.fe.m[m];
-    const int16_t* rank_t = reinterpret_cast<const int16_t*>(A.arena + fm.tab_off);
-    const __half* s_t = reinterpret_cast<const __half*>(A.arena + fm.tab_off + fm.nslots * 2);
-#pragma unroll 8
-    for (int i = lane; i < fm.nslots; i += 32) {
-      const int rk = rank_t[i];
-      const __half sv = s_t[i];
-      if (m == 2) {
-        const bool live = rk >= 0 && rk < A.rank_out;
-        item.rank_d[i] = static_cast<int16_t>(live ? rk : -1);
-        item.s_d[i] = __half2float(sv);
-        live_d += live;
-      } else if (rk >= 0 && rk < A.h_rank) {
-        pos_r[m * A.h_rank + rk] = static_cast<int16_t>(slot_pos(i));
-        s_r[m * A.h_rank + rk] = sv;
-      } else {
-        padded = true;
-      }
-    }
+  for (int q = 0; q < XT_NT_MAX / 32; ++q) {
+    const bool good = tk[q] >= 0 && tk[q] < A.T;
+    item.tok[lane + 32 * q] = good ? tk[q] : 0;
+    item.rw[lane + 32 * q] = good ? rw[q] : 0.f;
   }
-  __syncwarp();
-  for (int m = 0; m < 2; ++m)
-    for (int o0 = 0; o0 < A.h_rank / 8; o0 += 32) {
-      const int o = o0 + lane;
-      bool whole = o < A.h_rank / 8;
-      if (whole) {
-        const int16_t* p = pos_r + m * A.h_rank + 8 * o;
-        whole = p[0] >= 0 && (p[0] & 7) == 0;
-        for (int j = 1; j < 8; ++j) whole &= p[j] == p[0] + j;
-        if (whole) oct_r[m * (A.h_rank / 8) + o] = static_cast<int16_t>(p[0] >> 3);
-      }
-      const uint32_t broken = __ballot_sync(0xffffffffu, !whole && o < A.h_rank / 8);
-      if (lane == 0) item.broken[m][o0 >> 5] = broken;
-    }
-  for (int c = lane; c < item.fe.m[2].nslots >> 3; c += 32) {
-    const int16_t* r = item.rank_d + 8 * c;
-    bool whole = r[0] >= 0 && (r[0] & 7) == 0;
-    for (int j = 1; j < 8; ++j) whole &= r[j] == r[0] + j;
-    item.oct_d[c] = static_cast<int16_t>(whole ? r[0] : -1);
-  }
-  padded = __any_sync(0xffffffffu, padded);
-  live_d = __reduce_add_sync(0xffffffffu, live_d);
-  if (lane == 0) { item.padded = padded; item.all_ranks = live_d == A.rank_out; }
   if (lane == 0) { item.n = n; item.chunk0 = chunk0; item.nchunk = nchunk; }
 }
 
@@ -326,17 +268,18 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(xt_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     sm.act = base;
     size_t o = align_up_c(xt_act_bytes(A.max_slots, nt), 128);
-    sm.ring = base + o; o += static_cast<size_t>(2 * ring_h) * XT_STAGE_BYTES;
-    sm.prefix = reinterpret_cast<int*>(base + o); o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);
-    sm.s_r = reinterpret_cast<__half*>(base + o);
-    sm.pos_r = reinterpret_cast<int16_t*>(sm.s_r + 4 * h_rank);
-    sm.oct_r = sm.pos_r + 4 * h_rank;
+    sm.ring = base + o; o += static_cast<size_t>(2 * ring_h) * XT_SLOT_BYTES;
+    sm.prefix = reinterpret_cast<int*>(base + o);
+    sm.offset = sm.prefix + num_experts + 1;
+    o += align_up_c(static_cast<size_t>(2 * num_experts + 2) * 4, 128);
+    sm.tab = base + o;
   }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2 * XT_RING_MAX; ++i) { tc::mbar_init(&bars.w_full[i], 1); tc::mbar_init(&bars.w_empty[i], 1); }
+    for (int i = 0; i < 2 * XT_RING_MAX; ++i) { tc::mbar_init(&bars.w_full[i], 2); tc::mbar_init(&bars.w_empty[i], 1); }
     tc::mbar_init(&bars.act_ready, 1);
     tc::mbar_init(&bars.down_done, 2);
     for (int i = 0; i < 2; ++i) {
+      tc::mbar_init(&bars.tab[i], 1);
       tc::mbar_init(&bars.gu_done[i], 2);
       tc::mbar_init(&bars.z_ready[i], XT_EPI_WARPS);
       tc::mbar_init(&bars.z_free[i], 2);
@@ -347,8 +290,12 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
   // items before each expert (an item = up to nt consecutive assignments of one expert): every thread loads
   // its experts' counts in parallel, one warp then scans them
-  for (int e = threadIdx.x; e < num_experts; e += XT_THREADS)
-    sm.prefix[e + 1] = (A.expert_offsets[e + 1] - A.expert_offsets[e] + nt - 1) / nt;
+  for (int e = threadIdx.x; e < num_experts; e += XT_THREADS) {
+    const int o0 = A.expert_offsets[e], o1 = A.expert_offsets[e + 1];
+    sm.prefix[e + 1] = (o1 - o0 + nt - 1) / nt;
+    sm.offset[e + 1] = o1;
+    if (e == 0) sm.offset[0] = o0;
+  }
   __syncthreads();
   if (warp == 1) {
     int carry = 0;
@@ -374,8 +321,18 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   const uint32_t d_down = tmem_base + A.gu_bufs * 2 * XT_CHUNK;
   // the down product of a chunk is issued `lag` chunks late: one where tensor memory holds two gate/up accumulator pairs
   const int lag = A.gu_bufs - 1;
+  const TokTab lay(h_rank, A.max_slots);
+  // item number `round` of this CTA into its buffers; waits for its table, so that the barrier at the item's start
+  // publishes everything
+  auto load_item = [&](uint32_t round, int u) {
+    const uint32_t buf = round & 1u;
+    xt_load_item(items[buf], sm.tab + buf * lay.bytes, &bars.tab[buf], u, units, n_chunks, sm, A, lane);
+    const bool landed = xt_wait(&bars.tab[buf], (round >> 1) & 1u, abort_flag);
+    if (lane == 0) items[buf].ok = landed;
+    __syncwarp();
+  };
   if (warp == XT_LOOKUP_WARP && static_cast<int>(blockIdx.x) < units.n_units)
-    xt_load_item(items[0], sm, 0, blockIdx.x, units, n_chunks, A, lane);
+    load_item(0, blockIdx.x);
 
   // Positions in the cyclic buffers; every role steps through the same sequence of stages and chunks, so each keeps its
   // own copy across items.
@@ -384,8 +341,9 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   uint32_t item_round = 0;
 
   // Activation operand of an item, once per item, by the epilogue and converter warps.
-  auto stage_item = [&](const XtItem& item) {
-    const FastExpert& fe = item.fe;
+  auto stage_item = [&](const XtItem& item, const unsigned char* tab) {
+    const TokTabHead& head = *reinterpret_cast<const TokTabHead*>(tab);
+    const FastExpert& fe = head.fe;
     const int n_tok = item.n;
     constexpr int XT_STAGERS = (XT_EPI_WARPS + XT_DQ_WARPS) * 32;
     const int tid_s = threadIdx.x, warp_s = warp;
@@ -395,9 +353,9 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     // that straddle two groups of rows follow rank by rank.  Operand rows past the item's tokens keep whatever they
     // hold: they only reach accumulator rows that nobody reads.
     const int n_oct = h_rank >> 3;
-    const int16_t* pos_r = sm.pos_r + (item_round & 1) * 2 * h_rank;
-    const __half* s_r = sm.s_r + (item_round & 1) * 2 * h_rank;
-    const int16_t* oct_r = sm.oct_r + (item_round & 1) * 2 * n_oct;
+    const int16_t* pos_r = reinterpret_cast<const int16_t*>(tab + lay.pos_r);
+    const __half* s_r = reinterpret_cast<const __half*>(tab + lay.s_r);
+    const int16_t* oct_r = reinterpret_cast<const int16_t*>(tab + lay.oct_r);
     for (int o0 = 0; o0 < n_oct; o0 += 32) {
       const int o = o0 + lane;
       int dst[2];
@@ -437,7 +395,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     }
     for (int m = 0; m < 2; ++m)
       for (int w = 0; w < (n_oct + 31) >> 5; ++w)
-        for (uint32_t left = item.broken[m][w]; left; left &= left - 1) {
+        for (uint32_t left = head.broken[m][w]; left; left &= left - 1) {
           const int o = 32 * w + __ffs(left) - 1;
           for (int i = tid_s; i < 8 * n_tok; i += XT_STAGERS) {
             const int n = i >> 3, rk = 8 * o + (i & 7), pos = pos_r[m * h_rank + rk];
@@ -446,7 +404,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
                   __hmul((m ? A.h_up : A.h_gate)[static_cast<int64_t>(item.tok[n]) * h_rank + rk], s_r[m * h_rank + rk]);
           }
         }
-    if (item.padded) {        // padding slots: their weights are zero, their activations have to be finite
+    if (head.padded) {        // padding slots: their weights are zero, their activations have to be finite
       for (int m = 0; m < 2; ++m) {
         const int16_t* rank_t = reinterpret_cast<const int16_t*>(A.arena + fe.m[m].tab_off);
         for (int i = warp_s; i < fe.m[m].nslots; i += XT_STAGERS / 32) {
@@ -467,9 +425,11 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++item_round) {
       __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
       const XtItem& item = items[item_round & 1];
-      const FastExpert& fe = item.fe;
+      if (!item.ok) break;
+      const unsigned char* tab = sm.tab + (item_round & 1) * lay.bytes;
+      const FastExpert& fe = reinterpret_cast<const TokTabHead*>(tab)->fe;
       const int n_tok = item.n, nchunk = item.nchunk;
-      stage_item(item);
+      stage_item(item, tab);
       // ------------------------------------------------------------------ epilogue warps 0-7
       // warp = (TMEM lane quarter q: tokens 32 q .. 32 q + 31, half of the chunk's 64 columns); a thread owns a token
       const int q = warp & 3, half = warp >> 2;
@@ -526,22 +486,24 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         float* tbuf = reinterpret_cast<float*>(sm.act) + q * 32 * rank_out;
         float* trow = tbuf + lane * rank_out;
         const int x7 = lane & 7;
-        if (turn && !item.all_ranks) {
+        if (turn && !reinterpret_cast<const TokTabHead*>(tab)->all_ranks) {
           for (int i = half * 32 + lane; i < 8 * rank_out; i += 64) reinterpret_cast<float4*>(tbuf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
           asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
         }
         const int nslots_d = fe.m[2].nslots;
+        const float* s_d = reinterpret_cast<const float*>(tab + lay.s_d);
+        const int16_t *rank_d = reinterpret_cast<const int16_t*>(tab + lay.rank_d), *oct_d = reinterpret_cast<const int16_t*>(tab + lay.oct_d);
         for (int s0 = 16 * half; s0 < nslots_d; s0 += 32) {
           float v[16];
           tc::tmem_ld16(d_down + lane_sel + s0, v);
 #pragma unroll
           for (int i = 0; i < 16; i += 4) {
-            const float4 sv = *reinterpret_cast<const float4*>(item.s_d + s0 + i);
+            const float4 sv = *reinterpret_cast<const float4*>(s_d + s0 + i);
             v[i] *= sv.x * rw; v[i + 1] *= sv.y * rw; v[i + 2] *= sv.z * rw; v[i + 3] *= sv.w * rw;
           }
 #pragma unroll
           for (int h8 = 0; h8 < 2; ++h8) {
-            const int r0 = item.oct_d[(s0 >> 3) + h8];
+            const int r0 = oct_d[(s0 >> 3) + h8];
             const float* w = v + 8 * h8;
             if (turn && r0 >= 0) {
               *reinterpret_cast<float4*>(trow + 4 * ((r0 >> 2) ^ x7)) = make_float4(w[0], w[1], w[2], w[3]);
@@ -549,7 +511,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             } else {
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
-                const int r = item.rank_d[s0 + 8 * h8 + i];
+                const int r = rank_d[s0 + 8 * h8 + i];
                 if (r < 0) continue;
                 if (turn) trow[4 * ((r >> 2) ^ x7) + (r & 3)] = w[i];
                 else if (n < n_tok) acc_add(A.rank_accum, A.acc64, static_cast<int64_t>(item.tok[n]) * rank_out + r, w[i]);
@@ -559,12 +521,19 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         }
         if (turn) {
           asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
-          for (int i = half; i < 32 && 32 * q + i < n_tok; i += 2) {
-            float* dst = A.rank_accum + static_cast<int64_t>(item.tok[32 * q + i]) * rank_out;
-            const float* row = tbuf + i * rank_out;
-            for (int c = lane; c < rank_out >> 2; c += 32) {
-              const float4 x = *reinterpret_cast<const float4*>(row + 4 * (c ^ (i & 7)));
-              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * c), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
+          const int rows = min(32, n_tok - 32 * q), pieces = rank_out >> 2;
+          for (int i0 = half; i0 < rows; i0 += 8) {            // four rows in flight
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int i = i0 + 2 * j;
+              if (i >= rows) break;
+              float* dst = A.rank_accum + static_cast<int64_t>(item.tok[32 * q + i]) * rank_out;
+              const float* row = tbuf + i * rank_out;
+#pragma unroll 2
+              for (int c = lane; c < pieces; c += 32) {
+                const float4 x = *reinterpret_cast<const float4*>(row + 4 * (c ^ (i & 7)));
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * c), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
+              }
             }
           }
         }
@@ -584,11 +553,13 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++item_round) {
       __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
       const XtItem& item = items[item_round & 1];
-      const FastExpert& fe = item.fe;
+      if (!item.ok) break;
+      const unsigned char* tab = sm.tab + (item_round & 1) * lay.bytes;
+      const FastExpert& fe = reinterpret_cast<const TokTabHead*>(tab)->fe;
       const int chunk0 = item.chunk0, nchunk = item.nchunk;
       const int nblk_d = fe.m[2].nslots >> 4;
       const int n_mt = (nblk_d + 7) >> 3;   // 128-slot tiles of the down product (<= 3)
-      stage_item(item);
+      stage_item(item, tab);
       // ------------------------------------------------------------------ converters
       // Team 0 (four warps) feeds pipeline 0, team 1 pipeline 1; a team's warps take its stages in turn.  Step t of an item:
       // a stage per 32 slots of chunk t's gate (up) product, then four stages (64 slots x 32 columns) per 128-slot tile
@@ -597,11 +568,11 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       // blocks, one barrier wait, one proxy fence and one arrival per 2048 codes; six warps per team cover one another's loads.
       const int dw = warp - XT_DQ_WARP0;
       const int team = dw / XT_TEAM, wt = dw - team * XT_TEAM, g = lane >> 2, t4 = lane & 3;
-      unsigned char* ring = sm.ring + team * ring_h * XT_STAGE_BYTES + t4 * XT_W_STRIDE + g * 16;
+      unsigned char* ring = sm.ring + team * ring_h * XT_SLOT_BYTES + (wt & 1) * XT_STAGE_BYTES + t4 * XT_W_STRIDE + g * 16;
       uint64_t* w_full = &bars.w_full[team * ring_h];
       uint64_t* w_empty = &bars.w_empty[team * ring_h];
       // everything about the expert in registers: the barriers' memory clobbers would have it read again every stage
-      const int npairs = fe.m[team].nslots >> 5, nib_pairs = fe.m[team].nblk[0] >> 1, nib_d = fe.m[2].nblk[0];
+      const int npairs = fe.m[team].nslots >> 5, n_gu = (npairs + 1) & ~1, nib_pairs = fe.m[team].nblk[0] >> 1, nib_d = fe.m[2].nblk[0];
       const int n_d = team < n_mt ? 4 * ((n_mt - team + 1) >> 1) : 0;
       const int unit_bytes = fe.unit_bytes;
       const unsigned char* unit0 = A.arena + fe.unit_base;
@@ -610,7 +581,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       const unsigned char* scale_d = unit0 + fe.sec_off[2] + g * 4;
       const unsigned char* words_d = unit0 + fe.sec_off[5];
       auto fetch = [&](int t, int i, XtPre& p) {
-        if (t < nchunk && i < npairs) {
+        if (t < nchunk && i < n_gu) {
+          if (i >= npairs) return;         // an odd last stage has an empty partner in its slot
           const int ch = chunk0 + t;
           const int64_t tile = static_cast<int64_t>(ch >> 1) * unit_bytes;
           p.s = __ldg(reinterpret_cast<const uint4*>(scale_gu + tile + i * 64));
@@ -624,7 +596,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             for (int x = 0; x < 4; ++x) p.w[x].x = __ldg(w + x * 32);
           }
         } else {
-          const int j = t < nchunk ? i - npairs : i, ch = chunk0 + t - lag;
+          const int j = t < nchunk ? i - n_gu : i, ch = chunk0 + t - lag;
           const int64_t tile = static_cast<int64_t>(ch >> 1) * unit_bytes;
           const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * ((j >> 1) & 1), pr = 2 * (ch & 1) + (j & 1);
           uint32_t* ps = reinterpret_cast<uint32_t*>(&p.s);
@@ -639,11 +611,12 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         }
       };
       XtCycle my_c = ring_c;
-      my_c.advance(wt, ring_h);
+      my_c.advance(wt >> 1, ring_h);
       auto convert = [&](int t, int i, const XtPre& p) -> bool {
         if (!xt_wait(&w_empty[my_c.i], my_c.ph ^ 1, abort_flag)) return false;
-        unsigned char* dst = ring + my_c.i * XT_STAGE_BYTES;
-        if (t < nchunk && i < npairs) {
+        unsigned char* dst = ring + my_c.i * XT_SLOT_BYTES;
+        if (t < nchunk && i < n_gu) {
+          if (i >= npairs) return true;
           const __half2* sp = reinterpret_cast<const __half2*>(&p.s);
           const __half2 sc[4] = {sp[0], sp[1], sp[2], sp[3]};
           if (i < nib_pairs) {
@@ -654,7 +627,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             for (int x = 0; x < 4; ++x) dequant_pair_store<true>(p.w[x].x, p.w[x].x >> 8, sc, sc, dst + x * 256);
           }
         } else {
-          const int j = t < nchunk ? i - npairs : i;
+          const int j = t < nchunk ? i - n_gu : i;
           const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * ((j >> 1) & 1);
           const __half2* sp = reinterpret_cast<const __half2*>(&p.s);
 #pragma unroll
@@ -672,13 +645,13 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         tc::fence_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&w_full[my_c.i]);
-        my_c.i += XT_TEAM;                   // ring_h >= XT_TEAM: at most one wrap
+        my_c.i += XT_TEAM / 2;               // ring_h >= XT_TEAM / 2: at most one wrap
         if (my_c.i >= static_cast<uint32_t>(ring_h)) { my_c.i -= ring_h; my_c.ph ^= 1u; }
       };
       // this warp's stage after (t, i); false past its last one
       auto step = [&](int& t, int& i) -> bool {
         i += XT_TEAM;
-        for (int n = (t < nchunk ? npairs : 0) + (t >= lag ? n_d : 0); t < nchunk + lag && i >= n; n = (t < nchunk ? npairs : 0) + n_d) {
+        for (int n = (t < nchunk ? n_gu : 0) + (t >= lag ? n_d : 0); t < nchunk + lag && i >= n; n = (t < nchunk ? n_gu : 0) + n_d) {
           i -= n;
           ++t;
         }
@@ -694,7 +667,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         if (more) fetch(t, i, p);           // on its way while the converted stage is published and the next one is waited for
         publish();
       }
-      ring_c.advance(nchunk * (npairs + n_d), ring_h);
+      ring_c.advance(nchunk * (n_gu + n_d) / 2, ring_h);
     }
     __syncthreads();
     return;
@@ -704,21 +677,23 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++item_round) {
       __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
       const XtItem& item = items[item_round & 1];
-      const FastExpert& fe = item.fe;
+      if (!item.ok) break;
+      const unsigned char* tab = sm.tab + (item_round & 1) * lay.bytes;
+      const FastExpert& fe = reinterpret_cast<const TokTabHead*>(tab)->fe;
       const int nchunk = item.nchunk;
       const int nblk_d = fe.m[2].nslots >> 4;
       const int n_mt = (nblk_d + 7) >> 3;   // 128-slot tiles of the down product (<= 3)
       if (warp == XT_LOOKUP_WARP) {
         // ------------------------------------------------------------------ the next item, while this one runs
         if (u + static_cast<int>(gridDim.x) < units.n_units) {
-          XtItem& nx = items[(item_round + 1) & 1];
-          xt_load_item(nx, sm, (item_round + 1) & 1, u + gridDim.x, units, n_chunks, A, lane);
-          __syncwarp();
+          load_item(item_round + 1, u + gridDim.x);
+          const XtItem& nx = items[(item_round + 1) & 1];
+          const FastExpert& nfe = reinterpret_cast<const TokTabHead*>(sm.tab + ((item_round + 1) & 1) * lay.bytes)->fe;
           // its weights on their way to L2, one tile per lane (sizes and offsets are multiples of 16 bytes)
           const int t0 = nx.chunk0 >> 1, t1 = (nx.chunk0 + nx.nchunk + 1) >> 1;
-          for (int t = t0 + lane; t < t1; t += 32)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A.arena + nx.fe.unit_base + static_cast<int64_t>(t) * nx.fe.unit_bytes),
-                         "r"(nx.fe.unit_bytes)
+          for (int t = t0 + lane; t < t1 && nx.ok; t += 32)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A.arena + nfe.unit_base + static_cast<int64_t>(t) * nfe.unit_bytes),
+                         "r"(nfe.unit_bytes)
                          : "memory");
         }
       } else if (warp < XT_MMA_WARP0 + 2) {
@@ -730,18 +705,22 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         tc::fence_after_sync();
         // descriptors: constant upper part, start-address field advanced per block
         const uint64_t a_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.act) + pl * act_m_bytes, cs, 128);
-          const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring_h * XT_STAGE_BYTES;
+          const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring_h * XT_SLOT_BYTES;
         const uint64_t b_desc = tc::smem_desc_kmajor(ring0, XT_W_STRIDE, 128);
         uint64_t* w_full = &bars.w_full[pl * ring_h];
         uint64_t* w_empty = &bars.w_empty[pl * ring_h];
         const int npairs = fe.m[pl].nslots >> 5;
-        // the two MMAs of the next stage: `issue(b_desc, second)` with the stage's operand
-        auto on_stage = [&](auto&& issue) -> bool {
+        // the MMAs of the next slot: two per stage, `n` stages (1 or 2); issue(stage, K half, weight descriptor)
+        auto on_slot = [&](int n, auto&& issue) -> bool {
           if (!xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag)) return false;
           if (tc::elect_one()) {
-            const uint64_t bd = b_desc + ((ring_c.i * XT_STAGE_BYTES) >> 4);
-            issue(bd, 0u);
-            issue(bd + ((2 * XT_W_STRIDE) >> 4), 1u);
+            const uint64_t bd = b_desc + ((ring_c.i * XT_SLOT_BYTES) >> 4);
+            issue(0u, 0u, bd);
+            issue(0u, 1u, bd + ((2 * XT_W_STRIDE) >> 4));
+            if (n > 1) {
+              issue(1u, 0u, bd + (XT_STAGE_BYTES >> 4));
+              issue(1u, 1u, bd + ((XT_STAGE_BYTES + 2 * XT_W_STRIDE) >> 4));
+            }
             tc::mma_commit(&w_empty[ring_c.i]);
           }
           __syncwarp();
@@ -754,9 +733,12 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             if (k >= 1) ok = xt_wait(&bars.z_free[b], (k - 1) & 1, abort_flag);   // the z that took this accumulator's place is consumed
             tc::fence_after_sync();
             const uint32_t d_acc = tmem_base + (2 * b + pl) * XT_CHUNK;
-            for (int pr = 0; pr < npairs && ok; ++pr) {
+            for (int pr = 0; pr < npairs && ok; pr += 2) {
               const uint64_t ad = a_desc + ((4 * pr * cs) >> 4);
-              ok = on_stage([&](uint64_t bd, uint32_t j) { tc::mma_f16(d_acc, ad + ((j * 2 * cs) >> 4), bd, idesc, (pr > 0 ? 1u : 0u) | j); });
+              const uint32_t add = pr > 0 ? 1u : 0u;
+              ok = on_slot(npairs - pr, [&](uint32_t st, uint32_t j, uint64_t bd) {
+                tc::mma_f16(d_acc, ad + (((2 * st + j) * 2 * cs) >> 4), bd, idesc, add | st | j);
+              });
             }
             if (!ok) break;
             if (tc::elect_one()) tc::mma_commit(&bars.gu_done[b]);
@@ -766,12 +748,13 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             const uint32_t g = gu_round + t - lag, b = lag ? g & 1u : 0u;
             ok = xt_wait(&bars.z_ready[b], (lag ? g >> 1 : g) & 1, abort_flag);
             tc::fence_after_sync();
-            // 64 slots and 32 columns of z (16 tensor-memory columns, at the start of the half they came from) per stage
+            // per slot: 64 weight slots and the chunk's 64 columns of z, 32 per stage (16 tensor-memory columns, at the start
+            // of the half they came from)
             for (int mt = pl; mt < n_mt && ok; mt += 2)
-              for (int q = 0; q < 4 && ok; ++q) {
-                const uint32_t d_acc = d_down + mt * 128 + (q >> 1) * 64, za = tmem_base + 2 * b * XT_CHUNK + (q & 1) * 32;
-                const uint32_t add = t > lag || (q & 1) ? 1u : 0u;
-                ok = on_stage([&](uint64_t bd, uint32_t j) { tc::mma_f16_ta(d_acc, za + 8 * j, bd, idesc, add | j); });
+              for (int q = 0; q < 2 && ok; ++q) {
+                const uint32_t d_acc = d_down + mt * 128 + q * 64, za = tmem_base + 2 * b * XT_CHUNK;
+                const uint32_t add = t > lag ? 1u : 0u;
+                ok = on_slot(2, [&](uint32_t st, uint32_t j, uint64_t bd) { tc::mma_f16_ta(d_acc, za + 32 * st + 8 * j, bd, idesc, add | st | j); });
               }
             if (ok && tc::elect_one()) {
               tc::mma_commit(&bars.z_free[b]);
@@ -792,14 +775,14 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
 // matrix) and stages fit shared memory.  Tensor memory holds 128 columns per gate/up buffer and 128 per 128
 // slots of the down product.
 struct XtPlan { int nt, ring_h, gu_bufs; size_t smem; };
-constexpr size_t XT_SMEM_LIMIT = 227 * 1024 - 8192;     // dynamic part: the static part (two item descriptions, barriers) stays below 8 KB
+constexpr size_t XT_SMEM_LIMIT = 227 * 1024 - 3072;     // dynamic part: the static part (two item descriptions, barriers) stays below 3 KB
 static bool xt_plan(const bm_layer* L, XtPlan* out) {
-  if (L->num_experts > XT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > 3 * 128) return false;
+  if (!L->toktab_dev || L->num_experts > XT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > 3 * 128) return false;
   const int n_mt = (L->max_slots + 127) / 128;
   static const int cand[] = {128, 112, 96, 80, 64, 48, 32, 16};
   for (const int nt : cand) {
-    for (int ring = XT_RING_MAX; ring >= XT_TEAM; --ring) {
-      const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, L->rank_in, nt, ring);
+    for (int ring = XT_RING_MAX; ring >= XT_TEAM / 2; --ring) {
+      const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, TokTab(L->rank_in, L->max_slots).bytes, nt, ring);
       if (smem <= XT_SMEM_LIMIT) {
         *out = XtPlan{nt, ring, n_mt > 2 ? 1 : 2, smem};
         return true;
@@ -840,7 +823,8 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
     attr_once.mark(dev);
   }
   XtArgs a{};
-  a.fast = L->fast_dev;
+  a.toktab = L->toktab_dev;
+  a.tab_bytes = TokTab(L->rank_in, L->max_slots).bytes;
   a.arena = static_cast<const unsigned char*>(L->arena);
   a.h_gate = h_gate; a.h_up = h_up; a.h_rank = L->rank_in;
   a.token_indices = token_indices; a.expert_offsets = expert_offsets; a.route_w = route_w;
