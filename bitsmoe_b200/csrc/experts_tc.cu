@@ -50,16 +50,21 @@ constexpr int XT_RING_MAX = 5;            // operand slots per pipeline (at most
 constexpr int XT_W_STRIDE = 64 * 16 + 32;
 constexpr int XT_STAGE_BYTES = 4 * XT_W_STRIDE;
 constexpr int XT_SLOT_BYTES = 2 * XT_STAGE_BYTES;     // the MMA issuers take two stages per barrier
+constexpr int XT_D_STRIDE = 128 * 16 + 32;            // a slot of the down product: 128 rows x 32 positions
+static_assert(4 * XT_D_STRIDE <= XT_SLOT_BYTES, "a down slot fits");
+constexpr int XT_Z_STRIDE = 128 * 16 + 16;            // z operand: 128 rows x 64 positions
+constexpr int XT_Z_BYTES = (XT_CHUNK / 8) * XT_Z_STRIDE;
 // bytes between 8-position chunks of the token-side operands (padded: conflict-free stores)
 __host__ __device__ constexpr int xt_chunk_stride(int nt) { return nt * 16 + 16; }
 constexpr int XT_MAX_E = 1024;
 
 struct XtBars {
-  uint64_t w_full[2 * XT_RING_MAX], w_empty[2 * XT_RING_MAX];
-  uint64_t act_ready, down_done;
-  uint64_t tab[2];                        // an item's token-side table has landed
-  // per gate/up accumulator pair: products complete, z written over the gate half, z consumed by the down product
-  uint64_t gu_done[2], z_ready[2], z_free[2];
+  uint64_t w_full[2 * XT_RING_MAX], w_empty[2 * XT_RING_MAX];     // weight slots of the pipelines
+  uint64_t item_full[2], item_free[2];    // an item's description and table are there / no role needs them any more
+  uint64_t act_ready, act_free;           // activation operand written / every product with it complete
+  uint64_t gu_done[2], gu_free[2];        // gate/up accumulators of a chunk complete / read out
+  uint64_t z_ready, z_free;               // z operand of a chunk written / multiplied
+  uint64_t down_done, down_free;          // down sums of an item complete / read out
 };
 
 // Position in a cyclic buffer of n slots with the phase bit of its mbarriers.
@@ -79,7 +84,7 @@ struct XtItem {
   int tok[XT_NT_MAX];
   float rw[XT_NT_MAX];
   int n, chunk0, nchunk;
-  int ok;                                 // the table has landed
+  int pad_;
 };
 
 __device__ __forceinline__ bool xt_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
@@ -158,7 +163,8 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
 
 struct XtSmem {
   unsigned char* act;     // [2][nchunks][nt rows] canonical K-major, 16-byte chunks
-  unsigned char* ring;    // [2 pipelines][ring_h][XT_STAGE_BYTES]
+  unsigned char* z;       // [8 chunks][128 rows]; at the end of an item each epilogue warp's part turns the sums
+  unsigned char* ring;    // [2 pipelines][ring_h][XT_SLOT_BYTES]
   int* prefix;            // [E + 1] items before each expert
   int* offset;            // [E + 1] assignments before each expert
   unsigned char* tab;     // [2 items] token-side table of the item's expert (TokTab)
@@ -166,7 +172,7 @@ struct XtSmem {
 
 __host__ __device__ inline size_t xt_act_bytes(int max_slots, int nt) { return static_cast<size_t>(2) * (max_slots / 8) * xt_chunk_stride(nt); }
 __host__ __device__ inline size_t xt_smem_bytes(int max_slots, int num_experts, int tab_bytes, int nt, int ring_h) {
-  size_t o = align_up_c(xt_act_bytes(max_slots, nt), 128);
+  size_t o = align_up_c(xt_act_bytes(max_slots, nt), 128) + XT_Z_BYTES;
   o += static_cast<size_t>(2 * ring_h) * XT_SLOT_BYTES;
   o += align_up_c(static_cast<size_t>(2 * num_experts + 2) * 4, 128);     // items and assignments before each expert
   o += static_cast<size_t>(2) * tab_bytes;
@@ -260,14 +266,16 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   volatile int* abort_flag = &abort_flag_s;
   const int warp = tc::warp_index(), lane = threadIdx.x & 31;
   const int nt = A.nt, ring_h = A.ring_h, h_rank = A.h_rank, num_experts = A.num_experts;
-  const int cs = xt_chunk_stride(nt);     // bytes between 8-position chunks of act / z
+  const int cs = xt_chunk_stride(nt);     // bytes between 8-position chunks of act
   const int n_chunks = A.n_tiles * (N_TILE / XT_CHUNK);
   const uint32_t act_m_bytes = static_cast<uint32_t>(A.max_slots / 8) * cs;
+  const TokTab lay(h_rank, A.max_slots);
   XtSmem sm;
   {
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(xt_raw) + 1023) & ~static_cast<uintptr_t>(1023));
     sm.act = base;
     size_t o = align_up_c(xt_act_bytes(A.max_slots, nt), 128);
+    sm.z = base + o; o += XT_Z_BYTES;
     sm.ring = base + o; o += static_cast<size_t>(2 * ring_h) * XT_SLOT_BYTES;
     sm.prefix = reinterpret_cast<int*>(base + o);
     sm.offset = sm.prefix + num_experts + 1;
@@ -276,13 +284,17 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   }
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2 * XT_RING_MAX; ++i) { tc::mbar_init(&bars.w_full[i], 2); tc::mbar_init(&bars.w_empty[i], 1); }
-    tc::mbar_init(&bars.act_ready, 1);
+    tc::mbar_init(&bars.act_ready, XT_DQ_WARPS);
+    tc::mbar_init(&bars.act_free, 2);
     tc::mbar_init(&bars.down_done, 2);
+    tc::mbar_init(&bars.down_free, XT_EPI_WARPS);
+    tc::mbar_init(&bars.z_ready, XT_EPI_WARPS);
+    tc::mbar_init(&bars.z_free, 2);
     for (int i = 0; i < 2; ++i) {
-      tc::mbar_init(&bars.tab[i], 1);
+      tc::mbar_init(&bars.item_full[i], 2);
+      tc::mbar_init(&bars.item_free[i], XT_EPI_WARPS + XT_DQ_WARPS + 2);
       tc::mbar_init(&bars.gu_done[i], 2);
-      tc::mbar_init(&bars.z_ready[i], XT_EPI_WARPS);
-      tc::mbar_init(&bars.z_free[i], 2);
+      tc::mbar_init(&bars.gu_free[i], XT_EPI_WARPS);
     }
     tc::mbar_init_fence();
     abort_flag_s = 0;
@@ -321,132 +333,43 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   const uint32_t d_down = tmem_base + A.gu_bufs * 2 * XT_CHUNK;
   // the down product of a chunk is issued `lag` chunks late: one where tensor memory holds two gate/up accumulator pairs
   const int lag = A.gu_bufs - 1;
-  const TokTab lay(h_rank, A.max_slots);
-  // item number `round` of this CTA into its buffers; waits for its table, so that the barrier at the item's start
-  // publishes everything
-  auto load_item = [&](uint32_t round, int u) {
-    const uint32_t buf = round & 1u;
-    xt_load_item(items[buf], sm.tab + buf * lay.bytes, &bars.tab[buf], u, units, n_chunks, sm, A, lane);
-    const bool landed = xt_wait(&bars.tab[buf], (round >> 1) & 1u, abort_flag);
-    if (lane == 0) items[buf].ok = landed;
-    __syncwarp();
-  };
-  if (warp == XT_LOOKUP_WARP && static_cast<int>(blockIdx.x) < units.n_units)
-    load_item(0, blockIdx.x);
 
-  // Positions in the cyclic buffers; every role steps through the same sequence of stages and chunks, so each keeps its
-  // own copy across items.
-  XtCycle ring_c{0, 0};     // this pipeline's operand stages (converter team / its MMA issuer)
-  uint32_t gu_round = 0;    // chunks so far: chunk number g uses z buffer g & 1 for the (g >> 1)-th time
-  uint32_t item_round = 0;
-
-  // Activation operand of an item, once per item, by the epilogue and converter warps.
-  auto stage_item = [&](const XtItem& item, const unsigned char* tab) {
-    const TokTabHead& head = *reinterpret_cast<const TokTabHead*>(tab);
-    const FastExpert& fe = head.fe;
-    const int n_tok = item.n;
-    constexpr int XT_STAGERS = (XT_EPI_WARPS + XT_DQ_WARPS) * 32;
-    const int tid_s = threadIdx.x, warp_s = warp;
-    // act[m][chunk][n] = 8 consecutive contraction positions of token n: fp16(h[token, rank(slot)] * s(slot)).
-    // A warp takes tokens; a lane owns an octet of ranks, which the arena layout keeps together: one 16-byte load, four
-    // multiplications, one 16-byte store (pieces of one row are 16 bytes apart modulo 128: no bank conflicts).  Octets
-    // that straddle two groups of rows follow rank by rank.  Operand rows past the item's tokens keep whatever they
-    // hold: they only reach accumulator rows that nobody reads.
-    const int n_oct = h_rank >> 3;
-    const int16_t* pos_r = reinterpret_cast<const int16_t*>(tab + lay.pos_r);
-    const __half* s_r = reinterpret_cast<const __half*>(tab + lay.s_r);
-    const int16_t* oct_r = reinterpret_cast<const int16_t*>(tab + lay.oct_r);
-    for (int o0 = 0; o0 < n_oct; o0 += 32) {
-      const int o = o0 + lane;
-      int dst[2];
-      uint4 sc[2];
-#pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const int c = o < n_oct ? oct_r[m * n_oct + o] : -1;
-        dst[m] = c < 0 ? -1 : static_cast<int>(m * act_m_bytes) + c * cs;
-        sc[m] = c < 0 ? make_uint4(0u, 0u, 0u, 0u) : *reinterpret_cast<const uint4*>(s_r + m * h_rank + 8 * o);
-      }
-      for (int n0 = warp_s; n0 < n_tok; n0 += 4 * (XT_STAGERS / 32)) {
-        uint4 hv[4][2];                     // four tokens per round: eight loads in flight per lane
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int n = min(n0 + j * (XT_STAGERS / 32), n_tok - 1);
-          const int64_t row = static_cast<int64_t>(item.tok[n]) * h_rank + 8 * o;
-#pragma unroll
-          for (int m = 0; m < 2; ++m)
-            if (dst[m] >= 0) hv[j][m] = __ldg(reinterpret_cast<const uint4*>((m ? A.h_up : A.h_gate) + row));
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int n = n0 + j * (XT_STAGERS / 32);
-          if (n >= n_tok) break;
-#pragma unroll
-          for (int m = 0; m < 2; ++m)
-            if (dst[m] >= 0) {
-              uint4 r;
-              const __half2 *hp = reinterpret_cast<const __half2*>(&hv[j][m]), *sp = reinterpret_cast<const __half2*>(&sc[m]);
-              __half2* rp = reinterpret_cast<__half2*>(&r);
-#pragma unroll
-              for (int q = 0; q < 4; ++q) rp[q] = __hmul2(hp[q], sp[q]);       // one rounding of the exact product
-              *reinterpret_cast<uint4*>(sm.act + dst[m] + n * 16) = r;
-            }
-        }
-      }
-    }
-    for (int m = 0; m < 2; ++m)
-      for (int w = 0; w < (n_oct + 31) >> 5; ++w)
-        for (uint32_t left = head.broken[m][w]; left; left &= left - 1) {
-          const int o = 32 * w + __ffs(left) - 1;
-          for (int i = tid_s; i < 8 * n_tok; i += XT_STAGERS) {
-            const int n = i >> 3, rk = 8 * o + (i & 7), pos = pos_r[m * h_rank + rk];
-            if (pos >= 0)
-              *reinterpret_cast<__half*>(sm.act + m * act_m_bytes + (pos >> 3) * cs + (pos & 7) * 2 + n * 16) =
-                  __hmul((m ? A.h_up : A.h_gate)[static_cast<int64_t>(item.tok[n]) * h_rank + rk], s_r[m * h_rank + rk]);
-          }
-        }
-    if (head.padded) {        // padding slots: their weights are zero, their activations have to be finite
-      for (int m = 0; m < 2; ++m) {
-        const int16_t* rank_t = reinterpret_cast<const int16_t*>(A.arena + fe.m[m].tab_off);
-        for (int i = warp_s; i < fe.m[m].nslots; i += XT_STAGERS / 32) {
-          const int rk = rank_t[i], pos = slot_pos(i);
-          if (rk >= 0 && rk < h_rank) continue;
-          for (int n = lane; n < n_tok; n += 32)
-            *reinterpret_cast<__half*>(sm.act + m * act_m_bytes + (pos >> 3) * cs + (pos & 7) * 2 + n * 16) = __float2half(0.f);
-        }
-      }
-    }
-    tc::fence_async_smem();
-    asm volatile("bar.sync 1, %0;" ::"n"(XT_STAGERS) : "memory");
-    if (tid_s == 0) tc::mbar_arrive(&bars.act_ready);
-  };
+  // The roles run through this CTA's items independently; what they share is guarded by barriers only.  Item number
+  // `round` uses description and table buffer round & 1.  After a wait that gave up, every further wait gives up too.
+  uint32_t round = 0;
+  uint32_t gu_round = 0;    // chunks so far
+#define XT_ITEM_BEGIN                                                                                        \
+  const uint32_t ib = round & 1u;                                                                            \
+  if (!xt_wait(&bars.item_full[ib], (round >> 1) & 1u, abort_flag)) break;                                   \
+  const XtItem& item = items[ib];                                                                            \
+  const unsigned char* tab = sm.tab + ib * lay.bytes;                                                        \
+  const TokTabHead& head = *reinterpret_cast<const TokTabHead*>(tab);                                        \
+  const FastExpert& fe = head.fe;                                                                            \
+  const int nchunk = item.nchunk;
 
   if (warp < XT_EPI_WARPS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XT_REGS_EPI));
-    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++item_round) {
-      __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
-      const XtItem& item = items[item_round & 1];
-      if (!item.ok) break;
-      const unsigned char* tab = sm.tab + (item_round & 1) * lay.bytes;
-      const FastExpert& fe = reinterpret_cast<const TokTabHead*>(tab)->fe;
-      const int n_tok = item.n, nchunk = item.nchunk;
-      stage_item(item, tab);
-      // ------------------------------------------------------------------ epilogue warps 0-7
-      // warp = (TMEM lane quarter q: tokens 32 q .. 32 q + 31, half of the chunk's 64 columns); a thread owns a token
-      const int q = warp & 3, half = warp >> 2;
-      const uint32_t lane_sel = static_cast<uint32_t>(32 * q) << 16;
-      const int n = 32 * q + lane;
+    // -------------------------------------------------------------------- epilogue
+    // warp = (TMEM lane quarter q: tokens 32 q .. 32 q + 31, half of the chunk's 64 columns); a thread owns a token.
+    // Its part of the z operand -- four chunks of 32 rows -- is written and reused by this warp alone.
+    const int q = warp & 3, half = warp >> 2, n = 32 * q + lane;
+    const uint32_t lane_sel = static_cast<uint32_t>(32 * q) << 16;
+    unsigned char* zpart = sm.z + 4 * half * XT_Z_STRIDE + 32 * q * 16;
+    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++round) {
+      XT_ITEM_BEGIN
+      const int n_tok = item.n;
       const bool busy = 32 * q < n_tok;                               // any token in this quarter
       bool ok = true;
       for (int t = 0; t < nchunk && ok; ++t) {
-        const uint32_t gt = gu_round + t, b = lag ? gt & 1u : 0u;
-        ok = xt_wait(&bars.gu_done[b], (lag ? gt >> 1 : gt) & 1, abort_flag);
+        const uint32_t g = gu_round + t, b = lag ? g & 1u : 0u;
+        ok = xt_wait(&bars.gu_done[b], (lag ? g >> 1 : g) & 1u, abort_flag);
         if (!ok) break;
         tc::fence_after_sync();
+        // z in the contraction order of the down weights (pos32): 16-byte piece c holds columns 2c, 2c+1, 2c+8, 2c+9 of
+        // both blocks of 16
+        uint32_t zp[16];
         if (busy) {
           const uint32_t d_gate = tmem_base + 2 * b * XT_CHUNK + lane_sel + 32 * half, d_up = d_gate + XT_CHUNK;
-          // z in the contraction order of the down weights (pos32): 16-byte piece c holds columns 2c, 2c+1, 2c+8, 2c+9 of
-          // both blocks of 16
-          uint32_t zp[16];
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {          // 16 columns at a time: 32 of both would hold 64 registers
             float gv[16], uv[16];
@@ -458,41 +381,33 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
               zp[4 * (i & 3) + 2 * hh + (i >> 2)] = *reinterpret_cast<const uint32_t*>(&h2);
             }
           }
-          tc::tmem_st16(d_gate, zp);                // over the gate values this warp has just read
         }
         tc::fence_before_sync();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&bars.z_ready[b]);
+        if (lane == 0) tc::mbar_arrive(&bars.gu_free[b]);
+        if (g >= 1) ok = xt_wait(&bars.z_free, (g - 1) & 1u, abort_flag);     // the chunk before is multiplied
+        if (busy) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            *reinterpret_cast<uint4*>(zpart + c * XT_Z_STRIDE + lane * 16) = make_uint4(zp[4 * c], zp[4 * c + 1], zp[4 * c + 2], zp[4 * c + 3]);
+          tc::fence_async_smem();
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&bars.z_ready);
       }
-      if (ok) ok = xt_wait(&bars.down_done, item_round & 1, abort_flag);
-      if (busy) {                      // both warps of the quarter go on or neither: they meet at barriers below
-        uint32_t both;
-        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.and.aligned.pred q, %2, 64, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-                     : "=r"(both)
-                     : "r"(static_cast<uint32_t>(ok)), "r"(2 + q)
-                     : "memory");
-        ok = both != 0;
-      }
+      gu_round += nchunk;
+      if (ok) ok = xt_wait(&bars.down_done, round & 1u, abort_flag);
       if (ok && busy) {
         tc::fence_after_sync();
-        const int rank_out = A.rank_out;
-        const float rw = n < n_tok ? item.rw[n] : 0.f;
-        // A thread owns a token: adding straight from the registers costs a 32-byte sector per lane and instruction.  The
-        // quarter's two warps turn their 32 tokens x rank_out sums through the idle activation area, 16 bytes at a time
-        // where eight slots hold an aligned octet of ranks (piece index XORed with the token: conflict-free both ways),
-        // and add whole rows, 16 bytes per lane; ranks without a slot add zero.
-        const bool turn = A.acc64 == nullptr && (rank_out & 31) == 0 &&
-                          static_cast<size_t>((nt + 31) / 32) * 32 * rank_out * 4 <= xt_act_bytes(A.max_slots, nt);
-        float* tbuf = reinterpret_cast<float*>(sm.act) + q * 32 * rank_out;
-        float* trow = tbuf + lane * rank_out;
-        const int x7 = lane & 7;
-        if (turn && !reinterpret_cast<const TokTabHead*>(tab)->all_ranks) {
-          for (int i = half * 32 + lane; i < 8 * rank_out; i += 64) reinterpret_cast<float4*>(tbuf)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-          asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
-        }
-        const int nslots_d = fe.m[2].nslots;
+        const int rank_out = A.rank_out, nslots_d = fe.m[2].nslots;
         const float* s_d = reinterpret_cast<const float*>(tab + lay.s_d);
         const int16_t *rank_d = reinterpret_cast<const int16_t*>(tab + lay.rank_d), *oct_d = reinterpret_cast<const int16_t*>(tab + lay.oct_d);
+        const float rw = n < n_tok ? item.rw[n] : 0.f;
+        const int rows = min(32, n_tok - 32 * q);
+        // D_d * s * route weight -> rank_accum.  A thread owns a token: adding straight from the registers would touch a
+        // 32-byte sector per lane and instruction.  Sixteen slots at a time go through the warp's part of the (now idle) z
+        // area, so that an instruction adds the 64 bytes of eight tokens.  Octets of slots that are not an aligned octet
+        // of ranks, and the deterministic mode, add from the registers.
         for (int s0 = 16 * half; s0 < nslots_d; s0 += 32) {
           float v[16];
           tc::tmem_ld16(d_down + lane_sel + s0, v);
@@ -501,45 +416,47 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             const float4 sv = *reinterpret_cast<const float4*>(s_d + s0 + i);
             v[i] *= sv.x * rw; v[i + 1] *= sv.y * rw; v[i + 2] *= sv.z * rw; v[i + 3] *= sv.w * rw;
           }
+          int oct[2];
+          oct[0] = A.acc64 ? -1 : oct_d[s0 >> 3];
+          oct[1] = A.acc64 ? -1 : oct_d[(s0 >> 3) + 1];
+          __syncwarp();                            // the pieces of the sixteen slots before have been read
 #pragma unroll
-          for (int h8 = 0; h8 < 2; ++h8) {
-            const int r0 = oct_d[(s0 >> 3) + h8];
-            const float* w = v + 8 * h8;
-            if (turn && r0 >= 0) {
-              *reinterpret_cast<float4*>(trow + 4 * ((r0 >> 2) ^ x7)) = make_float4(w[0], w[1], w[2], w[3]);
-              *reinterpret_cast<float4*>(trow + 4 * (((r0 >> 2) + 1) ^ x7)) = make_float4(w[4], w[5], w[6], w[7]);
-            } else {
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const int r = rank_d[s0 + 8 * h8 + i];
-                if (r < 0) continue;
-                if (turn) trow[4 * ((r >> 2) ^ x7) + (r & 3)] = w[i];
-                else if (n < n_tok) acc_add(A.rank_accum, A.acc64, static_cast<int64_t>(item.tok[n]) * rank_out + r, w[i]);
-              }
-            }
-          }
-        }
-        if (turn) {
-          asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");
-          const int rows = min(32, n_tok - 32 * q), pieces = rank_out >> 2;
-          for (int i0 = half; i0 < rows; i0 += 8) {            // four rows in flight
+          for (int c = 0; c < 4; ++c)
+            *reinterpret_cast<float4*>(zpart + c * XT_Z_STRIDE + lane * 16) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+          __syncwarp();
+          const int piece = lane >> 3, r0 = oct[piece >> 1];
+          if (r0 >= 0) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const int i = i0 + 2 * j;
-              if (i >= rows) break;
-              float* dst = A.rank_accum + static_cast<int64_t>(item.tok[32 * q + i]) * rank_out;
-              const float* row = tbuf + i * rank_out;
-#pragma unroll 2
-              for (int c = lane; c < pieces; c += 32) {
-                const float4 x = *reinterpret_cast<const float4*>(row + 4 * (c ^ (i & 7)));
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + 4 * c), "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w) : "memory");
-              }
+              const int row = 8 * j + (lane & 7);
+              const float4 x = *reinterpret_cast<const float4*>(zpart + piece * XT_Z_STRIDE + row * 16);
+              if (row < rows)
+                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(A.rank_accum + static_cast<int64_t>(item.tok[32 * q + row]) * rank_out +
+                                                                                   r0 + 4 * (piece & 1)),
+                             "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w)
+                             : "memory");
             }
           }
+#pragma unroll
+          for (int h8 = 0; h8 < 2; ++h8)
+            if (oct[h8] < 0 && n < n_tok) {
+              for (int i = 0; i < 8; ++i) {
+                const int r = rank_d[s0 + 8 * h8 + i];
+                if (r >= 0) {
+                  float val = 0.f;
+#pragma unroll
+                  for (int k = 0; k < 16; ++k) val = k == 8 * h8 + i ? v[k] : val;
+                  acc_add(A.rank_accum, A.acc64, static_cast<int64_t>(item.tok[n]) * rank_out + r, val);
+                }
+              }
+            }
         }
         tc::fence_before_sync();
+        tc::fence_async_smem();
       }
-      gu_round += nchunk;
+      __syncwarp();
+      if (lane == 0) { tc::mbar_arrive(&bars.down_free); tc::mbar_arrive(&bars.item_free[ib]); }
+      if (!ok) break;
     }
     // every role ends on its own (they do not share a register count to come together with)
     tc::fence_before_sync();
@@ -550,28 +467,100 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   }
   if (warp < XT_DQ_WARP0 + XT_DQ_WARPS) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(XT_REGS_DQ));
-    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++item_round) {
-      __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
-      const XtItem& item = items[item_round & 1];
-      if (!item.ok) break;
-      const unsigned char* tab = sm.tab + (item_round & 1) * lay.bytes;
-      const FastExpert& fe = reinterpret_cast<const TokTabHead*>(tab)->fe;
-      const int chunk0 = item.chunk0, nchunk = item.nchunk;
-      const int nblk_d = fe.m[2].nslots >> 4;
-      const int n_mt = (nblk_d + 7) >> 3;   // 128-slot tiles of the down product (<= 3)
-      stage_item(item, tab);
-      // ------------------------------------------------------------------ converters
-      // Team 0 (four warps) feeds pipeline 0, team 1 pipeline 1; a team's warps take its stages in turn.  Step t of an item:
-      // a stage per 32 slots of chunk t's gate (up) product, then four stages (64 slots x 32 columns) per 128-slot tile
-      // of chunk t - 1's down product.  A stage is four 16 x 32 blocks; lane (g, t4) turns its words of each into two
-      // 16-byte pieces.  What bounds a warp is latency, not issue: a whole stage per warp gives it four independent
-      // blocks, one barrier wait, one proxy fence and one arrival per 2048 codes; six warps per team cover one another's loads.
-      const int dw = warp - XT_DQ_WARP0;
-      const int team = dw / XT_TEAM, wt = dw - team * XT_TEAM, g = lane >> 2, t4 = lane & 3;
-      unsigned char* ring = sm.ring + team * ring_h * XT_SLOT_BYTES + (wt & 1) * XT_STAGE_BYTES + t4 * XT_W_STRIDE + g * 16;
-      uint64_t* w_full = &bars.w_full[team * ring_h];
-      uint64_t* w_empty = &bars.w_empty[team * ring_h];
+    // -------------------------------------------------------------------- activation operand and converters
+    // Team 0 (six warps) feeds pipeline 0, team 1 pipeline 1; a team's warps take its stages in turn.  Step t of an item:
+    // a stage per 32 slots of chunk t's gate (up) product, then four stages (64 slots x 32 columns) per 128-slot tile of
+    // chunk t - lag's down product.  Stages 2 i and 2 i + 1 share a ring slot.  A stage is four 16 x 32 blocks; lane
+    // (g, t4) turns its words of each into two 16-byte pieces.  What bounds a warp is latency, not issue: a whole stage per
+    // warp gives it four independent blocks, one barrier wait, one proxy fence and one arrival per 2048 codes.
+    const int dw = warp - XT_DQ_WARP0;
+    const int team = dw / XT_TEAM, wt = dw - team * XT_TEAM, g = lane >> 2, t4 = lane & 3;
+    uint64_t* w_full = &bars.w_full[team * ring_h];
+    uint64_t* w_empty = &bars.w_empty[team * ring_h];
+    unsigned char* ring = sm.ring + team * ring_h * XT_SLOT_BYTES;
+    // where a stage's pieces go: 64-row stages lie one after the other, the two 64-row halves of a down slot share chunks
+    unsigned char* gu_dst = ring + (wt & 1) * XT_STAGE_BYTES + t4 * XT_W_STRIDE + g * 16;
+    unsigned char* dn_dst = ring + (wt & 1) * 1024 + t4 * XT_D_STRIDE + g * 16;
+    XtCycle ring_c{0, 0};
+    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++round) {
+      XT_ITEM_BEGIN
+      if (round > 0 && !xt_wait(&bars.act_free, (round - 1) & 1u, abort_flag)) break;
+      {
+        // act[m][chunk][n] = 8 consecutive contraction positions of token n: fp16(h[token, rank(slot)] * s(slot)).
+        // A warp takes tokens; a lane owns an octet of ranks, which the arena layout keeps together: one 16-byte load, four
+        // multiplications, one 16-byte store (pieces of one row are 16 bytes apart modulo 128: no bank conflicts).  Octets
+        // that straddle two groups of rows follow rank by rank.  Operand rows past the item's tokens keep whatever they
+        // hold: they only reach accumulator rows that nobody reads.
+        const int n_tok = item.n, n_oct = h_rank >> 3;
+        const int16_t* pos_r = reinterpret_cast<const int16_t*>(tab + lay.pos_r);
+        const __half* s_r = reinterpret_cast<const __half*>(tab + lay.s_r);
+        const int16_t* oct_r = reinterpret_cast<const int16_t*>(tab + lay.oct_r);
+        for (int o0 = 0; o0 < n_oct; o0 += 32) {
+          const int o = o0 + lane;
+          int dst[2];
+          uint4 sc[2];
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            const int c = o < n_oct ? oct_r[m * n_oct + o] : -1;
+            dst[m] = c < 0 ? -1 : static_cast<int>(m * act_m_bytes) + c * cs;
+            sc[m] = c < 0 ? make_uint4(0u, 0u, 0u, 0u) : *reinterpret_cast<const uint4*>(s_r + m * h_rank + 8 * o);
+          }
+          for (int n0 = dw; n0 < n_tok; n0 += 4 * XT_DQ_WARPS) {
+            uint4 hv[4][2];                     // four tokens per round: eight loads in flight per lane
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int n = min(n0 + j * XT_DQ_WARPS, n_tok - 1);
+              const int64_t row = static_cast<int64_t>(item.tok[n]) * h_rank + 8 * o;
+#pragma unroll
+              for (int m = 0; m < 2; ++m)
+                if (dst[m] >= 0) hv[j][m] = __ldg(reinterpret_cast<const uint4*>((m ? A.h_up : A.h_gate) + row));
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int n = n0 + j * XT_DQ_WARPS;
+              if (n >= n_tok) break;
+#pragma unroll
+              for (int m = 0; m < 2; ++m)
+                if (dst[m] >= 0) {
+                  uint4 r;
+                  const __half2 *hp = reinterpret_cast<const __half2*>(&hv[j][m]), *sp = reinterpret_cast<const __half2*>(&sc[m]);
+                  __half2* rp = reinterpret_cast<__half2*>(&r);
+#pragma unroll
+                  for (int k = 0; k < 4; ++k) rp[k] = __hmul2(hp[k], sp[k]);       // one rounding of the exact product
+                  *reinterpret_cast<uint4*>(sm.act + dst[m] + n * 16) = r;
+                }
+            }
+          }
+        }
+        const int tid_s = threadIdx.x - XT_DQ_WARP0 * 32;
+        for (int m = 0; m < 2; ++m)
+          for (int w = 0; w < (n_oct + 31) >> 5; ++w)
+            for (uint32_t left = head.broken[m][w]; left; left &= left - 1) {
+              const int o = 32 * w + __ffs(left) - 1;
+              for (int i = tid_s; i < 8 * n_tok; i += XT_DQ_WARPS * 32) {
+                const int n = i >> 3, rk = 8 * o + (i & 7), pos = pos_r[m * h_rank + rk];
+                if (pos >= 0)
+                  *reinterpret_cast<__half*>(sm.act + m * act_m_bytes + (pos >> 3) * cs + (pos & 7) * 2 + n * 16) =
+                      __hmul((m ? A.h_up : A.h_gate)[static_cast<int64_t>(item.tok[n]) * h_rank + rk], s_r[m * h_rank + rk]);
+              }
+            }
+        if (head.padded) {        // padding slots: their weights are zero, their activations have to be finite
+          for (int m = 0; m < 2; ++m) {
+            const int16_t* rank_t = reinterpret_cast<const int16_t*>(A.arena + fe.m[m].tab_off);
+            for (int i = dw; i < fe.m[m].nslots; i += XT_DQ_WARPS) {
+              const int rk = rank_t[i], pos = slot_pos(i);
+              if (rk >= 0 && rk < h_rank) continue;
+              for (int n = lane; n < n_tok; n += 32)
+                *reinterpret_cast<__half*>(sm.act + m * act_m_bytes + (pos >> 3) * cs + (pos & 7) * 2 + n * 16) = __float2half(0.f);
+            }
+          }
+        }
+        tc::fence_async_smem();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&bars.act_ready);
+      }
       // everything about the expert in registers: the barriers' memory clobbers would have it read again every stage
+      const int chunk0 = item.chunk0, nblk_d = fe.m[2].nslots >> 4, n_mt = (nblk_d + 7) >> 3;
       const int npairs = fe.m[team].nslots >> 5, n_gu = (npairs + 1) & ~1, nib_pairs = fe.m[team].nblk[0] >> 1, nib_d = fe.m[2].nblk[0];
       const int n_d = team < n_mt ? 4 * ((n_mt - team + 1) >> 1) : 0;
       const int unit_bytes = fe.unit_bytes;
@@ -580,6 +569,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       const unsigned char* words_gu = unit0 + fe.sec_off[3 + team];
       const unsigned char* scale_d = unit0 + fe.sec_off[2] + g * 4;
       const unsigned char* words_d = unit0 + fe.sec_off[5];
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&bars.item_free[ib]);
       auto fetch = [&](int t, int i, XtPre& p) {
         if (t < nchunk && i < n_gu) {
           if (i >= npairs) return;         // an odd last stage has an empty partner in its slot
@@ -596,9 +587,10 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             for (int x = 0; x < 4; ++x) p.w[x].x = __ldg(w + x * 32);
           }
         } else {
+          // per 128-slot tile: columns 0-31 of the chunk for slots 0-63 and 64-127, then columns 32-63
           const int j = t < nchunk ? i - n_gu : i, ch = chunk0 + t - lag;
           const int64_t tile = static_cast<int64_t>(ch >> 1) * unit_bytes;
-          const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * ((j >> 1) & 1), pr = 2 * (ch & 1) + (j & 1);
+          const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * (j & 1), pr = 2 * (ch & 1) + ((j >> 1) & 1);
           uint32_t* ps = reinterpret_cast<uint32_t*>(&p.s);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
@@ -614,9 +606,9 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       my_c.advance(wt >> 1, ring_h);
       auto convert = [&](int t, int i, const XtPre& p) -> bool {
         if (!xt_wait(&w_empty[my_c.i], my_c.ph ^ 1, abort_flag)) return false;
-        unsigned char* dst = ring + my_c.i * XT_SLOT_BYTES;
         if (t < nchunk && i < n_gu) {
           if (i >= npairs) return true;
+          unsigned char* dst = gu_dst + my_c.i * XT_SLOT_BYTES;
           const __half2* sp = reinterpret_cast<const __half2*>(&p.s);
           const __half2 sc[4] = {sp[0], sp[1], sp[2], sp[3]};
           if (i < nib_pairs) {
@@ -627,8 +619,9 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             for (int x = 0; x < 4; ++x) dequant_pair_store<true>(p.w[x].x, p.w[x].x >> 8, sc, sc, dst + x * 256);
           }
         } else {
+          unsigned char* dst = dn_dst + my_c.i * XT_SLOT_BYTES;
           const int j = t < nchunk ? i - n_gu : i;
-          const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * ((j >> 1) & 1);
+          const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * (j & 1);
           const __half2* sp = reinterpret_cast<const __half2*>(&p.s);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
@@ -659,116 +652,121 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       };
       XtPre p;
       int t = 0, i = wt - XT_TEAM;
-      bool more = step(t, i);
+      bool more = step(t, i), ok = true;
       if (more) fetch(t, i, p);
       while (more) {
-        if (!convert(t, i, p)) break;
+        if (!(ok = convert(t, i, p))) break;
         more = step(t, i);
         if (more) fetch(t, i, p);           // on its way while the converted stage is published and the next one is waited for
         publish();
       }
       ring_c.advance(nchunk * (n_gu + n_d) / 2, ring_h);
+      if (!ok) break;
     }
     __syncthreads();
     return;
   }
-  {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XT_REGS_MISC));
-    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++item_round) {
-      __syncthreads();   // previous item completely finished (TMEM read out), this item's description in place
-      const XtItem& item = items[item_round & 1];
-      if (!item.ok) break;
-      const unsigned char* tab = sm.tab + (item_round & 1) * lay.bytes;
-      const FastExpert& fe = reinterpret_cast<const TokTabHead*>(tab)->fe;
-      const int nchunk = item.nchunk;
-      const int nblk_d = fe.m[2].nslots >> 4;
-      const int n_mt = (nblk_d + 7) >> 3;   // 128-slot tiles of the down product (<= 3)
-      if (warp == XT_LOOKUP_WARP) {
-        // ------------------------------------------------------------------ the next item, while this one runs
-        if (u + static_cast<int>(gridDim.x) < units.n_units) {
-          load_item(item_round + 1, u + gridDim.x);
-          const XtItem& nx = items[(item_round + 1) & 1];
-          const FastExpert& nfe = reinterpret_cast<const TokTabHead*>(sm.tab + ((item_round + 1) & 1) * lay.bytes)->fe;
-          // its weights on their way to L2, one tile per lane (sizes and offsets are multiples of 16 bytes)
-          const int t0 = nx.chunk0 >> 1, t1 = (nx.chunk0 + nx.nchunk + 1) >> 1;
-          for (int t = t0 + lane; t < t1 && nx.ok; t += 32)
-            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A.arena + nfe.unit_base + static_cast<int64_t>(t) * nfe.unit_bytes),
-                         "r"(nfe.unit_bytes)
-                         : "memory");
-        }
-      } else if (warp < XT_MMA_WARP0 + 2) {
-        // ------------------------------------------------------------------ MMA issue, one thread per pipeline
-        // The whole warp waits (a lone waiting lane wakes up several times slower); one issues.
-        const int pl = warp - XT_MMA_WARP0;
-        const uint32_t idesc = tc::idesc_f16(128, 64);
-        bool ok = xt_wait(&bars.act_ready, item_round & 1, abort_flag);
-        tc::fence_after_sync();
-        // descriptors: constant upper part, start-address field advanced per block
-        const uint64_t a_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.act) + pl * act_m_bytes, cs, 128);
-          const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring_h * XT_SLOT_BYTES;
-        const uint64_t b_desc = tc::smem_desc_kmajor(ring0, XT_W_STRIDE, 128);
-        uint64_t* w_full = &bars.w_full[pl * ring_h];
-        uint64_t* w_empty = &bars.w_empty[pl * ring_h];
-        const int npairs = fe.m[pl].nslots >> 5;
-        // the MMAs of the next slot: two per stage, `n` stages (1 or 2); issue(stage, K half, weight descriptor)
-        auto on_slot = [&](int n, auto&& issue) -> bool {
-          if (!xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag)) return false;
-          if (tc::elect_one()) {
-            const uint64_t bd = b_desc + ((ring_c.i * XT_SLOT_BYTES) >> 4);
-            issue(0u, 0u, bd);
-            issue(0u, 1u, bd + ((2 * XT_W_STRIDE) >> 4));
-            if (n > 1) {
-              issue(1u, 0u, bd + (XT_STAGE_BYTES >> 4));
-              issue(1u, 1u, bd + ((XT_STAGE_BYTES + 2 * XT_W_STRIDE) >> 4));
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XT_REGS_MISC));
+  if (warp == XT_LOOKUP_WARP) {
+    // -------------------------------------------------------------------- descriptions, an item ahead of the roles
+    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++round) {
+      const uint32_t ib = round & 1u;
+      if (round >= 2 && !xt_wait(&bars.item_free[ib], ((round >> 1) - 1) & 1u, abort_flag)) break;
+      xt_load_item(items[ib], sm.tab + ib * lay.bytes, &bars.item_full[ib], u, units, n_chunks, sm, A, lane);
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&bars.item_full[ib]);
+      if (!xt_wait(&bars.item_full[ib], (round >> 1) & 1u, abort_flag)) break;
+      // the weights on their way to L2, one tile per lane (sizes and offsets are multiples of 16 bytes)
+      const FastExpert& fe = reinterpret_cast<const TokTabHead*>(sm.tab + ib * lay.bytes)->fe;
+      const int t0 = items[ib].chunk0 >> 1, t1 = (items[ib].chunk0 + items[ib].nchunk + 1) >> 1;
+      for (int t = t0 + lane; t < t1; t += 32)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A.arena + fe.unit_base + static_cast<int64_t>(t) * fe.unit_bytes),
+                     "r"(fe.unit_bytes)
+                     : "memory");
+      __syncwarp();
+    }
+  } else if (warp < XT_MMA_WARP0 + 2) {
+    // -------------------------------------------------------------------- MMA issue, one thread per pipeline
+    // The whole warp waits (a lone waiting lane wakes up several times slower); one issues.
+    const int pl = warp - XT_MMA_WARP0;
+    const uint32_t idesc_gu = tc::idesc_f16(128, 64), idesc_d = tc::idesc_f16(128, 128);
+    // descriptors: constant upper part, start-address field advanced per block
+    const uint64_t a_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.act) + pl * act_m_bytes, cs, 128);
+    const uint64_t z_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.z), XT_Z_STRIDE, 128);
+    const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring_h * XT_SLOT_BYTES;
+    const uint64_t gu_desc = tc::smem_desc_kmajor(ring0, XT_W_STRIDE, 128), dn_desc = tc::smem_desc_kmajor(ring0, XT_D_STRIDE, 128);
+    uint64_t* w_full = &bars.w_full[pl * ring_h];
+    uint64_t* w_empty = &bars.w_empty[pl * ring_h];
+    const uint32_t a_step = (2 * cs) >> 4;       // descriptor units per 16 contraction positions
+    XtCycle ring_c{0, 0};
+    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++round) {
+      XT_ITEM_BEGIN
+      const int npairs = fe.m[pl].nslots >> 5, n_mt = ((fe.m[2].nslots >> 4) + 7) >> 3;   // 128-slot tiles of the down product (<= 3)
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&bars.item_free[ib]);
+      bool ok = xt_wait(&bars.act_ready, round & 1u, abort_flag);
+      tc::fence_after_sync();
+      for (int t = 0; t < nchunk + lag && ok; ++t) {
+        if (t < nchunk) {
+          const uint32_t g = gu_round + t, b = lag ? g & 1u : 0u, k = lag ? g >> 1 : g;
+          if (k >= 1) ok = xt_wait(&bars.gu_free[b], (k - 1) & 1u, abort_flag);   // this accumulator's last contents are read out
+          tc::fence_after_sync();
+          const uint32_t d_acc = tmem_base + (2 * b + pl) * XT_CHUNK;
+          uint64_t ad = a_desc;
+          for (int pr = 0; pr < npairs && ok; pr += 2) {
+            if (!(ok = xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag))) break;
+            if (tc::elect_one()) {
+              const uint64_t bd = gu_desc + ((ring_c.i * XT_SLOT_BYTES) >> 4);
+              tc::mma_f16(d_acc, ad, bd, idesc_gu, pr > 0 ? 1u : 0u);
+              tc::mma_f16(d_acc, ad + a_step, bd + ((2 * XT_W_STRIDE) >> 4), idesc_gu, 1u);
+              if (pr + 1 < npairs) {
+                tc::mma_f16(d_acc, ad + 2 * a_step, bd + (XT_STAGE_BYTES >> 4), idesc_gu, 1u);
+                tc::mma_f16(d_acc, ad + 3 * a_step, bd + ((XT_STAGE_BYTES + 2 * XT_W_STRIDE) >> 4), idesc_gu, 1u);
+              }
+              tc::mma_commit(&w_empty[ring_c.i]);
             }
-            tc::mma_commit(&w_empty[ring_c.i]);
+            __syncwarp();
+            ad += 4 * a_step;
+            ring_c.next(ring_h);
+          }
+          if (!ok) break;
+          if (tc::elect_one()) {
+            tc::mma_commit(&bars.gu_done[b]);
+            if (t == nchunk - 1) tc::mma_commit(&bars.act_free);
           }
           __syncwarp();
-          ring_c.next(ring_h);
-          return true;
-        };
-        for (int t = 0; t < nchunk + lag && ok; ++t) {
-          if (t < nchunk) {
-            const uint32_t g = gu_round + t, b = lag ? g & 1u : 0u, k = lag ? g >> 1 : g;
-            if (k >= 1) ok = xt_wait(&bars.z_free[b], (k - 1) & 1, abort_flag);   // the z that took this accumulator's place is consumed
-            tc::fence_after_sync();
-            const uint32_t d_acc = tmem_base + (2 * b + pl) * XT_CHUNK;
-            for (int pr = 0; pr < npairs && ok; pr += 2) {
-              const uint64_t ad = a_desc + ((4 * pr * cs) >> 4);
-              const uint32_t add = pr > 0 ? 1u : 0u;
-              ok = on_slot(npairs - pr, [&](uint32_t st, uint32_t j, uint64_t bd) {
-                tc::mma_f16(d_acc, ad + (((2 * st + j) * 2 * cs) >> 4), bd, idesc, add | st | j);
-              });
-            }
-            if (!ok) break;
-            if (tc::elect_one()) tc::mma_commit(&bars.gu_done[b]);
-            __syncwarp();
-          }
-          if (t >= lag) {
-            const uint32_t g = gu_round + t - lag, b = lag ? g & 1u : 0u;
-            ok = xt_wait(&bars.z_ready[b], (lag ? g >> 1 : g) & 1, abort_flag);
-            tc::fence_after_sync();
-            // per slot: 64 weight slots and the chunk's 64 columns of z, 32 per stage (16 tensor-memory columns, at the start
-            // of the half they came from)
-            for (int mt = pl; mt < n_mt && ok; mt += 2)
-              for (int q = 0; q < 2 && ok; ++q) {
-                const uint32_t d_acc = d_down + mt * 128 + q * 64, za = tmem_base + 2 * b * XT_CHUNK;
-                const uint32_t add = t > lag ? 1u : 0u;
-                ok = on_slot(2, [&](uint32_t st, uint32_t j, uint64_t bd) { tc::mma_f16_ta(d_acc, za + 32 * st + 8 * j, bd, idesc, add | st | j); });
+        }
+        if (t >= lag) {
+          const uint32_t g = gu_round + t - lag;
+          if (t == lag && round > 0) ok = xt_wait(&bars.down_free, (round - 1) & 1u, abort_flag);   // the last item's sums are read out
+          if (ok) ok = xt_wait(&bars.z_ready, g & 1u, abort_flag);
+          tc::fence_after_sync();
+          for (int mt = pl; mt < n_mt && ok; mt += 2)
+            for (int kp = 0; kp < 2; ++kp) {                 // 32 columns of z per slot
+              if (!(ok = xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag))) break;
+              if (tc::elect_one()) {
+                const uint64_t bd = dn_desc + ((ring_c.i * XT_SLOT_BYTES) >> 4), zd = z_desc + ((4 * kp * XT_Z_STRIDE) >> 4);
+                tc::mma_f16(d_down + mt * 128, zd, bd, idesc_d, t > lag || kp > 0 ? 1u : 0u);
+                tc::mma_f16(d_down + mt * 128, zd + ((2 * XT_Z_STRIDE) >> 4), bd + ((2 * XT_D_STRIDE) >> 4), idesc_d, 1u);
+                tc::mma_commit(&w_empty[ring_c.i]);
               }
-            if (ok && tc::elect_one()) {
-              tc::mma_commit(&bars.z_free[b]);
-              if (t == nchunk + lag - 1) tc::mma_commit(&bars.down_done);
+              __syncwarp();
+              ring_c.next(ring_h);
             }
-            __syncwarp();
+          if (ok && tc::elect_one()) {
+            tc::mma_commit(&bars.z_free);
+            if (t == nchunk + lag - 1) tc::mma_commit(&bars.down_done);
           }
+          __syncwarp();
         }
       }
       gu_round += nchunk;
+      if (!ok) break;
     }
-    tc::fence_before_sync();
-    __syncthreads();
   }
+  tc::fence_before_sync();
+  __syncthreads();
+#undef XT_ITEM_BEGIN
 }
 
 // Item size and ring depth for a layer: the first candidate whose activation operand (2 KB per token at 256 row slots per
