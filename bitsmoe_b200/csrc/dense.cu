@@ -63,7 +63,7 @@ static int dense_mlp_small(const void* x, int x_dtype, const __half* wg, const _
   SkinnyArgs d{};
   d.seg[0] = SkSeg{wd, nullptr, y, H, y_dtype, 0, 0};
   d.n_seg = 1;
-  d.X = z; d.N = T; d.K = I; d.x_dtype = BM_F32; d.x_gate = token_gate_w ? gate : nullptr; d.residual = residual;
+  d.X = z; d.N = T; d.K = I; d.x_dtype = BM_F32; d.x_gate = token_gate_w ? gate : nullptr; d.residual = residual; d.overlap = 1;
   d.splits = skinny_splits(H, I);
   return launch_skinny_nt(d, st);
 }

@@ -28,9 +28,12 @@ constexpr int GT_WARP_EPI0 = 4, GT_EPI_WARPS = 8, GT_WARP_TR0 = 12, GT_TR_WARPS 
 
 __host__ __device__ constexpr int gt_a_bytes(int xd) { return xd == BM_F32 ? GT_BM * GT_BK * 4 : GT_BM * GT_BK * 2; }
 __host__ __device__ constexpr int gt_stage_bytes(int bn, int xd) { return gt_a_bytes(xd) + bn * GT_BK * 2; }
+// Ring depth; with rounding a multiple of the number of warp groups that round (2 or 3), see below.
 __host__ __device__ constexpr int gt_stages(int bn, int xd) {
-  return (216 * 1024) / gt_stage_bytes(bn, xd) < GT_MAX_STAGES ? (216 * 1024) / gt_stage_bytes(bn, xd) : GT_MAX_STAGES;
+  const int fit = (216 * 1024) / gt_stage_bytes(bn, xd) < GT_MAX_STAGES ? (216 * 1024) / gt_stage_bytes(bn, xd) : GT_MAX_STAGES;
+  return xd == BM_F16 || fit % 3 == 0 ? fit : fit / 2 * 2;
 }
+__host__ __device__ constexpr int gt_tr_groups(int bn, int xd) { return gt_stages(bn, xd) % 3 == 0 ? 3 : 2; }
 
 struct GtParams {
   void* C[2];
@@ -61,6 +64,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
                                                                  const __grid_constant__ CUtensorMap map_w0,
                                                                  const __grid_constant__ CUtensorMap map_w1, GtParams p) {
   constexpr int A_BYTES = gt_a_bytes(XD), B_BYTES = BN * GT_BK * 2, STAGE = A_BYTES + B_BYTES, NST = gt_stages(BN, XD);
+  constexpr int TR_GROUPS = gt_tr_groups(BN, XD), TR_PER_GROUP = GT_TR_WARPS / TR_GROUPS;
   constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
   extern __shared__ unsigned char gt_raw[];
   __shared__ __align__(8) uint64_t loaded[GT_MAX_STAGES], ready[GT_MAX_STAGES], empty[GT_MAX_STAGES], acc_full[2], acc_empty[2];
@@ -70,7 +74,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
   if (threadIdx.x == 0) {
     for (int i = 0; i < GT_MAX_STAGES; ++i) {
       tc::mbar_init(&loaded[i], 1);
-      tc::mbar_init(&ready[i], GT_TR_WARPS);
+      tc::mbar_init(&ready[i], TR_PER_GROUP);
       tc::mbar_init(&empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -134,45 +138,70 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
   } else if (warp >= GT_WARP_TR0 || warp == 2 || warp == 3) {
     // ------------------------------------------------------------------ rounding of the X slice to fp16, in place
     if (XD != BM_F16) {
+      // Rounding one slice is a chain (wait, load, convert, store, proxy fence, arrive) of about a thousand cycles however
+      // many warps share it, so groups of warps take the slices in turn and the chains overlap.  A group takes every
+      // TR_GROUPS-th stage of the ring: it sees every use of its stages, as its parity waits need.
       const int tw = warp >= GT_WARP_TR0 ? warp - GT_WARP_TR0 : warp + 2;      // 0 .. 5
-      uint32_t st = 0, ph = 0;
-      for (int tile = blockIdx.x; tile < p.ntiles && ok; tile += gridDim.x) {
-        for (int s = 0; s < nslices; ++s) {
-          if (!(ok = tc::mbar_wait(&loaded[st], ph))) break;
-          unsigned char* sa = smem + st * STAGE;
-          if (XD == BM_BF16) {
-            // 1024 pieces of 16 bytes, element for element (the swizzle only permutes whole pieces)
-#pragma unroll 2
-            for (int i = tw * 32 + lane; i < GT_BM * GT_BK * 2 / 16; i += GT_TR_WARPS * 32) {
-              uint4* q = reinterpret_cast<uint4*>(sa) + i;
-              const uint4 v = *q;
-              const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-              __half2 h[4];
+      const int grp = tw / TR_PER_GROUP, gw = tw - grp * TR_PER_GROUP;
+      const int cta = static_cast<int>(blockIdx.x), grid = static_cast<int>(gridDim.x);
+      const int total = p.ntiles > cta ? (p.ntiles - cta + grid - 1) / grid * nslices : 0;
+      uint32_t cur = grp, ph = 0;
+      for (int s = grp; s < total; s += TR_GROUPS) {
+        if (!(ok = tc::mbar_wait(&loaded[cur], ph))) break;
+        unsigned char* sa = smem + cur * STAGE;
+        if (XD == BM_BF16) {
+          // 1024 pieces of 16 bytes, element for element (the swizzle only permutes whole pieces)
+          constexpr int PIECES = GT_BM * GT_BK * 2 / 16, STEP = TR_PER_GROUP * 32;
 #pragma unroll
-              for (int j = 0; j < 4; ++j) h[j] = __floats2half2_rn(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u));
-              *q = *reinterpret_cast<uint4*>(h);
+          for (int i0 = 0; i0 < PIECES; i0 += 4 * STEP) {
+            uint4 v[4];
+            uint4* q = reinterpret_cast<uint4*>(sa) + i0 + gw * 32 + lane;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              if (i0 + gw * 32 + u * STEP < PIECES) v[u] = q[u * STEP];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              if (i0 + gw * 32 + u * STEP >= PIECES) break;
+              uint32_t* w = reinterpret_cast<uint32_t*>(&v[u]);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const __half2 h = __floats2half2_rn(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u));
+                w[j] = *reinterpret_cast<const uint32_t*>(&h);
+              }
+              q[u * STEP] = v[u];
             }
-          } else {
-            // row r, values 8 j .. 8 j + 7: two 16-byte pieces of box j / 4 -> piece j of the result row
-            const int j = lane & 7;
-#pragma unroll 2
-            for (int rg = tw; rg < GT_BM / 4; rg += GT_TR_WARPS) {
-              const int r = rg * 4 + (lane >> 3), sw = r & 7;
+          }
+        } else {
+          // row r, values 8 j .. 8 j + 7: two 16-byte pieces of box j / 4 -> piece j of the result row; a row's eight lanes
+          // have read before any of them overwrites the row's start
+          const int j = lane & 7, c4 = 2 * (j & 3);
+#pragma unroll 1
+          for (int rg = gw; rg < GT_BM / 4; rg += 2 * TR_PER_GROUP) {
+            float4 lo[2], hi[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              if (rg + u * TR_PER_GROUP >= GT_BM / 4) break;
+              const int r = (rg + u * TR_PER_GROUP) * 4 + (lane >> 3), sw = r & 7;
               const unsigned char* box = sa + (j >> 2) * (A_BYTES / 2) + r * 128;
-              const int c4 = 2 * (j & 3);
-              const float4 lo = *reinterpret_cast<const float4*>(box + ((c4 ^ sw) << 4));
-              const float4 hi = *reinterpret_cast<const float4*>(box + (((c4 + 1) ^ sw) << 4));
-              __half2 h[4] = {__floats2half2_rn(lo.x, lo.y), __floats2half2_rn(lo.z, lo.w), __floats2half2_rn(hi.x, hi.y),
-                              __floats2half2_rn(hi.z, hi.w)};
-              __syncwarp();          // the row's eight lanes have read before any of them overwrites the row's start
+              lo[u] = *reinterpret_cast<const float4*>(box + ((c4 ^ sw) << 4));
+              hi[u] = *reinterpret_cast<const float4*>(box + (((c4 + 1) ^ sw) << 4));
+            }
+            __syncwarp();
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+              if (rg + u * TR_PER_GROUP >= GT_BM / 4) break;
+              const int r = (rg + u * TR_PER_GROUP) * 4 + (lane >> 3), sw = r & 7;
+              __half2 h[4] = {__floats2half2_rn(lo[u].x, lo[u].y), __floats2half2_rn(lo[u].z, lo[u].w), __floats2half2_rn(hi[u].x, hi[u].y),
+                              __floats2half2_rn(hi[u].z, hi[u].w)};
               *reinterpret_cast<uint4*>(sa + r * 128 + ((j ^ sw) << 4)) = *reinterpret_cast<uint4*>(h);
             }
           }
-          tc::fence_async_smem();
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(&ready[st]);
-          if (++st == NST) { st = 0; ph ^= 1; }
         }
+        tc::fence_async_smem();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&ready[cur]);
+        cur += TR_GROUPS;
+        if (cur >= NST) { cur -= NST; ph ^= 1u; }
       }
     }
   } else if (warp >= GT_WARP_EPI0) {

@@ -501,8 +501,9 @@ extern "C" int bm_experts_forward(const bm_layer_t* L, const uint16_t* h_gate, c
 
 // y = fp16(rank_accum) . U_down^T (+ (z * sigmoid(gate)) . W_down^T of a shared expert) (+ residual), one launch.
 static int combine_small(const bm_layer_t* L, const float* rank_accum, int T, const __half* w_down, int w_bf16, const float* z, const float* gate,
-                         int inter, const void* residual, void* y, int y_dtype, cudaStream_t st) {
+                         int inter, const void* residual, void* y, int y_dtype, bool overlap, cudaStream_t st) {
   SkinnyArgs a{};
+  a.overlap = overlap;
   a.seg[0] = SkSeg{L->u_down, nullptr, y, L->hidden, y_dtype, 0, 0};
   a.n_seg = 1;
   a.X = rank_accum; a.N = T; a.K = L->rank_out; a.x_dtype = BM_F32;
@@ -521,7 +522,7 @@ extern "C" int bm_combine_down_basis(const bm_layer_t* L, const float* rank_accu
   if (T == 0) return BM_OK;
   BM_REQUIRE(rank_accum && y, BM_ERR_INVALID_ARG, "combine: null pointer");
   if (T <= SKINNY_MAX_TOKENS && skinny_fits(L->rank_out, 0, 1)) {
-    const int rc = combine_small(L, rank_accum, T, nullptr, 0, nullptr, nullptr, 0, residual, y, y_dtype, static_cast<cudaStream_t>(stream));
+    const int rc = combine_small(L, rank_accum, T, nullptr, 0, nullptr, nullptr, 0, residual, y, y_dtype, false, static_cast<cudaStream_t>(stream));
     if (rc != BM_ERR_UNSUPPORTED) return rc;
   }
   if (L->rank_out % 64 == 0) {
@@ -596,7 +597,7 @@ static int forward_small(const bm_layer_t* L, const bm_block_dense_t* d, const v
                             w.expert_offsets, w.route_flat, T, T * k, w.rank_accum, path, true, w.experts_ws, w.experts_ws_bytes, st);
   if (rc) return rc;
   return combine_small(L, w.rank_accum, T, shared ? h(d->sh_down) : nullptr, bf16, z, shared && d->sh_token_gate ? gate : nullptr,
-                       shared ? d->sh_intermediate : 0, residual, y, x_dtype, st);
+                       shared ? d->sh_intermediate : 0, residual, y, x_dtype, true, st);
 }
 
 extern "C" int bm_layer_forward(const bm_layer_t* L, const void* x, int x_dtype, const void* logits, int logits_dtype,

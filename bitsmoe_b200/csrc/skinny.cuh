@@ -47,6 +47,9 @@ struct SkinnyArgs {
   float4* zero;            // optional buffer the grid clears on its way (the next kernel's accumulator), 16-byte units
   int zero_n;
   RouteSmallArgs route;    // route.T > 0: one more cluster routes these tokens (splits must be 8)
+  // The launch may start while the kernel before it drains.  Weights are read before that kernel is complete, so only for
+  // a launch that follows another one of the same entry point: whatever wrote the weights came before that one.
+  int overlap;
   int row_tiles;           // filled in by the launcher
 };
 

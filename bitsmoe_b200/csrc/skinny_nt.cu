@@ -9,9 +9,9 @@
 //
 // What bounds a launch is latency: weights -> shared memory -> MMA -> cluster exchange.  Three things shorten the chain:
 // everything that multiplies the same x is one launch (SkSeg stacks; the gated pair of a shared expert leaves as
-// silu(g) * u), the routing of given logits is one more cluster of the same grid, and the kernel is launched with
-// programmatic stream serialisation: its weights, which no kernel of this library writes, are on their way to shared
-// memory while the previous kernel still runs.
+// silu(g) * u), the routing of given logits is one more cluster of the same grid, and a launch behind
+// another one of the same call is programmatically serialised: its weights are on their way to shared memory while the
+// previous kernel still runs.
 #include "route_small.cuh"
 
 namespace cg = cooperative_groups;
@@ -311,14 +311,17 @@ int launch_skinny_nt(SkinnyArgs a, cudaStream_t st) {
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = a.splits;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = a.splits > 1 ? 2 : 1;
+  if (a.overlap) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (a.splits > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = a.splits;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   count_launch();
   BM_CUDA(cudaLaunchKernelEx(&cfg, skinny_nt_kernel, a));
   return BM_OK;
