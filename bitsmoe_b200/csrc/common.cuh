@@ -196,14 +196,33 @@ struct GemmTcArgs {
   int x_dtype, c_dtype;
   int* status;
 };
-// Tiled-copy kernel first; BM_ERR_UNSUPPORTED (nothing launched) means: use launch_gemm_tc.
-int launch_gemm_tma(const GemmTcArgs& a, int problems, cudaStream_t st);
 int launch_gemm_tc(const GemmTcArgs& a, int problems, cudaStream_t st);
-// Both in order.
-inline int launch_gemm_basis(const GemmTcArgs& a, int problems, cudaStream_t st) {
-  const int rc = launch_gemm_tma(a, problems, st);
-  return rc == BM_ERR_UNSUPPORTED ? launch_gemm_tc(a, problems, st) : rc;
-}
+// The tiled-copy kernel (gemm_tma.cu): several stacks of weight rows sharing X in one launch.  C[m][n] = X[m] . W[n], or
+// with W_up the gated pair silu(X[m] . W[n]) * (X[m] . W_up[n]).
+constexpr int GEMM_MAX_SEG = 4;
+struct GemmSeg {
+  const __half* W;          // [rows, K]
+  const __half* W_up;
+  void* C;                  // [M, rows]
+  int rows, c_dtype;
+};
+struct GemmTmaArgs {
+  const void* X;            // [M, K]
+  int x_dtype, M, K;
+  GemmSeg seg[GEMM_MAX_SEG];
+  int n_seg;
+  // second contraction of a lone stack: += X2 [M, K2] fp16 . W2 [rows, K2]^T
+  const __half* X2;
+  const __half* W2;
+  int K2;
+  const void* residual;     // added to stack 0, of its type
+  const float* row_gate;    // [M] factor of the gated pair's rows, or null
+  int* status;
+};
+// BM_ERR_UNSUPPORTED, with nothing launched, when a shape or pointer does not suit tiled copies.
+int launch_gemm_tma(const GemmTmaArgs& a, cudaStream_t st);
+// One or two products sharing X: the tiled-copy kernel, else launch_gemm_tc.
+int launch_gemm_basis(const GemmTcArgs& a, int problems, cudaStream_t st);
 
 // NVTX range around a public entry point (route / projection / experts / combine / exchange show up as named ranges
 // in a timeline tool; without a tool attached a push or pop is one null-pointer test).

@@ -75,10 +75,34 @@ __global__ void __launch_bounds__(256) row_gate_kernel(const void* __restrict__ 
   const int t = blockIdx.x * (blockDim.x >> 5) + warp;
   if (t >= T) return;
   float acc = 0.f;
-  for (int i = lane; i < H; i += 32) acc += load_act(x, x_dtype, static_cast<int64_t>(t) * H + i) * __half2float(w[i]);
+  if (x_dtype != BM_F32 && H % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0) {
+    // 16 bytes per lane and load, four in flight: a pass over x at memory speed
+    const uint4* xr = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + static_cast<int64_t>(t) * H);
+    const uint4* wr = reinterpret_cast<const uint4*>(w);
+#pragma unroll 4
+    for (int i = lane; i < H / 8; i += 32) {
+      const uint4 xv = xr[i], wv = __ldg(wr + i);
+      const uint32_t *xp = reinterpret_cast<const uint32_t*>(&xv), *wp = reinterpret_cast<const uint32_t*>(&wv);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 xf = x_dtype == BM_F16 ? __half22float2(*reinterpret_cast<const __half2*>(xp + j))
+                                            : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(xp + j));
+        const float2 wf = __half22float2(*reinterpret_cast<const __half2*>(wp + j));
+        acc = fmaf(xf.x, wf.x, fmaf(xf.y, wf.y, acc));
+      }
+    }
+  } else {
+    for (int i = lane; i < H; i += 32) acc += load_act(x, x_dtype, static_cast<int64_t>(t) * H + i) * __half2float(w[i]);
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if (lane == 0) gate[t] = 1.f / (1.f + __expf(-acc));
+}
+
+int launch_row_gate(const void* x, int x_dtype, const __half* w, int T, int H, float* gate, cudaStream_t st) {
+  row_gate_kernel<<<(T + 7) / 8, 256, 0, st>>>(x, x_dtype, w, T, H, gate);
+  BM_LAUNCH_CHECK("row_gate_kernel");
+  return BM_OK;
 }
 
 // z[t, c] = fp16(silu(g) * u * gate[t]); g, u fp16 [T, I].
@@ -136,13 +160,21 @@ extern "C" int bm_dense_mlp_forward(const void* x, int x_dtype, const uint16_t* 
                            reinterpret_cast<const __half*>(w_down), reinterpret_cast<const __half*>(token_gate_w), T, hidden, intermediate,
                            residual, y, y_dtype, reinterpret_cast<float*>(ws), gate, st);
   if (rc != BM_ERR_UNSUPPORTED) return rc;
+  if (token_gate_w && (rc = launch_row_gate(x, x_dtype, reinterpret_cast<const __half*>(token_gate_w), T, hidden, gate, st))) return rc;
+  // gated pair in the epilogue of one launch where tiled copies take the shape
+  GemmTmaArgs a{};
+  a.X = x; a.x_dtype = x_dtype; a.M = T; a.K = hidden;
+  a.seg[0] = GemmSeg{reinterpret_cast<const __half*>(w_gate), reinterpret_cast<const __half*>(w_up), z, intermediate, BM_F16};
+  a.n_seg = 1;
+  a.row_gate = token_gate_w ? gate : nullptr;
+  rc = launch_gemm_tma(a, st);
+  if (rc == BM_OK)
+    return dense_xwT(z, BM_F16, reinterpret_cast<const __half*>(w_down), nullptr, y, nullptr, y_dtype, residual, T, hidden, intermediate, 1,
+                     nullptr, st);
+  if (rc != BM_ERR_UNSUPPORTED) return rc;
   rc = dense_xwT(x, x_dtype, reinterpret_cast<const __half*>(w_gate), reinterpret_cast<const __half*>(w_up), g, u, BM_F16, nullptr,
                  T, intermediate, hidden, 2, nullptr, st);
   if (rc) return rc;
-  if (token_gate_w) {
-    row_gate_kernel<<<(T + 7) / 8, 256, 0, st>>>(x, x_dtype, reinterpret_cast<const __half*>(token_gate_w), T, hidden, gate);
-    BM_LAUNCH_CHECK("row_gate_kernel");
-  }
   const int64_t pairs = static_cast<int64_t>(T) * intermediate / 2;
   const int blocks = static_cast<int>((pairs + 255) / 256 < 148 * 8 ? (pairs + 255) / 256 : 148 * 8);
   silu_mul_kernel<<<blocks, 256, 0, st>>>(reinterpret_cast<const __half2*>(g), reinterpret_cast<const __half2*>(u),

@@ -1,15 +1,18 @@
-// Shared-basis products for large token counts, warp-specialised: tiled TMA loads, tcgen05.mma, persistent CTAs.
-//   C[m][n] = sum_k X[m][k] * W[n][k],  X = activations (rows = tokens), W = fp16 basis matrix.
-//   h_gate / h_up = x . Vh^T  (bitsmoe/models/qwen3moe/bitsmoe_block.py:63-64)
-//   y = fp16(rank_accum) . U_down^T (+ residual)  (bitsmoe/models/base_block.py:414)
+// Dense products for large token counts, warp-specialised: tiled TMA loads, tcgen05.mma, persistent CTAs.
+//   C_i[m][n] = sum_k X[m][k] * W_i[n][k],  X = activations (rows = tokens), W_i = fp16 matrices ("stacks") sharing X
+//   router logits, h_gate / h_up = x . Vh^T, z = silu(x . Wg^T) * (x . Wu^T) of a shared expert: one launch
+//   (bitsmoe/models/qwen3moe/bitsmoe_block.py:45, :63-64)
+//   y = fp16(rank_accum) . U_down^T (+ z . W_down^T) (+ residual)   (bitsmoe/models/base_block.py:414)
 // A CTA walks 128 x BN output tiles (BN = 256, or 64 when the wide tile would leave most SMs idle).  Per tile, K is
 // streamed in slices of 64 through a ring of stages, both operands K-major with the 128-byte swizzle that the tensor
 // map writes and the MMA descriptor reads:
-//   warp 0      producer: cp.async.bulk.tensor (2-D tiles) of the X and W slices, completing on the stage's mbarrier
+//   warp 0      producer: cp.async.bulk.tensor (2-D tiles) of the X slice and of two half tiles of W rows -- neighbouring
+//               rows of a stack, or the same rows of a gated pair -- completing on the stage's mbarrier
 //   warp 1      MMA issue: four tcgen05.mma (M = 128, N = BN, K = 16) per slice, tcgen05.commit frees the stage; the
 //               accumulator alternates between two TMEM buffers, so the next tile's products run while this tile's
 //               accumulator is read out
-//   warps 4-11  epilogue: tcgen05.ld, residual, rounding, stores of whole 64- or 128-byte row pieces
+//   warps 4-11  epilogue: tcgen05.ld, residual / gated pair, rounding, and 32 x 32 blocks through shared memory into TMA
+//               stores (a lane owns an output row; its own stores would touch 32 rows per instruction)
 //   warps 12-15, 2, 3  only for bf16 / fp32 activations: round the landed X slice to fp16 in place (both MMA operands have to
 //               be fp16: a bf16 A with an fp16 B is not an encodable instruction).  bf16 -> fp16 is element for
 //               element; an fp32 slice is twice as large as its fp16 result, and the eight lanes that hold a row read
@@ -17,28 +20,38 @@
 // Every wait is bounded; a time-out raises the status word.
 #include <cuda.h>
 
+#include <cstring>
+
 #include "common.cuh"
 #include "tc05.cuh"
 
 namespace bm {
 
-
 constexpr int GT_BM = 128, GT_BK = 64, GT_THREADS = 512, GT_MAX_STAGES = 8;
 constexpr int GT_WARP_EPI0 = 4, GT_EPI_WARPS = 8, GT_WARP_TR0 = 12, GT_TR_WARPS = 6;    // transform: warps 12-15 and 2, 3
+constexpr int GT_STORE_BYTES = 32 * 64;                       // one 32 x 32 block of 16-bit results
+constexpr int GT_SMEM = 225 * 1024;                           // stages and store blocks
 
 __host__ __device__ constexpr int gt_a_bytes(int xd) { return xd == BM_F32 ? GT_BM * GT_BK * 4 : GT_BM * GT_BK * 2; }
 __host__ __device__ constexpr int gt_stage_bytes(int bn, int xd) { return gt_a_bytes(xd) + bn * GT_BK * 2; }
 // Ring depth; with rounding a multiple of the number of warp groups that round (2 or 3), see below.
 __host__ __device__ constexpr int gt_stages(int bn, int xd) {
-  const int fit = (216 * 1024) / gt_stage_bytes(bn, xd) < GT_MAX_STAGES ? (216 * 1024) / gt_stage_bytes(bn, xd) : GT_MAX_STAGES;
+  const int room = (GT_SMEM - GT_EPI_WARPS * 2 * GT_STORE_BYTES) / gt_stage_bytes(bn, xd);
+  const int fit = room < GT_MAX_STAGES ? room : GT_MAX_STAGES;
   return xd == BM_F16 || fit % 3 == 0 ? fit : fit / 2 * 2;
 }
 __host__ __device__ constexpr int gt_tr_groups(int bn, int xd) { return gt_stages(bn, xd) % 3 == 0 ? 3 : 2; }
 
+struct GtSeg {
+  void* C;
+  int rows, c_dtype, glu, tile0, map_w, map_up;       // glu: W_up at map_up pairs with W
+};
 struct GtParams {
-  void* C[2];
-  const void* residual;
-  int M, N, K, c_dtype, problems, tiles_n, ntiles;
+  CUtensorMap x, x2, w[GEMM_MAX_SEG + 2], w2, c[GEMM_MAX_SEG];
+  GtSeg seg[GEMM_MAX_SEG];
+  const void* residual;      // of stack 0
+  const float* row_gate;     // factor per row of a gated pair's result, or null
+  int n_seg, M, slices, slices2, tiles_n, ntiles, tma_store;
   int* status;
 };
 
@@ -47,6 +60,12 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
                    tc::smem_u32(dst)),
                "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(tc::smem_u32(bar))
                : "memory");
+}
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, const void* src) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x),
+               "r"(y), "r"(tc::smem_u32(src))
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 // K-major operand tile of 128-byte rows, 8-row groups 1024 bytes apart, 128-byte swizzle
 __device__ __forceinline__ uint64_t gt_desc_sw128(uint32_t saddr) {
@@ -59,11 +78,37 @@ __device__ __forceinline__ uint64_t gt_desc_sw128(uint32_t saddr) {
   return d;
 }
 
+__device__ __forceinline__ uint32_t pack16(float a, float b, int dtype) {
+  if (dtype == BM_F16) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// What output tile `tile` is: its row block, its stack and the first output row (of W) inside the stack.
+struct GtTile {
+  int m0, si, n0;
+  bool two;                  // both halves of the tile hold W rows
+};
+template <int BN>
+__device__ __forceinline__ GtTile gt_tile(const GtParams& p, int tile) {
+  GtTile t;
+  const int m_t = tile / p.tiles_n, r = tile - m_t * p.tiles_n;
+  t.m0 = m_t * GT_BM;
+  t.si = 0;
+  while (t.si + 1 < p.n_seg && r >= p.seg[t.si + 1].tile0) ++t.si;
+  const GtSeg& s = p.seg[t.si];
+  t.n0 = (r - s.tile0) * (s.glu ? BN / 2 : BN);
+  t.two = s.glu || t.n0 + BN / 2 < s.rows;
+  return t;
+}
+
 template <int BN, int XD>
-__global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_constant__ CUtensorMap map_x,
-                                                                 const __grid_constant__ CUtensorMap map_w0,
-                                                                 const __grid_constant__ CUtensorMap map_w1, GtParams p) {
-  constexpr int A_BYTES = gt_a_bytes(XD), B_BYTES = BN * GT_BK * 2, STAGE = A_BYTES + B_BYTES, NST = gt_stages(BN, XD);
+__global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_constant__ GtParams p) {
+  constexpr int A_BYTES = gt_a_bytes(XD), A2_BYTES = GT_BM * GT_BK * 2, H_BYTES = BN / 2 * GT_BK * 2, STAGE = A_BYTES + 2 * H_BYTES,
+                NST = gt_stages(BN, XD);
   constexpr int TR_GROUPS = gt_tr_groups(BN, XD), TR_PER_GROUP = GT_TR_WARPS / TR_GROUPS;
   constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
   extern __shared__ unsigned char gt_raw[];
@@ -88,24 +133,29 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
-  const int nslices = p.K / GT_BK;
+  const int slices = p.slices + p.slices2;       // of X . W, then of the second contraction
+  const int cta = static_cast<int>(blockIdx.x), grid = static_cast<int>(gridDim.x);
   bool ok = true;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (the whole warp waits, one lane issues)
     uint32_t st = 0, ph = 0;
-    for (int tile = blockIdx.x; tile < p.ntiles && ok; tile += gridDim.x) {
-      const int per_m = p.tiles_n * p.problems, m_t = tile / per_m, rem = tile - m_t * per_m;
-      const int z = rem / p.tiles_n, n_t = rem - z * p.tiles_n;
-      const CUtensorMap* mw = z ? &map_w1 : &map_w0;
-      for (int s = 0; s < nslices; ++s) {
+    for (int tile = cta; tile < p.ntiles && ok; tile += grid) {
+      const GtTile t = gt_tile<BN>(p, tile);
+      const GtSeg& sg = p.seg[t.si];
+      const CUtensorMap *mw = &p.w[sg.map_w], *mu = sg.glu ? &p.w[sg.map_up] : mw;
+      const int nu = sg.glu ? t.n0 : t.n0 + BN / 2;
+      for (int s = 0; s < slices; ++s) {
         if (!(ok = tc::mbar_wait(&empty[st], ph ^ 1))) break;
         if (tc::elect_one()) {
           unsigned char* sa = smem + st * STAGE;
-          tc::mbar_expect_tx(&loaded[st], A_BYTES + B_BYTES);
-          tma_load_2d(sa, &map_x, s * GT_BK, m_t * GT_BM, &loaded[st]);
-          if (XD == BM_F32) tma_load_2d(sa + A_BYTES / 2, &map_x, s * GT_BK + 32, m_t * GT_BM, &loaded[st]);   // an fp32 row of 64 values is two 128-byte boxes
-          tma_load_2d(sa + A_BYTES, mw, s * GT_BK, n_t * BN, &loaded[st]);
+          const bool first = s < p.slices;
+          const int k = (first ? s : s - p.slices) * GT_BK;
+          tc::mbar_expect_tx(&loaded[st], (first ? A_BYTES : A2_BYTES) + (t.two ? 2 : 1) * H_BYTES);
+          tma_load_2d(sa, first ? &p.x : &p.x2, k, t.m0, &loaded[st]);
+          if (XD == BM_F32 && first) tma_load_2d(sa + A_BYTES / 2, &p.x, k + 32, t.m0, &loaded[st]);   // an fp32 row of 64 values is two 128-byte boxes
+          tma_load_2d(sa + A_BYTES, first ? mw : &p.w2, k, t.n0, &loaded[st]);
+          if (t.two) tma_load_2d(sa + A_BYTES + H_BYTES, first ? mu : &p.w2, k, nu, &loaded[st]);
         }
         __syncwarp();
         if (++st == NST) { st = 0; ph ^= 1; }
@@ -114,12 +164,12 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issue (the whole warp waits, one issues)
     uint32_t st = 0, ph = 0, ti = 0;
-    const uint32_t idesc = tc::idesc_f16(GT_BM, BN);
-    for (int tile = blockIdx.x; tile < p.ntiles && ok; tile += gridDim.x, ++ti) {
+    for (int tile = cta; tile < p.ntiles && ok; tile += grid, ++ti) {
       const uint32_t ab = ti & 1u;
+      const uint32_t idesc = tc::idesc_f16(GT_BM, gt_tile<BN>(p, tile).two ? BN : BN / 2);
       if (ti >= 2 && !(ok = tc::mbar_wait(&acc_empty[ab], ((ti >> 1) - 1) & 1))) break;    // read out two tiles ago
       tc::fence_after_sync();
-      for (int s = 0; s < nslices; ++s) {
+      for (int s = 0; s < slices; ++s) {
         if (!(ok = tc::mbar_wait(XD == BM_F16 ? &loaded[st] : &ready[st], ph))) break;
         if (tc::elect_one()) {
           const uint32_t sa = tc::smem_u32(smem + st * STAGE);
@@ -143,13 +193,16 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
       // TR_GROUPS-th stage of the ring: it sees every use of its stages, as its parity waits need.
       const int tw = warp >= GT_WARP_TR0 ? warp - GT_WARP_TR0 : warp + 2;      // 0 .. 5
       const int grp = tw / TR_PER_GROUP, gw = tw - grp * TR_PER_GROUP;
-      const int cta = static_cast<int>(blockIdx.x), grid = static_cast<int>(gridDim.x);
-      const int total = p.ntiles > cta ? (p.ntiles - cta + grid - 1) / grid * nslices : 0;
+      const int total = p.ntiles > cta ? (p.ntiles - cta + grid - 1) / grid * slices : 0;
       uint32_t cur = grp, ph = 0;
+      int k = grp;                               // slice of its tile
       for (int s = grp; s < total; s += TR_GROUPS) {
         if (!(ok = tc::mbar_wait(&loaded[cur], ph))) break;
+        while (k >= slices) k -= slices;
         unsigned char* sa = smem + cur * STAGE;
-        if (XD == BM_BF16) {
+        if (k >= p.slices) {
+          // second contraction: fp16 already
+        } else if (XD == BM_BF16) {
           // 1024 pieces of 16 bytes, element for element (the swizzle only permutes whole pieces)
           constexpr int PIECES = GT_BM * GT_BK * 2 / 16, STEP = TR_PER_GROUP * 32;
 #pragma unroll
@@ -164,10 +217,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
               if (i0 + gw * 32 + u * STEP >= PIECES) break;
               uint32_t* w = reinterpret_cast<uint32_t*>(&v[u]);
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const __half2 h = __floats2half2_rn(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u));
-                w[j] = *reinterpret_cast<const uint32_t*>(&h);
-              }
+              for (int j = 0; j < 4; ++j) w[j] = pack16(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xffff0000u), BM_F16);
               q[u * STEP] = v[u];
             }
           }
@@ -191,9 +241,9 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
             for (int u = 0; u < 2; ++u) {
               if (rg + u * TR_PER_GROUP >= GT_BM / 4) break;
               const int r = (rg + u * TR_PER_GROUP) * 4 + (lane >> 3), sw = r & 7;
-              __half2 h[4] = {__floats2half2_rn(lo[u].x, lo[u].y), __floats2half2_rn(lo[u].z, lo[u].w), __floats2half2_rn(hi[u].x, hi[u].y),
-                              __floats2half2_rn(hi[u].z, hi[u].w)};
-              *reinterpret_cast<uint4*>(sa + r * 128 + ((j ^ sw) << 4)) = *reinterpret_cast<uint4*>(h);
+              *reinterpret_cast<uint4*>(sa + r * 128 + ((j ^ sw) << 4)) =
+                  make_uint4(pack16(lo[u].x, lo[u].y, BM_F16), pack16(lo[u].z, lo[u].w, BM_F16), pack16(hi[u].x, hi[u].y, BM_F16),
+                             pack16(hi[u].z, hi[u].w, BM_F16));
             }
           }
         }
@@ -202,83 +252,92 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
         if (lane == 0) tc::mbar_arrive(&ready[cur]);
         cur += TR_GROUPS;
         if (cur >= NST) { cur -= NST; ph ^= 1u; }
+        k += TR_GROUPS;
       }
     }
   } else if (warp >= GT_WARP_EPI0) {
     // ------------------------------------------------------------------ epilogue
+    // warp = (TMEM lane quarter q, every other block of 32 output columns)
     const int q = warp & 3, half = (warp - GT_WARP_EPI0) >> 2;
-    uint32_t ti = 0;
-    for (int tile = blockIdx.x; tile < p.ntiles && ok; tile += gridDim.x, ++ti) {
-      const int per_m = p.tiles_n * p.problems, m_t = tile / per_m, rem = tile - m_t * per_m;
-      const int z = rem / p.tiles_n, n_t = rem - z * p.tiles_n;
+    unsigned char* stores = smem + NST * STAGE + (warp - GT_WARP_EPI0) * 2 * GT_STORE_BYTES;
+    uint32_t ti = 0, sb = 0;
+    for (int tile = cta; tile < p.ntiles && ok; tile += grid, ++ti) {
+      const GtTile t = gt_tile<BN>(p, tile);
+      const GtSeg& sg = p.seg[t.si];
       const uint32_t ab = ti & 1u;
       if (!(ok = tc::mbar_wait(&acc_full[ab], (ti >> 1) & 1))) break;
       tc::fence_after_sync();
-      const int row = m_t * GT_BM + 32 * q + lane;
-      // N is a multiple of 8, so whole 16-byte accesses only need aligned bases
-      const bool vec_ok = ((reinterpret_cast<uintptr_t>(p.C[z]) | reinterpret_cast<uintptr_t>(p.residual)) & 15u) == 0;
-      const bool with_res = p.residual != nullptr && z == 0;
+      const int row0 = t.m0 + 32 * q, row = row0 + lane, N = sg.rows;
+      const bool with_res = p.residual != nullptr && t.si == 0;
+      const uint32_t acc = tmem_base + (static_cast<uint32_t>(32 * q) << 16) + ab * BN;
+      const int blocks = (sg.glu ? BN / 2 : t.two ? BN : BN / 2) / 32;
+      const float gate = sg.glu && p.row_gate && row < p.M ? p.row_gate[row] : 1.f;
 #pragma unroll 1
-      for (int c = 0; c < BN / 2; c += 32) {
+      for (int b = half; b < blocks; b += 2) {
+        const int n = t.n0 + 32 * b;
+        if (n >= N) break;
         float v[32];
-        const int col = half * (BN / 2) + c;
-        tc::tmem_ld32(tmem_base + (static_cast<uint32_t>(32 * q) << 16) + ab * BN + col, v);
-        const int n = n_t * BN + col;
-        if (row < p.M && n + 32 <= p.N && vec_ok) {
-          const size_t idx = static_cast<size_t>(row) * p.N + n;
-          if (with_res) {
-            if (p.c_dtype == BM_F32) {
-              const float4* rs = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.residual) + idx);
+        tc::tmem_ld32(acc + 32 * b, v);
+        if (sg.glu) {
 #pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const float4 r4 = __ldg(rs + i);
-                v[4 * i] += r4.x; v[4 * i + 1] += r4.y; v[4 * i + 2] += r4.z; v[4 * i + 3] += r4.w;
-              }
-            } else {
-              const uint4* rs = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.residual) + idx);
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const uint4 r4 = __ldg(rs + i);
-                const uint32_t w[4] = {r4.x, r4.y, r4.z, r4.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  float2 f;
-                  if (p.c_dtype == BM_F16) f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-                  else f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
-                  v[8 * i + 2 * j] += f.x;
-                  v[8 * i + 2 * j + 1] += f.y;
-                }
-              }
-            }
-          }
-          if (p.c_dtype == BM_F32) {
-#pragma unroll
-            for (int i = 0; i < 32; i += 4)
-              *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.C[z]) + idx + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-          } else {
-            uint32_t pk[16];
+          for (int h = 0; h < 2; ++h) {
+            float u[16];
+            tc::tmem_ld16(acc + BN / 2 + 32 * b + 16 * h, u);
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
-              if (p.c_dtype == BM_F16) {
-                const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-                pk[i] = *reinterpret_cast<const uint32_t*>(&h);
-              } else {
-                const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-                pk[i] = *reinterpret_cast<const uint32_t*>(&h);
+              const float g = v[16 * h + i];
+              v[16 * h + i] = __fdividef(g, 1.f + __expf(-g)) * u[i] * gate;
+            }
+          }
+        }
+        if (sg.c_dtype != BM_F32 && p.tma_store) {
+          // 32 rows of 64 bytes, 16-byte pieces in the order of the map's 64-byte swizzle; the block two before has left
+          unsigned char* blk = stores + sb * GT_STORE_BYTES;
+          sb ^= 1u;
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+          __syncwarp();
+          unsigned char* mine = blk + lane * 64;
+          const int sw = (lane >> 1) & 3;
+          if (with_res) {
+            const int r = lane >> 2, c = lane & 3;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int rr = 8 * i + r;
+              uint4 x = make_uint4(0u, 0u, 0u, 0u);
+              if (row0 + rr < p.M && n + 8 * c < N)
+                x = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.residual) + static_cast<size_t>(row0 + rr) * N + n + 8 * c));
+              *reinterpret_cast<uint4*>(blk + rr * 64 + ((c ^ ((rr >> 1) & 3)) << 4)) = x;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int c2 = 0; c2 < 4; ++c2) {
+              const uint4 x = *reinterpret_cast<const uint4*>(mine + ((c2 ^ sw) << 4));
+              const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                const float2 f = sg.c_dtype == BM_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j]))
+                                                      : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
+                v[8 * c2 + 2 * j] += f.x;
+                v[8 * c2 + 2 * j + 1] += f.y;
               }
             }
-            uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p.C[z]) + idx);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) dst[i] = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
           }
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+            *reinterpret_cast<uint4*>(mine + ((c ^ sw) << 4)) =
+                make_uint4(pack16(v[8 * c], v[8 * c + 1], sg.c_dtype), pack16(v[8 * c + 2], v[8 * c + 3], sg.c_dtype),
+                           pack16(v[8 * c + 4], v[8 * c + 5], sg.c_dtype), pack16(v[8 * c + 6], v[8 * c + 7], sg.c_dtype));
+          tc::fence_async_smem();
+          __syncwarp();
+          if (lane == 0) tma_store_2d(&p.c[t.si], n, row0, blk);       // rows and columns past the matrix are clipped
         } else if (row < p.M) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            if (n + i < p.N) {
-              const size_t idx = static_cast<size_t>(row) * p.N + n + i;
+            if (n + i < N) {
+              const size_t idx = static_cast<size_t>(row) * N + n + i;
               float val = v[i];
-              if (with_res) val += load_act(p.residual, p.c_dtype, idx);
-              store_act(p.C[z], p.c_dtype, idx, val);
+              if (with_res) val += load_act(p.residual, sg.c_dtype, idx);
+              store_act(sg.C, sg.c_dtype, idx, val);
             }
           }
         }
@@ -287,6 +346,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&acc_empty[ab]);
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
   }
   if (!ok && lane == 0 && p.status) atomicExch(p.status, BM_ERR_TIMEOUT);
   tc::fence_before_sync();
@@ -311,22 +371,22 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// [rows, cols] row-major, 128-byte-swizzled boxes of box_rows x 128 bytes
-static bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int elem_bytes, int box_rows) {
+// [rows, cols] row-major, boxes of box_rows x box_bytes (128 or 64) with the swizzle of that width
+static bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int elem_bytes, int box_rows, int box_bytes) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return false;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * elem_bytes};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / elem_bytes), static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_bytes / elem_bytes), static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
   return fn(map, elem_bytes == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(base), dims,
-            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, box_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 template <int BN, int XD>
-static int launch_one(const CUtensorMap& mx, const CUtensorMap& mw0, const CUtensorMap& mw1, const GtParams& p, int grid, cudaStream_t st) {
-  const int smem = gt_stages(BN, XD) * gt_stage_bytes(BN, XD) + 1024;
+static int launch_one(const GtParams& p, int grid, cudaStream_t st) {
+  const int smem = gt_stages(BN, XD) * gt_stage_bytes(BN, XD) + GT_EPI_WARPS * 2 * GT_STORE_BYTES + 1024;
   static PerDeviceOnce once;
   int dev = -1;
   BM_CUDA(cudaGetDevice(&dev));
@@ -334,17 +394,18 @@ static int launch_one(const CUtensorMap& mx, const CUtensorMap& mw0, const CUten
     BM_CUDA(cudaFuncSetAttribute(gemm_tma_kernel<BN, XD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     once.mark(dev);
   }
-  gemm_tma_kernel<BN, XD><<<grid, GT_THREADS, smem, st>>>(mx, mw0, mw1, p);
+  gemm_tma_kernel<BN, XD><<<grid, GT_THREADS, smem, st>>>(p);
   BM_LAUNCH_CHECK("gemm_tma_kernel");
   return BM_OK;
 }
 
 // Returns BM_ERR_UNSUPPORTED (without having launched anything) when the shape or the pointers do not suit tiled
-// copies; the caller then takes the cp.async kernel.
-int launch_gemm_tma(const GemmTcArgs& a, int problems, cudaStream_t st) {
+// copies; the caller then takes the cp.async kernel, a product at a time.
+int launch_gemm_tma(const GemmTmaArgs& a, cudaStream_t st) {
   const int xb = a.x_dtype == BM_F32 ? 4 : 2;
-  if (a.K % GT_BK != 0 || a.N % 8 != 0 || a.M <= 0 || problems < 1 || problems > 2) return BM_ERR_UNSUPPORTED;
-  if ((reinterpret_cast<uintptr_t>(a.X) | reinterpret_cast<uintptr_t>(a.W[0]) | reinterpret_cast<uintptr_t>(a.W[problems - 1])) & 15u)
+  auto aligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15u) == 0; };
+  if (a.K <= 0 || a.K % GT_BK != 0 || a.K2 % GT_BK != 0 || a.M <= 0 || a.n_seg < 1 || a.n_seg > GEMM_MAX_SEG || !aligned(a.X) || !aligned(a.X2) ||
+      !aligned(a.W2) || (a.K2 && a.n_seg != 1))
     return BM_ERR_UNSUPPORTED;
   static PerDeviceOnce once;
   static int sm_counts[MAX_DEVICES];
@@ -355,29 +416,59 @@ int launch_gemm_tma(const GemmTcArgs& a, int problems, cudaStream_t st) {
     BM_CUDA(cudaDeviceGetAttribute(&sm_counts[dev], cudaDevAttrMultiProcessorCount, dev));
     once.mark(dev);
   }
+  GtParams p;
+  memset(&p, 0, sizeof(p));
   const int tiles_m = (a.M + GT_BM - 1) / GT_BM;
-  const bool narrow = tiles_m * ((a.N + 255) / 256) * problems < sm_counts[dev] / 2;   // the wide tile would leave most SMs idle
+  auto lay_out = [&](int bn) {
+    p.tiles_n = 0;
+    for (int i = 0; i < a.n_seg; ++i) {
+      p.seg[i].tile0 = p.tiles_n;
+      const int per = a.seg[i].W_up ? bn / 2 : bn;
+      p.tiles_n += (a.seg[i].rows + per - 1) / per;
+    }
+    return tiles_m * p.tiles_n;
+  };
+  const bool narrow = lay_out(256) < sm_counts[dev] / 2;   // the wide tile would leave most SMs idle
   const int bn = narrow ? 64 : 256;
-  CUtensorMap mx, mw0, mw1;
-  if (!make_map(&mx, a.X, a.M, a.K, xb, GT_BM) || !make_map(&mw0, a.W[0], a.N, a.K, 2, bn) ||
-      !make_map(&mw1, a.W[problems - 1], a.N, a.K, 2, bn))
-    return BM_ERR_UNSUPPORTED;
-  GtParams p{};
-  p.C[0] = a.C[0]; p.C[1] = a.C[problems - 1];
-  p.residual = a.residual;
-  p.M = a.M; p.N = a.N; p.K = a.K; p.c_dtype = a.c_dtype; p.problems = problems;
-  p.tiles_n = (a.N + bn - 1) / bn;
-  p.ntiles = tiles_m * p.tiles_n * problems;
+  p.ntiles = lay_out(bn);
+  if (!make_map(&p.x, a.X, a.M, a.K, xb, GT_BM, 128)) return BM_ERR_UNSUPPORTED;
+  if (a.K2 && (!make_map(&p.x2, a.X2, a.M, a.K2, 2, GT_BM, 128) || !make_map(&p.w2, a.W2, a.seg[0].rows, a.K2, 2, bn / 2, 128))) return BM_ERR_UNSUPPORTED;
+  p.tma_store = aligned(a.residual);
+  int maps = 0;
+  for (int i = 0; i < a.n_seg; ++i) {
+    const GemmSeg& s = a.seg[i];
+    if (s.rows <= 0 || s.rows % 8 != 0 || !aligned(s.W) || !aligned(s.W_up) || maps + 2 > GEMM_MAX_SEG + 2) return BM_ERR_UNSUPPORTED;
+    GtSeg& d = p.seg[i];
+    d.C = s.C; d.rows = s.rows; d.c_dtype = s.c_dtype; d.glu = s.W_up != nullptr;
+    d.map_w = maps++;
+    if (!make_map(&p.w[d.map_w], s.W, s.rows, a.K, 2, bn / 2, 128)) return BM_ERR_UNSUPPORTED;
+    if (d.glu) {
+      d.map_up = maps++;
+      if (!make_map(&p.w[d.map_up], s.W_up, s.rows, a.K, 2, bn / 2, 128)) return BM_ERR_UNSUPPORTED;
+    }
+    if (s.c_dtype != BM_F32 && (!aligned(s.C) || !make_map(&p.c[i], s.C, a.M, s.rows, 2, 32, 64))) p.tma_store = 0;
+  }
+  p.residual = a.residual; p.row_gate = a.row_gate; p.n_seg = a.n_seg; p.M = a.M;
+  p.slices = a.K / GT_BK; p.slices2 = a.K2 / GT_BK;
   p.status = a.status;
   const int grid = p.ntiles < sm_counts[dev] ? p.ntiles : sm_counts[dev];
   if (narrow) {
-    if (a.x_dtype == BM_F32) return launch_one<64, BM_F32>(mx, mw0, mw1, p, grid, st);
-    if (a.x_dtype == BM_BF16) return launch_one<64, BM_BF16>(mx, mw0, mw1, p, grid, st);
-    return launch_one<64, BM_F16>(mx, mw0, mw1, p, grid, st);
+    if (a.x_dtype == BM_F32) return launch_one<64, BM_F32>(p, grid, st);
+    if (a.x_dtype == BM_BF16) return launch_one<64, BM_BF16>(p, grid, st);
+    return launch_one<64, BM_F16>(p, grid, st);
   }
-  if (a.x_dtype == BM_F32) return launch_one<256, BM_F32>(mx, mw0, mw1, p, grid, st);
-  if (a.x_dtype == BM_BF16) return launch_one<256, BM_BF16>(mx, mw0, mw1, p, grid, st);
-  return launch_one<256, BM_F16>(mx, mw0, mw1, p, grid, st);
+  if (a.x_dtype == BM_F32) return launch_one<256, BM_F32>(p, grid, st);
+  if (a.x_dtype == BM_BF16) return launch_one<256, BM_BF16>(p, grid, st);
+  return launch_one<256, BM_F16>(p, grid, st);
+}
+
+int launch_gemm_basis(const GemmTcArgs& a, int problems, cudaStream_t st) {
+  GemmTmaArgs t{};
+  t.X = a.X; t.x_dtype = a.x_dtype; t.M = a.M; t.K = a.K; t.residual = a.residual; t.status = a.status;
+  t.n_seg = problems;
+  for (int i = 0; i < problems; ++i) t.seg[i] = GemmSeg{a.W[i], nullptr, a.C[i], a.N, a.c_dtype};
+  const int rc = launch_gemm_tma(t, st);
+  return rc == BM_ERR_UNSUPPORTED ? launch_gemm_tc(a, problems, st) : rc;
 }
 
 }  // namespace bm

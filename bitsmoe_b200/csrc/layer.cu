@@ -687,6 +687,53 @@ static BlockWs carve_block_ws(const bm_layer_t* L, const bm_block_dense_t* d, in
   return w;
 }
 
+// A prefill batch of a whole block: everything that multiplies x in one launch (router logits, basis projection, the shared
+// expert's gated pair), routing, packed experts, and both down products in one launch.  BM_ERR_UNSUPPORTED, with nothing
+// launched that matters, when a shape or pointer does not suit the tiled-copy GEMM.
+static int forward_large(const bm_layer_t* L, const bm_block_dense_t& d, const void* x, int x_dtype, int T, int num_routed, int k, int renorm,
+                         int weight_round, const int32_t* global_to_local, void* logits, void* y, const LayerWs& w, const BlockWs& b,
+                         cudaStream_t st) {
+  const bool shared = d.sh_intermediate > 0;
+  if (!L->vh_gate || !L->vh_up || !L->u_down || L->rank_out % 64 != 0 || (shared && d.sh_intermediate % 64 != 0)) return BM_ERR_UNSUPPORTED;
+  auto h = [](const uint16_t* p) { return reinterpret_cast<const __half*>(p); };
+  const size_t mat = shared ? align_up(static_cast<size_t>(T) * d.sh_intermediate * 2, 256) : 0;
+  __half* z = static_cast<__half*>(b.dense_ws);
+  float* gate = reinterpret_cast<float*>(static_cast<unsigned char*>(b.dense_ws) + 3 * mat);
+  int rc;
+  if (shared && d.sh_token_gate && (rc = launch_row_gate(x, x_dtype, h(d.sh_token_gate), T, L->hidden, gate, st))) return rc;
+  GemmTmaArgs a{};
+  a.X = x; a.x_dtype = x_dtype; a.M = T; a.K = L->hidden; a.status = L->status_dev;
+  a.seg[0] = GemmSeg{h(d.gate_w), nullptr, logits, num_routed, x_dtype};
+  a.seg[1] = GemmSeg{L->vh_gate, nullptr, w.h_gate, L->rank_in, BM_F16};
+  a.seg[2] = GemmSeg{L->vh_up, nullptr, w.h_up, L->rank_in, BM_F16};
+  if (shared) a.seg[3] = GemmSeg{h(d.sh_gate), h(d.sh_up), z, d.sh_intermediate, BM_F16};
+  a.n_seg = shared ? 4 : 3;
+  a.row_gate = shared && d.sh_token_gate ? gate : nullptr;
+  if ((rc = launch_gemm_tma(a, st))) return rc;
+  BM_CUDA(cudaMemsetAsync(w.rank_accum, 0, sizeof(float) * static_cast<size_t>(T) * L->rank_out, st));
+  rc = bm_route(logits, x_dtype, T, num_routed, k, renorm, weight_round, global_to_local, L->num_experts, TILE_ROWS, w.topk_idx, w.topk_w,
+                w.token_indices, w.expert_offsets, w.route_flat, nullptr, nullptr, w.route_ws, w.route_ws_bytes, st);
+  if (rc) return rc;
+  rc = experts_forward_impl(L, reinterpret_cast<const uint16_t*>(w.h_gate), reinterpret_cast<const uint16_t*>(w.h_up), w.token_indices,
+                            w.expert_offsets, w.route_flat, T, T * k, w.rank_accum, BM_PATH_AUTO, true, w.experts_ws, w.experts_ws_bytes, st);
+  if (rc) return rc;
+  GemmTmaArgs c{};
+  c.X = w.rank_accum; c.x_dtype = BM_F32; c.M = T; c.K = L->rank_out; c.status = L->status_dev;
+  c.seg[0] = GemmSeg{L->u_down, nullptr, y, L->hidden, x_dtype};
+  c.n_seg = 1;
+  if (shared) { c.X2 = z; c.W2 = h(d.sh_down); c.K2 = d.sh_intermediate; }
+  rc = launch_gemm_tma(c, st);
+  if (rc != BM_ERR_UNSUPPORTED) return rc;
+  // y's rows do not suit tiled copies: the shared expert's product first, then the other one on top
+  if (shared) {
+    GemmTcArgs t{};
+    t.X = z; t.W[0] = t.W[1] = h(d.sh_down); t.C[0] = t.C[1] = b.res; t.M = T; t.N = L->hidden; t.K = d.sh_intermediate;
+    t.x_dtype = BM_F16; t.c_dtype = x_dtype; t.status = L->status_dev;
+    if ((rc = launch_gemm_tc(t, 1, st))) return rc;
+  }
+  return bm_combine_down_basis(L, w.rank_accum, T, shared ? b.res : nullptr, y, x_dtype, st);
+}
+
 extern "C" size_t bm_block_workspace_bytes(const bm_layer_t* L, const bm_block_dense_t* d, int32_t num_routed, int32_t T, int32_t k) {
   if (!L || !d || T < 0 || k <= 0) return 0;
   return carve_layer_ws(L, nullptr, T, k).total + carve_block_ws(L, d, num_routed, nullptr, T).total;
@@ -737,7 +784,9 @@ extern "C" int bm_block_forward(const bm_layer_t* L, const bm_block_dense_t* den
     cast_weights_kernel<<<dim3(148, 5), 256, 0, st>>>(c);
     BM_LAUNCH_CHECK("cast_weights_kernel");
   }
-  int rc = bm_gate_logits(x, x_dtype, d.gate_w, T, num_routed, L->hidden, logits, x_dtype, stream);
+  int rc = forward_large(L, d, x, x_dtype, T, num_routed, k, renorm, weight_round, global_to_local, logits, y, w, b, st);
+  if (rc != BM_ERR_UNSUPPORTED) return rc;
+  rc = bm_gate_logits(x, x_dtype, d.gate_w, T, num_routed, L->hidden, logits, x_dtype, stream);
   if (rc) return rc;
   if (shared) {
     rc = bm_dense_mlp_forward(x, x_dtype, d.sh_gate, d.sh_up, d.sh_down, d.sh_token_gate, T, L->hidden, d.sh_intermediate, nullptr, b.res,

@@ -59,6 +59,9 @@ bool skinny_fits(int K, int K2, int splits);
 // Cluster size along K for a product of `rows` output rows.
 int skinny_splits(int rows, int K);
 
+// gate[t] = sigmoid(x[t] . w) (dense.cu)
+int launch_row_gate(const void* x, int x_dtype, const __half* w, int T, int H, float* gate, cudaStream_t st);
+
 bool route_small_fits(int T, int E, int k);
 int launch_route_small(const RouteSmallArgs& a, cudaStream_t st);
 
