@@ -7,7 +7,7 @@
 // leaves the order open (torch.topk ties, an unstable argsort) this file fixes it:
 // ties go to the lower expert id, and inside an expert assignments are ordered by
 // ascending flat (token, slot) index.
-#include "common.cuh"
+#include "topk.cuh"
 
 namespace bm {
 
@@ -16,115 +16,21 @@ constexpr int ROUTE_BLOCK = 1024;           // assignments per block of the perm
 constexpr int ROUTE_WARPS = ROUTE_BLOCK / 32;
 
 // ---------------------------------------------------------------- top-k
-// One warp per token; probabilities live in a warp-private shared row.
-// Top-k of one token by one warp.  Up to ROUTE_REG_E experts stay in registers (lane l holds experts l, l+32, ...);
-// `p` is a warp-private shared row of E floats used only beyond that.
-constexpr int ROUTE_REG_PER_LANE = 8;
-constexpr int ROUTE_REG_E = 32 * ROUTE_REG_PER_LANE;
-
-__device__ __forceinline__ void warp_topk_token(const void* __restrict__ logits, int dtype, int t, int E, int k, int renorm,
-                                                int weight_round, float* p, int32_t* __restrict__ idx_out,
-                                                float* __restrict__ w_out) {
-  const int lane = threadIdx.x & 31;
-  float my_w = 0.f;   // lane j keeps the j-th selected weight (k <= 32)
-  int my_i = 0;
-  float wsum = 0.f;
-  if (E <= ROUTE_REG_E) {
-    float v[ROUTE_REG_PER_LANE];
-    float mx = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < ROUTE_REG_PER_LANE; ++i) {
-      const int e = lane + 32 * i;
-      v[i] = e < E ? load_act(logits, dtype, static_cast<int64_t>(t) * E + e) : -INFINITY;
-      mx = fmaxf(mx, v[i]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    float sum = 0.f;
-#pragma unroll
-    for (int i = 0; i < ROUTE_REG_PER_LANE; ++i) {
-      v[i] = lane + 32 * i < E ? expf(v[i] - mx) : -1.f;   // padding can never win
-      sum += fmaxf(v[i], 0.f);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const float inv = 1.f / sum;
-    for (int j = 0; j < k; ++j) {
-      float best = -1.f;
-      int bi = 0x7fffffff;
-#pragma unroll
-      for (int i = 0; i < ROUTE_REG_PER_LANE; ++i)
-        if (v[i] > best) { best = v[i]; bi = lane + 32 * i; }   // ascending e: the first hit wins ties
-      // probabilities are non-negative, so their bit patterns order like unsigned integers: two warp reductions
-      // (largest value, then the lowest expert id holding it) replace a ten-shuffle butterfly
-      const unsigned best_bits = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(best, 0.f)));
-      bi = static_cast<int>(__reduce_min_sync(0xffffffffu, __float_as_uint(fmaxf(best, 0.f)) == best_bits ? static_cast<unsigned>(bi) : 0x7fffffffu));
-      best = __uint_as_float(best_bits);
-      const float w = best * inv;
-      if (lane == j) { my_w = w; my_i = bi; }
-      wsum += w;
-#pragma unroll
-      for (int i = 0; i < ROUTE_REG_PER_LANE; ++i)
-        if (bi == lane + 32 * i) v[i] = -2.f;
-    }
-  } else {
-    float mx = -INFINITY;
-    for (int e = lane; e < E; e += 32) {
-      const float v = load_act(logits, dtype, static_cast<int64_t>(t) * E + e);
-      p[e] = v;
-      mx = fmaxf(mx, v);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    float sum = 0.f;
-    for (int e = lane; e < E; e += 32) {
-      const float v = expf(p[e] - mx);
-      p[e] = v;
-      sum += v;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    const float inv = 1.f / sum;
-    __syncwarp();
-    for (int j = 0; j < k; ++j) {
-      float best = -1.f;
-      int bi = 0x7fffffff;
-      for (int e = lane; e < E; e += 32) {
-        const float v = p[e];
-        if (v > best) { best = v; bi = e; }   // strided scan visits ascending e: first hit wins ties
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-      }
-      const float w = best * inv;
-      if (lane == j) { my_w = w; my_i = bi; }
-      wsum += w;
-      if (lane == 0) p[bi] = -2.f;
-      __syncwarp();
-    }
-  }
-  if (lane < k) {
-    float w = renorm ? my_w / wsum : my_w;
-    if (weight_round == BM_ROUND_F16) w = __half2float(__float2half_rn(w));
-    else if (weight_round == BM_ROUND_BF16) w = __bfloat162float(__float2bfloat16_rn(w));
-    idx_out[static_cast<int64_t>(t) * k + lane] = my_i;
-    w_out[static_cast<int64_t>(t) * k + lane] = w;
-  }
-  __syncwarp();
-}
-
-// One warp per token; probabilities live in a warp-private shared row.
+// One warp per token, the probabilities in registers.
+template <int REG>
 __global__ void __launch_bounds__(256) route_topk_kernel(const void* __restrict__ logits, int dtype, int T, int E, int k,
                                                         int renorm, int weight_round, int32_t* __restrict__ topk_idx,
                                                         float* __restrict__ topk_w) {
-  extern __shared__ float sm_prob[];  // [warps][E]
-  const int warp = threadIdx.x >> 5;
-  const int t = blockIdx.x * (blockDim.x >> 5) + warp;
+  const int lane = threadIdx.x & 31;
+  const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= T) return;
-  warp_topk_token(logits, dtype, t, E, k, renorm, weight_round, sm_prob + warp * E, topk_idx, topk_w);
+  int idx;
+  float w;
+  warp_topk<REG>(logits, dtype, t, E, k, renorm, weight_round, &idx, &w);
+  if (lane < k) {
+    topk_idx[static_cast<int64_t>(t) * k + lane] = idx;
+    topk_w[static_cast<int64_t>(t) * k + lane] = w;
+  }
 }
 
 // ---------------------------------------------------------------- permutation
@@ -277,7 +183,7 @@ __global__ void __launch_bounds__(ROUTE_BLOCK) route_build_fused_kernel(
   write_tile_table(s.scan, E, tile_rows, tile_table, max_tiles, counts, reinterpret_cast<int*>(s.warp_base), s.block_count);
 }
 
-// A > ROUTE_BLOCK: count per block, scan across blocks, scatter.
+// A > ROUTE_BLOCK: counts per block of assignments, prefixes across the blocks, scatter.
 __global__ void __launch_bounds__(ROUTE_BLOCK) route_count_kernel(const int32_t* __restrict__ topk_idx,
                                                                  const int32_t* __restrict__ g2l, int num_routed, int A, int E,
                                                                  int32_t* __restrict__ block_hist /*[nblocks][E]*/) {
@@ -290,62 +196,75 @@ __global__ void __launch_bounds__(ROUTE_BLOCK) route_count_kernel(const int32_t*
   for (int x = threadIdx.x; x < E; x += blockDim.x) block_hist[static_cast<int64_t>(blockIdx.x) * E + x] = s.block_count[x];
 }
 
+// block_hist -> exclusive prefixes over the blocks, and the experts' totals.  A CTA owns 32 experts (a lane each), its
+// warps cut the blocks into runs: sums, a prefix over the runs in shared memory, prefixes.
 __global__ void __launch_bounds__(ROUTE_BLOCK) route_scan_kernel(int32_t* __restrict__ block_hist, int nblocks, int E,
-                                                                int tile_rows, int32_t* __restrict__ expert_offsets,
-                                                                int32_t* __restrict__ tile_table, int max_tiles,
-                                                                int32_t* __restrict__ counts) {
-  __shared__ int tot[ROUTE_MAX_E];
-  __shared__ int off[ROUTE_MAX_E + 1];
-  __shared__ int scratch[ROUTE_MAX_E + 1];
-  __shared__ int chunk_tot[ROUTE_BLOCK];
-  // The blocks' histograms are cut into `chunks` runs per expert, one thread each: every thread sums its run (independent
-  // loads), the runs' totals are combined in shared memory, and a second walk over the run writes the exclusive prefixes.
-  // One thread per expert walking all the blocks would serialise nblocks dependent round trips to memory.
-  const int chunks = max(1, min(static_cast<int>(blockDim.x) / E, nblocks));
-  const int len = (nblocks + chunks - 1) / chunks;
-  const int x = threadIdx.x % E, c = threadIdx.x / E;
-  const int b0 = c * len, b1 = min(nblocks, b0 + len);
-  const bool active = c < chunks;
-  if (active) {
-    int sum = 0;
+                                                                int32_t* __restrict__ total) {
+  __shared__ int run_tot[ROUTE_WARPS][33];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, x = blockIdx.x * 32 + lane;
+  const int len = (nblocks + ROUTE_WARPS - 1) / ROUTE_WARPS, b0 = warp * len, b1 = min(nblocks, b0 + len);
+  int sum = 0;
+  if (x < E)
 #pragma unroll 8
     for (int b = b0; b < b1; ++b) sum += block_hist[static_cast<int64_t>(b) * E + x];
-    chunk_tot[c * E + x] = sum;
-  }
+  run_tot[warp][lane] = sum;
   __syncthreads();
-  if (active) {
-    int run = 0;
-    for (int cc = 0; cc < c; ++cc) run += chunk_tot[cc * E + x];
-    if (c == chunks - 1) tot[x] = run + chunk_tot[c * E + x];
+  int run = 0;
+  for (int w = 0; w < warp; ++w) run += run_tot[w][lane];
+  if (x >= E) return;
 #pragma unroll 8
-    for (int b = b0; b < b1; ++b) {
-      const int v = block_hist[static_cast<int64_t>(b) * E + x];
-      block_hist[static_cast<int64_t>(b) * E + x] = run;
-      run += v;
-    }
+  for (int b = b0; b < b1; ++b) {
+    const int v = block_hist[static_cast<int64_t>(b) * E + x];
+    block_hist[static_cast<int64_t>(b) * E + x] = run;
+    run += v;
   }
-  __syncthreads();
-  block_exclusive_scan(tot, off, E);
-  for (int i = threadIdx.x; i <= E; i += blockDim.x) expert_offsets[i] = off[i];
-  write_tile_table(off, E, tile_rows, tile_table, max_tiles, counts, scratch, tot);
+  if (warp == ROUTE_WARPS - 1) total[x] = run;
 }
 
+// Every block scans the totals for itself; the first one also writes the offsets and the tile table.
 __global__ void __launch_bounds__(ROUTE_BLOCK) route_scatter_kernel(
     const int32_t* __restrict__ topk_idx, const float* __restrict__ topk_w, const int32_t* __restrict__ g2l, int num_routed,
-    int A, int k, int E, const int32_t* __restrict__ block_hist, const int32_t* __restrict__ expert_offsets,
-    int32_t* __restrict__ token_indices, float* __restrict__ route_flat) {
+    int A, int k, int E, const int32_t* __restrict__ block_hist, const int32_t* __restrict__ total, int tile_rows,
+    int32_t* __restrict__ expert_offsets, int32_t* __restrict__ token_indices, float* __restrict__ route_flat, int32_t* __restrict__ tile_table,
+    int max_tiles, int32_t* __restrict__ counts) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   RouteSmem s = carve_route_smem(sm_raw, E);
+  block_exclusive_scan(total, s.scan, E);
   const int i = blockIdx.x * ROUTE_BLOCK + threadIdx.x;
   int e = -1;
   if (i < A) e = local_expert(topk_idx, g2l, i, num_routed, E);
   const int rank_w = block_count_and_rank(e, E, s);
   if (e >= 0) {
-    const int pos = expert_offsets[e] + block_hist[static_cast<int64_t>(blockIdx.x) * E + e] +
-                    s.warp_base[(threadIdx.x >> 5) * E + e] + rank_w;
+    const int pos = s.scan[e] + block_hist[static_cast<int64_t>(blockIdx.x) * E + e] + s.warp_base[(threadIdx.x >> 5) * E + e] + rank_w;
     token_indices[pos] = i / k;
     route_flat[pos] = topk_w[i];
   }
+  if (blockIdx.x == 0) {
+    for (int x = threadIdx.x; x <= E; x += blockDim.x) expert_offsets[x] = s.scan[x];
+    __syncthreads();
+    write_tile_table(s.scan, E, tile_rows, tile_table, max_tiles, counts, reinterpret_cast<int*>(s.warp_base), s.block_count);
+  }
+}
+
+// f<REG>() for the register class of E experts (E <= ROUTE_MAX_E)
+#define BM_TOPK_CLASS(E, CALL)                          \
+  do {                                                  \
+    if ((E) <= 64) { constexpr int REG = 2; CALL; }     \
+    else if ((E) <= 128) { constexpr int REG = 4; CALL; }  \
+    else if ((E) <= 256) { constexpr int REG = 8; CALL; }  \
+    else if ((E) <= 512) { constexpr int REG = 16; CALL; } \
+    else { constexpr int REG = 32; CALL; }              \
+  } while (0)
+
+static int set_route_attributes(int dev) {
+  static PerDeviceOnce attr_once;
+  if (attr_once.is_done(dev)) return BM_OK;
+  const int big = static_cast<int>(route_smem_bytes(ROUTE_MAX_E));
+  BM_CUDA(cudaFuncSetAttribute(route_build_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  BM_CUDA(cudaFuncSetAttribute(route_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  BM_CUDA(cudaFuncSetAttribute(route_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  attr_once.mark(dev);
+  return BM_OK;
 }
 
 }  // namespace bm
@@ -361,8 +280,8 @@ extern "C" int bm_route_topk(const void* logits, int logits_dtype, int32_t T, in
   if (T == 0) return BM_OK;
   BM_REQUIRE(logits && topk_idx && topk_w, BM_ERR_INVALID_ARG, "route_topk: null pointer");
   const int warps = 8;
-  route_topk_kernel<<<(T + warps - 1) / warps, warps * 32, sizeof(float) * warps * E, static_cast<cudaStream_t>(stream)>>>(
-      logits, logits_dtype, T, E, k, renorm, weight_round, topk_idx, topk_w);
+  BM_TOPK_CLASS(E, (route_topk_kernel<REG><<<(T + warps - 1) / warps, warps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
+                       logits, logits_dtype, T, E, k, renorm, weight_round, topk_idx, topk_w)));
   BM_LAUNCH_CHECK("route_topk_kernel");
   return BM_OK;
 }
@@ -379,8 +298,7 @@ extern "C" int32_t bm_route_max_tiles(int32_t T, int32_t k, int32_t num_local, i
 extern "C" size_t bm_route_build_workspace_bytes(int32_t T, int32_t k, int32_t num_local) {
   const int64_t A = static_cast<int64_t>(T) * k;
   if (A <= bm::ROUTE_BLOCK) return 0;
-  const int64_t nblocks = (A + bm::ROUTE_BLOCK - 1) / bm::ROUTE_BLOCK;
-  return bm::align_up(static_cast<size_t>(nblocks) * num_local * sizeof(int32_t), 256);
+  return bm::align_up(static_cast<size_t>((A + bm::ROUTE_BLOCK - 1) / bm::ROUTE_BLOCK + 1) * num_local * sizeof(int32_t), 256);     // histograms, totals
 }
 
 extern "C" int bm_route_build(const int32_t* topk_idx, const float* topk_w, const int32_t* global_to_local,
@@ -403,16 +321,10 @@ extern "C" int bm_route_build(const int32_t* topk_idx, const float* topk_w, cons
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int max_tiles = bm_route_max_tiles(T, k, num_local, tile_rows);
   const size_t smem = route_smem_bytes(num_local);
-  static PerDeviceOnce attr_once;
   int dev = -1;
   BM_CUDA(cudaGetDevice(&dev));
-  if (!attr_once.is_done(dev)) {
-    const int big = static_cast<int>(route_smem_bytes(ROUTE_MAX_E));
-    BM_CUDA(cudaFuncSetAttribute(route_build_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    BM_CUDA(cudaFuncSetAttribute(route_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    BM_CUDA(cudaFuncSetAttribute(route_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
-    attr_once.mark(dev);
-  }
+  const int rc = set_route_attributes(dev);
+  if (rc) return rc;
   if (A <= ROUTE_BLOCK) {
     route_build_fused_kernel<<<1, ROUTE_BLOCK, smem, st>>>(topk_idx, topk_w, global_to_local, num_routed, A, k, num_local, tile_rows,
                                                            token_indices, expert_offsets, route_flat, tile_table,
@@ -424,14 +336,14 @@ extern "C" int bm_route_build(const int32_t* topk_idx, const float* topk_w, cons
   const size_t need = bm_route_build_workspace_bytes(T, k, num_local);
   BM_REQUIRE(workspace && workspace_bytes >= need, BM_ERR_WORKSPACE, "route_build: workspace of %zu bytes needed, %zu given",
              need, workspace_bytes);
-  int32_t* block_hist = static_cast<int32_t*>(workspace);
+  int32_t* total = static_cast<int32_t*>(workspace);
+  int32_t* block_hist = total + num_local;
   route_count_kernel<<<nblocks, ROUTE_BLOCK, smem, st>>>(topk_idx, global_to_local, num_routed, A, num_local, block_hist);
   BM_LAUNCH_CHECK("route_count_kernel");
-  route_scan_kernel<<<1, ROUTE_BLOCK, 0, st>>>(block_hist, nblocks, num_local, tile_rows, expert_offsets, tile_table,
-                                               max_tiles, counts);
+  route_scan_kernel<<<(num_local + 31) / 32, ROUTE_BLOCK, 0, st>>>(block_hist, nblocks, num_local, total);
   BM_LAUNCH_CHECK("route_scan_kernel");
   route_scatter_kernel<<<nblocks, ROUTE_BLOCK, smem, st>>>(topk_idx, topk_w, global_to_local, num_routed, A, k, num_local, block_hist,
-                                                           expert_offsets, token_indices, route_flat);
+                                                           total, tile_rows, expert_offsets, token_indices, route_flat, tile_table, max_tiles, counts);
   BM_LAUNCH_CHECK("route_scatter_kernel");
   return BM_OK;
 }

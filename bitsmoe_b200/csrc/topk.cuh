@@ -36,25 +36,35 @@ __device__ __forceinline__ void warp_topk(const void* __restrict__ logits, int d
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const float inv = 1.f / sum;
+  // A lane keeps its best probability; only the lane whose probability was taken looks through its own again.
+  float best;
+  int bi;
+  auto look = [&]() {
+    best = v[0];
+    bi = 0;
+#pragma unroll
+    for (int i = 1; i < REG; ++i) {
+      bi = v[i] > best ? i : bi;                 // ascending e: the first hit wins ties
+      best = fmaxf(v[i], best);
+    }
+  };
+  look();
   float my_w = 0.f, wsum = 0.f;
   int my_i = 0;
   for (int j = 0; j < k; ++j) {
-    float best = -1.f;
-    int bi = 0x7fffffff;
-#pragma unroll
-    for (int i = 0; i < REG; ++i)
-      if (v[i] > best) { best = v[i]; bi = lane + 32 * i; }   // ascending e: the first hit wins ties
     // probabilities are non-negative, so their bit patterns order like unsigned integers: two warp reductions
     // (largest value, then the lowest expert id holding it) replace a ten-shuffle butterfly
     const unsigned bits = __float_as_uint(fmaxf(best, 0.f));
     const unsigned best_bits = __reduce_max_sync(0xffffffffu, bits);
-    bi = static_cast<int>(__reduce_min_sync(0xffffffffu, bits == best_bits ? static_cast<unsigned>(bi) : 0x7fffffffu));
+    const int e = static_cast<int>(__reduce_min_sync(0xffffffffu, bits == best_bits && best >= 0.f ? static_cast<unsigned>(lane + 32 * bi) : 0x7fffffffu));
     const float w = __uint_as_float(best_bits) * inv;
-    if (lane == j) { my_w = w; my_i = bi; }
+    if (lane == j) { my_w = w; my_i = e; }
     wsum += w;
+    if ((e & 31) == lane) {
 #pragma unroll
-    for (int i = 0; i < REG; ++i)
-      if (bi == lane + 32 * i) v[i] = -2.f;
+      for (int i = 0; i < REG; ++i) v[i] = e == lane + 32 * i ? -2.f : v[i];
+      look();
+    }
   }
   *idx = my_i;
   *weight = round_route_weight(renorm ? my_w / wsum : my_w, weight_round);
