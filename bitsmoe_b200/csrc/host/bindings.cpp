@@ -364,7 +364,7 @@ at::Tensor ints(const std::vector<int32_t>& v, int64_t cols) {
 }
 
 // (rank_major fp32 [rank, dim] CUDA, s fp32 [rank] on the same device, [(bits, [(start, end), ...]), ...], to_host) ->
-// (payload, rank_idx, tile_meta, slab_meta, scale, s, segments): payload, scale and s on the factor's device, or with
+// (payload, rank_idx, tile_meta, slab_meta, scale, s, segments, original indices, original rank): payload, scale and s on the factor's device, or with
 // to_host fetched in one copy into host tensors of their own
 PyObject* pack_matrix(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return guarded([&]() -> PyObject* {
@@ -401,28 +401,43 @@ PyObject* pack_matrix(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const int64_t stored = static_cast<int64_t>(rows.size());
     const c10::cuda::CUDAGuard guard(w.device());
     const auto dev = at::TensorOptions().device(w.device());
-    at::Tensor payload, scale, s_out;
+    at::Tensor payload, scale, s_out, tables[6];
+    auto make_tables = [&] {
+      tables[0] = ints(rows, 0);
+      tables[1] = ints(tile_meta, 3);
+      tables[2] = ints(slab_meta, 4);
+      tables[3] = ints(segments, 3);
+      tables[4] = ints(rows, 0);      // the original indices: a tensor of their own
+      tables[5] = at::empty({}, at::kInt);
+      *static_cast<int32_t*>(tables[5].data_ptr()) = static_cast<int32_t>(w.size(0));
+    };
     if (to_host) {
       // one device buffer and one pinned one: a single copy, then plain memory copies
       auto up = [](int64_t v) { return (v + 255) & ~static_cast<int64_t>(255); };
       const int64_t o_scale = up(words * 4), o_s = o_scale + up(scales * 2), total = o_s + stored * 2;
-      payload = at::empty({words}, at::kUInt32);
-      scale = at::empty({scales}, at::kHalf);
-      s_out = at::empty({stored}, at::kHalf);
+      at::Tensor h;
+      cudaStream_t stream = nullptr;
       if (total > 0) {
         const at::Tensor d = at::empty({total}, dev.dtype(at::kByte));
-        const at::Tensor h = at::empty({total}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
+        h = at::empty({total}, at::TensorOptions().dtype(at::kByte).pinned_memory(true));
         char* base = static_cast<char*>(d.data_ptr());
         check(bm_quantize_pack_matrix(static_cast<const float*>(w.data_ptr()), w.stride(0), static_cast<const float*>(s.data_ptr()),
                                       static_cast<int32_t>(dim), rows.data(), slabs.data(), static_cast<int32_t>(slabs.size() / 2),
                                       reinterpret_cast<uint32_t*>(base), reinterpret_cast<uint16_t*>(base + o_scale),
                                       reinterpret_cast<uint16_t*>(base + o_s), stream_of(w.device())));
-        const auto stream = c10::cuda::getCurrentCUDAStream(w.device().index());
-        const cudaError_t e = cudaMemcpyAsync(h.data_ptr(), base, total, cudaMemcpyDeviceToHost, stream.stream());
+        stream = c10::cuda::getCurrentCUDAStream(w.device().index()).stream();
+        const cudaError_t e = cudaMemcpyAsync(h.data_ptr(), base, total, cudaMemcpyDeviceToHost, stream);
         if (e != cudaSuccess) fail(PyExc_RuntimeError, cudaGetErrorString(e));
+      }
+      // everything that does not need the device's answer is made while it works
+      payload = at::empty({words}, at::kUInt32);
+      scale = at::empty({scales}, at::kHalf);
+      s_out = at::empty({stored}, at::kHalf);
+      make_tables();
+      if (total > 0) {
         cudaError_t done;
         Py_BEGIN_ALLOW_THREADS
-        done = cudaStreamSynchronize(stream.stream());
+        done = cudaStreamSynchronize(stream);
         Py_END_ALLOW_THREADS
         if (done != cudaSuccess) fail(PyExc_RuntimeError, cudaGetErrorString(done));
         const char* hb = static_cast<const char*>(h.data_ptr());
@@ -438,10 +453,11 @@ PyObject* pack_matrix(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                     static_cast<int32_t>(dim), rows.data(), slabs.data(), static_cast<int32_t>(slabs.size() / 2),
                                     static_cast<uint32_t*>(payload.data_ptr()), static_cast<uint16_t*>(scale.data_ptr()),
                                     static_cast<uint16_t*>(s_out.data_ptr()), stream_of(w.device())));
+      make_tables();
     }
-    const at::Tensor out[7] = {payload, ints(rows, 0), ints(tile_meta, 3), ints(slab_meta, 4), scale, s_out, ints(segments, 3)};
-    PyObject* r = PyTuple_New(7);
-    for (int i = 0; i < 7; ++i) PyTuple_SET_ITEM(r, i, THPVariable_Wrap(out[i]));
+    const at::Tensor out[9] = {payload, tables[0], tables[1], tables[2], scale, s_out, tables[3], tables[4], tables[5]};
+    PyObject* r = PyTuple_New(9);
+    for (int i = 0; i < 9; ++i) PyTuple_SET_ITEM(r, i, THPVariable_Wrap(out[i]));
     return r;
   });
 }

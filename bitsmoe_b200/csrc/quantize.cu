@@ -45,11 +45,14 @@ __device__ __forceinline__ void quantize_pack_group(const float (&x)[MICROS], co
   }
   // means are sums divided by the count, products and sums rounded separately (no fused multiply-add), as the
   // element-wise torch expressions of the reference round them
-  const float n_f = static_cast<float>(n_valid);
+  // (a count that is a power of two has an exact reciprocal: its product rounds to what the quotient rounds to)
+  const float n_f = static_cast<float>(n_valid), n_inv = 1.f / n_f;
+  const bool pow2 = (n_valid & (n_valid - 1)) == 0;
+  auto mean = [&](float sum) { return pow2 ? __fmul_rn(sum, n_inv) : __fdiv_rn(sum, n_f); };
   float sabs = 0.f;
 #pragma unroll
   for (int m = 0; m < MICROS; ++m) sabs = __fadd_rn(sabs, fabsf(x[m]));
-  const float mean_abs = fmaxf(__fdiv_rn(warp_sum(sabs), n_f), Q_EPS);
+  const float mean_abs = fmaxf(mean(warp_sum(sabs)), Q_EPS);
   const int hi = (1 << (bits - 1)) - 1, lo = -hi - 1;
   float q[MICROS];
   float scale;
@@ -60,16 +63,16 @@ __device__ __forceinline__ void quantize_pack_group(const float (&x)[MICROS], co
   } else if (bits <= 4) {
     scale = mean_abs;
     for (int it = 0; it < 50; ++it) {
-      float xq = 0.f, qq = 0.f;
+      float xq = 0.f;
+      int qq = 0;      // whole and below 2^24: the same sum in any order, so the integer adder takes it in one step
 #pragma unroll
       for (int m = 0; m < MICROS; ++m) {
         q[m] = fminf(fmaxf(rintf(__fdiv_rn(x[m], scale)), static_cast<float>(lo)), static_cast<float>(hi));
         xq = __fadd_rn(xq, __fmul_rn(x[m], q[m]));
-        qq = __fadd_rn(qq, __fmul_rn(q[m], q[m]));
+        qq += static_cast<int>(q[m]) * static_cast<int>(q[m]);
       }
-      xq = __fdiv_rn(warp_sum(xq), n_f);
-      qq = __fdiv_rn(warp_sum(qq), n_f);
-      const float next = fmaxf(__fdiv_rn(xq, __fadd_rn(qq, Q_EPS)), Q_EPS);
+      const float mean_qq = mean(static_cast<float>(__reduce_add_sync(0xffffffffu, qq)));
+      const float next = fmaxf(__fdiv_rn(mean(warp_sum(xq)), __fadd_rn(mean_qq, Q_EPS)), Q_EPS);
       if (next == scale) break;
       scale = next;
     }

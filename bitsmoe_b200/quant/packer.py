@@ -193,9 +193,8 @@ def pack_rank_major(rank_major: Tensor, s_vec: Tensor, segments, groupsize: int 
         if rows.stride(1) != 1 or rows.stride(0) < dim:
             rows = rows.contiguous()
         out = capi.host().pack_matrix(rows, s_vec.detach().to(torch.float32).contiguous(), bucket_ranges(segments, rank), to_host)
-        buf = dict(zip(("payload_buffer", "rank_idx_buffer", "tile_meta_buffer", "slab_meta_buffer", "scale_buffer", "s_buffer", "segments"), out))
-        buf["original_indices"] = buf["rank_idx_buffer"].clone()
-        buf["original_rank"] = torch.tensor(rank, dtype=torch.int32)
+        buf = dict(zip(("payload_buffer", "rank_idx_buffer", "tile_meta_buffer", "slab_meta_buffer", "scale_buffer", "s_buffer",
+                        "segments", "original_indices", "original_rank"), out))
         buf["groupsize"] = torch.tensor(groupsize, dtype=torch.int16)
         return buf
     tiles = (dim + N_TILE - 1) // N_TILE
