@@ -50,7 +50,7 @@ struct SkinnyArgs {
   // The launch may start while the kernel before it drains.  Weights are read before that kernel is complete, so only for
   // a launch that follows another one of the same entry point: whatever wrote the weights came before that one.
   int overlap;
-  int row_tiles;           // filled in by the launcher
+  int row_tiles, clusters; // filled in by the launcher
 };
 
 // BM_ERR_UNSUPPORTED (nothing launched) when the shape does not tile; the caller then takes a general GEMM.
