@@ -36,16 +36,23 @@ __device__ __forceinline__ void warp_topk(const void* __restrict__ logits, int d
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const float inv = 1.f / sum;
-  // A lane keeps its best probability; only the lane whose probability was taken looks through its own again.
-  float best;
-  int bi;
+  // A lane keeps the best two of its probabilities that come after the last one taken from it (largest first, equal ones by
+  // ascending expert id) and looks through its own again only when both are gone: with the choices spread over 32 lanes
+  // that is about k^2 / 64 times a token, where keeping one would look k times.
+  float best, second, last = INFINITY;
+  int bi, si, last_i = -1;
   auto look = [&]() {
-    best = v[0];
-    bi = 0;
+    best = second = -1.f;
+    bi = si = 0;
 #pragma unroll
-    for (int i = 1; i < REG; ++i) {
-      bi = v[i] > best ? i : bi;                 // ascending e: the first hit wins ties
-      best = fmaxf(v[i], best);
+    for (int i = 0; i < REG; ++i) {
+      const bool open = v[i] < last || (v[i] == last && i > last_i);
+      const float c = open ? v[i] : -1.f;
+      const bool first = c > best, next = c > second;      // ascending e: the earlier one wins ties
+      si = first ? bi : next ? i : si;
+      second = first ? best : next ? c : second;
+      bi = first ? i : bi;
+      best = first ? c : best;
     }
   };
   look();
@@ -60,10 +67,13 @@ __device__ __forceinline__ void warp_topk(const void* __restrict__ logits, int d
     const float w = __uint_as_float(best_bits) * inv;
     if (lane == j) { my_w = w; my_i = e; }
     wsum += w;
-    if ((e & 31) == lane) {
-#pragma unroll
-      for (int i = 0; i < REG; ++i) v[i] = e == lane + 32 * i ? -2.f : v[i];
-      look();
+    if (e == lane + 32 * bi && best >= 0.f) {
+      last = best;
+      last_i = bi;
+      best = second;
+      bi = si;
+      second = -1.f;
+      if (REG > 1 && best < 0.f) look();
     }
   }
   *idx = my_i;
