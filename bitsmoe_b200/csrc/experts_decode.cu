@@ -89,11 +89,13 @@ struct DecUnitInfo {
   int npass, tile0, ntiles, pad_;
 };
 
+// a / b for 0 <= a < 2^20, 1 <= b: the quotient of a + 1/2 stays 1 / (2 b) away from a whole number, more than its rounding
+__device__ __forceinline__ int div_small(int a, int b) { return static_cast<int>(__fdividef(static_cast<float>(a) + 0.5f, static_cast<float>(b))); }
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(DEC_CONSUMERS) : "memory"); }
 
-// Bounded wait shared by all roles: gives up when another thread of the CTA already did, or after limit_ns.
-__device__ __forceinline__ bool dec_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns) {
-  const uint32_t addr = tc::smem_u32(bar);
+// Bounded wait shared by all roles: one plain probe (a wait that is already over costs 35 cycles, with a suspend time
+// given 250), then a loop out of line that gives up when another thread of the CTA already did, or after limit_ns.
+__device__ __noinline__ bool dec_wait_slow(uint32_t addr, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns) {
   uint64_t t0 = 0;
   for (uint32_t i = 0;; ++i) {
     uint32_t done;
@@ -110,6 +112,15 @@ __device__ __forceinline__ bool dec_wait(uint64_t* bar, uint32_t parity, volatil
       else if (now - t0 > limit_ns) { *abort_flag = 1; return false; }
     }
   }
+}
+__device__ __forceinline__ bool dec_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, uint64_t limit_ns) {
+  const uint32_t addr = tc::smem_u32(bar);
+  uint32_t done;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(done)
+               : "r"(addr), "r"(parity)
+               : "memory");
+  return done ? true : dec_wait_slow(addr, parity, abort_flag, limit_ns);
 }
 
 __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -134,69 +145,76 @@ __device__ __forceinline__ void dense_afrag(uint32_t w, uint32_t (&a)[4]) {
 
 // `npairs` pairs of 16x16 blocks of one group against the token-side operand.  `wp` points at this lane's word(s) of
 // the first pair, consecutive pairs are `stride` words apart; `bp` points at this lane's eight halves of the first
-// pair (operand row g, position 8 t).  The products are sums over the STORED codes u = q + offset.
+// pair (operand row g, position 8 t).  The products are sums over the STORED codes u = q + offset.  The two blocks of a
+// pair go to accumulators of their own, and a pair's words and operands are read while the pair before is multiplied:
+// what bounds a tile is the latency of this chain, not the tensor pipe.
+template <bool DENSE>
+__device__ __forceinline__ uint2 pair_words(const uint32_t* wp) {
+  if (DENSE) { const uint32_t w = *wp; return make_uint2(w, w >> 8); }
+  return *reinterpret_cast<const uint2*>(wp);
+}
+template <bool DENSE>
+__device__ __forceinline__ void mma_pair(float (&acc)[2][4], const uint2& w, const uint4& b) {
+  uint32_t a[4], c[4];
+  if (DENSE) { dense_afrag(w.x, a); dense_afrag(w.y, c); }
+  else { nib_afrag(w.x, a); nib_afrag(w.y, c); }
+  mma_16816(acc[0], a, b.x, b.y);
+  mma_16816(acc[1], c, b.z, b.w);
+}
 template <bool DENSE>
 __device__ __forceinline__ void mma_pairs(const uint32_t* __restrict__ wp, int stride, int npairs, const __half* __restrict__ bp,
-                                          float (&acc)[4]) {
+                                          float (&acc)[2][4]) {
+  if (npairs <= 0) return;
+  uint2 w = pair_words<DENSE>(wp);
+  uint4 b = *reinterpret_cast<const uint4*>(bp);
 #pragma unroll 2
-  for (int p = 0; p < npairs; ++p) {
-    const uint4 b = *reinterpret_cast<const uint4*>(bp);
-    uint32_t a[4];
-    if (DENSE) {
-      const uint32_t w = *wp;
-      dense_afrag(w, a);
-      mma_16816(acc, a, b.x, b.y);
-      dense_afrag(w >> 8, a);
-      mma_16816(acc, a, b.z, b.w);
-    } else {
-      const uint2 w = *reinterpret_cast<const uint2*>(wp);
-      nib_afrag(w.x, a);
-      mma_16816(acc, a, b.x, b.y);
-      nib_afrag(w.y, a);
-      mma_16816(acc, a, b.z, b.w);
-    }
+  for (int p = 1; p < npairs; ++p) {
     wp += stride;
     bp += 32;
+    const uint2 w_next = pair_words<DENSE>(wp);
+    const uint4 b_next = *reinterpret_cast<const uint4*>(bp);
+    mma_pair<DENSE>(acc, w, b);
+    w = w_next;
+    b = b_next;
   }
+  mma_pair<DENSE>(acc, w, b);
 }
 
-// The same for the gate and up sections of one tile at once (equal group sizes): two independent accumulator chains.
+// The same for the gate and up sections of one tile at once (equal group sizes): four independent accumulator chains.
 template <bool DENSE>
 __device__ __forceinline__ void mma_pairs2(const uint32_t* __restrict__ wp0, const uint32_t* __restrict__ wp1, int stride, int npairs,
-                                           const __half* __restrict__ bp0, const __half* __restrict__ bp1, float (&acc0)[4],
-                                           float (&acc1)[4]) {
+                                           const __half* __restrict__ bp0, const __half* __restrict__ bp1, float (&acc0)[2][4],
+                                           float (&acc1)[2][4]) {
+  if (npairs <= 0) return;
+  uint2 w0 = pair_words<DENSE>(wp0), w1 = pair_words<DENSE>(wp1);
+  uint4 b0 = *reinterpret_cast<const uint4*>(bp0), b1 = *reinterpret_cast<const uint4*>(bp1);
 #pragma unroll 2
-  for (int p = 0; p < npairs; ++p) {
-    const uint4 b0 = *reinterpret_cast<const uint4*>(bp0);
-    const uint4 b1 = *reinterpret_cast<const uint4*>(bp1);
-    uint32_t a[4], c[4];
-    if (DENSE) {
-      const uint32_t w0 = *wp0, w1 = *wp1;
-      dense_afrag(w0, a);
-      dense_afrag(w1, c);
-      mma_16816(acc0, a, b0.x, b0.y);
-      mma_16816(acc1, c, b1.x, b1.y);
-      dense_afrag(w0 >> 8, a);
-      dense_afrag(w1 >> 8, c);
-      mma_16816(acc0, a, b0.z, b0.w);
-      mma_16816(acc1, c, b1.z, b1.w);
-    } else {
-      const uint2 w0 = *reinterpret_cast<const uint2*>(wp0);
-      const uint2 w1 = *reinterpret_cast<const uint2*>(wp1);
-      nib_afrag(w0.x, a);
-      nib_afrag(w1.x, c);
-      mma_16816(acc0, a, b0.x, b0.y);
-      mma_16816(acc1, c, b1.x, b1.y);
-      nib_afrag(w0.y, a);
-      nib_afrag(w1.y, c);
-      mma_16816(acc0, a, b0.z, b0.w);
-      mma_16816(acc1, c, b1.z, b1.w);
-    }
+  for (int p = 1; p < npairs; ++p) {
     wp0 += stride;
     wp1 += stride;
     bp0 += 32;
     bp1 += 32;
+    const uint2 w0_next = pair_words<DENSE>(wp0), w1_next = pair_words<DENSE>(wp1);
+    const uint4 b0_next = *reinterpret_cast<const uint4*>(bp0), b1_next = *reinterpret_cast<const uint4*>(bp1);
+    mma_pair<DENSE>(acc0, w0, b0);
+    mma_pair<DENSE>(acc1, w1, b1);
+    w0 = w0_next;
+    w1 = w1_next;
+    b0 = b0_next;
+    b1 = b1_next;
   }
+  mma_pair<DENSE>(acc0, w0, b0);
+  mma_pair<DENSE>(acc1, w1, b1);
+}
+
+// One 16-slot block of the down matrix against a tile's 128 columns (four pairs), whose operands `b` the caller holds.
+template <bool DENSE>
+__device__ __forceinline__ void mma_down(const uint32_t* __restrict__ wp, const uint4 (&b)[4], float (&acc)[2][4]) {
+  uint2 w[4];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) w[p] = pair_words<DENSE>(wp + p * (DENSE ? 32 : 64));
+#pragma unroll
+  for (int p = 0; p < 4; ++p) mma_pair<DENSE>(acc, w[p], b[p]);
 }
 
 __device__ __forceinline__ float sum8_halves(const uint4& v) {
@@ -214,7 +232,7 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
 // MAXMB: 16-slot blocks of the down matrix per warp (2: up to 256 slots, 4: up to 512); the smaller instance keeps the
 // kernel's code, which the instruction cache has to hold, short.
 template <int MAXMB>
-__global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecParams P) {
+__global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const DecParams P) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ DecUnitInfo info[2];
   __shared__ __align__(8) uint64_t bar_full[DEC_MAX_RING];
@@ -225,7 +243,7 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
   __shared__ int warp_tot[DEC_THREADS / 32];
   __shared__ float corr[2][2 * FAST_MAX_TOK];    // [buffer][matrix * 8 + token]: offset-weighted operand sums
   __shared__ __align__(16) float zsum_part[2][FAST_MAX_TOK][8]; // [buffer][token][warp]: partial sums of z over the warp's 16 columns
-  __shared__ int abort_raw;
+  __shared__ int abort_raw, first_expert;
   volatile int* abort_flag = &abort_raw;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -251,7 +269,7 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // ---- passes per expert (ceil(assignments / 8)) and their exclusive prefix: 4 consecutive experts per thread
-  int total_passes;
+  int total_passes, n_split;
   {
     const int e0 = tid * 4;
     int o[5];
@@ -281,20 +299,23 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
       all += n;
     }
     total_passes = all;
+    if (total_passes == 0) return;
+    // tile ranges: as many splits per expert as keep the number of units within one round of the grid
+    n_split = div_small(static_cast<int>(gridDim.x), total_passes);
+    n_split = n_split < 1 ? 1 : (n_split > P.n_tiles ? P.n_tiles : n_split);
+    n_split = div_small(P.n_tiles - 1, div_small(P.n_tiles + n_split - 1, n_split)) + 1;
+    // the CTA's first unit is found by the thread that holds its expert, the later ones by a search
+    const int first_pass = div_small(static_cast<int>(blockIdx.x), n_split);
     int run = before + incl - sum;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       if (e0 + i < P.num_experts) pbase[e0 + i] = static_cast<uint16_t>(run);
+      if (first_pass >= run && first_pass < run + pass[i]) first_expert = e0 + i;
       run += pass[i];
     }
     __syncthreads();
   }
-  if (total_passes == 0) return;
-  // tile ranges: as many splits per expert as keep the number of units within one round of the grid
-  int n_split = static_cast<int>(gridDim.x) / total_passes;
-  n_split = n_split < 1 ? 1 : (n_split > P.n_tiles ? P.n_tiles : n_split);
-  const int tiles_per = (P.n_tiles + n_split - 1) / n_split;
-  n_split = (P.n_tiles + tiles_per - 1) / tiles_per;
+  const int tiles_per = div_small(P.n_tiles + n_split - 1, n_split);
   const int n_units = total_passes * n_split;
   if (static_cast<int>(blockIdx.x) >= n_units) return;
 
@@ -309,8 +330,8 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
     int it = 0;
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++it) {
       const int ub = it & 1;
-      const int pu = u / n_split, sp = u - pu * n_split;
-      int lo = 0, hi = P.num_experts - 1;          // last expert whose prefix is <= pu
+      const int pu = div_small(u, n_split), sp = u - pu * n_split;
+      int lo = it == 0 ? first_expert : 0, hi = it == 0 ? lo : P.num_experts - 1;          // last expert whose prefix is <= pu
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (static_cast<int>(pbase[mid]) <= pu) lo = mid; else hi = mid - 1;
@@ -428,11 +449,14 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
           const int pos = slot_pos(slot);
           const float sv = __half2float(s_t[slot]);
           const bool live = rk >= 0 && rk < P.h_rank;
+          // rows past npass hold whatever is there: read and dropped, so that the eight reads need no branches
+          const __half* src = hrow + (live ? rk : 0);
+          __half hv[FAST_MAX_TOK];
 #pragma unroll
-          for (int n = 0; n < FAST_MAX_TOK; ++n) {
-            const float hv = (live && n < npass) ? __half2float(hrow[n * P.h_rank + rk]) : 0.f;
-            dst[n * lay.stride + pos] = __float2half_rn(hv * sv);
-          }
+          for (int n = 0; n < FAST_MAX_TOK; ++n) hv[n] = src[n * P.h_rank];
+#pragma unroll
+          for (int n = 0; n < FAST_MAX_TOK; ++n)
+            dst[n * lay.stride + pos] = __float2half_rn(live && n < npass ? __half2float(hv[n]) * sv : 0.f);
         }
       }
     }
@@ -450,29 +474,25 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
       const unsigned char* sec = ring + static_cast<size_t>(gs) * P.sec_bytes;
       const int nch = fe.m[m].nslots >> 3, nib_ch = fe.m[m].nblk[0] * 2;
       __half* act = reinterpret_cast<__half*>(smem_raw + lay.act + buf * lay.act_bytes);
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const int row = 2 * warp + j;          // = m * 8 + n
-        float sum = 0.f;
-        if ((row & 7) < npass) {
-          for (int c = lane; c < nch; c += 32) {
-            const uint4 hv = *reinterpret_cast<const uint4*>(hs + row * lay.stride + 8 * c);
-            const uint4 sv = *reinterpret_cast<const uint4*>(sec + 16 * c);
-            uint4 pr;
-            pr.x = hmul2_u32(hv.x, sv.x);
-            pr.y = hmul2_u32(hv.y, sv.y);
-            pr.z = hmul2_u32(hv.z, sv.z);
-            pr.w = hmul2_u32(hv.w, sv.w);
-            *reinterpret_cast<uint4*>(act + row * lay.stride + 8 * c) = pr;
-            sum += (c < nib_ch ? static_cast<float>(FAST_NIB_OFFSET) : static_cast<float>(FAST_DENSE_OFFSET)) * sum8_halves(pr);
-          }
-        } else {
-          for (int c = lane; c < nch; c += 32) *reinterpret_cast<uint4*>(act + row * lay.stride + 8 * c) = make_uint4(0u, 0u, 0u, 0u);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) corr[buf][row] = sum;
+      const int row = 2 * warp;          // = m * 8 + n; rows past npass are zero in hs
+      float sum0 = 0.f, sum1 = 0.f;
+      for (int c = lane; c < nch; c += 32) {
+        const uint4 sv = *reinterpret_cast<const uint4*>(sec + 16 * c);
+        const uint4 h0 = *reinterpret_cast<const uint4*>(hs + row * lay.stride + 8 * c);
+        const uint4 h1 = *reinterpret_cast<const uint4*>(hs + (row + 1) * lay.stride + 8 * c);
+        const uint4 p0 = make_uint4(hmul2_u32(h0.x, sv.x), hmul2_u32(h0.y, sv.y), hmul2_u32(h0.z, sv.z), hmul2_u32(h0.w, sv.w));
+        const uint4 p1 = make_uint4(hmul2_u32(h1.x, sv.x), hmul2_u32(h1.y, sv.y), hmul2_u32(h1.z, sv.z), hmul2_u32(h1.w, sv.w));
+        *reinterpret_cast<uint4*>(act + row * lay.stride + 8 * c) = p0;
+        *reinterpret_cast<uint4*>(act + (row + 1) * lay.stride + 8 * c) = p1;
+        const float off = c < nib_ch ? static_cast<float>(FAST_NIB_OFFSET) : static_cast<float>(FAST_DENSE_OFFSET);
+        sum0 += off * sum8_halves(p0);
+        sum1 += off * sum8_halves(p1);
       }
+      // the lower half warp finishes the first row, the upper half the second
+      float sum = (lane & 16 ? sum1 : sum0) + __shfl_xor_sync(0xffffffffu, lane & 16 ? sum0 : sum1, 16);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if ((lane & 15) == 0) corr[buf][row + (lane >> 4)] = sum;
       return true;
     };
 
@@ -501,11 +521,11 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
       uint32_t ns = ds + 1u, np = dp;
       if (ns >= R) { ns -= R; np ^= 1u; }
       // ---- gate / up: this warp owns columns 16*warp .. 16*warp+15 of the tile
-      float acc[2][4];
+      float acc[2][2][4];      // [matrix][block of a pair]
 #pragma unroll
-      for (int m = 0; m < 2; ++m)
+      for (int m = 0; m < 4; ++m)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[m][j] = 0.f;
+        for (int j = 0; j < 4; ++j) acc[m >> 1][m & 1][j] = 0.f;
       if (ok) ok = dec_wait(&bar_full[rs], rp, abort_flag, limit) && dec_wait(&bar_full[us], up_, abort_flag, limit);
       if (ok) {
         const __half* act = reinterpret_cast<const __half*>(smem_raw + lay.act + abuf * lay.act_bytes);
@@ -542,22 +562,18 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
           const int c = 16 * warp + g + (j >= 2 ? 8 : 0);
           const int n = 2 * t + (j & 1);
           const float unscale = j >= 2 ? DEC_UNSCALE_HI : DEC_UNSCALE_LO;
-          const float gv = acc[0][j] * unscale - ((j & 1) ? cg1 : cg0);
-          const float uv = acc[1][j] * unscale - ((j & 1) ? cu1 : cu0);
-          const float z = (c < n_valid && n < npass) ? __fdividef(gv, 1.f + __expf(-gv)) * uv : 0.f;
-          const __half zh = __float2half_rn(z);
+          const float gv = (acc[0][0][j] + acc[0][1][j]) * unscale - ((j & 1) ? cg1 : cg0);
+          const float uv = (acc[1][0][j] + acc[1][1][j]) * unscale - ((j & 1) ? cu1 : cu0);
+          const float z = __fdividef(gv, 1.f + __expf(-gv)) * uv;
+          const __half zh = __float2half_rn(c < n_valid && n < npass ? z : 0.f);
           zp[n * ZP_STRIDE + (j >= 2 ? zpos_hi : zpos_lo)] = zh;
           zs[j & 1] += __half2float(zh);
         }
-#pragma unroll
-        for (int o = 4; o < 32; o <<= 1) {
-          zs[0] += __shfl_xor_sync(0xffffffffu, zs[0], o);
-          zs[1] += __shfl_xor_sync(0xffffffffu, zs[1], o);
-        }
-        if (g == 0) {
-          zsum_part[buf][2 * t][warp] = zs[0];
-          zsum_part[buf][2 * t + 1][warp] = zs[1];
-        }
+        // the lower half warp finishes the even tokens, the upper half the odd ones
+        float zt = (lane & 16 ? zs[1] : zs[0]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? zs[0] : zs[1], 16);
+        zt += __shfl_xor_sync(0xffffffffu, zt, 4);
+        zt += __shfl_xor_sync(0xffffffffu, zt, 8);
+        if ((lane & 12) == 0) zsum_part[buf][2 * t + (lane >> 4)][warp] = zt;
       }
       // ---- the next tile's operand goes into the other buffer before the barrier; with one buffer it has to wait
       // until every warp is done with this tile's operand
@@ -572,6 +588,9 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
           const __half* scale_d = reinterpret_cast<const __half*>(sec);
           const uint32_t* dwords = reinterpret_cast<const uint32_t*>(sec + fd.nslots * 2);
           const __half* zrow = reinterpret_cast<const __half*>(smem_raw + lay.zp + buf * lay.zp_bytes) + g * ZP_STRIDE + 8 * t;
+          uint4 zb[4];
+#pragma unroll
+          for (int p = 0; p < 4; ++p) zb[p] = *reinterpret_cast<const uint4*>(zrow + 32 * p);
           float zsum[2];
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -583,22 +602,20 @@ __global__ void __launch_bounds__(DEC_THREADS) experts_decode_kernel(const DecPa
           for (int i2 = 0; i2 < MAXMB; ++i2) {
             const int mb = warp + 8 * i2;
             if (mb < nblk_d) {
-              float dacc[4] = {0.f, 0.f, 0.f, 0.f};
+              float dacc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
               float off;
+              const float2 sc = __half22float2(*reinterpret_cast<const __half2*>(scale_d + mb * 16 + 2 * g));     // rows g and g + 8
               // nibble words [mblock][pair][lane][2], dense words [mblock][pair][lane]
               if (mb < fd.nblk[0]) {
-                mma_pairs<false>(dwords + (mb * 128 + lane) * 2, 64, 4, zrow, dacc);
+                mma_down<false>(dwords + (mb * 128 + lane) * 2, zb, dacc);
                 off = static_cast<float>(FAST_NIB_OFFSET);
               } else {
-                mma_pairs<true>(dwords + fd.nblk[0] * 256 + (mb - fd.nblk[0]) * 128 + lane, 32, 4, zrow, dacc);
+                mma_down<true>(dwords + fd.nblk[0] * 256 + (mb - fd.nblk[0]) * 128 + lane, zb, dacc);
                 off = static_cast<float>(FAST_DENSE_OFFSET);
               }
-              const float2 sc = __half22float2(*reinterpret_cast<const __half2*>(scale_d + mb * 16 + 2 * g));     // rows g and g + 8
-              const float sc_lo = sc.x, sc_hi = sc.y;
-              dtot[i2][0] += sc_lo * (dacc[0] * DEC_UNSCALE_LO - off * zsum[0]);
-              dtot[i2][1] += sc_lo * (dacc[1] * DEC_UNSCALE_LO - off * zsum[1]);
-              dtot[i2][2] += sc_hi * (dacc[2] * DEC_UNSCALE_HI - off * zsum[0]);
-              dtot[i2][3] += sc_hi * (dacc[3] * DEC_UNSCALE_HI - off * zsum[1]);
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                dtot[i2][j] += (j < 2 ? sc.x : sc.y) * ((dacc[0][j] + dacc[1][j]) * (j < 2 ? DEC_UNSCALE_LO : DEC_UNSCALE_HI) - off * zsum[j & 1]);
             }
           }
         }
