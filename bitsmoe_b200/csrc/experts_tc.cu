@@ -12,20 +12,25 @@
 // accumulator pairs (2 x 128 columns) beside the down accumulator (256), so the products of a chunk run while the
 // previous one is turned into z.
 //
-// Warp roles (640 threads; warp 19 completes the last warpgroup):
+// Warp roles (768 threads; the last warp completes the last warpgroup):
 //   warps 0-7   epilogue (two per TMEM lane quarter, 32 columns each): tcgen05.ld D_g/D_u -> z = silu(g)*u -> fp16 z
-//               operand in shared memory; at the end of the item D_d * s * route weight is transposed through the idle
-//               activation area and added to rank_accum row by row (16-byte vector reductions).
-//   warp  16    looks up the next item while the current one runs and asks L2 for its weights
-//   warps 17,18 MMA issue, one thread each.  tcgen05.mma blocks its thread until the tensor pipe accepts it, so the
-//               waits and commits around a stage cost tensor time when one thread issues everything; two pipelines
-//               (17: gate products and the down product's even slot tiles, 18: up products and the odd ones) hide one
-//               another's bookkeeping and never write the same accumulator.
-//   warps 8-15  converters, one team of four warps per pipeline: arena words (nibble / dense 2-bit codes), read straight
+//               operand in shared memory; at the end of the item D_d * s * route weight is turned through the idle z area
+//               and added to rank_accum in 16-byte vector reductions, beside the next item's staging.
+//   warps 8-19  converters, one team of six warps per pipeline: arena words (nibble / dense 2-bit codes), read straight
 //               from L2 one stage ahead into registers, -> fp16 (q * scale) operand stages of 64 rows x 32 positions in the
-//               canonical K-major core-matrix layout, a ring of stages per pipeline, a stage per warp.
-// Epilogue and converter warps together build the activation operand act[n, slot] = fp16(h[token, rank(slot)] * s(slot))
-// once per item.
+//               canonical K-major core-matrix layout, a ring of two-stage slots per pipeline, a stage per warp.  Before an
+//               item's stages they build its activation operand act[n, slot] = fp16(h[token, rank(slot)] * s(slot)).
+//   warp  20    looks up the next item while the current one runs and asks L2 for its weights
+//   warps 21,22 MMA issue, one thread each: gate products and the down product's even slot tiles; up products and the odd
+//               ones.  The waits and commits of one pipeline hide behind the products of the other, and they never write
+//               the same accumulator.
+// The roles walk the items on their own barriers, so an item's staging runs beside the last products and sums of the one
+// before.
+//
+// What bounds it: the converters -- 5.3 K cycles per chunk of 64 columns at 256 slots (about 44 instructions for each pair
+// of 16 x 16 blocks), against 2.1 K of tensor pipe.  8192 tokens of 128 experts (rank 256, intermediate 768): 372 -> 185 us
+// over the transposed, single-role-loop form; 16384 tokens of 512 experts 690 -> 333 us.  Two CTAs that share the
+// converted weights through the cluster's shared memory took longer (257 us): five slots of ring do not cover the way over.
 //
 // The down product of a chunk is issued one chunk late (G0 U0 | G1 U1 D0 | G2 U2 D1 | ...).  Every mbarrier wait is
 // bounded in time and aborts the whole CTA through a shared flag.
@@ -120,8 +125,23 @@ __device__ __forceinline__ bool xt_wait(uint64_t* bar, uint32_t parity, volatile
 // (q * scale): r[0] = row g, k (2t, 2t+1); r[1] = row g+8, same k; r[2] = row g, k (2t+8, 2t+9); r[3] = row g+8.
 // The code sits in the mantissa of 1024 (fields at bit 0) or of 64 (fields at bit 4); subtracting
 // 1024 + offset or 64 + offset is exact, the multiplication by the scale rounds once, as fp16(q * scale) does.
+// The exponents 1024 and 64 as fp16 pairs, in registers: the compiler knows only that they are values, so (w & mask) | k
+// stays one instruction with one immediate (as constants they were loaded again for each use: 8192 tokens 185 -> 179 us).
+struct XtMagic {
+  uint32_t lo, hi;
+  __device__ __forceinline__ XtMagic() {
+    asm volatile("mov.b32 %0, 0x64006400;" : "=r"(lo));
+    asm volatile("mov.b32 %0, 0x54005400;" : "=r"(hi));
+  }
+};
+template <uint32_t MASK>
+__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t k) {
+  uint32_t v;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v) : "r"(w), "n"(MASK), "r"(k));
+  return v;
+}
 template <bool DENSE>
-__device__ __forceinline__ void dequant_block(uint32_t w, __half2 s0, __half2 s1, __half2 s2, __half2 s3, uint32_t (&r)[4]) {
+__device__ __forceinline__ void dequant_block(const XtMagic& k, uint32_t w, __half2 s0, __half2 s1, __half2 s2, __half2 s3, uint32_t (&r)[4]) {
   constexpr uint32_t mlo = DENSE ? 0x00030003u : 0x000F000Fu, mhi = DENSE ? 0x00300030u : 0x00F000F0u;
   constexpr uint32_t off = DENSE ? FAST_DENSE_OFFSET : FAST_NIB_OFFSET;
   constexpr uint32_t blo_bits = 0x64006400u + off * 0x00010001u;          // fp16x2 of 1024 + offset
@@ -129,7 +149,7 @@ __device__ __forceinline__ void dequant_block(uint32_t w, __half2 s0, __half2 s1
   const uint32_t blo_u = blo_bits, bhi_u = bhi_bits;
   const __half2 blo = *reinterpret_cast<const __half2*>(&blo_u), bhi = *reinterpret_cast<const __half2*>(&bhi_u);
   const uint32_t sh = w >> (DENSE ? 2 : 8);
-  uint32_t v[4] = {(w & mlo) | 0x64006400u, (w & mhi) | 0x54005400u, (sh & mlo) | 0x64006400u, (sh & mhi) | 0x54005400u};
+  uint32_t v[4] = {and_or<mlo>(w, k.lo), and_or<mhi>(w, k.hi), and_or<mlo>(sh, k.lo), and_or<mhi>(sh, k.hi)};
   const __half2 o0 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&v[0]), blo), s0);
   const __half2 o1 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&v[1]), bhi), s1);
   const __half2 o2 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&v[2]), blo), s2);
@@ -143,11 +163,11 @@ __device__ __forceinline__ void dequant_block(uint32_t w, __half2 s0, __half2 s1
 // The two blocks of a pair -> the two 16-byte chunks (rows 16x+g and 16x+g+8) of K-chunk 4*pair_in_stage + t.
 // `word0` / `word1` are the pair's two blocks (dense: the same word, the second shifted by 8).
 template <bool DENSE>
-__device__ __forceinline__ void dequant_pair_store(uint32_t word0, uint32_t word1, const __half2 (&sa)[4], const __half2 (&sb)[4],
+__device__ __forceinline__ void dequant_pair_store(const XtMagic& k, uint32_t word0, uint32_t word1, const __half2 (&sa)[4], const __half2 (&sb)[4],
                                                    unsigned char* dst) {
   uint32_t r0[4], r1[4];
-  dequant_block<DENSE>(word0, sa[0], sb[0], sa[1], sb[1], r0);
-  dequant_block<DENSE>(word1, sa[2], sb[2], sa[3], sb[3], r1);
+  dequant_block<DENSE>(k, word0, sa[0], sb[0], sa[1], sb[1], r0);
+  dequant_block<DENSE>(k, word1, sa[2], sb[2], sa[3], sb[3], r1);
   *reinterpret_cast<uint4*>(dst) = make_uint4(r0[0], r0[2], r1[0], r1[2]);
   *reinterpret_cast<uint4*>(dst + 128) = make_uint4(r0[1], r0[3], r1[1], r1[3]);
 }
@@ -481,7 +501,13 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     // where a stage's pieces go: 64-row stages lie one after the other, the two 64-row halves of a down slot share chunks
     unsigned char* gu_dst = ring + (wt & 1) * XT_STAGE_BYTES + t4 * XT_W_STRIDE + g * 16;
     unsigned char* dn_dst = ring + (wt & 1) * 1024 + t4 * XT_D_STRIDE + g * 16;
-    XtCycle ring_c{0, 0};
+    // The turns run on from item to item: a warp comes back to the ring after three slots, no more than it holds, so it sees
+    // every phase of the barriers that it waits at (a parity tells a phase from its neighbours only).
+    constexpr int SLOT_STEP = XT_TEAM / 2;
+    int slot0 = wt >> 1;                      // this warp's first slot of the item
+    XtCycle my_c{0, 0};                       // its place in the ring
+    const XtMagic magic;
+    my_c.advance(slot0, ring_h);
     for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++round) {
       XT_ITEM_BEGIN
       if (round > 0 && !xt_wait(&bars.act_free, (round - 1) & 1u, abort_flag)) break;
@@ -602,8 +628,6 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
           }
         }
       };
-      XtCycle my_c = ring_c;
-      my_c.advance(wt >> 1, ring_h);
       auto convert = [&](int t, int i, const XtPre& p) -> bool {
         if (!xt_wait(&w_empty[my_c.i], my_c.ph ^ 1, abort_flag)) return false;
         if (t < nchunk && i < n_gu) {
@@ -613,10 +637,10 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
           const __half2 sc[4] = {sp[0], sp[1], sp[2], sp[3]};
           if (i < nib_pairs) {
 #pragma unroll
-            for (int x = 0; x < 4; ++x) dequant_pair_store<false>(p.w[x].x, p.w[x].y, sc, sc, dst + x * 256);
+            for (int x = 0; x < 4; ++x) dequant_pair_store<false>(magic, p.w[x].x, p.w[x].y, sc, sc, dst + x * 256);
           } else {
 #pragma unroll
-            for (int x = 0; x < 4; ++x) dequant_pair_store<true>(p.w[x].x, p.w[x].x >> 8, sc, sc, dst + x * 256);
+            for (int x = 0; x < 4; ++x) dequant_pair_store<true>(magic, p.w[x].x, p.w[x].x >> 8, sc, sc, dst + x * 256);
           }
         } else {
           unsigned char* dst = dn_dst + my_c.i * XT_SLOT_BYTES;
@@ -628,8 +652,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             if (mb0 + v >= nblk_d) break;             // slots past the matrix: accumulator columns that nobody reads
             const __half2 lo = __low2half2(sp[v]), hi = __high2half2(sp[v]);
             const __half2 sa[4] = {lo, lo, lo, lo}, sb[4] = {hi, hi, hi, hi};
-            if (mb0 + v < nib_d) dequant_pair_store<false>(p.w[v].x, p.w[v].y, sa, sb, dst + v * 256);
-            else dequant_pair_store<true>(p.w[v].x, p.w[v].x >> 8, sa, sb, dst + v * 256);
+            if (mb0 + v < nib_d) dequant_pair_store<false>(magic, p.w[v].x, p.w[v].y, sa, sb, dst + v * 256);
+            else dequant_pair_store<true>(magic, p.w[v].x, p.w[v].x >> 8, sa, sb, dst + v * 256);
           }
         }
         return true;
@@ -638,7 +662,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         tc::fence_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&w_full[my_c.i]);
-        my_c.i += XT_TEAM / 2;               // ring_h >= XT_TEAM / 2: at most one wrap
+        my_c.i += SLOT_STEP;                 // ring_h >= SLOT_STEP: at most one wrap
         if (my_c.i >= static_cast<uint32_t>(ring_h)) { my_c.i -= ring_h; my_c.ph ^= 1u; }
       };
       // this warp's stage after (t, i); false past its last one
@@ -651,7 +675,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         return t < nchunk + lag;
       };
       XtPre p;
-      int t = 0, i = wt - XT_TEAM;
+      int t = 0, i = 2 * (slot0 - SLOT_STEP) + (wt & 1);
       bool more = step(t, i), ok = true;
       if (more) fetch(t, i, p);
       while (more) {
@@ -660,7 +684,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         if (more) fetch(t, i, p);           // on its way while the converted stage is published and the next one is waited for
         publish();
       }
-      ring_c.advance(nchunk * (n_gu + n_d) / 2, ring_h);
+      slot0 = (slot0 + SLOT_STEP - nchunk * (n_gu + n_d) / 2 % SLOT_STEP) % SLOT_STEP;
       if (!ok) break;
     }
     __syncthreads();
