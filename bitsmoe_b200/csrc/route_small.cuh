@@ -1,11 +1,13 @@
-// Routing of a decode batch (up to 256 tokens) by one thread-block cluster: top-k, per-expert counts, offsets and the
-// expert-contiguous permutation without a trip through global memory.
+// Routing of a decode batch (up to 256 tokens): top-k, per-expert counts, offsets and the expert-contiguous permutation
+// without a trip through global memory, by one thread-block cluster or, for a launch of its own with few tokens, one CTA.
 //
 // A token selects an expert at most once, so the assignments of an expert, in the order of the permutation (ascending
 // token), are the set bits of a token mask.  Every warp takes a token, keeps its choices in registers and sets its bits
 // in the masks of the cluster's first CTA (atomics on distributed shared memory); that CTA turns mask populations into
-// offsets; a choice's place is its expert's offset plus the bits below its own.  Latency bound: a few cluster barriers and
-// one block scan.
+// offsets; a choice's place is its expert's offset plus the bits below its own.  Latency bound: a few barriers and one
+// block scan.  Barriers across a cluster and atomics on another CTA's memory cost several times the local ones, so up to
+// RS_ONE_TOKENS tokens, one for each of 32 warps, stay in one CTA (a whole block of one token 26.9 -> 25.4 us; at 64 tokens,
+// two for a warp, the cluster is 0.9 us faster).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -16,31 +18,36 @@
 namespace bm {
 
 constexpr int RS_THREADS = 256, RS_CLUSTER = 8, RS_MAX_E = 512, RS_MAX_TOKENS = 256, RS_MASK_WORDS = RS_MAX_TOKENS / 32;
-constexpr int RS_ROUNDS = RS_MAX_TOKENS / (RS_CLUSTER * RS_THREADS / 32);    // tokens per warp at most
+constexpr int RS_ONE_THREADS = 1024, RS_ONE_TOKENS = 32;
 
 // Shared memory of the first CTA: masks [E][words], offsets [E + 1], scan scratch.
 struct RouteSmallSmem {
   uint32_t mask[RS_MAX_E * RS_MASK_WORDS];
   int offset[RS_MAX_E + 1];
-  int warp_tot[RS_THREADS / 32];
+  int warp_tot[RS_ONE_THREADS / 32];
 };
 
-template <int REG>
+// CL CTAs of THREADS threads
+template <int REG, int CL, int THREADS>
 __device__ __forceinline__ void route_small_impl(const RouteSmallArgs& a, RouteSmallSmem* sm) {
   namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = static_cast<int>(cluster.block_rank());
+  constexpr int WARPS = THREADS / 32, ROUNDS = CL == 1 ? 2 : RS_MAX_TOKENS / (CL * WARPS);    // tokens per warp at most
+  static_assert(CL > 1 || ROUNDS * WARPS >= RS_ONE_TOKENS, "a round for every token");
+  auto sync = [] { if constexpr (CL == 1) __syncthreads(); else cg::this_cluster().sync(); };
+  const int rank = CL == 1 ? 0 : static_cast<int>(cg::this_cluster().block_rank());
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int words = (a.T + 31) >> 5;
-  RouteSmallSmem* s0 = cluster.map_shared_rank(sm, 0);
+  RouteSmallSmem* s0 = sm;
+  if constexpr (CL > 1) s0 = cg::this_cluster().map_shared_rank(sm, 0);
   if (rank == 0)
-    for (int i = threadIdx.x; i < a.E * words; i += RS_THREADS) sm->mask[i] = 0u;
-  auto cleared = cluster.barrier_arrive();
-  int idx[RS_ROUNDS];
-  float w[RS_ROUNDS];
+    for (int i = threadIdx.x; i < a.E * words; i += THREADS) sm->mask[i] = 0u;
+  cg::cluster_group::arrival_token cleared;
+  if constexpr (CL > 1) cleared = cg::this_cluster().barrier_arrive();
+  int idx[ROUNDS];
+  float w[ROUNDS];
 #pragma unroll
-  for (int r = 0; r < RS_ROUNDS; ++r) {
-    const int t = (r * (RS_THREADS / 32) + warp) * RS_CLUSTER + rank;     // neighbouring tokens go to different SMs
+  for (int r = 0; r < ROUNDS; ++r) {
+    const int t = (r * WARPS + warp) * CL + rank;     // neighbouring tokens go to different SMs
     idx[r] = -1;
     w[r] = 0.f;
     if (t < a.T) {
@@ -53,15 +60,16 @@ __device__ __forceinline__ void route_small_impl(const RouteSmallArgs& a, RouteS
       }
     }
   }
-  cluster.barrier_wait(std::move(cleared));
+  if constexpr (CL > 1) cg::this_cluster().barrier_wait(std::move(cleared));
+  else __syncthreads();
 #pragma unroll
-  for (int r = 0; r < RS_ROUNDS; ++r) {
-    const int t = (r * (RS_THREADS / 32) + warp) * RS_CLUSTER + rank;
+  for (int r = 0; r < ROUNDS; ++r) {
+    const int t = (r * WARPS + warp) * CL + rank;
     if (idx[r] >= 0) atomicOr(&s0->mask[idx[r] * words + (t >> 5)], 1u << (t & 31));
   }
-  cluster.sync();
+  sync();
   if (rank == 0) {
-    constexpr int PER = RS_MAX_E / RS_THREADS;     // consecutive experts of a thread
+    constexpr int PER = RS_MAX_E > THREADS ? RS_MAX_E / THREADS : 1;     // consecutive experts of a thread
     int cnt[PER], sum = 0;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
@@ -80,7 +88,8 @@ __device__ __forceinline__ void route_small_impl(const RouteSmallArgs& a, RouteS
     if (lane == 31) sm->warp_tot[warp] = incl;
     __syncthreads();
     int run = incl - sum;
-    for (int q = 0; q < warp; ++q) run += sm->warp_tot[q];
+#pragma unroll
+    for (int q = 0; q < RS_MAX_E / (32 * PER); ++q) run += q < warp ? sm->warp_tot[q] : 0;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
       const int e = threadIdx.x * PER + i;
@@ -90,15 +99,15 @@ __device__ __forceinline__ void route_small_impl(const RouteSmallArgs& a, RouteS
       }
       run += cnt[i];
     }
-    if (a.E == RS_MAX_E && threadIdx.x == RS_THREADS - 1) {
+    if (THREADS * PER == RS_MAX_E && a.E == RS_MAX_E && threadIdx.x == THREADS - 1) {
       sm->offset[RS_MAX_E] = run;
       a.expert_offsets[RS_MAX_E] = run;
     }
   }
-  cluster.sync();
+  sync();
 #pragma unroll
-  for (int r = 0; r < RS_ROUNDS; ++r) {
-    const int t = (r * (RS_THREADS / 32) + warp) * RS_CLUSTER + rank;
+  for (int r = 0; r < ROUNDS; ++r) {
+    const int t = (r * WARPS + warp) * CL + rank;
     if (idx[r] >= 0) {
       const uint32_t* m = &s0->mask[idx[r] * words];
       int pos = s0->offset[idx[r]] + __popc(m[t >> 5] & ((1u << (t & 31)) - 1u));
@@ -107,14 +116,15 @@ __device__ __forceinline__ void route_small_impl(const RouteSmallArgs& a, RouteS
       a.route_flat[pos] = w[r];
     }
   }
-  cluster.sync();      // the first CTA's shared memory is read until here
+  if constexpr (CL > 1) sync();      // the first CTA's shared memory is read until here
 }
 
+template <int CL = RS_CLUSTER, int THREADS = RS_THREADS>
 __device__ __forceinline__ void route_small(const RouteSmallArgs& a, RouteSmallSmem* sm) {
-  if (a.E <= 64) route_small_impl<2>(a, sm);
-  else if (a.E <= 128) route_small_impl<4>(a, sm);
-  else if (a.E <= 256) route_small_impl<8>(a, sm);
-  else route_small_impl<16>(a, sm);
+  if (a.E <= 64) route_small_impl<2, CL, THREADS>(a, sm);
+  else if (a.E <= 128) route_small_impl<4, CL, THREADS>(a, sm);
+  else if (a.E <= 256) route_small_impl<8, CL, THREADS>(a, sm);
+  else route_small_impl<16, CL, THREADS>(a, sm);
 }
 
 }  // namespace bm

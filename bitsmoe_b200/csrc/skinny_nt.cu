@@ -385,19 +385,21 @@ int launch_skinny_nt(SkinnyArgs a, cudaStream_t st) {
 }
 
 // ---- routing on its own, behind the launch that computes the logits
-__global__ void __launch_bounds__(RS_THREADS) route_small_kernel(const __grid_constant__ RouteSmallArgs a) {
+template <int CL, int THREADS>
+__global__ void __launch_bounds__(THREADS) route_small_kernel(const __grid_constant__ RouteSmallArgs a) {
   __shared__ RouteSmallSmem sm;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  route_small(a, &sm);
+  route_small<CL, THREADS>(a, &sm);
 }
 
 bool route_small_fits(int T, int E, int k) { return T >= 1 && T <= RS_MAX_TOKENS && E >= 1 && E <= RS_MAX_E && k >= 1 && k <= 32 && k <= E; }
 
 int launch_route_small(const RouteSmallArgs& a, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(RS_CLUSTER);
-  cfg.blockDim = dim3(RS_THREADS);
+  const bool one = a.T <= RS_ONE_TOKENS;
+  cfg.gridDim = dim3(one ? 1 : RS_CLUSTER);
+  cfg.blockDim = dim3(one ? RS_ONE_THREADS : RS_THREADS);
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -407,9 +409,9 @@ int launch_route_small(const RouteSmallArgs& a, cudaStream_t st) {
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = one ? 1 : 2;
   count_launch();
-  BM_CUDA(cudaLaunchKernelEx(&cfg, route_small_kernel, a));
+  BM_CUDA(cudaLaunchKernelEx(&cfg, one ? route_small_kernel<1, RS_ONE_THREADS> : route_small_kernel<RS_CLUSTER, RS_THREADS>, a));
   return BM_OK;
 }
 
