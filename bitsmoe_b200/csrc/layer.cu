@@ -631,10 +631,11 @@ extern "C" int bm_layer_forward(const bm_layer_t* L, const void* x, int x_dtype,
   int rc = bm_route(logits, logits_dtype, T, num_routed, k, renorm, weight_round, global_to_local, L->num_experts, TILE_ROWS,
                     w.topk_idx, w.topk_w, w.token_indices, w.expert_offsets, w.route_flat, /*tile_table=*/nullptr, /*counts=*/nullptr,
                     w.route_ws, w.route_ws_bytes, route_stream);
-  // the accumulator of the expert stage is cleared off the critical path, beside the routing
+  // the routing's four launches are the longer of the two ways at large batches: the accumulator of the expert stage is
+  // cleared behind the basis projection
   const size_t acc_bytes = sizeof(float) * static_cast<size_t>(T) * L->rank_out;
   const int rc_basis = bm_basis_project(L, x, x_dtype, T, reinterpret_cast<uint16_t*>(w.h_gate), reinterpret_cast<uint16_t*>(w.h_up), stream);
-  const bool zeroed = cudaMemsetAsync(w.rank_accum, 0, acc_bytes, static_cast<cudaStream_t>(route_stream)) == cudaSuccess;
+  const bool zeroed = cudaMemsetAsync(w.rank_accum, 0, acc_bytes, st) == cudaSuccess;
   if (fork) {
     // always join, also on error, so that the side stream never stays attached to a capture
     cudaEventRecord(L->ev_join, L->side_stream);

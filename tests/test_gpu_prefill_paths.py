@@ -1,0 +1,96 @@
+"""GPU: edges of the prefill kernels -- items and units of the packed experts, the routing passes over several blocks, and
+the products whose rows, columns and contractions do not fill a tile."""
+import pytest
+import torch
+
+from bitsmoe_b200 import capi, synth
+from bitsmoe_b200.layer import dense_mlp, route_build, route_topk
+from tests import helpers
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _route(counts, k, T, gen):
+    """Permutation tables in which expert e has counts[e] assignments of distinct tokens."""
+    tok = torch.cat([torch.sort(torch.randperm(T, generator=gen, device=DEV)[:c]).values for c in counts]).to(torch.int32)
+    off = torch.zeros(len(counts) + 1, dtype=torch.int32, device=DEV)
+    off[1:] = torch.tensor(counts, device=DEV).cumsum(0)
+    return tok, off, torch.rand(tok.numel(), generator=gen, device=DEV)
+
+
+# assignments per expert around an item (128) and a pass (8), none at all, one expert alone; ranks whose row slots are an odd
+# number of pairs, are not whole octets of one group, or pass 256; intermediate sizes of one and of several tiles
+@pytest.mark.parametrize("rank,inter", [(64, 128), (80, 256), (256, 384), (328, 128)])
+@pytest.mark.parametrize("counts", [(1, 0, 127, 128, 129, 7), (9, 8, 300, 0, 255, 257), (512,)])
+def test_packed_experts_match_generic_kernel(rank, inter, counts):
+    cfg = synth.tiny(hidden=128, num_experts=len(counts), intermediate=inter, top_k=1, rank=rank)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=rank, device=DEV))
+    T = 520
+    gen = torch.Generator(device=DEV).manual_seed(11)
+    tok, off, rw = _route(counts, 1, T, gen)
+    hg, hu = layer.basis_project(synth.activations(cfg, T, seed=2, device=DEV, dtype=torch.bfloat16))
+    want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
+    for path in (capi.PATH_DECODE, capi.PATH_TENSOR):
+        try:
+            got = layer.experts_forward(hg, hu, tok, off, rw, path=path)
+        except capi.BitsMoEError as e:      # a layer whose largest expert does not fit that path
+            assert e.status == 2      # BM_ERR_UNSUPPORTED
+            continue
+        helpers.assert_close(got.cpu(), want.cpu(), what=f"path {path} rank {rank} counts {counts}")
+
+
+# token counts around the blocks of the counting pass; expert counts around a warp of the scan and the top-k's registers
+@pytest.mark.parametrize("T", [129, 1025, 4097, 16385])
+@pytest.mark.parametrize("E,k", [(2, 2), (33, 5), (128, 8), (512, 10)])
+def test_routing_is_the_stable_permutation(T, E, k):
+    logits = torch.randn(T, E, device=DEV).round(decimals=1)      # ties: the lower expert id comes first
+    idx, w = route_topk(logits, k, False, torch.float32)
+    p = torch.softmax(logits, -1)
+    order = torch.argsort(p, dim=-1, descending=True, stable=True)[:, :k]
+    assert torch.equal(idx.long(), order)
+    helpers.assert_close(w.cpu(), torch.gather(p, 1, order).cpu(), what="weights")
+    tok, off, rw, _, counts = route_build(idx, w, E)
+    flat, by = torch.sort(idx.reshape(-1), stable=True)
+    assert torch.equal(off[1:].long(), torch.bincount(flat.long(), minlength=E).cumsum(0))
+    assert int(counts[0]) == T * k
+    assert torch.equal(tok.long(), by // k) and torch.equal(rw, w.reshape(-1)[by])
+
+
+# rows around a tile of 128 and the decode kernel's 8, 64 and 256; inner sizes that are no multiple of a tile, or so many
+# that the decode products take several row tiles per block
+@pytest.mark.parametrize("T", [1, 9, 65, 256, 257, 385, 1000])
+@pytest.mark.parametrize("H,I", [(128, 48), (256, 200), (512, 2824), (1024, 4104)])
+def test_dense_mlp_matches_plain_products(T, H, I):
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn(T, H, generator=gen, device=DEV).to(torch.bfloat16)
+    g, u = ((torch.randn(I, H, generator=gen, device=DEV) / H ** 0.5).half() for _ in range(2))
+    d = (torch.randn(H, I, generator=gen, device=DEV) / I ** 0.5).half()
+    t = (torch.randn(H, generator=gen, device=DEV) / H ** 0.5).half()
+    xf = x.float()
+    want = torch.sigmoid(xf @ t.float())[:, None] * ((torch.nn.functional.silu(xf @ g.float().T) * (xf @ u.float().T)) @ d.float().T)
+    helpers.assert_close(dense_mlp(x, g, u, d, t).float().cpu(), want.cpu(), what=f"T={T} H={H} I={I}")
+
+
+# prefill blocks: tiles of 128 rows that are full, ragged or hold one row; router and shared widths that are ragged
+@pytest.mark.parametrize("T", [257, 384, 513])
+@pytest.mark.parametrize("E,shared,wdtype", [(5, 48, torch.bfloat16), (40, 200, torch.float16), (300, 0, torch.bfloat16)])
+def test_prefill_block_matches_stages(T, E, shared, wdtype):
+    cfg = synth.tiny(hidden=256, num_experts=E, intermediate=128, top_k=4, rank=64, shared_intermediate=shared, shared_gated=shared > 0)
+    s = synth.make_layer(cfg, seed=7, device=DEV)
+    layer = synth.to_packed_layer(s)
+    gen = torch.Generator(device=DEV).manual_seed(3)
+    x = synth.activations(cfg, T, seed=T, device=DEV, dtype=wdtype)
+    gate = (torch.randn(E, cfg.hidden, generator=gen, device=DEV) / 16).to(wdtype)
+    sh = tuple(s.shared[n].to(wdtype) for n in ("gate", "up", "down", "gate_logit_w")) if shared else None
+    y, logits = layer.block_forward(x, gate, 4, True, wdtype, sh)
+    xf = x.float()
+    helpers.assert_close(logits.cpu(), (xf @ gate.float().T).cpu(), what="router logits")
+    idx, w = route_topk(logits, 4, True, wdtype)
+    tok, off, rw, _, _ = route_build(idx, w, E)
+    hg, hu = layer.basis_project(x)
+    want = layer.combine_down_basis(layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC), torch.float32)
+    if shared:
+        g, u, d, t = (v.float() for v in sh)
+        want = want + torch.sigmoid(xf @ t.T) * ((torch.nn.functional.silu(xf @ g.T) * (xf @ u.T)) @ d.T)
+    helpers.assert_close(y.cpu(), want.cpu(), what=f"block T={T} E={E}")
