@@ -15,6 +15,11 @@
 // product accumulates in registers over all tiles of the unit and reaches rank_accum with one fp32 atomic per
 // (slot, token) per unit (the reference adds per CTA as well: bitsmoe/algorithms/cpp/mlp_forward.cu:2036-2066).
 //
+// What bounds it: the latency of a tile's chain (3.2 us a tile for each of two CTAs per SM: gate/up 1.1, z 0.5, next operand
+// 0.5, down 0.7, waits) and shared-memory reads.  Words and operands one pair ahead, accumulators of their own for the blocks
+// of a pair and an operand built without branches: a tile 4.5 -> 4.0 us in the first, 3.6 -> 3.2 in the later ones; a block of
+// 64 tokens 44.0 -> 42.3 us.
+//
 // Every wait is bounded (a launch parameter); a wait that gives up raises a CTA-wide abort flag, all threads leave
 // through the same barriers, and the layer's status word reports BM_ERR_TIMEOUT.
 #include "fast_layout.cuh"

@@ -7,6 +7,10 @@
 // leaves the order open (torch.topk ties, an unstable argsort) this file fixes it:
 // ties go to the lower expert id, and inside an expert assignments are ordered by
 // ascending flat (token, slot) index.
+//
+// What bounds it is latency: four dependent launches.  16384 tokens of 512 experts, top 10: top-k 52 -> 24.5 us (topk.cuh),
+// prefixes of the block histograms 16.5 -> 4 us (one block walked them; now a thread of a grid per expert, and the totals
+// are scanned where they are used), counting 5, scatter 8.
 #include "topk.cuh"
 
 namespace bm {

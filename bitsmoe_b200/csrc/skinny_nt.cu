@@ -11,7 +11,8 @@
 // everything that multiplies the same x is one launch (SkSeg stacks; the gated pair of a shared expert leaves as
 // silu(g) * u), the routing of given logits is one more cluster of the same grid, and a launch behind
 // another one of the same call is programmatically serialised: its weights are on their way to shared memory while the
-// previous kernel still runs.
+// previous kernel still runs.  A whole block of one token went from 60.6 us a call (seven launches and the host work between
+// them) to 25.5, 24 tokens of a 512-expert block with a gated shared expert from 130 to 53.
 #include <algorithm>
 
 #include "route_small.cuh"
