@@ -28,8 +28,8 @@
 // before.
 //
 // What bounds it: the converters -- 5.3 K cycles per chunk of 64 columns at 256 slots (about 44 instructions for each pair
-// of 16 x 16 blocks), against 2.1 K of tensor pipe.  8192 tokens of 128 experts (rank 256, intermediate 768): 372 -> 185 us
-// over the transposed, single-role-loop form; 16384 tokens of 512 experts 690 -> 333 us.  Two CTAs that share the
+// of 16 x 16 blocks), against 2.1 K of tensor pipe.  8192 tokens of 128 experts (rank 256, intermediate 768): 363 -> 179 us
+// over the transposed, single-role-loop form; 16384 tokens of 512 experts 653 -> 320 us.  Two CTAs that share the
 // converted weights through the cluster's shared memory took longer (257 us): five slots of ring do not cover the way over.
 //
 // The down product of a chunk is issued one chunk late (G0 U0 | G1 U1 D0 | G2 U2 D1 | ...).  Every mbarrier wait is
