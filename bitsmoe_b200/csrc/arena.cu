@@ -10,8 +10,31 @@ namespace bm {
 // Rows of a group by ascending rank, the ranks that come as whole aligned octets first: the kernels move such an octet of
 // a token's row as one 16-byte piece and take the remaining ranks one by one.
 static void order_by_octets(std::vector<int16_t>& rows, const std::vector<int32_t>& rank_idx) {
-  std::sort(rows.begin(), rows.end(), [&](int16_t a, int16_t b) { return rank_idx[a] != rank_idx[b] ? rank_idx[a] < rank_idx[b] : a < b; });
+  // ascending rank: ranks are small and distinct in a packed matrix, so each row drops into its rank's place
+  int top = -1;
+  bool distinct = true;
+  for (const int16_t r : rows) {
+    distinct = distinct && rank_idx[r] >= 0 && rank_idx[r] < 4096;
+    top = std::max(top, rank_idx[r]);
+  }
+  std::vector<int16_t> at;
+  if (distinct) {
+    at.assign(top + 1, -1);
+    for (const int16_t r : rows) {
+      distinct = distinct && at[rank_idx[r]] < 0;
+      at[rank_idx[r]] = r;
+    }
+  }
+  if (distinct) {
+    size_t n = 0;
+    for (const int16_t r : at)
+      if (r >= 0) rows[n++] = r;
+  } else {
+    std::sort(rows.begin(), rows.end(), [&](int16_t a, int16_t b) { return rank_idx[a] != rank_idx[b] ? rank_idx[a] < rank_idx[b] : a < b; });
+  }
   std::vector<int16_t> whole, rest;
+  whole.reserve(rows.size());
+  rest.reserve(rows.size());
   for (size_t i = 0; i < rows.size();) {
     const int r = rank_idx[rows[i]];
     bool oct = r >= 0 && r % 8 == 0 && i + 8 <= rows.size();
