@@ -227,6 +227,7 @@ struct XtArgs {
   long long* acc64;
   int* status;
   int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, ring_h, gu_bufs, tab_bytes;
+  int vec_add;            // every row of rank_accum starts on a 16-byte boundary (and takes fp32 adds)
 };
 
 // Locates unit `u` and copies what the roles need; one warp, an item ahead of the roles.
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         // D_d * s * route weight -> rank_accum.  A thread owns a token: adding straight from the registers would touch a
         // 32-byte sector per lane and instruction.  Sixteen slots at a time go through the warp's part of the (now idle) z
         // area, so that an instruction adds the 64 bytes of eight tokens.  Octets of slots that are not an aligned octet
-        // of ranks, and the deterministic mode, add from the registers.
+        // of ranks, rows that do not start on 16-byte boundaries, and the deterministic mode add from the registers.
         for (int s0 = 16 * half; s0 < nslots_d; s0 += 32) {
           float v[16];
           tc::tmem_ld16(d_down + lane_sel + s0, v);
@@ -437,8 +438,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
             v[i] *= sv.x * rw; v[i + 1] *= sv.y * rw; v[i + 2] *= sv.z * rw; v[i + 3] *= sv.w * rw;
           }
           int oct[2];
-          oct[0] = A.acc64 ? -1 : oct_d[s0 >> 3];
-          oct[1] = A.acc64 ? -1 : oct_d[(s0 >> 3) + 1];
+          oct[0] = A.vec_add ? oct_d[s0 >> 3] : -1;
+          oct[1] = A.vec_add ? oct_d[(s0 >> 3) + 1] : -1;
           __syncwarp();                            // the pieces of the sixteen slots before have been read
 #pragma unroll
           for (int c = 0; c < 4; ++c)
@@ -851,6 +852,8 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
   a.h_gate = h_gate; a.h_up = h_up; a.h_rank = L->rank_in;
   a.token_indices = token_indices; a.expert_offsets = expert_offsets; a.route_w = route_w;
   a.rank_accum = rank_accum; a.acc64 = acc64; a.status = L->status_dev;
+  // an octet's two 16-byte adds need the row's start, and so rank_out and the base, at multiples of four floats
+  a.vec_add = acc64 == nullptr && L->rank_out % 4 == 0 && (reinterpret_cast<uintptr_t>(rank_accum) & 15u) == 0;
   a.rank_out = L->rank_out; a.T = T; a.num_experts = L->num_experts; a.n_tiles = L->n_tiles; a.max_slots = L->max_slots;
   a.nt = plan.nt; a.ring_h = plan.ring_h; a.gu_bufs = plan.gu_bufs;
   experts_tc_kernel<<<sm_counts[dev], XT_THREADS, plan.smem, st>>>(a);

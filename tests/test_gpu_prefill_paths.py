@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from bitsmoe_b200 import capi, synth
-from bitsmoe_b200.layer import dense_mlp, route_build, route_topk
+from bitsmoe_b200.layer import PackedLayer, dense_mlp, route_build, route_topk
 from tests import helpers
 
 pytestmark = pytest.mark.gpu
@@ -38,6 +38,34 @@ def test_packed_experts_match_generic_kernel(rank, inter, counts):
             assert e.status == 2      # BM_ERR_UNSUPPORTED
             continue
         helpers.assert_close(got.cpu(), want.cpu(), what=f"path {path} rank {rank} counts {counts}")
+
+
+def _with_output_rank(rank_in, rank_out, inter, E):
+    """A layer whose down matrices have ``rank_out`` rows while gate and up have ``rank_in``."""
+    a = synth.make_layer(synth.tiny(hidden=128, num_experts=E, intermediate=inter, top_k=1, rank=rank_in), seed=1, device=DEV)
+    b = synth.make_layer(synth.tiny(hidden=128, num_experts=E, intermediate=inter, top_k=1, rank=rank_out), seed=2, device=DEV)
+    return PackedLayer(a.tables["gate"], a.tables["up"], b.tables["down"], inter, rank_out, a.vh_gate, a.vh_up, b.u_down)
+
+
+# rank_accum rows that start on a 16-byte boundary for every token, for every second or fourth one only, and (base one float
+# off) for none at all
+@pytest.mark.parametrize("rank_out,shift", [(256, 0), (256, 1), (252, 0), (250, 0), (250, 1), (241, 0), (72, 0)])
+def test_sums_reach_rows_of_any_alignment(rank_out, shift):
+    counts, T, lib = (130, 0, 61, 1), 140, capi.lib()
+    layer = _with_output_rank(256, rank_out, 256, len(counts))
+    gen = torch.Generator(device=DEV).manual_seed(5)
+    tok, off, rw = _route(counts, 1, T, gen)
+    hg, hu = layer.basis_project(torch.randn(T, 128, generator=gen, device=DEV).half())
+    want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
+    for path in (capi.PATH_DECODE, capi.PATH_TENSOR):
+        buf = torch.full((T * rank_out + 2,), 7.0, device=DEV)
+        acc = buf[shift:shift + T * rank_out].view(T, rank_out)
+        assert acc.data_ptr() % 16 == 4 * shift
+        capi.check(lib.bm_experts_forward(layer._handle, hg.data_ptr(), hu.data_ptr(), tok.data_ptr(), off.data_ptr(), rw.data_ptr(), T,
+                                          tok.numel(), acc.data_ptr(), path, None, 0, capi.stream_ptr(torch.device(DEV))))
+        layer.check_status()
+        helpers.assert_close(acc.cpu(), want.cpu(), what=f"path {path} rank_out {rank_out} shift {shift}")
+        assert buf[:shift].eq(7.0).all() and buf[shift + T * rank_out:].eq(7.0).all()
 
 
 # token counts around the blocks of the counting pass; expert counts around a warp of the scan and the top-k's registers
