@@ -10,9 +10,10 @@
 
 namespace bm {
 
-// 1 MiB of block histograms: ceil(T*k / 1024) * num_local int32 entries.  Every GPU that loads the
-// library holds this array until the process exits.
-constexpr size_t ROUTE_STATIC_SCRATCH_BYTES = 1u << 20;
+// 1 MiB of block histograms: ceil(T*k / 1024) * num_local int32 entries; behind them the experts' totals, one more row
+// of at most 1024.  Every GPU that loads the library holds this array until the process exits.
+constexpr size_t ROUTE_STATIC_HIST_BYTES = 1u << 20;
+constexpr size_t ROUTE_STATIC_SCRATCH_BYTES = ROUTE_STATIC_HIST_BYTES + 1024 * sizeof(int32_t);
 static __device__ __align__(256) unsigned char g_route_scratch[ROUTE_STATIC_SCRATCH_BYTES];
 
 // Device address of the array, per device ordinal.  Written without a lock: two host threads that race on the first
@@ -37,18 +38,20 @@ static int route_scratch_address(void** out) {
 
 }  // namespace bm
 
-extern "C" size_t bm_route_build_static_capacity(void) { return bm::ROUTE_STATIC_SCRATCH_BYTES; }
+extern "C" size_t bm_route_build_static_capacity(void) { return bm::ROUTE_STATIC_HIST_BYTES; }
 
 extern "C" int bm_route_build_static(const int32_t* topk_idx, const float* topk_w, const int32_t* global_to_local,
                                      int32_t num_routed, int32_t T, int32_t k, int32_t num_local, int32_t tile_rows, int32_t* token_indices,
                                      int32_t* expert_offsets, float* route_flat, int32_t* tile_table, int32_t* counts,
                                      void* stream) {
   using namespace bm;
-  const size_t need = bm_route_build_workspace_bytes(T, k, num_local);
-  BM_REQUIRE(need <= ROUTE_STATIC_SCRATCH_BYTES, BM_ERR_WORKSPACE,
-             "route_build_static: T*k=%lld assignments over %d experts need %zu bytes of scratch, the built-in array holds %zu; "
+  // the limit of the interface: histograms of at most 1 MiB (a block of assignments needs none); the totals always fit
+  const int64_t assign = static_cast<int64_t>(T) * k;
+  const int64_t hist = assign > 1024 ? (assign + 1023) / 1024 * num_local * static_cast<int64_t>(sizeof(int32_t)) : 0;
+  BM_REQUIRE(hist <= static_cast<int64_t>(ROUTE_STATIC_HIST_BYTES), BM_ERR_WORKSPACE,
+             "route_build_static: T*k=%lld assignments over %d experts need %lld bytes of histograms, the built-in array holds %zu; "
              "use bm_route_build with a caller-provided workspace",
-             static_cast<long long>(T) * k, num_local, need, ROUTE_STATIC_SCRATCH_BYTES);
+             static_cast<long long>(assign), num_local, static_cast<long long>(hist), ROUTE_STATIC_HIST_BYTES);
   void* scratch = nullptr;
   const int rc = route_scratch_address(&scratch);
   if (rc) return rc;

@@ -173,8 +173,8 @@ BM_API int bm_route_build(const int32_t* topk_idx, const float* topk_w, const in
 
 /* No counterpart in the reference.  Same result as bm_route_build, for hosts that cannot give the
  * library scratch memory (code that must stay off the CUDA allocator while serving, or a plug-in that
- * only ever receives input and output pointers): the per-block histogram table lives in a fixed
- * 1 MiB array inside the library instead of a caller workspace.  Calls nothing that allocates.
+ * only ever receives input and output pointers): the per-block histogram table (1 MiB) and the experts'
+ * totals live in a fixed array inside the library instead of a caller workspace.  Calls nothing that allocates.
  *  - limit: ceil(T*k/1024) * num_local * 4 bytes must fit bm_route_build_static_capacity();
  *    larger problems return BM_ERR_WORKSPACE and should use bm_route_build;
  *  - the first call on each device looks up the array's device address (that device must be

@@ -59,6 +59,20 @@ def test_static_route_build_matches_workspace_version_twice_in_a_row():
     assert status == capi.BM_OK and torch.equal(got[1], want[1]) and torch.equal(got[0], want[0])
 
 
+# problems whose block histograms fill the built-in table to the last entry, and one block more
+@pytest.mark.parametrize("T,E,k", [(65536, 512, 8), (32768, 1024, 8)])
+def test_static_route_build_takes_a_full_table(T, E, k):
+    assert T * k // 1024 * E * 4 == int(capi.lib().bm_route_build_static_capacity())
+    idx, w = _problem(T, E, k, 4)
+    want = route_build(idx, w, E)
+    status, got = _static_build(idx, w, E)
+    assert status == capi.BM_OK, capi.lib().bm_last_error()
+    n_tiles = int(want[4].cpu()[1])
+    assert all(torch.equal(got[i], want[i]) for i in (0, 1, 2, 4)) and torch.equal(got[3][:n_tiles], want[3][:n_tiles])
+    more = torch.cat([idx, idx[:1]]), torch.cat([w, w[:1]])
+    assert _static_build(*more, E)[0] == 4      # BM_ERR_WORKSPACE
+
+
 def test_static_route_build_rejects_what_does_not_fit():
     lib = capi.lib()
     cap = int(lib.bm_route_build_static_capacity())
