@@ -204,9 +204,9 @@ __global__ void __launch_bounds__(128) build_toktab_kernel(const FastExpert* __r
   int16_t *pos_r = reinterpret_cast<int16_t*>(t + lay.pos_r), *oct_r = reinterpret_cast<int16_t*>(t + lay.oct_r);
   float* s_d = reinterpret_cast<float*>(t + lay.s_d);
   int16_t *rank_d = reinterpret_cast<int16_t*>(t + lay.rank_d), *oct_d = reinterpret_cast<int16_t*>(t + lay.oct_d);
-  __shared__ int padded, live_d;
+  __shared__ int loose, live_d;
   __shared__ uint32_t broken[2][4];
-  if (threadIdx.x == 0) { padded = 0; live_d = 0; }
+  if (threadIdx.x == 0) { loose = 0; live_d = 0; }
   if (threadIdx.x < 8) broken[threadIdx.x >> 2][threadIdx.x & 3] = 0u;
   for (int i = threadIdx.x; i < 2 * rank_in; i += blockDim.x) { pos_r[i] = -1; s_r[i] = __float2half(0.f); }
   for (int i = threadIdx.x; i < max_slots; i += blockDim.x) { rank_d[i] = -1; s_d[i] = 0.f; }
@@ -224,13 +224,21 @@ __global__ void __launch_bounds__(128) build_toktab_kernel(const FastExpert* __r
         if (live) atomicAdd(&live_d, 1);
       } else if (rk >= 0 && rk < rank_in) {
         pos_r[m * rank_in + rk] = static_cast<int16_t>(slot_pos(i));
-        s_r[m * rank_in + rk] = s_t[i];
-      } else {
-        padded = 1;
       }
     }
   }
   __syncthreads();
+  // where several slots hold the same rank, one of them has the rank's entry; it gives the factor too
+  for (int m = 0; m < 2; ++m) {
+    const FastMat& fm = fe.m[m];
+    const int16_t* rank_t = reinterpret_cast<const int16_t*>(arena + fm.tab_off);
+    const __half* s_t = reinterpret_cast<const __half*>(arena + fm.tab_off + fm.nslots * 2);
+    for (int i = threadIdx.x; i < fm.nslots; i += blockDim.x) {
+      const int rk = rank_t[i];
+      if (rk >= 0 && rk < rank_in && pos_r[m * rank_in + rk] == slot_pos(i)) s_r[m * rank_in + rk] = s_t[i];
+      else loose = 1;
+    }
+  }
   for (int i = threadIdx.x; i < 2 * (rank_in / 8); i += blockDim.x) {
     const int m = i / (rank_in / 8), o = i - m * (rank_in / 8);
     const int16_t* p = pos_r + m * rank_in + 8 * o;
@@ -248,7 +256,7 @@ __global__ void __launch_bounds__(128) build_toktab_kernel(const FastExpert* __r
   __syncthreads();
   if (threadIdx.x == 0) {
     head->fe = fe;
-    head->padded = padded;
+    head->loose = loose;
     head->all_ranks = live_d == rank_out;
   }
   if (threadIdx.x < 8) head->broken[threadIdx.x >> 2][threadIdx.x & 3] = broken[threadIdx.x >> 2][threadIdx.x & 3];

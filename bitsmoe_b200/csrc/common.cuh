@@ -108,7 +108,7 @@ struct FastExpert {
 // and its sums back into rank order, as one contiguous copy.  All experts of a layer share the offsets.
 struct TokTabHead {
   FastExpert fe;
-  int32_t padded;           // gate or up has slots without a row
+  int32_t loose;            // gate or up has slots that no rank's position names: without a row, or with a rank that another slot has too
   int32_t all_ranks;        // every rank of rank_accum has a down slot
   uint32_t broken[2][4];    // gate, up: octets of ranks that are not one 16-byte piece of the operand row (bit per octet)
 };

@@ -571,14 +571,21 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
                       __hmul((m ? A.h_up : A.h_gate)[static_cast<int64_t>(item.tok[n]) * h_rank + rk], s_r[m * h_rank + rk]);
               }
             }
-        if (head.padded) {        // padding slots: their weights are zero, their activations have to be finite
+        // Slots that the octets above do not reach.  Padding: the weights are zero, the activations have to be finite.  A
+        // rank that several slots hold: each slot has weights and a factor of its own.
+        if (head.loose) {
           for (int m = 0; m < 2; ++m) {
+            const int nslots = fe.m[m].nslots;
             const int16_t* rank_t = reinterpret_cast<const int16_t*>(A.arena + fe.m[m].tab_off);
-            for (int i = dw; i < fe.m[m].nslots; i += XT_DQ_WARPS) {
+            const __half* s_t = reinterpret_cast<const __half*>(rank_t + nslots);
+            for (int i = dw; i < nslots; i += XT_DQ_WARPS) {
               const int rk = rank_t[i], pos = slot_pos(i);
-              if (rk >= 0 && rk < h_rank) continue;
+              const bool live = rk >= 0 && rk < h_rank;
+              if (live && pos_r[m * h_rank + rk] == pos) continue;
+              const __half sv = live ? s_t[i] : __float2half(0.f);
               for (int n = lane; n < n_tok; n += 32)
-                *reinterpret_cast<__half*>(sm.act + m * act_m_bytes + (pos >> 3) * cs + (pos & 7) * 2 + n * 16) = __float2half(0.f);
+                *reinterpret_cast<__half*>(sm.act + m * act_m_bytes + (pos >> 3) * cs + (pos & 7) * 2 + n * 16) =
+                    live ? __hmul((m ? A.h_up : A.h_gate)[static_cast<int64_t>(item.tok[n]) * h_rank + rk], sv) : sv;
             }
           }
         }

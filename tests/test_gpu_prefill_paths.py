@@ -68,6 +68,30 @@ def test_sums_reach_rows_of_any_alignment(rank_out, shift):
         assert buf[:shift].eq(7.0).all() and buf[shift + T * rank_out:].eq(7.0).all()
 
 
+# matrices in which several rows hold the same rank: single rows (of one width and of two), and a whole aligned octet twice
+def test_rows_that_repeat_a_rank():
+    E, rank, inter, T = 3, 64, 256, 200
+    s = synth.make_layer(synth.tiny(hidden=128, num_experts=E, intermediate=inter, top_k=1, rank=rank), seed=3, device=DEV)
+    for tag in ("gate", "up", "down"):
+        idx = [t.clone() for t in s.tables[tag]["rank_idx"]]
+        idx[0][40] = idx[0][41]
+        idx[0][2] = idx[0][60]
+        idx[1][8:16] = torch.arange(16, 24)
+        idx[1][48:56] = torch.arange(16, 24)
+        s.tables[tag]["rank_idx"] = idx
+    layer = synth.to_packed_layer(s)
+    gen = torch.Generator(device=DEV).manual_seed(6)
+    tok, off, rw = _route((150, 131, 20), 1, T, gen)
+    hg, hu = layer.basis_project(torch.randn(T, 128, generator=gen, device=DEV).half())
+    want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
+    for path in (capi.PATH_DECODE, capi.PATH_TENSOR):
+        nan = torch.full_like(hg, float("nan"))
+        layer.experts_forward(nan, nan, tok, off, rw, path=path)      # what a kernel does not write still holds these
+        got = layer.experts_forward(hg, hu, tok, off, rw, path=path)
+        layer.check_status()
+        helpers.assert_close(got.cpu(), want.cpu(), what=f"path {path}")
+
+
 # token counts around the blocks of the counting pass; expert counts around a warp of the scan and the top-k's registers
 @pytest.mark.parametrize("T", [129, 1025, 4097, 16385])
 @pytest.mark.parametrize("E,k", [(2, 2), (33, 5), (128, 8), (512, 10)])
