@@ -86,6 +86,7 @@ struct MatHost {
   int32_t n_rows = 0;
 };
 
+constexpr int DEFAULT_WAIT_LIMIT_US = 2000000;
 constexpr int FAST_MAX_TOK = 8;    // assignments per pass of the decode kernel (one MMA N-block)
 
 struct FastMat {
@@ -257,6 +258,7 @@ struct bm_layer {
   bool deterministic = false;      // rank_accum through 64-bit fixed-point atomics (bm_layer_set_option)
   int dec_ring = 0, dec_sec_bytes = 0, dec_grid = 0, dec_act_bufs = 2, dec_ctas = 0, dec_force_ctas = 0;
   size_t dec_smem = 0;
+  int wait_limit_us = bm::DEFAULT_WAIT_LIMIT_US;   // of the packed-expert kernels' waits (bm_layer_set_option)
   int* status_dev = nullptr;       // device flag set by a kernel whose bounded wait gave up
   cudaStream_t side_stream = nullptr;   // routing runs here, beside the basis projection
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;

@@ -33,7 +33,8 @@
 // converted weights through the cluster's shared memory took longer (257 us): five slots of ring do not cover the way over.
 //
 // The down product of a chunk is issued one chunk late (G0 U0 | G1 U1 D0 | G2 U2 D1 | ...).  Every mbarrier wait is
-// bounded in time and aborts the whole CTA through a shared flag.
+// bounded in time.  One that gives up raises a flag of the CTA; the roles then leave at their next wait that is not over, the
+// look-up warp behind its copy and the MMA issuers behind their MMAs, and tensor memory is given back after that.
 #include "fast_layout.cuh"
 #include "tc05.cuh"
 
@@ -70,6 +71,7 @@ struct XtBars {
   uint64_t gu_done[2], gu_free[2];        // gate/up accumulators of a chunk complete / read out
   uint64_t z_ready, z_free;               // z operand of a chunk written / multiplied
   uint64_t down_done, down_free;          // down sums of an item complete / read out
+  uint64_t drained[2];                    // every MMA of the pipeline complete (at the end of the kernel)
 };
 
 // Position in a cyclic buffer of n slots with the phase bit of its mbarriers.
@@ -92,6 +94,7 @@ struct XtItem {
   int pad_;
 };
 
+// abort_flag[0]: a wait of this CTA gave up; abort_flag[1]: the limit of a wait in microseconds
 __device__ __forceinline__ bool xt_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   const uint32_t addr = tc::smem_u32(bar);
   uint64_t t0 = 0;
@@ -107,7 +110,7 @@ __device__ __forceinline__ bool xt_wait_slow(uint64_t* bar, uint32_t parity, vol
     if ((i & 15u) == 15u) {
       const uint64_t now = tc::global_ns();
       if (t0 == 0) t0 = now;
-      else if (now - t0 > tc::WAIT_LIMIT_NS) { *abort_flag = 1; return false; }
+      else if (now - t0 > static_cast<uint64_t>(abort_flag[1]) * 1000u) { *abort_flag = 1; return false; }
     }
   }
 }
@@ -227,6 +230,7 @@ struct XtArgs {
   long long* acc64;
   int* status;
   int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, ring_h, gu_bufs, tab_bytes;
+  int wait_limit_us;
   int vec_add;            // every row of rank_accum starts on a 16-byte boundary (and takes fp32 adds)
 };
 
@@ -283,8 +287,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
   __shared__ __align__(8) XtBars bars;
   __shared__ XtItem items[2];             // this item and the next one (looked up while this one runs)
   __shared__ uint32_t tmem_slot;
-  __shared__ int abort_flag_s;
-  volatile int* abort_flag = &abort_flag_s;
+  __shared__ int abort_flag_s[2];
+  volatile int* abort_flag = abort_flag_s;
   const int warp = tc::warp_index(), lane = threadIdx.x & 31;
   const int nt = A.nt, ring_h = A.ring_h, h_rank = A.h_rank, num_experts = A.num_experts;
   const int cs = xt_chunk_stride(nt);     // bytes between 8-position chunks of act
@@ -316,9 +320,11 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       tc::mbar_init(&bars.item_free[i], XT_EPI_WARPS + XT_DQ_WARPS + 2);
       tc::mbar_init(&bars.gu_done[i], 2);
       tc::mbar_init(&bars.gu_free[i], XT_EPI_WARPS);
+      tc::mbar_init(&bars.drained[i], 1);
     }
     tc::mbar_init_fence();
-    abort_flag_s = 0;
+    abort_flag_s[0] = A.wait_limit_us == 0;
+    abort_flag_s[1] = A.wait_limit_us;
   }
   if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
   // items before each expert (an item = up to nt consecutive assignments of one expert): every thread loads
@@ -483,7 +489,7 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     tc::fence_before_sync();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
-    if (threadIdx.x == 0 && abort_flag_s) atomicExch(A.status, BM_ERR_TIMEOUT);
+    if (threadIdx.x == 0 && *abort_flag) atomicExch(A.status, BM_ERR_TIMEOUT);
     return;
   }
   if (warp < XT_DQ_WARP0 + XT_DQ_WARPS) {
@@ -707,7 +713,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       xt_load_item(items[ib], sm.tab + ib * lay.bytes, &bars.item_full[ib], u, units, n_chunks, sm, A, lane);
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&bars.item_full[ib]);
-      if (!xt_wait(&bars.item_full[ib], (round >> 1) & 1u, abort_flag)) break;
+      // the copy lands whatever the other roles do: waited for also when one of them has given up
+      if (!tc::mbar_wait(&bars.item_full[ib], (round >> 1) & 1u)) { *abort_flag = 1; break; }
       // the weights on their way to L2, one tile per lane (sizes and offsets are multiples of 16 bytes)
       const FastExpert& fe = reinterpret_cast<const TokTabHead*>(sm.tab + ib * lay.bytes)->fe;
       const int t0 = items[ib].chunk0 >> 1, t1 = (items[ib].chunk0 + items[ib].nchunk + 1) >> 1;
@@ -795,6 +802,9 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       gu_round += nchunk;
       if (!ok) break;
     }
+    if (tc::elect_one()) tc::mma_commit(&bars.drained[pl]);
+    __syncwarp();
+    if (!tc::mbar_wait(&bars.drained[pl], 0)) *abort_flag = 1;
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -861,6 +871,7 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
   a.rank_accum = rank_accum; a.acc64 = acc64; a.status = L->status_dev;
   // an octet's two 16-byte adds need the row's start, and so rank_out and the base, at multiples of four floats
   a.vec_add = acc64 == nullptr && L->rank_out % 4 == 0 && (reinterpret_cast<uintptr_t>(rank_accum) & 15u) == 0;
+  a.wait_limit_us = L->wait_limit_us;
   a.rank_out = L->rank_out; a.T = T; a.num_experts = L->num_experts; a.n_tiles = L->n_tiles; a.max_slots = L->max_slots;
   a.nt = plan.nt; a.ring_h = plan.ring_h; a.gu_bufs = plan.gu_bufs;
   experts_tc_kernel<<<sm_counts[dev], XT_THREADS, plan.smem, st>>>(a);

@@ -387,6 +387,11 @@ extern "C" int bm_layer_set_option(bm_layer_t* L, int32_t option, int32_t value)
     L->deterministic = value != 0;
     return BM_OK;
   }
+  if (option == BM_OPT_WAIT_LIMIT_US) {
+    BM_REQUIRE(value >= 0 && value <= DEFAULT_WAIT_LIMIT_US, BM_ERR_INVALID_ARG, "set_option: the wait limit must be 0..%d us", DEFAULT_WAIT_LIMIT_US);
+    L->wait_limit_us = value;
+    return BM_OK;
+  }
   BM_REQUIRE(option == BM_OPT_DECODE_CTAS_PER_SM, BM_ERR_INVALID_ARG, "set_option: unknown option %d", option);
   BM_REQUIRE(value >= 0 && value <= 3, BM_ERR_INVALID_ARG, "set_option: CTAs per SM must be 0..3");
   const bm_layer saved = *L;

@@ -136,8 +136,12 @@ BM_API int bm_layer_status(const bm_layer_t* layer, void* stream);
  *     instead of fp32 atomics (bitsmoe/algorithms/cpp/mlp_forward.cu:2062 uses fp32 atomics, whose result depends on
  *     arrival order): two runs on the same inputs are then bit-identical.  bm_experts_workspace_bytes /
  *     bm_layer_workspace_bytes grow by 8 bytes per rank_accum element; ask them again after switching.
+ *   BM_OPT_WAIT_LIMIT_US (0 .. 2000000, the default): longest time a packed-expert kernel waits at one of its barriers
+ *     before it gives up.  With 0 a kernel starts as if a wait had run out: every wait that is not over at once gives
+ *     up, the kernel leaves with its copies and products drained, its outputs are undefined and bm_layer_status()
+ *     reports BM_ERR_TIMEOUT.  It is how that way out is tested.
  * Returns BM_ERR_UNSUPPORTED when the layer's working set does not fit the requested geometry (nothing changes). */
-enum { BM_OPT_DECODE_CTAS_PER_SM = 0, BM_OPT_DETERMINISTIC = 1 };
+enum { BM_OPT_DECODE_CTAS_PER_SM = 0, BM_OPT_DETERMINISTIC = 1, BM_OPT_WAIT_LIMIT_US = 2 };
 BM_API int bm_layer_set_option(bm_layer_t* layer, int32_t option, int32_t value);
 
 /* No counterpart in the reference.  Launches a one-warp kernel whose only job is to wait (at most limit_us

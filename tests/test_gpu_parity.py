@@ -462,6 +462,29 @@ def test_bounded_wait_gives_up_and_reports_timeout(q30_small):
     assert float(torch.ones(4, device=DEV).sum()) == 4.0
 
 
+@pytest.mark.parametrize("path", [capi.PATH_TENSOR])
+@pytest.mark.parametrize("T", [8, 700])
+def test_expert_kernels_leave_cleanly_when_a_wait_gives_up(q30_small, path, T):
+    """With the limit at 0 the roles of every CTA leave at their first wait that is not over, with copies and products
+    under way: the launch ends, the time-out is reported once, and the next launches compute what they should."""
+    layer, packed, _ = q30_small
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    hg, hu = (torch.randn(T, layer.cfg.rank, generator=gen, device=DEV).half() for _ in range(2))
+    idx, w = packed.route_topk(torch.randn(T, layer.cfg.num_experts, generator=gen, device=DEV), layer.cfg.top_k, True, None)
+    args = (hg, hu, *route_build(idx, w, layer.cfg.num_experts)[:3])
+    want = packed.experts_forward(*args, path=capi.PATH_GENERIC)
+    packed.check_status()
+    for _ in range(3):
+        capi.check(capi.lib().bm_layer_set_option(packed._handle, 2, 0))
+        packed.experts_forward(*args, path=path)
+        with pytest.raises(capi.BitsMoEError, match="bounded wait"):
+            packed.check_status()
+        capi.check(capi.lib().bm_layer_set_option(packed._handle, 2, 2000000))
+        got = packed.experts_forward(*args, path=path)
+        packed.check_status()
+        helpers.assert_close(got.cpu(), want.cpu(), what=f"path {path} after a time-out")
+
+
 @pytest.mark.parametrize("T,E,H,dtype", [(1, 128, 2048, torch.bfloat16), (64, 128, 2048, torch.bfloat16), (64, 512, 2048, torch.float16),
                                          (7, 64, 2048, torch.float16), (1000, 128, 2048, torch.bfloat16), (33, 24, 384, torch.float32),
                                          # the tiled-copy GEMM: ragged rows, ragged and narrow outputs, one K slice, every input type
