@@ -20,13 +20,16 @@
 // of a pair and an operand built without branches: a tile 4.5 -> 4.0 us in the first, 3.6 -> 3.2 in the later ones; a block of
 // 64 tokens 44.0 -> 42.3 us.
 //
-// Every wait is bounded (a launch parameter); a wait that gives up raises a CTA-wide abort flag, all threads leave
-// through the same barriers, and the layer's status word reports BM_ERR_TIMEOUT.
+// Every wait is bounded (a launch parameter); a wait that gives up raises a CTA-wide flag, at which the others' waits give up
+// too.  The compute warps decide together, at the barrier that follows a wait, whether to leave: the flag may come up between
+// one warp's look and another's, and a warp that left alone would leave the others at the next barrier.  The layer's status
+// word reports BM_ERR_TIMEOUT.
 #include "fast_layout.cuh"
 #include "tc05.cuh"
 
 namespace bm {
 
+constexpr uint64_t DEC_DRAIN_LIMIT_NS = 100000000;   // of the wait for copies under way when a CTA has given up
 constexpr int DEC_THREADS = 288;             // 8 compute warps + 1 producer warp
 constexpr int DEC_CONSUMERS = 256;
 constexpr int DEC_MAX_E = 1024;
@@ -96,7 +99,15 @@ struct DecUnitInfo {
 
 // a / b for 0 <= a < 2^20, 1 <= b: the quotient of a + 1/2 stays 1 / (2 b) away from a whole number, more than its rounding
 __device__ __forceinline__ int div_small(int a, int b) { return static_cast<int>(__fdividef(static_cast<float>(a) + 0.5f, static_cast<float>(b))); }
-__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;" ::"n"(DEC_CONSUMERS) : "memory"); }
+// Barrier of the compute warps; true for all of them when `leave` is for any.
+__device__ __forceinline__ bool consumer_sync(bool leave) {
+  uint32_t any;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+               : "=r"(any)
+               : "r"(static_cast<uint32_t>(leave)), "n"(DEC_CONSUMERS)
+               : "memory");
+  return any != 0;
+}
 
 // Bounded wait shared by all roles: one plain probe (a wait that is already over costs 35 cycles, with a suspend time
 // given 250), then a loop out of line that gives up when another thread of the CTA already did, or after limit_ns.
@@ -268,7 +279,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const De
     tc::mbar_init(&bar_tail_empty[1], 8);
     tc::mbar_init(&bar_head_empty, 8);
     tc::mbar_init_fence();
-    abort_raw = 0;
+    abort_raw = limit == 0;
   }
   // everything above runs while the kernel before this one (launched with programmatic serialisation) drains
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -330,7 +341,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const De
   if (warp == 8) {
     // ------------------------------------------------------------------ producer warp
     // lane m (0..2) owns section m (gate, up, down) of every tile: its ring slot advances by 3 per tile
-    uint32_t my_slot = lane < 3 ? static_cast<uint32_t>(lane) : 0u, my_phase = 0;
+    uint32_t my_slot = lane < 3 ? static_cast<uint32_t>(lane) : 0u, my_phase = 0, issued = 0;
     bool ok = true;
     int it = 0;
     for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++it) {
@@ -402,25 +413,27 @@ __global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const De
           tc::mbar_expect_tx(&bar_full[my_slot], bytes);
           tc::bulk_g2s(ring + static_cast<size_t>(my_slot) * P.sec_bytes, src, bytes, &bar_full[my_slot]);
           src += fe.unit_bytes;
+          ++issued;
           my_slot += 3u;
           if (my_slot >= R) { my_slot -= R; my_phase ^= 1u; }
         }
       }
       ok = __all_sync(0xffffffffu, ok);
     }
-    if (*abort_flag) {
+    if (__any_sync(0xffffffffu, *abort_flag)) {
       // leave only after the copies already started have landed (or their wait ran out): every barrier that still
       // has a transaction pending completes its current phase when the bytes arrive
-      __syncwarp();
       if (lane < 3) {
-        // the last section this lane issued sits R/3 or fewer tiles back; waiting for the phase it was issued in is enough
+        // this lane's sections in the last R places: the slots of earlier ones were issued again, so those had landed
         uint32_t s = my_slot, ph = my_phase;
-        if (s < 3u) { s += R; ph ^= 1u; }
-        s -= 3u;
-        tc::mbar_wait(&bar_full[s], ph, limit);
+        for (uint32_t j = 0; j < issued && 3u * j < R; ++j) {
+          if (s < 3u) { s += R; ph ^= 1u; }
+          s -= 3u;
+          tc::mbar_wait(&bar_full[s], ph, DEC_DRAIN_LIMIT_NS);
+        }
       }
       if (lane == 0) {
-        for (int j = it > 2 ? it - 2 : 0; j < it; ++j) tc::mbar_wait(&bar_unit_full[j & 1], (j >> 1) & 1, limit);
+        for (int j = it > 2 ? it - 2 : 0; j < it; ++j) tc::mbar_wait(&bar_unit_full[j & 1], (j >> 1) & 1, DEC_DRAIN_LIMIT_NS);
         atomicExch(P.status, BM_ERR_TIMEOUT);
       }
     }
@@ -433,9 +446,10 @@ __global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const De
   const int zpos_lo = slot_pos(16 * warp + g), zpos_hi = slot_pos(16 * warp + g + 8);   // where this thread's z values go
   uint32_t rs = 0, rp = 0;      // ring slot and phase of the current tile's gate section
   int it = 0;
+  bool ok = true, leave = false;      // this warp's waits; what the compute warps decided
   for (int u = blockIdx.x; u < n_units; u += gridDim.x, ++it) {
     const int ub = it & 1;
-    bool ok = dec_wait(&bar_unit_full[ub], (it >> 1) & 1, abort_flag, limit);
+    ok = ok && dec_wait(&bar_unit_full[ub], (it >> 1) & 1, abort_flag, limit);
     const DecUnitInfo& si = info[ub];
     const FastExpert& fe = si.fe;
     const int npass = si.npass, tile0 = si.tile0, ntl = si.ntiles;
@@ -465,8 +479,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const De
         }
       }
     }
-    consumer_sync();
-    if (*abort_flag) break;
+    if ((leave = consumer_sync(!ok))) break;
     if (lane == 0) tc::mbar_arrive(&bar_head_empty);     // h rows and gate/up tables are consumed
 
     // Operand of one tile: act[buf][m][n][:] = hs[m][n][:] * scale_m(tile)[:], and the offset-weighted sum of every row.
@@ -502,8 +515,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const De
     };
 
     ok = ok && build_operand(0, rs, rp);
-    consumer_sync();
-    if (*abort_flag) break;
+    if ((leave = consumer_sync(!ok))) break;
 
     float dtot[MAXMB][4];
 #pragma unroll
@@ -583,8 +595,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const De
       // ---- the next tile's operand goes into the other buffer before the barrier; with one buffer it has to wait
       // until every warp is done with this tile's operand
       if (P.act_bufs == 2 && i + 1 < ntl && ok) ok = build_operand(buf ^ 1, ns, np);
-      consumer_sync();
-      if (*abort_flag) break;
+      if ((leave = consumer_sync(!ok))) break;
       // ---- down: slot blocks round-robin over the warps, contraction over the tile's 128 columns
       {
         ok = dec_wait(&bar_full[ds], dp, abort_flag, limit);
@@ -629,13 +640,12 @@ __global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const De
       }
       if (P.act_bufs == 1 && i + 1 < ntl) {
         if (ok) ok = build_operand(0, ns, np);
-        consumer_sync();
-        if (*abort_flag) break;
+        if ((leave = consumer_sync(!ok))) break;
       }
       rs = ns;
       rp = np;
     }
-    if (*abort_flag) break;
+    if (leave) break;
     // ---- unit epilogue: rank_accum[token, logical rank] += sum over the unit's tiles * S * route weight
     {
       const unsigned char* tab = smem_raw + lay.tab_d + ub * lay.tab_bytes;
@@ -664,7 +674,7 @@ __global__ void __launch_bounds__(DEC_THREADS, 2) experts_decode_kernel(const De
     __syncwarp();
     if (lane == 0) tc::mbar_arrive(&bar_tail_empty[ub]);
   }
-  if (*abort_flag && tid == 0) atomicExch(P.status, BM_ERR_TIMEOUT);
+  if ((leave || !ok) && lane == 0) atomicExch(P.status, BM_ERR_TIMEOUT);
 }
 
 // Launch geometry of the decode kernel for this layer on the current device: ring depth, shared memory, grid.
@@ -754,7 +764,7 @@ int launch_experts_decode(const bm_layer* L, const __half* h_gate, const __half*
   P.sec_bytes = L->dec_sec_bytes;
   P.ring = L->dec_ring;
   P.act_bufs = L->dec_act_bufs;
-  P.wait_limit_ns = tc::WAIT_LIMIT_NS;
+  P.wait_limit_ns = static_cast<unsigned long long>(L->wait_limit_us) * 1000u;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(L->dec_grid);
   cfg.blockDim = dim3(DEC_THREADS);

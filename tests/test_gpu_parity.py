@@ -462,8 +462,8 @@ def test_bounded_wait_gives_up_and_reports_timeout(q30_small):
     assert float(torch.ones(4, device=DEV).sum()) == 4.0
 
 
-@pytest.mark.parametrize("path", [capi.PATH_TENSOR])
-@pytest.mark.parametrize("T", [8, 700])
+@pytest.mark.parametrize("path", [capi.PATH_DECODE, capi.PATH_TENSOR])
+@pytest.mark.parametrize("T", [1, 8, 700])
 def test_expert_kernels_leave_cleanly_when_a_wait_gives_up(q30_small, path, T):
     """With the limit at 0 the roles of every CTA leave at their first wait that is not over, with copies and products
     under way: the launch ends, the time-out is reported once, and the next launches compute what they should."""
