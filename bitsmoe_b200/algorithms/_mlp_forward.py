@@ -62,6 +62,7 @@ def moe_packed_forward(h_gate, h_up, token_indices, expert_offsets, route_weight
     _check(h_gate.dim() == 2, "h_gate must be 2D [tokens, rank]")
     _check(h_up.dim() == 2, "h_up must be 2D [tokens, rank]")
     _check(h_gate.shape[0] == h_up.shape[0], "h_gate/h_up token dim mismatch")
+    _check(h_gate.shape[1] == h_up.shape[1], "h_gate/h_up rank dim mismatch")
     _check(token_indices.dim() == 1, "token_indices must be 1D")
     _check(expert_offsets.dim() == 1, "expert_offsets must be 1D")
     _check(route_weights.dim() == 1, "route_weights must be 1D")

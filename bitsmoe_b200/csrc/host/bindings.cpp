@@ -63,6 +63,7 @@ const uint16_t* wptr(const at::Tensor& t) { return static_cast<const uint16_t*>(
 struct HostLayer {
   bm_layer_t* handle = nullptr;
   c10::Device device{c10::kCUDA, 0};
+  int64_t hidden = 0, rank_in = 0, rank_out = 0, experts = 0;      // hidden 0: the layer has no basis matrices
   struct Ws { int64_t T, k, variant; at::Tensor buf; };
   std::vector<Ws> ws;
 
@@ -90,6 +91,20 @@ at::Tensor contiguous(const at::Tensor& t) { return t.is_contiguous() ? t : t.co
 void require_cuda(const at::Tensor& t, const char* what) {
   if (!t.is_cuda()) fail(PyExc_RuntimeError, std::string(what) + " requires CUDA tensors; there is no CPU path");
 }
+// The library takes pointers: what a tensor has to hold is checked here, where its size is known.
+void require(bool ok, const char* msg) {
+  if (!ok) fail(PyExc_RuntimeError, msg);
+}
+void require_matrix(const at::Tensor& t, int64_t rows, int64_t cols, const char* msg) {
+  require(t.dim() == 2 && t.size(0) == rows && t.size(1) == cols, msg);
+}
+void require_residual(const at::Tensor& residual, const at::Tensor& x) {
+  require(!residual.defined() || (residual.device() == x.device() && residual.numel() == x.numel()), "residual must have x's elements and device");
+}
+void require_map(const at::Tensor& g2l, int64_t num_routed, c10::Device device) {
+  require(!g2l.defined() || (g2l.scalar_type() == at::kInt && g2l.is_contiguous() && g2l.device() == device && g2l.numel() >= num_routed),
+          "global_to_local must be a contiguous int32 entry for every routed expert, on the layer's device");
+}
 void* stream_of(c10::Device d) { return c10::cuda::getCurrentCUDAStream(d.index()).stream(); }
 
 template <typename F>
@@ -109,12 +124,14 @@ void need_args(Py_ssize_t got, Py_ssize_t want) {
 }
 
 // ---- layers
-PyObject* layer_new(PyObject*, PyObject* const* a, Py_ssize_t n) {      // (handle, device index)
+PyObject* layer_new(PyObject*, PyObject* const* a, Py_ssize_t n) {      // (handle, device index, hidden, rank_in, rank_out, experts)
   return guarded([&] {
-    need_args(n, 2);
-    auto* L = new HostLayer();
-    L->handle = static_cast<bm_layer_t*>(PyLong_AsVoidPtr(a[0]));
-    L->device = c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(integer(a[1])));
+    need_args(n, 6);
+    HostLayer made;
+    made.handle = static_cast<bm_layer_t*>(PyLong_AsVoidPtr(a[0]));
+    made.device = c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(integer(a[1])));
+    made.hidden = integer(a[2]); made.rank_in = integer(a[3]); made.rank_out = integer(a[4]); made.experts = integer(a[5]);
+    auto* L = new HostLayer(std::move(made));
     return PyCapsule_New(L, CAPSULE, [](PyObject* o) { delete static_cast<HostLayer*>(PyCapsule_GetPointer(o, CAPSULE)); });
   });
 }
@@ -154,11 +171,18 @@ PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor x = contiguous(tensor(a[1])), logits = contiguous(tensor(a[2]));
     require_cuda(x, "forward");
     require_cuda(logits, "forward");
+    require(x.device() == L->device && logits.device() == L->device, "forward: x and logits must be on the layer's device");
+    require(x.dim() >= 1 && logits.dim() == 2 && logits.size(0) == x.size(0), "forward: x [T, H] and logits [T, E] must have the same tokens");
     const int32_t k = static_cast<int32_t>(integer(a[3]));
     const int64_t T = x.size(0);
+    require(L->hidden == 0 || x.numel() == T * L->hidden, "forward: the rows of x do not have the layer's hidden size");
     const int xd = dtype_code(x.scalar_type()), ld = dtype_code(logits.scalar_type());
     at::Tensor residual = opt_tensor(a[6]);
     const at::Tensor g2l = opt_tensor(a[7]), out = opt_tensor(a[9]);
+    require_residual(residual, x);
+    require_map(g2l, logits.size(1), L->device);
+    require(!out.defined() || (out.scalar_type() == x.scalar_type() && out.device() == x.device() && out.is_contiguous() && out.numel() == x.numel()),
+            "forward: out must be contiguous, of x's type and device, and hold x's elements");
     const c10::cuda::CUDAGuard guard(L->device);
     const at::Tensor y = out.defined() ? out : at::empty_like(x);
     if (residual.defined()) residual = contiguous(residual.scalar_type() == x.scalar_type() ? residual : residual.to(x.scalar_type()));
@@ -196,16 +220,23 @@ PyObject* block_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor x = contiguous(tensor(a[1]));
     const at::Tensor w[5] = {tensor(a[2]), opt_tensor(a[3]), opt_tensor(a[4]), opt_tensor(a[5]), opt_tensor(a[6])};
     if ((x.scalar_type() != at::kHalf && x.scalar_type() != at::kBFloat16) || !x.is_cuda() || x.device() != L->device ||
-        !block_weights_ok(w, 5, x) || x.dim() < 2 || x.size(-1) % 8 != 0)
+        !block_weights_ok(w, 5, x) || x.dim() < 2 || w[0].dim() != 2 || x.size(-1) == 0 || x.size(-1) % 8 != 0)
       Py_RETURN_NONE;
     bm_block_dense_t d{};
     d.gate_w = wptr(w[0]);
     d.sh_gate = wptr(w[1]); d.sh_up = wptr(w[2]); d.sh_down = wptr(w[3]); d.sh_token_gate = wptr(w[4]);
     d.sh_intermediate = w[1].defined() ? static_cast<int32_t>(w[1].size(0)) : 0;
     d.w_dtype = dtype_code(w[0].scalar_type());
-    const int64_t T = x.numel() / x.size(-1), E = w[0].size(0);
+    const int64_t H = x.size(-1), T = x.numel() / H, E = w[0].size(0), I = d.sh_intermediate;
+    require(L->hidden == 0 || H == L->hidden, "block_forward: the rows of x do not have the layer's hidden size");
+    require_matrix(w[0], E, H, "block_forward: the router weight must be [experts, hidden]");
+    if (w[1].defined()) require_matrix(w[1], I, H, "block_forward: the shared gate weight must be [intermediate, hidden]");
+    if (w[2].defined()) require_matrix(w[2], I, H, "block_forward: the shared up weight must be [intermediate, hidden]");
+    if (w[3].defined()) require_matrix(w[3], H, I, "block_forward: the shared down weight must be [hidden, intermediate]");
+    require(!w[4].defined() || w[4].numel() == H, "block_forward: the token gate's weight must have hidden elements");
     const int32_t k = static_cast<int32_t>(integer(a[7]));
     const at::Tensor g2l = opt_tensor(a[10]);
+    require_map(g2l, E, L->device);
     const c10::cuda::CUDAGuard guard(L->device);
     const at::Tensor y = at::empty_like(x), logits = at::empty({T, E}, x.options());
     const BlockNeed need{&d, static_cast<int32_t>(E)};
@@ -236,7 +267,13 @@ PyObject* dense_mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor wg = half(tensor(a[1])), wu = half(tensor(a[2])), wd = half(tensor(a[3]));
     const at::Tensor tg = a[4] == Py_None ? at::Tensor() : half(tensor(a[4]));
     at::Tensor residual = opt_tensor(a[5]);
+    require(x.dim() == 2 && wg.dim() == 2, "dense_mlp: x must be [T, H] and the gate weight [I, H]");
     const int32_t T = static_cast<int32_t>(x.size(0)), H = static_cast<int32_t>(x.size(1)), I = static_cast<int32_t>(wg.size(0));
+    require_matrix(wg, I, H, "dense_mlp: the gate weight must be [intermediate, hidden]");
+    require_matrix(wu, I, H, "dense_mlp: the up weight must be [intermediate, hidden]");
+    require_matrix(wd, H, I, "dense_mlp: the down weight must be [hidden, intermediate]");
+    require(!tg.defined() || tg.numel() == H, "dense_mlp: the token gate's weight must have hidden elements");
+    require_residual(residual, x);
     const int xd = dtype_code(x.scalar_type());
     const at::Tensor y = at::empty_like(x);
     if (residual.defined()) residual = contiguous(residual.scalar_type() == x.scalar_type() ? residual : residual.to(x.scalar_type()));
@@ -250,6 +287,15 @@ PyObject* dense_mlp(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 at::Tensor run_experts(HostLayer* L, const at::Tensor& hg, const at::Tensor& hu, const at::Tensor& tok, const at::Tensor& off,
                        const at::Tensor& rw, int64_t rank_out, int32_t path) {
+  // h_up may have fewer rows than h_gate: only the rows that token_indices names are read
+  for (const at::Tensor* h : {&hg, &hu})
+    require(h->device() == L->device && h->scalar_type() == at::kHalf && h->is_contiguous() && h->dim() == 2 && h->size(1) == L->rank_in,
+            "experts_forward: h_gate and h_up must be contiguous float16 [tokens, rank] of the layer's rank and device");
+  require(rank_out == L->rank_out, "experts_forward: rank_out is not the layer's");
+  require(tok.device() == L->device && tok.scalar_type() == at::kInt && tok.is_contiguous() && off.device() == L->device &&
+              off.scalar_type() == at::kInt && off.is_contiguous() && off.numel() == L->experts + 1 && rw.device() == L->device &&
+              rw.scalar_type() == at::kFloat && rw.is_contiguous() && rw.numel() >= tok.numel(),
+          "experts_forward: routing must be contiguous on the layer's device: int32 token_indices, int32 expert_offsets [experts + 1], float32 weights");
   const c10::cuda::CUDAGuard guard(L->device);
   const int32_t T = static_cast<int32_t>(hg.size(0)), A = static_cast<int32_t>(tok.numel());
   const at::Tensor out = at::empty({T, rank_out}, hg.options().dtype(at::kFloat));
@@ -315,7 +361,7 @@ PyObject* op_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return t.is_cuda() && t.scalar_type() == type && t.dim() == dim && t.is_contiguous();
     };
     if (!ok(hg, at::kHalf, 2) || !ok(hu, at::kHalf, 2) || !ok(tok, at::kInt, 1) || !ok(off, at::kInt, 1) || !ok(rw, at::kFloat, 1) ||
-        hg.size(0) != hu.size(0) || tok.numel() != rw.numel() || tok.numel() == 0 || off.numel() < 2)
+        hg.sizes() != hu.sizes() || tok.numel() != rw.numel() || tok.numel() == 0 || off.numel() < 2)
       Py_RETURN_NONE;
     for (int i = 5; i < 23; ++i)
       if ((!PyTuple_Check(a[i]) && !PyList_Check(a[i])) || PySequence_Fast_GET_SIZE(a[i]) != off.numel() - 1) Py_RETURN_NONE;

@@ -376,6 +376,9 @@ class SymmetricExpertParallel:
         G, T, k, r, r_out = self.world, self.T, self.top_k, pk.rank_in, pk.rank_out
         if x.shape[0] != T:
             raise ValueError(f"a wave holds {T} tokens per rank, got {x.shape[0]}")
+        if x.numel() != T * pk.hidden or logits.dim() != 2 or logits.shape[0] != T or out.numel() != x.numel() or not out.is_contiguous() or \
+                (residual is not None and residual.numel() != x.numel()):
+            raise ValueError("a wave takes x [T, H] and logits [T, E] and writes a contiguous out [T, H]")
         h, rt, part = self._own(area)
         sc = self._scratch[area]
         h_tab, r_tab, p_tab = self._tabs[area]

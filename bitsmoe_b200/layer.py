@@ -27,6 +27,11 @@ def _as(t: torch.Tensor, dtype: torch.dtype, device: torch.device) -> torch.Tens
     return t
 
 
+def _require(ok: bool, msg: str) -> None:
+    if not ok:
+        raise RuntimeError(msg)
+
+
 class PackedLayer:
     def __init__(self, gate: Dict[str, Sequence[torch.Tensor]], up: Dict[str, Sequence[torch.Tensor]],
                  down: Dict[str, Sequence[torch.Tensor]], intermediate_size: int, rank_out: int,
@@ -82,6 +87,11 @@ class PackedLayer:
             int(self.u_down.shape[0]) if self.u_down is not None else 0)
         if self.u_down is not None and int(self.u_down.shape[1]) != self.rank_out:
             raise RuntimeError(f"shared_u_down has {int(self.u_down.shape[1])} columns, rank_out is {self.rank_out}")
+        _require(self.vh_gate is None or (self.vh_gate.dim() == 2 and self.vh_gate.shape[0] == self.rank_in),
+                 "shared_vh_gate must be [rank, hidden]")
+        _require(self.vh_up is None or (self.vh_up.dim() == 2 and (self.vh_gate is None or self.vh_up.shape == self.vh_gate.shape)),
+                 "shared_vh_up must have shared_vh_gate's shape")
+        _require(self.u_down is None or self.u_down.shape[0] == self.hidden, "shared_u_down must have a row per hidden channel")
         d = capi.LayerDesc()
         d.num_experts, d.hidden, d.intermediate = n, self.hidden, self.intermediate_size
         d.rank_in, d.rank_out, d.act_type = self.rank_in, self.rank_out, int(act_type)
@@ -98,7 +108,7 @@ class PackedLayer:
                                            capi.stream_ptr(device), C.byref(h)))
         self._handle = h
         self._host = capi.host()
-        self._native = self._host.layer_new(h.value, device.index)
+        self._native = self._host.layer_new(h.value, device.index, self.hidden, self.rank_in, self.rank_out, n)
 
     # -- construction helpers -------------------------------------------------------------------------
     @classmethod
@@ -160,9 +170,14 @@ class PackedLayer:
         """h_gate, h_up [T, r] fp16; ``out`` may be a preallocated [2, T, r] fp16 tensor that receives both."""
         x = x.contiguous()
         T = x.shape[0]
+        _require(x.device == self.device and (self.vh_gate is None or x.numel() == T * self.hidden),
+                 "basis_project: x must be [T, H] of the layer's hidden size and device")
         if out is None:
             out = torch.empty((2, T, self.rank_in), dtype=torch.float16, device=self.device)
         hg, hu = out[0], out[1]
+        for h in (hg, hu):
+            _require(h.dtype == torch.float16 and h.device == self.device and h.is_contiguous() and h.numel() == T * self.rank_in,
+                     "basis_project: out must hold two contiguous float16 [T, rank] matrices on the layer's device")
         with torch.cuda.device(self.device):
             capi.check(capi.lib().bm_basis_project(self._handle, x.data_ptr(), capi.dtype_code(x.dtype), T,
                                                    hg.data_ptr(), hu.data_ptr(), capi.stream_ptr(self.device)))
@@ -175,6 +190,10 @@ class PackedLayer:
     def combine_down_basis(self, rank_accum: torch.Tensor, out_dtype: torch.dtype,
                            residual: Optional[torch.Tensor] = None) -> torch.Tensor:
         T = rank_accum.shape[0]
+        _require(rank_accum.dtype == torch.float32 and rank_accum.device == self.device and rank_accum.is_contiguous()
+                 and rank_accum.numel() == T * self.rank_out, "combine_down_basis: rank_accum must be contiguous float32 [T, rank_out]")
+        _require(residual is None or (residual.device == self.device and residual.numel() == T * self.hidden),
+                 "combine_down_basis: residual must be [T, H] on the layer's device")
         y = torch.empty((T, self.hidden), dtype=out_dtype, device=self.device)
         if residual is not None:
             residual = residual.to(out_dtype).contiguous()
@@ -230,6 +249,7 @@ def route_build(topk_idx: torch.Tensor, topk_w: torch.Tensor, num_local: int,
     dev = topk_idx.device
     topk_idx = topk_idx.to(torch.int32).contiguous()
     topk_w = topk_w.to(torch.float32).contiguous()
+    _require(topk_w.device == dev and topk_idx.dim() == 2 and topk_w.numel() == topk_idx.numel(), "route_build: topk_idx and topk_w must be [T, k] on one device")
     T, k = topk_idx.shape
     lib = capi.lib()
     max_tiles = int(lib.bm_route_max_tiles(T, k, num_local, tile_rows))
@@ -258,6 +278,7 @@ def gate_logits(x: torch.Tensor, gate_weight: torch.Tensor, out_dtype: Optional[
         raise RuntimeError("gate_logits requires CUDA tensors; there is no CPU path")
     x = x.contiguous()
     w = _as(gate_weight.detach(), torch.float16, x.device)
+    _require(x.dim() == 2 and w.dim() == 2 and w.shape[1] == x.shape[1], "gate_logits: x must be [T, H] and gate_weight [E, H]")
     out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype or x.dtype, device=x.device)
     with torch.cuda.device(x.device):
         capi.check(capi.lib().bm_gate_logits(x.data_ptr(), capi.dtype_code(x.dtype), w.data_ptr(), x.shape[0], w.shape[0],
