@@ -326,13 +326,24 @@ int launch_skinny_nt(SkinnyArgs a, cudaStream_t st) {
     const int per = glu ? mrows / 2 : mrows;
     a.row_tiles += (a.seg[i].rows + per - 1) / per;
   }
+  static PerDeviceOnce attr_once;
+  static int sm_counts[MAX_DEVICES];
+  int dev = -1;
+  BM_CUDA(cudaGetDevice(&dev));
+  BM_REQUIRE(dev >= 0 && dev < MAX_DEVICES, BM_ERR_UNSUPPORTED, "skinny_nt: device ordinal %d out of range", dev);
+  if (!attr_once.is_done(dev)) {
+    for (auto* kernel : {skinny_nt_kernel<false, SK_FEW>, skinny_nt_kernel<false, SK_MANY>, skinny_nt_kernel<true, SK_MANY>})
+      BM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SK_SMEM_LIMIT)));
+    BM_CUDA(cudaDeviceGetAttribute(&sm_counts[dev], cudaDevAttrMultiProcessorCount, dev));
+    attr_once.mark(dev);
+  }
   const bool route = a.route.T > 0;
   // One cluster per row tile while the device holds them all at once; more row tiles than that are a loop, which has the
   // next tile's weights in flight where a second wave would start from nothing (5 tokens, two shared experts of 1408: 59 -> 52
   // us a call).
   const int chunks = (a.N + SK_NTOK - 1) / SK_NTOK;
-  constexpr int SMS = 148;
-  auto resident = [](size_t bytes, int most) { const size_t n = 227 * 1024 / (bytes + 1024); return SMS * static_cast<int>(n > most ? most : n); };
+  const int sms = sm_counts[dev];
+  auto resident = [sms](size_t bytes, int most) { return sms * std::min(static_cast<int>(227 * 1024 / (bytes + 1024)), most); };
   size_t smem = sk_smem_bytes(a.K, a.K2, a.splits, a.N, 1);
   a.clusters = a.row_tiles;
   const int total = (a.row_tiles + (route ? 1 : 0)) * a.splits * chunks;
@@ -349,20 +360,12 @@ int launch_skinny_nt(SkinnyArgs a, cudaStream_t st) {
   if (a.clusters == a.row_tiles) {
     // small CTAs are placed several to an SM while other SMs stay empty: ask for the memory that spreads them evenly, with
     // a tenth to spare for clusters that do not fill their group of SMs (64 tokens: 47.2 -> 44.3 us a block)
-    const int per_sm = (total * 11 + 10 * SMS - 1) / (10 * SMS);
+    const int per_sm = (total * 11 + 10 * sms - 1) / (10 * sms);
     const size_t room = (227 * 1024 / std::min(per_sm, 8) - 1024) / 128 * 128;
     smem = std::max(smem, std::min(room, SK_SMEM_LIMIT));
   }
   BM_REQUIRE(!route || a.splits == RS_CLUSTER, BM_ERR_UNSUPPORTED, "skinny_nt: routing needs clusters of %d", RS_CLUSTER);
   if (route && smem < sizeof(RouteSmallSmem)) smem = sizeof(RouteSmallSmem);
-  static PerDeviceOnce attr_once;
-  int dev = -1;
-  BM_CUDA(cudaGetDevice(&dev));
-  if (!attr_once.is_done(dev)) {
-    for (auto* kernel : {skinny_nt_kernel<false, SK_FEW>, skinny_nt_kernel<false, SK_MANY>, skinny_nt_kernel<true, SK_MANY>})
-      BM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(SK_SMEM_LIMIT)));
-    attr_once.mark(dev);
-  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((a.clusters + (route ? 1 : 0)) * a.splits, chunks);
   cfg.blockDim = dim3(SK_THREADS);
