@@ -58,7 +58,6 @@ void plan_fast(const bm_layer* L, size_t base_bytes, FastPlan* P) {
   size_t off = align_up(base_bytes, 256);
   P->table_off = off;
   off += align_up(sizeof(FastExpert) * E, 256);
-  P->tabs_off = off;
   // pass 1: slots per matrix, per-expert tables
   for (int e = 0; e < E; ++e) {
     for (int w = 0; w < 3; ++w) {
@@ -117,7 +116,6 @@ void plan_fast(const bm_layer* L, size_t base_bytes, FastPlan* P) {
     P->toktab_off = off;
     off = align_up(off + static_cast<size_t>(TokTab(L->rank_in, P->max_slots).bytes) * E, 256);
   }
-  P->units_off = off;
   for (int e = 0; e < E; ++e) {
     FastExpert& fe = P->experts[e];
     int o = 0;
@@ -204,9 +202,9 @@ __global__ void __launch_bounds__(128) build_toktab_kernel(const FastExpert* __r
   int16_t *pos_r = reinterpret_cast<int16_t*>(t + lay.pos_r), *oct_r = reinterpret_cast<int16_t*>(t + lay.oct_r);
   float* s_d = reinterpret_cast<float*>(t + lay.s_d);
   int16_t *rank_d = reinterpret_cast<int16_t*>(t + lay.rank_d), *oct_d = reinterpret_cast<int16_t*>(t + lay.oct_d);
-  __shared__ int loose, live_d;
+  __shared__ int loose;
   __shared__ uint32_t broken[2][4];
-  if (threadIdx.x == 0) { loose = 0; live_d = 0; }
+  if (threadIdx.x == 0) loose = 0;
   if (threadIdx.x < 8) broken[threadIdx.x >> 2][threadIdx.x & 3] = 0u;
   for (int i = threadIdx.x; i < 2 * rank_in; i += blockDim.x) { pos_r[i] = -1; s_r[i] = __float2half(0.f); }
   for (int i = threadIdx.x; i < max_slots; i += blockDim.x) { rank_d[i] = -1; s_d[i] = 0.f; }
@@ -221,7 +219,6 @@ __global__ void __launch_bounds__(128) build_toktab_kernel(const FastExpert* __r
         const bool live = rk >= 0 && rk < rank_out;
         rank_d[i] = static_cast<int16_t>(live ? rk : -1);
         s_d[i] = __half2float(s_t[i]);
-        if (live) atomicAdd(&live_d, 1);
       } else if (rk >= 0 && rk < rank_in) {
         pos_r[m * rank_in + rk] = static_cast<int16_t>(slot_pos(i));
       }
@@ -257,7 +254,6 @@ __global__ void __launch_bounds__(128) build_toktab_kernel(const FastExpert* __r
   if (threadIdx.x == 0) {
     head->fe = fe;
     head->loose = loose;
-    head->all_ranks = live_d == rank_out;
   }
   if (threadIdx.x < 8) head->broken[threadIdx.x >> 2][threadIdx.x & 3] = broken[threadIdx.x >> 2][threadIdx.x & 3];
 }
@@ -357,14 +353,9 @@ __global__ void __launch_bounds__(256) arena_decode_kernel(const FastExpert* __r
 
 int build_fast(bm_layer* L, const FastPlan& P, cudaStream_t st) {
   unsigned char* arena = static_cast<unsigned char*>(L->arena);
-  // scratch for slot_row tables: placed at the start of the unit region, overwritten afterwards? No --
-  // kept in the tables region tail is not possible (kernels read it while writing units), so it is
-  // staged in the last unit block area only if it fits; simpler and safe: a dedicated tail.
-  const size_t rows_bytes = align_up(P.slot_row.size() * sizeof(int16_t), 256);
-  const size_t offs_bytes = align_up(P.slot_row_off.size() * sizeof(int32_t), 256);
+  // the slot_row tables are needed while the units are written: they lie behind the arena's last unit
   int16_t* d_rows = reinterpret_cast<int16_t*>(arena + P.total);
-  int32_t* d_offs = reinterpret_cast<int32_t*>(arena + P.total + rows_bytes);
-  (void)offs_bytes;
+  int32_t* d_offs = reinterpret_cast<int32_t*>(arena + P.total + align_up(P.slot_row.size() * sizeof(int16_t), 256));
   BM_CUDA(cudaMemcpyAsync(arena + P.table_off, P.experts.data(), sizeof(FastExpert) * P.experts.size(), cudaMemcpyHostToDevice, st));
   BM_CUDA(cudaMemcpyAsync(d_rows, P.slot_row.data(), P.slot_row.size() * sizeof(int16_t), cudaMemcpyHostToDevice, st));
   BM_CUDA(cudaMemcpyAsync(d_offs, P.slot_row_off.data(), P.slot_row_off.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));

@@ -110,7 +110,6 @@ struct FastExpert {
 struct TokTabHead {
   FastExpert fe;
   int32_t loose;            // gate or up has slots that no rank's position names: without a row, or with a rank that another slot has too
-  int32_t all_ranks;        // every rank of rank_accum has a down slot
   uint32_t broken[2][4];    // gate, up: octets of ranks that are not one 16-byte piece of the operand row (bit per octet)
 };
 constexpr int TOKTAB_MAX_RANK = 1024;
@@ -136,19 +135,12 @@ struct FastPlan {
   std::vector<int16_t> slot_row;      // concatenated per (expert, matrix): slot -> local row or -1
   std::vector<int32_t> slot_row_off;  // [E*3] element offset into slot_row
   size_t table_off = 0;               // FastExpert table
-  size_t tabs_off = 0;                // per-matrix rank/s/row tables
-  size_t units_off = 0;
   size_t toktab_off = 0;              // token-side tables (rank_in <= TOKTAB_MAX_RANK), 0 = none
   size_t total = 0;
   int max_unit_bytes = 0, max_slots = 0, max_words = 0;
 };
 
 __host__ __device__ inline int words_per_row(int bits) { return bits == 16 ? 16 : bits; }
-
-__host__ __device__ inline int code_offset(int bits) {
-  // u = q + offset for bits > 1; the 1-bit case is q = 2u - 1.
-  return bits == 1 ? 0 : (1 << (bits - 1));
-}
 
 inline bool supported_bits(int b) { return b == 1 || b == 2 || b == 3 || b == 4 || b == 6 || b == 8 || b == 16; }
 

@@ -35,7 +35,6 @@ constexpr int DEC_CONSUMERS = 256;
 constexpr int DEC_MAX_E = 1024;
 constexpr int DEC_MAX_MB = 4;                // 16-slot blocks of the down matrix per warp (8 warps: up to 512 slots)
 constexpr int DEC_MAX_RING = 12;
-constexpr int DEC_MIN_RING = 3;              // one tile
 constexpr int ZP_STRIDE = N_TILE + 32;       // halves; rows 64 bytes apart modulo 128: 16-byte operand loads of a quarter warp hit distinct banks
 
 // Rows g + 8 of every A fragment carry a factor 16 (fast_layout.cuh): accumulator registers 2 and 3 are scaled back
@@ -731,8 +730,6 @@ int plan_experts_decode(bm_layer* L) {
   L->dec_ok = true;
   return BM_OK;
 }
-
-bool experts_decode_fits(const bm_layer* L) { return L->dec_ok; }
 
 int launch_experts_decode(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
                           const int32_t* expert_offsets, const float* route_w, int T, int num_assign, float* rank_accum,

@@ -52,12 +52,7 @@ __device__ __forceinline__ void route_small_impl(const RouteSmallArgs& a, RouteS
     w[r] = 0.f;
     if (t < a.T) {
       warp_topk<REG>(a.logits, a.logits_dtype, t, a.E, a.k, a.renorm, a.weight_round, &idx[r], &w[r]);
-      if (lane >= a.k) idx[r] = -1;
-      else {
-        if (a.topk_idx) a.topk_idx[t * a.k + lane] = idx[r];
-        if (a.topk_w) a.topk_w[t * a.k + lane] = w[r];
-        if (static_cast<unsigned>(idx[r]) >= static_cast<unsigned>(a.E)) idx[r] = -1;
-      }
+      if (lane >= a.k || static_cast<unsigned>(idx[r]) >= static_cast<unsigned>(a.E)) idx[r] = -1;
     }
   }
   if constexpr (CL > 1) cg::this_cluster().barrier_wait(std::move(cleared));

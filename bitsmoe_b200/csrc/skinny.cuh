@@ -24,8 +24,6 @@ struct RouteSmallArgs {
   const void* logits;
   int logits_dtype;
   int T, E, k, renorm, weight_round;
-  int32_t* topk_idx;       // may be null
-  float* topk_w;           // may be null
   int32_t* token_indices;
   int32_t* expert_offsets;
   float* route_flat;
