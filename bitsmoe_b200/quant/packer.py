@@ -124,7 +124,6 @@ def quantize_rows(rows: Tensor, bits: int) -> Tuple[Tensor, Tensor]:
 
 def bucket_ranges(segments: Sequence[Tuple[int, Tuple[int, int]]], rank: int) -> List[Tuple[int, List[Tuple[int, int]]]]:
     """Row ranges per bit width, widest bucket first, ranges by ascending start; 0-bit rows are dropped."""
-    taken: List[Tuple[int, int]] = []
     by_bits: Dict[int, List[Tuple[int, int]]] = {}
     for bits, (s, e) in segments:
         bits, s, e = int(bits), int(s), int(e)
@@ -134,10 +133,12 @@ def bucket_ranges(segments: Sequence[Tuple[int, Tuple[int, int]]], rank: int) ->
             raise ValueError(f"Invalid segment range (s={s}, e={e}) for rank={rank}")
         if s == e:
             continue
-        if any(s < b and a < e for a, b in taken):
-            raise ValueError(f"Overlapping segments in range [{s}, {e})")
-        taken.append((s, e))
         by_bits.setdefault(bits, []).append((s, e))
+    # in ascending order two ranges overlap only if two neighbours do
+    taken = sorted(r for ranges in by_bits.values() for r in ranges)
+    for (_, end), (s, e) in zip(taken, taken[1:]):
+        if s < end:
+            raise ValueError(f"Overlapping segments in range [{s}, {e})")
     return [(bits, sorted(by_bits[bits])) for bits in sorted(by_bits, reverse=True) if bits != 0]
 
 

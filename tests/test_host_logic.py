@@ -67,6 +67,19 @@ def test_pack_single_weight_writes_checkpoint_schema():
         ppacker.pack_single_weight({0: {3: {"gate_proj": gate}}}, [(2, (0, 30)), (3, (20, 40))], sd, 0, 3, "gate_proj")
 
 
+def test_bucket_ranges_orders_and_rejects_overlaps():
+    ranges = [(i % 3 + 1, (5 * i, 5 * i + 4)) for i in range(20000)]
+    got = ppacker.bucket_ranges(ranges[::-1], 100000)
+    assert [b for b, _ in got] == [3, 2, 1]
+    assert got[0][1] == [r for b, r in ranges if b == 3]
+    assert ppacker.bucket_ranges([(2, (0, 8)), (0, (8, 12)), (4, (12, 20)), (4, (3, 3))], 20) == [(4, [(12, 20)]), (2, [(0, 8)])]
+    # neighbours, one inside the other with a third between their starts, equal ranges, a dropped range under a kept one
+    for bad in ([(2, (0, 8)), (3, (7, 9))], [(2, (0, 50)), (3, (50, 60)), (4, (10, 20))], [(2, (4, 8)), (3, (4, 8))], [(0, (0, 9)), (2, (8, 10))]):
+        for order in (bad, bad[::-1]):
+            with pytest.raises(ValueError, match="Overlapping"):
+                ppacker.bucket_ranges(order, 100)
+
+
 def test_oracle_forward_flavours_agree():
     layer = helpers.mixed_everything_layer()
     experts = helpers.decoded_experts(layer)
