@@ -174,7 +174,14 @@ struct GemmArgs {
   int a_dtype, c_dtype;
   int round_a_f16;       // round an fp32 A through fp16 first (rank_accum.half())
   int M, N, K;
+  int vec_a, vec_b;      // every A / B starts on a 16-byte boundary (filled in by the launcher)
 };
+
+// What 16-byte loads and tiled copies need of a base address (null counts as aligned).
+template <typename... P>
+inline bool aligned16(const P*... p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ...) & 15u) == 0;
+}
 
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 __host__ __device__ inline size_t align_up_c(size_t v, size_t a) { return (v + a - 1) / a * a; }

@@ -15,7 +15,7 @@ int launch_gemm_nt(const GemmArgs& g, int problems, cudaStream_t st);
 int dense_xwT(const void* X, int x_dtype, const __half* W0, const __half* W1, void* C0, void* C1, int c_dtype,
               const void* residual, int T, int N, int K, int problems, int* status, cudaStream_t st) {
   if (T == 0) return BM_OK;
-  const bool aligned = (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
+  const bool aligned = aligned16(X, W0, W1);
   if (T <= SKINNY_MAX_TOKENS && aligned && K % 8 == 0) {
     SkinnyArgs a{};
     a.n_seg = problems;

@@ -11,13 +11,19 @@ constexpr int G_BK = 32;
 constexpr int G_THREADS = 256;
 
 
-__device__ __forceinline__ void load8(const void* base, int dtype, int64_t idx, bool ok, int round_f16, float (&v)[8]) {
+__device__ __forceinline__ void load8(const void* base, int dtype, int64_t idx, bool ok, int vec, int round_f16, float (&v)[8]) {
   if (!ok) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = 0.f;
     return;
   }
-  if (dtype == BM_F32) {
+  if (!vec) {              // the base is off a 16-byte boundary
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      v[i] = load_act(base, dtype, idx + i);
+      if (dtype == BM_F32 && round_f16) v[i] = __half2float(__float2half_rn(v[i]));
+    }
+  } else if (dtype == BM_F32) {
     const float4 a = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + idx);
     const float4 b = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + idx + 4);
     v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
@@ -66,7 +72,7 @@ __global__ void __launch_bounds__(G_THREADS) gemm_nt_kernel(GemmArgs g) {
       const int r = v / (G_BK / 8), kc = (v % (G_BK / 8)) * 8;
       float f[8];
       const bool ok = (m0 + r < g.M) && (k0 + kc < g.K);
-      load8(A, g.a_dtype, static_cast<int64_t>(m0 + r) * g.K + k0 + kc, ok, g.round_a_f16, f);
+      load8(A, g.a_dtype, static_cast<int64_t>(m0 + r) * g.K + k0 + kc, ok, g.vec_a, g.round_a_f16, f);
 #pragma unroll
       for (int i = 0; i < 8; ++i) As[kc + i][r] = f[i];
     }
@@ -74,7 +80,7 @@ __global__ void __launch_bounds__(G_THREADS) gemm_nt_kernel(GemmArgs g) {
       const int r = v / (G_BK / 8), kc = (v % (G_BK / 8)) * 8;
       float f[8];
       const bool ok = (n0 + r < g.N) && (k0 + kc < g.K);
-      load8(B, BM_F16, static_cast<int64_t>(n0 + r) * g.K + k0 + kc, ok, 0, f);
+      load8(B, BM_F16, static_cast<int64_t>(n0 + r) * g.K + k0 + kc, ok, g.vec_b, 0, f);
 #pragma unroll
       for (int i = 0; i < 8; ++i) Bs[kc + i][r] = f[i];
     }
@@ -109,7 +115,10 @@ __global__ void __launch_bounds__(G_THREADS) gemm_nt_kernel(GemmArgs g) {
   }
 }
 
-int launch_gemm_nt(const GemmArgs& g, int problems, cudaStream_t st) {
+int launch_gemm_nt(const GemmArgs& args, int problems, cudaStream_t st) {
+  GemmArgs g = args;
+  g.vec_a = aligned16(g.A[0], g.A[1]);
+  g.vec_b = aligned16(g.B[0], g.B[1]);
   BM_REQUIRE(g.K % 8 == 0, BM_ERR_UNSUPPORTED, "gemm_nt: K=%d must be a multiple of 8", g.K);
   if (g.M == 0 || g.N == 0) return BM_OK;
   if (g.M <= 64) {

@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(GemmTcArgs a) {
 
 int launch_gemm_tc(const GemmTcArgs& a, int problems, cudaStream_t st) {
   BM_REQUIRE(a.K % TC_BK == 0, BM_ERR_UNSUPPORTED, "gemm_tc: K=%d must be a multiple of %d", a.K, TC_BK);
-  BM_REQUIRE((reinterpret_cast<uintptr_t>(a.X) & 15u) == 0, BM_ERR_UNSUPPORTED, "gemm_tc: activations must be 16-byte aligned");
+  BM_REQUIRE(aligned16(a.X, a.W[0], a.W[1]), BM_ERR_UNSUPPORTED, "gemm_tc: activations and weights must be 16-byte aligned");
   BM_REQUIRE(a.N % 8 == 0, BM_ERR_UNSUPPORTED, "gemm_tc: N=%d must be a multiple of 8", a.N);
   static PerDeviceOnce attr_once;
   int dev = -1;

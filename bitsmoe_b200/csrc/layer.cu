@@ -453,7 +453,7 @@ extern "C" int bm_basis_project(const bm_layer_t* L, const void* x, int x_dtype,
     const int rc = launch_skinny_nt(a, static_cast<cudaStream_t>(stream));
     if (rc != BM_ERR_UNSUPPORTED) return rc;       // shape does not tile (e.g. a very wide hidden size): the general GEMMs take it
   }
-  if (L->hidden % 64 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+  if (L->hidden % 64 == 0 && aligned16(x, L->vh_gate, L->vh_up)) {
     GemmTcArgs t{};
     t.X = x; t.W[0] = L->vh_gate; t.W[1] = L->vh_up; t.C[0] = h_gate; t.C[1] = h_up; t.residual = nullptr;
     t.M = T; t.N = L->rank_in; t.K = L->hidden; t.x_dtype = x_dtype; t.c_dtype = BM_F16; t.status = L->status_dev;
@@ -574,7 +574,7 @@ extern "C" int bm_combine_down_basis(const bm_layer_t* L, const float* rank_accu
     const int rc = combine_small(L, rank_accum, T, nullptr, 0, nullptr, nullptr, 0, residual, y, y_dtype, false, static_cast<cudaStream_t>(stream));
     if (rc != BM_ERR_UNSUPPORTED) return rc;
   }
-  if (L->rank_out % 64 == 0) {
+  if (L->rank_out % 64 == 0 && aligned16(rank_accum, L->u_down)) {
     GemmTcArgs t{};
     t.X = rank_accum; t.W[0] = t.W[1] = L->u_down; t.C[0] = t.C[1] = y; t.residual = residual;
     t.M = T; t.N = L->hidden; t.K = L->rank_out; t.x_dtype = BM_F32; t.c_dtype = y_dtype; t.status = L->status_dev;

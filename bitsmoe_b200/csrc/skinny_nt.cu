@@ -313,7 +313,7 @@ int skinny_splits(int rows, int K) {
 
 int launch_skinny_nt(SkinnyArgs a, cudaStream_t st) {
   BM_REQUIRE(a.N >= 1 && a.N <= SKINNY_MAX_TOKENS && a.n_seg >= 1 && a.n_seg <= SK_MAX_SEG && a.splits >= 1 && a.splits <= 8 &&
-                 (a.splits & (a.splits - 1)) == 0 && skinny_fits(a.K, a.K2, a.splits) && (reinterpret_cast<uintptr_t>(a.X) & 15u) == 0,
+                 (a.splits & (a.splits - 1)) == 0 && skinny_fits(a.K, a.K2, a.splits) && aligned16(a.X, a.W2, a.X2),
              BM_ERR_UNSUPPORTED, "skinny_nt: shape does not tile");
   const int mrows = sk_mrows(a.splits);
   a.row_tiles = 0;

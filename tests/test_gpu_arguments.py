@@ -115,3 +115,40 @@ def test_other_entries_refuse(env):
         with pytest.raises(RuntimeError):
             call()
     layer.check_status()
+
+
+def _shifted(t, by=1):
+    """The same values in a contiguous view that starts ``by`` elements off an aligned address."""
+    v = torch.empty(t.numel() + by, dtype=t.dtype, device=t.device)[by:].view(t.shape)
+    assert v.is_contiguous() and v.data_ptr() % 16
+    return v.copy_(t)
+
+
+# contiguous views may start anywhere: x, the basis, the router's and the shared expert's weights, each side of the batch size
+# at which the products change kernels
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("tokens", [5, 300])
+def test_products_take_views_at_any_address(env, tokens, dtype):
+    s, layer, gen = env["s"], env["layer"], torch.Generator(device=DEV).manual_seed(tokens)
+    x = torch.randn(tokens, H, generator=gen, device=DEV).to(dtype)
+    logits = torch.randn(tokens, E, generator=gen, device=DEV)
+    gate = (torch.randn(E, H, generator=gen, device=DEV) / 16).half()
+    sh = [(torch.randn(*d, generator=gen, device=DEV) / 16).half() for d in ((32, H), (32, H), (H, 32), (H,))]
+    moved = PackedLayer(s.tables["gate"], s.tables["up"], s.tables["down"], I, R, *(_shifted(b) for b in (s.vh_gate, s.vh_up, s.u_down)))
+    want = layer.forward(x, logits, K).cpu()
+    helpers.assert_close(layer.forward(_shifted(x, 3), logits, K).cpu(), want, what="x")
+    helpers.assert_close(moved.forward(x, logits, K).cpu(), want, what="basis")
+    res = x * 1e-4      # of the output's size
+    helpers.assert_close(moved.forward(x, logits, K, residual=_shifted(res), out=_shifted(x)).cpu(),
+                         layer.forward(x, logits, K, residual=res).cpu(), what="residual and out")
+    want = gate_logits(x, gate).cpu()
+    for a, b in ((_shifted(x), gate), (x, _shifted(gate, 5)), (_shifted(x.float()), gate)):
+        helpers.assert_close(gate_logits(a, b).cpu(), want, what="router")
+    want = dense_mlp(x, *sh).cpu()
+    for i in range(5):
+        args = [_shifted(t, 2 * i + 1) if j == i else t for j, t in enumerate([x, *sh])]
+        helpers.assert_close(dense_mlp(*args).cpu(), want, what=f"dense {i}")
+    y, lg = layer.block_forward(x, gate.to(dtype), K, True, None, tuple(t.to(dtype) for t in sh))
+    y2, lg2 = layer.block_forward(_shifted(x), gate.to(dtype), K, True, None, tuple(t.to(dtype) for t in sh))
+    helpers.assert_close(lg2.cpu(), lg.cpu(), what="block logits")
+    helpers.assert_close(y2.cpu(), y.cpu(), what="block")
