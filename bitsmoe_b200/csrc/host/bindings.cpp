@@ -64,17 +64,26 @@ struct HostLayer {
   bm_layer_t* handle = nullptr;
   c10::Device device{c10::kCUDA, 0};
   int64_t hidden = 0, rank_in = 0, rank_out = 0, experts = 0;      // hidden 0: the layer has no basis matrices
-  struct Ws { int64_t T, k, variant; at::Tensor buf; };
+  struct Ws { int64_t T, k, variant; at::Tensor buf; c10::cuda::CUDAStream stream; };
   std::vector<Ws> ws;
 
+  // A buffer may be dropped here while calls of another stream than the one it was made on still use it: the allocator
+  // learns of every such stream.
   const at::Tensor& workspace(int64_t T, int64_t k, int64_t variant, size_t need_if_new(const HostLayer&, int64_t, int64_t, const void*),
                               const void* arg) {
-    for (const Ws& w : ws)
-      if (w.T == T && w.k == k && w.variant == variant) return w.buf;
+    const c10::cuda::CUDAStream now = c10::cuda::getCurrentCUDAStream(device.index());
+    for (Ws& w : ws)
+      if (w.T == T && w.k == k && w.variant == variant) {
+        if (w.stream != now) {
+          w.buf.record_stream(now.unwrap());
+          w.stream = now;
+        }
+        return w.buf;
+      }
     const size_t need = need_if_new(*this, T, k, arg);
     at::Tensor buf = at::empty({static_cast<int64_t>(need < 256 ? 256 : need)}, at::TensorOptions().dtype(at::kByte).device(device));
     if (ws.size() > 8) ws.clear();
-    ws.push_back(Ws{T, k, variant, buf});
+    ws.push_back(Ws{T, k, variant, buf, now});
     return ws.back().buf;
   }
 };

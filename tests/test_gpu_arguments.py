@@ -117,6 +117,29 @@ def test_other_entries_refuse(env):
     layer.check_status()
 
 
+def test_dropped_workspace_waits_for_the_streams_that_use_it(env):
+    """A workspace made on one stream, used on another and dropped there (a layer keeps the last few shapes) must not be
+    handed out again while that use is still to come."""
+    layer = synth.to_packed_layer(env["s"])
+    xs = {t: env["x"].repeat(50, 1)[:t] for t in range(200, 212)}
+    lg = {t: env["logits"].repeat(50, 1)[:t] for t in xs}
+    ws = layer.workspace(200, K)
+    at, size = ws.data_ptr(), ws.numel()
+    del ws
+    side, awake = torch.cuda.Stream(), torch.cuda.Event()
+    with torch.cuda.stream(side):
+        env["layer"].forward(xs[200], lg[200], K)      # kernels loaded, this stream's pool filled
+        torch.cuda.synchronize()
+        torch.cuda._sleep(1_000_000_000)
+        awake.record()
+        for t in xs:
+            layer.forward(xs[t], lg[t], K)      # the first uses the buffer, a later one drops it
+    taken = [torch.empty(size, dtype=torch.uint8, device=DEV) for _ in range(4)]
+    assert not awake.query(), "the side stream should still sleep"
+    assert at not in [t.data_ptr() for t in taken]
+    torch.cuda.synchronize()
+
+
 def _shifted(t, by=1):
     """The same values in a contiguous view that starts ``by`` elements off an aligned address."""
     v = torch.empty(t.numel() + by, dtype=t.dtype, device=t.device)[by:].view(t.shape)
