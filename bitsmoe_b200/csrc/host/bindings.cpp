@@ -6,6 +6,7 @@
 // The semantics are those of bitsmoe_b200/layer.py, which calls these functions.
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ATen.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -68,12 +69,13 @@ struct HostLayer {
   std::vector<Ws> ws;
 
   // A buffer may be dropped here while calls of another stream than the one it was made on still use it: the allocator
-  // learns of every such stream.
-  const at::Tensor& workspace(int64_t T, int64_t k, int64_t variant, size_t need_if_new(const HostLayer&, int64_t, int64_t, const void*),
-                              const void* arg) {
+  // learns of every such stream.  A captured call gets one of its own from the graph's pool: the graph uses it as long as it
+  // lives, whatever is dropped here.
+  at::Tensor workspace(int64_t T, int64_t k, int64_t variant, size_t need_if_new(const HostLayer&, int64_t, int64_t, const void*), const void* arg) {
     const c10::cuda::CUDAStream now = c10::cuda::getCurrentCUDAStream(device.index());
+    const bool captured = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
     for (Ws& w : ws)
-      if (w.T == T && w.k == k && w.variant == variant) {
+      if (!captured && w.T == T && w.k == k && w.variant == variant) {
         if (w.stream != now) {
           w.buf.record_stream(now.unwrap());
           w.stream = now;
@@ -82,9 +84,10 @@ struct HostLayer {
       }
     const size_t need = need_if_new(*this, T, k, arg);
     at::Tensor buf = at::empty({static_cast<int64_t>(need < 256 ? 256 : need)}, at::TensorOptions().dtype(at::kByte).device(device));
+    if (captured) return buf;
     if (ws.size() > 8) ws.clear();
     ws.push_back(Ws{T, k, variant, buf, now});
-    return ws.back().buf;
+    return buf;
   }
 };
 
@@ -195,7 +198,7 @@ PyObject* layer_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const c10::cuda::CUDAGuard guard(L->device);
     const at::Tensor y = out.defined() ? out : at::empty_like(x);
     if (residual.defined()) residual = contiguous(residual.scalar_type() == x.scalar_type() ? residual : residual.to(x.scalar_type()));
-    const at::Tensor& ws = L->workspace(T, k, 0, layer_ws_need, nullptr);
+    const at::Tensor ws = L->workspace(T, k, 0, layer_ws_need, nullptr);
     check(bm_layer_forward(L->handle, x.data_ptr(), xd, logits.data_ptr(), ld, static_cast<int32_t>(T), static_cast<int32_t>(logits.size(1)), k,
                            integer(a[4]) != 0, static_cast<int32_t>(integer(a[5])), static_cast<const int32_t*>(ptr(g2l)), ptr(residual),
                            y.data_ptr(), static_cast<int32_t>(integer(a[8])), ws.data_ptr(), ws.nbytes(), stream_of(L->device)));
@@ -250,7 +253,7 @@ PyObject* block_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor y = at::empty_like(x), logits = at::empty({T, E}, x.options());
     const BlockNeed need{&d, static_cast<int32_t>(E)};
     const int64_t variant = 1 + 2 * d.sh_intermediate + (d.w_dtype == BM_BF16);
-    const at::Tensor& ws = L->workspace(T, k, variant, block_ws_need, &need);
+    const at::Tensor ws = L->workspace(T, k, variant, block_ws_need, &need);
     check(bm_block_forward(L->handle, &d, x.data_ptr(), dtype_code(x.scalar_type()), static_cast<int32_t>(T), static_cast<int32_t>(E), k,
                            integer(a[8]) != 0, static_cast<int32_t>(integer(a[9])), static_cast<const int32_t*>(ptr(g2l)), logits.data_ptr(),
                            y.data_ptr(), ws.data_ptr(), ws.nbytes(), stream_of(L->device)));

@@ -140,6 +140,26 @@ def test_dropped_workspace_waits_for_the_streams_that_use_it(env):
     torch.cuda.synchronize()
 
 
+def test_captured_call_keeps_its_workspace(env):
+    """A graph replays on the buffers that it was captured with; shapes met later must not free one of them."""
+    layer = synth.to_packed_layer(env["s"])
+    x, lg = env["x"].repeat(50, 1), env["logits"].repeat(50, 1)
+    want = layer.forward(x[:200], lg[:200], K)
+    size = layer.workspace(200, K).numel()
+    y, graph = torch.empty_like(want), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        layer.forward(x[:200], lg[:200], K, out=y)
+    for t in range(201, 212):
+        layer.forward(x[:t], lg[:t], K)
+    torch.cuda.synchronize()
+    others = [torch.full((size,), 7, dtype=torch.uint8, device=DEV) for _ in range(12)]
+    for _ in range(2):
+        y.zero_()
+        graph.replay()
+    helpers.assert_close(y.cpu(), want.cpu(), what="replay")
+    assert all(bool(t.eq(7).all()) for t in others), "the graph wrote into memory of other tensors"
+
+
 def _shifted(t, by=1):
     """The same values in a contiguous view that starts ``by`` elements off an aligned address."""
     v = torch.empty(t.numel() + by, dtype=t.dtype, device=t.device)[by:].view(t.shape)
