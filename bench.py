@@ -352,7 +352,7 @@ def probe(args):
 def init_dist(dev, world):
     if world > 1:
         import torch.distributed as dist
-        os.environ.setdefault("NCCL_NVLS_ENABLE", "0")     # plain peer traffic: no multicast objects on this pool
+        os.environ.setdefault("NCCL_NVLS_ENABLE", "0")     # plain peer traffic, no multicast objects
         dist.init_process_group("nccl", device_id=dev)
 
 
@@ -528,7 +528,7 @@ def decode_arm(args):
                 gstep(i)
             gms = timed(gstep, args.steps, sync) / args.steps
             extra[f"decode_{T}_with_router_linear"] = {"tokens": T, "ms_per_step": gms, "tokens_per_s": T / (gms * 1e-3),
-                                                       "note": "router logits computed inside the step (bm_gate_logits), then the same five launches"}
+                                                       "note": "router logits computed inside the step (bm_gate_logits, one launch), then the layer's three launches"}
         except Exception as ex:
             extra["router_linear_error"] = repr(ex)
         # the kernels to beat: the reference's own CUDA op, recompiled for sm_100a, at the op boundary on the same inputs
@@ -746,7 +746,7 @@ def ep_arm(args):
 
 # ------------------------------------------------------------------------------------------- stack workload
 def stack_arm(args):
-    """One decode step of a 48-layer stack (BASELINE.json configs[4]): per layer RMSNorm -> attention over a 2048-token
+    """One decode step of a 48-layer stack: per layer RMSNorm -> attention over a 2048-token
     KV cache (bf16 torch: library GEMMs and scaled_dot_product_attention) -> RMSNorm -> this library's MoE block
     (router Linear, routing, packed experts, down basis), expert-parallel over the ranks.  Weights are seeded random."""
     from bitsmoe_b200 import capi, ep, synth

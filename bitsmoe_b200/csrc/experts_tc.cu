@@ -27,10 +27,14 @@
 // The roles walk the items on their own barriers, so an item's staging runs beside the last products and sums of the one
 // before.
 //
-// What bounds it: the converters -- 5.3 K cycles per chunk of 64 columns at 256 slots (about 44 instructions for each pair
-// of 16 x 16 blocks), against 2.1 K of tensor pipe.  8192 tokens of 128 experts (rank 256, intermediate 768): 363 -> 179 us
-// over the transposed, single-role-loop form; 16384 tokens of 512 experts 653 -> 320 us.  Two CTAs that share the
-// converted weights through the cluster's shared memory took longer (257 us): five slots of ring do not cover the way over.
+// What bounds it: the chain of a converter warp, no pipe.  Clocks of every role at 8192 tokens of 128 experts (rank 256,
+// intermediate 768): a stage takes a converter warp 3.1 K cycles, of which about 1000 convert, 600 issue the next stage's
+// loads (addresses included), 200 fence and publish, 140 wait for load results and 570 for a free slot of the ring (four
+// per pipeline beside a 128-token operand), the rest bookkeeping; staging is 10 % of its time.  A chunk of 64 columns takes 7.0 K cycles all in, of
+// which its products need 2.05 K of tensor pipe; the MMA issuers wait for weights a quarter of theirs.  Counters at 2048
+// tokens: issue slots 45 % busy, tensor pipe 22 %, ALU 31 %.  The stage takes 179 us at 8192 tokens (363 in the transposed
+// form with one loop for all roles), 320 us at 16384 tokens of 512 experts (653).  Two CTAs that share the converted weights
+// through the cluster's shared memory took longer (257 us): the ring does not cover the way over.
 //
 // The down product of a chunk is issued one chunk late (G0 U0 | G1 U1 D0 | G2 U2 D1 | ...).  Every mbarrier wait is
 // bounded in time.  One that gives up raises a flag of the CTA; the roles then leave at their next wait that is not over, the
@@ -44,8 +48,8 @@ constexpr int XT_NT_MAX = 128;            // most tokens (assignments) per item:
 constexpr int XT_THREADS = 768;
 constexpr int XT_EPI_WARPS = 8, XT_DQ_WARP0 = 8, XT_DQ_WARPS = 12, XT_LOOKUP_WARP = 20, XT_MMA_WARP0 = 21;
 constexpr int XT_TEAM = XT_DQ_WARPS / 2;  // converter warps per pipeline
-// Registers per thread at launch and per role afterwards.  The converters keep two stages' words and four independent
-// blocks in flight; at the launch's 96 they spilled, and a spilled load result stalls its warp for the load's latency.
+// Registers per thread at launch (what 768 threads leave) and per role afterwards: the converters, which keep two stages'
+// words and four independent blocks in flight, take what the roles with little state give back.
 constexpr int XT_REGS = 80, XT_REGS_EPI = 80, XT_REGS_DQ = 88, XT_REGS_MISC = 56;
 static_assert(32 * (XT_EPI_WARPS * XT_REGS_EPI + XT_DQ_WARPS * XT_REGS_DQ + 4 * XT_REGS_MISC) <= XT_THREADS * XT_REGS,
               "the roles' registers come out of the launch's");
@@ -128,8 +132,8 @@ __device__ __forceinline__ bool xt_wait(uint64_t* bar, uint32_t parity, volatile
 // (q * scale): r[0] = row g, k (2t, 2t+1); r[1] = row g+8, same k; r[2] = row g, k (2t+8, 2t+9); r[3] = row g+8.
 // The code sits in the mantissa of 1024 (fields at bit 0) or of 64 (fields at bit 4); subtracting
 // 1024 + offset or 64 + offset is exact, the multiplication by the scale rounds once, as fp16(q * scale) does.
-// The exponents 1024 and 64 as fp16 pairs, in registers: the compiler knows only that they are values, so (w & mask) | k
-// stays one instruction with one immediate (as constants they were loaded again for each use: 8192 tokens 185 -> 179 us).
+// The exponents 1024 and 64 as fp16 pairs, held in registers as opaque values, so that (w & mask) | k needs one immediate
+// operand only (8192 tokens 185 -> 179 us against constants).
 struct XtMagic {
   uint32_t lo, hi;
   __device__ __forceinline__ XtMagic() {
@@ -175,8 +179,8 @@ __device__ __forceinline__ void dequant_pair_store(const XtMagic& k, uint32_t wo
   *reinterpret_cast<uint4*>(dst + 128) = make_uint4(r0[1], r0[3], r1[1], r1[3]);
 }
 
-// silu(g) * u with the hardware's exponential and reciprocal; flushing a subnormal exponential to zero does not reach the
-// sum 1 + e, and leaves out the rescaling around both instructions
+// silu(g) * u = g * u / (1 + e^-g), with e^-g as 2^(-g log2 e); where that power is subnormal and flushed to zero it could not
+// have changed the sum 1 + e^-g
 __device__ __forceinline__ float silu_mul(float g, float u) {
   float e, r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * g));
