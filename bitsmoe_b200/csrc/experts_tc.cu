@@ -1,50 +1,51 @@
 // Packed routed-expert forward for large token counts (prefill): fused mixed-bit grouped GEMM on the
-// 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory).
+// 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory), a pair of CTAs per work item.
 //
-// Work item = (expert, block of up to NT of its assignments; NT = 128 where it fits).  One persistent CTA per SM walks
-// the items.  The item's tokens are the 128 rows (M) of every product and the weights its columns (N); the tile's columns
-// are taken 64 at a time ("chunk"):
-//   gate/up:  D_g[n, c] = sum_slot act_g[n, slot] * W_g[c, slot]     (N = 64 columns c, K = row slots)
-//   down:     D_d[n, slot] += sum_c z[n, c] * W_d[slot, c]           (N = 128 row slots x 1..3, K = 64 columns c)
-// Tokens as rows make the epilogue cheap: a thread owns a token, so eight z values leave as one 16-byte store in the
-// order the down product reads them (the transposed orientation stored every z on its own, two bytes at a time), and 128
-// tokens share one conversion of the weights.  64 columns at a time leave room in tensor memory for two gate/up
-// accumulator pairs (2 x 128 columns) beside the down accumulator (256), so the products of a chunk run while the
-// previous one is turned into z.
+// Work item = (expert, block of up to 2 NT of its assignments; NT = 128 where it fits).  A persistent pair of CTAs (cluster of
+// two, cta_group::2) walks the items; each CTA holds half of the item's tokens as 128 rows (M) of every product and converts
+// half of the weights, its columns (N); the tensor cores read both halves, so the converted weights never cross the cluster.
+// The tile's columns are taken 64 at a time ("chunk"):
+//   gate/up:  D_g[n, c] = sum_slot act_g[n, slot] * W_g[c, slot]     (N = 64 columns c, 32 from each CTA; K = row slots)
+//   down:     D_d[n, slot] += sum_c z[n, c] * W_d[slot, c]           (N = 128 row slots x 1..3, 64 from each CTA; K = 64 columns c)
+// Tokens as rows make the epilogue cheap: a thread owns a token.  z goes back to tensor memory, over the gate sums it came
+// from, and is the A operand of the down product there.  64 columns at a time leave room in tensor memory for two gate/up
+// accumulator pairs (2 x 128 columns) beside the down accumulator (256), so the products of a chunk run while the previous
+// one is turned into z.
 //
 // Warp roles (768 threads; the last warp completes the last warpgroup):
-//   warps 0-7   epilogue (two per TMEM lane quarter, 32 columns each): tcgen05.ld D_g/D_u -> z = silu(g)*u -> fp16 z
-//               operand in shared memory; at the end of the item D_d * s * route weight is turned through the idle z area
-//               and added to rank_accum in 16-byte vector reductions, beside the next item's staging.
+//   warps 0-7   epilogue (two per TMEM lane quarter, 32 columns each): tcgen05.ld D_g/D_u -> z = silu(g)*u -> fp16, tcgen05.st;
+//               at the end of the item D_d * s * route weight is turned through shared memory and added to rank_accum in
+//               16-byte vector reductions, beside the next item's staging.
 //   warps 8-19  converters, one team of six warps per pipeline: arena words (nibble / dense 2-bit codes), read straight
-//               from L2 one stage ahead into registers, -> fp16 (q * scale) operand stages of 64 rows x 32 positions in the
+//               from L2 one stage ahead into registers, -> fp16 (q * scale) operand stages of 2048 codes in the
 //               canonical K-major core-matrix layout, a ring of two-stage slots per pipeline, a stage per warp.  Before an
 //               item's stages they build its activation operand act[n, slot] = fp16(h[token, rank(slot)] * s(slot)).
 //   warp  20    looks up the next item while the current one runs and asks L2 for its weights
-//   warps 21,22 MMA issue, one thread each: gate products and the down product's even slot tiles; up products and the odd
-//               ones.  The waits and commits of one pipeline hide behind the products of the other, and they never write
-//               the same accumulator.
+//   warps 21,22 (of the even CTA) MMA issue for both CTAs, one thread each: gate products and the down product's even slot
+//               tiles; up products and the odd ones.  The waits and commits of one pipeline hide behind the products of the
+//               other, and they never write the same accumulator.
 // The roles walk the items on their own barriers, so an item's staging runs beside the last products and sums of the one
-// before.
+// before.  What an MMA issuer waits for is signalled by both CTAs (mapped arrivals on the even CTA's barriers), what waits for
+// MMAs is signalled in both by the commit.
 //
-// What bounds it: the chain of a converter warp, no pipe.  Clocks of every role at 8192 tokens of 128 experts (rank 256,
-// intermediate 768): a stage takes a converter warp 3.1 K cycles, of which about 1000 convert, 600 issue the next stage's
-// loads (addresses included), 200 fence and publish, 140 wait for load results and 570 for a free slot of the ring (four
-// per pipeline beside a 128-token operand), the rest bookkeeping; staging is 10 % of its time.  A chunk of 64 columns takes 7.0 K cycles all in, of
-// which its products need 2.05 K of tensor pipe; the MMA issuers wait for weights a quarter of theirs.  Counters at 2048
-// tokens: issue slots 45 % busy, tensor pipe 22 %, ALU 31 %.  The stage takes 179 us at 8192 tokens (363 in the transposed
-// form with one loop for all roles), 320 us at 16384 tokens of 512 experts (653).  Two CTAs that share the converted weights
-// through the cluster's shared memory took longer (257 us): the ring does not cover the way over.
+// What bounds it: shared-memory bandwidth.  Every MMA of the gate and up products reads 4 KB of activations for 64 columns;
+// with the weights it is about 210 KB a chunk, and 48 KB of converted weights are stored, 2.0 K cycles at 128 bytes a cycle;
+// a chunk takes 2.4 K where an item has few tokens and 3.6 K at 128 rows a CTA, where epilogue and sums work beside it.
+// Converting in pairs halves the conversions per token, which set the pace before (7.0 K cycles a chunk of 128 tokens).
+// Stage of 8192 tokens of 128 experts (rank 256, intermediate 768): 176 -> 121 us; 2048 tokens 72 -> 61, 777 tokens 59 -> 52;
+// 16384 tokens of 512 experts 318 -> 238, 1200 of them (a dozen tokens a CTA and item) 114 -> 115.
+// The mapped arrivals carry no cluster-scope release: what they publish is read by the tensor cores of the CTA that wrote it
+// (behind the proxy fence); with the release a converter's arrival took 1.4 K cycles and the stage 165 us.
 //
 // The down product of a chunk is issued one chunk late (G0 U0 | G1 U1 D0 | G2 U2 D1 | ...).  Every mbarrier wait is
-// bounded in time.  One that gives up raises a flag of the CTA; the roles then leave at their next wait that is not over, the
-// look-up warp behind its copy and the MMA issuers behind their MMAs, and tensor memory is given back after that.
+// bounded in time.  One that gives up raises a flag in both CTAs; the roles then leave at their next wait that is not over, the
+// look-up warp behind its copy, both CTAs behind the MMAs issued so far, and tensor memory is given back after that.
 #include "fast_layout.cuh"
 #include "tc05.cuh"
 
 namespace bm {
 
-constexpr int XT_NT_MAX = 128;            // most tokens (assignments) per item: the rows of one MMA
+constexpr int XT_NT_MAX = 128;            // most tokens (assignments) of an item in a CTA: its rows of one MMA
 constexpr int XT_THREADS = 768;
 constexpr int XT_EPI_WARPS = 8, XT_DQ_WARP0 = 8, XT_DQ_WARPS = 12, XT_LOOKUP_WARP = 20, XT_MMA_WARP0 = 21;
 constexpr int XT_TEAM = XT_DQ_WARPS / 2;  // converter warps per pipeline
@@ -54,16 +55,15 @@ constexpr int XT_REGS = 80, XT_REGS_EPI = 80, XT_REGS_DQ = 88, XT_REGS_MISC = 56
 static_assert(32 * (XT_EPI_WARPS * XT_REGS_EPI + XT_DQ_WARPS * XT_REGS_DQ + 4 * XT_REGS_MISC) <= XT_THREADS * XT_REGS,
               "the roles' registers come out of the launch's");
 constexpr int XT_CHUNK = 64;              // tile columns per step
-constexpr int XT_RING_MAX = 5;            // operand slots per pipeline (at most), two stages each
-// A weight stage: 64 operand rows (columns of the chunk, or slots) x 32 contraction positions; bytes between its
-// 8-position chunks (padded: conflict-free 16-byte stores)
-constexpr int XT_W_STRIDE = 64 * 16 + 32;
-constexpr int XT_STAGE_BYTES = 4 * XT_W_STRIDE;
-constexpr int XT_SLOT_BYTES = 2 * XT_STAGE_BYTES;     // the MMA issuers take two stages per barrier
-constexpr int XT_D_STRIDE = 128 * 16 + 32;            // a slot of the down product: 128 rows x 32 positions
-static_assert(4 * XT_D_STRIDE <= XT_SLOT_BYTES, "a down slot fits");
-constexpr int XT_Z_STRIDE = 128 * 16 + 16;            // z operand: 128 rows x 64 positions
-constexpr int XT_Z_BYTES = (XT_CHUNK / 8) * XT_Z_STRIDE;
+constexpr int XT_RING_MAX = 8;            // operand slots per pipeline (at most; a power of two)
+// A weight slot: this CTA's half of the rows of one B operand, in two stages that two warps fill.
+//   gate/up  32 columns of the chunk x 128 row slots (four pairs of 16-slot blocks; a stage is two of them)
+//   down     64 slots of a 128-slot tile x the chunk's 64 columns (a stage is 32 of them)
+// Bytes between 8-position chunks, padded: the 16-byte stores of a quarter warp hit distinct banks.
+constexpr int XT_G_STRIDE = 32 * 16 + 32, XT_D_STRIDE = 64 * 16 + 32;
+constexpr int XT_SLOT_BYTES = 16 * XT_G_STRIDE;
+static_assert(8 * XT_D_STRIDE <= XT_SLOT_BYTES, "a down slot fits");
+constexpr int XT_TURN_BYTES = 2048;       // where an epilogue warp turns its sums: 16 tokens x 32 slots
 // bytes between 8-position chunks of the token-side operands (padded: conflict-free stores)
 __host__ __device__ constexpr int xt_chunk_stride(int nt) { return nt * 16 + 16; }
 constexpr int XT_MAX_E = 1024;
@@ -72,23 +72,10 @@ struct XtBars {
   uint64_t w_full[2 * XT_RING_MAX], w_empty[2 * XT_RING_MAX];     // weight slots of the pipelines
   uint64_t item_full[2], item_free[2];    // an item's description and table are there / no role needs them any more
   uint64_t act_ready, act_free;           // activation operand written / every product with it complete
-  uint64_t gu_done[2], gu_free[2];        // gate/up accumulators of a chunk complete / read out
-  uint64_t z_ready, z_free;               // z operand of a chunk written / multiplied
+  uint64_t gu_done[2];                    // gate/up accumulators of a chunk complete
+  uint64_t z_ready[2], z_free[2];         // accumulators read out and z written over them / z multiplied
   uint64_t down_done, down_free;          // down sums of an item complete / read out
   uint64_t drained[2];                    // every MMA of the pipeline complete (at the end of the kernel)
-};
-
-// Position in a cyclic buffer of n slots with the phase bit of its mbarriers.
-struct XtCycle {
-  uint32_t i, ph;
-  __device__ __forceinline__ void next(uint32_t n) {
-    if (++i == n) { i = 0; ph ^= 1u; }
-  }
-  __device__ __forceinline__ void advance(uint32_t k, uint32_t n) {
-    const uint32_t to = i + k, wraps = to / n;
-    i = to - wraps * n;
-    ph ^= wraps & 1u;
-  }
 };
 
 struct XtItem {
@@ -98,7 +85,11 @@ struct XtItem {
   int pad_;
 };
 
-// abort_flag[0]: a wait of this CTA gave up; abort_flag[1]: the limit of a wait in microseconds
+// abort_flag[0]: a wait of this CTA or of its peer gave up; abort_flag[1]: the limit of a wait in microseconds
+__device__ __noinline__ void xt_give_up(volatile int* abort_flag) {
+  *abort_flag = 1;
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(tc::cluster_map(tc::smem_u32(const_cast<int*>(abort_flag)), tc::cluster_rank() ^ 1u)), "r"(1) : "memory");
+}
 __device__ __forceinline__ bool xt_wait_slow(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   const uint32_t addr = tc::smem_u32(bar);
   uint64_t t0 = 0;
@@ -114,7 +105,7 @@ __device__ __forceinline__ bool xt_wait_slow(uint64_t* bar, uint32_t parity, vol
     if ((i & 15u) == 15u) {
       const uint64_t now = tc::global_ns();
       if (t0 == 0) t0 = now;
-      else if (now - t0 > static_cast<uint64_t>(abort_flag[1]) * 1000u) { *abort_flag = 1; return false; }
+      else if (now - t0 > static_cast<uint64_t>(abort_flag[1]) * 1000u) { xt_give_up(abort_flag); return false; }
     }
   }
 }
@@ -167,14 +158,13 @@ __device__ __forceinline__ void dequant_block(const XtMagic& k, uint32_t w, __ha
   r[3] = *reinterpret_cast<const uint32_t*>(&o3);
 }
 
-// The two blocks of a pair -> the two 16-byte chunks (rows 16x+g and 16x+g+8) of K-chunk 4*pair_in_stage + t.
+// The two blocks of a pair -> the two 16-byte chunks (rows g and g + 8 of the block) of an 8-position chunk.
 // `word0` / `word1` are the pair's two blocks (dense: the same word, the second shifted by 8).
 template <bool DENSE>
-__device__ __forceinline__ void dequant_pair_store(const XtMagic& k, uint32_t word0, uint32_t word1, const __half2 (&sa)[4], const __half2 (&sb)[4],
-                                                   unsigned char* dst) {
+__device__ __forceinline__ void dequant_pair_store(const XtMagic& k, const uint2& w, const __half2 (&sa)[4], const __half2 (&sb)[4], unsigned char* dst) {
   uint32_t r0[4], r1[4];
-  dequant_block<DENSE>(k, word0, sa[0], sb[0], sa[1], sb[1], r0);
-  dequant_block<DENSE>(k, word1, sa[2], sb[2], sa[3], sb[3], r1);
+  dequant_block<DENSE>(k, w.x, sa[0], sb[0], sa[1], sb[1], r0);
+  dequant_block<DENSE>(k, DENSE ? w.x >> 8 : w.y, sa[2], sb[2], sa[3], sb[3], r1);
   *reinterpret_cast<uint4*>(dst) = make_uint4(r0[0], r0[2], r1[0], r1[2]);
   *reinterpret_cast<uint4*>(dst + 128) = make_uint4(r0[1], r0[3], r1[1], r1[3]);
 }
@@ -190,25 +180,24 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
 
 struct XtSmem {
   unsigned char* act;     // [2][nchunks][nt rows] canonical K-major, 16-byte chunks
-  unsigned char* z;       // [8 chunks][128 rows]; at the end of an item each epilogue warp's part turns the sums
-  unsigned char* ring;    // [2 pipelines][ring_h][XT_SLOT_BYTES]
+  unsigned char* turn;    // [8 epilogue warps][XT_TURN_BYTES]
+  unsigned char* ring;    // [2 pipelines][ring][XT_SLOT_BYTES]
   int* prefix;            // [E + 1] items before each expert
-  int* offset;            // [E + 1] assignments before each expert
   unsigned char* tab;     // [2 items] token-side table of the item's expert (TokTab)
 };
 
 __host__ __device__ inline size_t xt_act_bytes(int max_slots, int nt) { return static_cast<size_t>(2) * (max_slots / 8) * xt_chunk_stride(nt); }
-__host__ __device__ inline size_t xt_smem_bytes(int max_slots, int num_experts, int tab_bytes, int nt, int ring_h) {
-  size_t o = align_up_c(xt_act_bytes(max_slots, nt), 128) + XT_Z_BYTES;
-  o += static_cast<size_t>(2 * ring_h) * XT_SLOT_BYTES;
-  o += align_up_c(static_cast<size_t>(2 * num_experts + 2) * 4, 128);     // items and assignments before each expert
+__host__ __device__ inline size_t xt_smem_bytes(int max_slots, int num_experts, int tab_bytes, int nt, int ring) {
+  size_t o = align_up_c(xt_act_bytes(max_slots, nt), 128) + XT_EPI_WARPS * XT_TURN_BYTES;
+  o += static_cast<size_t>(2 * ring) * XT_SLOT_BYTES;
+  o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);     // items before each expert
   o += static_cast<size_t>(2) * tab_bytes;
   // the MMAs read 128 operand rows whatever nt is: rows past nt of the last chunk lie in what follows the operand
-  return o + 1024;                                                   // slack for the 1024-byte base alignment
+  return o;
 }
 
 // Units of work.  Items that fill whole rounds of the grid are units of their own; the items of the last, partial round
-// are cut along the tile columns so that the round's CTAs share them evenly (their down sums meet in rank_accum anyway).
+// are cut along the tile columns so that the round's pairs share them evenly (their down sums meet in rank_accum anyway).
 struct XtUnits {
   int full, split, per, n_units;
   __device__ __forceinline__ XtUnits(int n_items, int grid, int n_chunks) {
@@ -233,14 +222,14 @@ struct XtArgs {
   float* rank_accum;
   long long* acc64;
   int* status;
-  int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, ring_h, gu_bufs, tab_bytes;
+  int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, ring_log2, gu_bufs, tab_bytes;
   int wait_limit_us;
   int vec_add;            // every row of rank_accum starts on a 16-byte boundary (and takes fp32 adds)
 };
 
 // Locates unit `u` and copies what the roles need; one warp, an item ahead of the roles.
 __device__ __forceinline__ void xt_load_item(XtItem& item, unsigned char* tab, uint64_t* bar, int u, const XtUnits& units, int n_chunks,
-                                             const XtSmem& sm, const XtArgs& A, int lane) {
+                                             const XtSmem& sm, const XtArgs& A, int lane, int rank) {
   int it = u, chunk0 = 0, nchunk = n_chunks;
   if (u >= units.full) {
     const int r = u - units.full, part = r % units.split;
@@ -258,10 +247,12 @@ __device__ __forceinline__ void xt_load_item(XtItem& item, unsigned char* tab, u
     tc::mbar_expect_tx(bar, A.tab_bytes);
     tc::bulk_g2s(tab, A.toktab + static_cast<size_t>(e) * A.tab_bytes, A.tab_bytes, bar);
   }
-  // an expert's assignments are spread evenly over its items
-  const int begin = sm.offset[e], cnt = sm.offset[e + 1] - begin, parts = sm.prefix[e + 1] - sm.prefix[e], j = it - sm.prefix[e];
-  const int a0 = begin + static_cast<int>(static_cast<int64_t>(cnt) * j / parts);
-  const int n = begin + static_cast<int>(static_cast<int64_t>(cnt) * (j + 1) / parts) - a0;
+  // an expert's assignments are spread evenly over its items, an item's over the two CTAs
+  const int begin = A.expert_offsets[e], cnt = A.expert_offsets[e + 1] - begin, parts = sm.prefix[e + 1] - sm.prefix[e], j = it - sm.prefix[e];
+  int a0 = begin + static_cast<int>(static_cast<int64_t>(cnt) * j / parts);
+  const int both = begin + static_cast<int>(static_cast<int64_t>(cnt) * (j + 1) / parts) - a0, first = (both + 1) >> 1;
+  const int n = rank ? both - first : first;
+  a0 += rank ? first : 0;
   int tk[XT_NT_MAX / 32];
   float rw[XT_NT_MAX / 32];
 #pragma unroll
@@ -282,62 +273,59 @@ __device__ __forceinline__ void xt_load_item(XtItem& item, unsigned char* tab, u
 // One converter stage's words and scales, on their way from L2.
 struct XtPre {
   uint2 w[4];
-  uint4 s;
+  uint4 s[2];
 };
 
-
-__global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_constant__ XtArgs A) {
-  extern __shared__ unsigned char xt_raw[];
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_constant__ XtArgs A) {
+  extern __shared__ __align__(128) unsigned char xt_raw[];
   __shared__ __align__(8) XtBars bars;
   __shared__ XtItem items[2];             // this item and the next one (looked up while this one runs)
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag_s[2];
   volatile int* abort_flag = abort_flag_s;
   const int warp = tc::warp_index(), lane = threadIdx.x & 31;
-  const int nt = A.nt, ring_h = A.ring_h, h_rank = A.h_rank, num_experts = A.num_experts;
+  const int rank = static_cast<int>(tc::cluster_rank()), pair = static_cast<int>(blockIdx.x) >> 1, n_pairs = static_cast<int>(gridDim.x) >> 1;
+  const int nt = A.nt, ring = 1 << A.ring_log2, h_rank = A.h_rank, num_experts = A.num_experts;
   const int cs = xt_chunk_stride(nt);     // bytes between 8-position chunks of act
   const int n_chunks = A.n_tiles * (N_TILE / XT_CHUNK);
   const uint32_t act_m_bytes = static_cast<uint32_t>(A.max_slots / 8) * cs;
   const TokTab lay(h_rank, A.max_slots);
   XtSmem sm;
   {
-    unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(xt_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+    unsigned char* base = xt_raw;
     sm.act = base;
     size_t o = align_up_c(xt_act_bytes(A.max_slots, nt), 128);
-    sm.z = base + o; o += XT_Z_BYTES;
-    sm.ring = base + o; o += static_cast<size_t>(2 * ring_h) * XT_SLOT_BYTES;
+    sm.turn = base + o; o += XT_EPI_WARPS * XT_TURN_BYTES;
+    sm.ring = base + o; o += static_cast<size_t>(2 * ring) * XT_SLOT_BYTES;
     sm.prefix = reinterpret_cast<int*>(base + o);
-    sm.offset = sm.prefix + num_experts + 1;
-    o += align_up_c(static_cast<size_t>(2 * num_experts + 2) * 4, 128);
+    o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);
     sm.tab = base + o;
   }
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2 * XT_RING_MAX; ++i) { tc::mbar_init(&bars.w_full[i], 2); tc::mbar_init(&bars.w_empty[i], 1); }
-    tc::mbar_init(&bars.act_ready, XT_DQ_WARPS);
+    // what the MMA issuers (of the even CTA) wait for is signalled by both CTAs, what waits for MMAs by their commits
+    for (int i = 0; i < 2 * XT_RING_MAX; ++i) { tc::mbar_init(&bars.w_full[i], 4); tc::mbar_init(&bars.w_empty[i], 1); }
+    tc::mbar_init(&bars.act_ready, 2 * XT_DQ_WARPS);
     tc::mbar_init(&bars.act_free, 2);
     tc::mbar_init(&bars.down_done, 2);
-    tc::mbar_init(&bars.down_free, XT_EPI_WARPS);
-    tc::mbar_init(&bars.z_ready, XT_EPI_WARPS);
-    tc::mbar_init(&bars.z_free, 2);
+    tc::mbar_init(&bars.down_free, 2 * XT_EPI_WARPS);
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&bars.item_full[i], 2);
-      tc::mbar_init(&bars.item_free[i], XT_EPI_WARPS + XT_DQ_WARPS + 2);
+      tc::mbar_init(&bars.item_free[i], XT_EPI_WARPS + XT_DQ_WARPS + (rank == 0 ? 2 : 0));
       tc::mbar_init(&bars.gu_done[i], 2);
-      tc::mbar_init(&bars.gu_free[i], XT_EPI_WARPS);
+      tc::mbar_init(&bars.z_ready[i], 2 * XT_EPI_WARPS);
+      tc::mbar_init(&bars.z_free[i], 2);
       tc::mbar_init(&bars.drained[i], 1);
     }
     tc::mbar_init_fence();
     abort_flag_s[0] = A.wait_limit_us == 0;
     abort_flag_s[1] = A.wait_limit_us;
   }
-  if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
-  // items before each expert (an item = up to nt consecutive assignments of one expert): every thread loads
+  tc::cluster_arrive();
+  // items before each expert (an item = up to 2 nt consecutive assignments of one expert): every thread loads
   // its experts' counts in parallel, one warp then scans them
   for (int e = threadIdx.x; e < num_experts; e += XT_THREADS) {
     const int o0 = A.expert_offsets[e], o1 = A.expert_offsets[e + 1];
-    sm.prefix[e + 1] = (o1 - o0 + nt - 1) / nt;
-    sm.offset[e + 1] = o1;
-    if (e == 0) sm.offset[0] = o0;
+    sm.prefix[e + 1] = (o1 - o0 + 2 * nt - 1) / (2 * nt);
   }
   __syncthreads();
   if (warp == 1) {
@@ -355,11 +343,15 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     }
     if (lane == 0) sm.prefix[0] = 0;
   }
+  tc::cluster_wait();                     // both CTAs run and their barriers are set up
+  if (warp == 0) tc::tmem_alloc_pair(&tmem_slot, 512);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
-  const XtUnits units(sm.prefix[num_experts], static_cast<int>(gridDim.x), n_chunks);
+  const XtUnits units(sm.prefix[num_experts], n_pairs, n_chunks);
+  const uint32_t lead_bars = tc::cluster_map(tc::smem_u32(&bars), 0);      // the barriers of the CTA that issues the MMAs
+  auto lead = [&](const uint64_t* bar) { return lead_bars + static_cast<uint32_t>(reinterpret_cast<const char*>(bar) - reinterpret_cast<const char*>(&bars)); };
   // tensor memory: gu_bufs x (gate 64 columns, up 64 columns), then the down product's slot tiles of 128 columns
   const uint32_t d_down = tmem_base + A.gu_bufs * 2 * XT_CHUNK;
   // the down product of a chunk is issued `lag` chunks late: one where tensor memory holds two gate/up accumulator pairs
@@ -382,11 +374,10 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XT_REGS_EPI));
     // -------------------------------------------------------------------- epilogue
     // warp = (TMEM lane quarter q: tokens 32 q .. 32 q + 31, half of the chunk's 64 columns); a thread owns a token.
-    // Its part of the z operand -- four chunks of 32 rows -- is written and reused by this warp alone.
     const int q = warp & 3, half = warp >> 2, n = 32 * q + lane;
     const uint32_t lane_sel = static_cast<uint32_t>(32 * q) << 16;
-    unsigned char* zpart = sm.z + 4 * half * XT_Z_STRIDE + 32 * q * 16;
-    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++round) {
+    unsigned char* turn = sm.turn + warp * XT_TURN_BYTES;
+    for (int u = pair; u < units.n_units; u += n_pairs, ++round) {
       XT_ITEM_BEGIN
       const int n_tok = item.n;
       const bool busy = 32 * q < n_tok;                               // any token in this quarter
@@ -396,8 +387,8 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         ok = xt_wait(&bars.gu_done[b], (lag ? g >> 1 : g) & 1u, abort_flag);
         if (!ok) break;
         tc::fence_after_sync();
-        // z in the contraction order of the down weights (pos32): 16-byte piece c holds columns 2c, 2c+1, 2c+8, 2c+9 of
-        // both blocks of 16
+        // z in the contraction order of the down weights (pos32): columns 4c .. 4c+3 of tensor memory, two halves each, hold
+        // columns 2c, 2c+1, 2c+8, 2c+9 of both blocks of 16
         uint32_t zp[16];
         if (busy) {
           const uint32_t d_gate = tmem_base + 2 * b * XT_CHUNK + lane_sel + 32 * half, d_up = d_gate + XT_CHUNK;
@@ -412,19 +403,11 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
               zp[4 * (i & 3) + 2 * hh + (i >> 2)] = *reinterpret_cast<const uint32_t*>(&h2);
             }
           }
+          tc::tmem_st16(d_gate, zp);                // over the first half of the gate sums that this warp has read
         }
         tc::fence_before_sync();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&bars.gu_free[b]);
-        if (g >= 1) ok = xt_wait(&bars.z_free, (g - 1) & 1u, abort_flag);     // the chunk before is multiplied
-        if (busy) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<uint4*>(zpart + c * XT_Z_STRIDE + lane * 16) = make_uint4(zp[4 * c], zp[4 * c + 1], zp[4 * c + 2], zp[4 * c + 3]);
-          tc::fence_async_smem();
-        }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&bars.z_ready);
+        if (lane == 0) tc::mbar_arrive_cluster(lead(&bars.z_ready[b]));
       }
       gu_round += nchunk;
       if (ok) ok = xt_wait(&bars.down_done, round & 1u, abort_flag);
@@ -434,92 +417,84 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         const float* s_d = reinterpret_cast<const float*>(tab + lay.s_d);
         const int16_t *rank_d = reinterpret_cast<const int16_t*>(tab + lay.rank_d), *oct_d = reinterpret_cast<const int16_t*>(tab + lay.oct_d);
         const float rw = n < n_tok ? item.rw[n] : 0.f;
-        const int rows = min(32, n_tok - 32 * q);
         // D_d * s * route weight -> rank_accum.  A thread owns a token: adding straight from the registers would touch a
-        // 32-byte sector per lane and instruction.  Sixteen slots at a time go through the warp's part of the (now idle) z
-        // area, so that an instruction adds the 64 bytes of eight tokens.  Octets of slots that are not an aligned octet
-        // of ranks, rows that do not start on 16-byte boundaries, and the deterministic mode add from the registers.
-        for (int s0 = 16 * half; s0 < nslots_d; s0 += 32) {
-          float v[16];
-          tc::tmem_ld16(d_down + lane_sel + s0, v);
+        // 32-byte sector per lane and instruction.  32 slots of 16 tokens at a time go through shared memory, so that an instruction adds 128 bytes of each of four tokens (128 KB in 5.1 K cycles of an SM, 8.1 K
+        // with 64 bytes of eight).  Octets of slots that are not an aligned octet of ranks, rows that do not start on
+        // 16-byte boundaries, and the deterministic mode add element by element.
+        for (int s0 = 32 * half; s0 < nslots_d; s0 += 64) {
+          float v[32];
+          tc::tmem_ld32(d_down + lane_sel + s0, v);
+          const bool whole = s0 + 16 < nslots_d;          // the matrix may end after 16 of the 32 slots
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
-            const float4 sv = *reinterpret_cast<const float4*>(s_d + s0 + i);
+          for (int i = 0; i < 32; i += 4) {
+            const float4 sv = i < 16 || whole ? *reinterpret_cast<const float4*>(s_d + s0 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
             v[i] *= sv.x * rw; v[i + 1] *= sv.y * rw; v[i + 2] *= sv.z * rw; v[i + 3] *= sv.w * rw;
           }
-          int oct[2];
-          oct[0] = A.vec_add ? oct_d[s0 >> 3] : -1;
-          oct[1] = A.vec_add ? oct_d[(s0 >> 3) + 1] : -1;
-          __syncwarp();                            // the pieces of the sixteen slots before have been read
+          // piece c (four slots) of token row r of sixteen, in an order that puts a row's eight pieces into distinct banks
+          auto at = [&](int c, int r) { return turn + (16 * c + (r ^ c)) * 16; };
+          const int piece = lane & 7, o = piece >> 1;
+          const int r0 = A.vec_add && (o < 2 || whole) ? oct_d[(s0 >> 3) + o] : -1;
+          const uint32_t odd = __ballot_sync(0xffffffffu, r0 < 0) & 0x55u;      // octets (by their first piece) that go element by element
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<float4*>(zpart + c * XT_Z_STRIDE + lane * 16) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
-          __syncwarp();
-          const int piece = lane >> 3, r0 = oct[piece >> 1];
-          if (r0 >= 0) {
+          for (int ph = 0; ph < 2; ++ph) {
+            const int first = 32 * q + 16 * ph, rows = min(16, n_tok - first);
+            if (rows <= 0) break;
+            __syncwarp();                            // the pieces before have been read
+            if ((lane >> 4) == ph) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int row = 8 * j + (lane & 7);
-              const float4 x = *reinterpret_cast<const float4*>(zpart + piece * XT_Z_STRIDE + row * 16);
-              if (row < rows)
-                asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(A.rank_accum + static_cast<int64_t>(item.tok[32 * q + row]) * rank_out +
-                                                                                   r0 + 4 * (piece & 1)),
-                             "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w)
-                             : "memory");
+              for (int c = 0; c < 8; ++c) *reinterpret_cast<float4*>(at(c, lane & 15)) = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
             }
-          }
+            __syncwarp();
+            if (r0 >= 0) {
 #pragma unroll
-          for (int h8 = 0; h8 < 2; ++h8)
-            if (oct[h8] < 0 && n < n_tok) {
-              for (int i = 0; i < 8; ++i) {
-                const int r = rank_d[s0 + 8 * h8 + i];
-                if (r >= 0) {
-                  float val = 0.f;
-#pragma unroll
-                  for (int k = 0; k < 16; ++k) val = k == 8 * h8 + i ? v[k] : val;
-                  acc_add(A.rank_accum, A.acc64, static_cast<int64_t>(item.tok[n]) * rank_out + r, val);
+              for (int j = 0; j < 4; ++j) {
+                const int row = 4 * j + (lane >> 3);
+                const float4 x = *reinterpret_cast<const float4*>(at(piece, row));
+                if (row < rows)
+                  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(A.rank_accum + static_cast<int64_t>(item.tok[first + row]) * rank_out +
+                                                                                     r0 + 4 * (piece & 1)),
+                               "f"(x.x), "f"(x.y), "f"(x.z), "f"(x.w)
+                               : "memory");
+              }
+            }
+            if (odd && (lane & 15) < rows) {          // two lanes a token: the even and the odd octets
+              for (int o2 = lane >> 4; o2 < (whole ? 4 : 2); o2 += 2) {
+                if (!((odd >> (2 * o2)) & 1u)) continue;
+                for (int i = 0; i < 8; ++i) {
+                  const int r = rank_d[s0 + 8 * o2 + i];
+                  if (r >= 0)
+                    acc_add(A.rank_accum, A.acc64, static_cast<int64_t>(item.tok[first + (lane & 15)]) * rank_out + r,
+                            *reinterpret_cast<const float*>(at(2 * o2 + (i >> 2), lane & 15) + 4 * (i & 3)));
                 }
               }
             }
+          }
         }
         tc::fence_before_sync();
         tc::fence_async_smem();
       }
       __syncwarp();
-      if (lane == 0) { tc::mbar_arrive(&bars.down_free); tc::mbar_arrive(&bars.item_free[ib]); }
+      if (lane == 0) { tc::mbar_arrive_cluster(lead(&bars.down_free)); tc::mbar_arrive(&bars.item_free[ib]); }
       if (!ok) break;
     }
-    // every role ends on its own (they do not share a register count to come together with)
-    tc::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tmem_base, 512);
-    if (threadIdx.x == 0 && *abort_flag) atomicExch(A.status, BM_ERR_TIMEOUT);
-    return;
-  }
-  if (warp < XT_DQ_WARP0 + XT_DQ_WARPS) {
+  } else if (warp < XT_DQ_WARP0 + XT_DQ_WARPS) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(XT_REGS_DQ));
     // -------------------------------------------------------------------- activation operand and converters
-    // Team 0 (six warps) feeds pipeline 0, team 1 pipeline 1; a team's warps take its stages in turn.  Step t of an item:
-    // a stage per 32 slots of chunk t's gate (up) product, then four stages (64 slots x 32 columns) per 128-slot tile of
-    // chunk t - lag's down product.  Stages 2 i and 2 i + 1 share a ring slot.  A stage is four 16 x 32 blocks; lane
-    // (g, t4) turns its words of each into two 16-byte pieces.  What bounds a warp is latency, not issue: a whole stage per
-    // warp gives it four independent blocks, one barrier wait, one proxy fence and one arrival per 2048 codes.
+    // Team 0 (six warps) feeds pipeline 0, team 1 pipeline 1.  Step t of an item is `n` stages of a team: a stage per 64
+    // slots (two pairs of blocks) of chunk t's gate (up) product, then two stages (64 slots x 32 columns each) per 128-slot
+    // tile of chunk t - lag's down product; stages 2 i and 2 i + 1 share a ring slot.  Warp w of the team takes stages w,
+    // w + 6, ... of every step: at 256 slots a matrix that is one stage, the same of every chunk, whose addresses and kinds of
+    // words are worked out once per item.  A stage is four 16 x 32 blocks; lane (g, t4) turns its words of each into two
+    // 16-byte pieces.
     const int dw = warp - XT_DQ_WARP0;
     const int team = dw / XT_TEAM, wt = dw - team * XT_TEAM, g = lane >> 2, t4 = lane & 3;
-    uint64_t* w_full = &bars.w_full[team * ring_h];
-    uint64_t* w_empty = &bars.w_empty[team * ring_h];
-    unsigned char* ring = sm.ring + team * ring_h * XT_SLOT_BYTES;
-    // where a stage's pieces go: 64-row stages lie one after the other, the two 64-row halves of a down slot share chunks
-    unsigned char* gu_dst = ring + (wt & 1) * XT_STAGE_BYTES + t4 * XT_W_STRIDE + g * 16;
-    unsigned char* dn_dst = ring + (wt & 1) * 1024 + t4 * XT_D_STRIDE + g * 16;
-    // The turns run on from item to item: a warp comes back to the ring after three slots, no more than it holds, so it sees
-    // every phase of the barriers that it waits at (a parity tells a phase from its neighbours only).
-    constexpr int SLOT_STEP = XT_TEAM / 2;
-    int slot0 = wt >> 1;                      // this warp's first slot of the item
-    XtCycle my_c{0, 0};                       // its place in the ring
+    uint64_t* w_empty = &bars.w_empty[team * ring];
+    const uint32_t w_full = lead(&bars.w_full[team * ring]);
+    unsigned char* ring0 = sm.ring + team * ring * XT_SLOT_BYTES;
     const XtMagic magic;
-    my_c.advance(slot0, ring_h);
-    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++round) {
+    uint32_t item_seq = 0;                    // ring slots that the pipeline has used before this item
+    uint32_t seen = 0;                        // every use of a slot before this one is known to be multiplied
+    for (int u = pair; u < units.n_units; u += n_pairs, ++round) {
       XT_ITEM_BEGIN
       if (round > 0 && !xt_wait(&bars.act_free, (round - 1) & 1u, abort_flag)) break;
       {
@@ -601,148 +576,175 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
         }
         tc::fence_async_smem();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&bars.act_ready);
+        if (lane == 0) tc::mbar_arrive_cluster(lead(&bars.act_ready));
       }
       // everything about the expert in registers: the barriers' memory clobbers would have it read again every stage
       const int chunk0 = item.chunk0, nblk_d = fe.m[2].nslots >> 4, n_mt = (nblk_d + 7) >> 3;
-      const int npairs = fe.m[team].nslots >> 5, n_gu = (npairs + 1) & ~1, nib_pairs = fe.m[team].nblk[0] >> 1, nib_d = fe.m[2].nblk[0];
-      const int n_d = team < n_mt ? 4 * ((n_mt - team + 1) >> 1) : 0;
+      const int npairs = fe.m[team].nslots >> 5, nib_pairs = fe.m[team].nblk[0] >> 1, nib_d = fe.m[2].nblk[0];
+      const int slots_gu = (npairs + 3) >> 2, slots_d = (n_mt - team + 1) >> 1, n = 2 * (slots_gu + slots_d);
       const int unit_bytes = fe.unit_bytes;
       const unsigned char* unit0 = A.arena + fe.unit_base;
-      const unsigned char* scale_gu = unit0 + fe.sec_off[team] + t4 * 16;
-      const unsigned char* words_gu = unit0 + fe.sec_off[3 + team];
-      const unsigned char* scale_d = unit0 + fe.sec_off[2] + g * 4;
-      const unsigned char* words_d = unit0 + fe.sec_off[5];
+      const int scale_gu = fe.sec_off[team] + t4 * 16, words_gu = fe.sec_off[3 + team], scale_d = fe.sec_off[2] + g * 4, words_d = fe.sec_off[5];
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&bars.item_free[ib]);
-      auto fetch = [&](int t, int i, XtPre& p) {
-        if (t < nchunk && i < n_gu) {
-          if (i >= npairs) return;         // an odd last stage has an empty partner in its slot
-          const int ch = chunk0 + t;
-          const int64_t tile = static_cast<int64_t>(ch >> 1) * unit_bytes;
-          p.s = __ldg(reinterpret_cast<const uint4*>(scale_gu + tile + i * 64));
-          if (i < nib_pairs) {              // columns 0-63 or 64-127 of the tile: blocks 0-3 or 4-7
-            const uint2* w = reinterpret_cast<const uint2*>(words_gu + tile + i * 2048 + (ch & 1) * 1024) + lane;
+      // The stage at hand: `kind` bit p: words of pair p (down: of block p) are nibbles; offsets of its words and scales in
+      // the unit block, `odd`: in the second chunk of a tile
+      int i = wt, t = 0, kind = 0, live = 0, w_off[2], s_off = 0, dst_off = 0;
+      bool gu = true;
+      auto set_up = [&]() {
+        gu = i < 2 * slots_gu;
+        if (gu) {
+          live = min(2, npairs - 2 * i);      // pairs (an odd last stage has an empty partner in its slot)
+          s_off = scale_gu + 2 * i * 64;
+          kind = 0;
 #pragma unroll
-            for (int x = 0; x < 4; ++x) p.w[x] = __ldg(w + x * 32);
-          } else {
-            const uint32_t* w = reinterpret_cast<const uint32_t*>(words_gu + tile + nib_pairs * 2048 + (i - nib_pairs) * 1024 + (ch & 1) * 512) + lane;
+          for (int p = 0; p < 2; ++p) {
+            const int pr = 2 * i + p;
+            const bool nib = pr < nib_pairs;
+            kind |= nib ? 1 << p : 0;
+            w_off[p] = words_gu + (nib ? pr * 2048 + 2 * rank * 256 + lane * 8 : nib_pairs * 2048 + (pr - nib_pairs) * 1024 + 2 * rank * 128 + lane * 4);
+          }
+          dst_off = (i & 1) * 8 * XT_G_STRIDE + t4 * XT_G_STRIDE + g * 16;
+        } else {
+          const int j = i - 2 * slots_gu, mb0 = 8 * (team + 2 * (j >> 1)) + 4 * rank;
+          live = min(4, nblk_d - mb0);        // blocks; slots past the matrix: accumulator columns that nobody reads
+          const int n_nib = min(max(nib_d - mb0, 0), 4);
+          kind = (1 << n_nib) - 1;
+          s_off = scale_d + mb0 * 32;
+          w_off[0] = words_d + (mb0 * 4 + (j & 1)) * 256 + lane * 8;                                              // of a nibble block
+          w_off[1] = words_d + nib_d * 1024 + ((mb0 - nib_d) * 4 + (j & 1)) * 128 + lane * 4;                     // of a dense block
+          dst_off = (j & 1) * 4 * XT_D_STRIDE + t4 * XT_D_STRIDE + g * 16;
+        }
+      };
+      auto fetch = [&](XtPre& p) {
+        const int ch = chunk0 + (gu ? t : t - lag), odd = ch & 1;
+        const unsigned char* b = unit0 + static_cast<int64_t>(ch >> 1) * unit_bytes;
+        if (gu) {
 #pragma unroll
-            for (int x = 0; x < 4; ++x) p.w[x].x = __ldg(w + x * 32);
+          for (int q = 0; q < 2; ++q) {
+            if (q >= live) break;
+            p.s[q] = __ldg(reinterpret_cast<const uint4*>(b + s_off + q * 64));
+            if (kind & (1 << q)) {
+              const uint2* w = reinterpret_cast<const uint2*>(b + w_off[q] + odd * 1024);
+              p.w[2 * q] = __ldg(w);
+              p.w[2 * q + 1] = __ldg(w + 32);
+            } else {
+              const uint32_t* w = reinterpret_cast<const uint32_t*>(b + w_off[q] + odd * 512);
+              p.w[2 * q].x = __ldg(w);
+              p.w[2 * q + 1].x = __ldg(w + 32);
+            }
           }
         } else {
-          // per 128-slot tile: columns 0-31 of the chunk for slots 0-63 and 64-127, then columns 32-63
-          const int j = t < nchunk ? i - n_gu : i, ch = chunk0 + t - lag;
-          const int64_t tile = static_cast<int64_t>(ch >> 1) * unit_bytes;
-          const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * (j & 1), pr = 2 * (ch & 1) + ((j >> 1) & 1);
-          uint32_t* ps = reinterpret_cast<uint32_t*>(&p.s);
+          uint32_t* ps = reinterpret_cast<uint32_t*>(p.s);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            const int mb = mb0 + v;
-            if (mb >= nblk_d) break;
-            ps[v] = __ldg(reinterpret_cast<const uint32_t*>(scale_d + tile + mb * 32));
-            if (mb < nib_d) p.w[v] = __ldg(reinterpret_cast<const uint2*>(words_d + tile + (mb * 4 + pr) * 256) + lane);
-            else p.w[v].x = __ldg(reinterpret_cast<const uint32_t*>(words_d + tile + nib_d * 1024 + ((mb - nib_d) * 4 + pr) * 128) + lane);
+            if (v >= live) break;
+            ps[v] = __ldg(reinterpret_cast<const uint32_t*>(b + s_off + v * 32));
+            if (kind & (1 << v)) p.w[v] = __ldg(reinterpret_cast<const uint2*>(b + w_off[0] + odd * 512 + v * 1024));
+            else p.w[v].x = __ldg(reinterpret_cast<const uint32_t*>(b + w_off[1] + odd * 256 + v * 512));
           }
         }
       };
-      auto convert = [&](int t, int i, const XtPre& p) -> bool {
-        if (!xt_wait(&w_empty[my_c.i], my_c.ph ^ 1, abort_flag)) return false;
-        if (t < nchunk && i < n_gu) {
-          if (i >= npairs) return true;
-          unsigned char* dst = gu_dst + my_c.i * XT_SLOT_BYTES;
-          const __half2* sp = reinterpret_cast<const __half2*>(&p.s);
-          const __half2 sc[4] = {sp[0], sp[1], sp[2], sp[3]};
-          if (i < nib_pairs) {
+      auto convert = [&](const XtPre& p, unsigned char* dst) {
+        if (gu) {
 #pragma unroll
-            for (int x = 0; x < 4; ++x) dequant_pair_store<false>(magic, p.w[x].x, p.w[x].y, sc, sc, dst + x * 256);
-          } else {
+          for (int q = 0; q < 2; ++q) {
+            if (q >= live) break;
+            const __half2* sp = reinterpret_cast<const __half2*>(&p.s[q]);
+            const __half2 sc[4] = {sp[0], sp[1], sp[2], sp[3]};
+            unsigned char* d = dst + q * 4 * XT_G_STRIDE;
+            if (kind & (1 << q)) {
 #pragma unroll
-            for (int x = 0; x < 4; ++x) dequant_pair_store<true>(magic, p.w[x].x, p.w[x].x >> 8, sc, sc, dst + x * 256);
+              for (int x = 0; x < 2; ++x) dequant_pair_store<false>(magic, p.w[2 * q + x], sc, sc, d + x * 256);
+            } else {
+#pragma unroll
+              for (int x = 0; x < 2; ++x) dequant_pair_store<true>(magic, p.w[2 * q + x], sc, sc, d + x * 256);
+            }
           }
         } else {
-          unsigned char* dst = dn_dst + my_c.i * XT_SLOT_BYTES;
-          const int j = t < nchunk ? i - n_gu : i;
-          const int mb0 = 8 * (team + 2 * (j >> 2)) + 4 * (j & 1);
-          const __half2* sp = reinterpret_cast<const __half2*>(&p.s);
+          const __half2* sp = reinterpret_cast<const __half2*>(p.s);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            if (mb0 + v >= nblk_d) break;             // slots past the matrix: accumulator columns that nobody reads
+            if (v >= live) break;
             const __half2 lo = __low2half2(sp[v]), hi = __high2half2(sp[v]);
             const __half2 sa[4] = {lo, lo, lo, lo}, sb[4] = {hi, hi, hi, hi};
-            if (mb0 + v < nib_d) dequant_pair_store<false>(magic, p.w[v].x, p.w[v].y, sa, sb, dst + v * 256);
-            else dequant_pair_store<true>(magic, p.w[v].x, p.w[v].x >> 8, sa, sb, dst + v * 256);
+            if (kind & (1 << v)) dequant_pair_store<false>(magic, p.w[v], sa, sb, dst + v * 256);
+            else dequant_pair_store<true>(magic, p.w[v], sa, sb, dst + v * 256);
           }
         }
-        return true;
       };
-      auto publish = [&]() {
-        tc::fence_async_smem();
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&w_full[my_c.i]);
-        my_c.i += SLOT_STEP;                 // ring_h >= SLOT_STEP: at most one wrap
-        if (my_c.i >= static_cast<uint32_t>(ring_h)) { my_c.i -= ring_h; my_c.ph ^= 1u; }
-      };
-      // this warp's stage after (t, i); false past its last one
-      auto step = [&](int& t, int& i) -> bool {
-        i += XT_TEAM;
-        for (int n = (t < nchunk ? n_gu : 0) + (t >= lag ? n_d : 0); t < nchunk + lag && i >= n; n = (t < nchunk ? n_gu : 0) + n_d) {
-          i -= n;
-          ++t;
+      // this warp's next stage; false past the last one
+      auto step = [&]() -> bool {
+        for (;;) {
+          i += XT_TEAM;
+          if (i >= n) { i = wt; ++t; }
+          if (t >= nchunk + lag) return false;
+          if (i < 2 * slots_gu ? t < nchunk : t >= lag) return true;
         }
-        return t < nchunk + lag;
       };
       XtPre p;
-      int t = 0, i = 2 * (slot0 - SLOT_STEP) + (wt & 1);
-      bool more = step(t, i), ok = true;
-      if (more) fetch(t, i, p);
+      bool ok = true, more = wt < n;
+      if (more && !(wt < 2 * slots_gu || lag == 0)) more = step();
+      if (more) { set_up(); fetch(p); }
       while (more) {
-        if (!(ok = convert(t, i, p))) break;
-        more = step(t, i);
-        if (more) fetch(t, i, p);           // on its way while the converted stage is published and the next one is waited for
-        publish();
+        // the use of a ring slot that this stage fills: steps before t, then this step's order (the last one has no gate / up)
+        const uint32_t pos = item_seq + t * (slots_gu + slots_d) - (t > 0 && lag ? slots_d : 0) + (i >> 1) - (t == nchunk ? slots_gu : 0);
+        // A parity tells a phase from its neighbours only: uses further apart than the ring are waited for one by one.
+        while (static_cast<int>(pos - seen) >= ring) {
+          const uint32_t last = min(seen + ring - 1, pos - ring);
+          if (!(ok = xt_wait(&w_empty[last & (ring - 1)], (last >> A.ring_log2) & 1u, abort_flag))) break;
+          seen = last + 1;
+        }
+        if (!ok) break;
+        convert(p, ring0 + (pos & (ring - 1)) * XT_SLOT_BYTES + dst_off);
+        const int i_was = i;
+        more = step();
+        if (more) {
+          if (i != i_was) set_up();
+          fetch(p);                         // on its way while the converted stage is published and the next one is waited for
+        }
+        tc::fence_async_smem();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive_cluster(w_full + (pos & (ring - 1)) * 8);
       }
-      slot0 = (slot0 + SLOT_STEP - nchunk * (n_gu + n_d) / 2 % SLOT_STEP) % SLOT_STEP;
+      item_seq += nchunk * (slots_gu + slots_d);
       if (!ok) break;
     }
-    __syncthreads();
-    return;
-  }
+  } else {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XT_REGS_MISC));
   if (warp == XT_LOOKUP_WARP) {
     // -------------------------------------------------------------------- descriptions, an item ahead of the roles
-    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++round) {
+    for (int u = pair; u < units.n_units; u += n_pairs, ++round) {
       const uint32_t ib = round & 1u;
       if (round >= 2 && !xt_wait(&bars.item_free[ib], ((round >> 1) - 1) & 1u, abort_flag)) break;
-      xt_load_item(items[ib], sm.tab + ib * lay.bytes, &bars.item_full[ib], u, units, n_chunks, sm, A, lane);
+      xt_load_item(items[ib], sm.tab + ib * lay.bytes, &bars.item_full[ib], u, units, n_chunks, sm, A, lane, rank);
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&bars.item_full[ib]);
       // the copy lands whatever the other roles do: waited for also when one of them has given up
-      if (!tc::mbar_wait(&bars.item_full[ib], (round >> 1) & 1u)) { *abort_flag = 1; break; }
-      // the weights on their way to L2, one tile per lane (sizes and offsets are multiples of 16 bytes)
+      if (!tc::mbar_wait(&bars.item_full[ib], (round >> 1) & 1u)) { xt_give_up(abort_flag); break; }
+      // the weights on their way to L2, one tile per lane, every other one by this CTA (sizes and offsets are multiples of 16 bytes)
       const FastExpert& fe = reinterpret_cast<const TokTabHead*>(sm.tab + ib * lay.bytes)->fe;
       const int t0 = items[ib].chunk0 >> 1, t1 = (items[ib].chunk0 + items[ib].nchunk + 1) >> 1;
-      for (int t = t0 + lane; t < t1; t += 32)
+      for (int t = t0 + 2 * lane + rank; t < t1; t += 64)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A.arena + fe.unit_base + static_cast<int64_t>(t) * fe.unit_bytes),
                      "r"(fe.unit_bytes)
                      : "memory");
       __syncwarp();
     }
-  } else if (warp < XT_MMA_WARP0 + 2) {
-    // -------------------------------------------------------------------- MMA issue, one thread per pipeline
+  } else if (warp < XT_MMA_WARP0 + 2 && rank == 0) {
+    // -------------------------------------------------------------------- MMA issue for both CTAs, one thread per pipeline
     // The whole warp waits (a lone waiting lane wakes up several times slower); one issues.
     const int pl = warp - XT_MMA_WARP0;
-    const uint32_t idesc_gu = tc::idesc_f16(128, 64), idesc_d = tc::idesc_f16(128, 128);
+    const uint32_t idesc_gu = tc::idesc_f16(256, 64), idesc_d = tc::idesc_f16(256, 128);
     // descriptors: constant upper part, start-address field advanced per block
     const uint64_t a_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.act) + pl * act_m_bytes, cs, 128);
-    const uint64_t z_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.z), XT_Z_STRIDE, 128);
-    const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring_h * XT_SLOT_BYTES;
-    const uint64_t gu_desc = tc::smem_desc_kmajor(ring0, XT_W_STRIDE, 128), dn_desc = tc::smem_desc_kmajor(ring0, XT_D_STRIDE, 128);
-    uint64_t* w_full = &bars.w_full[pl * ring_h];
-    uint64_t* w_empty = &bars.w_empty[pl * ring_h];
+    const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring * XT_SLOT_BYTES;
+    const uint64_t gu_desc = tc::smem_desc_kmajor(ring0, XT_G_STRIDE, 128), dn_desc = tc::smem_desc_kmajor(ring0, XT_D_STRIDE, 128);
+    uint64_t* w_full = &bars.w_full[pl * ring];
+    uint64_t* w_empty = &bars.w_empty[pl * ring];
     const uint32_t a_step = (2 * cs) >> 4;       // descriptor units per 16 contraction positions
-    XtCycle ring_c{0, 0};
-    for (int u = blockIdx.x; u < units.n_units; u += gridDim.x, ++round) {
+    uint32_t seq = 0;                            // uses of ring slots so far
+    for (int u = pair; u < units.n_units; u += n_pairs, ++round) {
       XT_ITEM_BEGIN
       const int npairs = fe.m[pl].nslots >> 5, n_mt = ((fe.m[2].nslots >> 4) + 7) >> 3;   // 128-slot tiles of the down product (<= 3)
       __syncwarp();
@@ -752,53 +754,53 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       for (int t = 0; t < nchunk + lag && ok; ++t) {
         if (t < nchunk) {
           const uint32_t g = gu_round + t, b = lag ? g & 1u : 0u, k = lag ? g >> 1 : g;
-          if (k >= 1) ok = xt_wait(&bars.gu_free[b], (k - 1) & 1u, abort_flag);   // this accumulator's last contents are read out
+          if (k >= 1) ok = xt_wait(&bars.z_free[b], (k - 1) & 1u, abort_flag);     // the z written over this accumulator is multiplied
           tc::fence_after_sync();
           const uint32_t d_acc = tmem_base + (2 * b + pl) * XT_CHUNK;
           uint64_t ad = a_desc;
-          for (int pr = 0; pr < npairs && ok; pr += 2) {
-            if (!(ok = xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag))) break;
+          for (int pr = 0; pr < npairs && ok; pr += 4, ++seq) {
+            const uint32_t sl = seq & (ring - 1);
+            if (!(ok = xt_wait(&w_full[sl], (seq >> A.ring_log2) & 1u, abort_flag))) break;
             if (tc::elect_one()) {
-              const uint64_t bd = gu_desc + ((ring_c.i * XT_SLOT_BYTES) >> 4);
-              tc::mma_f16(d_acc, ad, bd, idesc_gu, pr > 0 ? 1u : 0u);
-              tc::mma_f16(d_acc, ad + a_step, bd + ((2 * XT_W_STRIDE) >> 4), idesc_gu, 1u);
-              if (pr + 1 < npairs) {
-                tc::mma_f16(d_acc, ad + 2 * a_step, bd + (XT_STAGE_BYTES >> 4), idesc_gu, 1u);
-                tc::mma_f16(d_acc, ad + 3 * a_step, bd + ((XT_STAGE_BYTES + 2 * XT_W_STRIDE) >> 4), idesc_gu, 1u);
-              }
-              tc::mma_commit(&w_empty[ring_c.i]);
+              const uint64_t bd = gu_desc + ((sl * XT_SLOT_BYTES) >> 4);
+#pragma unroll
+              for (int h = 0; h < 8; ++h)         // 16 slots each
+                if (h < 2 || pr + (h >> 1) < npairs)
+                  tc::mma_f16_pair(d_acc, ad + h * a_step, bd + ((h * 2 * XT_G_STRIDE) >> 4), idesc_gu, pr > 0 || h > 0 ? 1u : 0u);
+              tc::mma_commit_pair(&w_empty[sl]);
             }
             __syncwarp();
-            ad += 4 * a_step;
-            ring_c.next(ring_h);
+            ad += 8 * a_step;
           }
           if (!ok) break;
           if (tc::elect_one()) {
-            tc::mma_commit(&bars.gu_done[b]);
-            if (t == nchunk - 1) tc::mma_commit(&bars.act_free);
+            tc::mma_commit_pair(&bars.gu_done[b]);
+            if (t == nchunk - 1) tc::mma_commit_pair(&bars.act_free);
           }
           __syncwarp();
         }
         if (t >= lag) {
-          const uint32_t g = gu_round + t - lag;
+          const uint32_t g = gu_round + t - lag, b = lag ? g & 1u : 0u;
           if (t == lag && round > 0) ok = xt_wait(&bars.down_free, (round - 1) & 1u, abort_flag);   // the last item's sums are read out
-          if (ok) ok = xt_wait(&bars.z_ready, g & 1u, abort_flag);
+          if (ok) ok = xt_wait(&bars.z_ready[b], (lag ? g >> 1 : g) & 1u, abort_flag);
           tc::fence_after_sync();
-          for (int mt = pl; mt < n_mt && ok; mt += 2)
-            for (int kp = 0; kp < 2; ++kp) {                 // 32 columns of z per slot
-              if (!(ok = xt_wait(&w_full[ring_c.i], ring_c.ph, abort_flag))) break;
-              if (tc::elect_one()) {
-                const uint64_t bd = dn_desc + ((ring_c.i * XT_SLOT_BYTES) >> 4), zd = z_desc + ((4 * kp * XT_Z_STRIDE) >> 4);
-                tc::mma_f16(d_down + mt * 128, zd, bd, idesc_d, t > lag || kp > 0 ? 1u : 0u);
-                tc::mma_f16(d_down + mt * 128, zd + ((2 * XT_Z_STRIDE) >> 4), bd + ((2 * XT_D_STRIDE) >> 4), idesc_d, 1u);
-                tc::mma_commit(&w_empty[ring_c.i]);
-              }
-              __syncwarp();
-              ring_c.next(ring_h);
+          const uint32_t d_z = tmem_base + 2 * b * XT_CHUNK;      // columns 0-31 of the chunk, and 32-63 32 columns on
+          for (int mt = pl; mt < n_mt && ok; mt += 2, ++seq) {
+            const uint32_t sl = seq & (ring - 1);
+            if (!(ok = xt_wait(&w_full[sl], (seq >> A.ring_log2) & 1u, abort_flag))) break;
+            if (tc::elect_one()) {
+              const uint64_t bd = dn_desc + ((sl * XT_SLOT_BYTES) >> 4);
+#pragma unroll
+              for (int h = 0; h < 4; ++h)           // 16 columns of z each
+                tc::mma_f16_pair_ta(d_down + mt * 128, d_z + 32 * (h >> 1) + 8 * (h & 1), bd + ((h * 2 * XT_D_STRIDE) >> 4), idesc_d,
+                                 t > lag || h > 0 ? 1u : 0u);
+              tc::mma_commit_pair(&w_empty[sl]);
             }
+            __syncwarp();
+          }
           if (ok && tc::elect_one()) {
-            tc::mma_commit(&bars.z_free);
-            if (t == nchunk + lag - 1) tc::mma_commit(&bars.down_done);
+            tc::mma_commit_pair(&bars.z_free[b]);
+            if (t == nchunk + lag - 1) tc::mma_commit_pair(&bars.down_done);
           }
           __syncwarp();
         }
@@ -806,29 +808,38 @@ __global__ void __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_
       gu_round += nchunk;
       if (!ok) break;
     }
-    if (tc::elect_one()) tc::mma_commit(&bars.drained[pl]);
+    if (tc::elect_one()) tc::mma_commit_pair(&bars.drained[pl]);
     __syncwarp();
-    if (!tc::mbar_wait(&bars.drained[pl], 0)) *abort_flag = 1;
   }
+  }
+  // Every role of both CTAs comes here on its own, also when a wait gave up.  Nothing of the pair is in flight behind the
+  // last commits, and neither CTA leaves while the other may still signal its barriers.
   tc::fence_before_sync();
   __syncthreads();
+  if (warp == XT_MMA_WARP0)
+    for (int i = 0; i < 2; ++i)
+      if (!tc::mbar_wait(&bars.drained[i], 0)) xt_give_up(abort_flag);
+  tc::cluster_arrive();
+  tc::cluster_wait();
+  if (warp == 0) tc::tmem_dealloc_pair(tmem_base, 512);
+  if (threadIdx.x == 0 && *abort_flag) atomicExch(A.status, BM_ERR_TIMEOUT);
 #undef XT_ITEM_BEGIN
 }
 
 // Item size and ring depth for a layer: the first candidate whose activation operand (2 KB per token at 256 row slots per
 // matrix) and stages fit shared memory.  Tensor memory holds 128 columns per gate/up buffer and 128 per 128
 // slots of the down product.
-struct XtPlan { int nt, ring_h, gu_bufs; size_t smem; };
+struct XtPlan { int nt, ring_log2, gu_bufs; size_t smem; };
 constexpr size_t XT_SMEM_LIMIT = 227 * 1024 - 3072;     // dynamic part: the static part (two item descriptions, barriers) stays below 3 KB
 static bool xt_plan(const bm_layer* L, XtPlan* out) {
   if (!L->toktab_dev || L->num_experts > XT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > 3 * 128) return false;
   const int n_mt = (L->max_slots + 127) / 128;
   static const int cand[] = {128, 112, 96, 80, 64, 48, 32, 16};
   for (const int nt : cand) {
-    for (int ring = XT_RING_MAX; ring >= XT_TEAM / 2; --ring) {
-      const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, TokTab(L->rank_in, L->max_slots).bytes, nt, ring);
+    for (int lg = 3; lg >= 2; --lg) {
+      const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, TokTab(L->rank_in, L->max_slots).bytes, nt, 1 << lg);
       if (smem <= XT_SMEM_LIMIT) {
-        *out = XtPlan{nt, ring, n_mt > 2 ? 1 : 2, smem};
+        *out = XtPlan{nt, lg, n_mt > 2 ? 1 : 2, smem};
         return true;
       }
     }
@@ -854,13 +865,14 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
   XtPlan plan;
   BM_REQUIRE(xt_plan(L, &plan), BM_ERR_UNSUPPORTED, "experts_tc: the layer's largest expert does not fit in shared memory");
   static PerDeviceOnce attr_once;
-  static int sm_counts[MAX_DEVICES];
+  static int grids[MAX_DEVICES];
   int dev = -1;
   BM_CUDA(cudaGetDevice(&dev));
   BM_REQUIRE(dev >= 0 && dev < MAX_DEVICES, BM_ERR_UNSUPPORTED, "experts_tc: device ordinal %d out of range", dev);
   if (!attr_once.is_done(dev)) {
     BM_CUDA(cudaFuncSetAttribute(experts_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(XT_SMEM_LIMIT)));
-    BM_CUDA(cudaDeviceGetAttribute(&sm_counts[dev], cudaDevAttrMultiProcessorCount, dev));
+    BM_CUDA(cudaDeviceGetAttribute(&grids[dev], cudaDevAttrMultiProcessorCount, dev));
+    grids[dev] &= ~1;
     cudaFuncAttributes fa;
     BM_CUDA(cudaFuncGetAttributes(&fa, experts_tc_kernel));
     BM_REQUIRE(fa.numRegs >= XT_REGS, BM_ERR_UNSUPPORTED, "experts_tc: built with %d registers per thread, %d expected", fa.numRegs, XT_REGS);
@@ -877,8 +889,8 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
   a.vec_add = acc64 == nullptr && L->rank_out % 4 == 0 && (reinterpret_cast<uintptr_t>(rank_accum) & 15u) == 0;
   a.wait_limit_us = L->wait_limit_us;
   a.rank_out = L->rank_out; a.T = T; a.num_experts = L->num_experts; a.n_tiles = L->n_tiles; a.max_slots = L->max_slots;
-  a.nt = plan.nt; a.ring_h = plan.ring_h; a.gu_bufs = plan.gu_bufs;
-  experts_tc_kernel<<<sm_counts[dev], XT_THREADS, plan.smem, st>>>(a);
+  a.nt = plan.nt; a.ring_log2 = plan.ring_log2; a.gu_bufs = plan.gu_bufs;
+  experts_tc_kernel<<<grids[dev], XT_THREADS, plan.smem, st>>>(a);
   BM_LAUNCH_CHECK("experts_tc_kernel");
   return BM_OK;
 }

@@ -40,6 +40,24 @@ def test_packed_experts_match_generic_kernel(rank, inter, counts):
         helpers.assert_close(got.cpu(), want.cpu(), what=f"path {path} rank {rank} counts {counts}")
 
 
+# whole rounds of items, so that a pair of CTAs walks several items of several chunks: both CTAs with tokens, one with none,
+# items of one and of 256, ranks of one to three slot tiles and of an odd number of pairs
+@pytest.mark.parametrize("rank,inter", [(64, 384), (96, 128), (256, 256), (328, 256)])
+def test_pairs_walk_several_items(rank, inter):
+    counts = tuple((1, 2, 0, 63, 64, 65, 255, 256, 257)[e % 9] for e in range(210))
+    cfg = synth.tiny(hidden=128, num_experts=len(counts), intermediate=inter, top_k=1, rank=rank)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=rank, device=DEV))
+    T = 300
+    gen = torch.Generator(device=DEV).manual_seed(17)
+    tok, off, rw = _route(counts, 1, T, gen)
+    hg, hu = layer.basis_project(synth.activations(cfg, T, seed=2, device=DEV, dtype=torch.bfloat16))
+    want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
+    for _ in range(3):
+        got = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_TENSOR)
+        layer.check_status()
+        helpers.assert_close(got.cpu(), want.cpu(), what=f"rank {rank} inter {inter}")
+
+
 def _with_output_rank(rank_in, rank_out, inter, E):
     """A layer whose down matrices have ``rank_out`` rows while gate and up have ``rank_in``."""
     a = synth.make_layer(synth.tiny(hidden=128, num_experts=E, intermediate=inter, top_k=1, rank=rank_in), seed=1, device=DEV)
