@@ -1,19 +1,20 @@
 // Packed routed-expert forward for large token counts (prefill): fused mixed-bit grouped GEMM on the
 // 5th-generation tensor cores (tcgen05.mma, accumulators in tensor memory), a pair of CTAs per work item.
 //
-// Work item = (expert, block of up to 2 NT of its assignments; NT = 128 where it fits).  A persistent pair of CTAs (cluster of
-// two, cta_group::2) walks the items; each CTA holds half of the item's tokens as 128 rows (M) of every product and converts
-// half of the weights, its columns (N); the tensor cores read both halves, so the converted weights never cross the cluster.
-// The tile's columns are taken 64 at a time ("chunk"):
-//   gate/up:  D_g[n, c] = sum_slot act_g[n, slot] * W_g[c, slot]     (N = 64 columns c, 32 from each CTA; K = row slots)
-//   down:     D_d[n, slot] += sum_c z[n, c] * W_d[slot, c]           (N = 128 row slots x 1..3, 64 from each CTA; K = 64 columns c)
-// Tokens as rows make the epilogue cheap: a thread owns a token.  z goes back to tensor memory, over the gate sums it came
-// from, and is the A operand of the down product there.  64 columns at a time leave room in tensor memory for two gate/up
-// accumulator pairs (2 x 128 columns) beside the down accumulator (256), so the products of a chunk run while the previous
-// one is turned into z.
+// Work item = (expert, block of up to 2 NT of its assignments; NT = ROWS = 128 or 64 where it fits).  A persistent pair of CTAs
+// (cluster of two, cta_group::2) walks the items; each CTA holds half of the item's tokens as ROWS rows (M) of every product and
+// converts half of the weights, its columns (N); the tensor cores read both halves, so the converted weights never cross the
+// cluster.  The tile's columns are taken a chunk (64, with 64 rows 128) at a time:
+//   gate/up:  D_g[n, c] = sum_slot act_g[n, slot] * W_g[c, slot]     (N = the chunk's columns c, half from each CTA; K = row slots)
+//   down:     D_d[n, slot] += sum_c z[n, c] * W_d[slot, c]           (N = 128 row slots x 1..3, 64 from each CTA; K = the chunk's columns)
+// Tokens as rows make the epilogue cheap: a thread owns a token.  Tensor memory holds two gate/up accumulator pairs beside the
+// down accumulator, so the products of a chunk run while the previous one is turned into z.  128 rows: a lane is a row; z goes
+// back to tensor memory, over the gate sums it came from, and is the A operand of the down product there.  64 rows: lanes 0-63
+// hold the lower half of an accumulator's columns, lanes 64-127 the upper half, which leaves columns for chunks of 128; z is an
+// operand in shared memory.
 //
 // Warp roles (768 threads; the last warp completes the last warpgroup):
-//   warps 0-7   epilogue (two per TMEM lane quarter, 32 columns each): tcgen05.ld D_g/D_u -> z = silu(g)*u -> fp16, tcgen05.st;
+//   warps 0-7   epilogue (two per TMEM lane quarter, 32 columns each): tcgen05.ld D_g/D_u -> z = silu(g)*u -> fp16;
 //               at the end of the item D_d * s * route weight is turned through shared memory and added to rank_accum in
 //               16-byte vector reductions, beside the next item's staging.
 //   warps 8-19  converters, one team of six warps per pipeline: arena words (nibble / dense 2-bit codes), read straight
@@ -28,19 +29,22 @@
 // before.  What an MMA issuer waits for is signalled by both CTAs (mapped arrivals on the even CTA's barriers), what waits for
 // MMAs is signalled in both by the commit.
 //
-// What bounds it: shared-memory bandwidth.  Every MMA of the gate and up products reads 4 KB of activations for 64 columns;
-// with the weights it is about 210 KB a chunk, and 48 KB of converted weights are stored, 2.0 K cycles at 128 bytes a cycle;
-// a chunk takes 2.4 K where an item has few tokens and 3.6 K at 128 rows a CTA, where epilogue and sums work beside it.
-// Converting in pairs halves the conversions per token, which set the pace before (7.0 K cycles a chunk of 128 tokens).
-// Stage of 8192 tokens of 128 experts (rank 256, intermediate 768): 176 -> 121 us; 2048 tokens 72 -> 61, 777 tokens 59 -> 52;
-// 16384 tokens of 512 experts 318 -> 238, 1200 of them (a dozen tokens a CTA and item) 114 -> 115.
+// What bounds it.  128 rows: the MMAs.  A chunk of 64 columns is 32 of N = 64, which take about 50 cycles each whatever their
+// rows (they read 4 KB of activations from shared memory), and 8 of N = 128: 2.1 K cycles of 3.6 K a chunk all in; the rest is
+// the way through ring, epilogue and arrivals, and 6 K cycles an item in which the activations are staged.  64 rows: the chain of
+// the converter warps (an MMA of 64 rows takes as long as one of 128, but N = 128 halves their number); a stage is about 280
+// instructions at 8 cycles each, and what the instruction cache holds of 24 warps in different roles matters: a copy of the
+// loop for each kind of stage took 60 us where one for all takes 40 (203 tokens), one for gate/up and down together 42.
+// Stage of 8192 tokens of 128 experts (rank 256, intermediate 768): 121 us (176 before weights were converted in pairs), 2048
+// tokens 59 (72), 777 tokens 45 (59), 300 tokens 40 (50); of 512 experts: 16384 tokens 235 us (318), 2048 tokens 99 (125 with 128
+// rows), 1050 tokens 90 (114).
 // The mapped arrivals carry no cluster-scope release: what they publish is read by the tensor cores of the CTA that wrote it
-// (behind the proxy fence); with the release a converter's arrival took 1.4 K cycles and the stage 165 us.
+// (behind the proxy fence); with the release a converter's arrival took 1.4 K cycles and the stage of 8192 tokens 165 us.
 //
 // The down product of a chunk is issued one chunk late (G0 U0 | G1 U1 D0 | G2 U2 D1 | ...).  Every mbarrier wait is
 // bounded in time.  One that gives up raises a flag in both CTAs; the roles then leave at their next wait that is not over, the
 // look-up warp behind its copy, both CTAs behind the MMAs issued so far, and tensor memory is given back after that.
-#include "fast_layout.cuh"
+#include "dequant.cuh"
 #include "tc05.cuh"
 
 namespace bm {
@@ -54,19 +58,28 @@ constexpr int XT_TEAM = XT_DQ_WARPS / 2;  // converter warps per pipeline
 constexpr int XT_REGS = 80, XT_REGS_EPI = 80, XT_REGS_DQ = 88, XT_REGS_MISC = 56;
 static_assert(32 * (XT_EPI_WARPS * XT_REGS_EPI + XT_DQ_WARPS * XT_REGS_DQ + 4 * XT_REGS_MISC) <= XT_THREADS * XT_REGS,
               "the roles' registers come out of the launch's");
-constexpr int XT_CHUNK = 64;              // tile columns per step
-constexpr int XT_RING_MAX = 8;            // operand slots per pipeline (at most; a power of two)
+constexpr int XT_ACC = 64;                // columns of tensor memory of a gate or up accumulator
+// Tile columns per step, by the rows (tokens) of a CTA: 64 rows of a pair's accumulator take half as many columns as it has
+__host__ __device__ constexpr int xt_chunk(int rows) { return rows > 64 ? 64 : 128; }
+// Operand slots per pipeline, by the rows (tokens) of a CTA
+__host__ __device__ constexpr int xt_ring(int rows) { return rows > 64 ? 4 : 6; }
+constexpr int XT_RING_MAX = 6;
 // A weight slot: this CTA's half of the rows of one B operand, in two stages that two warps fill.
-//   gate/up  32 columns of the chunk x 128 row slots (four pairs of 16-slot blocks; a stage is two of them)
-//   down     64 slots of a 128-slot tile x the chunk's 64 columns (a stage is 32 of them)
+//   gate/up  128 rows: 32 columns of the chunk x 128 row slots (four pairs of 16-slot blocks; a stage is two of them)
+//            64 rows: 64 columns x 64 slots (a stage is a pair)
+//   down     64 slots of a 128-slot tile x 64 columns (a stage is 32 of them)
 // Bytes between 8-position chunks, padded: the 16-byte stores of a quarter warp hit distinct banks.
-constexpr int XT_G_STRIDE = 32 * 16 + 32, XT_D_STRIDE = 64 * 16 + 32;
-constexpr int XT_SLOT_BYTES = 16 * XT_G_STRIDE;
-static_assert(8 * XT_D_STRIDE <= XT_SLOT_BYTES, "a down slot fits");
-constexpr int XT_TURN_BYTES = 2048;       // where an epilogue warp turns its sums: 16 tokens x 32 slots
+constexpr int XT_N32_STRIDE = 32 * 16 + 32, XT_N64_STRIDE = 64 * 16 + 32;
+__host__ __device__ constexpr int xt_g_stride(int rows) { return rows > 64 ? XT_N32_STRIDE : XT_N64_STRIDE; }
+constexpr int XT_D_STRIDE = XT_N64_STRIDE;
+constexpr int XT_SLOT_BYTES = 16 * XT_N32_STRIDE;
+static_assert(8 * XT_N64_STRIDE <= XT_SLOT_BYTES, "a slot of 64-row operands fits");
+constexpr int XT_Z_STRIDE = 64 * 16 + 16, XT_Z_BYTES = 16 * XT_Z_STRIDE;      // z operand in shared memory (64 rows x 128 columns): bytes between chunks, a buffer
+constexpr int XT_TURN_BYTES = 2048;       // where an epilogue warp turns its sums: 16 tokens x 32 slots (64 rows: its part of the idle z operand)
+__host__ __device__ constexpr int xt_z_or_turn_bytes(int rows) { return rows > 64 ? XT_EPI_WARPS * XT_TURN_BYTES : 2 * XT_Z_BYTES; }
 // bytes between 8-position chunks of the token-side operands (padded: conflict-free stores)
 __host__ __device__ constexpr int xt_chunk_stride(int nt) { return nt * 16 + 16; }
-constexpr int XT_MAX_E = 1024;
+constexpr int XT_MAX_E = 1024, XT_MAX_SLOTS = 3 * 128;
 
 struct XtBars {
   uint64_t w_full[2 * XT_RING_MAX], w_empty[2 * XT_RING_MAX];     // weight slots of the pipelines
@@ -119,77 +132,49 @@ __device__ __forceinline__ bool xt_wait(uint64_t* bar, uint32_t parity, volatile
   return done ? true : xt_wait_slow(bar, parity, abort_flag);
 }
 
-// One arena word (a 16x16 block's codes owned by lane (g, t), see fast_layout.cuh) -> four fp16 pairs
-// (q * scale): r[0] = row g, k (2t, 2t+1); r[1] = row g+8, same k; r[2] = row g, k (2t+8, 2t+9); r[3] = row g+8.
-// The code sits in the mantissa of 1024 (fields at bit 0) or of 64 (fields at bit 4); subtracting
-// 1024 + offset or 64 + offset is exact, the multiplication by the scale rounds once, as fp16(q * scale) does.
-// The exponents 1024 and 64 as fp16 pairs, held in registers as opaque values, so that (w & mask) | k needs one immediate
-// operand only (8192 tokens 185 -> 179 us against constants).
-struct XtMagic {
-  uint32_t lo, hi;
-  __device__ __forceinline__ XtMagic() {
-    asm volatile("mov.b32 %0, 0x64006400;" : "=r"(lo));
-    asm volatile("mov.b32 %0, 0x54005400;" : "=r"(hi));
+// How a group's words become weights (dequant.cuh), in registers: the converters hold one copy of their code for nibble and
+// dense words.  With a copy for each the instruction cache does not hold what 24 warps in different roles run.
+struct XtFields {
+  uint32_t mlo, mhi, shift, blo, bhi;
+  bool nib;
+  __device__ __forceinline__ explicit XtFields(bool n) : nib(n) {
+    const uint32_t off = n ? FAST_NIB_OFFSET : FAST_DENSE_OFFSET;
+    mlo = n ? 0x000F000Fu : 0x00030003u;
+    mhi = mlo << 4;
+    shift = n ? 8u : 2u;
+    blo = 0x64006400u + off * 0x00010001u;
+    bhi = 0x54005400u + off * 0x00100010u;
   }
 };
-template <uint32_t MASK>
-__device__ __forceinline__ uint32_t and_or(uint32_t w, uint32_t k) {
+__device__ __forceinline__ uint32_t xt_weight(uint32_t w, uint32_t mask, uint32_t magic, uint32_t sub, __half2 scale) {
   uint32_t v;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v) : "r"(w), "n"(MASK), "r"(k));
-  return v;
+  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(v) : "r"(w), "r"(mask), "r"(magic));
+  const __half2 o = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&sub)), scale);
+  return *reinterpret_cast<const uint32_t*>(&o);
 }
-template <bool DENSE>
-__device__ __forceinline__ void dequant_block(const XtMagic& k, uint32_t w, __half2 s0, __half2 s1, __half2 s2, __half2 s3, uint32_t (&r)[4]) {
-  constexpr uint32_t mlo = DENSE ? 0x00030003u : 0x000F000Fu, mhi = DENSE ? 0x00300030u : 0x00F000F0u;
-  constexpr uint32_t off = DENSE ? FAST_DENSE_OFFSET : FAST_NIB_OFFSET;
-  constexpr uint32_t blo_bits = 0x64006400u + off * 0x00010001u;          // fp16x2 of 1024 + offset
-  constexpr uint32_t bhi_bits = 0x54005400u + off * 0x00100010u;          // fp16x2 of 64 + offset
-  const uint32_t blo_u = blo_bits, bhi_u = bhi_bits;
-  const __half2 blo = *reinterpret_cast<const __half2*>(&blo_u), bhi = *reinterpret_cast<const __half2*>(&bhi_u);
-  const uint32_t sh = w >> (DENSE ? 2 : 8);
-  uint32_t v[4] = {and_or<mlo>(w, k.lo), and_or<mhi>(w, k.hi), and_or<mlo>(sh, k.lo), and_or<mhi>(sh, k.hi)};
-  const __half2 o0 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&v[0]), blo), s0);
-  const __half2 o1 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&v[1]), bhi), s1);
-  const __half2 o2 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&v[2]), blo), s2);
-  const __half2 o3 = __hmul2(__hsub2(*reinterpret_cast<__half2*>(&v[3]), bhi), s3);
-  r[0] = *reinterpret_cast<const uint32_t*>(&o0);
-  r[1] = *reinterpret_cast<const uint32_t*>(&o1);
-  r[2] = *reinterpret_cast<const uint32_t*>(&o2);
-  r[3] = *reinterpret_cast<const uint32_t*>(&o3);
-}
-
-// The two blocks of a pair -> the two 16-byte chunks (rows g and g + 8 of the block) of an 8-position chunk.
-// `word0` / `word1` are the pair's two blocks (dense: the same word, the second shifted by 8).
-template <bool DENSE>
-__device__ __forceinline__ void dequant_pair_store(const XtMagic& k, const uint2& w, const __half2 (&sa)[4], const __half2 (&sb)[4], unsigned char* dst) {
-  uint32_t r0[4], r1[4];
-  dequant_block<DENSE>(k, w.x, sa[0], sb[0], sa[1], sb[1], r0);
-  dequant_block<DENSE>(k, DENSE ? w.x >> 8 : w.y, sa[2], sb[2], sa[3], sb[3], r1);
-  *reinterpret_cast<uint4*>(dst) = make_uint4(r0[0], r0[2], r1[0], r1[2]);
-  *reinterpret_cast<uint4*>(dst + 128) = make_uint4(r0[1], r0[3], r1[1], r1[3]);
-}
-
-// silu(g) * u = g * u / (1 + e^-g), with e^-g as 2^(-g log2 e); where that power is subnormal and flushed to zero it could not
-// have changed the sum 1 + e^-g
-__device__ __forceinline__ float silu_mul(float g, float u) {
-  float e, r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-1.4426950408889634f * g));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
-  return g * u * r;
+// The two blocks of a pair -> the two 16-byte chunks (rows g and g + 8 of the block) of an 8-position chunk.  s[4]: scales of
+// row g and of row g + 8, positions 0-7 and 8-15 (a[]) of the first block, b[] of the second.
+__device__ __forceinline__ void xt_convert(const DqMagic& k, const XtFields& f, const uint2& w, __half2 a0, __half2 a1, __half2 a2, __half2 a3, __half2 b0,
+                                           __half2 b1, __half2 b2, __half2 b3, unsigned char* dst) {
+  const uint32_t y = f.nib ? w.y : w.x >> 8, xs = w.x >> f.shift, ys = y >> f.shift;
+  *reinterpret_cast<uint4*>(dst) = make_uint4(xt_weight(w.x, f.mlo, k.lo, f.blo, a0), xt_weight(xs, f.mlo, k.lo, f.blo, a2),
+                                              xt_weight(y, f.mlo, k.lo, f.blo, b0), xt_weight(ys, f.mlo, k.lo, f.blo, b2));
+  *reinterpret_cast<uint4*>(dst + 128) = make_uint4(xt_weight(w.x, f.mhi, k.hi, f.bhi, a1), xt_weight(xs, f.mhi, k.hi, f.bhi, a3),
+                                                    xt_weight(y, f.mhi, k.hi, f.bhi, b1), xt_weight(ys, f.mhi, k.hi, f.bhi, b3));
 }
 
 struct XtSmem {
   unsigned char* act;     // [2][nchunks][nt rows] canonical K-major, 16-byte chunks
-  unsigned char* turn;    // [8 epilogue warps][XT_TURN_BYTES]
+  unsigned char* z;       // 128 rows: [8 epilogue warps][XT_TURN_BYTES]; 64 rows: [2][16 chunks][64 rows]
   unsigned char* ring;    // [2 pipelines][ring][XT_SLOT_BYTES]
   int* prefix;            // [E + 1] items before each expert
   unsigned char* tab;     // [2 items] token-side table of the item's expert (TokTab)
 };
 
 __host__ __device__ inline size_t xt_act_bytes(int max_slots, int nt) { return static_cast<size_t>(2) * (max_slots / 8) * xt_chunk_stride(nt); }
-__host__ __device__ inline size_t xt_smem_bytes(int max_slots, int num_experts, int tab_bytes, int nt, int ring) {
-  size_t o = align_up_c(xt_act_bytes(max_slots, nt), 128) + XT_EPI_WARPS * XT_TURN_BYTES;
-  o += static_cast<size_t>(2 * ring) * XT_SLOT_BYTES;
+__host__ __device__ inline size_t xt_smem_bytes(int max_slots, int num_experts, int tab_bytes, int nt, int rows) {
+  size_t o = align_up_c(xt_act_bytes(max_slots, nt), 128) + xt_z_or_turn_bytes(rows);
+  o += static_cast<size_t>(2 * xt_ring(rows)) * XT_SLOT_BYTES;
   o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);     // items before each expert
   o += static_cast<size_t>(2) * tab_bytes;
   // the MMAs read 128 operand rows whatever nt is: rows past nt of the last chunk lie in what follows the operand
@@ -222,7 +207,7 @@ struct XtArgs {
   float* rank_accum;
   long long* acc64;
   int* status;
-  int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, ring_log2, gu_bufs, tab_bytes;
+  int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, gu_bufs, tab_bytes;
   int wait_limit_us;
   int vec_add;            // every row of rank_accum starts on a 16-byte boundary (and takes fp32 adds)
 };
@@ -276,6 +261,8 @@ struct XtPre {
   uint4 s[2];
 };
 
+// WIDE: more than 256 row slots a matrix; a step then has more stages than converter warps.
+template <int ROWS, bool WIDE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_constant__ XtArgs A) {
   extern __shared__ __align__(128) unsigned char xt_raw[];
   __shared__ __align__(8) XtBars bars;
@@ -285,9 +272,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
   volatile int* abort_flag = abort_flag_s;
   const int warp = tc::warp_index(), lane = threadIdx.x & 31;
   const int rank = static_cast<int>(tc::cluster_rank()), pair = static_cast<int>(blockIdx.x) >> 1, n_pairs = static_cast<int>(gridDim.x) >> 1;
-  const int nt = A.nt, ring = 1 << A.ring_log2, h_rank = A.h_rank, num_experts = A.num_experts;
+  constexpr uint32_t ring = xt_ring(ROWS);
+  const int nt = A.nt, h_rank = A.h_rank, num_experts = A.num_experts;
   const int cs = xt_chunk_stride(nt);     // bytes between 8-position chunks of act
-  const int n_chunks = A.n_tiles * (N_TILE / XT_CHUNK);
+  constexpr int CH = xt_chunk(ROWS), PER_TILE = N_TILE / CH, G_STRIDE = xt_g_stride(ROWS);
+  const int n_chunks = A.n_tiles * PER_TILE;
   const uint32_t act_m_bytes = static_cast<uint32_t>(A.max_slots / 8) * cs;
   const TokTab lay(h_rank, A.max_slots);
   XtSmem sm;
@@ -295,7 +284,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
     unsigned char* base = xt_raw;
     sm.act = base;
     size_t o = align_up_c(xt_act_bytes(A.max_slots, nt), 128);
-    sm.turn = base + o; o += XT_EPI_WARPS * XT_TURN_BYTES;
+    sm.z = base + o; o += xt_z_or_turn_bytes(ROWS);
     sm.ring = base + o; o += static_cast<size_t>(2 * ring) * XT_SLOT_BYTES;
     sm.prefix = reinterpret_cast<int*>(base + o);
     o += align_up_c(static_cast<size_t>(num_experts + 1) * 4, 128);
@@ -353,7 +342,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
   const uint32_t lead_bars = tc::cluster_map(tc::smem_u32(&bars), 0);      // the barriers of the CTA that issues the MMAs
   auto lead = [&](const uint64_t* bar) { return lead_bars + static_cast<uint32_t>(reinterpret_cast<const char*>(bar) - reinterpret_cast<const char*>(&bars)); };
   // tensor memory: gu_bufs x (gate 64 columns, up 64 columns), then the down product's slot tiles of 128 columns
-  const uint32_t d_down = tmem_base + A.gu_bufs * 2 * XT_CHUNK;
+  const uint32_t d_down = tmem_base + A.gu_bufs * 2 * XT_ACC;
   // the down product of a chunk is issued `lag` chunks late: one where tensor memory holds two gate/up accumulator pairs
   const int lag = A.gu_bufs - 1;
 
@@ -373,25 +362,28 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
   if (warp < XT_EPI_WARPS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XT_REGS_EPI));
     // -------------------------------------------------------------------- epilogue
-    // warp = (TMEM lane quarter q: tokens 32 q .. 32 q + 31, half of the chunk's 64 columns); a thread owns a token.
-    const int q = warp & 3, half = warp >> 2, n = 32 * q + lane;
+    // warp = (TMEM lane quarter q, half of the columns there); a thread owns a token.  128 rows: quarter q is tokens 32 q ..
+    // 32 q + 31.  64 rows: lanes 64-127 hold the same tokens as lanes 0-63 and the upper half of every product's columns.
+    const int q = warp & 3, half = warp >> 2, upper = ROWS > 64 ? 0 : q >> 1, n0 = 32 * (ROWS > 64 ? q : q & 1), n = n0 + lane;
     const uint32_t lane_sel = static_cast<uint32_t>(32 * q) << 16;
-    unsigned char* turn = sm.turn + warp * XT_TURN_BYTES;
+    // four runs of 512 bytes that no other epilogue warp writes
+    unsigned char* turn = ROWS > 64 ? sm.z + warp * XT_TURN_BYTES : sm.z + 4 * (2 * upper + half) * XT_Z_STRIDE + n0 * 16;
+    constexpr int TURN_STEP = ROWS > 64 ? 512 : XT_Z_STRIDE;
     for (int u = pair; u < units.n_units; u += n_pairs, ++round) {
       XT_ITEM_BEGIN
       const int n_tok = item.n;
-      const bool busy = 32 * q < n_tok;                               // any token in this quarter
+      const bool busy = n0 < n_tok;                               // any token in this quarter
       bool ok = true;
       for (int t = 0; t < nchunk && ok; ++t) {
         const uint32_t g = gu_round + t, b = lag ? g & 1u : 0u;
         ok = xt_wait(&bars.gu_done[b], (lag ? g >> 1 : g) & 1u, abort_flag);
         if (!ok) break;
         tc::fence_after_sync();
-        // z in the contraction order of the down weights (pos32): columns 4c .. 4c+3 of tensor memory, two halves each, hold
-        // columns 2c, 2c+1, 2c+8, 2c+9 of both blocks of 16
-        uint32_t zp[16];
         if (busy) {
-          const uint32_t d_gate = tmem_base + 2 * b * XT_CHUNK + lane_sel + 32 * half, d_up = d_gate + XT_CHUNK;
+          // z in the contraction order of the down weights (pos32): piece c of eight holds columns 2c, 2c+1, 2c+8, 2c+9 of both
+          // of this warp's blocks of 16
+          uint32_t zp[16];
+          const uint32_t d_gate = tmem_base + 2 * b * XT_ACC + lane_sel + 32 * half, d_up = d_gate + XT_ACC;
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {          // 16 columns at a time: 32 of both would hold 64 registers
             float gv[16], uv[16];
@@ -403,7 +395,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
               zp[4 * (i & 3) + 2 * hh + (i >> 2)] = *reinterpret_cast<const uint32_t*>(&h2);
             }
           }
-          tc::tmem_st16(d_gate, zp);                // over the first half of the gate sums that this warp has read
+          if (ROWS > 64) {
+            tc::tmem_st16(d_gate, zp);              // over the first half of the gate sums that this warp has read
+          } else {
+            unsigned char* dst = sm.z + b * XT_Z_BYTES + 4 * (2 * upper + half) * XT_Z_STRIDE + n * 16;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4*>(dst + c * XT_Z_STRIDE) = make_uint4(zp[4 * c], zp[4 * c + 1], zp[4 * c + 2], zp[4 * c + 3]);
+            tc::fence_async_smem();
+          }
         }
         tc::fence_before_sync();
         __syncwarp();
@@ -421,9 +420,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
         // 32-byte sector per lane and instruction.  32 slots of 16 tokens at a time go through shared memory, so that an instruction adds 128 bytes of each of four tokens (128 KB in 5.1 K cycles of an SM, 8.1 K
         // with 64 bytes of eight).  Octets of slots that are not an aligned octet of ranks, rows that do not start on
         // 16-byte boundaries, and the deterministic mode add element by element.
-        for (int s0 = 32 * half; s0 < nslots_d; s0 += 64) {
+        for (int col = 32 * half; col < XT_MAX_SLOTS; col += ROWS > 64 ? 64 : 128) {
+          // 64 rows: 64 columns of a 128-slot tile, which are its lower or its upper slots
+          const int s0 = col + 64 * upper;
+          if (s0 >= nslots_d) break;
           float v[32];
-          tc::tmem_ld32(d_down + lane_sel + s0, v);
+          tc::tmem_ld32(d_down + lane_sel + col, v);
           const bool whole = s0 + 16 < nslots_d;          // the matrix may end after 16 of the 32 slots
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
@@ -431,13 +433,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
             v[i] *= sv.x * rw; v[i + 1] *= sv.y * rw; v[i + 2] *= sv.z * rw; v[i + 3] *= sv.w * rw;
           }
           // piece c (four slots) of token row r of sixteen, in an order that puts a row's eight pieces into distinct banks
-          auto at = [&](int c, int r) { return turn + (16 * c + (r ^ c)) * 16; };
+          auto at = [&](int c, int r) { return turn + (c >> 1) * TURN_STEP + (16 * (c & 1) + (r ^ c)) * 16; };
           const int piece = lane & 7, o = piece >> 1;
           const int r0 = A.vec_add && (o < 2 || whole) ? oct_d[(s0 >> 3) + o] : -1;
           const uint32_t odd = __ballot_sync(0xffffffffu, r0 < 0) & 0x55u;      // octets (by their first piece) that go element by element
 #pragma unroll
           for (int ph = 0; ph < 2; ++ph) {
-            const int first = 32 * q + 16 * ph, rows = min(16, n_tok - first);
+            const int first = n0 + 16 * ph, rows = min(16, n_tok - first);
             if (rows <= 0) break;
             __syncwarp();                            // the pieces before have been read
             if ((lane >> 4) == ph) {
@@ -480,18 +482,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
   } else if (warp < XT_DQ_WARP0 + XT_DQ_WARPS) {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(XT_REGS_DQ));
     // -------------------------------------------------------------------- activation operand and converters
-    // Team 0 (six warps) feeds pipeline 0, team 1 pipeline 1.  Step t of an item is `n` stages of a team: a stage per 64
-    // slots (two pairs of blocks) of chunk t's gate (up) product, then two stages (64 slots x 32 columns each) per 128-slot
-    // tile of chunk t - lag's down product; stages 2 i and 2 i + 1 share a ring slot.  Warp w of the team takes stages w,
-    // w + 6, ... of every step: at 256 slots a matrix that is one stage, the same of every chunk, whose addresses and kinds of
-    // words are worked out once per item.  A stage is four 16 x 32 blocks; lane (g, t4) turns its words of each into two
+    // Team 0 (six warps) feeds pipeline 0, team 1 pipeline 1.  Step t of an item is `n` stages of a team: a stage per two pairs
+    // of blocks (64 rows: per pair) of chunk t's gate (up) product, then a stage (64 slots x 32 columns) per 32 columns and
+    // 128-slot tile of chunk t - lag's down product; stages 2 i and 2 i + 1 share a ring slot.  Warp w of the team takes stages w,
+    // w + 6, ... of every step: at 256 slots a matrix and 128 rows that is one stage, the same of every chunk, whose addresses and
+    // kinds of words are worked out once per item.  A stage is four 16 x 32 blocks; lane (g, t4) turns its words of each into two
     // 16-byte pieces.
     const int dw = warp - XT_DQ_WARP0;
     const int team = dw / XT_TEAM, wt = dw - team * XT_TEAM, g = lane >> 2, t4 = lane & 3;
     uint64_t* w_empty = &bars.w_empty[team * ring];
     const uint32_t w_full = lead(&bars.w_full[team * ring]);
     unsigned char* ring0 = sm.ring + team * ring * XT_SLOT_BYTES;
-    const XtMagic magic;
+    const DqMagic magic;
     uint32_t item_seq = 0;                    // ring slots that the pipeline has used before this item
     uint32_t seen = 0;                        // every use of a slot before this one is known to be multiplied
     for (int u = pair; u < units.n_units; u += n_pairs, ++round) {
@@ -574,6 +576,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
             }
           }
         }
+        // Every ring slot of the item before is multiplied; known before this item may begin, for the parities' sake (see acquire).
+        if (round > 0 && !xt_wait(&bars.down_done, (round - 1) & 1u, abort_flag)) break;
+        seen = item_seq;
         tc::fence_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive_cluster(lead(&bars.act_ready));
@@ -581,133 +586,145 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
       // everything about the expert in registers: the barriers' memory clobbers would have it read again every stage
       const int chunk0 = item.chunk0, nblk_d = fe.m[2].nslots >> 4, n_mt = (nblk_d + 7) >> 3;
       const int npairs = fe.m[team].nslots >> 5, nib_pairs = fe.m[team].nblk[0] >> 1, nib_d = fe.m[2].nblk[0];
-      const int slots_gu = (npairs + 3) >> 2, slots_d = (n_mt - team + 1) >> 1, n = 2 * (slots_gu + slots_d);
+      constexpr int GP = ROWS > 64 ? 2 : 1, DS = CH / 32;       // pairs of a gate/up stage, stages of a down tile
+      const int slots_gu = (npairs + 2 * GP - 1) / (2 * GP), slots_d = ((n_mt - team + 1) >> 1) * (DS / 2), per_step = slots_gu + slots_d;
       const int unit_bytes = fe.unit_bytes;
       const unsigned char* unit0 = A.arena + fe.unit_base;
       const int scale_gu = fe.sec_off[team] + t4 * 16, words_gu = fe.sec_off[3 + team], scale_d = fe.sec_off[2] + g * 4, words_d = fe.sec_off[5];
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&bars.item_free[ib]);
-      // The stage at hand: `kind` bit p: words of pair p (down: of block p) are nibbles; offsets of its words and scales in
-      // the unit block, `odd`: in the second chunk of a tile
-      int i = wt, t = 0, kind = 0, live = 0, w_off[2], s_off = 0, dst_off = 0;
-      bool gu = true;
-      auto set_up = [&]() {
-        gu = i < 2 * slots_gu;
-        if (gu) {
-          live = min(2, npairs - 2 * i);      // pairs (an odd last stage has an empty partner in its slot)
-          s_off = scale_gu + 2 * i * 64;
-          kind = 0;
+      // A stage: `kind` bit p: words of pair p (down: of block p) are nibbles; `live`: its pairs (blocks); offsets of its words and
+      // scales in the unit block and of its pieces in a ring slot.
+      struct Stage { int kind, live, w_off[2], s_off, dst_off; bool gu; };
+      auto describe = [&](int i) -> Stage {
+        Stage st;
+        st.gu = i < 2 * slots_gu;
+        if (st.gu) {
+          st.live = min(GP, npairs - GP * i);    // an odd last stage has an empty partner in its slot
+          st.s_off = scale_gu + GP * i * 64;
+          st.kind = 0;
 #pragma unroll
-          for (int p = 0; p < 2; ++p) {
-            const int pr = 2 * i + p;
+          for (int p = 0; p < GP; ++p) {
+            const int pr = GP * i + p;
             const bool nib = pr < nib_pairs;
-            kind |= nib ? 1 << p : 0;
-            w_off[p] = words_gu + (nib ? pr * 2048 + 2 * rank * 256 + lane * 8 : nib_pairs * 2048 + (pr - nib_pairs) * 1024 + 2 * rank * 128 + lane * 4);
+            st.kind |= nib ? 1 << p : 0;
+            st.w_off[p] = words_gu + (nib ? pr * 2048 + 4 / GP * rank * 256 + lane * 8 : nib_pairs * 2048 + (pr - nib_pairs) * 1024 + 4 / GP * rank * 128 + lane * 4);
           }
-          dst_off = (i & 1) * 8 * XT_G_STRIDE + t4 * XT_G_STRIDE + g * 16;
+          st.dst_off = (i & 1) * 4 * GP * G_STRIDE + t4 * G_STRIDE + g * 16;
         } else {
-          const int j = i - 2 * slots_gu, mb0 = 8 * (team + 2 * (j >> 1)) + 4 * rank;
-          live = min(4, nblk_d - mb0);        // blocks; slots past the matrix: accumulator columns that nobody reads
-          const int n_nib = min(max(nib_d - mb0, 0), 4);
-          kind = (1 << n_nib) - 1;
-          s_off = scale_d + mb0 * 32;
-          w_off[0] = words_d + (mb0 * 4 + (j & 1)) * 256 + lane * 8;                                              // of a nibble block
-          w_off[1] = words_d + nib_d * 1024 + ((mb0 - nib_d) * 4 + (j & 1)) * 128 + lane * 4;                     // of a dense block
-          dst_off = (j & 1) * 4 * XT_D_STRIDE + t4 * XT_D_STRIDE + g * 16;
+          const int j = i - 2 * slots_gu, mb0 = 8 * (team + 2 * (j / DS)) + 4 * rank, pr = j % DS;
+          st.live = min(4, nblk_d - mb0);        // blocks; slots past the matrix: accumulator columns that nobody reads
+          st.kind = (1 << min(max(nib_d - mb0, 0), 4)) - 1;
+          st.s_off = scale_d + mb0 * 32;
+          st.w_off[0] = words_d + (mb0 * 4 + pr) * 256 + lane * 8;                                              // of a nibble block
+          st.w_off[1] = words_d + nib_d * 1024 + ((mb0 - nib_d) * 4 + pr) * 128 + lane * 4;                     // of a dense block
+          st.dst_off = (j & 1) * 4 * XT_D_STRIDE + t4 * XT_D_STRIDE + g * 16;
         }
+        return st;
       };
-      auto fetch = [&](XtPre& p) {
-        const int ch = chunk0 + (gu ? t : t - lag), odd = ch & 1;
-        const unsigned char* b = unit0 + static_cast<int64_t>(ch >> 1) * unit_bytes;
-        if (gu) {
+      // its words and scales of chunk `c` of the item, whatever their kinds
+      auto fetch = [&](const Stage& st, int c, XtPre& p) {
+        const int ch = chunk0 + c, odd = ch % PER_TILE;
+        const unsigned char* b = unit0 + static_cast<int64_t>(ch / PER_TILE) * unit_bytes;
+        if (st.gu) {
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            if (q >= live) break;
-            p.s[q] = __ldg(reinterpret_cast<const uint4*>(b + s_off + q * 64));
-            if (kind & (1 << q)) {
-              const uint2* w = reinterpret_cast<const uint2*>(b + w_off[q] + odd * 1024);
-              p.w[2 * q] = __ldg(w);
-              p.w[2 * q + 1] = __ldg(w + 32);
+          for (int q = 0; q < GP; ++q) {
+            if (q >= st.live) break;
+            p.s[q] = __ldg(reinterpret_cast<const uint4*>(b + st.s_off + q * 64));
+            if (st.kind & (1 << q)) {
+              const uint2* w = reinterpret_cast<const uint2*>(b + st.w_off[q] + odd * 1024);
+#pragma unroll
+              for (int x = 0; x < 4 / GP; ++x) p.w[4 / GP * q + x] = __ldg(w + 32 * x);
             } else {
-              const uint32_t* w = reinterpret_cast<const uint32_t*>(b + w_off[q] + odd * 512);
-              p.w[2 * q].x = __ldg(w);
-              p.w[2 * q + 1].x = __ldg(w + 32);
+              const uint32_t* w = reinterpret_cast<const uint32_t*>(b + st.w_off[q] + odd * 512);
+#pragma unroll
+              for (int x = 0; x < 4 / GP; ++x) p.w[4 / GP * q + x].x = __ldg(w + 32 * x);
             }
           }
         } else {
           uint32_t* ps = reinterpret_cast<uint32_t*>(p.s);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            if (v >= live) break;
-            ps[v] = __ldg(reinterpret_cast<const uint32_t*>(b + s_off + v * 32));
-            if (kind & (1 << v)) p.w[v] = __ldg(reinterpret_cast<const uint2*>(b + w_off[0] + odd * 512 + v * 1024));
-            else p.w[v].x = __ldg(reinterpret_cast<const uint32_t*>(b + w_off[1] + odd * 256 + v * 512));
+            if (v >= st.live) break;
+            ps[v] = __ldg(reinterpret_cast<const uint32_t*>(b + st.s_off + v * 32));
+            if (st.kind & (1 << v)) p.w[v] = __ldg(reinterpret_cast<const uint2*>(b + st.w_off[0] + odd * 512 + v * 1024));
+            else p.w[v].x = __ldg(reinterpret_cast<const uint32_t*>(b + st.w_off[1] + odd * 256 + v * 512));
           }
         }
       };
-      auto convert = [&](const XtPre& p, unsigned char* dst) {
-        if (gu) {
+      auto convert = [&](const Stage& st, const XtPre& p, unsigned char* dst) {
+        if (st.gu) {
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            if (q >= live) break;
+          for (int q = 0; q < GP; ++q) {
+            if (q >= st.live) break;
             const __half2* sp = reinterpret_cast<const __half2*>(&p.s[q]);
-            const __half2 sc[4] = {sp[0], sp[1], sp[2], sp[3]};
-            unsigned char* d = dst + q * 4 * XT_G_STRIDE;
-            if (kind & (1 << q)) {
+            const XtFields f(st.kind & (1 << q));
 #pragma unroll
-              for (int x = 0; x < 2; ++x) dequant_pair_store<false>(magic, p.w[2 * q + x], sc, sc, d + x * 256);
-            } else {
-#pragma unroll
-              for (int x = 0; x < 2; ++x) dequant_pair_store<true>(magic, p.w[2 * q + x], sc, sc, d + x * 256);
-            }
+            for (int x = 0; x < 4 / GP; ++x)
+              xt_convert(magic, f, p.w[4 / GP * q + x], sp[0], sp[0], sp[1], sp[1], sp[2], sp[2], sp[3], sp[3], dst + q * 4 * G_STRIDE + x * 256);
           }
         } else {
           const __half2* sp = reinterpret_cast<const __half2*>(p.s);
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            if (v >= live) break;
+            if (v >= st.live) break;
             const __half2 lo = __low2half2(sp[v]), hi = __high2half2(sp[v]);
-            const __half2 sa[4] = {lo, lo, lo, lo}, sb[4] = {hi, hi, hi, hi};
-            if (kind & (1 << v)) dequant_pair_store<false>(magic, p.w[v], sa, sb, dst + v * 256);
-            else dequant_pair_store<true>(magic, p.w[v], sa, sb, dst + v * 256);
+            xt_convert(magic, XtFields(st.kind & (1 << v)), p.w[v], lo, hi, lo, hi, lo, hi, lo, hi, dst + v * 256);
           }
         }
       };
-      // this warp's next stage; false past the last one
+      // The use `seq` of a ring slot may begin once use seq - ring is multiplied.  The parity of the slot's barrier tells that
+      // from the use before only if the warp knows use seq - 2 ring to be multiplied: a warp's uses lie at most a ring apart,
+      // and the first one of an item less than two rings behind the last one of the item before.
+      auto acquire = [&](uint32_t seq) -> bool {
+        if (static_cast<int>(seq - seen) < static_cast<int>(ring)) return true;
+        const uint32_t before = seq - ring;
+        seen = before + 1;
+        return xt_wait(&w_empty[before % ring], (before / ring) & 1u, abort_flag);
+      };
+      // Stage i of step t.  Up to 256 slots a warp takes the same stages of every step (the ring covers what lies between them),
+      // so that one which takes a single stage describes it once; beyond, the item's stages in turn, three ring slots apart.
+      bool ok = true;
+      int i = WIDE ? wt - XT_TEAM : wt, t = 0;
       auto step = [&]() -> bool {
-        for (;;) {
-          i += XT_TEAM;
-          if (i >= n) { i = wt; ++t; }
-          if (t >= nchunk + lag) return false;
-          if (i < 2 * slots_gu ? t < nchunk : t >= lag) return true;
+        if (WIDE) {
+          i += XT_TEAM - (t == nchunk ? 2 * slots_gu : 0);
+          for (int nt = 0; t < nchunk + lag; ++t, i -= nt) {
+            nt = (t < nchunk ? 2 * slots_gu : 0) + (t >= lag ? 2 * slots_d : 0);
+            if (i < nt) break;
+          }
+          if (t == nchunk) i += 2 * slots_gu;
+        } else {
+          do {
+            i += XT_TEAM;
+            if (i >= 2 * per_step) { i = wt; ++t; }
+          } while (t < nchunk + lag && !(i < 2 * slots_gu ? t < nchunk : t >= lag));
         }
+        return t < nchunk + lag;
       };
       XtPre p;
-      bool ok = true, more = wt < n;
-      if (more && !(wt < 2 * slots_gu || lag == 0)) more = step();
-      if (more) { set_up(); fetch(p); }
+      Stage st;
+      bool more = WIDE ? step() : i < 2 * per_step && (i < 2 * slots_gu || lag == 0 || step());
+      if (more) {
+        st = describe(i);
+        fetch(st, st.gu ? t : t - lag, p);
+      }
       while (more) {
         // the use of a ring slot that this stage fills: steps before t, then this step's order (the last one has no gate / up)
-        const uint32_t pos = item_seq + t * (slots_gu + slots_d) - (t > 0 && lag ? slots_d : 0) + (i >> 1) - (t == nchunk ? slots_gu : 0);
-        // A parity tells a phase from its neighbours only: uses further apart than the ring are waited for one by one.
-        while (static_cast<int>(pos - seen) >= ring) {
-          const uint32_t last = min(seen + ring - 1, pos - ring);
-          if (!(ok = xt_wait(&w_empty[last & (ring - 1)], (last >> A.ring_log2) & 1u, abort_flag))) break;
-          seen = last + 1;
-        }
-        if (!ok) break;
-        convert(p, ring0 + (pos & (ring - 1)) * XT_SLOT_BYTES + dst_off);
+        const uint32_t pos = item_seq + t * per_step - (t > 0 && lag ? slots_d : 0) + (i >> 1) - (t == nchunk ? slots_gu : 0);
+        if (!(ok = acquire(pos))) break;
+        convert(st, p, ring0 + (pos % ring) * XT_SLOT_BYTES + st.dst_off);
         const int i_was = i;
         more = step();
         if (more) {
-          if (i != i_was) set_up();
-          fetch(p);                         // on its way while the converted stage is published and the next one is waited for
+          if (i != i_was) st = describe(i);
+          fetch(st, st.gu ? t : t - lag, p);      // on its way while the converted stage is published and the next one is waited for
         }
         tc::fence_async_smem();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive_cluster(w_full + (pos & (ring - 1)) * 8);
+        if (lane == 0) tc::mbar_arrive_cluster(w_full + (pos % ring) * 8);
       }
-      item_seq += nchunk * (slots_gu + slots_d);
+      item_seq += nchunk * per_step;
       if (!ok) break;
     }
   } else {
@@ -724,7 +741,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
       if (!tc::mbar_wait(&bars.item_full[ib], (round >> 1) & 1u)) { xt_give_up(abort_flag); break; }
       // the weights on their way to L2, one tile per lane, every other one by this CTA (sizes and offsets are multiples of 16 bytes)
       const FastExpert& fe = reinterpret_cast<const TokTabHead*>(sm.tab + ib * lay.bytes)->fe;
-      const int t0 = items[ib].chunk0 >> 1, t1 = (items[ib].chunk0 + items[ib].nchunk + 1) >> 1;
+      const int t0 = items[ib].chunk0 / PER_TILE, t1 = (items[ib].chunk0 + items[ib].nchunk + PER_TILE - 1) / PER_TILE;
       for (int t = t0 + 2 * lane + rank; t < t1; t += 64)
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(A.arena + fe.unit_base + static_cast<int64_t>(t) * fe.unit_bytes),
                      "r"(fe.unit_bytes)
@@ -735,14 +752,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
     // -------------------------------------------------------------------- MMA issue for both CTAs, one thread per pipeline
     // The whole warp waits (a lone waiting lane wakes up several times slower); one issues.
     const int pl = warp - XT_MMA_WARP0;
-    const uint32_t idesc_gu = tc::idesc_f16(256, 64), idesc_d = tc::idesc_f16(256, 128);
+    const uint32_t idesc_gu = tc::idesc_f16(2 * ROWS, CH), idesc_d = tc::idesc_f16(2 * ROWS, 128);
     // descriptors: constant upper part, start-address field advanced per block
     const uint64_t a_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.act) + pl * act_m_bytes, cs, 128);
     const uint32_t ring0 = tc::smem_u32(sm.ring) + pl * ring * XT_SLOT_BYTES;
-    const uint64_t gu_desc = tc::smem_desc_kmajor(ring0, XT_G_STRIDE, 128), dn_desc = tc::smem_desc_kmajor(ring0, XT_D_STRIDE, 128);
+    const uint64_t gu_desc = tc::smem_desc_kmajor(ring0, G_STRIDE, 128), dn_desc = tc::smem_desc_kmajor(ring0, XT_D_STRIDE, 128);
     uint64_t* w_full = &bars.w_full[pl * ring];
     uint64_t* w_empty = &bars.w_empty[pl * ring];
     const uint32_t a_step = (2 * cs) >> 4;       // descriptor units per 16 contraction positions
+    const uint64_t z_desc = tc::smem_desc_kmajor(tc::smem_u32(sm.z), XT_Z_STRIDE, 128);
     uint32_t seq = 0;                            // uses of ring slots so far
     for (int u = pair; u < units.n_units; u += n_pairs, ++round) {
       XT_ITEM_BEGIN
@@ -756,21 +774,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
           const uint32_t g = gu_round + t, b = lag ? g & 1u : 0u, k = lag ? g >> 1 : g;
           if (k >= 1) ok = xt_wait(&bars.z_free[b], (k - 1) & 1u, abort_flag);     // the z written over this accumulator is multiplied
           tc::fence_after_sync();
-          const uint32_t d_acc = tmem_base + (2 * b + pl) * XT_CHUNK;
+          const uint32_t d_acc = tmem_base + (2 * b + pl) * XT_ACC;
           uint64_t ad = a_desc;
-          for (int pr = 0; pr < npairs && ok; pr += 4, ++seq) {
-            const uint32_t sl = seq & (ring - 1);
-            if (!(ok = xt_wait(&w_full[sl], (seq >> A.ring_log2) & 1u, abort_flag))) break;
+          constexpr int SP = ROWS > 64 ? 4 : 2;       // pairs of a slot
+          for (int pr = 0; pr < npairs && ok; pr += SP, ++seq) {
+            const uint32_t sl = seq % ring;
+            if (!(ok = xt_wait(&w_full[sl], (seq / ring) & 1u, abort_flag))) break;
             if (tc::elect_one()) {
               const uint64_t bd = gu_desc + ((sl * XT_SLOT_BYTES) >> 4);
 #pragma unroll
-              for (int h = 0; h < 8; ++h)         // 16 slots each
+              for (int h = 0; h < 2 * SP; ++h)    // 16 slots each
                 if (h < 2 || pr + (h >> 1) < npairs)
-                  tc::mma_f16_pair(d_acc, ad + h * a_step, bd + ((h * 2 * XT_G_STRIDE) >> 4), idesc_gu, pr > 0 || h > 0 ? 1u : 0u);
+                  tc::mma_f16_pair(d_acc, ad + h * a_step, bd + ((h * 2 * G_STRIDE) >> 4), idesc_gu, pr > 0 || h > 0 ? 1u : 0u);
               tc::mma_commit_pair(&w_empty[sl]);
             }
             __syncwarp();
-            ad += 8 * a_step;
+            ad += 2 * SP * a_step;
           }
           if (!ok) break;
           if (tc::elect_one()) {
@@ -784,20 +803,25 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
           if (t == lag && round > 0) ok = xt_wait(&bars.down_free, (round - 1) & 1u, abort_flag);   // the last item's sums are read out
           if (ok) ok = xt_wait(&bars.z_ready[b], (lag ? g >> 1 : g) & 1u, abort_flag);
           tc::fence_after_sync();
-          const uint32_t d_z = tmem_base + 2 * b * XT_CHUNK;      // columns 0-31 of the chunk, and 32-63 32 columns on
-          for (int mt = pl; mt < n_mt && ok; mt += 2, ++seq) {
-            const uint32_t sl = seq & (ring - 1);
-            if (!(ok = xt_wait(&w_full[sl], (seq >> A.ring_log2) & 1u, abort_flag))) break;
-            if (tc::elect_one()) {
-              const uint64_t bd = dn_desc + ((sl * XT_SLOT_BYTES) >> 4);
+          const uint32_t d_z = tmem_base + 2 * b * XT_ACC;      // columns 0-31 of the chunk, and 32-63 32 columns on
+          for (int mt = pl; mt < n_mt && ok; mt += 2)
+            for (int kp = 0; kp < CH / 64; ++kp, ++seq) {      // 64 columns of z per slot
+              const uint32_t sl = seq % ring;
+              if (!(ok = xt_wait(&w_full[sl], (seq / ring) & 1u, abort_flag))) break;
+              if (tc::elect_one()) {
+                const uint64_t bd = dn_desc + ((sl * XT_SLOT_BYTES) >> 4);
 #pragma unroll
-              for (int h = 0; h < 4; ++h)           // 16 columns of z each
-                tc::mma_f16_pair_ta(d_down + mt * 128, d_z + 32 * (h >> 1) + 8 * (h & 1), bd + ((h * 2 * XT_D_STRIDE) >> 4), idesc_d,
-                                 t > lag || h > 0 ? 1u : 0u);
-              tc::mma_commit_pair(&w_empty[sl]);
+                for (int h = 0; h < 4; ++h) {         // 16 columns of z each
+                  const uint32_t add = t > lag || kp > 0 || h > 0 ? 1u : 0u;
+                  if (ROWS > 64)
+                    tc::mma_f16_pair_ta(d_down + mt * 128, d_z + 32 * (h >> 1) + 8 * (h & 1), bd + ((h * 2 * XT_D_STRIDE) >> 4), idesc_d, add);
+                  else
+                    tc::mma_f16_pair(d_down + mt * 128, z_desc + ((b * XT_Z_BYTES + (4 * kp + h) * 2 * XT_Z_STRIDE) >> 4), bd + ((h * 2 * XT_D_STRIDE) >> 4), idesc_d, add);
+                }
+                tc::mma_commit_pair(&w_empty[sl]);
+              }
+              __syncwarp();
             }
-            __syncwarp();
-          }
           if (ok && tc::elect_one()) {
             tc::mma_commit_pair(&bars.z_free[b]);
             if (t == nchunk + lag - 1) tc::mma_commit_pair(&bars.down_done);
@@ -829,19 +853,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
 // Item size and ring depth for a layer: the first candidate whose activation operand (2 KB per token at 256 row slots per
 // matrix) and stages fit shared memory.  Tensor memory holds 128 columns per gate/up buffer and 128 per 128
 // slots of the down product.
-struct XtPlan { int nt, ring_log2, gu_bufs; size_t smem; };
+// Assignments an expert up to which items of 2 x 64 tokens are taken.  2048 tokens of 128 experts, top 8 (128 each): 59 us against
+// 62 with 2 x 128; 4096 (256 each): 91 against 83; 2048 tokens of 512 experts, top 10 (40 each): 99 against 122; 1024 of 64
+// experts, top 6 (96 each): 46 against 49.
+constexpr int XT_FEW_ROWS = 160;
+struct XtPlan { int nt, gu_bufs; size_t smem; };
 constexpr size_t XT_SMEM_LIMIT = 227 * 1024 - 3072;     // dynamic part: the static part (two item descriptions, barriers) stays below 3 KB
-static bool xt_plan(const bm_layer* L, XtPlan* out) {
-  if (!L->toktab_dev || L->num_experts > XT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > 3 * 128) return false;
+static bool xt_plan(const bm_layer* L, int rows, XtPlan* out) {
+  if (!L->toktab_dev || L->num_experts > XT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > XT_MAX_SLOTS) return false;
   const int n_mt = (L->max_slots + 127) / 128;
-  static const int cand[] = {128, 112, 96, 80, 64, 48, 32, 16};
-  for (const int nt : cand) {
-    for (int lg = 3; lg >= 2; --lg) {
-      const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, TokTab(L->rank_in, L->max_slots).bytes, nt, 1 << lg);
-      if (smem <= XT_SMEM_LIMIT) {
-        *out = XtPlan{nt, lg, n_mt > 2 ? 1 : 2, smem};
-        return true;
-      }
+  for (int nt = rows; nt >= 16; nt -= 16) {
+    const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, TokTab(L->rank_in, L->max_slots).bytes, nt, rows);
+    if (smem <= XT_SMEM_LIMIT) {
+      *out = XtPlan{nt, n_mt > 2 ? 1 : 2, smem};
+      return true;
     }
   }
   return false;
@@ -851,33 +876,41 @@ static bool xt_plan(const bm_layer* L, XtPlan* out) {
 // decode path otherwise).
 bool experts_tc_fits(const bm_layer* L) {
   XtPlan p;
-  return xt_plan(L, &p);
+  return xt_plan(L, 128, &p);
 }
 
-int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
-                      const int32_t* expert_offsets, const float* route_w, int T, float* rank_accum, long long* acc64,
-                      cudaStream_t st) {
-  BM_REQUIRE(L->num_experts <= XT_MAX_E, BM_ERR_UNSUPPORTED, "experts_tc: more than %d experts", XT_MAX_E);
-  BM_REQUIRE(L->intermediate % N_TILE == 0, BM_ERR_UNSUPPORTED, "experts_tc: intermediate size must be a multiple of %d", N_TILE);
-  BM_REQUIRE(L->max_slots <= 3 * 128, BM_ERR_UNSUPPORTED, "experts_tc: %d row slots exceed the tensor-memory budget", L->max_slots);
-  BM_REQUIRE(L->rank_in % 8 == 0 && ((reinterpret_cast<uintptr_t>(h_gate) | reinterpret_cast<uintptr_t>(h_up)) & 15u) == 0,
-             BM_ERR_UNSUPPORTED, "experts_tc: rank-space rows must be 16-byte aligned (rank %d)", L->rank_in);
-  XtPlan plan;
-  BM_REQUIRE(xt_plan(L, &plan), BM_ERR_UNSUPPORTED, "experts_tc: the layer's largest expert does not fit in shared memory");
-  static PerDeviceOnce attr_once;
+template <int ROWS, bool WIDE>
+static int xt_launch(XtArgs a, size_t smem, cudaStream_t st) {
+  static PerDeviceOnce once;
   static int grids[MAX_DEVICES];
   int dev = -1;
   BM_CUDA(cudaGetDevice(&dev));
   BM_REQUIRE(dev >= 0 && dev < MAX_DEVICES, BM_ERR_UNSUPPORTED, "experts_tc: device ordinal %d out of range", dev);
-  if (!attr_once.is_done(dev)) {
-    BM_CUDA(cudaFuncSetAttribute(experts_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(XT_SMEM_LIMIT)));
+  if (!once.is_done(dev)) {
+    BM_CUDA(cudaFuncSetAttribute(experts_tc_kernel<ROWS, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(XT_SMEM_LIMIT)));
     BM_CUDA(cudaDeviceGetAttribute(&grids[dev], cudaDevAttrMultiProcessorCount, dev));
     grids[dev] &= ~1;
     cudaFuncAttributes fa;
-    BM_CUDA(cudaFuncGetAttributes(&fa, experts_tc_kernel));
+    BM_CUDA(cudaFuncGetAttributes(&fa, experts_tc_kernel<ROWS, WIDE>));
     BM_REQUIRE(fa.numRegs >= XT_REGS, BM_ERR_UNSUPPORTED, "experts_tc: built with %d registers per thread, %d expected", fa.numRegs, XT_REGS);
-    attr_once.mark(dev);
+    once.mark(dev);
   }
+  experts_tc_kernel<ROWS, WIDE><<<grids[dev], XT_THREADS, smem, st>>>(a);
+  BM_LAUNCH_CHECK("experts_tc_kernel");
+  return BM_OK;
+}
+
+int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
+                      const int32_t* expert_offsets, const float* route_w, int T, int num_assign, float* rank_accum, long long* acc64,
+                      cudaStream_t st) {
+  BM_REQUIRE(L->num_experts <= XT_MAX_E, BM_ERR_UNSUPPORTED, "experts_tc: more than %d experts", XT_MAX_E);
+  BM_REQUIRE(L->intermediate % N_TILE == 0, BM_ERR_UNSUPPORTED, "experts_tc: intermediate size must be a multiple of %d", N_TILE);
+  BM_REQUIRE(L->max_slots <= XT_MAX_SLOTS, BM_ERR_UNSUPPORTED, "experts_tc: %d row slots exceed the tensor-memory budget", L->max_slots);
+  BM_REQUIRE(L->rank_in % 8 == 0 && ((reinterpret_cast<uintptr_t>(h_gate) | reinterpret_cast<uintptr_t>(h_up)) & 15u) == 0,
+             BM_ERR_UNSUPPORTED, "experts_tc: rank-space rows must be 16-byte aligned (rank %d)", L->rank_in);
+  const int rows = L->max_slots <= 256 && num_assign <= static_cast<int64_t>(XT_FEW_ROWS) * L->num_experts ? 64 : 128;
+  XtPlan plan;
+  BM_REQUIRE(xt_plan(L, rows, &plan), BM_ERR_UNSUPPORTED, "experts_tc: the layer's largest expert does not fit in shared memory");
   XtArgs a{};
   a.toktab = L->toktab_dev;
   a.tab_bytes = TokTab(L->rank_in, L->max_slots).bytes;
@@ -889,10 +922,9 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
   a.vec_add = acc64 == nullptr && L->rank_out % 4 == 0 && (reinterpret_cast<uintptr_t>(rank_accum) & 15u) == 0;
   a.wait_limit_us = L->wait_limit_us;
   a.rank_out = L->rank_out; a.T = T; a.num_experts = L->num_experts; a.n_tiles = L->n_tiles; a.max_slots = L->max_slots;
-  a.nt = plan.nt; a.ring_log2 = plan.ring_log2; a.gu_bufs = plan.gu_bufs;
-  experts_tc_kernel<<<grids[dev], XT_THREADS, plan.smem, st>>>(a);
-  BM_LAUNCH_CHECK("experts_tc_kernel");
-  return BM_OK;
+  a.nt = plan.nt; a.gu_bufs = plan.gu_bufs;
+  if (L->max_slots > 256) return xt_launch<128, true>(a, plan.smem, st);
+  return rows > 64 ? xt_launch<128, false>(a, plan.smem, st) : xt_launch<64, false>(a, plan.smem, st);
 }
 
 }  // namespace bm

@@ -34,7 +34,7 @@ int launch_experts_decode(const bm_layer* L, const __half* h_gate, const __half*
                           long long* acc64, cudaStream_t st);
 bool experts_tc_fits(const bm_layer* L);
 int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
-                      const int32_t* expert_offsets, const float* route_w, int T, float* rank_accum, long long* acc64,
+                      const int32_t* expert_offsets, const float* route_w, int T, int num_assign, float* rank_accum, long long* acc64,
                       cudaStream_t st);
 int launch_experts_generic(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
                            const int32_t* expert_offsets, const float* route_w, int T, float* rank_accum,
@@ -525,7 +525,7 @@ static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, con
   const __half* hg = reinterpret_cast<const __half*>(h_gate);
   const __half* hu = reinterpret_cast<const __half*>(h_up);
   if (L->fast_ok && (path == BM_PATH_TENSOR || (path == BM_PATH_AUTO && num_assign > 16 * L->num_experts && experts_tc_fits(L))))
-    rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, rank_accum, acc64, st);
+    rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, num_assign, rank_accum, acc64, st);
   else if (L->fast_ok && (path == BM_PATH_DECODE || (path != BM_PATH_GENERIC && L->dec_ok && num_assign / 8 + L->num_experts < 60000)))
     rc = launch_experts_decode(L, hg, hu, token_indices, expert_offsets, route_weights, T, num_assign, rank_accum, acc64, st);
   else

@@ -41,10 +41,12 @@ def test_packed_experts_match_generic_kernel(rank, inter, counts):
 
 
 # whole rounds of items, so that a pair of CTAs walks several items of several chunks: both CTAs with tokens, one with none,
-# items of one and of 256, ranks of one to three slot tiles and of an odd number of pairs
+# items around 2 x 64 tokens and (many per expert on average) around 2 x 128, ranks of one to three slot tiles and of an odd number
+# of pairs
+@pytest.mark.parametrize("pattern", [(1, 2, 0, 63, 64, 65, 127, 128, 129), (255, 256, 257, 300, 1, 299, 254, 300, 300)])
 @pytest.mark.parametrize("rank,inter", [(64, 384), (96, 128), (256, 256), (328, 256)])
-def test_pairs_walk_several_items(rank, inter):
-    counts = tuple((1, 2, 0, 63, 64, 65, 255, 256, 257)[e % 9] for e in range(210))
+def test_pairs_walk_several_items(rank, inter, pattern):
+    counts = tuple(pattern[e % 9] for e in range(210))
     cfg = synth.tiny(hidden=128, num_experts=len(counts), intermediate=inter, top_k=1, rank=rank)
     layer = synth.to_packed_layer(synth.make_layer(cfg, seed=rank, device=DEV))
     T = 300
