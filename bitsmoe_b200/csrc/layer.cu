@@ -32,6 +32,9 @@ int plan_experts_decode(bm_layer* L);
 int launch_experts_decode(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
                           const int32_t* expert_offsets, const float* route_w, int T, int num_assign, float* rank_accum,
                           long long* acc64, cudaStream_t st);
+int plan_experts_batch(bm_layer* L);
+int launch_experts_batch(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices, const int32_t* expert_offsets,
+                         const float* route_w, int T, float* rank_accum, long long* acc64, cudaStream_t st);
 bool experts_tc_fits(const bm_layer* L);
 int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
                       const int32_t* expert_offsets, const float* route_w, int T, int num_assign, float* rank_accum, long long* acc64,
@@ -352,6 +355,7 @@ extern "C" int bm_layer_create(const bm_layer_desc_t* desc, void* arena, size_t 
     if (rc) { delete L; return rc; }
     L->fast_ok = true;
     rc = plan_experts_decode(L);
+    if (!rc) rc = plan_experts_batch(L);
     if (rc) { delete L; return rc; }
   }
   // host-side objects for the fork/join of routing and basis projection (no device memory)
@@ -524,8 +528,17 @@ static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, con
              "experts_forward: the decode path needs 1- to 4-bit rows and full tiles; this layer has neither");
   const __half* hg = reinterpret_cast<const __half*>(h_gate);
   const __half* hu = reinterpret_cast<const __half*>(h_up);
-  if (L->fast_ok && (path == BM_PATH_TENSOR || (path == BM_PATH_AUTO && num_assign > 16 * L->num_experts && experts_tc_fits(L))))
+  // The kernel by assignments per expert.  Up to 6 most experts need one pass of 8 tokens, and that kernel is the fastest at it
+  // (96 tokens, top 8 of 128 experts: 20.1 us against 24.3; 128 tokens: 31.4 against 24.4); where few experts leave room to cut
+  // every pass along its tiles, up to 8 (80 tokens, top 6 of 64 experts: 1.2 us).  Up to 24 passes of 16 tokens cost less than turning
+  // every expert into tensor-core operands (400 tokens, 25 each: 39 us against 40; 512 tokens, 32 each: 47 against 40).
+  const int64_t per16 = static_cast<int64_t>(num_assign) * 16 / L->num_experts;      // assignments per expert, in sixteenths
+  const int one_pass = 4 * L->num_experts >= L->bat_grid ? 6 : 8;
+  const bool batch = L->bat_ring && per16 > one_pass * 16 && (path == BM_PATH_DECODE ? num_assign / FAST_MAX_TOK + L->num_experts < 60000 : per16 <= 24 * 16);
+  if (L->fast_ok && (path == BM_PATH_TENSOR || (path == BM_PATH_AUTO && per16 > 16 * 16 && !batch && experts_tc_fits(L))))
     rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, num_assign, rank_accum, acc64, st);
+  else if (batch && (path == BM_PATH_AUTO || path == BM_PATH_DECODE))
+    rc = launch_experts_batch(L, hg, hu, token_indices, expert_offsets, route_weights, T, rank_accum, acc64, st);
   else if (L->fast_ok && (path == BM_PATH_DECODE || (path != BM_PATH_GENERIC && L->dec_ok && num_assign / 8 + L->num_experts < 60000)))
     rc = launch_experts_decode(L, hg, hu, token_indices, expert_offsets, route_weights, T, num_assign, rank_accum, acc64, st);
   else

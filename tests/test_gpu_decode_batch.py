@@ -3,7 +3,7 @@ one-call block against the same layer run stage by stage and plain fp32 products
 import pytest
 import torch
 
-from bitsmoe_b200 import synth
+from bitsmoe_b200 import capi, synth
 from bitsmoe_b200.layer import route_build, route_topk
 from tests import helpers
 
@@ -34,6 +34,35 @@ def test_fused_forward_matches_stages(T, E, k):
     logits = synth.router_logits(cfg, T, seed=T + 1, device=DEV)
     y = layer.forward(x, logits, k, True, torch.bfloat16)
     helpers.assert_close(y.cpu(), _staged(layer, x, logits, k, torch.bfloat16, E).cpu(), what=f"T={T} E={E}")
+
+
+# passes of 16: assignments per expert around one and two passes and none at all, on average more than eight; few units, cut along
+# the tiles, and more than one per CTA; ranks whose row slots are an odd number of pairs, are not whole octets, or pass 256
+@pytest.mark.parametrize("rank,inter", [(64, 256), (80, 128), (256, 384), (328, 128)])
+@pytest.mark.parametrize("E", [5, 400])
+def test_passes_of_sixteen_match_generic_kernel(rank, inter, E):
+    counts = [(15, 0, 16, 17, 33, 1, 32, 8)[e % 8] for e in range(E)]
+    T = 64
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=inter, top_k=1, rank=rank)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=rank, device=DEV))
+    gen = torch.Generator(device=DEV).manual_seed(E)
+    tok = torch.cat([torch.sort(torch.randperm(T, generator=gen, device=DEV)[:c]).values for c in counts]).to(torch.int32)
+    off = torch.zeros(E + 1, dtype=torch.int32, device=DEV)
+    off[1:] = torch.tensor(counts, device=DEV).cumsum(0)
+    rw = torch.rand(tok.numel(), generator=gen, device=DEV)
+    hg, hu = layer.basis_project(synth.activations(cfg, T, seed=2, device=DEV, dtype=torch.bfloat16))
+    want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
+    nan = torch.full_like(hg, float("nan"))
+    layer.experts_forward(nan, nan, tok, off, rw)      # what a kernel does not write still holds these
+    got = layer.experts_forward(hg, hu, tok, off, rw)
+    layer.check_status()
+    helpers.assert_close(got.cpu(), want.cpu(), what=f"rank {rank} E {E}")
+    capi.check(capi.lib().bm_layer_set_option(layer._handle, 2, 0))
+    layer.experts_forward(hg, hu, tok, off, rw)
+    with pytest.raises(capi.BitsMoEError, match="bounded wait"):
+        layer.check_status()
+    capi.check(capi.lib().bm_layer_set_option(layer._handle, 2, 2000000))
+    helpers.assert_close(layer.experts_forward(hg, hu, tok, off, rw).cpu(), want.cpu(), what=f"rank {rank} E {E} after a time-out")
 
 
 @pytest.mark.parametrize("T,wdtype,shared", [(1, torch.bfloat16, 0), (5, torch.float16, 48), (64, torch.bfloat16, 200), (70, torch.bfloat16, 48),
