@@ -3,8 +3,8 @@
 //   router logits, h_gate / h_up = x . Vh^T, z = silu(x . Wg^T) * (x . Wu^T) of a shared expert: one launch
 //   (bitsmoe/models/qwen3moe/bitsmoe_block.py:45, :63-64)
 //   y = fp16(rank_accum) . U_down^T (+ z . W_down^T) (+ residual)   (bitsmoe/models/base_block.py:414)
-// A CTA walks 128 x BN output tiles (BN = 256, or 64 when the wide tile would leave most SMs idle).  Per tile, K is
-// streamed in slices of 64 through a ring of stages, both operands K-major with the 128-byte swizzle that the tensor
+// A CTA walks 128 x BN output tiles (BN = 256, or 128 or 64 when the wide tile would leave most SMs idle; a few narrow tiles
+// split K over a cluster of two or four CTAs, whose sums meet in distributed shared memory).  Per tile, K is streamed in slices of 64 through a ring of stages, both operands K-major with the 128-byte swizzle that the tensor
 // map writes and the MMA descriptor reads:
 //   warp 0      producer: cp.async.bulk.tensor (2-D tiles) of the X slice and of two half tiles of W rows -- neighbouring
 //               rows of a stack, or the same rows of a gated pair -- completing on the stage's mbarrier
@@ -13,18 +13,24 @@
 //               accumulator is read out
 //   warps 4-11  epilogue: tcgen05.ld, residual / gated pair, rounding, and 32 x 32 blocks through shared memory into TMA
 //               stores (a lane owns an output row; its own stores would touch 32 rows per instruction)
-//   warps 12-15, 2, 3  only for bf16 / fp32 activations: round the landed X slice to fp16 in place (both MMA operands have to
+//   warps 12-15, 2, 3, and the epilogue warps before the end of a CTA's only tile: only for bf16 / fp32 activations: round the landed X slice to fp16 in place (both MMA operands have to
 //               be fp16: a bf16 A with an fp16 B is not an encodable instruction).  bf16 -> fp16 is element for
 //               element; an fp32 slice is twice as large as its fp16 result, and the eight lanes that hold a row read
 //               the row's 256 bytes before any of them writes its 16-byte piece of the 128-byte result row.
 // Every wait is bounded; a time-out raises the status word.
 //
-// Bound by the tensor pipe at its sustained clock.  16384 tokens, hidden 2048: router of 512 experts, basis pair 2 x 256 and
-// gated pair 2 x 512 with silu as one launch 119 us (1.15 PFLOP/s; as three launches and a pass over z 192), down basis and
-// shared down product 109 -> 59 us; 8192 tokens: basis pair 25 -> 23 us, down basis 30 -> 20 (TMA stores).
+// Small batches are bound by shared memory: a slice of a 128 x 64 tile is written (24 KB), rounded in place (32 KB) and read by the
+// MMA (24 KB), 550 cycles in all at 128 bytes a cycle; fp16 slices take 350, the rate at which an SM gets data from L2.  Basis
+// pair of 300 tokens 14.9 -> 9.3 us (clusters of four), 777 tokens 15.2 -> 11.8 (of two), 2048 tokens 15.7 -> 14.0 (epilogue warps
+// round too).
+//
+// Large ones are bound by the tensor pipe at its sustained clock.  16384 tokens, hidden 2048: router of 512 experts, basis pair
+// 2 x 256 and gated pair 2 x 512 with silu as one launch 119 us (1.15 PFLOP/s; as three launches and a pass over z 192), down basis
+// and shared down product 109 -> 59 us; 8192 tokens: basis pair 25 -> 23 us, down basis 30 -> 20 (TMA stores).
 #include <cuda.h>
 
 #include <cstring>
+#include <utility>
 
 #include "common.cuh"
 #include "tc05.cuh"
@@ -38,13 +44,23 @@ constexpr int GT_SMEM = 225 * 1024;                           // stages and stor
 
 __host__ __device__ constexpr int gt_a_bytes(int xd) { return xd == BM_F32 ? GT_BM * GT_BK * 4 : GT_BM * GT_BK * 2; }
 __host__ __device__ constexpr int gt_stage_bytes(int bn, int xd) { return gt_a_bytes(xd) + bn * GT_BK * 2; }
+// Split contraction: floats between the rows that a CTA receives from one CTA of its cluster (bn / split columns, padded), and
+// what is behind the stages: blocks on their way out, or the received sums.
+__host__ __device__ constexpr int gt_recv_row(int bn, int split) { return bn / split + 4; }
+__host__ __device__ constexpr int gt_tail_bytes(int bn, int split) {
+  return split > 1 ? split * GT_BM * gt_recv_row(bn, split) * 4 : GT_EPI_WARPS * 2 * GT_STORE_BYTES;
+}
 // Ring depth; with rounding a multiple of the number of warp groups that round (2 or 3), see below.
-__host__ __device__ constexpr int gt_stages(int bn, int xd) {
-  const int room = (GT_SMEM - GT_EPI_WARPS * 2 * GT_STORE_BYTES) / gt_stage_bytes(bn, xd);
+__host__ __device__ constexpr int gt_stages(int bn, int xd, int split) {
+  const int room = (GT_SMEM - gt_tail_bytes(bn, split)) / gt_stage_bytes(bn, xd);
   const int fit = room < GT_MAX_STAGES ? room : GT_MAX_STAGES;
   return xd == BM_F16 || fit % 3 == 0 ? fit : fit / 2 * 2;
 }
-__host__ __device__ constexpr int gt_tr_groups(int bn, int xd) { return gt_stages(bn, xd) % 3 == 0 ? 3 : 2; }
+__host__ __device__ constexpr int gt_tr_groups(int bn, int xd, int split) { return gt_stages(bn, xd, split) % 3 == 0 ? 3 : 2; }
+// where the epilogue warps round too: 3, 4 or 2 groups of 4, 3 or 7 of the 14 warps
+__host__ __device__ constexpr int gt_tr_groups_all(int bn, int xd, int split) {
+  return gt_stages(bn, xd, split) % 3 == 0 ? 3 : gt_stages(bn, xd, split) % 4 == 0 ? 4 : 2;
+}
 
 struct GtSeg {
   void* C;
@@ -109,11 +125,17 @@ __device__ __forceinline__ GtTile gt_tile(const GtParams& p, int tile) {
   return t;
 }
 
-template <int BN, int XD>
+// SPLIT > 1: a cluster of SPLIT CTAs per tile, each of which takes its share of the slices; the sums meet in shared memory, where
+// a CTA owns BN / 2 / SPLIT columns of either half of the tile.
+template <int BN, int XD, int SPLIT>
 __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_constant__ GtParams p) {
   constexpr int A_BYTES = gt_a_bytes(XD), A2_BYTES = GT_BM * GT_BK * 2, H_BYTES = BN / 2 * GT_BK * 2, STAGE = A_BYTES + 2 * H_BYTES,
-                NST = gt_stages(BN, XD);
-  constexpr int TR_GROUPS = gt_tr_groups(BN, XD), TR_PER_GROUP = GT_TR_WARPS / TR_GROUPS;
+                NST = gt_stages(BN, XD, SPLIT);
+  constexpr int TR_GROUPS = gt_tr_groups(BN, XD, SPLIT), TR_GROUPS_ALL = gt_tr_groups_all(BN, XD, SPLIT);
+  // one tile per CTA: the epilogue warps have nothing to do before its end, and round slices until then
+  const bool all_round = static_cast<int>(gridDim.x) >= p.ntiles * SPLIT;
+  const int tr_groups = all_round ? TR_GROUPS_ALL : TR_GROUPS;
+  const int tr_per = all_round ? (GT_TR_WARPS + GT_EPI_WARPS) / TR_GROUPS_ALL : GT_TR_WARPS / TR_GROUPS;
   constexpr uint32_t TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
   extern __shared__ unsigned char gt_raw[];
   __shared__ __align__(8) uint64_t loaded[GT_MAX_STAGES], ready[GT_MAX_STAGES], empty[GT_MAX_STAGES], acc_full[2], acc_empty[2];
@@ -123,7 +145,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
   if (threadIdx.x == 0) {
     for (int i = 0; i < GT_MAX_STAGES; ++i) {
       tc::mbar_init(&loaded[i], 1);
-      tc::mbar_init(&ready[i], TR_PER_GROUP);
+      tc::mbar_init(&ready[i], tr_per);
       tc::mbar_init(&empty[i], 1);
     }
     for (int i = 0; i < 2; ++i) {
@@ -133,12 +155,15 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
     tc::mbar_init_fence();
   }
   if (warp == 2) tc::tmem_alloc(&tmem_slot, TMEM_COLS);
+  if (SPLIT > 1) tc::cluster_arrive();           // waited for before anything is sent to another CTA
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
-  const int slices = p.slices + p.slices2;       // of X . W, then of the second contraction
-  const int cta = static_cast<int>(blockIdx.x), grid = static_cast<int>(gridDim.x);
+  // slices of X . W, then of the second contraction: this CTA's share
+  const int all = p.slices + p.slices2, rank = SPLIT > 1 ? static_cast<int>(blockIdx.x) % SPLIT : 0;
+  const int s_first = all * rank / SPLIT, s_end = all * (rank + 1) / SPLIT, slices = s_end - s_first;
+  const int cta = static_cast<int>(blockIdx.x) / SPLIT, grid = static_cast<int>(gridDim.x) / SPLIT;
   bool ok = true;
 
   if (warp == 0) {
@@ -149,7 +174,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
       const GtSeg& sg = p.seg[t.si];
       const CUtensorMap *mw = &p.w[sg.map_w], *mu = sg.glu ? &p.w[sg.map_up] : mw;
       const int nu = sg.glu ? t.n0 : t.n0 + BN / 2;
-      for (int s = 0; s < slices; ++s) {
+      for (int s = s_first; s < s_end; ++s) {
         if (!(ok = tc::mbar_wait(&empty[st], ph ^ 1))) break;
         if (tc::elect_one()) {
           unsigned char* sa = smem + st * STAGE;
@@ -189,27 +214,29 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
       if (ok && tc::elect_one()) tc::mma_commit(&acc_full[ab]);
       __syncwarp();
     }
-  } else if (warp >= GT_WARP_TR0 || warp == 2 || warp == 3) {
+  } else {
+    const bool epi = warp >= GT_WARP_EPI0 && warp < GT_WARP_EPI0 + GT_EPI_WARPS;
     // ------------------------------------------------------------------ rounding of the X slice to fp16, in place
-    if (XD != BM_F16) {
-      // Rounding one slice is a chain (wait, load, convert, store, proxy fence, arrive) of about a thousand cycles however
-      // many warps share it, so groups of warps take the slices in turn and the chains overlap.  A group takes every
-      // TR_GROUPS-th stage of the ring: it sees every use of its stages, as its parity waits need.
-      const int tw = warp >= GT_WARP_TR0 ? warp - GT_WARP_TR0 : warp + 2;      // 0 .. 5
-      const int grp = tw / TR_PER_GROUP, gw = tw - grp * TR_PER_GROUP;
+    if (XD != BM_F16 && (!epi || all_round)) {
+      // Rounding one slice is a chain (wait, load, convert, store, proxy fence, arrive), so groups of warps take the slices in
+      // turn and the chains overlap.  A group takes every tr_groups-th stage of the ring: it sees every use of its stages, as
+      // its parity waits need.
+      const int tw = warp >= GT_WARP_TR0 ? warp - GT_WARP_TR0 : warp < GT_WARP_EPI0 ? warp + 2 : warp - GT_WARP_EPI0 + GT_TR_WARPS;
+      const int grp = tw / tr_per, gw = tw - grp * tr_per;
       const int total = p.ntiles > cta ? (p.ntiles - cta + grid - 1) / grid * slices : 0;
       uint32_t cur = grp, ph = 0;
-      int k = grp;                               // slice of its tile
-      for (int s = grp; s < total; s += TR_GROUPS) {
+      int k = s_first + grp;                     // slice of its tile
+      for (int s = grp; s < total && grp < tr_groups; s += tr_groups) {
         if (!(ok = tc::mbar_wait(&loaded[cur], ph))) break;
-        while (k >= slices) k -= slices;
+        while (k >= s_end) k -= slices;
         unsigned char* sa = smem + cur * STAGE;
         if (k >= p.slices) {
           // second contraction: fp16 already
         } else if (XD == BM_BF16) {
           // 1024 pieces of 16 bytes, element for element (the swizzle only permutes whole pieces)
-          constexpr int PIECES = GT_BM * GT_BK * 2 / 16, STEP = TR_PER_GROUP * 32;
-#pragma unroll
+          constexpr int PIECES = GT_BM * GT_BK * 2 / 16;
+          const int STEP = tr_per * 32;
+#pragma unroll 1
           for (int i0 = 0; i0 < PIECES; i0 += 4 * STEP) {
             uint4 v[4];
             uint4* q = reinterpret_cast<uint4*>(sa) + i0 + gw * 32 + lane;
@@ -230,12 +257,12 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
           // have read before any of them overwrites the row's start
           const int j = lane & 7, c4 = 2 * (j & 3);
 #pragma unroll 1
-          for (int rg = gw; rg < GT_BM / 4; rg += 2 * TR_PER_GROUP) {
+          for (int rg = gw; rg < GT_BM / 4; rg += 2 * tr_per) {
             float4 lo[2], hi[2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-              if (rg + u * TR_PER_GROUP >= GT_BM / 4) break;
-              const int r = (rg + u * TR_PER_GROUP) * 4 + (lane >> 3), sw = r & 7;
+              if (rg + u * tr_per >= GT_BM / 4) break;
+              const int r = (rg + u * tr_per) * 4 + (lane >> 3), sw = r & 7;
               const unsigned char* box = sa + (j >> 2) * (A_BYTES / 2) + r * 128;
               lo[u] = *reinterpret_cast<const float4*>(box + ((c4 ^ sw) << 4));
               hi[u] = *reinterpret_cast<const float4*>(box + (((c4 + 1) ^ sw) << 4));
@@ -243,8 +270,8 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
             __syncwarp();
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-              if (rg + u * TR_PER_GROUP >= GT_BM / 4) break;
-              const int r = (rg + u * TR_PER_GROUP) * 4 + (lane >> 3), sw = r & 7;
+              if (rg + u * tr_per >= GT_BM / 4) break;
+              const int r = (rg + u * tr_per) * 4 + (lane >> 3), sw = r & 7;
               *reinterpret_cast<uint4*>(sa + r * 128 + ((j ^ sw) << 4)) =
                   make_uint4(pack16(lo[u].x, lo[u].y, BM_F16), pack16(lo[u].z, lo[u].w, BM_F16), pack16(hi[u].x, hi[u].y, BM_F16),
                              pack16(hi[u].z, hi[u].w, BM_F16));
@@ -254,103 +281,173 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
         tc::fence_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&ready[cur]);
-        cur += TR_GROUPS;
+        cur += tr_groups;
         if (cur >= NST) { cur -= NST; ph ^= 1u; }
-        k += TR_GROUPS;
+        k += tr_groups;
       }
     }
-  } else if (warp >= GT_WARP_EPI0) {
     // ------------------------------------------------------------------ epilogue
-    // warp = (TMEM lane quarter q, every other block of 32 output columns)
-    const int q = warp & 3, half = (warp - GT_WARP_EPI0) >> 2;
-    unsigned char* stores = smem + NST * STAGE + (warp - GT_WARP_EPI0) * 2 * GT_STORE_BYTES;
-    uint32_t ti = 0, sb = 0;
-    for (int tile = cta; tile < p.ntiles && ok; tile += grid, ++ti) {
-      const GtTile t = gt_tile<BN>(p, tile);
-      const GtSeg& sg = p.seg[t.si];
-      const uint32_t ab = ti & 1u;
-      if (!(ok = tc::mbar_wait(&acc_full[ab], (ti >> 1) & 1))) break;
-      tc::fence_after_sync();
-      const int row0 = t.m0 + 32 * q, row = row0 + lane, N = sg.rows;
-      const bool with_res = p.residual != nullptr && t.si == 0;
-      const uint32_t acc = tmem_base + (static_cast<uint32_t>(32 * q) << 16) + ab * BN;
-      const int blocks = (sg.glu ? BN / 2 : t.two ? BN : BN / 2) / 32;
-      const float gate = sg.glu && p.row_gate && row < p.M ? p.row_gate[row] : 1.f;
-#pragma unroll 1
-      for (int b = half; b < blocks; b += 2) {
-        const int n = t.n0 + 32 * b;
-        if (n >= N) break;
-        float v[32];
-        tc::tmem_ld32(acc + 32 * b, v);
-        if (sg.glu) {
+    if (epi) {
+      // warp = (TMEM lane quarter q, every other block of 32 output columns)
+      const int q = warp & 3, half = (warp - GT_WARP_EPI0) >> 2;
+      unsigned char* stores = smem + NST * STAGE + (warp - GT_WARP_EPI0) * 2 * GT_STORE_BYTES;
+      uint32_t ti = 0, sb = 0;
+      for (int tile = cta; tile < p.ntiles && ok; tile += grid, ++ti) {
+        const GtTile t = gt_tile<BN>(p, tile);
+        const GtSeg& sg = p.seg[t.si];
+        const uint32_t ab = ti & 1u;
+        if (!(ok = tc::mbar_wait(&acc_full[ab], (ti >> 1) & 1))) break;
+        tc::fence_after_sync();
+        if (SPLIT > 1) {
+          // (one tile per cluster) this warp's rows of one half of the tile -> the CTAs that own the columns
+          constexpr int RW = BN / 2 / SPLIT, ROW = gt_recv_row(BN, SPLIT);
+          tc::cluster_wait();
+          const uint32_t mine = tc::smem_u32(smem + NST * STAGE) + ((rank * GT_BM + 32 * q + lane) * ROW + half * RW) * 4;
+          const uint32_t acc = tmem_base + (static_cast<uint32_t>(32 * q) << 16) + ab * BN + half * (BN / 2);
+          if (half == 0 || t.two) {
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            float u[16];
-            tc::tmem_ld16(acc + BN / 2 + 32 * b + 16 * h, u);
+            for (int c0 = 0; c0 < BN / 2; c0 += 32) {
+              float v[32];
+              tc::tmem_ld32(acc + c0, v);
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float g = v[16 * h + i];
-              v[16 * h + i] = __fdividef(g, 1.f + __expf(-g)) * u[i] * gate;
-            }
-          }
-        }
-        if (sg.c_dtype != BM_F32 && p.tma_store) {
-          // 32 rows of 64 bytes, 16-byte pieces in the order of the map's 64-byte swizzle; the block two before has left
-          unsigned char* blk = stores + sb * GT_STORE_BYTES;
-          sb ^= 1u;
-          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-          __syncwarp();
-          unsigned char* mine = blk + lane * 64;
-          const int sw = (lane >> 1) & 3;
-          if (with_res) {
-            const int r = lane >> 2, c = lane & 3;
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int rr = 8 * i + r;
-              uint4 x = make_uint4(0u, 0u, 0u, 0u);
-              if (row0 + rr < p.M && n + 8 * c < N)
-                x = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.residual) + static_cast<size_t>(row0 + rr) * N + n + 8 * c));
-              *reinterpret_cast<uint4*>(blk + rr * 64 + ((c ^ ((rr >> 1) & 3)) << 4)) = x;
-            }
-            __syncwarp();
-#pragma unroll
-            for (int c2 = 0; c2 < 4; ++c2) {
-              const uint4 x = *reinterpret_cast<const uint4*>(mine + ((c2 ^ sw) << 4));
-              const uint32_t w[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float2 f = sg.c_dtype == BM_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j]))
-                                                      : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
-                v[8 * c2 + 2 * j] += f.x;
-                v[8 * c2 + 2 * j + 1] += f.y;
+              for (int j = 0; j < 32; j += 4) {
+                const int col = c0 + j;
+                asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(tc::cluster_map(mine + (col % RW) * 4, col / RW)), "f"(v[j]), "f"(v[j + 1]),
+                             "f"(v[j + 2]), "f"(v[j + 3])
+                             : "memory");
               }
             }
           }
+          break;
+        }
+        const int row0 = t.m0 + 32 * q, row = row0 + lane, N = sg.rows;
+        const bool with_res = p.residual != nullptr && t.si == 0;
+        const uint32_t acc = tmem_base + (static_cast<uint32_t>(32 * q) << 16) + ab * BN;
+        const int blocks = (sg.glu ? BN / 2 : t.two ? BN : BN / 2) / 32;
+        const float gate = sg.glu && p.row_gate && row < p.M ? p.row_gate[row] : 1.f;
+#pragma unroll 1
+        for (int b = half; b < blocks; b += 2) {
+          const int n = t.n0 + 32 * b;
+          if (n >= N) break;
+          float v[32];
+          tc::tmem_ld32(acc + 32 * b, v);
+          if (sg.glu) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c)
-            *reinterpret_cast<uint4*>(mine + ((c ^ sw) << 4)) =
-                make_uint4(pack16(v[8 * c], v[8 * c + 1], sg.c_dtype), pack16(v[8 * c + 2], v[8 * c + 3], sg.c_dtype),
-                           pack16(v[8 * c + 4], v[8 * c + 5], sg.c_dtype), pack16(v[8 * c + 6], v[8 * c + 7], sg.c_dtype));
-          tc::fence_async_smem();
-          __syncwarp();
-          if (lane == 0) tma_store_2d(&p.c[t.si], n, row0, blk);       // rows and columns past the matrix are clipped
-        } else if (row < p.M) {
+            for (int h = 0; h < 2; ++h) {
+              float u[16];
+              tc::tmem_ld16(acc + BN / 2 + 32 * b + 16 * h, u);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (n + i < N) {
-              const size_t idx = static_cast<size_t>(row) * N + n + i;
-              float val = v[i];
-              if (with_res) val += load_act(p.residual, sg.c_dtype, idx);
-              store_act(sg.C, sg.c_dtype, idx, val);
+              for (int i = 0; i < 16; ++i) {
+                const float g = v[16 * h + i];
+                v[16 * h + i] = __fdividef(g, 1.f + __expf(-g)) * u[i] * gate;
+              }
+            }
+          }
+          if (sg.c_dtype != BM_F32 && p.tma_store) {
+            // 32 rows of 64 bytes, 16-byte pieces in the order of the map's 64-byte swizzle; the block two before has left
+            unsigned char* blk = stores + sb * GT_STORE_BYTES;
+            sb ^= 1u;
+            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            __syncwarp();
+            unsigned char* mine = blk + lane * 64;
+            const int sw = (lane >> 1) & 3;
+            if (with_res) {
+              const int r = lane >> 2, c = lane & 3;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const int rr = 8 * i + r;
+                uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                if (row0 + rr < p.M && n + 8 * c < N)
+                  x = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.residual) + static_cast<size_t>(row0 + rr) * N + n + 8 * c));
+                *reinterpret_cast<uint4*>(blk + rr * 64 + ((c ^ ((rr >> 1) & 3)) << 4)) = x;
+              }
+              __syncwarp();
+#pragma unroll
+              for (int c2 = 0; c2 < 4; ++c2) {
+                const uint4 x = *reinterpret_cast<const uint4*>(mine + ((c2 ^ sw) << 4));
+                const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const float2 f = sg.c_dtype == BM_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j]))
+                                                        : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
+                  v[8 * c2 + 2 * j] += f.x;
+                  v[8 * c2 + 2 * j + 1] += f.y;
+                }
+              }
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              *reinterpret_cast<uint4*>(mine + ((c ^ sw) << 4)) =
+                  make_uint4(pack16(v[8 * c], v[8 * c + 1], sg.c_dtype), pack16(v[8 * c + 2], v[8 * c + 3], sg.c_dtype),
+                             pack16(v[8 * c + 4], v[8 * c + 5], sg.c_dtype), pack16(v[8 * c + 6], v[8 * c + 7], sg.c_dtype));
+            tc::fence_async_smem();
+            __syncwarp();
+            if (lane == 0) tma_store_2d(&p.c[t.si], n, row0, blk);       // rows and columns past the matrix are clipped
+          } else if (row < p.M) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) {
+              if (n + i < N) {
+                const size_t idx = static_cast<size_t>(row) * N + n + i;
+                float val = v[i];
+                if (with_res) val += load_act(p.residual, sg.c_dtype, idx);
+                store_act(sg.C, sg.c_dtype, idx, val);
+              }
             }
           }
         }
+        tc::fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&acc_empty[ab]);
       }
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&acc_empty[ab]);
+      if (SPLIT == 1 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+  }
+  if (SPLIT > 1) {
+    const bool epi = warp >= GT_WARP_EPI0 && warp < GT_WARP_EPI0 + GT_EPI_WARPS;
+    if (!epi || !ok) tc::cluster_wait();         // (the epilogue warps have, unless their accumulator did not come)
+    tc::cluster_arrive();
+    tc::cluster_wait();                          // every share of this CTA's columns is there
+    if (epi) {
+      constexpr int RW = BN / 2 / SPLIT, ROW = gt_recv_row(BN, SPLIT);
+      const GtTile t = gt_tile<BN>(p, cta);
+      const GtSeg& sg = p.seg[t.si];
+      const int i = threadIdx.x - 32 * GT_WARP_EPI0, r = i >> 1, h = i & 1, row = t.m0 + r, N = sg.rows;
+      const float* recv = reinterpret_cast<const float*>(smem + NST * STAGE) + r * ROW;
+      const float gate = sg.glu && p.row_gate && row < p.M ? p.row_gate[row] : 1.f;
+      const bool with_res = p.residual != nullptr && t.si == 0;
+      if (row < p.M && (sg.glu ? h == 0 : h == 0 || t.two)) {
+#pragma unroll
+        for (int c = 0; c < RW; c += 8) {
+          const int n = t.n0 + (sg.glu ? 0 : h * (BN / 2)) + rank * RW + c;
+          if (n >= N) break;                     // (rows of a stack come in eights)
+          float v[8] = {}, u[8] = {};
+#pragma unroll
+          for (int src = 0; src < SPLIT; ++src)
+#pragma unroll
+            for (int j = 0; j < 8; j += 4) {
+              const float4 a = *reinterpret_cast<const float4*>(recv + src * GT_BM * ROW + h * RW + c + j);
+              v[j] += a.x; v[j + 1] += a.y; v[j + 2] += a.z; v[j + 3] += a.w;
+              if (sg.glu) {
+                const float4 b = *reinterpret_cast<const float4*>(recv + src * GT_BM * ROW + RW + c + j);
+                u[j] += b.x; u[j + 1] += b.y; u[j + 2] += b.z; u[j + 3] += b.w;
+              }
+            }
+          const size_t idx = static_cast<size_t>(row) * N + n;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (sg.glu) v[j] = __fdividef(v[j], 1.f + __expf(-v[j])) * u[j] * gate;
+            if (with_res) v[j] += load_act(p.residual, sg.c_dtype, idx + j);
+          }
+          if (sg.c_dtype != BM_F32 && p.tma_store) {
+            *reinterpret_cast<uint4*>(static_cast<uint16_t*>(sg.C) + idx) = make_uint4(pack16(v[0], v[1], sg.c_dtype), pack16(v[2], v[3], sg.c_dtype),
+                                                                                       pack16(v[4], v[5], sg.c_dtype), pack16(v[6], v[7], sg.c_dtype));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) store_act(sg.C, sg.c_dtype, idx + j, v[j]);
+          }
+        }
+      }
+    }
   }
   if (!ok && lane == 0 && p.status) atomicExch(p.status, BM_ERR_TIMEOUT);
   tc::fence_before_sync();
@@ -388,19 +485,36 @@ static bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN, int XD>
+template <int BN, int XD, int SPLIT>
 static int launch_one(const GtParams& p, int grid, cudaStream_t st) {
-  const int smem = gt_stages(BN, XD) * gt_stage_bytes(BN, XD) + GT_EPI_WARPS * 2 * GT_STORE_BYTES + 1024;
+  const int smem = gt_stages(BN, XD, SPLIT) * gt_stage_bytes(BN, XD) + gt_tail_bytes(BN, SPLIT) + 1024;
   static PerDeviceOnce once;
   int dev = -1;
   BM_CUDA(cudaGetDevice(&dev));
   if (!once.is_done(dev)) {
-    BM_CUDA(cudaFuncSetAttribute(gemm_tma_kernel<BN, XD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    BM_CUDA(cudaFuncSetAttribute(gemm_tma_kernel<BN, XD, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     once.mark(dev);
   }
-  gemm_tma_kernel<BN, XD><<<grid, GT_THREADS, smem, st>>>(p);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid * SPLIT);
+  cfg.blockDim = dim3(GT_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = SPLIT;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = SPLIT > 1 ? 1 : 0;
+  BM_CUDA(cudaLaunchKernelEx(&cfg, gemm_tma_kernel<BN, XD, SPLIT>, p));
   BM_LAUNCH_CHECK("gemm_tma_kernel");
   return BM_OK;
+}
+template <int BN, int SPLIT>
+static int launch_typed(const GtParams& p, int x_dtype, int grid, cudaStream_t st) {
+  if (x_dtype == BM_F32) return launch_one<BN, BM_F32, SPLIT>(p, grid, st);
+  if (x_dtype == BM_BF16) return launch_one<BN, BM_BF16, SPLIT>(p, grid, st);
+  return launch_one<BN, BM_F16, SPLIT>(p, grid, st);
 }
 
 // Returns BM_ERR_UNSUPPORTED (without having launched anything) when the shape or the pointers do not suit tiled
@@ -432,8 +546,23 @@ int launch_gemm_tma(const GemmTmaArgs& a, cudaStream_t st) {
     }
     return tiles_m * p.tiles_n;
   };
-  const bool narrow = lay_out(256) < sm_counts[dev] / 2;   // the wide tile would leave most SMs idle
-  const int bn = narrow ? 64 : 256;
+  // Tile width and split of the contraction.  Where the wide tile would leave most SMs idle: what takes the fewest slices one
+  // after the other.  A slice of a 128-column tile counts 1.15 of a 64-column one, two more stand for start and end, three for
+  // the exchange of a split; clusters of four leave a few SMs of a group unused.  Basis pair of 2 x 256 rows, hidden 2048, bf16,
+  // us at 64 / 128 / 256 columns, then 64 split in 2 / 4: 300 tokens 13.2 14.5 18.8 11.6 9.4, 777 tokens 13.5 14.6 18.9 11.8 -,
+  // 2048 tokens 13.9 15.7 20.8 - -, 4096 tokens 28.3 16.2 21.4 - -, 6000 tokens 40.6 30.3 21.8 - -.
+  int bn = 256, split = 1;
+  if (lay_out(256) < sm_counts[dev] / 2) {
+    const int slices = (a.K + a.K2) / GT_BK;
+    double best = 1e30;
+    for (const auto& c : {std::make_pair(64, 1), std::make_pair(128, 1), std::make_pair(64, 2), std::make_pair(64, 4)}) {
+      const int tiles = lay_out(c.first), most = c.second == 4 ? sm_counts[dev] * 7 / 8 : sm_counts[dev];
+      if (c.second > 1 && (tiles * c.second > most || slices < 4 * c.second)) continue;
+      const int waves = (tiles * c.second + sm_counts[dev] - 1) / sm_counts[dev];
+      const double cost = waves * ((slices + c.second - 1) / c.second + 2) * (c.first > 64 ? 1.15 : 1.0) + (c.second > 1 ? 3 : 0);
+      if (cost < best) { best = cost; bn = c.first; split = c.second; }
+    }
+  }
   p.ntiles = lay_out(bn);
   if (!make_map(&p.x, a.X, a.M, a.K, xb, GT_BM, 128)) return BM_ERR_UNSUPPORTED;
   if (a.K2 && (!make_map(&p.x2, a.X2, a.M, a.K2, 2, GT_BM, 128) || !make_map(&p.w2, a.W2, a.seg[0].rows, a.K2, 2, bn / 2, 128))) return BM_ERR_UNSUPPORTED;
@@ -455,15 +584,10 @@ int launch_gemm_tma(const GemmTmaArgs& a, cudaStream_t st) {
   p.residual = a.residual; p.row_gate = a.row_gate; p.n_seg = a.n_seg; p.M = a.M;
   p.slices = a.K / GT_BK; p.slices2 = a.K2 / GT_BK;
   p.status = a.status;
-  const int grid = p.ntiles < sm_counts[dev] ? p.ntiles : sm_counts[dev];
-  if (narrow) {
-    if (a.x_dtype == BM_F32) return launch_one<64, BM_F32>(p, grid, st);
-    if (a.x_dtype == BM_BF16) return launch_one<64, BM_BF16>(p, grid, st);
-    return launch_one<64, BM_F16>(p, grid, st);
-  }
-  if (a.x_dtype == BM_F32) return launch_one<256, BM_F32>(p, grid, st);
-  if (a.x_dtype == BM_BF16) return launch_one<256, BM_BF16>(p, grid, st);
-  return launch_one<256, BM_F16>(p, grid, st);
+  const int grid = split > 1 || p.ntiles < sm_counts[dev] ? p.ntiles : sm_counts[dev];
+  if (bn == 64) return split == 1 ? launch_typed<64, 1>(p, a.x_dtype, grid, st) : split == 2 ? launch_typed<64, 2>(p, a.x_dtype, grid, st) : launch_typed<64, 4>(p, a.x_dtype, grid, st);
+  if (bn == 128) return launch_typed<128, 1>(p, a.x_dtype, grid, st);
+  return launch_typed<256, 1>(p, a.x_dtype, grid, st);
 }
 
 int launch_gemm_basis(const GemmTcArgs& a, int problems, cudaStream_t st) {

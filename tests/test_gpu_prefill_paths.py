@@ -166,3 +166,47 @@ def test_prefill_block_matches_stages(T, E, shared, wdtype):
         g, u, d, t = (v.float() for v in sh)
         want = want + torch.sigmoid(xf @ t.T) * ((torch.nn.functional.silu(xf @ g.T) * (xf @ u.T)) @ d.T)
     helpers.assert_close(y.cpu(), want.cpu(), what=f"block T={T} E={E}")
+
+
+# contractions split over two and four CTAs: uneven shares (17 slices), stacks that fill part of a tile, ragged token counts; the
+# last pair of sizes has the down basis split as well
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("hidden,rank", [(512, 72), (1024, 40), (1088, 104), (1024, 512)])
+@pytest.mark.parametrize("T", [257, 300, 513])
+def test_split_contractions_vs_double(hidden, rank, T, dtype):
+    cfg = synth.tiny(hidden=hidden, num_experts=2, intermediate=128, rank=rank)
+    raw = synth.make_layer(cfg, seed=rank, device=DEV)
+    layer = synth.to_packed_layer(raw)
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn(T, hidden, generator=gen, device=DEV).to(dtype)
+
+    def check(got, a, w, extra, eps):
+        # operands are fp16; fp32 sums of n products err by n * 2^-24 of the sum of magnitudes, the result by its own rounding
+        a, w = a.half().double(), w.half().double()
+        want = a @ w.t() + extra.double()
+        bound = eps * want.abs() + a.shape[1] * 2.0 ** -24 * (a.abs() @ w.abs().t() + extra.double().abs()) + 2.0 ** -24
+        worst = float(((got.double() - want).abs() / bound).max())
+        assert worst <= 1.0, worst
+
+    eps = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8, torch.float32: 0.0}
+    zero = torch.zeros((), device=DEV)
+    for got, w in zip(layer.basis_project(x), (raw.vh_gate, raw.vh_up)):
+        check(got, x, w.to(DEV), zero, eps[torch.float16])
+    acc = torch.randn(T, rank, generator=gen, device=DEV) * 0.05
+    res = torch.randn(T, hidden, generator=gen, device=DEV).to(dtype)
+    check(layer.combine_down_basis(acc, dtype, residual=res), acc, raw.u_down.to(DEV), res, eps[dtype])
+    layer.check_status()
+
+
+@pytest.mark.parametrize("T,inter", [(257, 64), (400, 192)])
+def test_split_gated_pair(T, inter):
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn(T, 1024, generator=gen, device=DEV).half()
+    wg, wu = (torch.randn(inter, 1024, generator=gen, device=DEV).half() / 32 for _ in range(2))
+    wd = (torch.randn(1024, inter, generator=gen, device=DEV) / inter ** 0.5).half()
+    g, u = x.double() @ wg.double().t(), x.double() @ wu.double().t()
+    z = torch.nn.functional.silu(g) * u
+    want = z @ wd.double().t()
+    # z is rounded to fp16 (one rounding, and what the fp32 sums and __expf add: a few 2^-20), y as well
+    bound = 2.0 ** -10 * (z.abs() @ wd.double().abs().t()) + 2.0 ** -11 * want.abs() + 2.0 ** -24
+    assert float(((dense_mlp(x, wg, wu, wd).double() - want).abs() / bound).max()) <= 1.0
