@@ -55,6 +55,38 @@ struct PerDeviceOnce {
   void mark(int dev) { if (dev >= 0 && dev < MAX_DEVICES) done[dev].store(1, std::memory_order_release); }
 };
 
+// What a kernel's launch may overlap of the launches before it on the same stream (programmatic serialisation).
+enum LaunchAfter {
+  AFTER_ALL = 0,       // an ordinary launch
+  AFTER_READS = 1,     // starts while they drain, waits for them before it touches memory
+  AFTER_BESIDE = 2     // reads nothing that they write and writes nothing that they read: waits for them before it ends, so that
+                       // whoever waits for it has waited for them
+};
+template <typename... P, typename... A>
+inline cudaError_t launch_after(LaunchAfter after, int cluster, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  cfg.attrs = attr;
+  if (after != AFTER_ALL) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+// The next launch may be set up / what the launches before wrote is there (both without effect on ordinary launches).
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // One packed matrix as the device sees it (pointers into the caller's buffers).
 struct MatDev {
   const uint32_t* payload;
@@ -195,6 +227,9 @@ struct GemmTcArgs {
   int M, N, K;
   int x_dtype, c_dtype;
   int* status;
+  LaunchAfter after;
+  float4* zero;           // optional buffer cleared on the way (the expert stage's accumulator), 16-byte units
+  int64_t zero_n;
 };
 int launch_gemm_tc(const GemmTcArgs& a, int problems, cudaStream_t st);
 // The tiled-copy kernel (gemm_tma.cu): several stacks of weight rows sharing X in one launch.  C[m][n] = X[m] . W[n], or
@@ -218,11 +253,20 @@ struct GemmTmaArgs {
   const void* residual;     // added to stack 0, of its type
   const float* row_gate;    // [M] factor of the gated pair's rows, or null
   int* status;
+  LaunchAfter after;
+  float4* zero;             // optional buffer cleared on the way, 16-byte units
+  int64_t zero_n;
 };
 // BM_ERR_UNSUPPORTED, with nothing launched, when a shape or pointer does not suit tiled copies.
 int launch_gemm_tma(const GemmTmaArgs& a, cudaStream_t st);
 // One or two products sharing X: the tiled-copy kernel, else launch_gemm_tc.
 int launch_gemm_basis(const GemmTcArgs& a, int problems, cudaStream_t st);
+
+// bm_route with its first launch placed as `after` says; `beside_follows`: the next launch on the stream is an AFTER_BESIDE one.
+int route_tokens(const void* logits, int logits_dtype, int32_t T, int32_t E_routed, int32_t k, int32_t renorm, int32_t weight_round,
+                 const int32_t* global_to_local, int32_t num_local, int32_t tile_rows, int32_t* topk_idx, float* topk_w,
+                 int32_t* token_indices, int32_t* expert_offsets, float* route_flat, int32_t* tile_table, int32_t* counts, void* workspace,
+                 size_t workspace_bytes, LaunchAfter after, bool beside_follows, cudaStream_t st);
 
 // NVTX range around a public entry point (route / projection / experts / combine / exchange show up as named ranges
 // in a timeline tool; without a tool attached a push or pop is one null-pointer test).
@@ -260,6 +304,4 @@ struct bm_layer {
   int bat_ring = 0, bat_sec_bytes = 0, bat_smem = 0, bat_grid = 0;      // of experts_batch_kernel (bat_ring 0: not for this layer)
   int wait_limit_us = bm::DEFAULT_WAIT_LIMIT_US;   // of the packed-expert kernels' waits (bm_layer_set_option)
   int* status_dev = nullptr;       // device flag set by a kernel whose bounded wait gave up
-  cudaStream_t side_stream = nullptr;   // routing runs here, beside the basis projection
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
 };

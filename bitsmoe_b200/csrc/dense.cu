@@ -11,25 +11,27 @@ namespace bm {
 int launch_gemm_nt(const GemmArgs& g, int problems, cudaStream_t st);
 
 // C_i [T, N] = X [T, K] . W_i [N, K]^T for `problems` (1 or 2) weight matrices sharing X; residual (problem 0 only) may
-// be null.  Chooses the kernel by shape.
+// be null.  Chooses the kernel by shape: where both suit, the skinny one up to `skinny_tokens`.
 int dense_xwT(const void* X, int x_dtype, const __half* W0, const __half* W1, void* C0, void* C1, int c_dtype,
-              const void* residual, int T, int N, int K, int problems, int* status, cudaStream_t st) {
+              const void* residual, int T, int N, int K, int problems, int* status, LaunchAfter after, int skinny_tokens, cudaStream_t st) {
   if (T == 0) return BM_OK;
-  const bool aligned = aligned16(X, W0, W1);
-  if (T <= SKINNY_MAX_TOKENS && aligned && K % 8 == 0) {
+  const bool aligned = aligned16(X, W0, W1), tiled = aligned && K % 64 == 0 && N % 8 == 0;
+  if (T <= (tiled ? skinny_tokens : SKINNY_MAX_TOKENS) && aligned && K % 8 == 0) {
     SkinnyArgs a{};
     a.n_seg = problems;
     a.seg[0] = SkSeg{W0, nullptr, C0, N, c_dtype, 0, 0};
     a.seg[1] = SkSeg{W1, nullptr, C1, N, c_dtype, 0, 0};
     a.X = X; a.N = T; a.K = K; a.x_dtype = x_dtype; a.residual = residual;
     a.splits = skinny_splits(N * problems, K);
+    a.overlap = after != AFTER_ALL;
     const int rc = launch_skinny_nt(a, st);
     if (rc != BM_ERR_UNSUPPORTED) return rc;
   }
-  if (aligned && K % 64 == 0 && N % 8 == 0) {
+  if (tiled) {
     GemmTcArgs t{};
     t.X = X; t.W[0] = W0; t.W[1] = problems > 1 ? W1 : W0; t.C[0] = C0; t.C[1] = problems > 1 ? C1 : C0;
     t.residual = residual; t.M = T; t.N = N; t.K = K; t.x_dtype = x_dtype; t.c_dtype = c_dtype; t.status = status;
+    t.after = after;
     return launch_gemm_basis(t, problems, st);
   }
   GemmArgs g{};
@@ -68,39 +70,70 @@ static int dense_mlp_small(const void* x, int x_dtype, const __half* wg, const _
   return launch_skinny_nt(d, st);
 }
 
-// gate[t] = sigmoid(x[t] . w): one warp per token.
-__global__ void __launch_bounds__(256) row_gate_kernel(const void* __restrict__ x, int x_dtype, const __half* __restrict__ w, int T,
-                                                       int H, float* __restrict__ gate) {
+// gate[t] = sigmoid(x[t] . w), w fp16 or bf16 rounded to it.  A warp takes two tokens, whose loads share those of w: a pass over x at
+// memory speed.  It runs beside the rounding of a block's weights, which it does not read (16384 x 2048 bf16 and 4.2 M weights: 25 -> 22 us).
+__device__ __forceinline__ float2 row_gate_pair(uint32_t v, int dtype) {
+  if (dtype == BM_F16) return __half22float2(*reinterpret_cast<const __half2*>(&v));
+  return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+}
+constexpr int RG_TOKENS = 2;
+__global__ void __launch_bounds__(256) row_gate_kernel(const void* __restrict__ x, int x_dtype, const uint16_t* __restrict__ w, int w_dtype, int T,
+                                                       int H, float* __restrict__ gate, int beside) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * (blockDim.x >> 5) + warp;
-  if (t >= T) return;
-  float acc = 0.f;
+  const int t0 = (blockIdx.x * (blockDim.x >> 5) + warp) * RG_TOKENS;
+  grid_launch_dependents();
+  if (!beside) grid_wait();
+  auto weight = [&](uint32_t v) {
+    const float2 f = row_gate_pair(v, w_dtype);
+    return w_dtype == BM_F16 ? f : __half22float2(__floats2half2_rn(f.x, f.y));
+  };
   if (x_dtype != BM_F32 && H % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0) {
-    // 16 bytes per lane and load, four in flight: a pass over x at memory speed
-    const uint4* xr = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + static_cast<int64_t>(t) * H);
+    float acc[RG_TOKENS] = {};
+    const uint4* xr[RG_TOKENS];
+#pragma unroll
+    for (int u = 0; u < RG_TOKENS; ++u) xr[u] = reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(x) + static_cast<int64_t>(min(t0 + u, T - 1)) * H);
     const uint4* wr = reinterpret_cast<const uint4*>(w);
 #pragma unroll 4
     for (int i = lane; i < H / 8; i += 32) {
-      const uint4 xv = xr[i], wv = __ldg(wr + i);
-      const uint32_t *xp = reinterpret_cast<const uint32_t*>(&xv), *wp = reinterpret_cast<const uint32_t*>(&wv);
+      uint4 xv[RG_TOKENS];
+#pragma unroll
+      for (int u = 0; u < RG_TOKENS; ++u) xv[u] = __ldg(xr[u] + i);
+      const uint4 wv = __ldg(wr + i);
+      const uint32_t* wp = reinterpret_cast<const uint32_t*>(&wv);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 xf = x_dtype == BM_F16 ? __half22float2(*reinterpret_cast<const __half2*>(xp + j))
-                                            : __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(xp + j));
-        const float2 wf = __half22float2(*reinterpret_cast<const __half2*>(wp + j));
-        acc = fmaf(xf.x, wf.x, fmaf(xf.y, wf.y, acc));
+        const float2 wf = weight(wp[j]);
+#pragma unroll
+        for (int u = 0; u < RG_TOKENS; ++u) {
+          const float2 xf = row_gate_pair(reinterpret_cast<const uint32_t*>(&xv[u])[j], x_dtype);
+          acc[u] = fmaf(xf.x, wf.x, fmaf(xf.y, wf.y, acc[u]));
+        }
       }
     }
-  } else {
-    for (int i = lane; i < H; i += 32) acc += load_act(x, x_dtype, static_cast<int64_t>(t) * H + i) * __half2float(w[i]);
-  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-  if (lane == 0) gate[t] = 1.f / (1.f + __expf(-acc));
+    for (int u = 0; u < RG_TOKENS; ++u) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc[u] += __shfl_xor_sync(0xffffffffu, acc[u], o);
+      if (lane == 0 && t0 + u < T) gate[t0 + u] = 1.f / (1.f + __expf(-acc[u]));
+    }
+  } else {
+    for (int t = t0; t < min(t0 + RG_TOKENS, T); ++t) {
+      float acc = 0.f;
+      for (int i = lane; i < H; i += 32) {
+        const float wf = w_dtype == BM_F16 ? load_act(w, BM_F16, i) : __half2float(__float2half_rn(load_act(w, BM_BF16, i)));
+        acc += load_act(x, x_dtype, static_cast<int64_t>(t) * H + i) * wf;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (lane == 0) gate[t] = 1.f / (1.f + __expf(-acc));
+    }
+  }
+  if (beside) grid_wait();
 }
 
-int launch_row_gate(const void* x, int x_dtype, const __half* w, int T, int H, float* gate, cudaStream_t st) {
-  row_gate_kernel<<<(T + 7) / 8, 256, 0, st>>>(x, x_dtype, w, T, H, gate);
+int launch_row_gate(const void* x, int x_dtype, const uint16_t* w, int w_dtype, int T, int H, float* gate, LaunchAfter after, cudaStream_t st) {
+  const int per = 8 * RG_TOKENS;
+  BM_CUDA(launch_after(after, 1, row_gate_kernel, dim3((T + per - 1) / per), 256, 0, st, x, x_dtype, w, w_dtype, T, H, gate, after == AFTER_BESIDE));
   BM_LAUNCH_CHECK("row_gate_kernel");
   return BM_OK;
 }
@@ -129,7 +162,7 @@ extern "C" int bm_gate_logits(const void* x, int x_dtype, const uint16_t* gate_w
   if (T == 0) return BM_OK;
   BM_REQUIRE(x && gate_w && logits, BM_ERR_INVALID_ARG, "gate_logits: null pointer");
   return dense_xwT(x, x_dtype, reinterpret_cast<const __half*>(gate_w), nullptr, logits, nullptr, logits_dtype, nullptr, T, num_routed,
-                   hidden, 1, nullptr, static_cast<cudaStream_t>(stream));
+                   hidden, 1, nullptr, AFTER_ALL, SKINNY_MAX_TOKENS, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" size_t bm_dense_mlp_workspace_bytes(int32_t T, int32_t intermediate) {
@@ -160,20 +193,21 @@ extern "C" int bm_dense_mlp_forward(const void* x, int x_dtype, const uint16_t* 
                            reinterpret_cast<const __half*>(w_down), reinterpret_cast<const __half*>(token_gate_w), T, hidden, intermediate,
                            residual, y, y_dtype, reinterpret_cast<float*>(ws), gate, st);
   if (rc != BM_ERR_UNSUPPORTED) return rc;
-  if (token_gate_w && (rc = launch_row_gate(x, x_dtype, reinterpret_cast<const __half*>(token_gate_w), T, hidden, gate, st))) return rc;
+  if (token_gate_w && (rc = launch_row_gate(x, x_dtype, token_gate_w, BM_F16, T, hidden, gate, AFTER_ALL, st))) return rc;
   // gated pair in the epilogue of one launch where tiled copies take the shape
   GemmTmaArgs a{};
   a.X = x; a.x_dtype = x_dtype; a.M = T; a.K = hidden;
   a.seg[0] = GemmSeg{reinterpret_cast<const __half*>(w_gate), reinterpret_cast<const __half*>(w_up), z, intermediate, BM_F16};
   a.n_seg = 1;
   a.row_gate = token_gate_w ? gate : nullptr;
+  a.after = token_gate_w ? AFTER_READS : AFTER_ALL;
   rc = launch_gemm_tma(a, st);
   if (rc == BM_OK)
     return dense_xwT(z, BM_F16, reinterpret_cast<const __half*>(w_down), nullptr, y, nullptr, y_dtype, residual, T, hidden, intermediate, 1,
-                     nullptr, st);
+                     nullptr, AFTER_READS, SKINNY_MAX_TOKENS, st);
   if (rc != BM_ERR_UNSUPPORTED) return rc;
   rc = dense_xwT(x, x_dtype, reinterpret_cast<const __half*>(w_gate), reinterpret_cast<const __half*>(w_up), g, u, BM_F16, nullptr,
-                 T, intermediate, hidden, 2, nullptr, st);
+                 T, intermediate, hidden, 2, nullptr, AFTER_ALL, SKINNY_MAX_TOKENS, st);
   if (rc) return rc;
   const int64_t pairs = static_cast<int64_t>(T) * intermediate / 2;
   const int blocks = static_cast<int>((pairs + 255) / 256 < 148 * 8 ? (pairs + 255) / 256 : 148 * 8);
@@ -181,5 +215,5 @@ extern "C" int bm_dense_mlp_forward(const void* x, int x_dtype, const uint16_t* 
                                           token_gate_w ? gate : nullptr, pairs, intermediate / 2, reinterpret_cast<__half2*>(z));
   BM_LAUNCH_CHECK("silu_mul_kernel");
   return dense_xwT(z, BM_F16, reinterpret_cast<const __half*>(w_down), nullptr, y, nullptr, y_dtype, residual, T, hidden, intermediate, 1,
-                   nullptr, st);
+                   nullptr, AFTER_ALL, SKINNY_MAX_TOKENS, st);
 }

@@ -310,6 +310,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
     abort_flag_s[1] = A.wait_limit_us;
   }
   tc::cluster_arrive();
+  grid_launch_dependents();
+  grid_wait();
   // items before each expert (an item = up to 2 nt consecutive assignments of one expert): every thread loads
   // its experts' counts in parallel, one warp then scans them
   for (int e = threadIdx.x; e < num_experts; e += XT_THREADS) {
@@ -895,7 +897,7 @@ static int xt_launch(XtArgs a, size_t smem, cudaStream_t st) {
     BM_REQUIRE(fa.numRegs >= XT_REGS, BM_ERR_UNSUPPORTED, "experts_tc: built with %d registers per thread, %d expected", fa.numRegs, XT_REGS);
     once.mark(dev);
   }
-  experts_tc_kernel<ROWS, WIDE><<<grids[dev], XT_THREADS, smem, st>>>(a);
+  BM_CUDA(launch_after(AFTER_READS, /*cluster: the kernel's own*/ 1, experts_tc_kernel<ROWS, WIDE>, dim3(grids[dev]), XT_THREADS, smem, st, a));
   BM_LAUNCH_CHECK("experts_tc_kernel");
   return BM_OK;
 }

@@ -71,8 +71,10 @@ struct GtParams {
   GtSeg seg[GEMM_MAX_SEG];
   const void* residual;      // of stack 0
   const float* row_gate;     // factor per row of a gated pair's result, or null
-  int n_seg, M, slices, slices2, tiles_n, ntiles, tma_store;
+  int n_seg, M, slices, slices2, tiles_n, ntiles, tma_store, beside;
   int* status;
+  float4* zero;              // cleared by the epilogue warps
+  int64_t zero_n;
 };
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
@@ -160,6 +162,8 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
+  grid_launch_dependents();
+  if (!p.beside) grid_wait();
   // slices of X . W, then of the second contraction: this CTA's share
   const int all = p.slices + p.slices2, rank = SPLIT > 1 ? static_cast<int>(blockIdx.x) % SPLIT : 0;
   const int s_first = all * rank / SPLIT, s_end = all * (rank + 1) / SPLIT, slices = s_end - s_first;
@@ -216,6 +220,10 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
     }
   } else {
     const bool epi = warp >= GT_WARP_EPI0 && warp < GT_WARP_EPI0 + GT_EPI_WARPS;
+    if (epi && p.zero)
+      for (int64_t i = static_cast<int64_t>(blockIdx.x) * (32 * GT_EPI_WARPS) + threadIdx.x - 32 * GT_WARP_EPI0; i < p.zero_n;
+           i += static_cast<int64_t>(gridDim.x) * (32 * GT_EPI_WARPS))
+        p.zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     // ------------------------------------------------------------------ rounding of the X slice to fp16, in place
     if (XD != BM_F16 && (!epi || all_round)) {
       // Rounding one slice is a chain (wait, load, convert, store, proxy fence, arrive), so groups of warps take the slices in
@@ -450,6 +458,7 @@ __global__ void __launch_bounds__(GT_THREADS, 1) gemm_tma_kernel(const __grid_co
     }
   }
   if (!ok && lane == 0 && p.status) atomicExch(p.status, BM_ERR_TIMEOUT);
+  if (p.beside) grid_wait();
   tc::fence_before_sync();
   __syncthreads();
   if (warp == 2) tc::tmem_dealloc(tmem_base, TMEM_COLS);
@@ -486,7 +495,7 @@ static bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int
 }
 
 template <int BN, int XD, int SPLIT>
-static int launch_one(const GtParams& p, int grid, cudaStream_t st) {
+static int launch_one(const GtParams& p, LaunchAfter after, int grid, cudaStream_t st) {
   const int smem = gt_stages(BN, XD, SPLIT) * gt_stage_bytes(BN, XD) + gt_tail_bytes(BN, SPLIT) + 1024;
   static PerDeviceOnce once;
   int dev = -1;
@@ -495,26 +504,15 @@ static int launch_one(const GtParams& p, int grid, cudaStream_t st) {
     BM_CUDA(cudaFuncSetAttribute(gemm_tma_kernel<BN, XD, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     once.mark(dev);
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid * SPLIT);
-  cfg.blockDim = dim3(GT_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = SPLIT;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = SPLIT > 1 ? 1 : 0;
-  BM_CUDA(cudaLaunchKernelEx(&cfg, gemm_tma_kernel<BN, XD, SPLIT>, p));
+  BM_CUDA(launch_after(after, SPLIT, gemm_tma_kernel<BN, XD, SPLIT>, dim3(grid * SPLIT), GT_THREADS, smem, st, p));
   BM_LAUNCH_CHECK("gemm_tma_kernel");
   return BM_OK;
 }
 template <int BN, int SPLIT>
-static int launch_typed(const GtParams& p, int x_dtype, int grid, cudaStream_t st) {
-  if (x_dtype == BM_F32) return launch_one<BN, BM_F32, SPLIT>(p, grid, st);
-  if (x_dtype == BM_BF16) return launch_one<BN, BM_BF16, SPLIT>(p, grid, st);
-  return launch_one<BN, BM_F16, SPLIT>(p, grid, st);
+static int launch_typed(const GtParams& p, int x_dtype, LaunchAfter after, int grid, cudaStream_t st) {
+  if (x_dtype == BM_F32) return launch_one<BN, BM_F32, SPLIT>(p, after, grid, st);
+  if (x_dtype == BM_BF16) return launch_one<BN, BM_BF16, SPLIT>(p, after, grid, st);
+  return launch_one<BN, BM_F16, SPLIT>(p, after, grid, st);
 }
 
 // Returns BM_ERR_UNSUPPORTED (without having launched anything) when the shape or the pointers do not suit tiled
@@ -584,19 +582,24 @@ int launch_gemm_tma(const GemmTmaArgs& a, cudaStream_t st) {
   p.residual = a.residual; p.row_gate = a.row_gate; p.n_seg = a.n_seg; p.M = a.M;
   p.slices = a.K / GT_BK; p.slices2 = a.K2 / GT_BK;
   p.status = a.status;
+  p.beside = a.after == AFTER_BESIDE;
+  p.zero = a.zero; p.zero_n = a.zero_n;
   const int grid = split > 1 || p.ntiles < sm_counts[dev] ? p.ntiles : sm_counts[dev];
-  if (bn == 64) return split == 1 ? launch_typed<64, 1>(p, a.x_dtype, grid, st) : split == 2 ? launch_typed<64, 2>(p, a.x_dtype, grid, st) : launch_typed<64, 4>(p, a.x_dtype, grid, st);
-  if (bn == 128) return launch_typed<128, 1>(p, a.x_dtype, grid, st);
-  return launch_typed<256, 1>(p, a.x_dtype, grid, st);
+  if (bn == 64) return split == 1 ? launch_typed<64, 1>(p, a.x_dtype, a.after, grid, st) : split == 2 ? launch_typed<64, 2>(p, a.x_dtype, a.after, grid, st) : launch_typed<64, 4>(p, a.x_dtype, a.after, grid, st);
+  if (bn == 128) return launch_typed<128, 1>(p, a.x_dtype, a.after, grid, st);
+  return launch_typed<256, 1>(p, a.x_dtype, a.after, grid, st);
 }
 
 int launch_gemm_basis(const GemmTcArgs& a, int problems, cudaStream_t st) {
   GemmTmaArgs t{};
   t.X = a.X; t.x_dtype = a.x_dtype; t.M = a.M; t.K = a.K; t.residual = a.residual; t.status = a.status;
   t.n_seg = problems;
+  t.after = a.after; t.zero = a.zero; t.zero_n = a.zero_n;
   for (int i = 0; i < problems; ++i) t.seg[i] = GemmSeg{a.W[i], nullptr, a.C[i], a.N, a.c_dtype};
   const int rc = launch_gemm_tma(t, st);
-  return rc == BM_ERR_UNSUPPORTED ? launch_gemm_tc(a, problems, st) : rc;
+  if (rc != BM_ERR_UNSUPPORTED) return rc;
+  if (a.zero) BM_CUDA(cudaMemsetAsync(a.zero, 0, static_cast<size_t>(a.zero_n) * 16, st));
+  return launch_gemm_tc(a, problems, st);
 }
 
 }  // namespace bm

@@ -358,23 +358,11 @@ extern "C" int bm_layer_create(const bm_layer_desc_t* desc, void* arena, size_t 
     if (!rc) rc = plan_experts_batch(L);
     if (rc) { delete L; return rc; }
   }
-  // host-side objects for the fork/join of routing and basis projection (no device memory)
-  if (cudaStreamCreateWithFlags(&L->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&L->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&L->ev_join, cudaEventDisableTiming) != cudaSuccess) {
-    L->side_stream = nullptr;
-    (void)cudaGetLastError();
-  }
   *out = L;
   return BM_OK;
 }
 
 extern "C" int bm_layer_destroy(bm_layer_t* layer) {
-  if (layer) {
-    if (layer->ev_fork) cudaEventDestroy(layer->ev_fork);
-    if (layer->ev_join) cudaEventDestroy(layer->ev_join);
-    if (layer->side_stream) cudaStreamDestroy(layer->side_stream);
-  }
   delete layer;
   return BM_OK;
 }
@@ -440,28 +428,33 @@ extern "C" int bm_layer_decode_codes(const bm_layer_t* L, int32_t e, int32_t whi
   return BM_OK;
 }
 
-extern "C" int bm_basis_project(const bm_layer_t* L, const void* x, int x_dtype, int32_t T, uint16_t* h_gate,
-                                uint16_t* h_up, void* stream) {
-  bm::NvtxRange nvtx_range("bm_basis_project");
+// With `zero` the buffer (16-byte units) is cleared on the way.
+static int basis_project(const bm_layer_t* L, const void* x, int x_dtype, int32_t T, uint16_t* h_gate, uint16_t* h_up, LaunchAfter after, float4* zero,
+                         int64_t zero_n, cudaStream_t st) {
   BM_REQUIRE(L != nullptr, BM_ERR_INVALID_ARG, "basis_project: null layer");
   BM_REQUIRE(L->vh_gate && L->vh_up, BM_ERR_INVALID_ARG, "missing shared_vh basis for packed routed experts");
   BM_REQUIRE(T >= 0 && x_dtype >= BM_F16 && x_dtype <= BM_F32, BM_ERR_INVALID_ARG, "basis_project: bad arguments");
   if (T == 0) return BM_OK;
   BM_REQUIRE(x && h_gate && h_up, BM_ERR_INVALID_ARG, "basis_project: null pointer");
-  if (T <= SKINNY_MAX_TOKENS && L->hidden % 128 == 0) {
+  // On its own, the skinny product up to 160 tokens, whose chunks of 64 still fit the device at once (bf16, us against the tiled one: 128 tokens
+  // 7.8 / 9.0, 160 tokens 8.9 / 9.1, 203 tokens 12.4 / 9.1); the tiled one runs beside the launches before it.
+  const bool tiled = L->hidden % 64 == 0 && L->rank_in % 8 == 0 && aligned16(x, L->vh_gate, L->vh_up);
+  if (T <= (!tiled ? SKINNY_MAX_TOKENS : after == AFTER_ALL ? 160 : 0) && L->hidden % 128 == 0) {
     SkinnyArgs a{};
     a.seg[0] = SkSeg{L->vh_gate, nullptr, h_gate, L->rank_in, BM_F16, 0, 0};
     a.seg[1] = SkSeg{L->vh_up, nullptr, h_up, L->rank_in, BM_F16, 0, 0};
     a.n_seg = 2;
     a.X = x; a.N = T; a.K = L->hidden; a.x_dtype = x_dtype; a.splits = 8;
-    const int rc = launch_skinny_nt(a, static_cast<cudaStream_t>(stream));
+    a.zero = zero; a.zero_n = static_cast<int>(zero_n);
+    const int rc = launch_skinny_nt(a, st);
     if (rc != BM_ERR_UNSUPPORTED) return rc;       // shape does not tile (e.g. a very wide hidden size): the general GEMMs take it
   }
   if (L->hidden % 64 == 0 && aligned16(x, L->vh_gate, L->vh_up)) {
     GemmTcArgs t{};
     t.X = x; t.W[0] = L->vh_gate; t.W[1] = L->vh_up; t.C[0] = h_gate; t.C[1] = h_up; t.residual = nullptr;
     t.M = T; t.N = L->rank_in; t.K = L->hidden; t.x_dtype = x_dtype; t.c_dtype = BM_F16; t.status = L->status_dev;
-    return launch_gemm_basis(t, 2, static_cast<cudaStream_t>(stream));
+    t.after = after; t.zero = zero; t.zero_n = zero_n;
+    return launch_gemm_basis(t, 2, st);
   }
   GemmArgs g{};
   g.A[0] = g.A[1] = x;
@@ -476,7 +469,14 @@ extern "C" int bm_basis_project(const bm_layer_t* L, const void* x, int x_dtype,
   g.M = T;
   g.N = L->rank_in;
   g.K = L->hidden;
-  return launch_gemm_nt(g, 2, static_cast<cudaStream_t>(stream));
+  if (zero) BM_CUDA(cudaMemsetAsync(zero, 0, static_cast<size_t>(zero_n) * 16, st));
+  return launch_gemm_nt(g, 2, st);
+}
+
+extern "C" int bm_basis_project(const bm_layer_t* L, const void* x, int x_dtype, int32_t T, uint16_t* h_gate,
+                                uint16_t* h_up, void* stream) {
+  bm::NvtxRange nvtx_range("bm_basis_project");
+  return basis_project(L, x, x_dtype, T, h_gate, h_up, AFTER_ALL, nullptr, 0, static_cast<cudaStream_t>(stream));
 }
 
 // fixed-point accumulators -> fp32 rank_accum (deterministic mode)
@@ -575,23 +575,25 @@ static int combine_small(const bm_layer_t* L, const float* rank_accum, int T, co
   return launch_skinny_nt(a, st);
 }
 
-extern "C" int bm_combine_down_basis(const bm_layer_t* L, const float* rank_accum, int32_t T, const void* residual,
-                                     void* y, int y_dtype, void* stream) {
-  bm::NvtxRange nvtx_range("bm_combine_down_basis");
+static int combine_down_basis(const bm_layer_t* L, const float* rank_accum, int32_t T, const void* residual, void* y, int y_dtype, LaunchAfter after,
+                              cudaStream_t st) {
   BM_REQUIRE(L != nullptr, BM_ERR_INVALID_ARG, "combine: null layer");
   BM_REQUIRE(L->u_down, BM_ERR_INVALID_ARG, "missing shared_u_down for packed routed experts");
   BM_REQUIRE(T >= 0 && y_dtype >= BM_F16 && y_dtype <= BM_F32, BM_ERR_INVALID_ARG, "combine: bad arguments");
   if (T == 0) return BM_OK;
   BM_REQUIRE(rank_accum && y, BM_ERR_INVALID_ARG, "combine: null pointer");
-  if (T <= SKINNY_MAX_TOKENS && skinny_fits(L->rank_out, 0, 1)) {
-    const int rc = combine_small(L, rank_accum, T, nullptr, 0, nullptr, nullptr, 0, residual, y, y_dtype, false, static_cast<cudaStream_t>(stream));
+  // Up to two chunks of 64 tokens go to the skinny product (us against the tiled one: 64 tokens 5.1 / 6.1, 128 tokens 6.1 / 6.1, 203 tokens 7.9 / 6.2).
+  const bool tiled = L->rank_out % 64 == 0 && L->hidden % 8 == 0 && aligned16(rank_accum, L->u_down);
+  if ((T <= 128 || (T <= SKINNY_MAX_TOKENS && !tiled)) && skinny_fits(L->rank_out, 0, 1)) {
+    const int rc = combine_small(L, rank_accum, T, nullptr, 0, nullptr, nullptr, 0, residual, y, y_dtype, after != AFTER_ALL, st);
     if (rc != BM_ERR_UNSUPPORTED) return rc;
   }
   if (L->rank_out % 64 == 0 && aligned16(rank_accum, L->u_down)) {
     GemmTcArgs t{};
     t.X = rank_accum; t.W[0] = t.W[1] = L->u_down; t.C[0] = t.C[1] = y; t.residual = residual;
     t.M = T; t.N = L->hidden; t.K = L->rank_out; t.x_dtype = BM_F32; t.c_dtype = y_dtype; t.status = L->status_dev;
-    return launch_gemm_basis(t, 1, static_cast<cudaStream_t>(stream));
+    t.after = after;
+    return launch_gemm_basis(t, 1, st);
   }
   GemmArgs g{};
   g.A[0] = g.A[1] = rank_accum;
@@ -604,7 +606,13 @@ extern "C" int bm_combine_down_basis(const bm_layer_t* L, const float* rank_accu
   g.M = T;
   g.N = L->hidden;
   g.K = L->rank_out;
-  return launch_gemm_nt(g, 1, static_cast<cudaStream_t>(stream));
+  return launch_gemm_nt(g, 1, st);
+}
+
+extern "C" int bm_combine_down_basis(const bm_layer_t* L, const float* rank_accum, int32_t T, const void* residual,
+                                     void* y, int y_dtype, void* stream) {
+  bm::NvtxRange nvtx_range("bm_combine_down_basis");
+  return combine_down_basis(L, rank_accum, T, residual, y, y_dtype, AFTER_ALL, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" size_t bm_layer_workspace_bytes(const bm_layer_t* L, int32_t T, int32_t k) {
@@ -612,7 +620,7 @@ extern "C" size_t bm_layer_workspace_bytes(const bm_layer_t* L, int32_t T, int32
   return carve_layer_ws(L, nullptr, T, k).total;
 }
 
-// A decode batch (up to 256 tokens) in three or four launches, each starting while the one before drains:
+// A decode batch in three or four launches, each starting while the one before drains:
 //   1. everything that multiplies x -- the basis projection and, for a whole block, router logits, the shared expert's
 //      gated pair and its token gate -- with the expert stage's accumulator cleared on the way; given logits are routed
 //      by one more cluster of the same grid
@@ -620,12 +628,25 @@ extern "C" size_t bm_layer_workspace_bytes(const bm_layer_t* L, int32_t T, int32
 //   3. packed experts
 //   4. down basis, shared expert's down product and residual
 // BM_ERR_UNSUPPORTED, with nothing launched, when a shape does not tile; the general path takes it.
+//
+// Up to how many tokens, where the chain of tiled products (forward_large, the general layer path) takes the sizes, us a call of these
+// launches / of the chain.  Layer, 128 experts, fp16: 64 tokens 30.6 / 31.9, 80 32.1 / 31.4, 203 46.5 / 36.9; 64 experts, bf16, whose tiled
+// product of x has to be rounded in shared memory, behind the shared experts: 112 tokens 158 / 160, 144 205 / 201.  Block of 128 experts, bf16:
+// 64 tokens 37.6 / 39.1, 80 39.7 / 39.7, 203 72.7 / 53.3.  Of 512 experts and a gated shared one, whose first launch no longer fits
+// the device at once with a second chunk of tokens: 48 tokens 71.5 / 73.8, 64 81.1 / 76.2, 96 113.8 / 77.8, 256 200.7 / 85.1.
+static int small_tokens(const bm_layer_t* L, const bm_block_dense_t* d, int x_dtype) {
+  const bool shared = d && d->sh_intermediate > 0;
+  if (L->hidden % 64 != 0 || L->rank_in % 8 != 0 || L->rank_out % 64 != 0 || (shared && d->sh_intermediate % 64 != 0) || (d && L->num_experts % 8 != 0))
+    return SKINNY_MAX_TOKENS;
+  if (d) return shared ? 48 : 80;
+  return x_dtype == BM_F16 ? 64 : 128;
+}
 static int forward_small(const bm_layer_t* L, const bm_block_dense_t* d, const void* x, int x_dtype, void* logits, int logits_dtype, int T,
                          int k, int renorm, int weight_round, const void* residual, void* y, int path, const LayerWs& w, float* z, float* gate,
                          cudaStream_t st) {
   const bool shared = d && d->sh_intermediate > 0;
   if (!x || !y || !logits || x_dtype < BM_F16 || x_dtype > BM_F32 || logits_dtype < BM_F16 || logits_dtype > BM_F32) return BM_ERR_UNSUPPORTED;
-  if (T > SKINNY_MAX_TOKENS || L->hidden % 128 != 0 || (reinterpret_cast<uintptr_t>(x) & 15u) || !L->vh_gate || !L->vh_up || !L->u_down ||
+  if (T > small_tokens(L, d, x_dtype) || L->hidden % 128 != 0 || (reinterpret_cast<uintptr_t>(x) & 15u) || !L->vh_gate || !L->vh_up || !L->u_down ||
       !skinny_fits(L->hidden, 0, 8) || !skinny_fits(L->rank_out, shared ? d->sh_intermediate : 0, 1) || !route_small_fits(T, L->num_experts, k))
     return BM_ERR_UNSUPPORTED;
   auto aligned = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
@@ -681,43 +702,32 @@ extern "C" int bm_layer_forward(const bm_layer_t* L, const void* x, int x_dtype,
                                  w, nullptr, nullptr, static_cast<cudaStream_t>(stream));
     if (rc != BM_ERR_UNSUPPORTED) return rc;
   }
-  // routing depends only on the logits and the basis projection only on x: run them side by side
+  // One stream, every launch set up while the one before it runs.  The basis projection depends only on x and runs beside the
+  // routing's placement, which takes a cluster; the accumulator of the expert stage is cleared by its idle warps.
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const bool fork = L->side_stream != nullptr && L->ev_fork != nullptr && L->ev_join != nullptr;
-  void* route_stream = stream;
-  if (fork) {
-    BM_CUDA(cudaEventRecord(L->ev_fork, st));
-    BM_CUDA(cudaStreamWaitEvent(L->side_stream, L->ev_fork, 0));
-    route_stream = L->side_stream;
-  }
-  int rc = bm_route(logits, logits_dtype, T, num_routed, k, renorm, weight_round, global_to_local, L->num_experts, TILE_ROWS,
-                    w.topk_idx, w.topk_w, w.token_indices, w.expert_offsets, w.route_flat, /*tile_table=*/nullptr, /*counts=*/nullptr,
-                    w.route_ws, w.route_ws_bytes, route_stream);
-  // the routing's four launches are the longer of the two ways at large batches: the accumulator of the expert stage is
-  // cleared behind the basis projection
-  const size_t acc_bytes = sizeof(float) * static_cast<size_t>(T) * L->rank_out;
-  const int rc_basis = bm_basis_project(L, x, x_dtype, T, reinterpret_cast<uint16_t*>(w.h_gate), reinterpret_cast<uint16_t*>(w.h_up), stream);
-  const bool zeroed = cudaMemsetAsync(w.rank_accum, 0, acc_bytes, st) == cudaSuccess;
-  if (fork) {
-    // always join, also on error, so that the side stream never stays attached to a capture
-    cudaEventRecord(L->ev_join, L->side_stream);
-    cudaStreamWaitEvent(st, L->ev_join, 0);
-  }
+  int rc = route_tokens(logits, logits_dtype, T, num_routed, k, renorm, weight_round, global_to_local, L->num_experts, TILE_ROWS, w.topk_idx, w.topk_w,
+                        w.token_indices, w.expert_offsets, w.route_flat, /*tile_table=*/nullptr, /*counts=*/nullptr, w.route_ws, w.route_ws_bytes,
+                        AFTER_ALL, /*beside_follows=*/true, st);
   if (rc) return rc;
-  if (rc_basis) return rc_basis;
+  const size_t acc_bytes = sizeof(float) * static_cast<size_t>(T) * L->rank_out;
+  const bool zeroed = acc_bytes % 16 == 0;
+  rc = basis_project(L, x, x_dtype, T, reinterpret_cast<uint16_t*>(w.h_gate), reinterpret_cast<uint16_t*>(w.h_up), AFTER_BESIDE,
+                     zeroed ? reinterpret_cast<float4*>(w.rank_accum) : nullptr, static_cast<int64_t>(acc_bytes / 16), st);
+  if (rc) return rc;
   // Dropped assignments (experts that are not packed) leave a shorter list; the kernels walk
   // expert_offsets, so passing the upper bound T*k as num_assign is safe.
   rc = experts_forward_impl(L, reinterpret_cast<const uint16_t*>(w.h_gate), reinterpret_cast<const uint16_t*>(w.h_up),
                             w.token_indices, w.expert_offsets, w.route_flat, T, T * k, w.rank_accum, path, zeroed, w.experts_ws,
                             w.experts_ws_bytes, stream);
   if (rc) return rc;
-  return bm_combine_down_basis(L, w.rank_accum, T, residual, y, x_dtype == BM_F32 ? BM_F32 : x_dtype, stream);
+  return combine_down_basis(L, w.rank_accum, T, residual, y, x_dtype == BM_F32 ? BM_F32 : x_dtype, AFTER_READS, st);
 }
 
 // bf16 weights -> fp16, several matrices per launch (piece i: n[i] groups of eight values)
 struct CastArgs { const uint4* src[5]; uint4* dst[5]; int n[5]; };
 __global__ void __launch_bounds__(256) cast_weights_kernel(const __grid_constant__ CastArgs a) {
   const int p = blockIdx.y;
+  grid_launch_dependents();
   for (int i = blockIdx.x * 256 + threadIdx.x; i < a.n[p]; i += gridDim.x * 256) {
     uint4 v = __ldg(a.src[p] + i);
     uint32_t* o = reinterpret_cast<uint32_t*>(&v);
@@ -755,7 +765,7 @@ static BlockWs carve_block_ws(const bm_layer_t* L, const bm_block_dense_t* d, in
 // launched that matters, when a shape or pointer does not suit the tiled-copy GEMM.
 static int forward_large(const bm_layer_t* L, const bm_block_dense_t& d, const void* x, int x_dtype, int T, int num_routed, int k, int renorm,
                          int weight_round, const int32_t* global_to_local, void* logits, void* y, const LayerWs& w, const BlockWs& b,
-                         cudaStream_t st) {
+                         const uint16_t* token_gate, int token_gate_dtype, LaunchAfter after, cudaStream_t st) {
   const bool shared = d.sh_intermediate > 0;
   if (!L->vh_gate || !L->vh_up || !L->u_down || L->rank_out % 64 != 0 || (shared && d.sh_intermediate % 64 != 0)) return BM_ERR_UNSUPPORTED;
   auto h = [](const uint16_t* p) { return reinterpret_cast<const __half*>(p); };
@@ -763,7 +773,10 @@ static int forward_large(const bm_layer_t* L, const bm_block_dense_t& d, const v
   __half* z = static_cast<__half*>(b.dense_ws);
   float* gate = reinterpret_cast<float*>(static_cast<unsigned char*>(b.dense_ws) + 3 * mat);
   int rc;
-  if (shared && d.sh_token_gate && (rc = launch_row_gate(x, x_dtype, h(d.sh_token_gate), T, L->hidden, gate, st))) return rc;
+  if (shared && d.sh_token_gate) {
+    if ((rc = launch_row_gate(x, x_dtype, token_gate, token_gate_dtype, T, L->hidden, gate, after == AFTER_ALL ? AFTER_ALL : AFTER_BESIDE, st))) return rc;
+    after = AFTER_READS;
+  }
   GemmTmaArgs a{};
   a.X = x; a.x_dtype = x_dtype; a.M = T; a.K = L->hidden; a.status = L->status_dev;
   a.seg[0] = GemmSeg{h(d.gate_w), nullptr, logits, num_routed, x_dtype};
@@ -772,10 +785,11 @@ static int forward_large(const bm_layer_t* L, const bm_block_dense_t& d, const v
   if (shared) a.seg[3] = GemmSeg{h(d.sh_gate), h(d.sh_up), z, d.sh_intermediate, BM_F16};
   a.n_seg = shared ? 4 : 3;
   a.row_gate = shared && d.sh_token_gate ? gate : nullptr;
+  a.after = after;
+  a.zero = reinterpret_cast<float4*>(w.rank_accum); a.zero_n = static_cast<int64_t>(T) * L->rank_out / 4;      // (rank_out is a multiple of 64)
   if ((rc = launch_gemm_tma(a, st))) return rc;
-  BM_CUDA(cudaMemsetAsync(w.rank_accum, 0, sizeof(float) * static_cast<size_t>(T) * L->rank_out, st));
-  rc = bm_route(logits, x_dtype, T, num_routed, k, renorm, weight_round, global_to_local, L->num_experts, TILE_ROWS, w.topk_idx, w.topk_w,
-                w.token_indices, w.expert_offsets, w.route_flat, nullptr, nullptr, w.route_ws, w.route_ws_bytes, st);
+  rc = route_tokens(logits, x_dtype, T, num_routed, k, renorm, weight_round, global_to_local, L->num_experts, TILE_ROWS, w.topk_idx, w.topk_w,
+                    w.token_indices, w.expert_offsets, w.route_flat, nullptr, nullptr, w.route_ws, w.route_ws_bytes, AFTER_READS, /*beside_follows=*/false, st);
   if (rc) return rc;
   rc = experts_forward_impl(L, reinterpret_cast<const uint16_t*>(w.h_gate), reinterpret_cast<const uint16_t*>(w.h_up), w.token_indices,
                             w.expert_offsets, w.route_flat, T, T * k, w.rank_accum, BM_PATH_AUTO, true, w.experts_ws, w.experts_ws_bytes, st);
@@ -784,6 +798,7 @@ static int forward_large(const bm_layer_t* L, const bm_block_dense_t& d, const v
   c.X = w.rank_accum; c.x_dtype = BM_F32; c.M = T; c.K = L->rank_out; c.status = L->status_dev;
   c.seg[0] = GemmSeg{L->u_down, nullptr, y, L->hidden, x_dtype};
   c.n_seg = 1;
+  c.after = AFTER_READS;
   if (shared) { c.X2 = z; c.W2 = h(d.sh_down); c.K2 = d.sh_intermediate; }
   rc = launch_gemm_tma(c, st);
   if (rc != BM_ERR_UNSUPPORTED) return rc;
@@ -847,7 +862,8 @@ extern "C" int bm_block_forward(const bm_layer_t* L, const bm_block_dense_t* den
     cast_weights_kernel<<<dim3(148, 5), 256, 0, st>>>(c);
     BM_LAUNCH_CHECK("cast_weights_kernel");
   }
-  int rc = forward_large(L, d, x, x_dtype, T, num_routed, k, renorm, weight_round, global_to_local, logits, y, w, b, st);
+  int rc = forward_large(L, d, x, x_dtype, T, num_routed, k, renorm, weight_round, global_to_local, logits, y, w, b, dense->sh_token_gate, d.w_dtype,
+                         d.w_dtype == BM_BF16 ? AFTER_READS : AFTER_ALL, st);
   if (rc != BM_ERR_UNSUPPORTED) return rc;
   rc = bm_gate_logits(x, x_dtype, d.gate_w, T, num_routed, L->hidden, logits, x_dtype, stream);
   if (rc) return rc;

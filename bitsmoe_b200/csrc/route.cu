@@ -11,6 +11,8 @@
 // What bounds it is latency: four dependent launches.  16384 tokens of 512 experts, top 10: top-k 52 -> 24.5 us (topk.cuh),
 // prefixes of the block histograms 16.5 -> 4 us (one block walked them; now a thread of a grid per expert, and the totals
 // are scanned where they are used), counting 5, scatter 8.
+#include <cooperative_groups.h>
+
 #include "topk.cuh"
 
 namespace bm {
@@ -27,6 +29,8 @@ __global__ void __launch_bounds__(256) route_topk_kernel(const void* __restrict_
                                                         float* __restrict__ topk_w) {
   const int lane = threadIdx.x & 31;
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  grid_launch_dependents();
+  grid_wait();
   if (t >= T) return;
   int idx;
   float w;
@@ -171,6 +175,8 @@ __global__ void __launch_bounds__(ROUTE_BLOCK) route_build_fused_kernel(
     float* __restrict__ route_flat, int32_t* __restrict__ tile_table, int max_tiles, int32_t* __restrict__ counts) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   RouteSmem s = carve_route_smem(sm_raw, E);
+  grid_launch_dependents();
+  grid_wait();
   const int i = threadIdx.x;
   int e = -1;
   if (i < A) e = local_expert(topk_idx, g2l, i, num_routed, E);
@@ -187,12 +193,92 @@ __global__ void __launch_bounds__(ROUTE_BLOCK) route_build_fused_kernel(
   write_tile_table(s.scan, E, tile_rows, tile_table, max_tiles, counts, reinterpret_cast<int*>(s.warp_base), s.block_count);
 }
 
-// A > ROUTE_BLOCK: counts per block of assignments, prefixes across the blocks, scatter.
+// Up to PLACE_CTAS x 1024 x PLACE_ROUNDS assignments by one cluster.  A CTA takes `rounds` x 1024 consecutive ones, a warp `rounds` x 32 of
+// them, which it counts round by round into a table of its own; prefixes over the warps, over the CTAs (distributed shared memory) and
+// over the experts give every assignment its place.
+constexpr int PLACE_CTAS = 8, PLACE_ROUNDS = 8;
+template <int ROUNDS>
+__global__ void __launch_bounds__(ROUTE_BLOCK) route_place_kernel(
+    const int32_t* __restrict__ topk_idx, const float* __restrict__ topk_w, const int32_t* __restrict__ g2l, int num_routed,
+    int A, int k, int E, int tile_rows, int32_t* __restrict__ token_indices, int32_t* __restrict__ expert_offsets,
+    float* __restrict__ route_flat, int32_t* __restrict__ tile_table, int max_tiles, int32_t* __restrict__ counts) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  const RouteSmem s = carve_route_smem(sm_raw, E);      // warp_base: counts, then prefixes over the warps; block_count: this CTA's counts
+  int* const total = reinterpret_cast<int*>(sm_raw + route_smem_bytes_dev(E));
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int rank = static_cast<int>(cluster.block_rank()), ctas = static_cast<int>(cluster.num_blocks());
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  grid_launch_dependents();
+  for (int i = threadIdx.x; i < ROUTE_WARPS * E / 2; i += ROUTE_BLOCK) reinterpret_cast<uint32_t*>(s.warp_base)[i] = 0u;
+  grid_wait();
+  const int i0 = (rank * ROUTE_WARPS + warp) * (32 * ROUNDS) + lane;
+  int e[ROUNDS], pos[ROUNDS];
+#pragma unroll
+  for (int r = 0; r < ROUNDS; ++r) e[r] = i0 + 32 * r < A ? local_expert(topk_idx, g2l, i0 + 32 * r, num_routed, E) : -1;
+  __syncthreads();
+  uint16_t* const mine = s.warp_base + warp * E;
+#pragma unroll
+  for (int r = 0; r < ROUNDS; ++r) {
+    const unsigned peers = __match_any_sync(0xffffffffu, e[r]);
+    const int below = __popc(peers & ((1u << lane) - 1u)), had = e[r] >= 0 ? mine[e[r]] : 0;
+    __syncwarp();
+    if (e[r] >= 0 && below == 0) mine[e[r]] = static_cast<uint16_t>(had + __popc(peers));
+    __syncwarp();
+    pos[r] = had + below;
+  }
+  __syncthreads();
+  for (int x = threadIdx.x; x < E; x += ROUTE_BLOCK) {
+    int run = 0;
+#pragma unroll 8
+    for (int w = 0; w < ROUTE_WARPS; ++w) {
+      const int c = s.warp_base[w * E + x];
+      s.warp_base[w * E + x] = static_cast<uint16_t>(run);      // a CTA holds at most PLACE_ROUNDS x 1024 of an expert
+      run += c;
+    }
+    s.block_count[x] = run;
+  }
+  cluster.sync();
+  int before = 0;
+  const int x = threadIdx.x;
+  if (x < E) {
+    int all = 0;
+#pragma unroll
+    for (int c = 0; c < PLACE_CTAS; ++c) {
+      const int n = c < ctas ? cluster.map_shared_rank(s.block_count, c)[x] : 0;
+      before += c < rank ? n : 0;
+      all += n;
+    }
+    total[x] = all;
+  }
+  const auto read = cluster.barrier_arrive();              // a CTA's counts may go once everybody has read them
+  __syncthreads();
+  block_exclusive_scan(total, s.scan, E);
+  if (x < E) total[x] = s.scan[x] + before;                // where this CTA's assignments of the expert start
+  __syncthreads();
+#pragma unroll
+  for (int r = 0; r < ROUNDS; ++r) {
+    if (e[r] < 0) continue;
+    const int at = total[e[r]] + mine[e[r]] + pos[r], i = i0 + 32 * r;
+    token_indices[at] = i / k;
+    route_flat[at] = topk_w[i];
+  }
+  cluster.barrier_wait(cg::cluster_group::arrival_token(read));
+  if (rank == 0) {
+    for (int j = threadIdx.x; j <= E; j += ROUTE_BLOCK) expert_offsets[j] = s.scan[j];
+    __syncthreads();
+    write_tile_table(s.scan, E, tile_rows, tile_table, max_tiles, counts, reinterpret_cast<int*>(s.warp_base), s.block_count);
+  }
+}
+
+// More assignments: counts per block of assignments, prefixes across the blocks, scatter.
 __global__ void __launch_bounds__(ROUTE_BLOCK) route_count_kernel(const int32_t* __restrict__ topk_idx,
                                                                  const int32_t* __restrict__ g2l, int num_routed, int A, int E,
                                                                  int32_t* __restrict__ block_hist /*[nblocks][E]*/) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   RouteSmem s = carve_route_smem(sm_raw, E);
+  grid_launch_dependents();
+  grid_wait();
   const int i = blockIdx.x * ROUTE_BLOCK + threadIdx.x;
   int e = -1;
   if (i < A) e = local_expert(topk_idx, g2l, i, num_routed, E);
@@ -206,6 +292,8 @@ __global__ void __launch_bounds__(ROUTE_BLOCK) route_scan_kernel(int32_t* __rest
                                                                 int32_t* __restrict__ total) {
   __shared__ int run_tot[ROUTE_WARPS][33];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, x = blockIdx.x * 32 + lane;
+  grid_launch_dependents();
+  grid_wait();
   const int len = (nblocks + ROUTE_WARPS - 1) / ROUTE_WARPS, b0 = warp * len, b1 = min(nblocks, b0 + len);
   int sum = 0;
   if (x < E)
@@ -233,6 +321,8 @@ __global__ void __launch_bounds__(ROUTE_BLOCK) route_scatter_kernel(
     int max_tiles, int32_t* __restrict__ counts) {
   extern __shared__ __align__(16) unsigned char sm_raw[];
   RouteSmem s = carve_route_smem(sm_raw, E);
+  grid_launch_dependents();
+  grid_wait();
   block_exclusive_scan(total, s.scan, E);
   const int i = blockIdx.x * ROUTE_BLOCK + threadIdx.x;
   int e = -1;
@@ -267,15 +357,16 @@ static int set_route_attributes(int dev) {
   BM_CUDA(cudaFuncSetAttribute(route_build_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   BM_CUDA(cudaFuncSetAttribute(route_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
   BM_CUDA(cudaFuncSetAttribute(route_scatter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big));
+  for (auto* kernel : {route_place_kernel<1>, route_place_kernel<2>, route_place_kernel<4>, route_place_kernel<8>})
+    BM_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, big + ROUTE_MAX_E * static_cast<int>(sizeof(int))));
   attr_once.mark(dev);
   return BM_OK;
 }
 
 }  // namespace bm
 
-extern "C" int bm_route_topk(const void* logits, int logits_dtype, int32_t T, int32_t E, int32_t k, int32_t renorm,
-                             int32_t weight_round, int32_t* topk_idx, float* topk_w, void* stream) {
-  bm::NvtxRange nvtx_range("bm_route_topk");
+static int route_topk(const void* logits, int logits_dtype, int32_t T, int32_t E, int32_t k, int32_t renorm,
+                             int32_t weight_round, int32_t* topk_idx, float* topk_w, bm::LaunchAfter after, cudaStream_t st) {
   using namespace bm;
   BM_REQUIRE(T >= 0 && E > 0 && k > 0, BM_ERR_INVALID_ARG, "route_topk: bad sizes T=%d E=%d k=%d", T, E, k);
   BM_REQUIRE(k <= 32 && k <= E, BM_ERR_UNSUPPORTED, "route_topk: top_k=%d must be <= min(32, E=%d)", k, E);
@@ -284,10 +375,16 @@ extern "C" int bm_route_topk(const void* logits, int logits_dtype, int32_t T, in
   if (T == 0) return BM_OK;
   BM_REQUIRE(logits && topk_idx && topk_w, BM_ERR_INVALID_ARG, "route_topk: null pointer");
   const int warps = 8;
-  BM_TOPK_CLASS(E, (route_topk_kernel<REG><<<(T + warps - 1) / warps, warps * 32, 0, static_cast<cudaStream_t>(stream)>>>(
-                       logits, logits_dtype, T, E, k, renorm, weight_round, topk_idx, topk_w)));
+  BM_TOPK_CLASS(E, BM_CUDA(launch_after(after, 1, route_topk_kernel<REG>, dim3((T + warps - 1) / warps), warps * 32, 0, st, logits, logits_dtype, T,
+                                        E, k, renorm, weight_round, topk_idx, topk_w)));
   BM_LAUNCH_CHECK("route_topk_kernel");
   return BM_OK;
+}
+
+extern "C" int bm_route_topk(const void* logits, int logits_dtype, int32_t T, int32_t E, int32_t k, int32_t renorm,
+                             int32_t weight_round, int32_t* topk_idx, float* topk_w, void* stream) {
+  bm::NvtxRange nvtx_range("bm_route_topk");
+  return route_topk(logits, logits_dtype, T, E, k, renorm, weight_round, topk_idx, topk_w, bm::AFTER_ALL, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int32_t bm_route_max_tiles(int32_t T, int32_t k, int32_t num_local, int32_t tile_rows) {
@@ -305,12 +402,11 @@ extern "C" size_t bm_route_build_workspace_bytes(int32_t T, int32_t k, int32_t n
   return bm::align_up(static_cast<size_t>((A + bm::ROUTE_BLOCK - 1) / bm::ROUTE_BLOCK + 1) * num_local * sizeof(int32_t), 256);     // histograms, totals
 }
 
-extern "C" int bm_route_build(const int32_t* topk_idx, const float* topk_w, const int32_t* global_to_local,
+static int route_build(const int32_t* topk_idx, const float* topk_w, const int32_t* global_to_local,
                               int32_t num_routed, int32_t T,
                               int32_t k, int32_t num_local, int32_t tile_rows, int32_t* token_indices,
                               int32_t* expert_offsets, float* route_flat, int32_t* tile_table, int32_t* counts,
-                              void* workspace, size_t workspace_bytes, void* stream) {
-  bm::NvtxRange nvtx_range("bm_route_build");
+                              void* workspace, size_t workspace_bytes, bm::LaunchAfter after, bool beside_follows, cudaStream_t st) {
   using namespace bm;
   BM_REQUIRE(T >= 0 && k > 0 && num_local > 0 && num_routed > 0, BM_ERR_INVALID_ARG, "route_build: bad sizes");
   BM_REQUIRE(global_to_local != nullptr || num_routed == num_local, BM_ERR_INVALID_ARG,
@@ -322,7 +418,6 @@ extern "C" int bm_route_build(const int32_t* topk_idx, const float* topk_w, cons
   BM_REQUIRE(A64 < (1ll << 30), BM_ERR_UNSUPPORTED, "route_build: too many assignments");
   const int A = static_cast<int>(A64);
   BM_REQUIRE(A == 0 || (topk_idx && topk_w && token_indices && route_flat), BM_ERR_INVALID_ARG, "route_build: null pointer");
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int max_tiles = bm_route_max_tiles(T, k, num_local, tile_rows);
   const size_t smem = route_smem_bytes(num_local);
   int dev = -1;
@@ -330,9 +425,8 @@ extern "C" int bm_route_build(const int32_t* topk_idx, const float* topk_w, cons
   const int rc = set_route_attributes(dev);
   if (rc) return rc;
   if (A <= ROUTE_BLOCK) {
-    route_build_fused_kernel<<<1, ROUTE_BLOCK, smem, st>>>(topk_idx, topk_w, global_to_local, num_routed, A, k, num_local, tile_rows,
-                                                           token_indices, expert_offsets, route_flat, tile_table,
-                                                           max_tiles, counts);
+    BM_CUDA(launch_after(after, 1, route_build_fused_kernel, dim3(1), ROUTE_BLOCK, smem, st, topk_idx, topk_w, global_to_local, num_routed, A, k,
+                         num_local, tile_rows, token_indices, expert_offsets, route_flat, tile_table, max_tiles, counts));
     BM_LAUNCH_CHECK("route_build_fused_kernel");
     return BM_OK;
   }
@@ -340,16 +434,48 @@ extern "C" int bm_route_build(const int32_t* topk_idx, const float* topk_w, cons
   const size_t need = bm_route_build_workspace_bytes(T, k, num_local);
   BM_REQUIRE(workspace && workspace_bytes >= need, BM_ERR_WORKSPACE, "route_build: workspace of %zu bytes needed, %zu given",
              need, workspace_bytes);
+  // One launch of a cluster against three over all SMs, us on 128 experts: 8192 assignments 6.6 / 10.8, 16384 9.0 / 11.3, 32768 13.6 / 11.4,
+  // 65536 23.4 / 12.5 (eight SMs scatter 4-byte words).  With a launch beside it the cluster's time does not show up to the largest.
+  if (A <= PLACE_CTAS * ROUTE_BLOCK * (beside_follows ? PLACE_ROUNDS : 2)) {
+    int rounds = 1, ctas = 2;
+    while (rounds * PLACE_CTAS * ROUTE_BLOCK < A) rounds *= 2;
+    while (ctas * rounds * ROUTE_BLOCK < A) ctas *= 2;
+    auto* kernel = rounds == 1 ? route_place_kernel<1> : rounds == 2 ? route_place_kernel<2> : rounds == 4 ? route_place_kernel<4> : route_place_kernel<8>;
+    BM_CUDA(launch_after(after, ctas, kernel, dim3(ctas), ROUTE_BLOCK, smem + num_local * sizeof(int), st, topk_idx, topk_w, global_to_local, num_routed,
+                         A, k, num_local, tile_rows, token_indices, expert_offsets, route_flat, tile_table, max_tiles, counts));
+    BM_LAUNCH_CHECK("route_place_kernel");
+    return BM_OK;
+  }
   int32_t* total = static_cast<int32_t*>(workspace);
   int32_t* block_hist = total + num_local;
-  route_count_kernel<<<nblocks, ROUTE_BLOCK, smem, st>>>(topk_idx, global_to_local, num_routed, A, num_local, block_hist);
+  BM_CUDA(launch_after(after, 1, route_count_kernel, dim3(nblocks), ROUTE_BLOCK, smem, st, topk_idx, global_to_local, num_routed, A, num_local, block_hist));
   BM_LAUNCH_CHECK("route_count_kernel");
-  route_scan_kernel<<<(num_local + 31) / 32, ROUTE_BLOCK, 0, st>>>(block_hist, nblocks, num_local, total);
+  BM_CUDA(launch_after(AFTER_READS, 1, route_scan_kernel, dim3((num_local + 31) / 32), ROUTE_BLOCK, 0, st, block_hist, nblocks, num_local, total));
   BM_LAUNCH_CHECK("route_scan_kernel");
-  route_scatter_kernel<<<nblocks, ROUTE_BLOCK, smem, st>>>(topk_idx, topk_w, global_to_local, num_routed, A, k, num_local, block_hist,
-                                                           total, tile_rows, expert_offsets, token_indices, route_flat, tile_table, max_tiles, counts);
+  BM_CUDA(launch_after(AFTER_READS, 1, route_scatter_kernel, dim3(nblocks), ROUTE_BLOCK, smem, st, topk_idx, topk_w, global_to_local, num_routed, A, k,
+                       num_local, block_hist, total, tile_rows, expert_offsets, token_indices, route_flat, tile_table, max_tiles, counts));
   BM_LAUNCH_CHECK("route_scatter_kernel");
   return BM_OK;
+}
+
+extern "C" int bm_route_build(const int32_t* topk_idx, const float* topk_w, const int32_t* global_to_local,
+                              int32_t num_routed, int32_t T,
+                              int32_t k, int32_t num_local, int32_t tile_rows, int32_t* token_indices,
+                              int32_t* expert_offsets, float* route_flat, int32_t* tile_table, int32_t* counts,
+                              void* workspace, size_t workspace_bytes, void* stream) {
+  bm::NvtxRange nvtx_range("bm_route_build");
+  return route_build(topk_idx, topk_w, global_to_local, num_routed, T, k, num_local, tile_rows, token_indices, expert_offsets, route_flat,
+                     tile_table, counts, workspace, workspace_bytes, bm::AFTER_ALL, false, static_cast<cudaStream_t>(stream));
+}
+
+int bm::route_tokens(const void* logits, int logits_dtype, int32_t T, int32_t E_routed, int32_t k, int32_t renorm, int32_t weight_round,
+                     const int32_t* global_to_local, int32_t num_local, int32_t tile_rows, int32_t* topk_idx, float* topk_w,
+                     int32_t* token_indices, int32_t* expert_offsets, float* route_flat, int32_t* tile_table, int32_t* counts, void* workspace,
+                     size_t workspace_bytes, LaunchAfter after, bool beside_follows, cudaStream_t st) {
+  const int rc = route_topk(logits, logits_dtype, T, E_routed, k, renorm, weight_round, topk_idx, topk_w, after, st);
+  if (rc) return rc;
+  return route_build(topk_idx, topk_w, global_to_local, E_routed, T, k, num_local, tile_rows, token_indices, expert_offsets, route_flat, tile_table,
+                     counts, workspace, workspace_bytes, T > 0 ? AFTER_READS : after, beside_follows, st);
 }
 
 extern "C" int bm_route(const void* logits, int logits_dtype, int32_t T, int32_t E_routed, int32_t k, int32_t renorm,
@@ -358,9 +484,7 @@ extern "C" int bm_route(const void* logits, int logits_dtype, int32_t T, int32_t
                         float* route_flat, int32_t* tile_table, int32_t* counts, void* workspace, size_t workspace_bytes,
                         void* stream) {
   bm::NvtxRange nvtx_range("bm_route");
-  using namespace bm;
-  int rc = bm_route_topk(logits, logits_dtype, T, E_routed, k, renorm, weight_round, topk_idx, topk_w, stream);
-  if (rc) return rc;
-  return bm_route_build(topk_idx, topk_w, global_to_local, E_routed, T, k, num_local, tile_rows, token_indices,
-                        expert_offsets, route_flat, tile_table, counts, workspace, workspace_bytes, stream);
+  return bm::route_tokens(logits, logits_dtype, T, E_routed, k, renorm, weight_round, global_to_local, num_local, tile_rows, topk_idx, topk_w,
+                          token_indices, expert_offsets, route_flat, tile_table, counts, workspace, workspace_bytes, bm::AFTER_ALL, false,
+                          static_cast<cudaStream_t>(stream));
 }

@@ -5,7 +5,7 @@
 
 namespace bm {
 
-constexpr int SKINNY_MAX_TOKENS = 256;   // above this the tcgen05 GEMM streams the weights fewer times
+constexpr int SKINNY_MAX_TOKENS = 256;   // callers hand over to the tcgen05 GEMM at their own, lower counts where it takes the shape
 constexpr int SK_MAX_SEG = 6;
 
 // One stack of output rows: C[n][m] = sum_k W[m][k] X[n][k] for m < rows, stored at C[n * rows + m].  With W_up set the
@@ -58,7 +58,7 @@ bool skinny_fits(int K, int K2, int splits);
 int skinny_splits(int rows, int K);
 
 // gate[t] = sigmoid(x[t] . w) (dense.cu)
-int launch_row_gate(const void* x, int x_dtype, const __half* w, int T, int H, float* gate, cudaStream_t st);
+int launch_row_gate(const void* x, int x_dtype, const uint16_t* w, int w_dtype, int T, int H, float* gate, LaunchAfter after, cudaStream_t st);
 
 bool route_small_fits(int T, int E, int k);
 int launch_route_small(const RouteSmallArgs& a, cudaStream_t st);

@@ -113,8 +113,8 @@ def test_rows_that_repeat_a_rank():
 
 
 # token counts around the blocks of the counting pass; expert counts around a warp of the scan and the top-k's registers
-@pytest.mark.parametrize("T", [129, 1025, 4097, 16385])
-@pytest.mark.parametrize("E,k", [(2, 2), (33, 5), (128, 8), (512, 10)])
+@pytest.mark.parametrize("T", [129, 205, 1025, 2048, 2049, 4097, 16385])
+@pytest.mark.parametrize("E,k", [(2, 2), (33, 5), (128, 8), (512, 10), (1024, 4)])
 def test_routing_is_the_stable_permutation(T, E, k):
     logits = torch.randn(T, E, device=DEV).round(decimals=1)      # ties: the lower expert id comes first
     idx, w = route_topk(logits, k, False, torch.float32)
@@ -210,3 +210,27 @@ def test_split_gated_pair(T, inter):
     # z is rounded to fp16 (one rounding, and what the fp32 sums and __expf add: a few 2^-20), y as well
     bound = 2.0 ** -10 * (z.abs() @ wd.double().abs().t()) + 2.0 ** -11 * want.abs() + 2.0 ** -24
     assert float(((dense_mlp(x, wg, wu, wd).double() - want).abs() / bound).max()) <= 1.0
+
+
+# the layer's one call against its stages: assignments that one, two, four and eight rounds of the routing's cluster take and more than it
+# takes, tokens around the launch chains' limits, a rank that is no multiple of a slice
+@pytest.mark.parametrize("T,E,k,rank", [(49, 8, 2, 64), (65, 8, 2, 64), (129, 8, 2, 64), (129, 8, 2, 72), (300, 40, 8, 64), (2049, 16, 4, 64),
+                                        (4097, 16, 4, 64), (8193, 8, 4, 64), (16385, 8, 4, 64)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_layer_call_is_its_stages(T, E, k, rank, dtype):
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=128, top_k=k, rank=rank)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=T, device=DEV))
+    layer.set_deterministic(True)
+    gen = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn(T, 128, generator=gen, device=DEV).to(dtype)
+    logits = torch.randn(T, E, generator=gen, device=DEV)
+    res = torch.randn(T, 128, generator=gen, device=DEV).to(dtype)
+    idx, w = route_topk(logits, k, True, dtype)
+    tok, off, rw, _, _ = route_build(idx, w, E)
+    hg, hu = layer.basis_project(x)
+    want = layer.combine_down_basis(layer.experts_forward(hg, hu, tok, off, rw), dtype, residual=res)
+    for _ in range(2):
+        got = layer.forward(x, logits, k, True, dtype, residual=res)
+        layer.check_status()
+        # (products of another kernel may differ in the last place of h, and so of y)
+        helpers.assert_close(got.float().cpu(), want.float().cpu(), rtol=2.0 ** -7, atol=2e-3, what="layer call")
