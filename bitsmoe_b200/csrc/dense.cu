@@ -49,6 +49,9 @@ int dense_xwT(const void* X, int x_dtype, const __half* W0, const __half* W1, vo
 static int dense_mlp_small(const void* x, int x_dtype, const __half* wg, const __half* wu, const __half* wd, const __half* token_gate_w,
                            int T, int H, int I, const void* residual, void* y, int y_dtype, float* z, float* gate, cudaStream_t st) {
   if (token_gate_w && x_dtype == BM_F32) return BM_ERR_UNSUPPORTED;     // the gate's logit is taken from the unrounded fp32 row
+  // From 17 tokens on a pair whose row tiles are more than a wave of CTAs goes to the tiled product (us, two shared experts of 1408, bf16:
+  // 8 tokens 24.2 / 29.8, 16 29.1 / 29.4, 24 32.0 / 27.4, 64 68 / 23.6, 256 244 / 27.5; intermediate size 512: 64 tokens 13.9 / 15.9, 80 21.3 / 15.9).
+  if (T > 16 && H % 64 == 0 && I % 64 == 0 && skinny_many_waves((I + 15) / 16, 8, T)) return BM_ERR_UNSUPPORTED;
   if (T > SKINNY_MAX_TOKENS || H % 8 != 0 || I % 8 != 0 || !skinny_fits(H, 0, 8) || !skinny_fits(I, 0, skinny_splits(H, I)))
     return BM_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wg) | reinterpret_cast<uintptr_t>(wu) | reinterpret_cast<uintptr_t>(wd) |
@@ -202,9 +205,9 @@ extern "C" int bm_dense_mlp_forward(const void* x, int x_dtype, const uint16_t* 
   a.row_gate = token_gate_w ? gate : nullptr;
   a.after = token_gate_w ? AFTER_READS : AFTER_ALL;
   rc = launch_gemm_tma(a, st);
-  if (rc == BM_OK)
+  if (rc == BM_OK)      // (behind a tiled pair the tiled product of z is the faster one as well: 33 tokens 26.0 -> 23.4 us a call)
     return dense_xwT(z, BM_F16, reinterpret_cast<const __half*>(w_down), nullptr, y, nullptr, y_dtype, residual, T, hidden, intermediate, 1,
-                     nullptr, AFTER_READS, SKINNY_MAX_TOKENS, st);
+                     nullptr, AFTER_READS, /*skinny_tokens=*/0, st);
   if (rc != BM_ERR_UNSUPPORTED) return rc;
   rc = dense_xwT(x, x_dtype, reinterpret_cast<const __half*>(w_gate), reinterpret_cast<const __half*>(w_up), g, u, BM_F16, nullptr,
                  T, intermediate, hidden, 2, nullptr, AFTER_ALL, SKINNY_MAX_TOKENS, st);

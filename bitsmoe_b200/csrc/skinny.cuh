@@ -54,6 +54,8 @@ struct SkinnyArgs {
 // BM_ERR_UNSUPPORTED (nothing launched) when the shape does not tile; the caller then takes a general GEMM.
 int launch_skinny_nt(SkinnyArgs a, cudaStream_t st);
 bool skinny_fits(int K, int K2, int splits);
+// Whether the product's grid is more than one wave of the device (three CTAs an SM).
+bool skinny_many_waves(int row_tiles, int splits, int T);
 // Cluster size along K for a product of `rows` output rows.
 int skinny_splits(int rows, int K);
 

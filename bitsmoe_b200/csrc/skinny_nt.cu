@@ -311,6 +311,12 @@ int skinny_splits(int rows, int K) {
   return 8;
 }
 
+bool skinny_many_waves(int row_tiles, int splits, int T) {
+  int dev = -1, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+  return row_tiles * splits * ((T + SK_NTOK - 1) / SK_NTOK) > SK_FEW * sms;
+}
+
 int launch_skinny_nt(SkinnyArgs a, cudaStream_t st) {
   BM_REQUIRE(a.N >= 1 && a.N <= SKINNY_MAX_TOKENS && a.n_seg >= 1 && a.n_seg <= SK_MAX_SEG && a.splits >= 1 && a.splits <= 8 &&
                  (a.splits & (a.splits - 1)) == 0 && skinny_fits(a.K, a.K2, a.splits) && aligned16(a.X, a.W2, a.X2),
