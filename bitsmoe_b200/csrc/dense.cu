@@ -74,23 +74,26 @@ static int dense_mlp_small(const void* x, int x_dtype, const __half* wg, const _
 }
 
 // gate[t] = sigmoid(x[t] . w), w fp16 or bf16 rounded to it.  A warp takes two tokens, whose loads share those of w: a pass over x at
-// memory speed.  It runs beside the rounding of a block's weights, which it does not read (16384 x 2048 bf16 and 4.2 M weights: 25 -> 22 us).
-__device__ __forceinline__ float2 row_gate_pair(uint32_t v, int dtype) {
-  if (dtype == BM_F16) return __half22float2(*reinterpret_cast<const __half2*>(&v));
+// memory speed.  It runs beside the rounding of a block's weights, which it does not read (16384 x 2048 bf16 and 4.2 M weights: 25 -> 20 us, 3 of them from types
+// that the compiler knows, so that a lane's loads are in flight together).
+template <int DTYPE>
+__device__ __forceinline__ float2 row_gate_pair(uint32_t v) {
+  if (DTYPE == BM_F16) return __half22float2(*reinterpret_cast<const __half2*>(&v));
   return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
 }
 constexpr int RG_TOKENS = 2;
-__global__ void __launch_bounds__(256) row_gate_kernel(const void* __restrict__ x, int x_dtype, const uint16_t* __restrict__ w, int w_dtype, int T,
-                                                       int H, float* __restrict__ gate, int beside) {
+template <int XD, int WD>
+__global__ void __launch_bounds__(256) row_gate_kernel(const void* __restrict__ x, const uint16_t* __restrict__ w, int T, int H, float* __restrict__ gate,
+                                                       int beside) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t0 = (blockIdx.x * (blockDim.x >> 5) + warp) * RG_TOKENS;
   grid_launch_dependents();
   if (!beside) grid_wait();
   auto weight = [&](uint32_t v) {
-    const float2 f = row_gate_pair(v, w_dtype);
-    return w_dtype == BM_F16 ? f : __half22float2(__floats2half2_rn(f.x, f.y));
+    const float2 f = row_gate_pair<WD>(v);
+    return WD == BM_F16 ? f : __half22float2(__floats2half2_rn(f.x, f.y));
   };
-  if (x_dtype != BM_F32 && H % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0) {
+  if (XD != BM_F32 && H % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0) {
     float acc[RG_TOKENS] = {};
     const uint4* xr[RG_TOKENS];
 #pragma unroll
@@ -108,7 +111,7 @@ __global__ void __launch_bounds__(256) row_gate_kernel(const void* __restrict__ 
         const float2 wf = weight(wp[j]);
 #pragma unroll
         for (int u = 0; u < RG_TOKENS; ++u) {
-          const float2 xf = row_gate_pair(reinterpret_cast<const uint32_t*>(&xv[u])[j], x_dtype);
+          const float2 xf = row_gate_pair<XD>(reinterpret_cast<const uint32_t*>(&xv[u])[j]);
           acc[u] = fmaf(xf.x, wf.x, fmaf(xf.y, wf.y, acc[u]));
         }
       }
@@ -123,8 +126,8 @@ __global__ void __launch_bounds__(256) row_gate_kernel(const void* __restrict__ 
     for (int t = t0; t < min(t0 + RG_TOKENS, T); ++t) {
       float acc = 0.f;
       for (int i = lane; i < H; i += 32) {
-        const float wf = w_dtype == BM_F16 ? load_act(w, BM_F16, i) : __half2float(__float2half_rn(load_act(w, BM_BF16, i)));
-        acc += load_act(x, x_dtype, static_cast<int64_t>(t) * H + i) * wf;
+        const float wf = WD == BM_F16 ? load_act(w, BM_F16, i) : __half2float(__float2half_rn(load_act(w, BM_BF16, i)));
+        acc += load_act(x, XD, static_cast<int64_t>(t) * H + i) * wf;
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
@@ -136,7 +139,11 @@ __global__ void __launch_bounds__(256) row_gate_kernel(const void* __restrict__ 
 
 int launch_row_gate(const void* x, int x_dtype, const uint16_t* w, int w_dtype, int T, int H, float* gate, LaunchAfter after, cudaStream_t st) {
   const int per = 8 * RG_TOKENS;
-  BM_CUDA(launch_after(after, 1, row_gate_kernel, dim3((T + per - 1) / per), 256, 0, st, x, x_dtype, w, w_dtype, T, H, gate, after == AFTER_BESIDE));
+  const bool wh = w_dtype == BM_F16;
+  auto* kernel = x_dtype == BM_F32 ? (wh ? row_gate_kernel<BM_F32, BM_F16> : row_gate_kernel<BM_F32, BM_BF16>)
+                 : x_dtype == BM_F16 ? (wh ? row_gate_kernel<BM_F16, BM_F16> : row_gate_kernel<BM_F16, BM_BF16>)
+                                     : (wh ? row_gate_kernel<BM_BF16, BM_F16> : row_gate_kernel<BM_BF16, BM_BF16>);
+  BM_CUDA(launch_after(after, 1, kernel, dim3((T + per - 1) / per), 256, 0, st, x, w, T, H, gate, after == AFTER_BESIDE));
   BM_LAUNCH_CHECK("row_gate_kernel");
   return BM_OK;
 }

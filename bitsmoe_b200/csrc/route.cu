@@ -8,8 +8,9 @@
 // ties go to the lower expert id, and inside an expert assignments are ordered by
 // ascending flat (token, slot) index.
 //
-// What bounds it is latency: four dependent launches.  16384 tokens of 512 experts, top 10: top-k 52 -> 24.5 us (topk.cuh),
-// prefixes of the block histograms 16.5 -> 4 us (one block walked them; now a thread of a grid per expert, and the totals
+// What bounds it is latency: dependent launches, two up to the sizes that one cluster places, four above.  Top-k and placement of 6216
+// assignments of 128 experts 20 us (four launches one behind the other) -> 10.  16384 tokens of 512 experts, top 10: top-k 52 -> 24.5 us
+// (topk.cuh), prefixes of the block histograms 16.5 -> 4 us (one block walked them; now a thread of a grid per expert, and the totals
 // are scanned where they are used), counting 5, scatter 8.
 #include <cooperative_groups.h>
 
