@@ -19,8 +19,10 @@
 //               the row's 256 bytes before any of them writes its 16-byte piece of the 128-byte result row.
 // Every wait is bounded; a time-out raises the status word.
 //
-// Small batches are bound by shared memory: a slice of a 128 x 64 tile is written (24 KB), rounded in place (32 KB) and read by the
-// MMA (24 KB), 550 cycles in all at 128 bytes a cycle; fp16 slices take 350, the rate at which an SM gets data from L2.  Basis
+// Small batches of bf16 or fp32 rows are bound by the rounding: 550 to 600 cycles a slice of 128 rows, whatever the tile's width and
+// however many warps share it; fp16 slices take 350, the rate at which an SM gets data from L2.  Measured and not taken: the rounded
+// slice into tensor memory instead of shared memory (basis pair of 777 tokens 11.8 -> 11.6 us, 8192 tokens 22.1 -> 21.3, but 2048
+// tokens 14.0 -> 15.2), conversion by integer shifts (777 tokens 12.9).  Basis
 // pair of 300 tokens 14.9 -> 9.3 us (clusters of four), 777 tokens 15.2 -> 11.8 (of two), 2048 tokens 15.7 -> 14.0 (epilogue warps
 // round too).
 //
