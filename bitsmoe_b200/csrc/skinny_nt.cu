@@ -366,7 +366,10 @@ int launch_skinny_nt(SkinnyArgs a, cudaStream_t st) {
   if (a.clusters == a.row_tiles) {
     // small CTAs are placed several to an SM while other SMs stay empty: ask for the memory that spreads them evenly, with
     // a tenth to spare for clusters that do not fill their group of SMs (64 tokens: 47.2 -> 44.3 us a block)
-    const int per_sm = (total * 11 + 10 * sms - 1) / (10 * sms);
+    int per_sm = (total * 11 + 10 * sms - 1) / (10 * sms);
+    // one CTA an SM leaves clusters without a whole group of SMs, and the last ones wait for a second wave (basis pair of 64 tokens, 16
+    // clusters of eight: 11.4 -> 7.5 us, of one token 8.3 -> 5.1)
+    if (a.splits > 1 && per_sm == 1 && total * 5 > sms * 4) per_sm = 2;
     const size_t room = (227 * 1024 / std::min(per_sm, 8) - 1024) / 128 * 128;
     smem = std::max(smem, std::min(room, SK_SMEM_LIMIT));
   }
