@@ -65,7 +65,7 @@ def parse():
                     help="ep workload: waves per step and rank (2: the exchange of one runs beside the compute of the other; "
                          "measured no faster than 1 at the default sizes)")
     ap.add_argument("--no-extras", action="store_true", help="headline only (skip other batch sizes / prefill / cpu / reference kernels)")
-    ap.add_argument("--path", type=int, default=0, help="experts path: 0 auto, 1 generic, 2 decode, 3 tensor")
+    ap.add_argument("--path", type=int, default=0, help="experts path: 0 auto, 1 generic, 2 decode, 3 tensor, 4 batch")
     ap.add_argument("--probe", default=None, choices=["experts", "forward"],
                     help="no timing: run the packed-experts stage or the whole layer forward --steps times over --layers "
                          "rotating weight sets with --tokens tokens (Zipf(1.1) routing above 256 tokens) and exit; the "

@@ -18,7 +18,7 @@ HOST_PATH = os.path.join(_PKG, "_lib", "_bm_host.so")
 BM_OK = 0
 BM_F16, BM_BF16, BM_F32 = 0, 1, 2
 ROUND_NONE, ROUND_F16, ROUND_BF16 = 0, 1, 2
-PATH_AUTO, PATH_GENERIC, PATH_DECODE, PATH_TENSOR = 0, 1, 2, 3
+PATH_AUTO, PATH_GENERIC, PATH_DECODE, PATH_TENSOR, PATH_BATCH = 0, 1, 2, 3, 4
 GATE, UP, DOWN = 0, 1, 2
 
 _DTYPES = {torch.float16: BM_F16, torch.bfloat16: BM_BF16, torch.float32: BM_F32}

@@ -500,7 +500,7 @@ static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, con
                                 void* workspace, size_t workspace_bytes, void* stream) {
   BM_REQUIRE(L != nullptr, BM_ERR_INVALID_ARG, "experts_forward: null layer");
   BM_REQUIRE(T >= 0 && num_assign >= 0, BM_ERR_INVALID_ARG, "experts_forward: negative sizes");
-  BM_REQUIRE(path >= BM_PATH_AUTO && path <= BM_PATH_TENSOR, BM_ERR_INVALID_ARG, "experts_forward: unknown path %d", path);
+  BM_REQUIRE(path >= BM_PATH_AUTO && path <= BM_PATH_BATCH, BM_ERR_INVALID_ARG, "experts_forward: unknown path %d", path);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (T == 0) return BM_OK;
   BM_REQUIRE(rank_accum, BM_ERR_INVALID_ARG, "experts_forward: null rank_accum");
@@ -526,20 +526,27 @@ static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, con
              "experts_forward: the tensor path needs 1- to 4-bit rows and full tiles; this layer has neither");
   BM_REQUIRE(path != BM_PATH_DECODE || L->fast_ok, BM_ERR_UNSUPPORTED,
              "experts_forward: the decode path needs 1- to 4-bit rows and full tiles; this layer has neither");
+  BM_REQUIRE(path != BM_PATH_BATCH || L->fast_ok, BM_ERR_UNSUPPORTED,
+             "experts_forward: the batch path needs 1- to 4-bit rows and full tiles; this layer has neither");
   const __half* hg = reinterpret_cast<const __half*>(h_gate);
   const __half* hu = reinterpret_cast<const __half*>(h_up);
-  // The kernel by assignments per expert.  Up to 6 most experts need one pass of 8 tokens, and that kernel is the fastest at it
+  // AUTO: the kernel by assignments per expert.  Up to 6 most experts need one pass of 8 tokens, and that kernel is the fastest at it
   // (96 tokens, top 8 of 128 experts: 20.1 us against 24.3; 128 tokens: 31.4 against 24.4); where few experts leave room to cut
   // every pass along its tiles, up to 8 (80 tokens, top 6 of 64 experts: 1.2 us).  Up to 24 passes of 16 tokens cost less than turning
   // every expert into tensor-core operands (400 tokens, 25 each: 39 us against 40; 512 tokens, 32 each: 47 against 40).
   const int64_t per16 = static_cast<int64_t>(num_assign) * 16 / L->num_experts;      // assignments per expert, in sixteenths
   const int one_pass = 4 * L->num_experts >= L->bat_grid ? 6 : 8;
-  const bool batch = L->bat_ring && per16 > one_pass * 16 && (path == BM_PATH_DECODE ? num_assign / FAST_MAX_TOK + L->num_experts < 60000 : per16 <= 24 * 16);
-  if (L->fast_ok && (path == BM_PATH_TENSOR || (path == BM_PATH_AUTO && per16 > 16 * 16 && !batch && experts_tc_fits(L))))
+  if (path == BM_PATH_AUTO) {
+    if (L->bat_ring && per16 > one_pass * 16 && per16 <= 24 * 16) path = BM_PATH_BATCH;
+    else if (L->fast_ok && per16 > 16 * 16 && experts_tc_fits(L)) path = BM_PATH_TENSOR;
+    else if (L->fast_ok && L->dec_ok && num_assign / FAST_MAX_TOK + L->num_experts < 60000) path = BM_PATH_DECODE;
+    else path = BM_PATH_GENERIC;
+  }
+  if (path == BM_PATH_TENSOR)
     rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, num_assign, rank_accum, acc64, st);
-  else if (batch && (path == BM_PATH_AUTO || path == BM_PATH_DECODE))
+  else if (path == BM_PATH_BATCH)
     rc = launch_experts_batch(L, hg, hu, token_indices, expert_offsets, route_weights, T, rank_accum, acc64, st);
-  else if (L->fast_ok && (path == BM_PATH_DECODE || (path != BM_PATH_GENERIC && L->dec_ok && num_assign / 8 + L->num_experts < 60000)))
+  else if (path == BM_PATH_DECODE)
     rc = launch_experts_decode(L, hg, hu, token_indices, expert_offsets, route_weights, T, num_assign, rank_accum, acc64, st);
   else
     rc = launch_experts_generic(L, hg, hu, token_indices, expert_offsets, route_weights, T, rank_accum, acc64, st);

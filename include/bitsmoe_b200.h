@@ -38,7 +38,10 @@ enum {
 
 enum { BM_F16 = 0, BM_BF16 = 1, BM_F32 = 2 };          /* element types of activations */
 enum { BM_ROUND_NONE = 0, BM_ROUND_F16 = 1, BM_ROUND_BF16 = 2 };
-enum { BM_PATH_AUTO = 0, BM_PATH_GENERIC = 1, BM_PATH_DECODE = 2, BM_PATH_TENSOR = 3 };
+/* Kernels of the packed experts: any bit width, passes of 8 assignments (experts_decode_kernel), tcgen05 (experts_tc_kernel), passes of
+ * 16 assignments (experts_batch_kernel).  AUTO chooses by assignments per expert and by what the layer allows; a kernel that is asked
+ * for by name runs, or the call reports BM_ERR_UNSUPPORTED. */
+enum { BM_PATH_AUTO = 0, BM_PATH_GENERIC = 1, BM_PATH_DECODE = 2, BM_PATH_TENSOR = 3, BM_PATH_BATCH = 4 };
 enum { BM_GATE = 0, BM_UP = 1, BM_DOWN = 2 };
 
 BM_API int bm_abi_version(void);
@@ -131,7 +134,8 @@ BM_API int bm_layer_has_fast_layout(const bm_layer_t* layer);
 BM_API int bm_layer_status(const bm_layer_t* layer, void* stream);
 
 /* No counterpart in the reference.  Tuning knobs of a layer; set between forwards, never while one is in flight.
- *   BM_OPT_DECODE_CTAS_PER_SM: resident CTAs per SM of the decode kernel (1, 2 or 3; 0 = the library's choice).
+ *   BM_OPT_DECODE_CTAS_PER_SM: resident CTAs per SM of the decode kernel (1, 2 or 3; 0 = the library's choice); the other kernels
+ *     keep their own.
  *   BM_OPT_DETERMINISTIC (0 / 1): the packed-expert kernels add into rank_accum through 64-bit fixed-point atomics
  *     instead of fp32 atomics (bitsmoe/algorithms/cpp/mlp_forward.cu:2062 uses fp32 atomics, whose result depends on
  *     arrival order): two runs on the same inputs are then bit-identical.  bm_experts_workspace_bytes /

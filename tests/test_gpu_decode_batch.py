@@ -54,9 +54,10 @@ def test_passes_of_sixteen_match_generic_kernel(rank, inter, E):
     want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
     nan = torch.full_like(hg, float("nan"))
     layer.experts_forward(nan, nan, tok, off, rw)      # what a kernel does not write still holds these
-    got = layer.experts_forward(hg, hu, tok, off, rw)
-    layer.check_status()
-    helpers.assert_close(got.cpu(), want.cpu(), what=f"rank {rank} E {E}")
+    for path in (capi.PATH_AUTO, capi.PATH_BATCH):
+        got = layer.experts_forward(hg, hu, tok, off, rw, path=path)
+        layer.check_status()
+        helpers.assert_close(got.cpu(), want.cpu(), what=f"path {path} rank {rank} E {E}")
     capi.check(capi.lib().bm_layer_set_option(layer._handle, 2, 0))
     layer.experts_forward(hg, hu, tok, off, rw)
     with pytest.raises(capi.BitsMoEError, match="bounded wait"):

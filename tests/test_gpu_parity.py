@@ -293,6 +293,8 @@ def test_decode_path_refused_without_arena(mixed):
     args = [o[k].to(DEV) for k in ("h_gate", "h_up", "token_indices", "expert_offsets", "route_flat")]
     with pytest.raises(capi.BitsMoEError, match="decode path needs"):
         packed.experts_forward(*args, path=capi.PATH_DECODE)
+    with pytest.raises(capi.BitsMoEError, match="batch path needs"):
+        packed.experts_forward(*args, path=capi.PATH_BATCH)
 
 
 @pytest.mark.parametrize("T", [300, 1000])
@@ -372,7 +374,7 @@ def test_arena_holds_one_bit_rows(low_bits):
             assert np.array_equal(packed.decode_codes(e, which, source=1).cpu().numpy(), want), (tag, e, "arena")
 
 
-@pytest.mark.parametrize("path", [capi.PATH_DECODE, capi.PATH_TENSOR])
+@pytest.mark.parametrize("path", [capi.PATH_DECODE, capi.PATH_TENSOR, capi.PATH_BATCH])
 @pytest.mark.parametrize("T", [3, 40])
 def test_one_to_four_bit_rows_on_fast_paths(low_bits, T, path):
     layer, packed, experts = low_bits
@@ -413,7 +415,7 @@ def test_fast_paths_shape_sweep(case):
         args = [o[kk].to(DEV) for kk in ("h_gate", "h_up", "token_indices", "expert_offsets", "route_flat")]
         gen = packed.experts_forward(*args, path=capi.PATH_GENERIC)
         helpers.assert_close(gen, o["rank_accum"], rtol=1e-3, atol=1e-5, what=f"sweep {case} T={T} generic vs oracle")
-        paths = (capi.PATH_DECODE, capi.PATH_TENSOR) if packed.has_fast_layout else ()
+        paths = (capi.PATH_DECODE, capi.PATH_TENSOR, capi.PATH_BATCH) if packed.has_fast_layout else ()
         if r > 256:
             paths = paths[:1] + (capi.PATH_AUTO,)      # wide ranks: the tensor path shrinks its items or AUTO takes another path
         for path in paths:
@@ -462,7 +464,7 @@ def test_bounded_wait_gives_up_and_reports_timeout(q30_small):
     assert float(torch.ones(4, device=DEV).sum()) == 4.0
 
 
-@pytest.mark.parametrize("path", [capi.PATH_DECODE, capi.PATH_TENSOR])
+@pytest.mark.parametrize("path", [capi.PATH_DECODE, capi.PATH_TENSOR, capi.PATH_BATCH])
 @pytest.mark.parametrize("T", [1, 8, 700])
 def test_expert_kernels_leave_cleanly_when_a_wait_gives_up(q30_small, path, T):
     """With the limit at 0 the roles of every CTA leave at their first wait that is not over, with copies and products
@@ -568,7 +570,7 @@ def test_fused_packer_path_builds_the_same_layer_as_the_host_path():
         assert torch.equal(a, b), key
 
 
-@pytest.mark.parametrize("path,T", [(capi.PATH_DECODE, 64), (capi.PATH_TENSOR, 700), (capi.PATH_GENERIC, 40)])
+@pytest.mark.parametrize("path,T", [(capi.PATH_DECODE, 64), (capi.PATH_TENSOR, 700), (capi.PATH_GENERIC, 40), (capi.PATH_BATCH, 200)])
 def test_deterministic_mode_is_bit_reproducible(q30_small, path, T):
     """With fixed-point accumulation two runs give identical bits whatever order the CTAs arrive in, and the values
     agree with the fp32-atomic mode to fp32 rounding."""

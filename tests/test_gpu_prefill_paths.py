@@ -31,7 +31,7 @@ def test_packed_experts_match_generic_kernel(rank, inter, counts):
     tok, off, rw = _route(counts, 1, T, gen)
     hg, hu = layer.basis_project(synth.activations(cfg, T, seed=2, device=DEV, dtype=torch.bfloat16))
     want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
-    for path in (capi.PATH_DECODE, capi.PATH_TENSOR):
+    for path in (capi.PATH_DECODE, capi.PATH_TENSOR, capi.PATH_BATCH):
         try:
             got = layer.experts_forward(hg, hu, tok, off, rw, path=path)
         except capi.BitsMoEError as e:      # a layer whose largest expert does not fit that path
@@ -77,7 +77,7 @@ def test_sums_reach_rows_of_any_alignment(rank_out, shift):
     tok, off, rw = _route(counts, 1, T, gen)
     hg, hu = layer.basis_project(torch.randn(T, 128, generator=gen, device=DEV).half())
     want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
-    for path in (capi.PATH_DECODE, capi.PATH_TENSOR):
+    for path in (capi.PATH_DECODE, capi.PATH_TENSOR, capi.PATH_BATCH):
         buf = torch.full((T * rank_out + 2,), 7.0, device=DEV)
         acc = buf[shift:shift + T * rank_out].view(T, rank_out)
         assert acc.data_ptr() % 16 == 4 * shift
@@ -86,6 +86,33 @@ def test_sums_reach_rows_of_any_alignment(rank_out, shift):
         layer.check_status()
         helpers.assert_close(acc.cpu(), want.cpu(), what=f"path {path} rank_out {rank_out} shift {shift}")
         assert buf[:shift].eq(7.0).all() and buf[shift + T * rank_out:].eq(7.0).all()
+
+
+# A kernel that is asked for by name runs whatever the load.  One tile and one assignment a token: in deterministic mode a row's bits then
+# depend on the kernel alone, not on how many tokens share its pass, and the two kernels round weights and operand at different places.
+def test_named_kernels_run_at_any_load():
+    E, counts = 12, [17, 9, 0, 24, 12, 1, 31, 8, 16, 40, 7, 15]
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=128, top_k=1, rank=64)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=4, device=DEV))
+    layer.set_deterministic(True)
+    T = sum(counts)
+    gen = torch.Generator(device=DEV).manual_seed(12)
+    hg, hu = layer.basis_project(torch.randn(T, 128, generator=gen, device=DEV).half())
+    rw = torch.rand(T, generator=gen, device=DEV)
+    start = [sum(counts[:e]) for e in range(E)]
+
+    def run(path, first, last):      # every expert's assignments first .. last - 1
+        rows = [range(s + min(first, c), s + min(last, c)) for s, c in zip(start, counts)]
+        tok = torch.tensor([i for r in rows for i in r], dtype=torch.int32, device=DEV)
+        off = torch.tensor([0] + [len(r) for r in rows], device=DEV).cumsum(0).to(torch.int32)
+        return layer.experts_forward(hg, hu, tok, off, rw[tok.long()], path=path)
+
+    whole = {path: run(path, 0, T) for path in (capi.PATH_DECODE, capi.PATH_BATCH, capi.PATH_AUTO)}
+    for path in (capi.PATH_DECODE, capi.PATH_BATCH):
+        assert torch.equal(whole[path], sum(run(path, i, i + 4) for i in range(0, max(counts), 4))), path
+    layer.check_status()
+    assert not torch.equal(whole[capi.PATH_DECODE], whole[capi.PATH_BATCH])
+    assert torch.equal(whole[capi.PATH_AUTO], whole[capi.PATH_BATCH])      # 15 assignments an expert
 
 
 # matrices in which several rows hold the same rank: single rows (of one width and of two), and a whole aligned octet twice
@@ -104,7 +131,7 @@ def test_rows_that_repeat_a_rank():
     tok, off, rw = _route((150, 131, 20), 1, T, gen)
     hg, hu = layer.basis_project(torch.randn(T, 128, generator=gen, device=DEV).half())
     want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
-    for path in (capi.PATH_DECODE, capi.PATH_TENSOR):
+    for path in (capi.PATH_DECODE, capi.PATH_TENSOR, capi.PATH_BATCH):
         nan = torch.full_like(hg, float("nan"))
         layer.experts_forward(nan, nan, tok, off, rw, path=path)      # what a kernel does not write still holds these
         got = layer.experts_forward(hg, hu, tok, off, rw, path=path)

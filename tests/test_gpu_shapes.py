@@ -30,7 +30,7 @@ def test_full_shapes_layer_forward(shaped, T):
     o = oforward.layer_forward(x, logits, layer.vh_gate.cpu(), layer.vh_up.cpu(), layer.u_down.cpu(), experts, cfg.top_k,
                                cfg.norm_topk_prob, wdt)
     assert packed.has_fast_layout
-    for path in (capi.PATH_DECODE, capi.PATH_TENSOR, capi.PATH_GENERIC):
+    for path in (capi.PATH_DECODE, capi.PATH_TENSOR, capi.PATH_BATCH, capi.PATH_GENERIC):
         y = packed.forward(x.to(DEV), logits.to(DEV), cfg.top_k, cfg.norm_topk_prob, wdt, path=path)
         packed.check_status()
         helpers.assert_close(y, o["y_fp32"], what=f"{cfg.name} T={T} path={path}")
@@ -112,6 +112,13 @@ def test_full_shapes_decode_rank_accum(shaped, T):
     layer, packed, experts = shaped
     args, idx, w = _routed_problem(layer, packed, T, seed=700 + T)
     _check_stage(layer, packed, experts, args, idx, w, capi.PATH_DECODE, f"{layer.cfg.name} decode T={T}", 5e-3, 1e-4)
+
+
+@pytest.mark.parametrize("T", [8, 203])
+def test_full_shapes_batch_rank_accum(shaped, T):
+    layer, packed, experts = shaped
+    args, idx, w = _routed_problem(layer, packed, T, seed=800 + T)
+    _check_stage(layer, packed, experts, args, idx, w, capi.PATH_BATCH, f"{layer.cfg.name} batch T={T}", 5e-3, 1e-4)
 
 
 def test_full_shapes_prefill_rank_accum_zipf(shaped):
