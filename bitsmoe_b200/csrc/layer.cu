@@ -1,5 +1,7 @@
 // C ABI glue: error reporting, layer planning / creation over the reference's buffers,
 // stage entry points and the composed layer forward.
+#include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <new>
@@ -494,6 +496,39 @@ extern "C" size_t bm_experts_workspace_bytes(const bm_layer_t* L, int32_t T, int
   return T > 0 ? experts_ws_need(L, T) : 0;
 }
 
+// Passes of `size` assignments that the experts need together, where each has a Poisson number of them, `load` on average (choices
+// spread evenly over the experts): experts * sum over j of P(more than j * size).
+static int expected_passes(int experts, double load, int size) {
+  double p = std::exp(-load), at_most = p, passes = 0.0;
+  for (int n = 0, next = 0;;) {
+    if (n == next) {
+      if (1.0 - at_most < 1e-4) return static_cast<int>(experts * passes + 0.5);
+      passes += 1.0 - at_most;
+      next += size;
+    }
+    at_most += p *= load / ++n;
+  }
+}
+// Tiles, one after the other, of the CTA with the most where `passes` units of all tiles go over a grid of two CTAs an SM in whole rounds,
+// and what is left as a round cut along the tiles (with `cut_last` always, else only as the first one).  A round of up to a third of the
+// grid counts half: its CTAs have an SM each.
+static double longest_cta(int passes, int tiles, int grid, bool cut_last) {
+  const int rest = passes % grid, full = passes / grid, split = rest && (cut_last || !full) ? std::max(1, grid / rest) : 1;
+  const int per = (tiles + split - 1) / split, units = rest * ((tiles + per - 1) / per);
+  return full * tiles + (rest == 0 ? 0.0 : 3 * units <= grid ? 0.5 * per : per);
+}
+// Whether passes of 16 (experts_batch_kernel) take less time than passes of 8 (experts_decode_kernel).  Both are as slow as their longest
+// CTA: 7.3 us and 5.2 a tile against 7 and 4.1, and with one pass more than half of the grid a CTA has twice the tiles.  us of the stage with
+// passes of 8 / of 16: 128 experts of 6 tiles, 4 assignments each 18.9 / 22.2, 7 each 30.9 / 23.0, 12 each 32.1 / 23.0, 14 each 31.9 / 38.4, 16 each
+// 46.3 / 38.2; 160 experts of 12 tiles, 8 each 56.7 / 70.1, 12 each 84.9 / 70.2; 16 of 4 tiles, 8 each 9.1 / 10.4; 48 of 6 tiles, 6 each 14.9 / 12.4; 512
+// of 4 tiles, 7 each 51.7 / 53.7, 9 each 60.5 / 54.0.  Over 19 shapes at 2 to 24 assignments an expert this takes 1.001 of the faster kernel's time.
+static bool batch_passes_pay(const bm_layer* L, double load) {
+  if (load <= 4.0) return false;      // one pass of 8 for nearly every expert
+  const double t8 = longest_cta(expected_passes(L->num_experts, load, FAST_MAX_TOK), L->n_tiles, L->dec_grid, false);
+  const double t16 = longest_cta(expected_passes(L->num_experts, load, 2 * FAST_MAX_TOK), L->n_tiles, L->bat_grid, true);
+  return 7.3 + 5.2 * t16 < 7.0 + 4.1 * t8;
+}
+
 static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, const uint16_t* h_up,
                                 const int32_t* token_indices, const int32_t* expert_offsets, const float* route_weights,
                                 int32_t T, int32_t num_assign, float* rank_accum, int32_t path, bool already_zero,
@@ -530,17 +565,14 @@ static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, con
              "experts_forward: the batch path needs 1- to 4-bit rows and full tiles; this layer has neither");
   const __half* hg = reinterpret_cast<const __half*>(h_gate);
   const __half* hu = reinterpret_cast<const __half*>(h_up);
-  // AUTO: the kernel by assignments per expert.  Up to 6 most experts need one pass of 8 tokens, and that kernel is the fastest at it
-  // (96 tokens, top 8 of 128 experts: 20.1 us against 24.3; 128 tokens: 31.4 against 24.4); where few experts leave room to cut
-  // every pass along its tiles, up to 8 (80 tokens, top 6 of 64 experts: 1.2 us).  Up to 24 passes of 16 tokens cost less than turning
-  // every expert into tensor-core operands (400 tokens, 25 each: 39 us against 40; 512 tokens, 32 each: 47 against 40).
-  const int64_t per16 = static_cast<int64_t>(num_assign) * 16 / L->num_experts;      // assignments per expert, in sixteenths
-  const int one_pass = 4 * L->num_experts >= L->bat_grid ? 6 : 8;
   if (path == BM_PATH_AUTO) {
-    if (L->bat_ring && per16 > one_pass * 16 && per16 <= 24 * 16) path = BM_PATH_BATCH;
-    else if (L->fast_ok && per16 > 16 * 16 && experts_tc_fits(L)) path = BM_PATH_TENSOR;
-    else if (L->fast_ok && L->dec_ok && num_assign / FAST_MAX_TOK + L->num_experts < 60000) path = BM_PATH_DECODE;
-    else path = BM_PATH_GENERIC;
+    // Up to 24 assignments an expert passes cost less than turning every expert into tensor-core operands (400 tokens, top 8 of 128
+    // experts, 25 each: 39 us against 40; 512 tokens, 32 each: 47 against 40).
+    const double load = static_cast<double>(num_assign) / L->num_experts;
+    const bool decode = L->dec_ok && num_assign / FAST_MAX_TOK + L->num_experts < 60000, few = L->bat_ring && load <= 24.0;
+    if (few && (!decode || batch_passes_pay(L, load))) path = BM_PATH_BATCH;
+    else if (L->fast_ok && load > 16.0 && !few && experts_tc_fits(L)) path = BM_PATH_TENSOR;
+    else path = L->fast_ok && decode ? BM_PATH_DECODE : BM_PATH_GENERIC;
   }
   if (path == BM_PATH_TENSOR)
     rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, num_assign, rank_accum, acc64, st);

@@ -107,12 +107,29 @@ def test_named_kernels_run_at_any_load():
         off = torch.tensor([0] + [len(r) for r in rows], device=DEV).cumsum(0).to(torch.int32)
         return layer.experts_forward(hg, hu, tok, off, rw[tok.long()], path=path)
 
-    whole = {path: run(path, 0, T) for path in (capi.PATH_DECODE, capi.PATH_BATCH, capi.PATH_AUTO)}
+    whole = {path: run(path, 0, T) for path in (capi.PATH_DECODE, capi.PATH_BATCH)}
     for path in (capi.PATH_DECODE, capi.PATH_BATCH):
         assert torch.equal(whole[path], sum(run(path, i, i + 4) for i in range(0, max(counts), 4))), path
     layer.check_status()
     assert not torch.equal(whole[capi.PATH_DECODE], whole[capi.PATH_BATCH])
-    assert torch.equal(whole[capi.PATH_AUTO], whole[capi.PATH_BATCH])      # 15 assignments an expert
+
+
+# The automatic choice, told by its bits in deterministic mode: passes of 16 where they leave the longest CTA less work than passes of 8
+# (not with a tile a CTA either way, nor where they just exceed half of the grid), products on tcgen05 above 24 assignments an expert
+@pytest.mark.parametrize("E,inter,load,path", [(16, 512, 8, capi.PATH_DECODE), (16, 1536, 12, capi.PATH_BATCH), (48, 768, 6, capi.PATH_BATCH),
+                                               (128, 768, 4, capi.PATH_DECODE), (128, 768, 8, capi.PATH_BATCH), (128, 768, 12, capi.PATH_BATCH),
+                                               (128, 768, 14, capi.PATH_DECODE), (128, 768, 17, capi.PATH_BATCH), (128, 768, 25, capi.PATH_TENSOR),
+                                               (160, 1536, 8, capi.PATH_DECODE), (160, 1536, 12, capi.PATH_BATCH)])
+def test_automatic_choice_of_kernel(E, inter, load, path):
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=inter, top_k=1, rank=64)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=8, device=DEV))
+    layer.set_deterministic(True)
+    gen = torch.Generator(device=DEV).manual_seed(13)
+    tok, off, rw = _route([load] * E, 1, 64, gen)
+    hg, hu = layer.basis_project(torch.randn(64, 128, generator=gen, device=DEV).half())
+    runs = {p: layer.experts_forward(hg, hu, tok, off, rw, path=p) for p in (capi.PATH_AUTO, capi.PATH_DECODE, capi.PATH_BATCH, capi.PATH_TENSOR)}
+    layer.check_status()
+    assert [p for p in runs if p and torch.equal(runs[p], runs[capi.PATH_AUTO])] == [path]
 
 
 # matrices in which several rows hold the same rank: single rows (of one width and of two), and a whole aligned octet twice
