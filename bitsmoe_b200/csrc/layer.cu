@@ -568,10 +568,10 @@ static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, con
   if (path == BM_PATH_AUTO) {
     // Up to 24 assignments an expert passes cost less than turning every expert into tensor-core operands (400 tokens, top 8 of 128
     // experts, 25 each: 39 us against 40; 512 tokens, 32 each: 47 against 40).
-    const double load = static_cast<double>(num_assign) / L->num_experts;
-    const bool decode = L->dec_ok && num_assign / FAST_MAX_TOK + L->num_experts < 60000, few = L->bat_ring && load <= 24.0;
-    if (few && (!decode || batch_passes_pay(L, load))) path = BM_PATH_BATCH;
-    else if (L->fast_ok && load > 16.0 && !few && experts_tc_fits(L)) path = BM_PATH_TENSOR;
+    const int64_t per16 = static_cast<int64_t>(num_assign) * 16 / L->num_experts;      // assignments per expert, in sixteenths
+    const bool decode = L->dec_ok && num_assign / FAST_MAX_TOK + L->num_experts < 60000, few = L->bat_ring && per16 <= 24 * 16;
+    if (few && (!decode || batch_passes_pay(L, static_cast<double>(num_assign) / L->num_experts))) path = BM_PATH_BATCH;
+    else if (L->fast_ok && per16 > 16 * 16 && !few && experts_tc_fits(L)) path = BM_PATH_TENSOR;
     else path = L->fast_ok && decode ? BM_PATH_DECODE : BM_PATH_GENERIC;
   }
   if (path == BM_PATH_TENSOR)
