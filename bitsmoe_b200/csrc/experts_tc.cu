@@ -903,14 +903,14 @@ static int xt_launch(XtArgs a, size_t smem, cudaStream_t st) {
 }
 
 int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
-                      const int32_t* expert_offsets, const float* route_w, int T, int num_assign, float* rank_accum, long long* acc64,
+                      const int32_t* expert_offsets, const float* route_w, int T, int expected_assign, float* rank_accum, long long* acc64,
                       cudaStream_t st) {
   BM_REQUIRE(L->num_experts <= XT_MAX_E, BM_ERR_UNSUPPORTED, "experts_tc: more than %d experts", XT_MAX_E);
   BM_REQUIRE(L->intermediate % N_TILE == 0, BM_ERR_UNSUPPORTED, "experts_tc: intermediate size must be a multiple of %d", N_TILE);
   BM_REQUIRE(L->max_slots <= XT_MAX_SLOTS, BM_ERR_UNSUPPORTED, "experts_tc: %d row slots exceed the tensor-memory budget", L->max_slots);
   BM_REQUIRE(L->rank_in % 8 == 0 && ((reinterpret_cast<uintptr_t>(h_gate) | reinterpret_cast<uintptr_t>(h_up)) & 15u) == 0,
              BM_ERR_UNSUPPORTED, "experts_tc: rank-space rows must be 16-byte aligned (rank %d)", L->rank_in);
-  const int rows = L->max_slots <= 256 && num_assign <= static_cast<int64_t>(XT_FEW_ROWS) * L->num_experts ? 64 : 128;
+  const int rows = L->max_slots <= 256 && expected_assign <= static_cast<int64_t>(XT_FEW_ROWS) * L->num_experts ? 64 : 128;
   XtPlan plan;
   BM_REQUIRE(xt_plan(L, rows, &plan), BM_ERR_UNSUPPORTED, "experts_tc: the layer's largest expert does not fit in shared memory");
   XtArgs a{};

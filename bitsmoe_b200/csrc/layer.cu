@@ -39,7 +39,7 @@ int launch_experts_batch(const bm_layer* L, const __half* h_gate, const __half* 
                          const float* route_w, int T, float* rank_accum, long long* acc64, cudaStream_t st);
 bool experts_tc_fits(const bm_layer* L);
 int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
-                      const int32_t* expert_offsets, const float* route_w, int T, int num_assign, float* rank_accum, long long* acc64,
+                      const int32_t* expert_offsets, const float* route_w, int T, int expected_assign, float* rank_accum, long long* acc64,
                       cudaStream_t st);
 int launch_experts_generic(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
                            const int32_t* expert_offsets, const float* route_w, int T, float* rank_accum,
@@ -529,9 +529,10 @@ static bool batch_passes_pay(const bm_layer* L, double load) {
   return 7.3 + 5.2 * t16 < 7.0 + 4.1 * t8;
 }
 
+// `num_assign` bounds the list's length, `expected` is what the choice of a kernel takes it for.
 static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, const uint16_t* h_up,
                                 const int32_t* token_indices, const int32_t* expert_offsets, const float* route_weights,
-                                int32_t T, int32_t num_assign, float* rank_accum, int32_t path, bool already_zero,
+                                int32_t T, int32_t num_assign, int32_t expected, float* rank_accum, int32_t path, bool already_zero,
                                 void* workspace, size_t workspace_bytes, void* stream) {
   BM_REQUIRE(L != nullptr, BM_ERR_INVALID_ARG, "experts_forward: null layer");
   BM_REQUIRE(T >= 0 && num_assign >= 0, BM_ERR_INVALID_ARG, "experts_forward: negative sizes");
@@ -568,14 +569,14 @@ static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, con
   if (path == BM_PATH_AUTO) {
     // Up to 24 assignments an expert passes cost less than turning every expert into tensor-core operands (400 tokens, top 8 of 128
     // experts, 25 each: 39 us against 40; 512 tokens, 32 each: 47 against 40).
-    const int64_t per16 = static_cast<int64_t>(num_assign) * 16 / L->num_experts;      // assignments per expert, in sixteenths
+    const int64_t per16 = static_cast<int64_t>(expected) * 16 / L->num_experts;      // assignments per expert, in sixteenths
     const bool decode = L->dec_ok && num_assign / FAST_MAX_TOK + L->num_experts < 60000, few = L->bat_ring && per16 <= 24 * 16;
-    if (few && (!decode || batch_passes_pay(L, static_cast<double>(num_assign) / L->num_experts))) path = BM_PATH_BATCH;
+    if (few && (!decode || batch_passes_pay(L, static_cast<double>(expected) / L->num_experts))) path = BM_PATH_BATCH;
     else if (L->fast_ok && per16 > 16 * 16 && !few && experts_tc_fits(L)) path = BM_PATH_TENSOR;
     else path = L->fast_ok && decode ? BM_PATH_DECODE : BM_PATH_GENERIC;
   }
   if (path == BM_PATH_TENSOR)
-    rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, num_assign, rank_accum, acc64, st);
+    rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, expected, rank_accum, acc64, st);
   else if (path == BM_PATH_BATCH)
     rc = launch_experts_batch(L, hg, hu, token_indices, expert_offsets, route_weights, T, rank_accum, acc64, st);
   else if (path == BM_PATH_DECODE)
@@ -596,7 +597,7 @@ extern "C" int bm_experts_forward(const bm_layer_t* L, const uint16_t* h_gate, c
                                   const float* route_weights, int32_t T, int32_t num_assign, float* rank_accum,
                                   int32_t path, void* workspace, size_t workspace_bytes, void* stream) {
   bm::NvtxRange nvtx_range("bm_experts_forward");
-  return experts_forward_impl(L, h_gate, h_up, token_indices, expert_offsets, route_weights, T, num_assign, rank_accum, path,
+  return experts_forward_impl(L, h_gate, h_up, token_indices, expert_offsets, route_weights, T, num_assign, num_assign, rank_accum, path,
                               false, workspace, workspace_bytes, stream);
 }
 
@@ -716,10 +717,15 @@ static int forward_small(const bm_layer_t* L, const bm_block_dense_t* d, const v
   if (rc) return rc;
   if (d && (rc = launch_route_small(r, st))) return rc;
   rc = experts_forward_impl(L, reinterpret_cast<const uint16_t*>(w.h_gate), reinterpret_cast<const uint16_t*>(w.h_up), w.token_indices,
-                            w.expert_offsets, w.route_flat, T, T * k, w.rank_accum, path, true, w.experts_ws, w.experts_ws_bytes, st);
+                            w.expert_offsets, w.route_flat, T, T * k, T * k, w.rank_accum, path, true, w.experts_ws, w.experts_ws_bytes, st);
   if (rc) return rc;
   return combine_small(L, w.rank_accum, T, shared ? h(d->sh_down) : nullptr, bf16, z, shared && d->sh_token_gate ? gate : nullptr,
                        shared ? d->sh_intermediate : 0, residual, y, x_dtype, true, st);
+}
+
+// Assignments of T tokens that the packed experts get where choices spread evenly over the routed ones.
+static int32_t expected_assign(const bm_layer_t* L, int32_t T, int32_t k, int32_t num_routed) {
+  return static_cast<int32_t>(static_cast<int64_t>(T) * k * std::min(L->num_experts, num_routed) / num_routed);
 }
 
 extern "C" int bm_layer_forward(const bm_layer_t* L, const void* x, int x_dtype, const void* logits, int logits_dtype,
@@ -754,9 +760,10 @@ extern "C" int bm_layer_forward(const bm_layer_t* L, const void* x, int x_dtype,
                      zeroed ? reinterpret_cast<float4*>(w.rank_accum) : nullptr, static_cast<int64_t>(acc_bytes / 16), st);
   if (rc) return rc;
   // Dropped assignments (experts that are not packed) leave a shorter list; the kernels walk
-  // expert_offsets, so passing the upper bound T*k as num_assign is safe.
+  // expert_offsets, so passing the upper bound T*k as num_assign is safe.  The kernel is chosen for the packed experts' share of the
+  // routed ones (a shard of 64 of 128 experts, 96 tokens, top 8: six each, not twelve; stage 17.4 -> 15.0 us).
   rc = experts_forward_impl(L, reinterpret_cast<const uint16_t*>(w.h_gate), reinterpret_cast<const uint16_t*>(w.h_up),
-                            w.token_indices, w.expert_offsets, w.route_flat, T, T * k, w.rank_accum, path, zeroed, w.experts_ws,
+                            w.token_indices, w.expert_offsets, w.route_flat, T, T * k, expected_assign(L, T, k, num_routed), w.rank_accum, path, zeroed, w.experts_ws,
                             w.experts_ws_bytes, stream);
   if (rc) return rc;
   return combine_down_basis(L, w.rank_accum, T, residual, y, x_dtype == BM_F32 ? BM_F32 : x_dtype, AFTER_READS, st);
@@ -831,7 +838,7 @@ static int forward_large(const bm_layer_t* L, const bm_block_dense_t& d, const v
                     w.token_indices, w.expert_offsets, w.route_flat, nullptr, nullptr, w.route_ws, w.route_ws_bytes, AFTER_READS, /*beside_follows=*/false, st);
   if (rc) return rc;
   rc = experts_forward_impl(L, reinterpret_cast<const uint16_t*>(w.h_gate), reinterpret_cast<const uint16_t*>(w.h_up), w.token_indices,
-                            w.expert_offsets, w.route_flat, T, T * k, w.rank_accum, BM_PATH_AUTO, true, w.experts_ws, w.experts_ws_bytes, st);
+                            w.expert_offsets, w.route_flat, T, T * k, expected_assign(L, T, k, num_routed), w.rank_accum, BM_PATH_AUTO, true, w.experts_ws, w.experts_ws_bytes, st);
   if (rc) return rc;
   GemmTmaArgs c{};
   c.X = w.rank_accum; c.x_dtype = BM_F32; c.M = T; c.K = L->rank_out; c.status = L->status_dev;

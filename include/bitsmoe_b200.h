@@ -213,7 +213,8 @@ BM_API int bm_basis_project(const bm_layer_t* layer, const void* x, int x_dtype,
 BM_API size_t bm_experts_workspace_bytes(const bm_layer_t* layer, int32_t T, int32_t num_assign, int32_t path);
 /* The op contract of moe_packed_forward (bitsmoe/algorithms/cpp/mlp_forward_binding.cpp:53-155,
  * bitsmoe/algorithms/cpp/mlp_forward.cu:2701-3074): rank_accum fp32 [T, rank_out] is
- * overwritten with  sum over assignments of  route_w * s_down * (W_down . (silu(g) * u)). */
+ * overwritten with  sum over assignments of  route_w * s_down * (W_down . (silu(g) * u)).  num_assign bounds the length
+ * of the lists (expert_offsets[num_experts] is what counts); BM_PATH_AUTO chooses the kernel as if they had that length. */
 BM_API int bm_experts_forward(const bm_layer_t* layer, const uint16_t* h_gate, const uint16_t* h_up,
                        const int32_t* token_indices, const int32_t* expert_offsets, const float* route_weights,
                        int32_t T, int32_t num_assign, float* rank_accum, int32_t path,

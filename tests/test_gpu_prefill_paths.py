@@ -132,6 +132,24 @@ def test_automatic_choice_of_kernel(E, inter, load, path):
     assert [p for p in runs if p and torch.equal(runs[p], runs[capi.PATH_AUTO])] == [path]
 
 
+# A shard of the experts: the kernel is chosen for its share of the assignments, not for all of them
+@pytest.mark.parametrize("T,path", [(96, capi.PATH_DECODE), (128, capi.PATH_DECODE), (256, capi.PATH_BATCH), (512, capi.PATH_TENSOR)])
+def test_a_shard_is_chosen_for_by_its_share(T, path):
+    E, routed, k = 64, 128, 8
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=768, top_k=k, rank=64)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=9, device=DEV))
+    layer.set_deterministic(True)
+    gen = torch.Generator(device=DEV).manual_seed(14)
+    x = torch.randn(T, 128, generator=gen, device=DEV).half()
+    logits = torch.randn(T, routed, generator=gen, device=DEV)
+    g2l = torch.full((routed,), -1, dtype=torch.int32, device=DEV)
+    g2l[1::2] = torch.arange(E, dtype=torch.int32, device=DEV)
+    runs = {p: layer.forward(x, logits, k, True, torch.float16, global_to_local=g2l, path=p).clone()
+            for p in (capi.PATH_AUTO, capi.PATH_DECODE, capi.PATH_BATCH, capi.PATH_TENSOR)}
+    layer.check_status()
+    assert [p for p in runs if p and torch.equal(runs[p], runs[capi.PATH_AUTO])] == [path]
+
+
 # matrices in which several rows hold the same rank: single rows (of one width and of two), and a whole aligned octet twice
 def test_rows_that_repeat_a_rank():
     E, rank, inter, T = 3, 64, 256, 200
