@@ -296,3 +296,25 @@ def test_layer_call_is_its_stages(T, E, k, rank, dtype):
         layer.check_status()
         # (products of another kernel may differ in the last place of h, and so of y)
         helpers.assert_close(got.float().cpu(), want.float().cpu(), rtol=2.0 ** -7, atol=2e-3, what="layer call")
+
+
+# placement of a layer call's assignments by one cluster: the edges of four and of eight rounds and the first size beyond, tables of
+# many experts, choices spread out, gathered on few experts, and (top 1) all on one, whose prefixes are the largest
+@pytest.mark.parametrize("E,k", [(128, 8), (512, 10), (1024, 4), (128, 1)])
+def test_placement_of_many_assignments(E, k):
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=128, top_k=k, rank=64)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=E + k, device=DEV))
+    layer.set_deterministic(True)
+    gen = torch.Generator(device=DEV).manual_seed(15)
+    for T in (16384 // k + 1, 32768 // k, 32768 // k + 1, 65536 // k, 65536 // k + 1):
+        x = torch.randn(T, 128, generator=gen, device=DEV).half()
+        for skew in (0.0, 3.0, 100.0):
+            logits = torch.randn(T, E, generator=gen, device=DEV) - skew * torch.log(torch.arange(1.0, E + 1, device=DEV)).flip(0)
+            idx, w = route_topk(logits, k, True, torch.float16)
+            flat, by = torch.sort(idx.reshape(-1), stable=True)
+            off = torch.zeros(E + 1, dtype=torch.int32, device=DEV)
+            off[1:] = torch.bincount(flat.long(), minlength=E).cumsum(0)
+            acc = layer.experts_forward(*layer.basis_project(x), (by // k).to(torch.int32), off, w.reshape(-1)[by])
+            # sums do not depend on their order here, and the products are the same launches: every bit agrees
+            assert torch.equal(layer.forward(x, logits, k, True, torch.float16), layer.combine_down_basis(acc, torch.float16)), (T, skew)
+    layer.check_status()
