@@ -11,11 +11,13 @@
 // What bounds it: issue slots.  Turning a word into fp16(q * scale) takes 3.5 instructions for two codes and mma.sync holds a
 // scheduler 8.5 cycles, which do not overlap: a tile costs an SM 2.7 K cycles and 0.8 K for every eight tokens (gate and up 1.9 K of
 // them at 16).  The decode kernel (experts_decode.cu), with less work per code and its weights' scale in the operand, takes 2.8 K
-// with eight tokens, but a second pass doubles that.  128 tokens on 128 experts (8 each) 31.4 -> 24.4 us, 203 tokens 32.4 -> 25.2,
-// 300 tokens 40 (tensor path) -> 39; 64 experts of 1408 columns, 128 tokens 30.7 -> 23.4.  Measured and not taken: 32 tokens a
-// pass (203 tokens 33 us, 256 tokens 33 against 39, skewed 300 tokens 53 against 39), a third CTA per SM (80 registers: 203 tokens
-// 27.5), the scale in the operand instead of the weights (203 tokens 27).  Against 64 bits the stage is off by 4.2e-4 (203 tokens; the
-// decode kernel by 4.7e-4, whose operand is rounded twice).
+// with eight tokens, but a second pass doubles that.  128 tokens on 128 experts of six tiles (8 each) 31.1 -> 22.7 us, 64 experts of
+// eleven tiles 31.3 -> 22.7.  The stage takes as long as its longest CTA, 7.3 us and 5.2 a tile, and the last round is cut by an integer
+// quotient: up to 148 passes on 296 CTAs leave a CTA three of the six tiles (203 tokens 32 -> 23 us), 149 all six (38 us).  203 tokens
+// are 145 +- 3 passes, so one load in eight takes the longer time.
+// Measured and not taken: 32 tokens a pass (203 tokens 33 us, 256 tokens 33 against 39, skewed 300 tokens 53 against 39), a third CTA
+// per SM (80 registers: 203 tokens 27.5), the scale in the operand instead of the weights (203 tokens 27).  Against 64 bits the stage
+// is off by 4.2e-4 (203 tokens; the decode kernel by 4.7e-4, whose operand is rounded twice).
 //
 // Every wait is bounded; one that gives up raises a flag, the warps agree at the next barrier to leave, and the status word reports
 // BM_ERR_TIMEOUT behind the copies under way.
