@@ -510,18 +510,19 @@ static int expected_passes(int experts, double load, int size) {
   }
 }
 // Tiles, one after the other, of the CTA with the most where `passes` units of all tiles go over a grid of two CTAs an SM in whole rounds,
-// and what is left as a round cut along the tiles (with `cut_last` always, else only as the first one).  A round of up to a third of the
-// grid counts half: its CTAs have an SM each.
+// and what is left as a round cut along the tiles (with `cut_last` always, else only as the first one).  Where there is no more than a third
+// of a round it counts half: its CTAs have an SM each.
 static double longest_cta(int passes, int tiles, int grid, bool cut_last) {
   const int rest = passes % grid, full = passes / grid, split = rest && (cut_last || !full) ? std::max(1, grid / rest) : 1;
   const int per = (tiles + split - 1) / split, units = rest * ((tiles + per - 1) / per);
-  return full * tiles + (rest == 0 ? 0.0 : 3 * units <= grid ? 0.5 * per : per);
+  return full * tiles + (rest == 0 ? 0.0 : !full && 3 * units <= grid ? 0.5 * per : per);
 }
 // Whether passes of 16 (experts_batch_kernel) take less time than passes of 8 (experts_decode_kernel).  Both are as slow as their longest
 // CTA: 7.3 us and 5.2 a tile against 7 and 4.1, and with one pass more than half of the grid a CTA has twice the tiles.  us of the stage with
 // passes of 8 / of 16: 128 experts of 6 tiles, 4 assignments each 18.9 / 22.2, 7 each 30.9 / 23.0, 12 each 32.1 / 23.0, 14 each 31.9 / 38.4, 16 each
 // 46.3 / 38.2; 160 experts of 12 tiles, 8 each 56.7 / 70.1, 12 each 84.9 / 70.2; 16 of 4 tiles, 8 each 9.1 / 10.4; 48 of 6 tiles, 6 each 14.9 / 12.4; 512
-// of 4 tiles, 7 each 51.7 / 53.7, 9 each 60.5 / 54.0.  Over 19 shapes at 2 to 24 assignments an expert this takes 1.001 of the faster kernel's time.
+// of 4 tiles, 7 each 51.7 / 53.7 (under a skewed load passes of 8 are more: a block of 330 tokens 104 / 96), 9 each 60.5 / 54.0.  Over 19 shapes
+// at 2 to 24 assignments an expert this takes 1.001 of the faster kernel's time.
 static bool batch_passes_pay(const bm_layer* L, double load) {
   if (load <= 4.0) return false;      // one pass of 8 for nearly every expert
   const double t8 = longest_cta(expected_passes(L->num_experts, load, FAST_MAX_TOK), L->n_tiles, L->dec_grid, false);
