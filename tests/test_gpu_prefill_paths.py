@@ -286,16 +286,21 @@ def test_layer_call_is_its_stages(T, E, k, rank, dtype):
     gen = torch.Generator(device=DEV).manual_seed(T)
     x = torch.randn(T, 128, generator=gen, device=DEV).to(dtype)
     logits = torch.randn(T, E, generator=gen, device=DEV)
-    res = torch.randn(T, 128, generator=gen, device=DEV).to(dtype)
     idx, w = route_topk(logits, k, True, dtype)
     tok, off, rw, _, _ = route_build(idx, w, E)
     hg, hu = layer.basis_project(x)
-    want = layer.combine_down_basis(layer.experts_forward(hg, hu, tok, off, rw), dtype, residual=res)
-    for _ in range(2):
-        got = layer.forward(x, logits, k, True, dtype, residual=res)
-        layer.check_status()
-        # (products of another kernel may differ in the last place of h, and so of y)
-        helpers.assert_close(got.float().cpu(), want.float().cpu(), rtol=2.0 ** -7, atol=2e-3, what="layer call")
+    acc = layer.experts_forward(hg, hu, tok, off, rw)
+    # alone, and on a residual of the experts' own size: beside a larger one a wrong or missing result would pass
+    alone = layer.combine_down_basis(acc, dtype)
+    res = (torch.randn(T, 128, generator=gen, device=DEV) * alone.float().std()).to(dtype)
+    for residual, want in ((None, alone), (res, layer.combine_down_basis(acc, dtype, residual=res))):
+        for _ in range(2):
+            got = layer.forward(x, logits, k, True, dtype, residual=residual)
+            layer.check_status()
+            # (products of another kernel may differ in the last place of h, and so of y: the bounds on peak and norm are what counts)
+            helpers.assert_close(got, want, rtol=2.0 ** -7, atol=2e-3, what="layer call")
+        with pytest.raises(AssertionError):
+            helpers.assert_close(torch.zeros_like(got) if residual is None else residual, want, rtol=2.0 ** -7, atol=2e-3, what="nothing from the experts")
 
 
 # placement of a layer call's assignments by one cluster: the edges of four and of eight rounds and the first size beyond, tables of
