@@ -38,8 +38,12 @@
 // Stage of 8192 tokens of 128 experts (rank 256, intermediate 768): 121 us (176 before weights were converted in pairs), 2048
 // tokens 59 (72), 777 tokens 45 (59), 300 tokens 40 (50); of 512 experts: 16384 tokens 235 us (318), 2048 tokens 99 (125 with 128
 // rows), 1050 tokens 90 (114).
-// The mapped arrivals carry no cluster-scope release: what they publish is read by the tensor cores of the CTA that wrote it
-// (behind the proxy fence); with the release a converter's arrival took 1.4 K cycles and the stage of 8192 tokens 165 us.
+// The mapped arrivals carry no cluster-scope release: what they publish is read by the tensor core of the CTA that wrote it, behind
+// the proxy fence, and is in shared memory before the arrival leaves.  The PTX memory model does not promise this order to the other CTA's
+// issuer; it rests on the hardware.  A form that it does cover -- arrivals within a CTA, passed on by warps of the odd CTA with
+// .release.cluster and waited for with .acquire.cluster -- gives the same bits in deterministic mode (1200 runs of 520 to 4096
+// tokens, two shapes) and takes a layer call of 8192 tokens from 180 to 208 us, a block of 777 from 78 to 100, 2048 tokens of 64 experts from
+// 155 to 163; with the release in the converters' own arrivals, 1.4 K cycles each, the stage of 8192 tokens takes 165 us.
 //
 // The down product of a chunk is issued one chunk late (G0 U0 | G1 U1 D0 | G2 U2 D1 | ...).  Every mbarrier wait is
 // bounded in time.  One that gives up raises a flag in both CTAs; the roles then leave at their next wait that is not over, the
