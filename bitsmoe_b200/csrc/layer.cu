@@ -602,6 +602,17 @@ extern "C" int bm_experts_forward(const bm_layer_t* L, const uint16_t* h_gate, c
                               false, workspace, workspace_bytes, stream);
 }
 
+extern "C" int bm_experts_forward_expecting(const bm_layer_t* L, const uint16_t* h_gate, const uint16_t* h_up,
+                                            const int32_t* token_indices, const int32_t* expert_offsets,
+                                            const float* route_weights, int32_t T, int32_t num_assign, int32_t num_expected,
+                                            float* rank_accum, int32_t path, void* workspace, size_t workspace_bytes, void* stream) {
+  bm::NvtxRange nvtx_range("bm_experts_forward");
+  BM_REQUIRE(num_expected >= 0 && num_expected <= num_assign, BM_ERR_INVALID_ARG, "experts_forward: %d assignments expected of at most %d",
+             num_expected, num_assign);
+  return experts_forward_impl(L, h_gate, h_up, token_indices, expert_offsets, route_weights, T, num_assign, num_expected, rank_accum, path,
+                              false, workspace, workspace_bytes, stream);
+}
+
 // y = fp16(rank_accum) . U_down^T (+ (z * sigmoid(gate)) . W_down^T of a shared expert) (+ residual), one launch.
 static int combine_small(const bm_layer_t* L, const float* rank_accum, int T, const __half* w_down, int w_bf16, const float* z, const float* gate,
                          int inter, const void* residual, void* y, int y_dtype, bool overlap, cudaStream_t st) {

@@ -219,6 +219,12 @@ BM_API int bm_experts_forward(const bm_layer_t* layer, const uint16_t* h_gate, c
                        const int32_t* token_indices, const int32_t* expert_offsets, const float* route_weights,
                        int32_t T, int32_t num_assign, float* rank_accum, int32_t path,
                        void* workspace, size_t workspace_bytes, void* stream);
+/* The same where the lists are expected to be shorter than their bound, as on a rank that holds a share of the experts:
+ * BM_PATH_AUTO chooses the kernel for num_expected <= num_assign assignments.  Any length up to num_assign is right. */
+BM_API int bm_experts_forward_expecting(const bm_layer_t* layer, const uint16_t* h_gate, const uint16_t* h_up,
+                       const int32_t* token_indices, const int32_t* expert_offsets, const float* route_weights,
+                       int32_t T, int32_t num_assign, int32_t num_expected, float* rank_accum, int32_t path,
+                       void* workspace, size_t workspace_bytes, void* stream);
 /* y = fp16(rank_accum) @ U_down^T (+ residual) in y_dtype (bitsmoe/models/base_block.py:414 and the
  * adds of qwen3moe/bitsmoe_block.py:95, deepseekv2/bitsmoe_block.py:123-124).  residual may be NULL. */
 BM_API int bm_combine_down_basis(const bm_layer_t* layer, const float* rank_accum, int32_t T,

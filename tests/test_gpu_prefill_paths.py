@@ -150,6 +150,33 @@ def test_a_shard_is_chosen_for_by_its_share(T, path):
     assert [p for p in runs if p and torch.equal(runs[p], runs[capi.PATH_AUTO])] == [path]
 
 
+# lists shorter than their bound (a rank of an expert-parallel group): chosen for the expected length, right for any
+def test_expected_length_chooses_the_kernel():
+    E, bound, load = 48, 48 * 6, [3] * 48
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=768, top_k=1, rank=64)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=10, device=DEV))
+    layer.set_deterministic(True)
+    lib, gen, T = capi.lib(), torch.Generator(device=DEV).manual_seed(16), 64
+    hg, hu = layer.basis_project(torch.randn(T, 128, generator=gen, device=DEV).half())
+    tok, off, rw = _route(load, 1, T, gen)
+    ws = torch.empty(lib.bm_experts_workspace_bytes(layer._handle, T, bound, capi.PATH_AUTO), dtype=torch.uint8, device=DEV)
+
+    def run(expected, num_assign=bound):
+        acc = torch.empty(T, layer.rank_out, device=DEV)
+        capi.check(lib.bm_experts_forward_expecting(layer._handle, hg.data_ptr(), hu.data_ptr(), tok.data_ptr(), off.data_ptr(), rw.data_ptr(), T,
+                                                    num_assign, expected, acc.data_ptr(), capi.PATH_AUTO, ws.data_ptr(), ws.numel(),
+                                                    capi.stream_ptr(acc.device)))
+        layer.check_status()
+        return acc
+
+    by_path = {p: layer.experts_forward(hg, hu, tok, off, rw, path=p) for p in (capi.PATH_DECODE, capi.PATH_BATCH)}
+    for expected, path in ((0, capi.PATH_DECODE), (len(tok), capi.PATH_DECODE), (bound, capi.PATH_BATCH)):
+        assert [p for p in by_path if torch.equal(by_path[p], run(expected))] == [path]
+    for expected in (-1, bound + 1):
+        with pytest.raises(capi.BitsMoEError, match="expected of at most"):
+            run(expected)
+
+
 # matrices in which several rows hold the same rank: single rows (of one width and of two), and a whole aligned octet twice
 def test_rows_that_repeat_a_rank():
     E, rank, inter, T = 3, 64, 256, 200
