@@ -1,7 +1,7 @@
 // Packed routed-expert forward for batches of some tokens per expert: weights on the tensor cores (mma.sync) with 16 tokens a pass.
 //
 // Work unit = (expert, pass of up to 16 of its assignments, range of its 128-column tiles); passes that fill whole rounds of the
-// grid (two CTAs an SM) are units of their own, those of the last, partial round are cut along the tiles.  A unit gathers its
+// grid (two CTAs an SM) are units of their own, those of the last, partial round are cut along the tiles, evenly.  A unit gathers its
 // tokens' rows once into the operand hs = fp16(h[rank] * s) (16-byte octets, as the tensor path stages them).  Per tile the eight
 // warps turn the section's words into A fragments -- fp16(q * scale), the very weights the tensor path multiplies -- for two
 // blocks of eight tokens: gate and up into z = silu(g) * u (shared memory), one barrier, down into accumulators that stay in
@@ -12,9 +12,10 @@
 // scheduler 8.5 cycles, which do not overlap: a tile costs an SM 2.7 K cycles and 0.8 K for every eight tokens (gate and up 1.9 K of
 // them at 16).  The decode kernel (experts_decode.cu), with less work per code and its weights' scale in the operand, takes 2.8 K
 // with eight tokens, but a second pass doubles that.  128 tokens on 128 experts of six tiles (8 each) 31.1 -> 22.7 us, 64 experts of
-// eleven tiles 31.3 -> 22.7.  The stage takes as long as its longest CTA, 7.3 us and 5.2 a tile, and the last round is cut by an integer
-// quotient: up to 148 passes on 296 CTAs leave a CTA three of the six tiles (203 tokens 32 -> 23 us), 149 all six (38 us).  203 tokens
-// are 145 +- 3 passes, so one load in eight takes the longer time.
+// eleven tiles 31.3 -> 22.7.  The stage takes as long as its longest CTA, 7.3 us and 5.2 a tile; a second unit costs 4.8 (operand, sums, the way
+// through the ring).  148 passes on 296 CTAs leave a CTA three of six tiles (22.9 us); cut by an integer quotient 149 to 295 left one all six
+// (37.7), in even shares 149 to 197 passes take 28 to 31 us, 198 to 246 36, and behind whole rounds 445 64 instead of 70.  203 tokens are 145 +- 3
+// passes, one load in eight more than 148.
 // Measured and not taken: 32 tokens a pass (203 tokens 33 us, 256 tokens 33 against 39, skewed 300 tokens 53 against 39), a third CTA
 // per SM (80 registers: 203 tokens 27.5), the scale in the operand instead of the weights (203 tokens 27).  Against 64 bits the stage
 // is off by 4.2e-4 (203 tokens; the decode kernel by 4.7e-4, whose operand is rounded twice).
@@ -52,6 +53,8 @@ __host__ __device__ inline BtLayout bt_layout(int max_slots, int sec_bytes, int 
   L.total = o;
   return L;
 }
+// Whether a last round of `all` tiles is handed out in even shares: where the longest one is shorter than `per`, the tiles of a pass's part.
+__device__ __forceinline__ bool bt_even_shares(int all, int per, int grid) { return all <= (per - 1) * grid; }
 // Place of 16-byte piece c of token row n: the rows that a quarter warp reads (n, n + 1) lie in distinct banks.
 __device__ __forceinline__ int bt_piece(int n, int c) { return (c ^ ((n & 1) << 2)) * 16; }
 
@@ -152,7 +155,7 @@ __global__ void __launch_bounds__(BT_THREADS, 2) experts_batch_kernel(const __gr
   extern __shared__ __align__(128) unsigned char bt_smem[];
   __shared__ BtUnit info[2];
   __shared__ __align__(8) uint64_t bar_full[BT_MAX_RING], bar_tab[2];
-  __shared__ int warp_tot[BT_WARPS], abort_s[2];
+  __shared__ int warp_tot[BT_WARPS], abort_s[2], n_units_s;
   volatile int* abort_flag = abort_s;
   const int tid = threadIdx.x, warp = tc::warp_index(), lane = tid & 31, g = lane >> 2, t = lane & 3;
   const BtLayout lay = bt_layout(A.max_slots, A.sec_bytes, A.ring, A.num_experts, A.tab_bytes);
@@ -211,14 +214,29 @@ __global__ void __launch_bounds__(BT_THREADS, 2) experts_batch_kernel(const __gr
     }
     __syncthreads();
   }
-  // Passes that fill whole rounds of the grid are units of their own, those of the last, partial round are cut along the tiles.
-  const int grid = static_cast<int>(gridDim.x);
-  const int rem = total % grid, full = total - rem;
-  int split = rem ? min(grid / rem, A.n_tiles) : 1;
-  const int per = (A.n_tiles + split - 1) / split;
-  split = (A.n_tiles + per - 1) / per;
-  const int n_units = full + rem * split;
-  if (static_cast<int>(blockIdx.x) >= n_units) return;
+  // Passes that fill whole rounds of the grid are units of their own.  Those of the last, partial round are cut along the tiles: into equal
+  // parts, a part a CTA, or, where that leaves the longest part a tile more than an even share of all, into such shares of the passes laid
+  // end to end, which may hold the end of one pass and the start of the next (two units).  One warp works it out: divisions in all eight
+  // took 0.4 us of issue slots.
+  const int grid = static_cast<int>(gridDim.x), cta = static_cast<int>(blockIdx.x);
+  const int rounds = total / grid, rem = total - rounds * grid;
+  int last_pass = 0, last_tile = 0, last_ntiles[2] = {0, 0};      // this CTA's units of the last round: the second one starts the next pass
+  if (warp == 0 && rem) {
+    const int parts = min(grid / rem, A.n_tiles), per = (A.n_tiles + parts - 1) / parts, all = rem * A.n_tiles;
+    if (bt_even_shares(all, per, grid)) {
+      const int first = cta * all / grid, end = (cta + 1) * all / grid;
+      last_pass = first / A.n_tiles;
+      last_tile = first - last_pass * A.n_tiles;
+      last_ntiles[0] = min(end - first, A.n_tiles - last_tile);
+      last_ntiles[1] = end - first - last_ntiles[0];
+    } else {
+      const int used = (A.n_tiles + per - 1) / per;
+      last_pass = cta / used;
+      last_tile = (cta - last_pass * used) * per;
+      last_ntiles[0] = last_pass < rem ? min(per, A.n_tiles - last_tile) : 0;
+    }
+  }
+  if (tid == 0) n_units_s = rounds + (last_ntiles[0] > 0) + (last_ntiles[1] > 0);
 
   const DqMagic magic;
   // ---- unit look-up (warp 0): issued with `begin`, in shared memory after `finish`
@@ -227,13 +245,13 @@ __global__ void __launch_bounds__(BT_THREADS, 2) experts_batch_kernel(const __gr
   int nx_tok = 0, nx_n = 0, nx_tile0 = 0, nx_ntiles = 0;
   float nx_rw = 0.f;
   int looked_up = 0;                            // units whose tables are on their way or there
-  auto look_up = [&](int u, int it) {
-    int pu = u, tile0 = 0, ntl = A.n_tiles;
-    if (u >= full) {
-      const int r = u - full, part = r % split;
-      pu = full + r / split;
-      tile0 = part * per;
-      ntl = min(per, A.n_tiles - tile0);
+  auto look_up = [&](int it) {
+    int pu = cta + it * grid, tile0 = 0, ntl = A.n_tiles;
+    if (it >= rounds) {
+      const bool second = it > rounds;
+      pu = rounds * grid + last_pass + second;
+      tile0 = second ? 0 : last_tile;
+      ntl = second ? last_ntiles[1] : last_ntiles[0];
     }
     int lo = 0, hi = A.num_experts - 1;           // last expert whose prefix is <= pu
     while (lo < hi) {
@@ -242,9 +260,13 @@ __global__ void __launch_bounds__(BT_THREADS, 2) experts_batch_kernel(const __gr
     }
     // an expert's assignments are spread evenly over its passes
     const int e = lo, begin = soff[e], cnt = soff[e + 1] - begin, parts = (cnt + BT_NT - 1) / BT_NT, j = pu - pbase[e];
-    const int a0 = begin + static_cast<int>(static_cast<int64_t>(cnt) * j / parts);
+    int a0 = begin, end = begin + cnt;
+    if (parts > 1) {      // (64-bit divisions)
+      a0 = begin + static_cast<int>(static_cast<int64_t>(cnt) * j / parts);
+      end = begin + static_cast<int>(static_cast<int64_t>(cnt) * (j + 1) / parts);
+    }
     ++looked_up;
-    nx_n = begin + static_cast<int>(static_cast<int64_t>(cnt) * (j + 1) / parts) - a0;
+    nx_n = end - a0;
     nx_tile0 = tile0;
     nx_ntiles = ntl;
 #pragma unroll
@@ -299,16 +321,18 @@ __global__ void __launch_bounds__(BT_THREADS, 2) experts_batch_kernel(const __gr
   auto advance = [&]() { if (++rs == R) { rs = 0; rp ^= 1u; } };
   bool ok = A.wait_limit_us != 0, leave = false;      // this warp's waits; what the warps decided
   int it = 0;
-  if (warp == 0) {
-    look_up(blockIdx.x, 0);
+  if (warp == 0 && rounds + last_ntiles[0] > 0) {
+    look_up(0);
     look_up_done(0);
     if (lane == 0) issue(R, 1);
   }
   __syncthreads();
-  for (int u = blockIdx.x; u < n_units; u += grid, ++it) {
+  const int n_units = n_units_s;                // of this CTA
+  for (; it < n_units; ++it) {
     const BtUnit& si = info[it & 1];
     const FastExpert& fe = si.fe;
-    const int npass = si.npass, ntl = si.ntiles, next_u = u + grid;
+    const int npass = si.npass, ntl = si.ntiles;
+    const bool more = it + 1 < n_units;
     const unsigned char* tab = bt_smem + lay.tab + (it & 1) * tab_stride;
     ok = ok && bt_wait(&bar_tab[it & 1], (it >> 1) & 1, abort_flag);
     // ---- operand rows hs[m][n][position] = fp16(h[token, rank] * s).  A lane owns an octet of ranks, which the arena layout
@@ -386,7 +410,7 @@ __global__ void __launch_bounds__(BT_THREADS, 2) experts_batch_kernel(const __gr
     if ((leave = __syncthreads_or(!ok))) break;
     // every warp is done with the unit before: its ring slots, its description and its tables
     if (tid == 0) issue(used + R, it + 1);
-    if (warp == 0 && next_u < n_units) look_up(next_u, it + 1);
+    if (warp == 0 && more) look_up(it + 1);
 
     float dacc[MAXMB][BT_NP][4];
 #pragma unroll
@@ -435,10 +459,10 @@ __global__ void __launch_bounds__(BT_THREADS, 2) experts_batch_kernel(const __gr
           }
         }
       }
-      if (warp == 0 && i == 0 && next_u < n_units) look_up_done(it + 1);
+      if (warp == 0 && i == 0 && more) look_up_done(it + 1);
       if ((leave = __syncthreads_or(!ok))) break;
       // every warp has read this tile's gate and up sections and the down section before them
-      if (tid == 0) issue(used + 2 + R, next_u < n_units ? it + 2 : it + 1);
+      if (tid == 0) issue(used + 2 + R, more ? it + 2 : it + 1);
       used += 3;
       // ---- down: slot blocks round-robin over the warps, contraction over the tile's 128 columns
       ok = bt_wait(&bar_full[rs], rp, abort_flag);

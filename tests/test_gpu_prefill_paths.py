@@ -114,6 +114,25 @@ def test_named_kernels_run_at_any_load():
     assert not torch.equal(whole[capi.PATH_DECODE], whole[capi.PATH_BATCH])
 
 
+# passes of 16 around the numbers at which the last round is handed out in even shares of its tiles (here 6, on 296 CTAs: 149 to 246
+# passes), alone and behind a whole round; a share holds the end of one pass and the start of the next
+@pytest.mark.parametrize("passes", [148, 149, 150, 197, 198, 246, 247, 296, 297, 296 + 149, 296 + 246])
+def test_passes_in_even_shares(passes):
+    E, T = 8, 960
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=768, top_k=1, rank=64)
+    layer = synth.to_packed_layer(synth.make_layer(cfg, seed=11, device=DEV))
+    layer.set_deterministic(True)
+    gen = torch.Generator(device=DEV).manual_seed(passes)
+    parts = [passes // E + (e < passes % E) for e in range(E)]
+    tok, off, rw = _route([16 * n - (7 if n > 1 else 0) for n in parts], 1, T, gen)
+    hg, hu = layer.basis_project(torch.randn(T, 128, generator=gen, device=DEV).half())
+    want = layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_GENERIC)
+    got = [layer.experts_forward(hg, hu, tok, off, rw, path=capi.PATH_BATCH) for _ in range(2)]
+    layer.check_status()
+    helpers.assert_close(got[0], want, what=f"{passes} passes")
+    assert torch.equal(*got)
+
+
 # The automatic choice, told by its bits in deterministic mode: passes of 16 where they leave the longest CTA less work than passes of 8
 # (not with a tile a CTA either way, nor where they just exceed half of the grid), products on tcgen05 above 24 assignments an expert
 @pytest.mark.parametrize("E,inter,load,path", [(16, 512, 8, capi.PATH_DECODE), (16, 1536, 12, capi.PATH_BATCH), (48, 768, 6, capi.PATH_BATCH),
