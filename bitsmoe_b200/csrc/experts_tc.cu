@@ -10,8 +10,8 @@
 // Tokens as rows make the epilogue cheap: a thread owns a token.  Tensor memory holds two gate/up accumulator pairs beside the
 // down accumulator, so the products of a chunk run while the previous one is turned into z.  128 rows: a lane is a row; z goes
 // back to tensor memory, over the gate sums it came from, and is the A operand of the down product there.  64 rows: lanes 0-63
-// hold the lower half of an accumulator's columns, lanes 64-127 the upper half, which leaves columns for chunks of 128; z is an
-// operand in shared memory.
+// hold the lower half of an accumulator's columns, lanes 64-127 the upper half, which leaves columns for chunks of 128 and for three down
+// tiles (matrices of 257 to 384 slots take this form at any load); z is an operand in shared memory.
 //
 // Warp roles (768 threads; the last warp completes the last warpgroup):
 //   warps 0-7   epilogue (two per TMEM lane quarter, 32 columns each): tcgen05.ld D_g/D_u -> z = silu(g)*u -> fp16;
@@ -48,10 +48,15 @@
 // The down product of a chunk is issued one chunk late (G0 U0 | G1 U1 D0 | G2 U2 D1 | ...).  Every mbarrier wait is
 // bounded in time.  One that gives up raises a flag in both CTAs; the roles then leave at their next wait that is not over, the
 // look-up warp behind its copy, both CTAs behind the MMAs issued so far, and tensor memory is given back after that.
+#include <algorithm>
+#include <limits>
+
 #include "dequant.cuh"
 #include "tc05.cuh"
 
 namespace bm {
+
+int expected_passes(int experts, double load, int size);      // layer.cu
 
 constexpr int XT_NT_MAX = 128;            // most tokens (assignments) of an item in a CTA: its rows of one MMA
 constexpr int XT_THREADS = 768;
@@ -65,6 +70,7 @@ static_assert(32 * (XT_EPI_WARPS * XT_REGS_EPI + XT_DQ_WARPS * XT_REGS_DQ + 4 * 
 constexpr int XT_ACC = 64;                // columns of tensor memory of a gate or up accumulator
 // Tile columns per step, by the rows (tokens) of a CTA: 64 rows of a pair's accumulator take half as many columns as it has
 __host__ __device__ constexpr int xt_chunk(int rows) { return rows > 64 ? 64 : 128; }
+__host__ __device__ constexpr int xt_down_cols(int rows) { return rows > 64 ? 128 : 64; }
 // Operand slots per pipeline, by the rows (tokens) of a CTA
 __host__ __device__ constexpr int xt_ring(int rows) { return rows > 64 ? 4 : 6; }
 constexpr int XT_RING_MAX = 6;
@@ -211,7 +217,7 @@ struct XtArgs {
   float* rank_accum;
   long long* acc64;
   int* status;
-  int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, gu_bufs, tab_bytes;
+  int h_rank, rank_out, T, num_experts, n_tiles, max_slots, nt, tab_bytes;
   int wait_limit_us;
   int vec_add;            // every row of rank_accum starts on a 16-byte boundary (and takes fp32 adds)
 };
@@ -265,7 +271,7 @@ struct XtPre {
   uint4 s[2];
 };
 
-// WIDE: more than 256 row slots a matrix; a step then has more stages than converter warps.
+// WIDE: more than 256 row slots a matrix (64 rows); a step then has more stages than the warps can keep apart by their place in it.
 template <int ROWS, bool WIDE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) experts_tc_kernel(const __grid_constant__ XtArgs A) {
   extern __shared__ __align__(128) unsigned char xt_raw[];
@@ -279,6 +285,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
   constexpr uint32_t ring = xt_ring(ROWS);
   const int nt = A.nt, h_rank = A.h_rank, num_experts = A.num_experts;
   const int cs = xt_chunk_stride(nt);     // bytes between 8-position chunks of act
+  constexpr int D_COLS = xt_down_cols(ROWS);      // of tensor memory per 128-slot tile of the down product
   constexpr int CH = xt_chunk(ROWS), PER_TILE = N_TILE / CH, G_STRIDE = xt_g_stride(ROWS);
   const int n_chunks = A.n_tiles * PER_TILE;
   const uint32_t act_m_bytes = static_cast<uint32_t>(A.max_slots / 8) * cs;
@@ -347,10 +354,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
   const XtUnits units(sm.prefix[num_experts], n_pairs, n_chunks);
   const uint32_t lead_bars = tc::cluster_map(tc::smem_u32(&bars), 0);      // the barriers of the CTA that issues the MMAs
   auto lead = [&](const uint64_t* bar) { return lead_bars + static_cast<uint32_t>(reinterpret_cast<const char*>(bar) - reinterpret_cast<const char*>(&bars)); };
-  // tensor memory: gu_bufs x (gate 64 columns, up 64 columns), then the down product's slot tiles of 128 columns
-  const uint32_t d_down = tmem_base + A.gu_bufs * 2 * XT_ACC;
-  // the down product of a chunk is issued `lag` chunks late: one where tensor memory holds two gate/up accumulator pairs
-  const int lag = A.gu_bufs - 1;
+  // tensor memory: two times gate (64 columns) and up (64), then the down product's slot tiles
+  const uint32_t d_down = tmem_base + 2 * 2 * XT_ACC;
+  constexpr int lag = 1;                  // chunks that the down product of a chunk is issued late
 
   // The roles run through this CTA's items independently; what they share is guarded by barriers only.  Item number
   // `round` uses description and table buffer round & 1.  After a wait that gave up, every further wait gives up too.
@@ -381,8 +387,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
       const bool busy = n0 < n_tok;                               // any token in this quarter
       bool ok = true;
       for (int t = 0; t < nchunk && ok; ++t) {
-        const uint32_t g = gu_round + t, b = lag ? g & 1u : 0u;
-        ok = xt_wait(&bars.gu_done[b], (lag ? g >> 1 : g) & 1u, abort_flag);
+        const uint32_t g = gu_round + t, b = g & 1u;
+        ok = xt_wait(&bars.gu_done[b], (g >> 1) & 1u, abort_flag);
         if (!ok) break;
         tc::fence_after_sync();
         if (busy) {
@@ -431,7 +437,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
           const int s0 = col + 64 * upper;
           if (s0 >= nslots_d) break;
           float v[32];
-          tc::tmem_ld32(d_down + lane_sel + col, v);
+          tc::tmem_ld32(d_down + lane_sel + (ROWS > 64 ? col : col >> 1 & ~63 | 32 * half), v);
           const bool whole = s0 + 16 < nslots_d;          // the matrix may end after 16 of the 32 slots
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
@@ -710,14 +716,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
       };
       XtPre p;
       Stage st;
-      bool more = WIDE ? step() : i < 2 * per_step && (i < 2 * slots_gu || lag == 0 || step());
+      bool more = WIDE ? step() : i < 2 * per_step && (i < 2 * slots_gu || step());
       if (more) {
         st = describe(i);
         fetch(st, st.gu ? t : t - lag, p);
       }
       while (more) {
         // the use of a ring slot that this stage fills: steps before t, then this step's order (the last one has no gate / up)
-        const uint32_t pos = item_seq + t * per_step - (t > 0 && lag ? slots_d : 0) + (i >> 1) - (t == nchunk ? slots_gu : 0);
+        const uint32_t pos = item_seq + t * per_step - (t > 0 ? slots_d : 0) + (i >> 1) - (t == nchunk ? slots_gu : 0);
         if (!(ok = acquire(pos))) break;
         convert(st, p, ring0 + (pos % ring) * XT_SLOT_BYTES + st.dst_off);
         const int i_was = i;
@@ -777,7 +783,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
       tc::fence_after_sync();
       for (int t = 0; t < nchunk + lag && ok; ++t) {
         if (t < nchunk) {
-          const uint32_t g = gu_round + t, b = lag ? g & 1u : 0u, k = lag ? g >> 1 : g;
+          const uint32_t g = gu_round + t, b = g & 1u, k = g >> 1;
           if (k >= 1) ok = xt_wait(&bars.z_free[b], (k - 1) & 1u, abort_flag);     // the z written over this accumulator is multiplied
           tc::fence_after_sync();
           const uint32_t d_acc = tmem_base + (2 * b + pl) * XT_ACC;
@@ -805,9 +811,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
           __syncwarp();
         }
         if (t >= lag) {
-          const uint32_t g = gu_round + t - lag, b = lag ? g & 1u : 0u;
+          const uint32_t g = gu_round + t - lag, b = g & 1u;
           if (t == lag && round > 0) ok = xt_wait(&bars.down_free, (round - 1) & 1u, abort_flag);   // the last item's sums are read out
-          if (ok) ok = xt_wait(&bars.z_ready[b], (lag ? g >> 1 : g) & 1u, abort_flag);
+          if (ok) ok = xt_wait(&bars.z_ready[b], (g >> 1) & 1u, abort_flag);
           tc::fence_after_sync();
           const uint32_t d_z = tmem_base + 2 * b * XT_ACC;      // columns 0-31 of the chunk, and 32-63 32 columns on
           for (int mt = pl; mt < n_mt && ok; mt += 2)
@@ -820,9 +826,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
                 for (int h = 0; h < 4; ++h) {         // 16 columns of z each
                   const uint32_t add = t > lag || kp > 0 || h > 0 ? 1u : 0u;
                   if (ROWS > 64)
-                    tc::mma_f16_pair_ta(d_down + mt * 128, d_z + 32 * (h >> 1) + 8 * (h & 1), bd + ((h * 2 * XT_D_STRIDE) >> 4), idesc_d, add);
+                    tc::mma_f16_pair_ta(d_down + mt * D_COLS, d_z + 32 * (h >> 1) + 8 * (h & 1), bd + ((h * 2 * XT_D_STRIDE) >> 4), idesc_d, add);
                   else
-                    tc::mma_f16_pair(d_down + mt * 128, z_desc + ((b * XT_Z_BYTES + (4 * kp + h) * 2 * XT_Z_STRIDE) >> 4), bd + ((h * 2 * XT_D_STRIDE) >> 4), idesc_d, add);
+                    tc::mma_f16_pair(d_down + mt * D_COLS, z_desc + ((b * XT_Z_BYTES + (4 * kp + h) * 2 * XT_Z_STRIDE) >> 4), bd + ((h * 2 * XT_D_STRIDE) >> 4), idesc_d, add);
                 }
                 tc::mma_commit_pair(&w_empty[sl]);
               }
@@ -857,21 +863,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(XT_THREADS, 1) exper
 }
 
 // Item size and ring depth for a layer: the first candidate whose activation operand (2 KB per token at 256 row slots per
-// matrix) and stages fit shared memory.  Tensor memory holds 128 columns per gate/up buffer and 128 per 128
-// slots of the down product.
-// Assignments an expert up to which items of 2 x 64 tokens are taken.  2048 tokens of 128 experts, top 8 (128 each): 59 us against
-// 62 with 2 x 128; 4096 (256 each): 91 against 83; 2048 tokens of 512 experts, top 10 (40 each): 99 against 122; 1024 of 64
-// experts, top 6 (96 each): 46 against 49.
-constexpr int XT_FEW_ROWS = 160;
-struct XtPlan { int nt, gu_bufs; size_t smem; };
+// matrix) and stages fit shared memory.  Tensor memory holds two gate/up buffers of 128 columns and 128 (64 rows: 64) per 128 slots of
+// the down product: with 128 rows up to 256 slots.
+struct XtPlan { int nt; size_t smem; };
 constexpr size_t XT_SMEM_LIMIT = 227 * 1024 - 3072;     // dynamic part: the static part (two item descriptions, barriers) stays below 3 KB
 static bool xt_plan(const bm_layer* L, int rows, XtPlan* out) {
   if (!L->toktab_dev || L->num_experts > XT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > XT_MAX_SLOTS) return false;
-  const int n_mt = (L->max_slots + 127) / 128;
+  if (2 * 2 * XT_ACC + (L->max_slots + 127) / 128 * xt_down_cols(rows) > 512) return false;      // columns of tensor memory
   for (int nt = rows; nt >= 16; nt -= 16) {
     const size_t smem = xt_smem_bytes(L->max_slots, L->num_experts, TokTab(L->rank_in, L->max_slots).bytes, nt, rows);
     if (smem <= XT_SMEM_LIMIT) {
-      *out = XtPlan{nt, n_mt > 2 ? 1 : 2, smem};
+      *out = XtPlan{nt, smem};
       return true;
     }
   }
@@ -882,7 +884,35 @@ static bool xt_plan(const bm_layer* L, int rows, XtPlan* out) {
 // decode path otherwise).
 bool experts_tc_fits(const bm_layer* L) {
   XtPlan p;
-  return xt_plan(L, 128, &p);
+  return xt_plan(L, 64, &p) || xt_plan(L, 128, &p);
+}
+
+// The stage as a model, us: the tiles and units of the pair with the most, items of `2 nt` assignments spread evenly.  Fits to thirteen layer shapes (8
+// to 512 experts, 4 to 16 tiles, rank 128 to 384) at 17 to 180 assignments an expert, off by 4 %.
+static double xt_us(const bm_layer* L, int rows, int nt, double load) {
+  int dev = -1, sms = 148;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int pairs = sms / 2, items = std::max(1, expected_passes(L->num_experts, load, 2 * nt)), rest = items % pairs, full = items / pairs;
+  const int split = rest ? std::min(L->n_tiles, pairs / rest) : 1, last = rest ? (L->n_tiles + split - 1) / split : 0;
+  const double tiles = full * L->n_tiles + last, more = full - (rest == 0), slots = L->max_slots / 256.0;
+  if (L->max_slots > 256) return 14.7 + 3.6 * tiles + 2.6 * more;
+  return rows == 64 ? 11.9 + (0.9 + 1.3 * slots) * tiles + 3.1 * more : 14.4 + (1.1 + 1.55 * slots) * tiles + 5.8 * more;
+}
+// Rows of a CTA for this load.  More than 256 slots: always 64 (128 experts of 6 tiles and rank 384, 32 assignments each 57 us against 89 with 128
+// rows, which left tensor memory for one pair of accumulators only; 128 each 96 / 94; 256 each 142 / 158).  Else the smaller estimate: with 64 rows
+// an item is half as large and a quarter cheaper, so that they pay until many experts need a second one.  us with 64 / with 128: 128 experts of 6 tiles,
+// 64 each 41 / 51, 120 each 48 / 53, 128 each 58 / 52, 150 each 66 / 53, 256 each 84 / 74; 512 of 4 tiles, 108 each 99 / 125, 136 each 153 / 126; 64 of 11 tiles
+// and rank 128, 112 each 31 / 35, 128 each 41 / 35.  Under skewed loads the two are 3 % apart between 100 and
+// 150 each, 64 rows ahead where experts are few (hence the 8 %).
+static int xt_rows(const bm_layer* L, double load, double* us) {
+  XtPlan few, many;
+  const bool fits = xt_plan(L, 64, &few);
+  const double t64 = fits ? xt_us(L, 64, few.nt, load) : 0.0;
+  if (fits && L->max_slots > 256) { *us = t64; return 64; }
+  const double t128 = xt_plan(L, 128, &many) ? xt_us(L, 128, many.nt, load) : std::numeric_limits<double>::infinity();
+  const bool take64 = fits && t64 <= 1.08 * t128;
+  *us = take64 ? t64 : t128;
+  return take64 ? 64 : 128;
 }
 
 template <int ROWS, bool WIDE>
@@ -914,7 +944,8 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
   BM_REQUIRE(L->max_slots <= XT_MAX_SLOTS, BM_ERR_UNSUPPORTED, "experts_tc: %d row slots exceed the tensor-memory budget", L->max_slots);
   BM_REQUIRE(L->rank_in % 8 == 0 && ((reinterpret_cast<uintptr_t>(h_gate) | reinterpret_cast<uintptr_t>(h_up)) & 15u) == 0,
              BM_ERR_UNSUPPORTED, "experts_tc: rank-space rows must be 16-byte aligned (rank %d)", L->rank_in);
-  const int rows = L->max_slots <= 256 && expected_assign <= static_cast<int64_t>(XT_FEW_ROWS) * L->num_experts ? 64 : 128;
+  double us;
+  const int rows = xt_rows(L, static_cast<double>(expected_assign) / L->num_experts, &us);
   XtPlan plan;
   BM_REQUIRE(xt_plan(L, rows, &plan), BM_ERR_UNSUPPORTED, "experts_tc: the layer's largest expert does not fit in shared memory");
   XtArgs a{};
@@ -928,8 +959,8 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
   a.vec_add = acc64 == nullptr && L->rank_out % 4 == 0 && (reinterpret_cast<uintptr_t>(rank_accum) & 15u) == 0;
   a.wait_limit_us = L->wait_limit_us;
   a.rank_out = L->rank_out; a.T = T; a.num_experts = L->num_experts; a.n_tiles = L->n_tiles; a.max_slots = L->max_slots;
-  a.nt = plan.nt; a.gu_bufs = plan.gu_bufs;
-  if (L->max_slots > 256) return xt_launch<128, true>(a, plan.smem, st);
+  a.nt = plan.nt;
+  if (L->max_slots > 256) return xt_launch<64, true>(a, plan.smem, st);
   return rows > 64 ? xt_launch<128, false>(a, plan.smem, st) : xt_launch<64, false>(a, plan.smem, st);
 }
 

@@ -38,6 +38,7 @@ int plan_experts_batch(bm_layer* L);
 int launch_experts_batch(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices, const int32_t* expert_offsets,
                          const float* route_w, int T, float* rank_accum, long long* acc64, cudaStream_t st);
 bool experts_tc_fits(const bm_layer* L);
+int expected_passes(int experts, double load, int size);
 int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
                       const int32_t* expert_offsets, const float* route_w, int T, int expected_assign, float* rank_accum, long long* acc64,
                       cudaStream_t st);
@@ -498,8 +499,16 @@ extern "C" size_t bm_experts_workspace_bytes(const bm_layer_t* L, int32_t T, int
 
 // Passes of `size` assignments that the experts need together, where each has a Poisson number of them, `load` on average (choices
 // spread evenly over the experts): experts * sum over j of P(more than j * size).
-static int expected_passes(int experts, double load, int size) {
-  double p = std::exp(-load), at_most = p, passes = 0.0;
+int bm::expected_passes(int experts, double load, int size) {
+  double passes = 0.0;
+  if (load > 32.0) {      // a normal number is close enough, and its sum has few terms
+    for (int n = 0;; n += size) {
+      const double more = 0.5 * std::erfc((n + 0.5 - load) / std::sqrt(2.0 * load));
+      if (more < 1e-4) return static_cast<int>(experts * passes + 0.5);
+      passes += more;
+    }
+  }
+  double p = std::exp(-load), at_most = p;
   for (int n = 0, next = 0;;) {
     if (n == next) {
       if (1.0 - at_most < 1e-4) return static_cast<int>(experts * passes + 0.5);

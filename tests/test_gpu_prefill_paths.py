@@ -21,7 +21,7 @@ def _route(counts, k, T, gen):
 
 # assignments per expert around an item (128) and a pass (8), none at all, one expert alone; ranks whose row slots are an odd
 # number of pairs, are not whole octets of one group, or pass 256; intermediate sizes of one and of several tiles
-@pytest.mark.parametrize("rank,inter", [(64, 128), (80, 256), (256, 384), (328, 128)])
+@pytest.mark.parametrize("rank,inter", [(64, 128), (80, 256), (256, 384), (328, 128), (384, 256)])
 @pytest.mark.parametrize("counts", [(1, 0, 127, 128, 129, 7), (9, 8, 300, 0, 255, 257), (512,)])
 def test_packed_experts_match_generic_kernel(rank, inter, counts):
     cfg = synth.tiny(hidden=128, num_experts=len(counts), intermediate=inter, top_k=1, rank=rank)
