@@ -914,6 +914,11 @@ static int xt_rows(const bm_layer* L, double load, double* us) {
   *us = take64 ? t64 : t128;
   return take64 ? 64 : 128;
 }
+double experts_tc_us(const bm_layer* L, double load) {
+  double us;
+  xt_rows(L, load, &us);
+  return us;
+}
 
 template <int ROWS, bool WIDE>
 static int xt_launch(XtArgs a, size_t smem, cudaStream_t st) {

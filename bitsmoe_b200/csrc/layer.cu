@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <new>
 #include <string>
 
@@ -37,7 +38,9 @@ int launch_experts_decode(const bm_layer* L, const __half* h_gate, const __half*
 int plan_experts_batch(bm_layer* L);
 int launch_experts_batch(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices, const int32_t* expert_offsets,
                          const float* route_w, int T, float* rank_accum, long long* acc64, cudaStream_t st);
+bool experts_batch_even_shares(int all, int per, int grid);
 bool experts_tc_fits(const bm_layer* L);
+double experts_tc_us(const bm_layer* L, double load);
 int expected_passes(int experts, double load, int size);
 int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
                       const int32_t* expert_offsets, const float* route_w, int T, int expected_assign, float* rank_accum, long long* acc64,
@@ -509,34 +512,70 @@ int bm::expected_passes(int experts, double load, int size) {
     }
   }
   double p = std::exp(-load), at_most = p;
-  for (int n = 0, next = 0;;) {
+  for (int n = 0, next = 0; 1.0 - at_most >= 1e-4;) {
     if (n == next) {
-      if (1.0 - at_most < 1e-4) return static_cast<int>(experts * passes + 0.5);
       passes += 1.0 - at_most;
       next += size;
     }
     at_most += p *= load / ++n;
   }
+  return static_cast<int>(experts * passes + 0.5);
 }
-// Tiles, one after the other, of the CTA with the most where `passes` units of all tiles go over a grid of two CTAs an SM in whole rounds,
-// and what is left as a round cut along the tiles (with `cut_last` always, else only as the first one).  Where there is no more than a third
-// of a round it counts half: its CTAs have an SM each.
-static double longest_cta(int passes, int tiles, int grid, bool cut_last) {
-  const int rest = passes % grid, full = passes / grid, split = rest && (cut_last || !full) ? std::max(1, grid / rest) : 1;
-  const int per = (tiles + split - 1) / split, units = rest * ((tiles + per - 1) / per);
-  return full * tiles + (rest == 0 ? 0.0 : !full && 3 * units <= grid ? 0.5 * per : per);
+// What the two kernels of passes take, us, as a model: both are as slow as their longest CTA.  `slots`: row slots of a matrix in units of 256.
+// The costs of a unit and of a tile are fits to the stage of twelve layer shapes (8 to 512 experts, 4 to 16 tiles, rank 128 to 384) at 3 to
+// 32 assignments an expert (off by 4 to 8 %, most of it where the passes are about to need another round, so that each takes the mean of
+// three numbers of passes); choices spread evenly.  With the tensor path's estimate (experts_tc.cu) they choose the kernel: over these
+// shapes at 3 to 64 assignments an expert the layer call takes 1.003 of the fastest kernel's time, 1.008 where the experts' shares fall as
+// rank^-0.5 and 1.035 as 1 / rank, which nobody on the host knows.
+template <typename F>
+static double mean_near(int passes, F tiles) {
+  double sum = 0.0;
+  for (const double q : {0.95, 1.0, 1.05}) sum += tiles(std::max(1, static_cast<int>(q * passes + 0.5)));
+  return sum / 3.0;
 }
-// Whether passes of 16 (experts_batch_kernel) take less time than passes of 8 (experts_decode_kernel).  Both are as slow as their longest
-// CTA: 7.3 us and 5.2 a tile against 7 and 4.1, and with one pass more than half of the grid a CTA has twice the tiles.  us of the stage with
-// passes of 8 / of 16: 128 experts of 6 tiles, 4 assignments each 18.9 / 22.2, 7 each 30.9 / 23.0, 12 each 32.1 / 23.0, 14 each 31.9 / 38.4, 16 each
-// 46.3 / 38.2; 160 experts of 12 tiles, 8 each 56.7 / 70.1, 12 each 84.9 / 70.2; 16 of 4 tiles, 8 each 9.1 / 10.4; 48 of 6 tiles, 6 each 14.9 / 12.4; 512
-// of 4 tiles, 7 each 51.7 / 53.7 (under a skewed load passes of 8 are more: a block of 330 tokens 104 / 96), 9 each 60.5 / 54.0.  Over 19 shapes
-// at 2 to 24 assignments an expert this takes 1.001 of the faster kernel's time.
-static bool batch_passes_pay(const bm_layer* L, double load) {
-  if (load <= 4.0) return false;      // one pass of 8 for nearly every expert
-  const double t8 = longest_cta(expected_passes(L->num_experts, load, FAST_MAX_TOK), L->n_tiles, L->dec_grid, false);
-  const double t16 = longest_cta(expected_passes(L->num_experts, load, 2 * FAST_MAX_TOK), L->n_tiles, L->bat_grid, true);
-  return 7.3 + 5.2 * t16 < 7.0 + 4.1 * t8;
+// experts_decode_kernel: a first round is cut along the tiles, later ones are not.  A round of at most half of the grid has an SM to a CTA.
+static double decode_us(const bm_layer* L, double load, double slots) {
+  const int grid = L->dec_grid, tiles = L->n_tiles;
+  const double longest = mean_near(expected_passes(L->num_experts, load, FAST_MAX_TOK), [&](int passes) {
+    const int rest = passes % grid, full = passes / grid;
+    if (full == 0) {
+      const int split = std::min(tiles, grid / passes), per = (tiles + split - 1) / split;
+      return 8 * passes * ((tiles + per - 1) / per) <= 3 * grid ? 0.5 * per : per;
+    }
+    return full * tiles + (rest == 0 ? 0.0 : 2 * rest <= grid ? 0.65 * tiles : tiles) + 0.9 * (full - (rest == 0));
+  });
+  return 5.0 + 2.0 * slots + 1.95 * (1.0 + slots) * longest * (L->dec_ctas == 1 ? 0.6 : 1.0);
+}
+// experts_batch_kernel: the last round is cut, evenly where that saves a tile, and a second unit costs nearly one.  Inside a call its start
+// hides less behind the launches before it than the other one's (1.5 us).
+static double batch_us(const bm_layer* L, double load, double slots) {
+  const int grid = L->bat_grid, tiles = L->n_tiles;
+  return 4.5 + 4.5 * slots + mean_near(expected_passes(L->num_experts, load, 2 * FAST_MAX_TOK), [&](int passes) {
+    const int rest = passes % grid, full = passes / grid;
+    const int split = rest ? std::min(tiles, grid / rest) : 1, per = (tiles + split - 1) / split;
+    const bool even = rest && experts_batch_even_shares(rest * tiles, per, grid);
+    const double last = rest == 0 ? 0.0 : even ? static_cast<double>(rest) * tiles / grid : full == 0 && 3 * rest * ((tiles + per - 1) / per) <= grid ? 0.5 * per : per;
+    const int more = full - (rest == 0) + even;      // units after the first
+    return (0.9 + 4.3 * slots) * (full * tiles + last) + 4.8 * slots * more;
+  });
+}
+// The kernel for `expected` assignments of at most `num_assign`: the one with the smallest estimate that the layer allows.  us of the stage with passes of
+// 8 / of 16 / on tcgen05: 128 experts of 6 tiles, 4 assignments each 18.9 / 22.2 / 38, 7 each 31.0 / 23.1 / 38, 14 each 31.5 / 31.2 / 38, 20 each
+// 46.6 / 36.5 / 38.8, 28 each 57 / 38.8 / 39.5; 160 of 12 tiles, 8 each 56.3 / 48.4 / 74, 24 each 105 / 78.7 / 74.7; 16 of 4 tiles, 8 each 9.0 / 10.5 / 13, 32
+// each 10.8 / 12.6 / 14.2; 512 of 4 tiles, 7 each 50.7 / 51.5 / 85, 20 each 99.9 / 82.8 / 85.8.
+static int choose_path(const bm_layer* L, int32_t num_assign, int32_t expected) {
+  const double load = static_cast<double>(expected) / L->num_experts, slots = L->max_slots / 256.0;
+  const bool decode = L->fast_ok && L->dec_ok && num_assign / FAST_MAX_TOK + L->num_experts < 60000;
+  int path = BM_PATH_GENERIC;
+  double best = std::numeric_limits<double>::infinity();
+  auto take = [&](int candidate, double us) { if (us < best) { best = us; path = candidate; } };
+  const bool tensor = L->fast_ok && experts_tc_fits(L);
+  if (tensor) take(BM_PATH_TENSOR, experts_tc_us(L, load));
+  if (load <= 64.0 || !tensor) {
+    if (decode) take(BM_PATH_DECODE, decode_us(L, load, slots));
+    if (L->bat_ring && (load > 4.0 || !decode)) take(BM_PATH_BATCH, batch_us(L, load, slots));      // (up to 4 one pass of 8 is enough for nearly every expert)
+  }
+  return path;
 }
 
 // `num_assign` bounds the list's length, `expected` is what the choice of a kernel takes it for.
@@ -576,15 +615,7 @@ static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, con
              "experts_forward: the batch path needs 1- to 4-bit rows and full tiles; this layer has neither");
   const __half* hg = reinterpret_cast<const __half*>(h_gate);
   const __half* hu = reinterpret_cast<const __half*>(h_up);
-  if (path == BM_PATH_AUTO) {
-    // Up to 24 assignments an expert passes cost less than turning every expert into tensor-core operands (400 tokens, top 8 of 128
-    // experts, 25 each: 39 us against 40; 512 tokens, 32 each: 47 against 40).
-    const int64_t per16 = static_cast<int64_t>(expected) * 16 / L->num_experts;      // assignments per expert, in sixteenths
-    const bool decode = L->dec_ok && num_assign / FAST_MAX_TOK + L->num_experts < 60000, few = L->bat_ring && per16 <= 24 * 16;
-    if (few && (!decode || batch_passes_pay(L, static_cast<double>(expected) / L->num_experts))) path = BM_PATH_BATCH;
-    else if (L->fast_ok && per16 > 16 * 16 && !few && experts_tc_fits(L)) path = BM_PATH_TENSOR;
-    else path = L->fast_ok && decode ? BM_PATH_DECODE : BM_PATH_GENERIC;
-  }
+  if (path == BM_PATH_AUTO) path = choose_path(L, num_assign, expected);
   if (path == BM_PATH_TENSOR)
     rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, expected, rank_accum, acc64, st);
   else if (path == BM_PATH_BATCH)

@@ -118,7 +118,7 @@ def test_named_kernels_run_at_any_load():
 # passes), alone and behind a whole round; a share holds the end of one pass and the start of the next
 @pytest.mark.parametrize("passes", [148, 149, 150, 197, 198, 246, 247, 296, 297, 296 + 149, 296 + 246])
 def test_passes_in_even_shares(passes):
-    E, T = 8, 960
+    E, T = 8, 1200
     cfg = synth.tiny(hidden=128, num_experts=E, intermediate=768, top_k=1, rank=64)
     layer = synth.to_packed_layer(synth.make_layer(cfg, seed=11, device=DEV))
     layer.set_deterministic(True)
@@ -133,14 +133,14 @@ def test_passes_in_even_shares(passes):
     assert torch.equal(*got)
 
 
-# The automatic choice, told by its bits in deterministic mode: passes of 16 where they leave the longest CTA less work than passes of 8
-# (not with a tile a CTA either way, nor where they just exceed half of the grid), products on tcgen05 above 24 assignments an expert
-@pytest.mark.parametrize("E,inter,load,path", [(16, 512, 8, capi.PATH_DECODE), (16, 1536, 12, capi.PATH_BATCH), (48, 768, 6, capi.PATH_BATCH),
+# The automatic choice, told by its bits in deterministic mode: passes of 8 while one is enough for most experts or where few experts leave
+# room to cut them, passes of 16 up to about 24 assignments an expert, products on tcgen05 above
+@pytest.mark.parametrize("E,inter,load,path", [(16, 512, 8, capi.PATH_DECODE), (16, 1536, 20, capi.PATH_DECODE), (48, 768, 6, capi.PATH_DECODE),
                                                (128, 768, 4, capi.PATH_DECODE), (128, 768, 8, capi.PATH_BATCH), (128, 768, 12, capi.PATH_BATCH),
-                                               (128, 768, 14, capi.PATH_DECODE), (128, 768, 17, capi.PATH_BATCH), (128, 768, 25, capi.PATH_TENSOR),
-                                               (160, 1536, 8, capi.PATH_DECODE), (160, 1536, 12, capi.PATH_BATCH)])
+                                               (128, 768, 18, capi.PATH_BATCH), (128, 768, 40, capi.PATH_TENSOR), (160, 1536, 4, capi.PATH_DECODE),
+                                               (160, 1536, 8, capi.PATH_BATCH), (160, 1536, 26, capi.PATH_TENSOR)])
 def test_automatic_choice_of_kernel(E, inter, load, path):
-    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=inter, top_k=1, rank=64)
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=inter, top_k=1, rank=256)
     layer = synth.to_packed_layer(synth.make_layer(cfg, seed=8, device=DEV))
     layer.set_deterministic(True)
     gen = torch.Generator(device=DEV).manual_seed(13)
@@ -155,7 +155,7 @@ def test_automatic_choice_of_kernel(E, inter, load, path):
 @pytest.mark.parametrize("T,path", [(96, capi.PATH_DECODE), (128, capi.PATH_DECODE), (256, capi.PATH_BATCH), (512, capi.PATH_TENSOR)])
 def test_a_shard_is_chosen_for_by_its_share(T, path):
     E, routed, k = 64, 128, 8
-    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=768, top_k=k, rank=64)
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=768, top_k=k, rank=256)
     layer = synth.to_packed_layer(synth.make_layer(cfg, seed=9, device=DEV))
     layer.set_deterministic(True)
     gen = torch.Generator(device=DEV).manual_seed(14)
@@ -171,8 +171,8 @@ def test_a_shard_is_chosen_for_by_its_share(T, path):
 
 # lists shorter than their bound (a rank of an expert-parallel group): chosen for the expected length, right for any
 def test_expected_length_chooses_the_kernel():
-    E, bound, load = 48, 48 * 6, [3] * 48
-    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=768, top_k=1, rank=64)
+    E, bound, load = 48, 48 * 22, [3] * 48
+    cfg = synth.tiny(hidden=128, num_experts=E, intermediate=768, top_k=1, rank=256)
     layer = synth.to_packed_layer(synth.make_layer(cfg, seed=10, device=DEV))
     layer.set_deterministic(True)
     lib, gen, T = capi.lib(), torch.Generator(device=DEV).manual_seed(16), 64
