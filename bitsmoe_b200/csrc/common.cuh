@@ -301,6 +301,7 @@ struct bm_layer {
   bool deterministic = false;      // rank_accum through 64-bit fixed-point atomics (bm_layer_set_option)
   int dec_ring = 0, dec_sec_bytes = 0, dec_grid = 0, dec_act_bufs = 2, dec_ctas = 0, dec_force_ctas = 0;
   size_t dec_smem = 0;
+  int sms = 148;                   // of the device that the layer was created on
   int bat_ring = 0, bat_sec_bytes = 0, bat_smem = 0, bat_grid = 0;      // of experts_batch_kernel (bat_ring 0: not for this layer)
   int wait_limit_us = bm::DEFAULT_WAIT_LIMIT_US;   // of the packed-expert kernels' waits (bm_layer_set_option)
   int* status_dev = nullptr;       // device flag set by a kernel whose bounded wait gave up

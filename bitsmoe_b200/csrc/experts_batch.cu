@@ -547,10 +547,11 @@ bool experts_batch_even_shares(int all, int per, int grid) { return bt_even_shar
 // Ring depth and grid for this layer on the current device; bat_ring = 0 where the layer does not suit the kernel.
 int plan_experts_batch(bm_layer* L) {
   L->bat_ring = 0;
-  if (!L->fast_ok || !L->toktab_dev || L->num_experts > BT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > 512 || L->rank_in % 8 != 0) return BM_OK;
   int dev = -1, sm_count = 0, smem_sm = 0;
   BM_CUDA(cudaGetDevice(&dev));
   BM_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
+  L->sms = sm_count;
+  if (!L->fast_ok || !L->toktab_dev || L->num_experts > BT_MAX_E || L->intermediate % N_TILE != 0 || L->max_slots > 512 || L->rank_in % 8 != 0) return BM_OK;
   BM_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
   const void* kernel = L->max_slots <= 256 ? reinterpret_cast<const void*>(experts_batch_kernel<2>) : reinterpret_cast<const void*>(experts_batch_kernel<4>);
   cudaFuncAttributes fa;

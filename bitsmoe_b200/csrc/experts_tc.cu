@@ -35,7 +35,7 @@
 // the converter warps (an MMA of 64 rows takes as long as one of 128, but N = 128 halves their number); a stage is about 280
 // instructions at 8 cycles each, and what the instruction cache holds of 24 warps in different roles matters: a copy of the
 // loop for each kind of stage took 60 us where one for all takes 40 (203 tokens), one for gate/up and down together 42.
-// Stage of 8192 tokens of 128 experts (rank 256, intermediate 768): 121 us (176 before weights were converted in pairs), 2048
+// Stage of 8192 tokens of 128 experts (rank 256, intermediate 768): 118 us (176 before weights were converted in pairs), 2048
 // tokens 59 (72), 777 tokens 45 (59), 300 tokens 40 (50); of 512 experts: 16384 tokens 235 us (318), 2048 tokens 99 (125 with 128
 // rows), 1050 tokens 90 (114).
 // The mapped arrivals carry no cluster-scope release: what they publish is read by the tensor core of the CTA that wrote it, behind
@@ -890,9 +890,7 @@ bool experts_tc_fits(const bm_layer* L) {
 // The stage as a model, us: the tiles and units of the pair with the most, items of `2 nt` assignments spread evenly.  Fits to thirteen layer shapes (8
 // to 512 experts, 4 to 16 tiles, rank 128 to 384) at 17 to 180 assignments an expert, off by 4 %.
 static double xt_us(const bm_layer* L, int rows, int nt, double load) {
-  int dev = -1, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int pairs = sms / 2, items = std::max(1, expected_passes(L->num_experts, load, 2 * nt)), rest = items % pairs, full = items / pairs;
+  const int pairs = L->sms / 2, items = std::max(1, expected_passes(L->num_experts, load, 2 * nt)), rest = items % pairs, full = items / pairs;
   const int split = rest ? std::min(L->n_tiles, pairs / rest) : 1, last = rest ? (L->n_tiles + split - 1) / split : 0;
   const double tiles = full * L->n_tiles + last, more = full - (rest == 0), slots = L->max_slots / 256.0;
   if (L->max_slots > 256) return 14.7 + 3.6 * tiles + 2.6 * more;
@@ -914,9 +912,9 @@ static int xt_rows(const bm_layer* L, double load, double* us) {
   *us = take64 ? t64 : t128;
   return take64 ? 64 : 128;
 }
-double experts_tc_us(const bm_layer* L, double load) {
+double experts_tc_us(const bm_layer* L, double load, int* rows) {
   double us;
-  xt_rows(L, load, &us);
+  *rows = xt_rows(L, load, &us);
   return us;
 }
 
@@ -942,7 +940,7 @@ static int xt_launch(XtArgs a, size_t smem, cudaStream_t st) {
 }
 
 int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
-                      const int32_t* expert_offsets, const float* route_w, int T, int expected_assign, float* rank_accum, long long* acc64,
+                      const int32_t* expert_offsets, const float* route_w, int T, int expected_assign, int rows, float* rank_accum, long long* acc64,
                       cudaStream_t st) {
   BM_REQUIRE(L->num_experts <= XT_MAX_E, BM_ERR_UNSUPPORTED, "experts_tc: more than %d experts", XT_MAX_E);
   BM_REQUIRE(L->intermediate % N_TILE == 0, BM_ERR_UNSUPPORTED, "experts_tc: intermediate size must be a multiple of %d", N_TILE);
@@ -950,7 +948,7 @@ int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_u
   BM_REQUIRE(L->rank_in % 8 == 0 && ((reinterpret_cast<uintptr_t>(h_gate) | reinterpret_cast<uintptr_t>(h_up)) & 15u) == 0,
              BM_ERR_UNSUPPORTED, "experts_tc: rank-space rows must be 16-byte aligned (rank %d)", L->rank_in);
   double us;
-  const int rows = xt_rows(L, static_cast<double>(expected_assign) / L->num_experts, &us);
+  if (rows == 0) rows = xt_rows(L, static_cast<double>(expected_assign) / L->num_experts, &us);
   XtPlan plan;
   BM_REQUIRE(xt_plan(L, rows, &plan), BM_ERR_UNSUPPORTED, "experts_tc: the layer's largest expert does not fit in shared memory");
   XtArgs a{};

@@ -40,10 +40,10 @@ int launch_experts_batch(const bm_layer* L, const __half* h_gate, const __half* 
                          const float* route_w, int T, float* rank_accum, long long* acc64, cudaStream_t st);
 bool experts_batch_even_shares(int all, int per, int grid);
 bool experts_tc_fits(const bm_layer* L);
-double experts_tc_us(const bm_layer* L, double load);
+double experts_tc_us(const bm_layer* L, double load, int* rows);
 int expected_passes(int experts, double load, int size);
 int launch_experts_tc(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
-                      const int32_t* expert_offsets, const float* route_w, int T, int expected_assign, float* rank_accum, long long* acc64,
+                      const int32_t* expert_offsets, const float* route_w, int T, int expected_assign, int rows, float* rank_accum, long long* acc64,
                       cudaStream_t st);
 int launch_experts_generic(const bm_layer* L, const __half* h_gate, const __half* h_up, const int32_t* token_indices,
                            const int32_t* expert_offsets, const float* route_w, int T, float* rank_accum,
@@ -504,6 +504,7 @@ extern "C" size_t bm_experts_workspace_bytes(const bm_layer_t* L, int32_t T, int
 // spread evenly over the experts): experts * sum over j of P(more than j * size).
 int bm::expected_passes(int experts, double load, int size) {
   double passes = 0.0;
+  if (size > load + 5.0 * std::sqrt(load) + 5.0) return static_cast<int>(experts * (1.0 - std::exp(-load)) + 0.5);      // one at most
   if (load > 32.0) {      // a normal number is close enough, and its sum has few terms
     for (int n = 0;; n += size) {
       const double more = 0.5 * std::erfc((n + 0.5 - load) / std::sqrt(2.0 * load));
@@ -563,14 +564,14 @@ static double batch_us(const bm_layer* L, double load, double slots) {
 // 8 / of 16 / on tcgen05: 128 experts of 6 tiles, 4 assignments each 18.9 / 22.2 / 38, 7 each 31.0 / 23.1 / 38, 14 each 31.5 / 31.2 / 38, 20 each
 // 46.6 / 36.5 / 38.8, 28 each 57 / 38.8 / 39.5; 160 of 12 tiles, 8 each 56.3 / 48.4 / 74, 24 each 105 / 78.7 / 74.7; 16 of 4 tiles, 8 each 9.0 / 10.5 / 13, 32
 // each 10.8 / 12.6 / 14.2; 512 of 4 tiles, 7 each 50.7 / 51.5 / 85, 20 each 99.9 / 82.8 / 85.8.
-static int choose_path(const bm_layer* L, int32_t num_assign, int32_t expected) {
+static int choose_path(const bm_layer* L, int32_t num_assign, int32_t expected, int* rows) {
   const double load = static_cast<double>(expected) / L->num_experts, slots = L->max_slots / 256.0;
   const bool decode = L->fast_ok && L->dec_ok && num_assign / FAST_MAX_TOK + L->num_experts < 60000;
   int path = BM_PATH_GENERIC;
   double best = std::numeric_limits<double>::infinity();
   auto take = [&](int candidate, double us) { if (us < best) { best = us; path = candidate; } };
   const bool tensor = L->fast_ok && experts_tc_fits(L);
-  if (tensor) take(BM_PATH_TENSOR, experts_tc_us(L, load));
+  if (tensor && (load > 8.0 || !(decode || L->bat_ring))) take(BM_PATH_TENSOR, experts_tc_us(L, load, rows));
   if (load <= 64.0 || !tensor) {
     if (decode) take(BM_PATH_DECODE, decode_us(L, load, slots));
     if (L->bat_ring && (load > 4.0 || !decode)) take(BM_PATH_BATCH, batch_us(L, load, slots));      // (up to 4 one pass of 8 is enough for nearly every expert)
@@ -615,9 +616,10 @@ static int experts_forward_impl(const bm_layer_t* L, const uint16_t* h_gate, con
              "experts_forward: the batch path needs 1- to 4-bit rows and full tiles; this layer has neither");
   const __half* hg = reinterpret_cast<const __half*>(h_gate);
   const __half* hu = reinterpret_cast<const __half*>(h_up);
-  if (path == BM_PATH_AUTO) path = choose_path(L, num_assign, expected);
+  int rows = 0;      // of the tensor path's CTAs, where the choice has looked at them
+  if (path == BM_PATH_AUTO) path = choose_path(L, num_assign, expected, &rows);
   if (path == BM_PATH_TENSOR)
-    rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, expected, rank_accum, acc64, st);
+    rc = launch_experts_tc(L, hg, hu, token_indices, expert_offsets, route_weights, T, expected, rows, rank_accum, acc64, st);
   else if (path == BM_PATH_BATCH)
     rc = launch_experts_batch(L, hg, hu, token_indices, expert_offsets, route_weights, T, rank_accum, acc64, st);
   else if (path == BM_PATH_DECODE)
