@@ -724,13 +724,14 @@ extern "C" size_t bm_layer_workspace_bytes(const bm_layer_t* L, int32_t T, int32
 // BM_ERR_UNSUPPORTED, with nothing launched, when a shape does not tile; the general path takes it.
 //
 // Up to how many tokens, where the chain of tiled products (forward_large, the general layer path) takes the sizes.  The limits are
-// crossovers of three layer shapes, us a call of these launches / of the chain.  Layer of 128 experts, fp16: 56 tokens 30.4 / 32.9, 80 32.7 /
-// 33.2, 112 38.2 / 37.3, 200 47.9 / 38.4; of 64 experts, bf16, whose rows the chain rounds in shared memory: 112 tokens 35.7 / 37.6, 129 39.2 / 37.8.
-// Block of 128 experts, bf16: 65 tokens 39.6 / 39.9, 81 40.2 / 40.3, 112 46.4 / 45.2, 200 65.6 / 47.4; of 512 experts and a gated shared one: 40
-// tokens 55.1 / 56.6, 49 74.2 / 74.3, 64 82.9 / 75.4, 96 117 / 78.  Other shapes cross elsewhere, as the first launch grows with rows and chunks
-// of 64 tokens and the routing cluster with tokens times experts.  Earlier: a gated block of 64 experts at 40 tokens 41.4 / 40.4, a block of
-// 256 experts and hidden size 4096 with a shared one at 40 tokens 75.6 / 61.2 and without at 65 tokens 81.3 / 57.3, a layer of 512 experts at 56
-// tokens 56.6 / 50.2.  Later, by 0.8 us at most: fp16 layers of 16 to 128 experts up to 96 tokens.
+// crossovers of three shapes of hidden size 2048, us a call of these launches / of the chain.  Layer of 128 experts, fp16: 56 tokens 29.8 / 31.3, 72 32.3 /
+// 32.0, 112 37.8 / 36.2; of 64 experts, bf16, whose rows the chain rounds in shared memory: 112 tokens 36.5 / 37.4, 129 39.7 / 37.9.  Block of 128
+// experts, bf16: 64 tokens 37.5 / 38.7, 80 39.8 / 39.2, 112 46.2 / 43.9; of 512 experts and a gated shared one: 40 tokens 52.7 / 53.5, 48 71.0 / 71.3, 64
+// 80.1 / 73.1.  Other shapes cross elsewhere, as the first launch grows with rows, hidden size and chunks of 64 tokens and the routing cluster
+// with tokens times experts.  Earlier: layers of 160 experts and hidden size 5120 (56 tokens 57.2 / 52.3, 112 83.6 / 71.6), of 512 experts (56: 54.5 /
+// 49.3); blocks of 256 experts and hidden size 4096 (24: 66.4 / 65.1, 72: 140 / 98), of 160 and 5120 (48: 59.5 / 57.7, 72: 94.9 / 70.3); with a gated shared
+// expert blocks of 16 to 128 experts (40: 36.9 / 34.2, 44.4 / 43.7, 46.4 / 44.1) and of 256 (24: 81.7 / 75.0, 40: 138 / 110).  Later, by 0.9 us at most: fp16
+// layers of 16 and 64 experts up to 128 and 96 tokens.
 static int small_tokens(const bm_layer_t* L, const bm_block_dense_t* d, int x_dtype) {
   const bool shared = d && d->sh_intermediate > 0;
   if (L->hidden % 64 != 0 || L->rank_in % 8 != 0 || L->rank_out % 64 != 0 || (shared && d->sh_intermediate % 64 != 0) || (d && L->num_experts % 8 != 0))
